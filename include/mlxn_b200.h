@@ -358,7 +358,7 @@ int mlxn_peer_barrier(mlxn_encoder *enc, uint32_t rank, uint32_t world, void *co
 
 /* ---- tuning and introspection (no upstream counterpart) -------------------------------------- */
 /* Selects kernel variants for cross-checks: key/value pairs
- *   "qmv" = auto | mma | tc | stream | simple   (auto: per shape and m, the fastest of the register-level tensor-core
+ *   "qmv" = auto | split | mma | tc | stream | simple   (auto: per shape and m, the fastest of the register-level tensor-core
  *           kernel "mma" and the tensor-memory kernel "tc", the streaming SIMT kernel for shapes neither takes;
  *           mma, stream and simple give bit-reproducible results, tc may differ in the last bit from run to run),
  *   "qmm" = tc | simt,

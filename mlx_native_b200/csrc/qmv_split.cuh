@@ -1,0 +1,1294 @@
+// Mat-vec for few activation rows, dense and expert-routed: y[m, n] = x[m, k] . W[n, k]^T with W in GGML blocks.
+//
+// HBM bounds the operation (6.4 TB/s measured copy rate: 23 bytes per cycle and SM); what a kernel loses against that is latency
+// (launch, activations, waits between stages) and instructions (integer operations issue at half rate).  Hence:
+//
+//  * The activations of a CTA stay in shared memory for all its weight rows: f16 hi + lo halves (scaled by a power of two per
+//    row, so that both stay in range), in the order of the B registers of mma.sync.m16n8k16.  One row is split by every CTA
+//    itself (2 us, less than another launch), several rows by qmv_pack_kernel, and arrive by bulk copies.  The loop over the
+//    weights only unpacks codes: the raw 4/5/6/8-bit codes as f16 subnormals (exact integers n 2^-24), so products are exact and
+//    sums are f32.
+//  * The 8 columns of an MMA are (activation row, hi | lo): one multiply serves up to four rows (NS = 2 sets: eight rows).
+//  * A warp works on up to four 16-row tiles at a time: one tile at a time leaves the pipes idle between dependent steps (Q4_0,
+//    75776 x 4096: 2.7 TB/s against 5.0).
+//  * K may be split over the CTAs of a cluster (1, 2, 4, 8): a matrix of few rows still fills the chip, and long activation rows
+//    still fit into shared memory.  The ranks' partial sums travel through distributed shared memory (st.async) and are added in
+//    rank order by the CTA that owns the row: no atomics, results are bit-reproducible.
+//  * A producer warp fills a ring of stages (16-row tiles x SU units of 64 K values) by TMA: tensor copies where every weight row
+//    starts on a 16-byte boundary (ALN), else one bulk copy per row of the 16-byte superset of its segment, so every K that is a
+//    multiple of the block and every 2-byte aligned weight address takes this kernel (Q8_0 2873 x 2880, five rows: 11.7 us where
+//    the kernel that reads blocks from global memory took 181).
+//  * Expert-routed: every CTA sorts the (token, slot) pairs by expert itself (at most 256 pairs), and the rows of one expert share
+//    a pass over its weights, four at a time.
+#pragma once
+#include "tensor_map.cuh"
+
+#include <cstdio>
+#include <cstdlib>
+#include <atomic>
+#include <cmath>
+#include <type_traits>
+
+#include "common.cuh"
+#include "ptx.cuh"
+
+namespace mlxn {
+
+constexpr int kSpWarps = 8;                         // consumer warps
+constexpr int kSpThreads = (kSpWarps + 1) * 32;     // and one producer warp
+constexpr int kSpTiles = 4;                         // 16-row tiles of a chunk, at most
+__host__ __device__ constexpr int sp_tiles(int sets) { return sets == 2 ? 2 : kSpTiles; }
+constexpr int kSpMaxOps = 8;                        // mat-vecs one launch carries
+constexpr int kSpMaxSlots = 8;
+constexpr int kSpMaxPairs = 256;                    // (token, slot) pairs of a routed launch
+
+// SU: units (64 K values) of a stage, a multiple of the warps.  NG: scale groups of a unit.  OFF: code bias.
+template <int T> struct SpTraits;
+template <> struct SpTraits<GT_Q4_0> { static constexpr int B256 = 144, SU = 16, NG = 2, OFF = 8; };
+template <> struct SpTraits<GT_Q8_0> { static constexpr int B256 = 272, SU = 8, NG = 2, OFF = 128; };
+template <> struct SpTraits<GT_Q4_K> { static constexpr int B256 = 144, SU = 16, NG = 2, OFF = 1; };
+template <> struct SpTraits<GT_Q5_K> { static constexpr int B256 = 176, SU = 16, NG = 2, OFF = 1; };
+template <> struct SpTraits<GT_Q6_K> { static constexpr int B256 = 210, SU = 8, NG = 4, OFF = 32; };
+
+// Bytes of shared memory per row of a stage: an odd multiple of 16 (32-bit reads of eight rows hit distinct banks).
+template <int T> __host__ __device__ constexpr uint32_t sp_pitch(bool aln) {
+    const uint32_t lead = aln && T != GT_Q6_K ? 0u : 14u;
+    return 16u * (((SpTraits<T>::SU / 4 * SpTraits<T>::B256 + lead + 15u) / 16u) | 1u);
+}
+
+struct SpOp {
+    const uint8_t *w;
+    const float *x;
+    const float *x2;          // fused SwiGLU: the activations are silu(x) * x2
+    float *y;
+    uint32_t n, k, m;
+    uint32_t chunk_end;       // chunks (of tr tiles) of the ops up to and including this one
+    uint32_t row_bytes;
+    uint32_t units;           // ceil(k / 64)
+    uint32_t slice;           // units per cluster rank (a multiple of 4)
+    uint32_t xkey;            // ops with equal keys have the same activations
+    uint32_t x_div;           // routed: the activation row of pair p is p / x_div
+    uint32_t y_ld, y_col0, n_peer;
+    float *y_peer[kMaxPeers];
+    uint64_t expert_stride;
+    // packed activations (see qmv_pack_kernel): per row pk_units x 256 bytes of B registers, pk_units x NG bias sums, one scale
+    const uint8_t *xp;
+    const float *xsum, *xinv;
+    uint32_t pk_units;
+    uint32_t row_end;         // rows to pack of the ops up to and including this one
+};
+struct SpBatch {
+    SpOp op[kSpMaxOps];
+    const uint32_t *ids;      // routed: expert of every pair
+    uint32_t nops, npairs, n_experts;
+    uint32_t nent;            // dense: groups of mp activation rows; routed: counted on the device
+    uint32_t mp;              // activation rows of an entry (1, 2, 4 or 8)
+    uint32_t tr;              // tiles of a chunk
+    uint32_t run;             // consecutive chunks a cluster takes at a time (0: a contiguous share)
+    uint32_t early_weights;
+    uint32_t *status;
+    uint32_t nslots;          // ring depth, and what lies behind the ring in shared memory
+    uint32_t xf_off, cc_off, tab_off, red_off, recv_off;
+    uint32_t xstride, cstride;   // bytes from one activation row to the next
+    uint32_t packed;          // the activations have been packed by qmv_pack_kernel
+};
+struct SpMaps {
+    CUtensorMap m[kSpMaxOps];
+};
+
+// ---- shared-memory access by 32-bit address -----------------------------------------------------------
+namespace sp {
+__device__ __forceinline__ uint32_t ld32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+template <uint32_t OFF> __device__ __forceinline__ uint32_t ld32i(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+template <uint32_t OFF> __device__ __forceinline__ uint32_t ld16i(uint32_t a) {
+    uint32_t v;
+    asm volatile("{ .reg .u16 t; ld.shared.u16 t, [%1+%2]; cvt.u32.u16 %0, t; }" : "=r"(v) : "r"(a), "n"(OFF));
+    return v;
+}
+template <uint32_t OFF> __device__ __forceinline__ void ld128i(uint32_t a, uint32_t (&v)[4]) {
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4+%5];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a), "n"(OFF));
+}
+__device__ __forceinline__ void st32(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void st64(uint32_t a, uint32_t v0, uint32_t v1) {
+    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(v0), "r"(v1) : "memory");
+}
+__device__ __forceinline__ void st128(uint32_t a, float v0, float v1, float v2, float v3) {
+    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(a), "f"(v0), "f"(v1), "f"(v2), "f"(v3) : "memory");
+}
+__device__ __forceinline__ float h_lo(uint32_t w) {
+    float f;
+    asm("{ .reg .f16 l, h; mov.b32 {l, h}, %1; cvt.f32.f16 %0, l; }" : "=f"(f) : "r"(w));
+    return f;
+}
+__device__ __forceinline__ float h_hi(uint32_t w) {
+    float f;
+    asm("{ .reg .f16 l, h; mov.b32 {l, h}, %1; cvt.f32.f16 %0, h; }" : "=f"(f) : "r"(w));
+    return f;
+}
+// D = A (16 x 16) B (16 x 8) + C: lane (g = lane / 4, t = lane % 4) holds a0/a1 = rows g / g + 8, k 2t..; a2/a3 the same,
+// k 2t + 8..; b0, b1 likewise for column g; c0, c1 = row g, columns 2t, 2t + 1; c2, c3 = row g + 8.
+__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1,
+                                    float c0, float c1, float c2, float c3) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+template <int I, int N, class F> __device__ __forceinline__ void each(F &&f) {
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        each<I + 1, N>(f);
+    }
+}
+}  // namespace sp
+__device__ __forceinline__ void bulk_g2s_a(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
+namespace sp {
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+// a store to another CTA's shared memory that counts as 4 arrived bytes on a barrier there
+__device__ __forceinline__ void st_async(uint32_t a, float v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a), "r"(__float_as_uint(v)), "r"(bar)
+                 : "memory");
+}
+// Power of two that brings amax into [2^13, 2^14), and its inverse; 1 for an all-zero or non-finite run.
+__device__ __forceinline__ void pow2(float amax, float &s, float &inv) {
+    s = inv = 1.f;
+    if (amax > 0.f && amax < 3.0e38f) {
+        int e = 13 + 127 - (int)((__float_as_uint(amax) >> 23) & 0xffu);
+        e = max(-100, min(100, e));
+        s = __uint_as_float((uint32_t)(e + 127) << 23);
+        inv = __uint_as_float((uint32_t)(127 - e) << 23);
+    }
+}
+}  // namespace sp
+
+// Where in its unit the four values lie that quad lane t multiplies in MMA q, as two pairs of consecutive elements.  Q4_0 and
+// Q8_0 with aligned rows work on pairs of blocks: the even block starts on a 4-byte boundary, so its codes (2 bytes in)
+// straddle the words; lanes 1..3 take whole words and lane 0 the two half words at either end, which sit in the words that
+// hold the pair's two scales.  (Q6_K: relative to the super-block.)
+template <int T, bool ALN> __device__ __forceinline__ void sp_pairs(uint32_t u, uint32_t q, uint32_t t, uint32_t &p0, uint32_t &p1) {
+    if constexpr (T == GT_Q6_K) {
+        p0 = 128u * ((u >> 1) & 1u) + 32u * q + 16u * (u & 1u) + 4u * t;
+        p1 = p0 + 2;
+    } else if constexpr ((T == GT_Q4_0 || T == GT_Q8_0) && ALN) {
+        const uint32_t h = q & 1u;
+        if (q >= 2) {
+            p0 = 32 + 16 * h + 4 * t;
+            p1 = p0 + 2;
+        } else if (T == GT_Q8_0 && h) {
+            p0 = 14 + 4 * t;
+            p1 = 16 + 4 * t;
+        } else {
+            p0 = t ? 4 * t - 2 : 0;
+            p1 = t ? 4 * t : (T == GT_Q8_0 ? 30 : 14);
+            if (T == GT_Q4_0) { p0 += 16 * h; p1 += 16 * h; }
+        }
+    } else {
+        p0 = 16u * q + 4u * t;
+        p1 = p0 + 2;
+    }
+}
+
+// One unit (64 K values) of a stage against NT tiles.  a0 / a1: shared address of rows g and g + 8 of tile 0 at the unit's
+// first byte (Q4_K, Q5_K, Q6_K: of its super-block), lead-in included; tiles are 16 PITCH bytes apart.  bf: the B registers
+// [set][MMA][2]; cc: per set and scale group what the bias (Q4_K, Q5_K: the minimum) owes; tab: the warp's scale table.
+template <int T, bool ALN, int NT, int NS, bool ONE, int TM>
+__device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, uint32_t t, uint32_t g, uint32_t tab, bool half,
+                                        const uint32_t (&bf)[NS][4][2], const float (&cc)[NS][SpTraits<T>::NG], float (&acc)[TM][NS][4]) {
+    constexpr uint32_t TS = 16u * sp_pitch<T>(ALN);
+    if constexpr (T == GT_Q4_0 || T == GT_Q8_0) {
+        constexpr bool Q8 = T == GT_Q8_0;
+        constexpr uint32_t BB = Q8 ? 34u : 18u;
+        // row g + 8 relative to row g is a compile-time distance only with aligned rows
+        const uint32_t b0[2] = {ALN ? a0 + 4 * t : (a0 & ~3u) + 4 * t, ALN ? a1 + 4 * t : (a1 & ~3u) + 4 * t};
+        const uint32_t e0 = a0 + (t ? 4 * t : (Q8 ? 32u : 16u)), e1 = a1 + (t ? 4 * t : (Q8 ? 32u : 16u));
+        const uint32_t sel = t ? 0x3210u : 0x5432u;
+        uint32_t se[2], so[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const bool mis = !ALN && ((h ? a1 : a0) & 2u) != 0;
+            se[h] = mis ? 0x7654u : 0x5432u;
+            so[h] = mis ? 0x5432u : 0x3210u;
+        }
+        sp::each<0, NT>([&](auto J) {
+            constexpr uint32_t o = decltype(J)::value * TS;
+            uint32_t w[4][2];   // even block, MMA 0 / 1; odd block, MMA 0 / 1 (Q4_0: one word per block)
+            float d0[2], d1[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t b = b0[h];
+                [[maybe_unused]] const uint32_t e = h ? e1 : e0, a = h ? a1 : a0;
+                if constexpr (ALN) {
+                    const uint32_t s0 = sp::ld32i<o>(b), s1 = sp::ld32i<o>(e);
+                    w[0][h] = __byte_perm(s0, s1, sel);
+                    if constexpr (Q8) {
+                        w[1][h] = sp::ld32i<o + 16>(b);
+                        w[2][h] = sp::ld32i<o + 36>(b);
+                        w[3][h] = sp::ld32i<o + 52>(b);
+                    } else {
+                        w[2][h] = sp::ld32i<o + 20>(b);
+                    }
+                    if constexpr (ONE) {   // one activation row: only lane 0 of a quad holds results, and it has the scales
+                        d0[h] = sp::h_lo(s0);
+                        d1[h] = sp::h_hi(s1);
+                    }
+                } else {
+                    w[0][h] = __byte_perm(sp::ld32i<o>(b), sp::ld32i<o + 4>(b), se[h]);
+                    if constexpr (Q8) {
+                        w[1][h] = __byte_perm(sp::ld32i<o + 16>(b), sp::ld32i<o + 20>(b), se[h]);
+                        w[2][h] = __byte_perm(sp::ld32i<o + 36>(b), sp::ld32i<o + 40>(b), so[h]);
+                        w[3][h] = __byte_perm(sp::ld32i<o + 52>(b), sp::ld32i<o + 56>(b), so[h]);
+                    } else {
+                        w[2][h] = __byte_perm(sp::ld32i<o + 20>(b), sp::ld32i<o + 24>(b), so[h]);
+                    }
+                }
+                if constexpr (!ALN || !ONE) {
+                    d0[h] = sp::h_lo(sp::ld16i<o>(a));
+                    d1[h] = sp::h_lo(sp::ld16i<o + BB>(a));
+                    if constexpr (!ALN) d1[h] = half ? 0.f : d1[h];
+                }
+            }
+            uint32_t a[4][4];
+            if constexpr (Q8) {   // codes + 128 as f16 subnormals: bytes 0, 2 and bytes 1, 3 of a word into halves
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const uint32_t x0 = w[q][0] ^ 0x80808080u, x1 = w[q][1] ^ 0x80808080u;
+                    a[q][0] = __byte_perm(x0, 0u, 0x4240); a[q][1] = __byte_perm(x1, 0u, 0x4240);
+                    a[q][2] = __byte_perm(x0, 0u, 0x4341); a[q][3] = __byte_perm(x1, 0u, 0x4341);
+                }
+            } else {              // low nibbles: elements 0..15; high nibbles (x 16, the activations carry 1 / 16): 16..31
+#pragma unroll
+                for (int b = 0; b < 2; b++) {
+                    const uint32_t x0 = w[2 * b][0], x1 = w[2 * b][1], y0 = x0 >> 8, y1 = x1 >> 8;
+                    a[2 * b][0] = x0 & 0x000F000Fu; a[2 * b][1] = x1 & 0x000F000Fu;
+                    a[2 * b][2] = y0 & 0x000F000Fu; a[2 * b][3] = y1 & 0x000F000Fu;
+                    a[2 * b + 1][0] = x0 & 0x00F000F0u; a[2 * b + 1][1] = x1 & 0x00F000F0u;
+                    a[2 * b + 1][2] = y0 & 0x00F000F0u; a[2 * b + 1][3] = y1 & 0x00F000F0u;
+                }
+            }
+            constexpr int j = decltype(J)::value;
+#pragma unroll
+            for (int s = 0; s < NS; s++) {
+                float r0[4], r1[4];
+                sp::mma(r0, a[0][0], a[0][1], a[0][2], a[0][3], bf[s][0][0], bf[s][0][1], 0.f, 0.f, 0.f, 0.f);
+                sp::mma(r1, a[2][0], a[2][1], a[2][2], a[2][3], bf[s][2][0], bf[s][2][1], 0.f, 0.f, 0.f, 0.f);
+                sp::mma(r0, a[1][0], a[1][1], a[1][2], a[1][3], bf[s][1][0], bf[s][1][1], r0[0], r0[1], r0[2], r0[3]);
+                sp::mma(r1, a[3][0], a[3][1], a[3][2], a[3][3], bf[s][3][0], bf[s][3][1], r1[0], r1[1], r1[2], r1[3]);
+                acc[j][s][0] = fmaf(d1[0], r1[0] + cc[s][1], fmaf(d0[0], r0[0] + cc[s][0], acc[j][s][0]));
+                acc[j][s][1] = fmaf(d1[0], r1[1], fmaf(d0[0], r0[1], acc[j][s][1]));
+                acc[j][s][2] = fmaf(d1[1], r1[2] + cc[s][1], fmaf(d0[1], r0[2] + cc[s][0], acc[j][s][2]));
+                acc[j][s][3] = fmaf(d1[1], r1[3], fmaf(d0[1], r0[3], acc[j][s][3]));
+            }
+        });
+    } else if constexpr (T == GT_Q4_K || T == GT_Q5_K) {
+        constexpr bool Q5 = T == GT_Q5_K;
+        const uint32_t pu = u & 3u, qo = (Q5 ? 48u : 16u) + 32 * pu + 4 * t;
+        const uint32_t q0 = a0 + qo, q1 = a1 + qo, h0 = a0 + 16 + 4 * t, h1 = a1 + 16 + 4 * t, tr = tab + g * 16;
+        sp::each<0, NT>([&](auto J) {
+            constexpr int j = decltype(J)::value;
+            constexpr uint32_t o = j * TS;
+            uint32_t x[2][2];   // [first / second 16 elements][row g, g + 8]
+            x[0][0] = sp::ld32i<o>(q0); x[1][0] = sp::ld32i<o + 16>(q0);
+            x[0][1] = sp::ld32i<o>(q1); x[1][1] = sp::ld32i<o + 16>(q1);
+            uint32_t p0[4], p1[4];   // d sc, d sc', dmin m, dmin m' of rows g and g + 8
+            sp::ld128i<j * 256u>(tr, p0);
+            sp::ld128i<j * 256u + 128u>(tr, p1);
+            uint32_t a[4][4];
+            if constexpr (Q5) {   // five-bit codes, one per byte: nibble | fifth bit << 4
+                uint32_t f[2][2];
+                f[0][0] = sp::ld32i<o>(h0) >> (2 * pu); f[1][0] = sp::ld32i<o + 16>(h0) >> (2 * pu);
+                f[0][1] = sp::ld32i<o>(h1) >> (2 * pu); f[1][1] = sp::ld32i<o + 16>(h1) >> (2 * pu);
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const uint32_t lo = (x[e][h] & 0x0F0F0F0Fu) | ((f[e][h] & 0x01010101u) << 4);
+                        const uint32_t hi = ((x[e][h] >> 4) & 0x0F0F0F0Fu) | ((f[e][h] & 0x02020202u) << 3);
+                        a[e][h] = __byte_perm(lo, 0u, 0x4240); a[e][h + 2] = __byte_perm(lo, 0u, 0x4341);
+                        a[e + 2][h] = __byte_perm(hi, 0u, 0x4240); a[e + 2][h + 2] = __byte_perm(hi, 0u, 0x4341);
+                    }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const uint32_t y = x[e][h] >> 8;
+                        a[e][h] = x[e][h] & 0x000F000Fu; a[e][h + 2] = y & 0x000F000Fu;
+                        a[e + 2][h] = x[e][h] & 0x00F000F0u; a[e + 2][h + 2] = y & 0x00F000F0u;
+                    }
+            }
+#pragma unroll
+            for (int s = 0; s < NS; s++) {
+                float r0[4], r1[4];
+                sp::mma(r0, a[0][0], a[0][1], a[0][2], a[0][3], bf[s][0][0], bf[s][0][1], 0.f, 0.f, 0.f, 0.f);
+                sp::mma(r1, a[2][0], a[2][1], a[2][2], a[2][3], bf[s][2][0], bf[s][2][1], 0.f, 0.f, 0.f, 0.f);
+                sp::mma(r0, a[1][0], a[1][1], a[1][2], a[1][3], bf[s][1][0], bf[s][1][1], r0[0], r0[1], r0[2], r0[3]);
+                sp::mma(r1, a[3][0], a[3][1], a[3][2], a[3][3], bf[s][3][0], bf[s][3][1], r1[0], r1[1], r1[2], r1[3]);
+                const float c0 = cc[s][0], c1 = cc[s][1];
+                auto f = [](uint32_t v) { return __uint_as_float(v); };
+                acc[j][s][0] = fmaf(f(p0[1]), r1[0], fmaf(f(p0[0]), r0[0], fmaf(f(p0[3]), c1, fmaf(f(p0[2]), c0, acc[j][s][0]))));
+                acc[j][s][1] = fmaf(f(p0[1]), r1[1], fmaf(f(p0[0]), r0[1], acc[j][s][1]));
+                acc[j][s][2] = fmaf(f(p1[1]), r1[2], fmaf(f(p1[0]), r0[2], fmaf(f(p1[3]), c1, fmaf(f(p1[2]), c0, acc[j][s][2]))));
+                acc[j][s][3] = fmaf(f(p1[1]), r1[3], fmaf(f(p1[0]), r0[3], acc[j][s][3]));
+            }
+        });
+    } else {
+        const uint32_t nh = (u >> 1) & 1u, js = u & 1u, tr = tab + g * 16;
+        const uint32_t lo = 64 * nh + 16 * js + 4 * t, ho = 128 + 32 * nh + 16 * js + 4 * t;
+        // super-blocks are 210 bytes: where one starts 2 bytes past a word boundary, words are joined from two.  With aligned
+        // rows that is the same for all rows (SHIFT known per call), else a matter of the row.
+        auto body = [&](auto SHIFT) {
+            constexpr int shift = decltype(SHIFT)::value;   // 0: word-aligned, 1: joined, 2: per row
+            const uint32_t b0 = a0 & ~3u, b1 = a1 & ~3u;
+            const uint32_t L[2] = {b0 + lo, b1 + lo}, H[2] = {b0 + ho, b1 + ho};
+            const uint32_t sl[2] = {(a0 & 2u) ? 0x5432u : 0x3210u, (a1 & 2u) ? 0x5432u : 0x3210u};
+            sp::each<0, NT>([&](auto J) {
+                constexpr int j = decltype(J)::value;
+                constexpr uint32_t o = j * TS;
+                uint32_t qv[2][4];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    uint32_t A = sp::ld32i<o>(L[h]), B = sp::ld32i<o + 32>(L[h]), X = sp::ld32i<o>(H[h]);
+                    if constexpr (shift != 0) {
+                        const uint32_t s = shift == 1 ? 0x5432u : sl[h];
+                        A = __byte_perm(A, sp::ld32i<o + 4>(L[h]), s);
+                        B = __byte_perm(B, sp::ld32i<o + 36>(L[h]), s);
+                        X = __byte_perm(X, sp::ld32i<o + 4>(H[h]), s);
+                    }
+                    qv[h][0] = (A & 0x0F0F0F0Fu) | ((X & 0x03030303u) << 4);
+                    qv[h][1] = (B & 0x0F0F0F0Fu) | ((X & 0x0C0C0C0Cu) << 2);
+                    qv[h][2] = ((A >> 4) & 0x0F0F0F0Fu) | (X & 0x30303030u);
+                    qv[h][3] = ((B >> 4) & 0x0F0F0F0Fu) | ((X & 0xC0C0C0C0u) >> 2);
+                }
+                uint32_t p0[4], p1[4];
+                sp::ld128i<j * 256u>(tr, p0);
+                sp::ld128i<j * 256u + 128u>(tr, p1);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const uint32_t x0 = __byte_perm(qv[0][q], 0u, 0x4240), x2 = __byte_perm(qv[0][q], 0u, 0x4341);
+                    const uint32_t x1 = __byte_perm(qv[1][q], 0u, 0x4240), x3 = __byte_perm(qv[1][q], 0u, 0x4341);
+                    const float pa = __uint_as_float(p0[q]), pb = __uint_as_float(p1[q]);
+#pragma unroll
+                    for (int s = 0; s < NS; s++) {
+                        float r[4];
+                        sp::mma(r, x0, x1, x2, x3, bf[s][q][0], bf[s][q][1], 0.f, 0.f, 0.f, 0.f);
+                        acc[j][s][0] = fmaf(pa, r[0] + cc[s][q], acc[j][s][0]);
+                        acc[j][s][1] = fmaf(pa, r[1], acc[j][s][1]);
+                        acc[j][s][2] = fmaf(pb, r[2] + cc[s][q], acc[j][s][2]);
+                        acc[j][s][3] = fmaf(pb, r[3], acc[j][s][3]);
+                    }
+                }
+            });
+        };
+        if constexpr (ALN) {
+            if (a0 & 2u) body(std::integral_constant<int, 1>{});
+            else body(std::integral_constant<int, 0>{});
+        } else {
+            body(std::integral_constant<int, 2>{});
+        }
+    }
+}
+
+// Scale table of one unit for one row: d * scale of the unit's groups (Q6_K: four), or d sc, d sc', dmin m, dmin m' of its
+// two sub-blocks (Q4_K, Q5_K; 6-bit fields as in src/gguf/mod.rs:440-452).  rb: shared address of the row's super-block.
+template <int T> __device__ __forceinline__ void sp_table_row(uint32_t dst, uint32_t rb, uint32_t u) {
+    if constexpr (T == GT_Q6_K) {
+        const uint32_t s = rb + 192 + 8 * ((u >> 1) & 1u) + (u & 1u);
+        const float d = sp::h_lo(sp::ld16i<208>(rb));
+        sp::st128(dst, d * (float)lds_s8(s), d * (float)lds_s8(s + 2), d * (float)lds_s8(s + 4), d * (float)lds_s8(s + 6));
+    } else {
+        const uint32_t pu = u & 3u, dd = sp::ld32(rb), s0 = sp::ld32i<4>(rb), s1 = sp::ld32i<8>(rb);
+        const float d = sp::h_lo(dd), dmin = sp::h_hi(dd);
+        uint32_t c0, c1, m0, m1;
+        if (pu < 2) {
+            const uint32_t a = s0 >> (16 * pu), b = s1 >> (16 * pu);
+            c0 = a & 63u; c1 = (a >> 8) & 63u;
+            m0 = b & 63u; m1 = (b >> 8) & 63u;
+        } else {
+            const uint32_t sh = 16 * (pu - 2);
+            const uint32_t a = sp::ld32i<12>(rb) >> sh, lo = s0 >> sh, hi = s1 >> sh;
+            c0 = (a & 15u) | (((lo >> 6) & 3u) << 4);
+            c1 = ((a >> 8) & 15u) | (((lo >> 14) & 3u) << 4);
+            m0 = ((a >> 4) & 15u) | (((hi >> 6) & 3u) << 4);
+            m1 = ((a >> 12) & 15u) | (((hi >> 14) & 3u) << 4);
+        }
+        sp::st128(dst, d * (float)c0, d * (float)c1, dmin * (float)m0, dmin * (float)m1);
+    }
+}
+
+// A chunk of work: `nt` consecutive tiles of op `op` for entry `ent`, from the op's tile `tile` on.  Chunks are dealt out in runs:
+// cluster c takes the runs c, c + clusters, ..., so that at any time the whole chip reads one stretch of the weights (a
+// contiguous share per CTA keeps hundreds of distant pages open at once and ran at half the rate).
+struct SpChunk {
+    uint32_t ent, op, tile, nt;
+};
+__device__ __forceinline__ SpChunk sp_chunk(const SpBatch &b, uint32_t i) {
+    SpChunk c;
+    const uint32_t all = b.op[b.nops - 1].chunk_end;
+    c.ent = i / all;
+    const uint32_t r = i - c.ent * all;
+    c.op = 0;
+    while (r >= b.op[c.op].chunk_end) c.op++;
+    c.tile = (r - (c.op ? b.op[c.op - 1].chunk_end : 0u)) * b.tr;
+    c.nt = min(b.tr, (b.op[c.op].n + 15u) / 16u - c.tile);
+    return c;
+}
+
+// Packs activation rows into B register order for the kernel below: f16 hi + lo halves under one power of two per row, per scale
+// group what the codes' bias owes, and the inverse scale.  One block per row.  Several rows (or row groups: Q4_K has no other form
+// for many rows) are packed once instead of by every CTA, where eight rows cost more time than the weights of a 12288 x 4096 matrix.
+template <int T, bool ALN>
+__global__ void __launch_bounds__(256) qmv_pack_kernel(const __grid_constant__ SpBatch bt) {
+    constexpr int NG = SpTraits<T>::NG;
+    constexpr float kOff = -(float)SpTraits<T>::OFF / 16777216.0f;
+    __shared__ float s_am[8];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, q = (tid >> 2) & 3u, tt = tid & 3u;
+    uint32_t op = 0;   // (ops that share another's activations have no rows of their own here)
+    while (blockIdx.x >= bt.op[op].row_end) op++;
+    const SpOp &P = bt.op[op];
+    const size_t row = blockIdx.x - (op ? bt.op[op - 1].row_end : 0u);
+    const uint32_t k = P.k, units = P.units, pk_units = P.pk_units;
+    const float *x = P.x;
+    uint8_t *xp = const_cast<uint8_t *>(P.xp);
+    float *xsum = const_cast<float *>(P.xsum), *xinv = const_cast<float *>(P.xinv);
+    grid_dependency_wait();
+    allow_dependents();   // (not earlier: the kernel behind may overwrite what this one's predecessors still read)
+    const float *xr = x + row * k;
+    auto load = [&](uint32_t u, float (&v)[4]) {
+        uint32_t p0, p1;
+        sp_pairs<T, ALN>(u, q, tt, p0, p1);
+        const uint32_t kb = T == GT_Q6_K ? 256u * (u >> 2) : 64u * u;
+        v[0] = v[1] = v[2] = v[3] = 0.f;
+        if (u >= units) return;
+        if (kb + p0 < k) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(xr + kb + p0));
+        if (kb + p1 < k) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[2]), "=f"(v[3]) : "l"(xr + kb + p1));
+    };
+    constexpr int HELD = 8;   // a pass of the block takes 16 units; K = 8192 stays in registers
+    float v[HELD][4], am = 0.f;
+#pragma unroll
+    for (int p = 0; p < HELD; p++) {
+        if (16u * p >= pk_units) break;
+        load(16u * p + (tid >> 4), v[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < HELD; p++) {
+        if (16u * p >= pk_units) break;
+#pragma unroll
+        for (int e = 0; e < 4; e++) am = fmaxf(am, fabsf(v[p][e]));
+    }
+    for (uint32_t u = 16u * HELD + (tid >> 4); u < pk_units; u += 16) {
+        float z[4];
+        load(u, z);
+#pragma unroll
+        for (int e = 0; e < 4; e++) am = fmaxf(am, fabsf(z[e]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+    if (lane == 0) s_am[warp] = am;
+    __syncthreads();
+    am = s_am[lane & 7u];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+    float s, inv;
+    sp::pow2(am, s, inv);
+    if (tid == 0) xinv[row] = inv * 16777216.0f;
+    // codes that stay in the high nibble of their byte are 16 times too large: their activations / 16
+    const float f = (T == GT_Q4_0 && (q & 1u)) || (T == GT_Q4_K && q >= 2) ? s * 0.0625f : s;
+    auto put = [&](uint32_t u, const float (&z)[4]) {
+        float sum = (z[0] + z[1]) + (z[2] + z[3]);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if constexpr (NG == 2) sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+        const __half2 h02 = __floats2half2_rn(z[0] * f, z[2] * f), h13 = __floats2half2_rn(z[1] * f, z[3] * f);
+        const float2 f02 = __half22float2(h02), f13 = __half22float2(h13);
+        const __half2 l02 = __floats2half2_rn(fmaf(z[0], f, -f02.x), fmaf(z[2], f, -f02.y));
+        const __half2 l13 = __floats2half2_rn(fmaf(z[1], f, -f13.x), fmaf(z[3], f, -f13.y));
+        if (u >= pk_units) return;
+        uint2 *d = reinterpret_cast<uint2 *>(xp + (row * pk_units + u) * 256u + (q >> 1) * 128u + tt * 32u + (q & 1u) * 8u);
+        d[0] = make_uint2(*reinterpret_cast<const uint32_t *>(&h02), *reinterpret_cast<const uint32_t *>(&h13));
+        d[2] = make_uint2(*reinterpret_cast<const uint32_t *>(&l02), *reinterpret_cast<const uint32_t *>(&l13));
+        if ((tid & (NG == 4 ? 3u : 7u)) == 0) xsum[(row * pk_units + u) * NG + (NG == 4 ? q : q >> 1)] = kOff * (sum * s);
+    };
+#pragma unroll
+    for (int p = 0; p < HELD; p++) {
+        if (16u * p >= pk_units) break;
+        put(16u * p + (tid >> 4), v[p]);
+    }
+    for (uint32_t u0 = 16u * HELD; u0 < pk_units; u0 += 16) {
+        float z[4];
+        load(u0 + (tid >> 4), z);
+        put(u0 + (tid >> 4), z);
+    }
+}
+
+// MPC: 1 = one activation row, 4 = up to four (one set of columns), 8 = up to eight (two sets).
+template <int T, bool ALN, int MPC>
+__global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_constant__ SpBatch bt, const __grid_constant__ SpMaps maps) {
+    using K = SpTraits<T>;
+    constexpr int NS = MPC > 4 ? 2 : 1, NG = K::NG, SU = K::SU, TM = sp_tiles(NS);
+    constexpr bool TABLE = T == GT_Q4_K || T == GT_Q5_K || T == GT_Q6_K;
+    constexpr uint32_t PITCH = sp_pitch<T>(ALN), TILE = 16 * PITCH;
+    constexpr uint32_t UB = T == GT_Q8_0 ? 68u : 36u;               // bytes of a unit (Q4_0, Q8_0)
+    constexpr float kOff = -(float)K::OFF / 16777216.0f;
+
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 127u) & ~127u;      // (the same in every CTA of a cluster)
+    __shared__ __align__(8) uint64_t full[kSpMaxSlots], empty[kSpMaxSlots], sync_bar[3], recv_bar[4], x_bar, c_bar;
+    __shared__ float s_inv[kSpWarps][8];                            // inverse activation scales of a warp's share of K
+    __shared__ volatile uint32_t abort_flag;
+    __shared__ uint32_t s_nent;
+    __shared__ uint32_t s_id[kSpMaxPairs];                          // routed: expert of every pair
+    __shared__ uint16_t s_ord[kSpMaxPairs], s_ent[kSpMaxPairs + 1]; // pairs by expert; entry e = pairs s_ord[s_ent[e] ..]
+    __shared__ uint32_t s_wcnt[kSpWarps];
+
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    uint32_t ranks, rank;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    rank = sp::cluster_rank();
+    const uint32_t mp = bt.mp, tr = bt.tr, R = 16u * tr, STAGE = tr * TILE;
+
+    if (tid == 0) {
+        abort_flag = 0;
+        for (uint32_t s = 0; s < bt.nslots; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], kSpWarps);
+        }
+        for (int s = 0; s < 3; s++) mbar_init(&sync_bar[s], kSpWarps);
+        for (int s = 0; s < 4; s++) mbar_init(&recv_bar[s], 1);
+        mbar_init(&x_bar, 1);
+        mbar_init(&c_bar, kSpWarps);
+        mbar_init_fence();
+    }
+    if (bt.ids) {
+        grid_dependency_wait();   // the expert ids belong to the kernels ahead
+        for (uint32_t p = tid; p < kSpMaxPairs; p += kSpThreads) s_id[p] = p < bt.npairs ? min(__ldcg(bt.ids + p), bt.n_experts) : 0xFFFFFFFFu;
+    }
+    __syncwarp();
+    if (ranks > 1) sp::cluster_sync();   // the others' barriers exist before anything is sent there
+    else __syncthreads();
+    allow_dependents();
+    if (bt.ids) {
+        // rank of every pair by (expert, pair); an entry starts at every mp-th pair of an expert
+        uint32_t pos = 0, before = 0, me = 0;
+        if (tid < bt.npairs) {
+            me = s_id[tid];
+            for (uint32_t q = 0; q < bt.npairs; q++) {
+                const uint32_t o = s_id[q];
+                const bool eq = o == me && q < tid;
+                before += eq ? 1u : 0u;
+                pos += (o < me || eq) ? 1u : 0u;
+            }
+            s_ord[pos] = (uint16_t)(tid | (before % mp == 0 ? 0x8000u : 0u));
+        }
+        __syncthreads();
+        bool start = false;
+        if (tid < bt.npairs) {
+            const uint32_t v = s_ord[tid];
+            start = (v & 0x8000u) != 0;
+        }
+        const uint32_t bal = __ballot_sync(0xffffffffu, start);
+        if (warp < kSpWarps && lane == 0) s_wcnt[warp] = __popc(bal);
+        __syncthreads();
+        uint32_t at = 0, total = 0;
+        for (uint32_t w = 0; w < kSpWarps; w++) {
+            if (w < warp) at += s_wcnt[w];
+            total += s_wcnt[w];
+        }
+        if (start) s_ent[at + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)tid;
+        if (tid == 0) {
+            s_ent[total] = (uint16_t)bt.npairs;
+            s_nent = total;
+        }
+        if (tid < bt.npairs) s_ord[tid] &= 0x7FFFu;
+        __syncthreads();
+    }
+    const uint32_t nent = bt.ids ? s_nent : bt.nent;
+    const uint32_t chunks = nent * bt.op[bt.nops - 1].chunk_end;
+    const uint32_t ncl = gridDim.x / ranks, run = bt.run ? bt.run : (chunks + ncl - 1) / ncl, first = blockIdx.x / ranks * run, skip = (gridDim.x / ranks - 1) * run;
+
+    if (warp == kSpWarps) {
+        // ======================= producer =======================
+        if (!bt.early_weights) grid_dependency_wait();
+        uint64_t pol;
+        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+        uint32_t slot = 0, ph = 1;   // (a slot's first wait passes)
+        bool ok = true;
+        for (uint32_t at = first, left = run; ok && at < chunks; at++) {
+            const SpChunk c = sp_chunk(bt, at);
+            if (--left == 0) {
+                left = run;
+                at += skip;
+            }
+            const SpOp &P = bt.op[c.op];
+            const uint32_t u0 = rank * P.slice;
+            const uint32_t un = u0 < P.units ? min(P.slice, P.units - u0) : 0u;
+            const uint32_t ex = bt.ids ? s_id[s_ord[s_ent[c.ent]]] : 0u;
+            for (uint32_t u = 0; u < un; u += SU) {
+                if (!mbar_wait(&empty[slot], ph, &abort_flag, bt.status, ST_WAIT_EMPTY_TIMEOUT, 0u)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t dst = base + slot * STAGE;
+                const uint32_t off = (u0 + u) / 4 * (uint32_t)K::B256;
+                if constexpr (ALN) {
+                    if (lane == 0) {
+                        mbar_expect_tx(&full[slot], c.nt * TILE);
+                        for (uint32_t j = 0; j < c.nt; j++)
+                            asm volatile(
+                                "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;"
+                                ::"r"(dst + j * TILE), "l"(&maps.m[c.op]), "r"((off & ~15u) >> 3), "r"((c.tile + j) * 16u), "r"(ex),
+                                  "r"(smem_u32(&full[slot])), "l"(pol)
+                                : "memory");
+                    }
+                } else {
+                    // one bulk copy per row: the 16-byte superset of the row's segment (an expert that does not exist: expert 0,
+                    // whose products are not stored)
+                    const uint32_t len = min((uint32_t)(SU / 4 * K::B256), P.row_bytes - off);
+                    const uint8_t *w = P.w + (ex < bt.n_experts ? (uint64_t)ex * P.expert_stride : 0ull) + off;
+                    uint32_t tx = 0;
+                    for (uint32_t r = lane; r < c.nt * 16u; r += 32) {
+                        const uint32_t row = c.tile * 16u + r;
+                        if (row < P.n) tx += (((uint32_t)(uintptr_t)(w + (uint64_t)row * P.row_bytes) & 15u) + len + 15u) & ~15u;
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) tx += __shfl_xor_sync(0xffffffffu, tx, o);
+                    if (lane == 0) mbar_expect_tx(&full[slot], tx);
+                    __syncwarp();
+                    for (uint32_t r = lane; r < c.nt * 16u; r += 32) {
+                        const uint32_t row = c.tile * 16u + r;
+                        if (row >= P.n) continue;
+                        const uintptr_t src = (uintptr_t)(w + (uint64_t)row * P.row_bytes);
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
+                                         dst + r * PITCH),
+                                     "l"(src & ~(uintptr_t)15), "r"((((uint32_t)src & 15u) + len + 15u) & ~15u), "r"(smem_u32(&full[slot])), "l"(pol)
+                                     : "memory");
+                    }
+                }
+                if (++slot == bt.nslots) {
+                    slot = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+    } else {
+        // ======================= consumers =======================
+        const uint32_t g = lane >> 2, t = lane & 3u;
+        const uint32_t xf = base + bt.xf_off, ccb = base + bt.cc_off, tab = base + bt.tab_off + warp * (R * 16u), red = base + bt.red_off;
+        const uint32_t xs = bt.xstride, cs = bt.cstride;
+        const uint32_t xlane = xf + (MPC == 1 ? 0u : ((g >> 1) & (mp - 1)) * xs) + (t * 2 + (g & 1u)) * 16u;
+        const uint32_t clane = ccb + (MPC == 1 ? 0u : (t & (mp - 1)) * cs);
+        uint32_t slot = 0, ph = 0, cur = 0xFFFFFFFFu;
+        bool ok = true;
+        auto wait = [&](uint64_t &bar, uint32_t parity, uint32_t code) {
+            ok = mbar_wait(&bar, parity, &abort_flag, bt.status, code, 0u) && ok;
+            return ok;
+        };
+        // (finished chunks are remembered by their number alone: registers are what this kernel is short of)
+        auto store = [&](uint32_t at, uint32_t col, uint32_t row, float v) {
+            const SpChunk d = sp_chunk(bt, at);
+            const SpOp &P = bt.op[d.op];
+            const uint32_t grow = d.tile * 16u + row, e0 = bt.ids ? (uint32_t)s_ent[d.ent] : d.ent * mp;
+            const uint32_t cnt = bt.ids ? s_ent[d.ent + 1] - e0 : min(mp, P.m - e0);
+            if (col >= cnt || row >= d.nt * 16u || grow >= P.n) return;
+            const uint32_t pair = bt.ids ? (uint32_t)s_ord[e0 + col] : e0 + col;
+            const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
+            if (bt.ids && s_id[pair] >= bt.n_experts) v = 0.f;   // an id that names no expert
+            P.y[o] = v;
+            for (uint32_t pr = 0; pr < P.n_peer; pr++) P.y_peer[pr][o] = v;
+        };
+        const uint32_t share = R / ranks;   // rows of a chunk that a rank finishes
+        // the CTA's sums of chunk j, in warp order: results, or for the rank that finishes the row
+        auto add = [&](uint32_t j, uint32_t d) {
+            if (!wait(sync_bar[j & 1u], (j >> 1) & 1u, ST_WAIT_EMPTY_TIMEOUT)) return false;
+            const uint32_t part = red + (j & 1u) * (kSpWarps * mp * R * 4u), buf = j & 3u;
+            for (uint32_t q = tid; q < mp * R; q += 256) {
+                const uint32_t col = q / R, row = q - col * R;
+                float v = 0.f;
+#pragma unroll
+                for (int w = 0; w < kSpWarps; w++) v += __uint_as_float(sp::ld32(part + ((w * mp + col) * R + row) * 4));
+                if (ranks == 1) {
+                    store(d, col, row, v);
+                } else {
+                    const uint32_t to = row / share;
+                    const uint32_t a = base + bt.recv_off + (((buf * ranks + rank) * mp + col) * share + row - to * share) * 4;
+                    sp::st_async(sp::map_rank(a, to), v, sp::map_rank(smem_u32(&recv_bar[buf]), to));
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sync_bar[2]);
+            if (ranks > 1 && tid == 0) mbar_expect_tx(&recv_bar[buf], mp * R * 4u);
+            return true;
+        };
+        // the ranks' sums of chunk j, in rank order (a rank sends chunk j + 4 only when it has this one's j + 2: four buffers)
+        auto finish = [&](uint32_t j, uint32_t d) {
+            const uint32_t buf = j & 3u;
+            if (!wait(recv_bar[buf], (j >> 2) & 1u, ST_WAIT_FULL_TIMEOUT)) return false;
+            for (uint32_t q = tid; q < mp * share; q += 256) {
+                const uint32_t col = q / share, row = q - col * share;
+                float v = 0.f;
+                for (uint32_t r = 0; r < ranks; r++) v += __uint_as_float(sp::ld32(base + bt.recv_off + (((buf * ranks + r) * mp + col) * share + row) * 4));
+                store(d, col, rank * share + row, v);
+            }
+            return true;
+        };
+        uint32_t x_ph = 0, c_ph = 0;
+        auto csync = [&]() {   // all warps
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&c_bar);
+            const bool r = wait(c_bar, c_ph, ST_WAIT_EMPTY_TIMEOUT);
+            c_ph ^= 1u;
+            return r;
+        };
+        uint32_t d1 = 0, d2 = 0;
+        uint32_t i = 0;   // the CTA's chunks so far
+        if (!bt.ids) grid_dependency_wait();   // the activations belong to the kernels ahead until those are done
+        for (uint32_t at = first, left = run; ok && at < chunks; at++, i++) {
+            const SpChunk c = sp_chunk(bt, at);
+            const uint32_t this_at = at;
+            if (--left == 0) {
+                left = run;
+                at += skip;
+            }
+            const SpOp &P = bt.op[c.op];
+            const uint32_t u0 = rank * P.slice;
+            const uint32_t un = u0 < P.units ? min(P.slice, P.units - u0) : 0u;
+            uint32_t e0 = 0, cnt, ex = 0;
+            if (bt.ids) {
+                e0 = s_ent[c.ent];
+                cnt = s_ent[c.ent + 1] - e0;
+                ex = s_id[s_ord[e0]];
+            } else {
+                e0 = c.ent * mp;
+                cnt = min(mp, P.m - e0);
+            }
+            const uint32_t key = c.ent * kSpMaxOps + P.xkey;
+            if (MPC > 1 && key != cur && bt.packed) {
+                // the rows' slices come ready from the pack kernel's scratch area
+                if (cur != 0xFFFFFFFFu && !csync()) break;   // nobody reads the entry before any more
+                cur = key;
+                const uint32_t un4 = (un + 3) & ~3u, xb = un4 * 256u, cb = un4 * NG * 4u;
+                if (warp == 0) {
+                    if (lane == 0) mbar_expect_tx(&x_bar, cnt * (xb + cb));
+                    __syncwarp();
+                    if (lane < cnt && un) {
+                        const uint8_t *px = P.xp + ((size_t)(e0 + lane) * P.pk_units + u0) * 256u;
+                        bulk_g2s_a(xf + lane * xs, px, xb, &x_bar);
+                        bulk_g2s_a(ccb + lane * cs, reinterpret_cast<const uint8_t *>(P.xsum) + ((size_t)(e0 + lane) * P.pk_units + u0) * (NG * 4u), cb, &x_bar);
+                    }
+                }
+                if (lane < cnt) s_inv[warp][lane] = __ldcg(P.xinv + e0 + lane);
+                if (!wait(x_bar, x_ph, ST_WAIT_FULL_TIMEOUT)) break;
+                x_ph ^= 1u;
+                __syncwarp();
+            }
+            if (key != cur) {
+                // ---- the entry's activations of this warp's units: f16 hi + lo in B register order.  A pass takes two units
+                // (lane = (unit of the pass, MMA q, quad lane tt), four values each) ----
+                cur = key;
+                const uint32_t q = (lane >> 2) & 3u, tt = lane & 3u, hf = lane >> 4;
+                uint32_t p0, p1;
+                sp_pairs<T, ALN>(warp, q, tt, p0, p1);
+                const uint32_t kb = (T == GT_Q6_K ? 256u * ((u0 + warp) >> 2) : 64u * (u0 + warp)) + 512u * hf;
+                const uint32_t mine = un > warp ? (un - warp + 7) / 8 : 0u;          // the warp's units
+                const float f0 = (T == GT_Q4_0 && (q & 1u)) || (T == GT_Q4_K && q >= 2) ? 0.0625f : 1.f;   // codes left in the high nibble are 16 times too large
+                const uint32_t d0 = xf + ((warp + 8 * hf) * 2 + (q >> 1)) * 128u + tt * 32u + (q & 1u) * 8u;
+                const uint32_t c0 = ccb + ((warp + 8 * hf) * NG + (NG == 4 ? q : q >> 1)) * 4u;
+                const bool head = (lane & (NG == 4 ? 3u : 7u)) == 0;
+                __syncwarp();
+                if constexpr (MPC == 1) {
+                    constexpr uint32_t r = 0;
+                    const uint32_t row = e0;
+                    const float *x = P.x + (size_t)row * P.k + kb, *y = P.x2 ? P.x2 + (size_t)row * P.k + kb : nullptr;
+                    auto load = [&](uint32_t p, float (&v)[4]) {
+                        v[0] = v[1] = v[2] = v[3] = 0.f;
+                        const uint32_t o = 1024u * p;
+                        if (2 * p + hf >= mine) return;
+                        const bool i0 = kb + o + p0 < P.k, i1 = kb + o + p1 < P.k;
+                        if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(x + o + p0));
+                        if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[2]), "=f"(v[3]) : "l"(x + o + p1));
+                        if (y) {   // silu(gate) * up, as src/shaders/silu_mul.metal:17-30
+                            float w[4] = {0.f, 0.f, 0.f, 0.f};
+                            if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[0]), "=f"(w[1]) : "l"(y + o + p0));
+                            if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[2]), "=f"(w[3]) : "l"(y + o + p1));
+#pragma unroll
+                            for (int e = 0; e < 4; e++) v[e] = v[e] / (1.0f + expf(-v[e])) * w[e];
+                        }
+                    };
+                    auto peak = [](const float (&v)[4]) { return fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))); };
+                    constexpr int HELD = 4;   // passes whose values stay in registers; those beyond are loaded again
+                    float v[HELD][4], am = 0.f;
+#pragma unroll
+                    for (int p = 0; p < HELD; p++) load(p, v[p]);
+#pragma unroll
+                    for (int p = 0; p < HELD; p++) am = fmaxf(am, peak(v[p]));
+                    for (uint32_t p = HELD; 2 * p < mine; p++) {
+                        float z[4];
+                        load(p, z);
+                        am = fmaxf(am, peak(z));
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+                    float s, inv;
+                    sp::pow2(am, s, inv);
+                    if (lane == 0) s_inv[warp][r] = inv * 16777216.0f;
+                    const float f = s * f0;
+                    auto put = [&](uint32_t p, const float (&z)[4]) {
+                        float sum = (z[0] + z[1]) + (z[2] + z[3]);
+                        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                        if constexpr (NG == 2) sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                        const __half2 h02 = __floats2half2_rn(z[0] * f, z[2] * f), h13 = __floats2half2_rn(z[1] * f, z[3] * f);
+                        const float2 f02 = __half22float2(h02), f13 = __half22float2(h13);
+                        const __half2 l02 = __floats2half2_rn(fmaf(z[0], f, -f02.x), fmaf(z[2], f, -f02.y));
+                        const __half2 l13 = __floats2half2_rn(fmaf(z[1], f, -f13.x), fmaf(z[3], f, -f13.y));
+                        if (2 * p + hf < mine) {
+                            const uint32_t d = d0 + p * 4096u;
+                            sp::st64(d, *reinterpret_cast<const uint32_t *>(&h02), *reinterpret_cast<const uint32_t *>(&h13));
+                            sp::st64(d + 16, *reinterpret_cast<const uint32_t *>(&l02), *reinterpret_cast<const uint32_t *>(&l13));
+                            if (head) sp::st32(c0 + p * (64u * NG), __float_as_uint(kOff * (sum * s)));
+                        }
+                    };
+#pragma unroll
+                    for (int p = 0; p < HELD; p++)
+                        if (2u * p < mine) put(p, v[p]);
+                    for (uint32_t p = HELD; 2 * p < mine; p++) {
+                        float z[4];
+                        load(p, z);
+                        put(p, z);
+                    }
+                } else {
+                // Four passes are in flight at a time: of one row, or of two or four rows where a row has fewer.
+                const uint32_t passes = (mine + 1) / 2, sh = passes <= 1 ? 0u : passes == 2 ? 1u : 2u, rows = 4u >> sh;
+                for (uint32_t rb = 0; rb < cnt; rb += rows) {
+                    const float *x[4], *y[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const uint32_t r = min(rb + (j >> sh), cnt - 1);
+                        const size_t o = (size_t)(bt.ids ? (uint32_t)s_ord[e0 + r] / P.x_div : e0 + r) * P.k + kb;
+                        x[j] = P.x + o;
+                        y[j] = P.x2 ? P.x2 + o : nullptr;
+                    }
+                    auto load = [&](const float *xr, const float *yr, uint32_t p, float (&v)[4]) {
+                        v[0] = v[1] = v[2] = v[3] = 0.f;
+                        const uint32_t o = 1024u * p;
+                        if (2 * p + hf >= mine) return;
+                        const bool i0 = kb + o + p0 < P.k, i1 = kb + o + p1 < P.k;
+                        if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(xr + o + p0));
+                        if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[2]), "=f"(v[3]) : "l"(xr + o + p1));
+                        if (yr) {   // silu(gate) * up, as src/shaders/silu_mul.metal:17-30
+                            float w[4] = {0.f, 0.f, 0.f, 0.f};
+                            if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[0]), "=f"(w[1]) : "l"(yr + o + p0));
+                            if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[2]), "=f"(w[3]) : "l"(yr + o + p1));
+#pragma unroll
+                            for (int e = 0; e < 4; e++) v[e] = v[e] / (1.0f + expf(-v[e])) * w[e];
+                        }
+                    };
+                    auto peak = [](const float (&v)[4]) { return fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))); };
+                    auto put = [&](uint32_t r, uint32_t p, float s, const float (&z)[4]) {
+                        const float f = s * f0;
+                        float sum = (z[0] + z[1]) + (z[2] + z[3]);
+                        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                        if constexpr (NG == 2) sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                        const __half2 h02 = __floats2half2_rn(z[0] * f, z[2] * f), h13 = __floats2half2_rn(z[1] * f, z[3] * f);
+                        const float2 f02 = __half22float2(h02), f13 = __half22float2(h13);
+                        const __half2 l02 = __floats2half2_rn(fmaf(z[0], f, -f02.x), fmaf(z[2], f, -f02.y));
+                        const __half2 l13 = __floats2half2_rn(fmaf(z[1], f, -f13.x), fmaf(z[3], f, -f13.y));
+                        if (2 * p + hf < mine && r < cnt) {
+                            const uint32_t d = d0 + p * 4096u + r * xs;
+                            sp::st64(d, *reinterpret_cast<const uint32_t *>(&h02), *reinterpret_cast<const uint32_t *>(&h13));
+                            sp::st64(d + 16, *reinterpret_cast<const uint32_t *>(&l02), *reinterpret_cast<const uint32_t *>(&l13));
+                            if (head) sp::st32(c0 + p * (64u * NG) + r * cs, __float_as_uint(kOff * (sum * s)));
+                        }
+                    };
+                    float v[4][4], am[4], s[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) load(x[j], y[j], j & ((1u << sh) - 1u), v[j]);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) am[j] = peak(v[j]);
+                    for (uint32_t p = 4; p < passes; p++) {   // a long row: its other passes are loaded twice
+                        float z[4];
+                        load(x[0], y[0], p, z);
+                        am[0] = fmaxf(am[0], peak(z));
+                    }
+                    if (sh == 1) {
+                        am[0] = fmaxf(am[0], am[1]);
+                        am[2] = fmaxf(am[2], am[3]);
+                    } else if (sh == 2) {
+                        am[0] = fmaxf(fmaxf(am[0], am[1]), fmaxf(am[2], am[3]));
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                        for (int j = 0; j < 4; j++) am[j] = fmaxf(am[j], __shfl_xor_sync(0xffffffffu, am[j], o));
+                    if (sh == 1) {
+                        am[1] = am[0];
+                        am[3] = am[2];
+                    } else if (sh == 2) {
+                        am[1] = am[2] = am[3] = am[0];
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {   // one power of two brings the row's largest value into [2^13, 2^14)
+                        float inv;
+                        sp::pow2(am[j], s[j], inv);
+                        if (lane == 0 && rb + (j >> sh) < cnt) s_inv[warp][rb + (j >> sh)] = inv * 16777216.0f;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; j++) put(rb + (j >> sh), j & ((1u << sh) - 1u), s[j], v[j]);
+                    for (uint32_t p = 4; p < passes; p++) {
+                        float z[4];
+                        load(x[0], y[0], p, z);
+                        put(rb, p, s[0], z);
+                    }
+                }
+                }
+                __syncwarp();
+            }
+
+            float acc[TM][NS][4];
+#pragma unroll
+            for (int j = 0; j < TM; j++)
+#pragma unroll
+                for (int s = 0; s < NS; s++) acc[j][s][0] = acc[j][s][1] = acc[j][s][2] = acc[j][s][3] = 0.f;
+
+            for (uint32_t us = 0; us < un; us += SU) {
+                const uint32_t off = (u0 + us) / 4 * (uint32_t)K::B256;
+                // where a row's data starts in its 16-byte superset (tiles are 16 rows: the same for every tile)
+                const uint32_t wl = ALN ? 0u : ((uint32_t)(uintptr_t)P.w + (ex < bt.n_experts ? ex : 0u) * (uint32_t)P.expert_stride + off) & 15u;
+                const uint32_t rb15 = P.row_bytes & 15u;
+                auto lead = [&](uint32_t row) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + row * rb15) & 15u; };
+                if (!mbar_wait(&full[slot], ph, &abort_flag, bt.status, ST_WAIT_FULL_TIMEOUT, 0u)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t stage = base + slot * STAGE;
+                const uint32_t r0 = stage + g * PITCH + lead(g), r1 = stage + (g + 8) * PITCH + lead(g + 8);
+#pragma unroll
+                for (int i = 0; i < SU / kSpWarps; i++) {
+                    const uint32_t ul = warp + 8u * i, uu = us + ul;
+                    if (uu >= un) break;
+                    uint32_t bf[NS][4][2];
+                    float cc[NS][NG];
+#pragma unroll
+                    for (int s = 0; s < NS; s++) {
+                        uint32_t v[4];
+                        const uint32_t xa = xlane + uu * 256u + s * 4u * xs, ca = clane + uu * NG * 4u + s * 4u * cs;
+                        sp::ld128i<0>(xa, v);
+                        bf[s][0][0] = v[0]; bf[s][0][1] = v[1]; bf[s][1][0] = v[2]; bf[s][1][1] = v[3];
+                        sp::ld128i<128>(xa, v);
+                        bf[s][2][0] = v[0]; bf[s][2][1] = v[1]; bf[s][3][0] = v[2]; bf[s][3][1] = v[3];
+#pragma unroll
+                        for (int q = 0; q < NG; q++) cc[s][q] = __uint_as_float(sp::ld32(ca + q * 4u));
+                    }
+                    const uint32_t ub = TABLE ? (ul >> 2) * (uint32_t)K::B256 : ul * UB;
+                    if constexpr (TABLE) {
+                        __syncwarp();   // the table of the unit before has been read
+#pragma unroll
+                        for (int rr = 0; rr < TM / 2; rr++) {
+                            const uint32_t r = lane + 32u * rr;
+                            if (r < 16u * c.nt) sp_table_row<T>(tab + r * 16, stage + r * PITCH + lead(r) + ub, ul);
+                        }
+                        __syncwarp();
+                    }
+                    // (an odd number of blocks: the second block of the last unit lies past the row)
+                    const bool half = (u0 + uu) * 64 + 32 >= P.k;
+                    auto tiles = [&](auto NT) { sp_unit<T, ALN, decltype(NT)::value, NS, MPC == 1>(r0 + ub, r1 + ub, ul, t, g, tab, half, bf, cc, acc); };
+                    if (c.nt == 1) tiles(std::integral_constant<int, 1>{});
+                    else if (TM == 2 || c.nt == 2) tiles(std::integral_constant<int, 2>{});
+                    else if (c.nt == 3) tiles(std::integral_constant<int, TM == 2 ? 2 : 3>{});
+                    else tiles(std::integral_constant<int, TM>{});
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[slot]);
+                if (++slot == bt.nslots) {
+                    slot = 0;
+                    ph ^= 1u;
+                }
+            }
+            if (!ok) break;
+
+            // ---- the warps' partial sums go to shared memory; they are added one chunk later, and what the other ranks send is
+            // waited for two chunks later, so that nobody stands still for the slowest warp or for the way between SMs ----
+            if (i >= 2 && !wait(sync_bar[2], i & 1u, ST_WAIT_EMPTY_TIMEOUT)) break;   // chunk i - 2 has been read out of the area
+            const uint32_t part = red + (i & 1u) * (kSpWarps * mp * R * 4u);
+#pragma unroll
+            for (int j = 0; j < TM; j++)
+#pragma unroll
+                for (int s = 0; s < NS; s++) {
+                    const uint32_t col = t + 4 * s;
+                    if (col < mp && j < (int)c.nt) {
+                        const float inv = s_inv[warp][col];
+                        const uint32_t a = part + ((warp * mp + col) * R + 16 * j + g) * 4;
+                        sp::st32(a, __float_as_uint((acc[j][s][0] + acc[j][s][1]) * inv));
+                        sp::st32(a + 32, __float_as_uint((acc[j][s][2] + acc[j][s][3]) * inv));
+                    }
+                }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sync_bar[i & 1u]);
+            if (i >= 1 && !add(i - 1, d1)) break;
+            if (i >= 2 && ranks > 1 && !finish(i - 2, d2)) break;
+            d2 = d1;
+            d1 = this_at;
+        }
+        if (ok && i >= 1) ok = add(i - 1, d1);
+        if (ok && ranks > 1 && i >= 2) ok = finish(i - 2, d2);
+        if (ok && ranks > 1 && i >= 1) ok = finish(i - 1, d1);
+    }
+    if (abort_flag)   // let copies in flight land before the CTA's shared memory is released
+        for (int i = 0; i < 200; i++) __nanosleep(5000);
+    __syncwarp();
+    // nobody leaves while a peer may still send here
+    if (ranks > 1) asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// ------------------------------------------------------------------------------------------------
+// host side
+// ------------------------------------------------------------------------------------------------
+struct SpShape {          // geometry of a launch
+    uint32_t ranks, tr, nslots, grid;
+    size_t smem;
+};
+
+// Two CTAs share an SM: 228 KB less 1 KB each for the system and the kernel's static 2.5 KB.
+constexpr size_t kSpSmem = 110 * 1024;
+
+template <int T> inline size_t sp_tail(bool aln, uint32_t ranks, uint32_t tr, uint32_t mp, uint32_t xunits, SpBatch *b) {
+    (void)aln;
+    const size_t r = 16u * tr;
+    const size_t xf = (size_t)xunits * mp * 256, cc = (((size_t)xunits * SpTraits<T>::NG * 4 + 16) * mp + 127) / 128 * 128;
+    const size_t tab = SpTraits<T>::B256 == 272 || T == GT_Q4_0 ? 0 : (size_t)kSpWarps * r * 16;
+    const size_t red = (size_t)2 * kSpWarps * mp * r * 4, recv = ranks > 1 ? (size_t)4 * mp * r * 4 : 0;
+    if (b) {
+        b->cc_off = b->xf_off + (uint32_t)xf;
+        b->tab_off = b->cc_off + (uint32_t)cc;
+        b->red_off = b->tab_off + (uint32_t)tab;
+        b->recv_off = b->red_off + (uint32_t)red;
+        b->xstride = xunits * 256;
+        b->cstride = xunits * SpTraits<T>::NG * 4 + 16;   // (+ 16: four rows in distinct banks)
+    }
+    return xf + cc + tab + red + recv;
+}
+
+template <int T, bool ALN, int MPC>
+static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, uint32_t tr, uint64_t entries, uint32_t xunits, int sm_count, cudaStream_t st) {
+    const uint32_t STAGE = tr * 16 * sp_pitch<T>(ALN);
+    bt.tr = tr;
+    uint32_t per = 0;   // chunks of an entry
+    for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].chunk_end = per += ((bt.op[i].n + 15) / 16 + tr - 1) / tr;
+    const uint64_t chunks = per * entries;
+    // one entry: neighbouring chunks go to different clusters; several: a contiguous share each, since a change of entry means other
+    // activations
+    bt.run = 1;
+    if (const char *e = exp_env("MLXN_SP_RUN")) bt.run = (uint32_t)atoi(e);
+    const size_t tail = sp_tail<T>(ALN, ranks, tr, bt.mp, xunits, nullptr);
+    uint32_t nslots = (uint32_t)((kSpSmem - 128 - tail) / STAGE);
+    if (nslots > (uint32_t)kSpMaxSlots) nslots = kSpMaxSlots;
+    if (tail + STAGE + 128 > kSpSmem || nslots < 1) return cudaErrorInvalidConfiguration;
+    bt.nslots = nslots;
+    bt.xf_off = nslots * STAGE;
+    sp_tail<T>(ALN, ranks, tr, bt.mp, xunits, &bt);
+    const size_t smem = (size_t)nslots * STAGE + tail + 128;
+    auto kernel = qmv_split_kernel<T, ALN, MPC>;
+    static std::atomic<uint32_t> prepared[64] = {};   // per device: attribute set, and the clusters that fit (bits 8.. by log2 ranks)
+    static std::atomic<uint32_t> fit[64][4] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!prepared[dev].load(std::memory_order_acquire)) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpSmem);
+        if (e != cudaSuccess) return e;
+        prepared[dev].store(1, std::memory_order_release);
+    }
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = ranks;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kSpThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    // clusters that are resident at the same time (a cluster lives in one GPC, so not every SM may be covered)
+    uint32_t ncl = (uint32_t)(2 * sm_count) / ranks;
+    if (ranks > 1) {
+        const int l = ranks == 2 ? 1 : ranks == 4 ? 2 : 3;
+        uint32_t f = fit[dev][l].load(std::memory_order_relaxed);
+        if (!f) {
+            int n = 0;
+            cfg.gridDim = dim3(ncl * ranks);
+            cfg.dynamicSmemBytes = kSpSmem;   // (the largest the kernel is launched with)
+            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+                (void)cudaGetLastError();
+                n = (int)ncl;
+            }
+            cfg.dynamicSmemBytes = smem;
+            f = (uint32_t)n;
+            fit[dev][l].store(f, std::memory_order_relaxed);
+        }
+        ncl = f < ncl ? f : ncl;
+    }
+    if (entries > 1) bt.run = 0;   // (counted on the device: only there the entries of a routed launch are known)
+    if (chunks < ncl) ncl = (uint32_t)chunks;
+    cfg.gridDim = dim3(ncl * ranks);
+    return cudaLaunchKernelEx(&cfg, kernel, bt, maps);
+}
+
+// Chooses the cluster size and the tiles of a chunk.
+template <int T, bool ALN, int MPC>
+static cudaError_t sp_choose(SpBatch &bt, const SpMaps &maps, uint64_t tiles, uint64_t entries, uint32_t max_units, bool routed, int sm_count, cudaStream_t st) {
+    constexpr int NS = MPC > 4 ? 2 : 1;
+    uint32_t best_c = 0, best_tr = 0;
+    double best = 1e30;
+    int force_c = 0, force_tr = 0;
+    if (const char *e = exp_env("MLXN_SP_C")) force_c = atoi(e);
+    if (const char *e = exp_env("MLXN_SP_TR")) force_tr = atoi(e);
+    for (uint32_t c = 1; c <= (routed ? 1u : 8u); c *= 2) {
+        const uint32_t slice = ((max_units + c - 1) / c + 3) / 4 * 4;
+        if (c > 1 && slice * (c - 1) >= max_units) continue;   // a rank without work
+        for (uint32_t tr = 1; tr <= (uint32_t)sp_tiles(NS); tr++) {
+            if ((force_c && !routed && (int)c != force_c) || (force_tr && (int)tr != force_tr)) continue;
+            const size_t stage = (size_t)tr * 16 * sp_pitch<T>(ALN), tail = sp_tail<T>(ALN, c, tr, bt.mp, (slice + 1) & ~1u, nullptr);
+            if (tail + 2 * stage + 128 > kSpSmem) continue;
+            const double slots = (double)((kSpSmem - 128 - tail) / stage);
+            const double ncl = (double)(2 * sm_count / (int)c), chunks = ceil(ceil((double)tiles / tr) / ncl);
+            // Measured (12288 x 4096 and 4096 x 4096, all types): a chunk takes 1.9 us of waits and sums whatever its size, plus
+            // 0.23 us per tile and unit of a warp (Q6_K 0.3; two sets of columns 1.5 times that, and there four ranks wait for
+            // one another for 4.5 us a chunk).
+            const double unit = (T == GT_Q6_K ? 0.3 : 0.23) * (NS == 2 ? 1.5 : 1.0);
+            // One row: splitting it takes 0.27 us per unit of a warp and CTA.
+            const double cost = (bt.packed ? 1.0 : 0.3 + 0.27 * ceil(slice / 8.0)) + chunks * ((NS == 2 && c == 4 ? 4.5 : 1.9) + tr * unit * ceil(slice / 8.0)) + (c > 1 ? 0.3 : 0.0) + (slots < 3 ? 0.3 : 0.0);
+            if (cost < best) {
+                best = cost;
+                best_c = c;
+                best_tr = tr;
+            }
+        }
+    }
+    if (!best_c) return cudaErrorInvalidConfiguration;
+    for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].slice = ((bt.op[i].units + best_c - 1) / best_c + 3) / 4 * 4;
+    const uint32_t xunits = (((max_units + best_c - 1) / best_c + 3) / 4 * 4 + 1) & ~1u;
+    return sp_launch<T, ALN, MPC>(bt, maps, best_c, best_tr, entries, xunits, sm_count, st);
+}
+
+// Scratch bytes of a mat-vec's packed activations.
+template <int T> inline size_t sp_pack_bytes(uint32_t m, uint32_t k) {
+    return ((size_t)m * (((k + 63) / 64 + 3) & ~3u) * (256 + 4 * SpTraits<T>::NG) + (size_t)m * 4 + 255) / 256 * 256;
+}
+
+// Instantiated once per block type (qmv_split_*.cu).  `ops`: dense, or all routed over the same pairs.
+template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, uint8_t *scratch, int *launches, cudaStream_t st) {
+    if (nops < 1 || nops > kSpMaxOps) return cudaErrorInvalidValue;
+    const bool routed = ops[0].ids != nullptr;
+    bool aln = true;
+    for (int i = 0; i < nops; i++) {
+        const uint64_t rb = (uint64_t)(ops[i].k / BlockTraits<T>::QK) * BlockTraits<T>::BYTES;
+        aln = aln && rb % 16 == 0 && ((uintptr_t)ops[i].w & 15u) == 0 && (!routed || ops[i].expert_stride % 16 == 0);
+    }
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return cudaErrorNotSupported;
+    static thread_local SpBatch bt;
+    alignas(64) static thread_local SpMaps maps;
+    bt.nops = (uint32_t)nops;
+    bt.ids = ops[0].ids;
+    bt.npairs = routed ? ops[0].nprob : 0;
+    bt.n_experts = routed ? ops[0].n_experts : 1;
+    bt.status = ops[0].status;
+    bt.early_weights = routed ? 0u : 1u;
+    uint32_t rows = 1, tiles = 0, max_units = 0;
+    for (int i = 0; i < nops; i++) {
+        const QmvArgs &a = ops[i];
+        SpOp &P = bt.op[i];
+        P.w = a.w;
+        P.x = a.x;
+        P.x2 = a.x2;
+        P.y = a.y;
+        P.n = a.n;
+        P.k = a.k;
+        P.m = a.m;
+        tiles += (a.n + 15) / 16;
+        P.row_bytes = (a.k / BlockTraits<T>::QK) * BlockTraits<T>::BYTES;
+        P.units = (a.k + 63) / 64;
+        P.x_div = a.top_k ? a.top_k : 1;
+        P.y_ld = qmv_ld(a);
+        P.y_col0 = a.y_col0;
+        P.n_peer = a.n_peer;
+        for (int q = 0; q < kMaxPeers; q++) P.y_peer[q] = q < (int)a.n_peer ? a.y_peer[q] : nullptr;
+        P.expert_stride = routed ? a.expert_stride : 0;
+        P.xkey = (uint32_t)i;
+        P.pk_units = (P.units + 3) & ~3u;
+        for (int q = 0; q < i; q++)
+            if (ops[q].x == a.x && ops[q].x2 == a.x2 && ops[q].m == a.m && ops[q].k == a.k && ops[q].top_k == a.top_k) {
+                P.xkey = bt.op[q].xkey;
+                P.xp = bt.op[q].xp;
+                P.xsum = bt.op[q].xsum;
+                P.xinv = bt.op[q].xinv;
+                break;
+            }
+        if (!routed && P.xkey == (uint32_t)i) {
+            const size_t u = (size_t)a.m * P.pk_units;
+            P.xp = scratch;
+            P.xsum = reinterpret_cast<float *>(scratch + u * 256);
+            P.xinv = P.xsum + u * SpTraits<T>::NG;
+            scratch += sp_pack_bytes<T>(a.m, a.k);
+        }
+        if (!a.early_weights) bt.early_weights = 0;
+        rows = a.m > rows ? a.m : rows;
+        max_units = P.units > max_units ? P.units : max_units;
+        if (aln) {
+            const cuuint64_t dim[3] = {P.row_bytes / 8, a.n, routed ? a.n_experts : 1}, stride[2] = {P.row_bytes, routed ? a.expert_stride : (uint64_t)P.row_bytes * a.n};
+            const cuuint32_t box[3] = {sp_pitch<T>(true) / 8, 16, 1}, one[3] = {1, 1, 1};
+            if (enc(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<uint8_t *>(a.w), dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                return cudaErrorInvalidValue;
+        }
+    }
+    // rows of an entry: dense, as many as fit two sets of columns; routed, one set (most experts have few rows)
+    bt.mp = routed ? (ops[0].nprob <= 1 ? 1u : 4u) : rows <= 1 ? 1u : rows <= 2 ? 2u : rows <= 4 ? 4u : 8u;
+    bt.nent = routed ? 0u : (rows + bt.mp - 1) / bt.mp;
+    const uint64_t entries = routed ? ops[0].nprob : bt.nent, all = tiles * entries;
+    bt.packed = !routed && bt.mp > 1;
+    *launches = 1;
+    auto go = [&](auto ALN) {
+        constexpr bool A = decltype(ALN)::value;
+        if (bt.packed) {
+            uint32_t end = 0;
+            for (int i = 0; i < nops; i++) bt.op[i].row_end = end += bt.op[i].xkey == (uint32_t)i ? bt.op[i].m : 0u;
+            const cudaError_t e = launch_overlapped(qmv_pack_kernel<T, A>, dim3(end), dim3(256), 0, st, bt);
+            if (e != cudaSuccess) return e;
+            ++*launches;
+        }
+        if (bt.mp == 1) return sp_choose<T, A, 1>(bt, maps, all, entries, max_units, routed, sm_count, st);
+        if (bt.mp <= 4) return sp_choose<T, A, 4>(bt, maps, all, entries, max_units, routed, sm_count, st);
+        return sp_choose<T, A, 8>(bt, maps, all, entries, max_units, routed, sm_count, st);
+    };
+    if (aln) return go(std::true_type{});
+    if constexpr (T == GT_Q4_K || T == GT_Q5_K) return cudaErrorNotSupported;   // (144- and 176-byte blocks: only a misaligned base)
+    else return go(std::false_type{});
+}
+
+}  // namespace mlxn

@@ -34,6 +34,11 @@ bool qmv_stream_available(int ggml_type, const QmvArgs &a, int sm_count);
 constexpr size_t kMvBatchMax = 16;   // mat-vecs one launch of the register-level kernel carries (kMwMaxProbs)
 bool qmv_mma_pair_mode(int ggml_type, const QmvArgs &a);
 cudaError_t launch_qmv_mma(int ggml_type, const QmvArgs *ops, int nops, int sm_count, int ctas_per_sm, int tpw, cudaStream_t st);
+bool qmv_split_supported(int ggml_type, const QmvArgs &a);
+bool qmv_split_aligned(int ggml_type, const QmvArgs &a);
+constexpr size_t kMvSplitMax = 8;    // mat-vecs one launch of the split kernel carries (kSpMaxOps)
+size_t qmv_split_scratch_bytes(const QmvArgs *ops, int nops);
+cudaError_t launch_qmv_split(int ggml_type, const QmvArgs *ops, int nops, int sm_count, uint8_t *scratch, int *launches, cudaStream_t st);
 cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t nt, uint8_t *scratch, cudaStream_t st,
                           int *launches);
 cudaError_t launch_qmm_simt(int ggml_type, const QmmArgs &a, bool routed, uint32_t max_rows, cudaStream_t st);
@@ -91,7 +96,7 @@ void mlxn_detail_count_launches(int launches) {
     g_last_kernel = "qmm_tc";
 }
 
-static std::atomic<int> g_opt_qmv{-1}, g_opt_qmm{-1};  // -1 unset; qmv: 0 simple, 1 stream, 2 tc, 3 auto, 4 mma; qmm: 0 simt, 1 tc
+static std::atomic<int> g_opt_qmv{-1}, g_opt_qmm{-1};  // -1 unset; qmv: 0 simple, 1 stream, 2 tc, 3 auto, 4 mma, 5 split; qmm: 0 simt, 1 tc
 static std::atomic<int> g_opt_mma_ctas{2}, g_opt_mma_tpw{0};   // tuning knobs of the register-level mat-vec
 static std::atomic<int> g_opt_mv_batch{1};                     // coalesce conflict-free mat-vecs into one launch
 // ... and mat-vecs that depend on one another (barriers inside the launch).  Off by default: measured on B200 a barrier
@@ -102,7 +107,7 @@ static int opt_qmv() {
     if (v < 0) {
         const char *e = getenv("MLXN_QMV");
         v = (e && strcmp(e, "simple") == 0) ? 0 : (e && strcmp(e, "stream") == 0) ? 1 : (e && strcmp(e, "tc") == 0) ? 2
-            : (e && strcmp(e, "mma") == 0) ? 4 : 3;
+            : (e && strcmp(e, "mma") == 0) ? 4 : (e && strcmp(e, "split") == 0) ? 5 : 3;
         g_opt_qmv = v;
     }
     return v;
@@ -291,6 +296,7 @@ struct mlxn_encoder {
     int pend_type = 0, pend_lane = 0;
     uint32_t pend_mp = 0;
     bool pend_pair = false;
+    bool pend_split = false;          // they are mat-vecs of the split kernel (qmv_split.cuh)
     bool grp_pend_only = false;       // every operation of the current group is in `pend` (none has been launched yet)
     uint32_t *status_host = nullptr;  // pinned
 };
@@ -348,7 +354,8 @@ extern "C" int mlxn_set_option(const char *key, const char *value) {
         else if (strcmp(value, "stream") == 0) g_opt_qmv = 1;
         else if (strcmp(value, "simple") == 0) g_opt_qmv = 0;
         else if (strcmp(value, "mma") == 0) g_opt_qmv = 4;
-        else return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: qmv must be 'auto', 'mma', 'tc', 'stream' or 'simple'");
+        else if (strcmp(value, "split") == 0) g_opt_qmv = 5;
+        else return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: qmv must be 'auto', 'split', 'mma', 'tc', 'stream' or 'simple'");
         return MLXN_OK;
     }
     if (strcmp(key, "qmv_batch") == 0) {
@@ -911,7 +918,12 @@ static int encoder_flush_pending(mlxn_encoder *e) {
     const bool q6_one_row_small = e->pend_type == GT_Q6_K && a0.m == 1 && (uint64_t)a0.n * a0.k < (1ull << 23);
     const bool lone_other = e->pend.size() == 1 && opt_qmv() == 3 && a0.n_peer == 0 && !a0.ids && e->pend_type != GT_Q4_K &&
                             (q6_one_row_small || a0.m > 2);
-    if (lone_other) {
+    if (e->pend_split) {
+        uint8_t *scratch = nullptr;
+        const size_t need = qmv_split_scratch_bytes(e->pend.data(), (int)e->pend.size());
+        if (!need || (rc = encoder_scratch_on(e, e->pend_lane, need, &scratch)) == MLXN_OK)
+            err = launch_qmv_split(e->pend_type, e->pend.data(), (int)e->pend.size(), e->dev->sm_count, scratch, &launches, st);
+    } else if (lone_other) {
         if (!q6_one_row_small && qmv_tc_supported(e->pend_type, a0)) {
             uint8_t *scratch = nullptr;
             if ((rc = encoder_scratch_on(e, e->pend_lane, qmv_tc_scratch_bytes(a0), &scratch)) == MLXN_OK) {
@@ -1515,6 +1527,35 @@ struct ShardOut {            // row-sharded output: see QmvArgs
     uint32_t y_ld = 0, y_col0 = 0, n_peer = 0;
     float *peer[kMaxPeers] = {};
 };
+// Adds mat-vecs to the encoder's open batch (launching it first where the new one does not fit in), as operation over `bufs`.
+static int batch_mv(mlxn_encoder *enc, int type, const QmvArgs &a, uint32_t mp, bool other_rows, std::initializer_list<OpBuf> bufs) {
+    const bool batch = g_opt_mv_batch.load() != 0;
+    const QmvArgs *h = enc->pend.empty() ? nullptr : &enc->pend[0];
+    // (routed ones share the launch's bucketing: the same pairs of the same experts)
+    const bool fits = batch && h && enc->pend_split && enc->pend_type == type && enc->pend_mp == mp && enc->pend_pair == other_rows &&
+                      enc->pend.size() < kMvSplitMax && h->ids == a.ids && h->nprob == a.nprob && h->n_experts == a.n_experts &&
+                      (a.ids ? h->k == a.k : a.m <= 8 || h->m == a.m);
+    int rc;
+    if (h && !fits && (rc = encoder_flush_pending(enc))) return rc;
+    if ((rc = op_begin(enc, bufs, true))) return rc;
+    if (enc->pend.empty()) {   // (a conflict found by op_begin has launched the batch and started a new group)
+        enc->pend_type = type;
+        enc->pend_mp = mp;
+        enc->pend_pair = other_rows;
+        enc->pend_split = true;
+        enc->pend_lane = enc->cur_lane;
+    }
+    enc->pend.push_back(a);
+    for (const OpBuf &ob : bufs) {
+        if (!ob.b) continue;
+        std::lock_guard<std::mutex> lk(ob.b->st->mu);
+        ob.b->st->pend_enc = enc;
+    }
+    g_last_kernel = "qmv_mma";
+    g_dispatch.fetch_add(1);
+    return batch ? MLXN_OK : encoder_flush_pending(enc);
+}
+
 static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, mlxn_buffer *input, mlxn_buffer *weight,
                        mlxn_buffer *output, const mlxn_qmm_params *p, const ShardOut *sh = nullptr) {
     int rc = touch_kernel(reg, dev, mv_kernel_name((int)p->ggml_type));
@@ -1555,6 +1596,30 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
         a.early_weights = weight->st->kernel_written ? 0u : 1u;
         return a;
     };
+    // The split kernel takes what the kernels with tensor maps do not (rows that do not start on 16-byte boundaries, any K; one or
+    // two rows of Q6_K stay with the streaming kernel, which is ahead there: 4096 x 2560 7.6 us against 9.7), Q4_K with more than
+    // four rows, and what it measured faster on, as one of a dependent chain: its fixed cost is higher and so is its rate.
+    //   one row:     24576 x 4096 Q4_0 17.6 us against 24.1, 12288 x 4096 11.3 / 12.4, 4096 x 4096 6.6 / 5.6
+    //   two rows:    24576 x 4096 20.0 / 26.1, 12288 x 4096 12.2 / 13.5, 4096 x 4096 7.9 / 7.4
+    //   four rows:   12288 x 4096 15.0 / 17.3, 4096 x 4096 8.4 / 9.5, 1024 x 4096 6.6 / 5.3, 4096 x 12288 17.7 / 16.8
+    // A mat-vec that can leave with an open batch of it joins that batch whatever its size.
+    if ((mode == 3 || mode == 5) && !g_opt_mv_chain.load()) {
+        const int t = (int)p->ggml_type;
+        QmvArgs a = make_args(0);
+        a.m = p->m;
+        const bool aligned = qmv_split_aligned(t, a);
+        const uint64_t values = (uint64_t)p->n * p->k;
+        bool pays;
+        if (!aligned) pays = t != GT_Q6_K || (p->m > 2 && !qmv_mma_pair_mode(t, a));
+        else if (p->m == 1) pays = values >= (48ull << 20);
+        else if (p->m == 2) pays = values >= (48ull << 20) && p->k <= 8192;
+        else if (p->m <= 4) pays = values >= (16ull << 20) && (p->k <= 8192 || t == GT_Q4_K);
+        else pays = t == GT_Q4_K;
+        if (!enc->pend.empty() && enc->pend_split && enc->pend_type == t && !enc->pend[0].ids && enc->pend_mp == mv_row_class(p->m) && aligned) pays = true;
+        pays = pays || mode == 5;
+        if (pays && qmv_split_supported(t, a) && (p->m <= 8 || !sh))
+            return batch_mv(enc, t, a, p->m <= 8 ? mv_row_class(p->m) : 16u, !aligned, {{input, false}, {weight, false}, {output, true}});
+    }
     // A mat-vec for the register-level kernel is not launched at once: it waits for the operations that follow, and
     // conflict-free mat-vecs of the same block type leave as one kernel (upstream dispatches the operations between
     // two barriers concurrently, src/encoder.rs:837-853).  The group ends, and the kernel is launched, at the first
@@ -1564,7 +1629,7 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
         if (wants_mma(a0) && qmv_mma_supported((int)p->ggml_type, a0)) {
             const bool batch = g_opt_mv_batch.load() != 0;
             const bool pair = qmv_mma_pair_mode((int)p->ggml_type, a0);
-            const bool fits = batch && !enc->pend.empty() && enc->pend_type == (int)p->ggml_type &&
+            const bool fits = batch && !enc->pend.empty() && !enc->pend_split && enc->pend_type == (int)p->ggml_type &&
                               enc->pend_mp == mv_row_class(a0.m) && enc->pend_pair == pair && enc->pend.size() < kMvBatchMax;
             if (!enc->pend.empty() && !fits && (rc = encoder_flush_pending(enc))) return rc;
             // A mat-vec that depends on the batch it would join (it reads a result of the batch, or writes over one)
@@ -1579,6 +1644,7 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
             if (enc->pend.empty()) {
                 enc->pend_type = (int)p->ggml_type;
                 enc->pend_mp = mv_row_class(a0.m);
+                enc->pend_split = false;
                 enc->pend_pair = pair;
                 enc->pend_lane = enc->cur_lane;
             }
@@ -1886,15 +1952,18 @@ static int dispatch_id_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *de
     // Few rows (decode): every (token, slot) row is one mat-vec of the register-level kernel, and the rows of this call,
     // and of the calls around it that do not depend on it (gate and up of one layer), leave as one launch.
     const int mode = opt_qmv();
+    if ((mode == 3 || mode == 5) && qmv_split_supported(t, a))
+        return batch_mv(enc, t, a, 1u, !qmv_split_aligned(t, a), {{input, false}, {up, false}, {weight, false}, {ids, false}, {output, true}});
     if ((mode == 3 || mode == 4) && rows <= kMvBatchMax && qmv_mma_supported_routed(t, a)) {
         const bool batch = g_opt_mv_batch.load() != 0;
-        const bool fits = batch && !enc->pend.empty() && enc->pend_type == t && enc->pend_mp == 1 && !enc->pend_pair &&
+        const bool fits = batch && !enc->pend.empty() && !enc->pend_split && enc->pend_type == t && enc->pend_mp == 1 && !enc->pend_pair &&
                           enc->pend.size() + rows <= kMvBatchMax;
         if (!enc->pend.empty() && !fits && (rc = encoder_flush_pending(enc))) return rc;
         if ((rc = op_begin(enc, {{input, false}, {up, false}, {weight, false}, {ids, false}, {output, true}}, true))) return rc;
         if (enc->pend.empty()) {
             enc->pend_type = t;
             enc->pend_mp = 1;
+            enc->pend_split = false;
             enc->pend_pair = false;
             enc->pend_lane = enc->cur_lane;
         }
@@ -2087,7 +2156,9 @@ extern "C" int mlxn_moe_ffn_layer(mlxn_encoder *enc, mlxn_registry *reg, mlxn_de
         if ((rc = mlxn_quantized_matmul_id_ggml(enc, reg, dev, x, gate_w, ids, gate_out, &pg))) return rc;
         if ((rc = mlxn_quantized_matmul_id_ggml(enc, reg, dev, x, up_w, ids, up_out, &pu))) return rc;
         const int td = (int)p->down_type;
-        if (!id_routes_to_mm(&pd) && (td == GT_Q4_0 || td == GT_Q8_0 || td == GT_Q6_K)) {
+        // (the down projection's rows are pairs: few tokens stay on the mat-vec route, with f32 operands, even where there are
+        //  more pairs than the routing threshold)
+        if (pairs <= 256 && (td == GT_Q4_0 || td == GT_Q8_0 || td == GT_Q6_K)) {
             mlxn_qmm_id_params ps = pd;
             return mlxn_quantized_matmul_id_swiglu(enc, reg, dev, gate_out, up_out, down_w, ids, down_out, &ps);
         }

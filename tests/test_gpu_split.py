@@ -1,0 +1,92 @@
+"""The split mat-vec (csrc/qmv_split.cuh) at the edges of its tiles, slices, alignments and row groups, against the oracle."""
+import numpy as np
+import pytest
+
+import mlx_native_b200 as mx
+from oracle import oracle as orc
+from tests.gpu_util import MV_TOL, TYPES, Ctx, norm_err, normal_acts, normal_weights
+from tests.test_oracle_q5k import random_q5k_blocks
+
+pytestmark = pytest.mark.gpu
+ALL = dict(TYPES, Q4_K=(mx.GgmlType.Q4_K, orc.Q4_K))
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    mx.set_option("qmv", "split")          # wherever it can, not only where it is the faster kernel
+    yield Ctx()
+    mx.set_option("qmv", "auto")
+
+
+# 16-row tiles, units of 64 values, slices of 256 over up to 8 ranks, sets of 4 activation rows; K that is no multiple of 256
+# (rows at any even address), of 64 (half a unit), or shorter than a slice
+@pytest.mark.parametrize("tname,n,k,m", [
+    ("Q4_0", 1, 32, 1), ("Q4_0", 17, 96, 2), ("Q4_0", 15, 256, 3), ("Q4_0", 333, 2880, 5), ("Q4_0", 64, 4096, 8), ("Q4_0", 2500, 1056, 1),
+    ("Q8_0", 1, 32, 8), ("Q8_0", 31, 160, 1), ("Q8_0", 2873, 2880, 5), ("Q8_0", 48, 512, 4), ("Q8_0", 130, 12288, 8), ("Q8_0", 1030, 4128, 2),
+    ("Q6_K", 1, 256, 1), ("Q6_K", 33, 768, 7), ("Q6_K", 70, 2048, 2), ("Q6_K", 19, 5120, 8), ("Q6_K", 1001, 2560, 1), ("Q6_K", 12, 14336, 3),
+    ("Q4_K", 16, 256, 1), ("Q4_K", 65, 768, 6), ("Q4_K", 40, 3584, 4), ("Q4_K", 130, 1024, 9), ("Q4_K", 50, 2304, 33)])
+def test_dense(ctx, tname, n, k, m):
+    gtype, otype = ALL[tname]
+    wq = normal_weights(n + k + m, n, k, otype)
+    x = normal_acts(n + m, m, k)
+    x[:, ::7] *= 1e-4          # (one power-of-two scale per row and slice)
+    y = ctx.matmul(gtype, wq, x, n, k)
+    y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8)
+    assert norm_err(y, y_ref, ad) <= MV_TOL
+    assert np.array_equal(y.view(np.uint32), ctx.matmul(gtype, wq, x, n, k).view(np.uint32))
+
+
+@pytest.mark.parametrize("tname,offset", [("Q4_0", 2), ("Q4_0", 12), ("Q8_0", 6), ("Q8_0", 14), ("Q6_K", 2), ("Q6_K", 10)])
+@pytest.mark.parametrize("m", [1, 6])
+def test_weights_at_any_even_address(ctx, tname, offset, m):
+    gtype, otype = TYPES[tname]
+    n, k = 77, 2048
+    wq = normal_weights(5, n, k, otype)
+    big = np.zeros(wq.size + 64, np.uint8)
+    big[offset:offset + wq.size] = wq
+    x = normal_acts(1, m, k)
+    y = ctx.matmul(gtype, wq, x, n, k, weight_buf=ctx.buf(big, mx.DType.U8).slice_view(offset, wq.size))
+    y_ref, ad = orc.qmatmul(otype, wq, x, n, k)
+    assert norm_err(y, y_ref, ad) <= MV_TOL
+
+
+# routed: experts without rows, with one row, with more than a pass takes (4); ids that name no expert; aligned rows and not
+@pytest.mark.parametrize("tname,T,top_k,E,n,k", [
+    ("Q4_0", 1, 8, 16, 40, 512), ("Q4_0", 32, 8, 8, 65, 288), ("Q8_0", 24, 8, 128, 48, 768), ("Q8_0", 7, 3, 5, 17, 96), ("Q6_K", 20, 4, 6, 50, 768),
+    ("Q6_K", 3, 1, 4, 130, 2048), ("Q4_K", 32, 4, 16, 33, 2048), ("Q5_K", 9, 8, 32, 100, 512), ("Q5_K", 32, 8, 4, 16, 256)])
+def test_routed(ctx, tname, T, top_k, E, n, k):
+    rng = np.random.default_rng(T * 100 + n)
+    if tname == "Q5_K":
+        gtype, otype = mx.GgmlType.Q5_K, orc.Q5_K
+        w = random_q5k_blocks(rng, E * n * (k // 256))
+    else:
+        gtype, otype = ALL[tname]
+        w = normal_weights(E + n, E * n, k, otype)
+    x = normal_acts(T, T, k)
+    ids = rng.integers(0, E, T * top_k).astype(np.uint32)
+    bad = np.zeros(ids.size, bool)
+    if ids.size > 20:
+        bad[[5, 11]] = True
+    y, _ = ctx.matmul_id(gtype, w, w.size // E, x, np.where(bad, 0xFFFFFFFF, ids).astype(np.uint32), top_k, n, k, E)
+    y_ref, ad = orc.qmatmul_id(otype, w, w.size // E, x, ids, top_k, n, k, E, nthreads=8)
+    assert norm_err(y[~bad], y_ref[~bad], ad[~bad]) <= MV_TOL
+    assert np.all(y[bad] == 0)
+
+
+def test_batch_of_different_shapes(ctx):
+    """Mat-vecs of one launch that differ in rows, K (ranks without work for the shorter one), activations and row count."""
+    gtype, otype = TYPES["Q8_0"]
+    d = ctx.device
+    shapes = [(100, 4096, 8), (33, 512, 5), (16, 4096, 7), (257, 1024, 8)]
+    ws = [normal_weights(i, n, k, otype) for i, (n, k, m) in enumerate(shapes)]
+    xs = [normal_acts(i, m, k) for i, (n, k, m) in enumerate(shapes)]
+    bufs = [(ctx.buf(x, mx.DType.F32), ctx.buf(w, mx.DType.U8), d.alloc_buffer(m * n * 4, mx.DType.F32)) for x, w, (n, k, m) in zip(xs, ws, shapes)]
+    mx.reset_counters()
+    enc = d.command_encoder()
+    for (xb, wb, yb), (n, k, m) in zip(bufs, shapes):
+        mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, wb, yb, mx.GgmlQuantizedMatmulParams(m, n, k, gtype))
+    enc.commit_and_wait()
+    assert mx.kernel_launch_count() == 2          # the activations of all of them packed by one kernel, then one mat-vec kernel
+    for (xb, wb, yb), w, x, (n, k, m) in zip(bufs, ws, xs, shapes):
+        y_ref, ad = orc.qmatmul(otype, w, x, n, k)
+        assert norm_err(yb.as_slice(np.float32).reshape(m, n), y_ref, ad) <= MV_TOL
