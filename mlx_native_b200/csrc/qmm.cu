@@ -187,20 +187,38 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const uint32_t *htpe, 
     if (tid == 0) tiles[0] = carry_s < max_tiles ? carry_s : max_tiles;
 }
 
-// Packs activation rows into f16 tiles of NT rows x 64 columns laid out exactly as the tensor core
+// How a dense mat-mat's work is dealt out when CTAs share tiles: tiles (weight tile fastest) x raw stages of 256 K values in one row,
+// cut into `ctas` contiguous ranges.  No tile is cut twice (a range is at least a tile long, or exactly half a tile): a shared
+// tile is the sum of two parts added onto zeros, which is the same in either order.
+struct TcShare {
+    uint32_t ctas;        // 0: every CTA takes whole tiles
+    uint32_t n_wt, nraw;  // weight-row tiles; raw stages of a tile
+    uint32_t total;       // tiles x nraw
+    __host__ __device__ uint32_t begin(uint32_t cta) const { return (uint32_t)((uint64_t)total * cta / ctas); }
+};
+
+// Packs activation rows into f16 tiles of nt rows (a multiple of 16) x 64 columns laid out exactly as the tensor core
 // reads a K-major 128-byte-swizzled operand: row r, 16-byte chunk j (8 halves) of a tile lives at
-// (r/8)*1024 + (r%8)*128 + ((j ^ (r%8)) * 16).  Tile (t, kc) starts at ((t*nchunks + kc) * NT*128) bytes.
-// grid (nchunks, ntile_bound); 256 threads.
-template <int NT>
-__global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t zero_y) {
-    // grid (K-chunk lanes, tiles): CTA (c, t) packs the chunks c, c + gridDim.x, ... of tile t, so that the tile's
-    // routing lookups (a chain of dependent loads) are paid once per CTA, not once per chunk.
-    const uint32_t t = blockIdx.y;
+// (r/8)*1024 + (r%8)*128 + ((j ^ (r%8)) * 16).  Tile (t, kc) starts at ((t*nchunks + kc) * nt*128) bytes.
+// A CTA packs a slice of 64 rows, which is two 16-byte columns per thread and chunk: with whole tiles of 256 rows per CTA,
+// 512 x 4096 activations took 10 us, most of it one load after another; with slices 6.
+// grid (tiles x slices, K-chunk lanes), 256 threads.
+constexpr uint32_t kPackRows = 64;
+__global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t nt, const TcShare sh) {
+    // CTA (t, c) packs the chunks c, c + gridDim.y, ... of its slice, so that the slice's routing lookups (a chain of
+    // dependent loads) are paid once per CTA, not once per chunk.
+    const uint32_t slices = (nt + kPackRows - 1) / kPackRows, t = blockIdx.x / slices, r0 = (blockIdx.x - t * slices) * kPackRows;
     allow_dependents();   // the mat-mat kernel behind may set itself up; it waits for this grid before it reads anything
-    if (zero_y) {  // split-K tiles add their halves into y with atomics (dense form only)
-        const size_t total = (size_t)a.m * a.n, ncta = (size_t)gridDim.x * gridDim.y, cta = (size_t)t * gridDim.x + blockIdx.x;
-        const size_t per = (total + ncta - 1) / ncta, lo = cta * per, hi = lo + per < total ? lo + per : total;
-        for (size_t i = lo + threadIdx.x; i < hi; i += 256) a.y[i] = 0.f;
+    if (sh.ctas) {  // output tiles that two CTAs of the mat-mat share are added up in y (dense form only): zero them, 64 rows at a time
+        const uint32_t jobs = (sh.ctas - 1) * slices, ncta = gridDim.x * gridDim.y;
+        for (uint32_t j = blockIdx.y * gridDim.x + blockIdx.x; j < jobs; j += ncta) {
+            const uint32_t b = j / slices, pos = sh.begin(b + 1), tile = pos / sh.nraw;
+            if (tile * sh.nraw == pos) continue;   // the boundary between two CTAs is one between tiles
+            const uint32_t tt = tile / sh.n_wt, col = (tile - tt * sh.n_wt) * 128u + (threadIdx.x & 127u), lo = (j - b * slices) * kPackRows;
+            const uint32_t end = min(a.m, tt * nt + min(nt, lo + kPackRows));
+            if (col < a.n)
+                for (uint32_t row = tt * nt + lo + (threadIdx.x >> 7); row < end; row += 2) a.y[(size_t)row * a.n + col] = 0.f;
+        }
     }
     uint32_t e = 0, mt = t, nrows = a.m;
     if (a.hids) {
@@ -209,14 +227,13 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
         mt = a.tiles[2 + 2 * t];
         nrows = a.htpe[e];
     }
-    constexpr int kPer = (NT * 8 + 255) / 256;   // (row, 16-byte column) pairs per thread: the same ones in every chunk
+    constexpr int kPer = 2;   // (row, 16-byte column) pairs per thread: the same ones in every chunk
     const float *src_row[kPer];
 #pragma unroll
     for (int i = 0; i < kPer; i++) {
-        const uint32_t q = threadIdx.x + i * 256, r = q >> 3;
-        const uint32_t row = mt * NT + r;
+        const uint32_t r = r0 + ((threadIdx.x + i * 256) >> 3), row = mt * nt + r;
         src_row[i] = nullptr;
-        if (q < NT * 8 && row < nrows) {
+        if (r < nt && row < nrows) {
             int64_t src = row;
             if (a.hids) {
                 const int32_t id = a.hids[(size_t)e * a.hids_stride + row];
@@ -226,13 +243,13 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
             if (src >= 0) src_row[i] = a.x_bf16 ? reinterpret_cast<const float *>(a.x_bf16) : a.x + (size_t)src * a.k;
         }
     }
-    for (uint32_t kc = blockIdx.x; kc < nchunks; kc += gridDim.x) {
-        uint8_t *tile = xpack + ((size_t)t * nchunks + kc) * (size_t)(NT * 128);
+    for (uint32_t kc = blockIdx.y; kc < nchunks; kc += gridDim.y) {
+        uint8_t *tile = xpack + ((size_t)t * nchunks + kc) * (size_t)(nt * 128);
 #pragma unroll
         for (int i = 0; i < kPer; i++) {
             const uint32_t q = threadIdx.x + i * 256;
-            if (q >= NT * 8) break;
-            const uint32_t r = q >> 3, j = q & 7u;
+            const uint32_t r = r0 + (q >> 3), j = q & 7u;
+            if (r >= nt) break;
             const uint32_t k0 = kc * 64 + 8 * j;
             uint4 out = make_uint4(0, 0, 0, 0);
             if (src_row[i] && k0 < a.k) {
@@ -240,7 +257,7 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
                 float v[8];
                 if (a.x_bf16) {
                     // eight consecutive K values lie inside one head (head_dim is a multiple of 32): 16 bytes of bf16
-                    const uint32_t h = k0 / a.head_dim, d0 = k0 - h * a.head_dim, row = mt * NT + r;
+                    const uint32_t h = k0 / a.head_dim, d0 = k0 - h * a.head_dim, row = mt * nt + r;
                     const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(a.x_bf16 + ((size_t)h * a.m + row) * a.head_dim + d0));
                     const uint32_t w4[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
@@ -280,8 +297,10 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
 // =================================================================================================
 // qmm_tc
 // =================================================================================================
-constexpr int kTcDequantWarps = 16;  // two sets of 8: set s dequantises the K stages with st % 2 == s
-constexpr int kTcThreads = (kTcDequantWarps + 4) * 32;  // + activation producer, MMA, weight producer, second MMA warp
+// Dequantising warps of a CTA: 16 in two sets of 8, set s dequantises the K stages with st % 2 == s; or, with two CTAs on an SM (PAIR),
+// one set that takes all stages.  Beside them the activation producer, MMA, weight producer and second MMA warp.
+__host__ __device__ constexpr int tc_dequant_warps(bool pair) { return pair ? 8 : 16; }
+__host__ __device__ constexpr int tc_threads(bool pair) { return (tc_dequant_warps(pair) + 4) * 32; }
 constexpr int kTcRowsW = 128;                           // weight rows per tile (UMMA M)
 
 template <int T> struct TcTraits;
@@ -556,40 +575,48 @@ struct TcCfg {
     uint32_t debug;       // experiment switches: 1 = skip dequantisation, 2 = skip raw copies, 4 = skip MMA, 8 = skip B copies
     uint32_t n_wt;        // weight-row tiles, ceil(n / 128)
     uint32_t ntiles;      // activation tiles: the count (dense) or its bound (routed: the list's length is read on the device)
-    uint32_t ksplit;      // K split factor (1 or 2)
+    uint32_t nt;          // activation rows of a tile (a multiple of 16, at most NT)
+    TcShare share;        // the CTAs' ranges where tiles are shared
     uint32_t stage_off;   // byte offset of the two staged output tiles (narrow tiles only), 0 = write y straight from registers
-    uint32_t raw_tma;     // raw weight stages arrive as one tensor copy each (needs `aligned`); otherwise 16-byte cp.async
+    uint32_t raw_tma;     // raw weight stages arrive as tensor copies; otherwise 16-byte cp.async
+    uint32_t row_group;   // log2 of the copies of a stage: the map's rows are groups of 1, 2, 4 or 8 weight rows (see launch_tc_tn)
 };
 
 // ring of dequantised weight stages held in tensor memory: the columns the accumulators leave free.  Tiles of 64
 // activation rows (two 64-column accumulators) keep six stages in columns [128, 512), wider ones four in [256, 512):
 // the ring's depth over the latency of the loop dequantise -> MMA -> commit -> reuse is what bounds a narrow tile.
-template <int NT> struct TcRing {
-    static constexpr int kStages = NT <= 64 ? 6 : 4;
-    static constexpr int kColBase = NT <= 64 ? 128 : 256;
+template <int NT, bool PAIR> struct TcRing {
+    static constexpr int kStages = PAIR ? 3 : NT <= 64 ? 6 : 4;
+    static constexpr int kColBase = PAIR ? 64 : NT <= 64 ? 128 : 256;
 };
 constexpr int kTcACols = 64;       // one stage: 128 K values as f16 pairs = 64 32-bit columns
-constexpr int kTcTmemCols = 512;
+constexpr int kTcTmemCols = 512;   // of an SM: two CTAs have half each
 
-// grid = min(work items, SMs) persistent CTAs; kTcThreads threads; 1 CTA per SM.
+// grid = min(work items, SMs) persistent CTAs; tc_threads(PAIR) threads; 1 CTA per SM, or 2 (PAIR).
 //
-// Data flow per work item (one 128-row weight tile x one NT-row activation tile, all of K or one K split):
+// Data flow per work item (one 128-row weight tile x one NT-row activation tile, all of K or, where tiles are shared, a part of it):
 //   raw GGML blocks  --cp.async-->  shared-memory ring  --dequantise (16 warps)-->  f16 pairs in registers
 //   --tcgen05.st-->  tensor-memory ring (A operand)  --tcgen05.mma, B = packed activations from the bulk-copy
 //   ring in shared memory-->  f32 accumulator in tensor memory  --tcgen05.ld-->  y.
 // The dequantised weights never touch shared memory: its bandwidth is the scarce resource here (the tensor
 // core already reads the whole activation tile from it for every MMA).
-template <int T, int NT, bool SH>
-__global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, const TcCfg c, const uint8_t *xpack,
+//
+// PAIR: two CTAs per SM, each with one set of dequantising warps, one accumulator and half of tensor memory.  For routed calls, whose
+// items are short (64 rows, K of a few raw stages): what an item costs beside its stages -- accumulator drain, read-back, the first
+// stages of the next one, 5000 cycles -- is then time in which the other CTA works.  128 experts, 512 tokens, 8 of them each: Q4_0
+// 768 x 2048 80 -> 62 us, Q6_K 2048 x 768 (rows of 630 bytes, now tensor copies) 175 -> 102 us; weights once at 6.4 TB/s: 18 and 25 us.
+template <int T, int NT, bool SH, bool PAIR>
+__global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(const QmmArgs a, const TcCfg c, const uint8_t *xpack,
                                                                 const __grid_constant__ CUtensorMap wmap) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // tensor-core operand tiles need 1024-byte alignment (128-byte swizzle atoms): align by hand
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES, KR = TcTraits<T>::KR;
-    constexpr int kMaxB = 8, kMaxRaw = 6;
-    constexpr int kTcAStages = TcRing<NT>::kStages, kTcAColBase = TcRing<NT>::kColBase;
+    constexpr int kMaxB = PAIR ? 6 : 8, kMaxRaw = 6, kTcDequantWarps = tc_dequant_warps(PAIR);
+    constexpr int kTcAStages = TcRing<NT, PAIR>::kStages, kTcAColBase = TcRing<NT, PAIR>::kColBase;
+    static_assert(!PAIR || (NT == 64 && !SH), "two CTAs per SM: tiles of 64 rows");
     static_assert(kMaxB / 2 <= kTcAStages, "an activation chunk's place is freed by a stage_done phase the producer can still see");
-    constexpr int kNumMma = NT <= 128 ? 2 : 1;   // issuing threads, each with its own accumulator
+    constexpr int kNumMma = PAIR || NT > 128 ? 1 : 2;   // issuing threads, each with its own accumulator
     __shared__ __align__(8) uint64_t a_full[kTcAStages], stage_done[kTcAStages], b_full[kMaxB];
     __shared__ __align__(8) uint64_t raw_full[kMaxRaw], raw_empty[kMaxRaw], acc_full, acc_empty, orow_ready[2], stage_ready[2];
     __shared__ uint32_t tmem_base_s;
@@ -606,6 +633,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t tid = threadIdx.x - kCtrlWarps * 32;   // index among the dequantising threads (wraps for warps 0-3)
     const uint32_t row_bytes = (a.k / QK) * BB;
+    const bool raw_tma = PAIR || c.raw_tma != 0;
 
     // ---- set-up that needs nothing from the kernels ahead in the stream (it overlaps their tail: the kernel is
     // ---- launched with programmatic stream serialisation), then the wait for them
@@ -616,13 +644,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
             peer_y[4] = a.y_peer[4]; peer_y[5] = a.y_peer[5]; peer_y[6] = a.y_peer[6];
         }
         for (uint32_t s = 0; s < kTcAStages; s++) {
-            mbar_init(&a_full[s], kTcDequantWarps / 2);  // the eight warps of one set
+            mbar_init(&a_full[s], 8);  // the eight warps of one set
             mbar_init(&stage_done[s], 1);
         }
         for (uint32_t s = 0; s < c.b_stages; s++) mbar_init(&b_full[s], 1);
         for (uint32_t s = 0; s < c.raw_slots; s++) {
             // one asynchronous arrival per copying thread, or the weight producer's single arrival with the byte count
-            mbar_init(&raw_full[s], c.raw_tma ? 1u : kTcDequantWarps * 32);
+            mbar_init(&raw_full[s], raw_tma ? 1u : kTcDequantWarps * 32);
             mbar_init(&raw_empty[s], kTcDequantWarps);
         }
         mbar_init(&acc_full, kNumMma);
@@ -634,20 +662,23 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
         mbar_init_fence();
     }
     if (warp == kWarpMma0) {  // the first MMA warp owns tensor memory
-        tmem_alloc(&tmem_base_s, kTcTmemCols);
+        tmem_alloc(&tmem_base_s, kTcTmemCols / (PAIR ? 2 : 1));
         tmem_relinquish();
     }
-    grid_dependency_wait();   // the packed activations, the tile list and (split-K) the zeroed y are complete
+    grid_dependency_wait();   // the packed activations, the tile list and the zeros of shared tiles are complete
     allow_dependents();
 
-    // ---- work items: (weight-row tile, K split, token tile), weight tile fastest; CTA b takes items b, b + grid, ...
-    // Every role walks the same item sequence; ring slots and barrier phases run on across items, so the next
+    // ---- work items: (weight-row tile, token tile), weight tile fastest; CTA b takes items b, b + grid, ... or, where
+    // tiles are shared (TcShare), the parts of tiles that lie in its range.  Every role walks the same item sequence; ring slots and barrier phases run on across items, so the next
     // item's weights are already on their way while this item's accumulator is read back.
     const uint32_t n_tt = a.hids ? min(a.tiles[0], c.ntiles) : c.ntiles;   // uniform for the whole CTA
-    const uint32_t total_items = c.n_wt * c.ksplit * n_tt;
+    const uint32_t total_items = c.n_wt * n_tt;
     const uint32_t nraw_all = (a.k + KR - 1) / KR;
+    const bool shared = !PAIR && c.share.ctas != 0;
+    const uint32_t nt = PAIR ? (uint32_t)NT : c.nt;
+    const uint32_t pos0 = shared ? c.share.begin(blockIdx.x) : blockIdx.x, pos1 = shared ? c.share.begin(blockIdx.x + 1) : total_items;
     struct Item {
-        uint32_t tt, e, mt, n0, r_lo, nraw, nst, nck, kc_lo;
+        uint32_t tt, e, mt, n0, r_lo, nraw, nst, nck, kc_lo, next;
         const uint8_t *wbase;
     };
     // routed: the (expert, row tile) pairs of the CTA's first items, fetched once (a lookup per item would put a
@@ -657,16 +688,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
     if (a.hids && threadIdx.x < kMetaItems) {
         const uint32_t item = blockIdx.x + threadIdx.x * gridDim.x;
         if (item < total_items) {
-            const uint32_t tt = item / (c.n_wt * c.ksplit);
+            const uint32_t tt = item / c.n_wt;
             meta[threadIdx.x][0] = a.tiles[1 + 2 * tt];
             meta[threadIdx.x][1] = a.tiles[2 + 2 * tt];
         }
     }
-    auto load_item = [&](uint32_t item) -> Item {
+    auto load_item = [&](uint32_t pos) -> Item {
         Item it;
-        const uint32_t rest = item / c.n_wt, wt = item - rest * c.n_wt;
-        const uint32_t z = c.ksplit == 1 ? 0u : rest % c.ksplit;
-        it.tt = c.ksplit == 1 ? rest : rest / c.ksplit;
+        const uint32_t item = shared ? pos / nraw_all : pos;
+        it.r_lo = shared ? pos - item * nraw_all : 0u;
+        const uint32_t r_hi = shared ? min(nraw_all, it.r_lo + (pos1 - pos)) : nraw_all;
+        it.next = shared ? pos + (r_hi - it.r_lo) : pos + gridDim.x;
+        it.tt = item / c.n_wt;
+        const uint32_t wt = item - it.tt * c.n_wt;
         it.e = 0;
         it.mt = it.tt;
         if (a.hids) {
@@ -681,9 +715,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
         }
         it.wbase = a.w + (size_t)it.e * a.expert_stride;
         it.n0 = wt * kTcRowsW;
-        // split-K: this item takes the raw stages [r_lo, r_hi) of K and adds its part of the tile into y
-        it.r_lo = c.ksplit == 1 ? 0u : (z * nraw_all) / c.ksplit;   // (ksplit <= 2 and nraw_all < 2^24: no overflow)
-        const uint32_t r_hi = c.ksplit == 1 ? nraw_all : ((z + 1) * nraw_all) / c.ksplit;
         it.nraw = r_hi - it.r_lo;
         it.kc_lo = it.r_lo * (KR / 64);
         it.nst = min((a.k + 127) / 128, r_hi * (KR / 128)) - it.r_lo * (KR / 128);   // tensor-memory stages
@@ -696,7 +727,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
     tc_fence_after();
     const uint32_t tmem_d = tmem_base_s;
     const uint32_t smem_base = smem_u32(smem);
-    const uint32_t b_bytes = NT * 128;                 // one 64-wide K chunk of the activation tile
+    const uint32_t b_bytes = nt * 128;                 // one 64-wide K chunk of the activation tile
     const uint32_t raw_stage_bytes = kTcRowsW * c.seg_stride;
     // wait styles: the single producer / MMA warps spin (they are the critical path and cost one warp's issue
     // slots); the dequantising warps space their polls out
@@ -727,8 +758,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
         if (lane == 0) {
             uint32_t s = 0, G = 0;
             bool ok = true;
-            for (uint32_t item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
-                const Item it = load_item(item);
+            for (uint32_t pos = pos0; ok && pos < pos1;) {
+                const Item it = load_item(pos);
+                pos = it.next;
                 for (uint32_t kc = 0; kc < 2 * it.nst; kc++, G++) {
                     if (G >= c.b_stages) {
                         const uint32_t j = (G - c.b_stages) >> 1;
@@ -750,17 +782,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
             }
         }
     } else if (warp == kWarpWeights) {
-        // ======================= weight producer warp: one tensor copy per raw stage =======================
-        // The weights as a 3-D tensor of 32-bit words [expert][row][row_bytes / 4]; a raw stage is the box
-        // (1, 128 rows, seg_stride / 4 words) at the stage's K offset, rounded down to 16 bytes for Q6_K
-        // (210-byte super-blocks; readers skip the lead-in).  Rows past n arrive as zeros.  The copies run
-        // raw_slots - 1 stages ahead of the dequantisation, across item boundaries.
-        if (c.raw_tma && lane == 0) {
+        // ======================= weight producer warp: tensor copies of raw stages =======================
+        // The weights as a 3-D tensor of 32-bit words [expert][row group][words]; a raw stage is 128 rows' bytes of 256 K values, each
+        // from the 16-byte boundary below (readers skip the lead-in).  A copy brings one row of every group: rows i, i + G, ... of the
+        // tile land together, i = 0 .. G - 1.  Rows past n arrive as zeros.  The copies run raw_slots - 1 stages ahead of the
+        // dequantisation, across item boundaries.
+        if (raw_tma && lane == 0) {
             const uint32_t R = c.raw_slots;
             uint32_t slot = 0, ph = 0, requested = 0;
             bool ok = true;
-            for (uint32_t item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
-                const Item it = load_item(item);
+            for (uint32_t pos = pos0; ok && pos < pos1;) {
+                const Item it = load_item(pos);
+                pos = it.next;
                 for (uint32_t r = 0; r < it.nraw; r++, requested++) {
                     if (requested >= R &&
                         !mbar_wait(&raw_empty[slot], ph ^ 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, wmode_cr)) {
@@ -768,13 +801,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                         break;
                     }
                     TRACE(0, 1, requested);
-                    const uint32_t kb = ((it.r_lo + r) * (KR / QK) * BB) & ~15u;   // byte offset of the stage in the row
+                    const uint32_t kb = (it.r_lo + r) * (KR / QK) * BB;   // byte offset of the stage in a row
                     mbar_expect_tx(&raw_full[slot], raw_stage_bytes);
-                    asm volatile(
-                        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                        ::"r"(smem_base + c.raw_off + slot * raw_stage_bytes), "l"(&wmap), "r"(kb >> 2), "r"(it.n0), "r"(it.e),
-                          "r"(smem_u32(&raw_full[slot]))
-                        : "memory");
+                    for (uint32_t i = 0; i < 1u << c.row_group; i++)
+                        asm volatile(
+                            "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                            ::"r"(smem_base + c.raw_off + slot * raw_stage_bytes + i * (raw_stage_bytes >> c.row_group)), "l"(&wmap),
+                              "r"(((i * row_bytes + kb) & ~15u) >> 2), "r"(it.n0 >> c.row_group), "r"(it.e), "r"(smem_u32(&raw_full[slot]))
+                            : "memory");
                     if (++slot == R) { slot = 0; ph ^= 1u; }
                 }
             }
@@ -790,15 +824,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
         // and there the MMAs are long enough to hide the issue).
         const uint32_t w = warp == kWarpMma0 ? 0u : 1u;
         if (lane == 0 && w < (uint32_t)kNumMma) {
-            constexpr uint32_t idesc = umma_idesc_f16(kTcRowsW, NT);
+            const uint32_t idesc = umma_idesc_f16(kTcRowsW, nt);
             const uint64_t bd0 = umma_desc_k_sw128(smem_base + c.b_off);
             const uint64_t b_step = b_bytes >> 4;  // descriptor address field is in 16-byte units
             const bool do_mma = !(MLXN_DBG(c) & 4u);
             const uint32_t d_col = tmem_d + w * NT;
             uint32_t sa = 0, aph = 0, sb = 0, bph = 0, nitem = 0;   // ring positions of the stage being looked at
             bool ok = true;
-            for (uint32_t item = blockIdx.x; ok && item < total_items; item += gridDim.x, nitem++) {
-                const Item it = load_item(item);
+            for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
+                const Item it = load_item(pos);
+                pos = it.next;
                 // the accumulators of the item before have been read back
                 if (nitem > 0 &&
                     !mbar_wait(&acc_empty, (nitem - 1) & 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, wmode_cr))
@@ -857,8 +892,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
         // 32 (w % 4) + l of the tile -- the tensor-memory lane its warp may address -- and the 64-element half
         // (w / 4) % 2 of the stage: thirty-two packed f16 pairs = one 32-column store.
         const uint32_t dw = warp - kCtrlWarps;   // 0..15
-        const uint32_t q4 = dw & 3u, half = (dw >> 2) & 1u, set = dw >> 3;
+        const uint32_t q4 = dw & 3u, half = (dw >> 2) & 1u, set0 = dw >> 3;
         const uint32_t rr = q4 * 32 + lane;
+        const uint32_t srow = ((rr & ((1u << c.row_group) - 1u)) << (7 - c.row_group)) + (rr >> c.row_group);   // the row's place in a raw stage
         // Raw weight rows are short (144..272 bytes per stage and row), too short for one bulk copy each to be
         // efficient, so all dequantising threads stream them as 16-byte cp.async chunks, a few raw stages ahead
         // of the one being dequantised.  Each row is fetched as the 16-byte aligned superset of its (only
@@ -868,15 +904,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
         constexpr int kRawSlots = 5;            // (128 rows x at most 19 chunks) / 512 threads, rounded up
         constexpr uint32_t kSegFull = (KR / QK) * BB;
         constexpr uint32_t kCmax = (kSegFull + 30u) >> 4;  // most 16-byte chunks a row segment can need
-        static_assert(kTcRowsW * kCmax <= kRawSlots * kTcDequantWarps * 32, "raw copy slots");
+        static_assert(PAIR || kTcRowsW * kCmax <= kRawSlots * kTcDequantWarps * 32, "raw copy slots");
         static_assert(KR == 256, "a raw stage feeds one K stage of each set");
         const uint8_t *slot_src[kRawSlots];     // start of the thread's row (global), for the item being requested
         uint32_t slot_dst[kRawSlots];           // row's place inside a raw stage + chunk offset (shared, relative)
         uint32_t slot_cc[kRawSlots];            // chunk index within the row, 0xFFFFFFFF = unused in this item
         // request cursor: runs ahead of the dequantisation, across item boundaries
-        uint32_t q_item = blockIdx.x, q_r = 0, q_nraw = 0, q_rlo = 0;
+        uint32_t q_pos = pos0, q_next = pos0, q_r = 0, q_nraw = 0, q_rlo = 0;
         auto open_request_item = [&]() {
-            const Item it = load_item(q_item);
+            const Item it = load_item(q_pos);
+            q_next = it.next;
             const uint32_t rows_here = min((uint32_t)kTcRowsW, a.n - it.n0);
 #pragma unroll
             for (int i = 0; i < kRawSlots; i++) {
@@ -891,7 +928,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
             q_nraw = it.nraw;
             q_rlo = it.r_lo;
         };
-        if (!c.raw_tma && q_item < total_items) open_request_item();
+        if (!raw_tma && q_pos < pos1) open_request_item();
         auto issue_raw = [&](uint32_t r, uint32_t slot) {
             const uint32_t k0 = r * KR;
             const uint32_t seg_bytes = (min((uint32_t)KR, a.k - k0) / QK) * BB;
@@ -919,25 +956,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
         bool ok = true;
         const uint32_t a_dst = tmem_d + ((q4 * 32) << 16) + kTcAColBase + 32 * half;
         const uint32_t g = dw >> 2;
-        for (uint32_t item = blockIdx.x; ok && item < total_items; item += gridDim.x, nitem++) {
-            const Item it = load_item(item);
+        for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
+            const Item it = load_item(pos);
+            pos = it.next;
             const uint32_t n0 = it.n0;
             const bool row_ok = n0 + rr < a.n;
             const uint32_t row_lo4 = (uint32_t)((uintptr_t)(it.wbase + (size_t)(n0 + rr) * row_bytes) & 15u);
             // the item's output-row table: every thread fetches the entries it will publish now (the loads stay in
             // flight behind the K loop) and stores them just before the epilogue
             static_assert(NT <= kTcDequantWarps * 32, "one output-row entry per thread");
-            if (q4 == 0 && half == 0) TRACE(2 + set, 1, nitem);
+            if (q4 == 0 && half == 0) TRACE(2 + set0, 1, nitem);
             uint32_t o_nrows = a.m;
             int32_t o_id = -1;
-            const uint32_t o_row = it.mt * NT + tid;
-            if (a.hids && tid < NT) {
+            const uint32_t o_row = it.mt * nt + tid;
+            if (a.hids && tid < nt) {
                 o_nrows = a.htpe[it.e];
                 if (o_row < a.hids_stride) o_id = a.hids[(size_t)it.e * a.hids_stride + o_row];
             }
             for (uint32_t r = 0; ok && r < it.nraw; r++) {
                 // keep D raw stages requested ahead of the one being read
-                while (!c.raw_tma && q_item < total_items && requested - consumed < D + 1) {
+                while (!raw_tma && q_pos < pos1 && requested - consumed < D + 1) {
                     if (requested >= R &&
                         !mbar_wait(&raw_empty[islot], iph ^ 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, wmode_dq)) {
                         ok = false;
@@ -947,13 +985,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                     requested++;
                     if (++islot == R) { islot = 0; iph ^= 1u; }
                     if (++q_r == q_nraw) {
-                        q_item += gridDim.x;
-                        if (!c.raw_tma && q_item < total_items) open_request_item();
+                        q_pos = q_next;
+                        if (q_pos < pos1) open_request_item();
                     }
                 }
                 if (!ok) break;
                 if (!mbar_wait(&raw_full[rs], rph, &abort_flag, a.status, ST_WAIT_FULL_TIMEOUT, wmode_dq)) { ok = false; break; }
-                if (q4 == 0 && half == 0) TRACE(2 + set, 2, r);
+                if (q4 == 0 && half == 0) TRACE(2 + set0, 2, r);
+                for (uint32_t set = set0; set < 2; set += kTcDequantWarps / 8) {   // (PAIR: the one set takes both K stages)
                 const uint32_t st = 2 * r + set;       // this set's K stage inside raw stage r
                 if (st < it.nst) {
                     const uint32_t J = J0 + st;        // its number in the CTA's whole run
@@ -966,13 +1005,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                         break;
                     }
                     tc_fence_after();
-                    if (q4 == 0 && half == 0) TRACE(2 + set, 3, r);
+                    if (q4 == 0 && half == 0) TRACE(2 + set0, 3, r);
                     const uint32_t r_abs = it.r_lo + r;
                     const uint32_t pre = (row_lo4 + ((r_abs * KR) / QK) * BB) & 15u;
-                    const uint32_t seg = smem_base + c.raw_off + rs * raw_stage_bytes + rr * c.seg_stride + pre;
+                    const uint32_t seg = smem_base + c.raw_off + rs * raw_stage_bytes + srow * c.seg_stride + pre;
                 uint32_t regs[32];
                 if (T != GT_Q4_K && c.aligned && row_ok && !(MLXN_DBG(c) & 1u)) {   // (Q4_K: the generic extraction below)
-                    const uint32_t stage_row = smem_base + c.raw_off + rs * raw_stage_bytes + rr * c.seg_stride;
+                    const uint32_t stage_row = smem_base + c.raw_off + rs * raw_stage_bytes + srow * c.seg_stride;
                     if constexpr (T == GT_Q6_K) {
                         dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half, regs);
                         dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half + 1, regs + 16);
@@ -1004,18 +1043,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                         }
                     }
                 }
-                    if (q4 == 0 && half == 0) TRACE(2 + set, 8, r);
+                    if (q4 == 0 && half == 0) TRACE(2 + set0, 8, r);
                     tmem_st_32x32_x32(a_dst + sa * kTcACols, regs);
                     tmem_st_wait();
-                    if (q4 == 0 && half == 0) TRACE(2 + set, 9, r);
+                    if (q4 == 0 && half == 0) TRACE(2 + set0, 9, r);
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&a_full[sa]);
-                    if (q4 == 0 && half == 0) TRACE(2 + set, 4, r);
+                    if (q4 == 0 && half == 0) TRACE(2 + set0, 4, r);
                 }
+                }
+                if (!ok) break;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&raw_empty[rs]);  // this warp is done reading the raw stage
-                if (q4 == 0 && half == 0) TRACE(2 + set, 10, r);
+                if (q4 == 0 && half == 0) TRACE(2 + set0, 10, r);
                 consumed++;
                 if (++rs == R) { rs = 0; rph ^= 1u; }
             }
@@ -1026,7 +1067,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                 int32_t *wtab = orow[nitem & 1u];
                 if (tid < NT) {
                     int32_t o = -1;
-                    if (o_row < o_nrows) {
+                    if (tid < nt && o_row < o_nrows) {
                         if (a.hids) {
                             if (o_id >= 0 && (uint32_t)o_id < a.total_rows) o = o_id;
                         } else {
@@ -1039,12 +1080,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                 if (lane == 0) mbar_arrive(&orow_ready[nitem & 1u]);
             }
             if (!mbar_wait(&orow_ready[nitem & 1u], (nitem >> 1) & 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, wmode_dq)) break;
-            if (q4 == 0 && half == 0) TRACE(2 + set, 5, nitem);
+            if (q4 == 0 && half == 0) TRACE(2 + set0, 5, nitem);
             if (!mbar_wait(&acc_full, nitem & 1u, &abort_flag, a.status, ST_WAIT_MMA_TIMEOUT, wmode_dq)) break;
             tc_fence_after();
-            if (q4 == 0 && half == 0) TRACE(2 + set, 6, nitem);
+            if (q4 == 0 && half == 0) TRACE(2 + set0, 6, nitem);
             const int32_t *tab = orow[nitem & 1u];
             const uint32_t wrow = n0 + rr;
+            const bool part = it.nraw < nraw_all;   // another CTA has the rest of this tile's K
             if (c.stage_off) {
                 // Staged read-back (narrow tiles): the accumulator goes to shared memory as [activation row][weight
                 // row], tensor memory is handed back to the MMA warps at once, and every warp then writes whole
@@ -1052,7 +1094,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                 constexpr uint32_t kPitch = kTcRowsW + 4;   // floats per staged row
                 float *stg = reinterpret_cast<float *>(smem + c.stage_off) + (nitem & 1u) * (NT * kPitch);
 #pragma unroll 1
-                for (uint32_t col = g * 32; col < NT; col += (kTcDequantWarps / 4) * 32) {
+                for (uint32_t col = g * 32; col < nt; col += (kTcDequantWarps / 4) * 32) {
                     uint32_t v[32];
                     tmem_ld_32x32(tmem_d + ((q4 * 32) << 16) + col, v);
                     if (kNumMma == 2 && it.nst >= 2) {
@@ -1090,11 +1132,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                         }
                     }
                 }
-                if (q4 == 0 && half == 0) TRACE(2 + set, 7, nitem);
+                if (q4 == 0 && half == 0) TRACE(2 + set0, 7, nitem);
                 continue;
             }
 #pragma unroll 1
-            for (uint32_t col = g * 32; col < NT; col += (kTcDequantWarps / 4) * 32) {
+            for (uint32_t col = g * 32; col < nt; col += (kTcDequantWarps / 4) * 32) {
                 uint32_t v[32];
                 tmem_ld_32x32(tmem_d + ((q4 * 32) << 16) + col, v);
                 if (kNumMma == 2 && it.nst >= 2) {   // the odd K stages went into the second accumulator
@@ -1111,7 +1153,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                         for (int j = 0; j < 32; j++) {
                             const int32_t o = tab[col + j];
                             if (o >= 0) {
-                                if (c.ksplit > 1) atomicAdd(&a.y[(size_t)o * a.n + wrow], __uint_as_float(v[j]));
+                                if (part) atomicAdd(&a.y[(size_t)o * a.n + wrow], __uint_as_float(v[j]));
                                 else a.y[(size_t)o * a.n + wrow] = __uint_as_float(v[j]);
                             }
                         }
@@ -1131,7 +1173,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty);   // the MMA warp may start the next item's accumulation
-            if (q4 == 0 && half == 0) TRACE(2 + set, 7, nitem);
+            if (q4 == 0 && half == 0) TRACE(2 + set0, 7, nitem);
         }
     }
     if (abort_flag) {  // let copies in flight land before the CTA's shared memory is released
@@ -1141,7 +1183,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
     __syncthreads();
     if (warp == kWarpMma0) {
         tc_fence_after();
-        tmem_dealloc(tmem_d, kTcTmemCols);
+        tmem_dealloc(tmem_d, kTcTmemCols / (PAIR ? 2 : 1));
     }
 }
 
@@ -1174,37 +1216,54 @@ size_t qmm_tc_scratch_bytes(const QmmArgs &a, uint32_t nt, bool routed) {
     return header + tiles * nchunks * (size_t)nt * 128;
 }
 
-// Activation rows per tile.  Routed calls use 64 (few rows per expert).  Dense calls take the tile that
-// minimises waves x per-tile cost, where a tile costs about max(NT, 160) (tensor time vs the fixed
-// dequantisation of its 128 weight rows); ties go to the larger tile, which dequantises less in total.
-// Split-K factor for a dense call: 2 when the tile grid alone would fill at most ~half of the SMs and K is long
-// enough to share (two halves added onto a zeroed y give the same sum in either order).
-uint32_t qmm_tc_ksplit(uint32_t nt, uint32_t rows, uint32_t n, uint32_t k, int sm_count, bool routed) {
-    if (routed || exp_env("MLXN_TC_NO_SPLITK")) return 1;
-    const uint64_t tiles = (uint64_t)((n + kTcRowsW - 1) / kTcRowsW) * ((rows + nt - 1) / nt);
-    return (tiles * 2 <= (uint64_t)sm_count + sm_count / 8 && k >= 2048) ? 2u : 1u;
+// Activation rows per tile and the CTAs' shares.  Routed calls use tiles of 64 rows, whole.  A dense call takes the combination
+// that costs least.  A K stage of 128 values costs nt + 390 (units of 1.74 ns: 4096 x 4096 Q4_0 in one wave takes 30 us with 64
+// rows, 33 with 128, 38 with 192 and 41 with 256: the chain from raw block to tensor memory bounds a stage, the multiplication adds
+// to it), an item 2000 beside its stages.
+//   * whole tiles: waves x tile.
+//   * shared tiles, as many CTAs as SMs: no last wave, but one more hand-off, and the shared tiles are zeroed and added up in y.  Has
+//     to promise 11 %: Q4_0 512 x 12288 x 4096 (1.3 waves of 256 rows) takes 66 us where whole tiles of 128 rows took 86; Q6_K 2048 x
+//     4096 x 12288 (1.7 waves) took 300 us for the whole call, with whole tiles 295.
+//   * every tile in two halves, where all halves fit on the chip at once and K is long enough (8 raw stages).
+// Rows are spread evenly: 333 rows are two tiles of 176, not 256 and 77.
+struct TcPlan {
+    uint32_t nt, ctas, shared;
+};
+static uint64_t tc_plan(uint32_t nt, uint64_t rows, uint64_t n, uint64_t k, uint64_t sms, bool sharded, TcPlan &p) {
+    const uint64_t tiles = (n + kTcRowsW - 1) / kTcRowsW * ((rows + nt - 1) / nt), nraw = (k + 255) / 256;
+    const uint64_t tile = 2 * nraw * (nt + 390);   // a tile's stages
+    uint64_t best = (tiles + sms - 1) / sms * (tile + 2000);
+    p = {nt, (uint32_t)(tiles < sms ? tiles : sms), 0};
+    if (sharded || tiles * nraw >= (1ull << 31)) return best;
+    if (tiles > sms && nraw >= 2) {
+        const uint64_t cost = (tiles * tile / sms + (tiles / sms + 2) * 3000) * 111 / 100;
+        if (cost < best) {
+            best = cost;
+            p = {nt, (uint32_t)sms, 1};
+        }
+    } else if (2 * tiles <= sms && nraw >= 8) {
+        const uint64_t cost = tile / 2 + 4600;
+        if (cost < best) {
+            best = cost;
+            p = {nt, (uint32_t)(2 * tiles), 1};
+        }
+    }
+    return best;
 }
 
-uint32_t qmm_tc_pick_nt(int ggml_type, uint32_t rows, uint32_t n, int sm_count, bool routed) {
-    if (routed || rows <= 64) return 64;
-    (void)ggml_type;
-    const uint32_t cap = 256u;
-    const uint32_t cands[3] = {256, 128, 64};
-    uint32_t best = cap;
+uint32_t qmm_tc_pick_nt(uint32_t rows, uint32_t n, uint32_t k, int sm_count, bool routed, bool sharded) {
+    if (routed) return 64;
+    uint32_t best = 256;
     uint64_t best_cost = ~0ull;
-    const uint32_t wt = (n + kTcRowsW - 1) / kTcRowsW;
-    for (uint32_t nt : cands) {
-        if (nt > cap) continue;
-        if (nt / 2 >= rows && nt > 64) continue;  // more than half of the tile would be padding
-        // (K is not known here: assume it is long enough to split when the grid is small)
-        const uint64_t ks = qmm_tc_ksplit(nt, rows, n, 4096, sm_count, false);
-        const uint64_t tiles = (uint64_t)wt * ((rows + nt - 1) / nt) * ks;
-        const uint64_t waves = (tiles + sm_count - 1) / (uint64_t)sm_count;
-        const uint64_t cost = waves * (nt > 160 ? nt : 160) / ks;
-        if (cost < best_cost) {
+    for (uint32_t tt = (rows + 255) / 256, last = tt + 8; tt <= last; tt++) {
+        const uint32_t nt = ((rows + tt - 1) / tt + 15) / 16 * 16;
+        TcPlan p;
+        const uint64_t cost = tc_plan(nt, rows, n, k, (uint64_t)sm_count, sharded, p);
+        if (best_cost == ~0ull || cost * 103 / 100 < best_cost) {   // (near a tie, the larger tile: it converts less in all)
             best_cost = cost;
             best = nt;
         }
+        if (nt == 16) break;
     }
     return best;
 }
@@ -1215,10 +1274,13 @@ bool qmm_tc_supported(const QmmArgs &a) {
     return true;
 }
 
-template <int T, int NT, bool SH>
-static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint8_t *scratch, cudaStream_t st, int *launches) {
+template <int T, int NT, bool SH, bool PAIR = false>
+static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint32_t nt, uint8_t *scratch, cudaStream_t st, int *launches) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES, KR = TcTraits<T>::KR;
     TcCfg c{};
+    c.nt = nt;
+    TcPlan plan;
+    tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count_of_device(), SH || routed, plan);
     {
         const char *dbg = exp_env("MLXN_TC_DEBUG");
         c.debug = dbg ? (uint32_t)atoi(dbg) : 0u;
@@ -1231,38 +1293,45 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint8_t *scratch, cudaSt
     c.nchunks = (a.k + 63) / 64;
     c.seg_stride = round_up_u((KR / QK) * BB + 15, 16) + 16;
     if ((c.seg_stride / 16) % 2 == 0) c.seg_stride += 16;  // odd multiple of 16 B: rows spread over the banks
-    // Aligned weights arrive by tensor copies: one per raw stage instead of 16-byte copies from every thread.
-    // The box is the stage's bytes of 128 rows (Q6_K: 224 bytes cover 210 plus the lead-in; 240 keeps the row
-    // pitch an odd multiple of 16).  A 3-D map [expert][row][words]; dense calls are one expert.
+    // The weights arrive by tensor copies instead of 16-byte copies from every thread.  A copy has to start on a 16-byte boundary, which
+    // every G-th row does (G = 1, 2, 4 or 8): the map's rows are groups of G weight rows, and a raw stage is G copies, each of one row
+    // of every group.  The box is a stage's bytes of a row and the lead-in, an odd multiple of 16 (the rows' pitch in shared memory).
+    // A 3-D map [expert][row group][words]; dense calls are one expert.  Needs n to be a multiple of G.
     alignas(64) CUtensorMap wmap;
     memset(&wmap, 0, sizeof(wmap));
-    if (c.aligned && !exp_env("MLXN_TC_NO_TMA")) {
+    {
         EncodeTiledFn enc = encode_tiled_fn();
         const uint32_t row_bytes = (a.k / QK) * BB;
-        const uint32_t box_bytes = T == GT_Q6_K ? 240u : (uint32_t)((KR / QK) * BB);
+        uint32_t lg = 0;
+        while ((row_bytes << lg) & 15u) lg++;
+        constexpr uint32_t kSeg = (KR / QK) * BB;
+        const uint32_t box_bytes = lg == 0 && kSeg % 16 == 0 ? kSeg : ((kSeg + 14 + 15) / 16 | 1u) * 16;
         const uint32_t n_exp = routed ? a.n_experts : 1u;
         const uint64_t estride = routed ? a.expert_stride : (uint64_t)a.n * row_bytes;
-        if (enc && n_exp >= 1 && (uint64_t)row_bytes * a.n <= estride) {
-            const cuuint64_t gdim[3] = {row_bytes / 4, a.n, n_exp};
-            const cuuint64_t gstride[2] = {row_bytes, estride};
-            const cuuint32_t box[3] = {box_bytes / 4, (cuuint32_t)kTcRowsW, 1};
+        const bool fits = (((uintptr_t)a.w | estride) & 15u) == 0 && a.n % (1u << lg) == 0 && (uint64_t)row_bytes * a.n <= estride;
+        if (enc && n_exp >= 1 && fits && !exp_env("MLXN_TC_NO_TMA")) {
+            const cuuint64_t gdim[3] = {((uint64_t)row_bytes << lg) / 4, a.n >> lg, n_exp};
+            const cuuint64_t gstride[2] = {(uint64_t)row_bytes << lg, estride};
+            const cuuint32_t box[3] = {box_bytes / 4, (cuuint32_t)(kTcRowsW >> lg), 1};
             const cuuint32_t estr[3] = {1, 1, 1};
             if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint8_t *>(a.w), gdim, gstride, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS) {
                 c.raw_tma = 1;
+                c.row_group = lg;
                 c.seg_stride = box_bytes;
             }
         }
     }
-    const uint32_t b_bytes = NT * 128;  // one 64-wide K chunk of the activation tile
+    if (PAIR && !c.raw_tma) return launch_tc_tn<T, NT, SH, false>(a, routed, nt, scratch, st, launches);
+    const uint32_t b_bytes = nt * 128;  // one 64-wide K chunk of the activation tile
     const uint32_t raw_slot = kTcRowsW * c.seg_stride;
-    uint32_t limit = 222 * 1024;  // + 1 KB alignment slack + ~3 KB of static shared memory <= 227 KB
+    // + 1 KB alignment slack + 1 to 3 KB of static shared memory: 227 KB, or half of 228 KB less the 1 KB that the system takes of each CTA
+    uint32_t limit = (PAIR ? 108 : 222) * 1024;
     // narrow tiles stage their result in shared memory (two tiles of NT x 132 floats) and write whole output rows
     const uint32_t stage_bytes = 2u * NT * (kTcRowsW + 4) * 4u;
-    // (the row-sharded form never splits K: its tiles go straight to every rank's buffer)
-    constexpr bool sharded = SH;                         // a.y_ld != 0 || a.n_peer != 0
-    const bool staged = NT == 64 && (sharded || qmm_tc_ksplit(NT, a.m, a.n, a.k, sm_count_of_device(), routed) == 1) &&
+    // (the row-sharded form never shares tiles: they go straight to every rank's buffer)
+    const bool staged = NT == 64 && !PAIR && !plan.shared &&
                         ((((uintptr_t)a.y) | ((uintptr_t)qmm_ld(a) * 4u) | ((uintptr_t)a.y_col0 * 4u)) & 15u) == 0 && a.n_peer == 0 &&
                         !exp_env("MLXN_TC_NO_STAGED_OUT");
     if (staged) limit -= stage_bytes;
@@ -1270,7 +1339,7 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint8_t *scratch, cudaSt
     uint32_t b_stages = (limit - 2 * raw_slot) / b_bytes;
     // (a 64-row tile's chunks are 8 KB: eight of them where four raw slots still fit beside them, the loop being
     // bound by how far the copies run ahead of the MMAs)
-    const uint32_t b_cap = (NT == 64 && limit >= 8 * b_bytes + 4 * raw_slot) ? 8u : 6u;
+    const uint32_t b_cap = (NT == 64 && !PAIR && limit >= 8 * b_bytes + 4 * raw_slot) ? 8u : 6u;
     if (b_stages > b_cap) b_stages = b_cap;
     if (const char *e = exp_env("MLXN_TC_STAGES")) {  // experiment switch
         const uint32_t v = (uint32_t)atoi(e);
@@ -1291,31 +1360,35 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint8_t *scratch, cudaSt
     if (staged) c.stage_off = c.raw_off + raw_bytes;
     const size_t smem = (size_t)c.raw_off + raw_bytes + (staged ? stage_bytes : 0u) + 1024;  // + slack for manual 1024-byte alignment
 
-    const uint32_t ksplit = sharded ? 1u : qmm_tc_ksplit(NT, a.m, a.n, a.k, sm_count_of_device(), routed);
     size_t tiles;
     uint8_t *xpack = scratch;
     if (routed) {
-        tiles = (size_t)a.total_rows / NT + a.n_experts;
+        tiles = (size_t)a.total_rows / nt + a.n_experts;
         if (tiles > a.total_rows) tiles = a.total_rows;
         if (tiles == 0) tiles = 1;
         const size_t header = ((1 + 2 * tiles) * 4 + 1023) / 1024 * 1024;
         uint32_t *tl = reinterpret_cast<uint32_t *>(scratch);
         if (!(a.reuse & 1u)) {   // (an earlier call of the same layer built the list: same buckets, same NT)
-            build_tiles_kernel<<<1, 256, 0, st>>>(a.htpe, a.n_experts, NT, (uint32_t)tiles, tl);
+            build_tiles_kernel<<<1, 256, 0, st>>>(a.htpe, a.n_experts, nt, (uint32_t)tiles, tl);
             (*launches)++;
         }
         a.tiles = tl;
         xpack = scratch + header;
     } else {
-        tiles = (a.m + NT - 1) / NT;
+        tiles = (a.m + nt - 1) / nt;
         a.tiles = nullptr;
     }
+    c.n_wt = (a.n + kTcRowsW - 1) / kTcRowsW;
+    c.ntiles = (uint32_t)tiles;
+    const uint32_t nraw = (a.k + KR - 1) / KR;
+    if (plan.shared) c.share = {plan.ctas, c.n_wt, nraw, (uint32_t)(c.n_wt * tiles * nraw)};
     if (!(a.reuse & 2u)) {   // (... or packed the same activation rows already)
         // enough CTAs to fill the GPU a few times over, few enough that a tile's routing lookups are amortised
         uint32_t lanes = c.nchunks;
-        while (lanes > 1 && (uint64_t)lanes * tiles > 2048) lanes = (lanes + 1) / 2;
-        dim3 grid(lanes, (unsigned)tiles);
-        pack_x_kernel<NT><<<grid, 256, 0, st>>>(a, xpack, c.nchunks, ksplit > 1 ? 1u : 0u);
+        const uint64_t slices = (uint64_t)tiles * ((nt + kPackRows - 1) / kPackRows);
+        while (lanes > 1 && (uint64_t)lanes * slices > 2048) lanes = (lanes + 1) / 2;
+        dim3 grid((unsigned)slices, lanes);
+        pack_x_kernel<<<grid, 256, 0, st>>>(a, xpack, c.nchunks, nt, c.share);
         (*launches)++;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -1325,42 +1398,34 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint8_t *scratch, cudaSt
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (smem > attr_smem[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(qmm_tc_kernel<T, NT, SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(qmm_tc_kernel<T, NT, SH, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         attr_smem[dev] = smem;
     }
-    c.n_wt = (a.n + kTcRowsW - 1) / kTcRowsW;
-    c.ntiles = (uint32_t)tiles;
-    c.ksplit = ksplit;
-    // persistent CTAs, one per SM, each walking its share of the (weight tile, K split, activation tile) items
-    const uint64_t items = (uint64_t)c.n_wt * tiles * ksplit;
-    uint32_t ctas = (uint32_t)sm_count_of_device();
-    if (const char *e = exp_env("MLXN_TC_CTAS")) {  // experiment switch
-        const int v = atoi(e);
-        if (v >= 1 && v <= 4096) ctas = (uint32_t)v;
+    // persistent CTAs, one per SM (PAIR: two), each walking its items
+    uint32_t ctas = plan.ctas;
+    if (routed) {
+        const uint64_t items = (uint64_t)c.n_wt * tiles;
+        ctas = (uint32_t)sm_count_of_device() * (PAIR ? 2u : 1u);
+        if (items < ctas) ctas = (uint32_t)items;
     }
-    if (items < ctas) ctas = (uint32_t)items;
     if (ctas == 0) return cudaSuccess;
     (*launches)++;
-    return launch_overlapped(qmm_tc_kernel<T, NT, SH>, dim3(ctas), dim3(kTcThreads), smem, st, a, c, xpack, wmap);
+    return launch_overlapped(qmm_tc_kernel<T, NT, SH, PAIR>, dim3(ctas), dim3(tc_threads(PAIR)), smem, st, a, c, xpack, wmap);
 }
 
 template <int T> static cudaError_t launch_tc_t(const QmmArgs &a, bool routed, uint32_t nt, uint8_t *scratch, cudaStream_t st,
                                                 int *launches) {
+    if (nt == 0 || nt % 16 != 0 || nt > 256 || (routed && nt != 64)) return cudaErrorInvalidValue;
     if (a.y_ld != 0 || a.n_peer != 0) {   // row-sharded result: the instantiation with the peer stores
-        switch (nt) {
-        case 64: return launch_tc_tn<T, 64, true>(a, routed, scratch, st, launches);
-        case 128: return launch_tc_tn<T, 128, true>(a, routed, scratch, st, launches);
-        case 256: return launch_tc_tn<T, 256, true>(a, routed, scratch, st, launches);
-        default: return cudaErrorInvalidValue;
-        }
+        if (nt <= 64) return launch_tc_tn<T, 64, true>(a, routed, nt, scratch, st, launches);
+        if (nt <= 128) return launch_tc_tn<T, 128, true>(a, routed, nt, scratch, st, launches);
+        return launch_tc_tn<T, 256, true>(a, routed, nt, scratch, st, launches);
     }
-    switch (nt) {
-    case 64: return launch_tc_tn<T, 64, false>(a, routed, scratch, st, launches);
-    case 128: return launch_tc_tn<T, 128, false>(a, routed, scratch, st, launches);
-    case 256: return launch_tc_tn<T, 256, false>(a, routed, scratch, st, launches);
-    default: return cudaErrorInvalidValue;
-    }
+    if (routed) return launch_tc_tn<T, 64, false, true>(a, routed, nt, scratch, st, launches);
+    if (nt <= 64) return launch_tc_tn<T, 64, false>(a, routed, nt, scratch, st, launches);
+    if (nt <= 128) return launch_tc_tn<T, 128, false>(a, routed, nt, scratch, st, launches);
+    return launch_tc_tn<T, 256, false>(a, routed, nt, scratch, st, launches);
 }
 
 // tcgen05 mat-mat.  `scratch` must hold qmm_tc_scratch_bytes(a, nt, routed) bytes and start on a 256-byte boundary (the packed
@@ -1489,8 +1554,11 @@ extern "C" int mlxn_quantized_matmul_ggml_mm_noalloc(void *cuda_stream, const vo
     a.n_experts = 1;
     a.total_rows = params->m;
     a.status = nullptr;  // no status word: a wait that gives up still ends the kernel, but is not reported
-    const uint32_t nt = qmm_tc_pick_nt(t, a.m, a.n, sms, false);
-    const size_t need = qmm_tc_scratch_bytes(a, nt, false);
+    uint32_t nt = qmm_tc_pick_nt(a.m, a.n, a.k, sms, false, false);
+    size_t need = qmm_tc_scratch_bytes(a, nt, false);
+    // (the fastest tile may pad the rows more than another one that still fits)
+    for (uint32_t other : {256u, 128u, 64u})
+        if (need > MLXN_NOALLOC_SCRATCH_BYTES) need = qmm_tc_scratch_bytes(a, nt = other, false);
     if (need > MLXN_NOALLOC_SCRATCH_BYTES) {
         char msg[256];
         snprintf(msg, sizeof(msg),
