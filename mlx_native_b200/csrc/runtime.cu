@@ -181,10 +181,14 @@ struct mlxn_registry {
 
 // Device status words (see ST_* in common.cuh).  Ref-counted: the kernels of a captured graph keep writing to the
 // block of the encoder that recorded them, so the block must outlive that encoder for as long as the graph exists.
+// The status word itself is pinned host memory that kernels address directly: they write it only when a wait has given up, and the
+// host reads it after the wait for the commit's event, without a copy of its own in every command buffer.
 struct StatusBlock {
     std::atomic<int> refs{1};
     int ordinal = 0;
-    uint32_t *dev = nullptr;
+    uint32_t *dev = nullptr;        // zeroed words for barriers between a kernel's blocks
+    uint32_t *word = nullptr;       // status: the host's address ...
+    uint32_t *word_dev = nullptr;   // ... and the device's
 };
 static void status_block_release(StatusBlock *sb) {
     if (sb && sb->refs.fetch_sub(1) == 1) {
@@ -192,6 +196,7 @@ static void status_block_release(StatusBlock *sb) {
         cudaGetDevice(&prev);
         cudaSetDevice(sb->ordinal);
         cudaFree(sb->dev);
+        cudaFreeHost(sb->word);
         cudaSetDevice(prev);
         delete sb;
     }
@@ -289,6 +294,8 @@ struct mlxn_encoder {
     std::vector<std::pair<void *, size_t>> cap_retired;   // arenas outgrown during the capture: also the graph's
     StatusBlock *sb = nullptr;
     uint32_t *status_dev = nullptr;   // == sb->dev
+    uint32_t *status_word = nullptr;  // == sb->word_dev: what kernels are given
+    uint32_t *status_host = nullptr;  // == sb->word
     // Mat-vecs of the current concurrent group that have been encoded but not launched: the reference dispatches the
     // operations of a group concurrently; here up to 8 of them (same block type, same activation-row class) leave as
     // ONE kernel whose CTAs share the work of all of them.  Launched by the first thing that ends the group.
@@ -298,7 +305,6 @@ struct mlxn_encoder {
     bool pend_pair = false;
     bool pend_split = false;          // they are mat-vecs of the split kernel (qmv_split.cuh)
     bool grp_pend_only = false;       // every operation of the current group is in `pend` (none has been launched yet)
-    uint32_t *status_host = nullptr;  // pinned
 };
 
 // ------------------------------------------------------------------------------------------------
@@ -787,15 +793,21 @@ extern "C" int mlxn_encoder_create(mlxn_device *dev, mlxn_encoder **out) {
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming);
     if (err == cudaSuccess) err = cudaEventCreate(&e->ev_start);
     if (err == cudaSuccess) err = cudaEventCreate(&e->ev_end);
-    // status word, then (256 bytes in) the zero-initialised flag words the tensor-core mat-vec's CTAs hand work over with
+    // zero-initialised words that the blocks of a kernel hand work over with, and the status word
     if (err == cudaSuccess) err = cudaMalloc((void **)&e->status_dev, kStatusBlockBytes);
     if (err == cudaSuccess) err = cudaMemset(e->status_dev, 0, kStatusBlockBytes);
     if (err == cudaSuccess) {
         e->sb = new StatusBlock();
         e->sb->ordinal = dev->ordinal;
         e->sb->dev = e->status_dev;
+        err = cudaHostAlloc((void **)&e->sb->word, 4, cudaHostAllocMapped);
+        if (err == cudaSuccess) {
+            *e->sb->word = 0;
+            err = cudaHostGetDevicePointer((void **)&e->sb->word_dev, e->sb->word, 0);
+        }
+        e->status_host = e->sb->word;
+        e->status_word = e->sb->word_dev;
     }
-    if (err == cudaSuccess) err = cudaHostAlloc((void **)&e->status_host, 4, cudaHostAllocDefault);
     if (err != cudaSuccess) {
         for (int l = 0; l < kLanes; l++) {
             if (e->lanes[l]) cudaStreamDestroy(e->lanes[l]);
@@ -812,7 +824,6 @@ extern "C" int mlxn_encoder_create(mlxn_device *dev, mlxn_encoder **out) {
         delete e;
         return cuda_fail(err, "encoder creation");
     }
-    *e->status_host = 0;
     g_cmd_buf.fetch_add(1);
     *out = e;
     return MLXN_OK;
@@ -872,7 +883,6 @@ extern "C" void mlxn_encoder_destroy(mlxn_encoder *enc) {
     }
     for (auto &pr : enc->cap_retired) scratch_give(enc->ordinal, pr.first, pr.second);
     status_block_release(enc->sb);
-    cudaFreeHost(enc->status_host);
     cudaEventDestroy(enc->ev_start);
     cudaEventDestroy(enc->ev_end);
     cudaEventDestroy(enc->ev_fork);
@@ -1025,7 +1035,6 @@ extern "C" int mlxn_encoder_commit(mlxn_encoder *enc) {
             st->has_last = true;
         }
     }
-    CUDA_TRY(cudaMemcpyAsync(enc->status_host, enc->status_dev, 4, cudaMemcpyDeviceToHost, enc->lanes[0]), "status copy");
     CUDA_TRY(cudaEventRecord(enc->ev_end, enc->lanes[0]), "event record");
     enc->committed = true;
     return MLXN_OK;
@@ -1436,7 +1445,7 @@ extern "C" int mlxn_debug_wait_probe(mlxn_encoder *enc, uint32_t limit_us) {
     int rc = encoder_begin_work(enc);
     if (rc) return rc;
     if ((rc = encoder_join_lanes(enc))) return rc;
-    wait_probe_kernel<<<1, 32, 0, enc->lanes[0]>>>(enc->status_dev, (uint64_t)limit_us * 1000ull);
+    wait_probe_kernel<<<1, 32, 0, enc->lanes[0]>>>(enc->status_word, (uint64_t)limit_us * 1000ull);
     CUDA_TRY(cudaGetLastError(), "wait probe launch");
     g_launches.fetch_add(1);
     return MLXN_OK;
@@ -1492,7 +1501,7 @@ extern "C" int mlxn_peer_barrier(mlxn_encoder *enc, uint32_t rank, uint32_t worl
     if ((rc = encoder_join_lanes(enc))) return rc;   // everything encoded so far is ahead of the barrier
     PeerFlags table{};
     for (uint32_t r = 0; r < world; r++) table.p[r] = static_cast<uint32_t *>(flag_ptrs[r]);
-    peer_barrier_kernel<<<1, 32, 0, enc->lanes[0]>>>(rank, world, table, epoch, (uint64_t)limit_us * 1000ull, enc->status_dev);
+    peer_barrier_kernel<<<1, 32, 0, enc->lanes[0]>>>(rank, world, table, epoch, (uint64_t)limit_us * 1000ull, enc->status_word);
     CUDA_TRY(cudaGetLastError(), "peer barrier launch");
     g_launches.fetch_add(1);
     g_barrier.fetch_add(1);
@@ -1592,7 +1601,7 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
         a.top_k = 1;
         a.n_experts = 1;
         a.expert_stride = 0;
-        a.status = enc->status_dev;
+        a.status = enc->status_word;
         a.early_weights = weight->st->kernel_written ? 0u : 1u;
         return a;
     };
@@ -1711,7 +1720,7 @@ static int dispatch_mm(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
     a.top_k = 1;
     a.n_experts = 1;
     a.total_rows = p->m;
-    a.status = enc->status_dev;
+    a.status = enc->status_word;
     if (sh) {
         a.y_ld = sh->y_ld;
         a.y_col0 = sh->y_col0;
@@ -1862,7 +1871,7 @@ extern "C" int mlxn_quantized_matmul_mm_tensor_perm021(mlxn_encoder *enc, mlxn_r
     a.top_k = 1;
     a.n_experts = 1;
     a.total_rows = p->m;
-    a.status = enc->status_dev;
+    a.status = enc->status_word;
     const uint32_t nt = qmm_tc_pick_nt(p->m, p->n, p->k, dev->sm_count, false, false);
     uint8_t *scratch = nullptr;
     if ((rc = encoder_scratch(enc, qmm_tc_scratch_bytes(a, nt, false), &scratch))) return rc;
@@ -1948,7 +1957,7 @@ static int dispatch_id_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *de
     a.top_k = up ? 1 : p->top_k;   // (fused: every output row has its own input row)
     a.n_experts = p->n_experts;
     a.expert_stride = p->expert_stride;
-    a.status = enc->status_dev;
+    a.status = enc->status_word;
     // Few rows (decode): every (token, slot) row is one mat-vec of the register-level kernel, and the rows of this call,
     // and of the calls around it that do not depend on it (gate and up of one layer), leave as one launch.
     const int mode = opt_qmv();
@@ -2033,7 +2042,7 @@ static int dispatch_id_mm_stages(mlxn_encoder *enc, mlxn_registry *reg, mlxn_dev
     a.n_experts = p->n_experts;
     a.total_rows = p->n_tokens * p->top_k;
     a.expert_stride = p->expert_stride;
-    a.status = enc->status_dev;
+    a.status = enc->status_word;
     if (opt_qmm_tc() && qmm_tc_supported(a)) {
         const uint32_t nt = qmm_tc_pick_nt(p->n_tokens, p->n, p->k, dev->sm_count, true, false);
         uint8_t *scratch = nullptr;
@@ -2211,7 +2220,7 @@ extern "C" int mlxn_moe_ffn_layer(mlxn_encoder *enc, mlxn_registry *reg, mlxn_de
         a.n_experts = q.n_experts;
         a.total_rows = (uint32_t)pairs;
         a.expert_stride = q.expert_stride;
-        a.status = enc->status_dev;
+        a.status = enc->status_word;
         a.reuse = reuse;
         int launches = 0;
         CUDA_TRY(launch_qmm_tc((int)q.ggml_type, a, true, nt, tc, enc->stream, &launches), "mat-mat launch");
