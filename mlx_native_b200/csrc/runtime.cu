@@ -2165,9 +2165,9 @@ extern "C" int mlxn_moe_ffn_layer(mlxn_encoder *enc, mlxn_registry *reg, mlxn_de
         if ((rc = mlxn_quantized_matmul_id_ggml(enc, reg, dev, x, gate_w, ids, gate_out, &pg))) return rc;
         if ((rc = mlxn_quantized_matmul_id_ggml(enc, reg, dev, x, up_w, ids, up_out, &pu))) return rc;
         const int td = (int)p->down_type;
-        // (the down projection's rows are pairs: few tokens stay on the mat-vec route, with f32 operands, even where there are
-        //  more pairs than the routing threshold)
-        if (pairs <= 256 && (td == GT_Q4_0 || td == GT_Q8_0 || td == GT_Q6_K)) {
+        // (the down projection's rows are pairs: with more of them than the routing threshold it takes the grouped mat-mat, as in the
+        //  chain, although gate and up are mat-vecs; anything else would not be the chain bit for bit)
+        if (!id_routes_to_mm(&pd) && (td == GT_Q4_0 || td == GT_Q8_0 || td == GT_Q6_K)) {
             mlxn_qmm_id_params ps = pd;
             return mlxn_quantized_matmul_id_swiglu(enc, reg, dev, gate_out, up_out, down_w, ids, down_out, &ps);
         }

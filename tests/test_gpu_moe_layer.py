@@ -92,6 +92,27 @@ def test_layer_call_equals_the_chain(ctx, T, E, top_k, hidden, ffn, gname, dname
         assert launches <= 3
 
 
+# few tokens with more pairs than the routing threshold: gate and up are mat-vecs, the down projection is the grouped mat-mat, as in the
+# chain -- also where ffn is longer than the routed mat-vecs of many pairs take, and whatever kernel the mat-vecs are told to use
+@pytest.mark.parametrize("T,E,top_k,hidden,ffn,gname,dname,qmv", [
+    (5, 16, 8, 512, 256, "Q4_0", "Q6_K", "auto"), (24, 16, 4, 512, 256, "Q8_0", "Q8_0", "auto"), (32, 8, 8, 256, 512, "Q6_K", "Q4_0", "auto"),
+    (17, 4, 2, 256, 4096, "Q4_0", "Q8_0", "auto"), (24, 16, 4, 512, 256, "Q4_0", "Q8_0", "stream")])
+def test_few_tokens_many_pairs_equal_the_chain(ctx, T, E, top_k, hidden, ffn, gname, dname, qmv):
+    assert T <= mx.MM_ID_ROUTING_THRESHOLD < T * top_k
+    L = make_layer(E, hidden, ffn, gname, dname, seed=300 + T)
+    x = normal_acts(T, T, hidden)
+    ids = route(T, E, top_k, seed=T)
+    mx.set_option("qmv", qmv)
+    try:
+        g0, _, d0 = run_chain(ctx, L, x, ids, T, top_k, E, hidden, ffn)
+        g1, _, d1, _ = run_layer(ctx, L, x, ids, T, top_k, E, hidden, ffn)
+    finally:
+        mx.set_option("qmv", "auto")
+    assert mx.last_kernel_name() == "qmm_tc_id"
+    assert np.array_equal(g0.view(np.uint32), g1.view(np.uint32))
+    assert np.array_equal(d0.view(np.uint32), d1.view(np.uint32))
+
+
 def test_layer_call_against_the_oracle_and_bad_ids(ctx):
     T, E, top_k, hidden, ffn = 64, 8, 2, 256, 256
     L = make_layer(E, hidden, ffn, "Q4_0", "Q6_K", seed=77)
