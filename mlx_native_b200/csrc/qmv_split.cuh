@@ -741,7 +741,10 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             if (ranks > 1 && tid == 0) mbar_expect_tx(&recv_bar[buf], mp * R * 4u);
             return true;
         };
-        // the ranks' sums of chunk j, in rank order (a rank sends chunk j + 4 only when it has this one's j + 2: four buffers)
+        // The ranks' sums of chunk j, in rank order.  Four buffers are enough although other warps of this rank send and read on:
+        // chunk j + 4 comes here from a rank all of whose warps have finished j + 2; that takes rows of j + 2 sent by this rank,
+        // which its warps send only once every one of them has arrived on sync_bar for j + 2; and a warp does that after it has read
+        // chunk j here.
         auto finish = [&](uint32_t j, uint32_t d) {
             const uint32_t buf = j & 3u;
             if (!wait(recv_bar[buf], (j >> 2) & 1u, ST_WAIT_FULL_TIMEOUT)) return false;
@@ -1031,6 +1034,8 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
 
             // ---- the warps' partial sums go to shared memory; they are added one chunk later, and what the other ranks send is
             // waited for two chunks later, so that nobody stands still for the slowest warp or for the way between SMs ----
+            // (finish comes before this warp's arrivals for chunk i: four receive buffers rest on that, see there)
+            if (i >= 2 && ranks > 1 && !finish(i - 2, d2)) break;
             if (i >= 2 && !wait(sync_bar[2], i & 1u, ST_WAIT_EMPTY_TIMEOUT)) break;   // chunk i - 2 has been read out of the area
             const uint32_t part = red + (i & 1u) * (kSpWarps * mp * R * 4u);
 #pragma unroll
@@ -1048,7 +1053,6 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             __syncwarp();
             if (lane == 0) mbar_arrive(&sync_bar[i & 1u]);
             if (i >= 1 && !add(i - 1, d1)) break;
-            if (i >= 2 && ranks > 1 && !finish(i - 2, d2)) break;
             d2 = d1;
             d1 = this_at;
         }

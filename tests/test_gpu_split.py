@@ -22,6 +22,7 @@ def ctx():
 # (rows at any even address), of 64 (half a unit), or shorter than a slice
 @pytest.mark.parametrize("tname,n,k,m", [
     ("Q4_0", 1, 32, 1), ("Q4_0", 17, 96, 2), ("Q4_0", 15, 256, 3), ("Q4_0", 333, 2880, 5), ("Q4_0", 64, 4096, 8), ("Q4_0", 2500, 1056, 1),
+    ("Q4_0", 12000, 4128, 8),                                      # several chunks per cluster: every receive buffer used again
     ("Q8_0", 1, 32, 8), ("Q8_0", 31, 160, 1), ("Q8_0", 2873, 2880, 5), ("Q8_0", 48, 512, 4), ("Q8_0", 130, 12288, 8), ("Q8_0", 1030, 4128, 2),
     ("Q6_K", 1, 256, 1), ("Q6_K", 33, 768, 7), ("Q6_K", 70, 2048, 2), ("Q6_K", 19, 5120, 8), ("Q6_K", 1001, 2560, 1), ("Q6_K", 12, 14336, 3),
     ("Q4_K", 16, 256, 1), ("Q4_K", 65, 768, 6), ("Q4_K", 40, 3584, 4), ("Q4_K", 130, 1024, 9), ("Q4_K", 50, 2304, 33)])
