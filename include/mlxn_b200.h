@@ -370,6 +370,11 @@ int mlxn_set_option(const char *key, const char *value);
  * status word and returns normally.  The next commit_and_wait reports MLXN_COMMAND_BUFFER_ERROR; the encoder and
  * the device stay usable (src/encoder.rs:1867-1878 is the upstream path that surfaces a failed command buffer). */
 int mlxn_debug_wait_probe(mlxn_encoder *enc, uint32_t limit_us);
+/* The geometry that the split mat-vec kernel takes for a product: CTAs that share K and 16-row tiles of a chunk, both 0 where it does
+ * not take the product.  n_experts == 0: dense, n_tokens activation rows; `misaligned`: bytes by which the weights miss a
+ * 16-byte boundary.  Looks at sizes alone and needs no GPU. */
+int mlxn_debug_split_geometry(const mlxn_qmm_id_params *params, uint32_t misaligned, uint32_t sm_count, uint32_t *ranks,
+                              uint32_t *tiles);
 /* Name of the kernel variant the last operation on this thread launched (for tests and profiles). */
 const char *mlxn_last_kernel_name(void);
 

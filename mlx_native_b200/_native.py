@@ -125,6 +125,7 @@ SIGNATURES = {
     "mlxn_quantized_matmul_ggml_mm_noalloc": (i32, [vp, vp, vp, vp, C.POINTER(QmmParams)]),
     "mlxn_peer_barrier": (i32, [vp, u32, u32, C.POINTER(C.c_void_p), u32, u32]),
     "mlxn_set_option": (i32, [C.c_char_p, C.c_char_p]),
+    "mlxn_debug_split_geometry": (i32, [C.POINTER(QmmIdParams), u32, u32, C.POINTER(u32), C.POINTER(u32)]),
     "mlxn_debug_wait_probe": (i32, [vp, u32]),
     "mlxn_last_kernel_name": (C.c_char_p, []),
 }

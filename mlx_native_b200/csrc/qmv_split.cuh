@@ -1162,41 +1162,50 @@ static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, ui
     return cudaLaunchKernelEx(&cfg, kernel, bt, maps);
 }
 
-// Chooses the cluster size and the tiles of a chunk.
-template <int T, bool ALN, int MPC>
-static cudaError_t sp_choose(SpBatch &bt, const SpMaps &maps, uint64_t tiles, uint64_t entries, uint32_t max_units, bool routed, int sm_count, cudaStream_t st) {
-    constexpr int NS = MPC > 4 ? 2 : 1;
-    uint32_t best_c = 0, best_tr = 0;
+// Chooses the cluster size and the tiles of a chunk; ranks == 0: no geometry fits.  qmv_split_supported asks the same function, so that
+// no call is promised this kernel and then refused.
+struct SpPick {
+    uint32_t ranks, tr;
+};
+template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool routed, uint64_t tiles, uint32_t max_units, int sm_count) {
+    const uint32_t sets = mp > 4 ? 2u : 1u;
+    SpPick pick{0, 0};
     double best = 1e30;
     int force_c = 0, force_tr = 0;
     if (const char *e = exp_env("MLXN_SP_C")) force_c = atoi(e);
     if (const char *e = exp_env("MLXN_SP_TR")) force_tr = atoi(e);
     for (uint32_t c = 1; c <= (routed ? 1u : 8u); c *= 2) {
         const uint32_t slice = ((max_units + c - 1) / c + 3) / 4 * 4;
-        if (c > 1 && slice * (c - 1) >= max_units) continue;   // a rank without work
-        for (uint32_t tr = 1; tr <= (uint32_t)sp_tiles(NS); tr++) {
+        // a rank without work: only where nothing smaller fits (K = 10304 with eight rows: seven slices of 24 units do, four of 44 do not)
+        if (c > 1 && slice * (c - 1) >= max_units && pick.ranks) continue;
+        for (uint32_t tr = 1; tr <= (uint32_t)sp_tiles((int)sets); tr++) {
             if ((force_c && !routed && (int)c != force_c) || (force_tr && (int)tr != force_tr)) continue;
-            const size_t stage = (size_t)tr * 16 * sp_pitch<T>(ALN), tail = sp_tail<T>(ALN, c, tr, bt.mp, (slice + 1) & ~1u, nullptr);
+            const size_t stage = (size_t)tr * 16 * sp_pitch<T>(aln), tail = sp_tail<T>(aln, c, tr, mp, (slice + 1) & ~1u, nullptr);
             if (tail + 2 * stage + 128 > kSpSmem) continue;
             const double slots = (double)((kSpSmem - 128 - tail) / stage);
             const double ncl = (double)(2 * sm_count / (int)c), chunks = ceil(ceil((double)tiles / tr) / ncl);
             // Measured (12288 x 4096 and 4096 x 4096, all types): a chunk takes 1.9 us of waits and sums whatever its size, plus
             // 0.23 us per tile and unit of a warp (Q6_K 0.3; two sets of columns 1.5 times that, and there four ranks wait for
             // one another for 4.5 us a chunk).
-            const double unit = (T == GT_Q6_K ? 0.3 : 0.23) * (NS == 2 ? 1.5 : 1.0);
+            const double unit = (T == GT_Q6_K ? 0.3 : 0.23) * (sets == 2 ? 1.5 : 1.0);
             // One row: splitting it takes 0.27 us per unit of a warp and CTA.
-            const double cost = (bt.packed ? 1.0 : 0.3 + 0.27 * ceil(slice / 8.0)) + chunks * ((NS == 2 && c == 4 ? 4.5 : 1.9) + tr * unit * ceil(slice / 8.0)) + (c > 1 ? 0.3 : 0.0) + (slots < 3 ? 0.3 : 0.0);
+            const double cost = (packed ? 1.0 : 0.3 + 0.27 * ceil(slice / 8.0)) + chunks * ((sets == 2 && c == 4 ? 4.5 : 1.9) + tr * unit * ceil(slice / 8.0)) + (c > 1 ? 0.3 : 0.0) + (slots < 3 ? 0.3 : 0.0);
             if (cost < best) {
                 best = cost;
-                best_c = c;
-                best_tr = tr;
+                pick = {c, tr};
             }
         }
     }
-    if (!best_c) return cudaErrorInvalidConfiguration;
-    for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].slice = ((bt.op[i].units + best_c - 1) / best_c + 3) / 4 * 4;
-    const uint32_t xunits = (((max_units + best_c - 1) / best_c + 3) / 4 * 4 + 1) & ~1u;
-    return sp_launch<T, ALN, MPC>(bt, maps, best_c, best_tr, entries, xunits, sm_count, st);
+    return pick;
+}
+
+template <int T, bool ALN, int MPC>
+static cudaError_t sp_choose(SpBatch &bt, const SpMaps &maps, uint64_t tiles, uint64_t entries, uint32_t max_units, bool routed, int sm_count, cudaStream_t st) {
+    const SpPick pick = sp_pick<T>(ALN, bt.mp, bt.packed != 0, routed, tiles, max_units, sm_count);
+    if (!pick.ranks) return cudaErrorInvalidConfiguration;
+    for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].slice = ((bt.op[i].units + pick.ranks - 1) / pick.ranks + 3) / 4 * 4;
+    const uint32_t xunits = (((max_units + pick.ranks - 1) / pick.ranks + 3) / 4 * 4 + 1) & ~1u;
+    return sp_launch<T, ALN, MPC>(bt, maps, pick.ranks, pick.tr, entries, xunits, sm_count, st);
 }
 
 // Scratch bytes of a mat-vec's packed activations.

@@ -34,7 +34,7 @@ bool qmv_stream_available(int ggml_type, const QmvArgs &a, int sm_count);
 constexpr size_t kMvBatchMax = 16;   // mat-vecs one launch of the register-level kernel carries (kMwMaxProbs)
 bool qmv_mma_pair_mode(int ggml_type, const QmvArgs &a);
 cudaError_t launch_qmv_mma(int ggml_type, const QmvArgs *ops, int nops, int sm_count, int ctas_per_sm, int tpw, cudaStream_t st);
-bool qmv_split_supported(int ggml_type, const QmvArgs &a);
+bool qmv_split_supported(int ggml_type, const QmvArgs &a, int sm_count);
 bool qmv_split_aligned(int ggml_type, const QmvArgs &a);
 constexpr size_t kMvSplitMax = 8;    // mat-vecs one launch of the split kernel carries (kSpMaxOps)
 size_t qmv_split_scratch_bytes(const QmvArgs *ops, int nops);
@@ -1626,7 +1626,7 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
         else pays = t == GT_Q4_K;
         if (!enc->pend.empty() && enc->pend_split && enc->pend_type == t && !enc->pend[0].ids && enc->pend_mp == mv_row_class(p->m) && aligned) pays = true;
         pays = pays || mode == 5;
-        if (pays && qmv_split_supported(t, a) && (p->m <= 8 || !sh))
+        if (pays && qmv_split_supported(t, a, dev->sm_count) && (p->m <= 8 || !sh))
             return batch_mv(enc, t, a, p->m <= 8 ? mv_row_class(p->m) : 16u, !aligned, {{input, false}, {weight, false}, {output, true}});
     }
     // A mat-vec for the register-level kernel is not launched at once: it waits for the operations that follow, and
@@ -1961,7 +1961,7 @@ static int dispatch_id_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *de
     // Few rows (decode): every (token, slot) row is one mat-vec of the register-level kernel, and the rows of this call,
     // and of the calls around it that do not depend on it (gate and up of one layer), leave as one launch.
     const int mode = opt_qmv();
-    if ((mode == 3 || mode == 5) && qmv_split_supported(t, a))
+    if ((mode == 3 || mode == 5) && qmv_split_supported(t, a, dev->sm_count))
         return batch_mv(enc, t, a, 1u, !qmv_split_aligned(t, a), {{input, false}, {up, false}, {weight, false}, {ids, false}, {output, true}});
     if ((mode == 3 || mode == 4) && rows <= kMvBatchMax && qmv_mma_supported_routed(t, a)) {
         const bool batch = g_opt_mv_batch.load() != 0;

@@ -25,7 +25,10 @@ def ctx():
     ("Q4_0", 12000, 4128, 8),                                      # several chunks per cluster: every receive buffer used again
     ("Q8_0", 1, 32, 8), ("Q8_0", 31, 160, 1), ("Q8_0", 2873, 2880, 5), ("Q8_0", 48, 512, 4), ("Q8_0", 130, 12288, 8), ("Q8_0", 1030, 4128, 2),
     ("Q6_K", 1, 256, 1), ("Q6_K", 33, 768, 7), ("Q6_K", 70, 2048, 2), ("Q6_K", 19, 5120, 8), ("Q6_K", 1001, 2560, 1), ("Q6_K", 12, 14336, 3),
-    ("Q4_K", 16, 256, 1), ("Q4_K", 65, 768, 6), ("Q4_K", 40, 3584, 4), ("Q4_K", 130, 1024, 9), ("Q4_K", 50, 2304, 33)])
+    ("Q4_K", 16, 256, 1), ("Q4_K", 65, 768, 6), ("Q4_K", 40, 3584, 4), ("Q4_K", 130, 1024, 9), ("Q4_K", 50, 2304, 33),
+    # eight columns where four slices of K do not fit and eight leave the last rank without work
+    ("Q4_0", 40, 10304, 5), ("Q4_0", 21, 12544, 8), ("Q8_0", 33, 12352, 8), ("Q8_0", 18, 10752, 5), ("Q6_K", 20, 12544, 8), ("Q6_K", 37, 10496, 5),
+    ("Q4_K", 24, 10752, 8), ("Q4_K", 24, 10496, 40), ("Q4_K", 17, 12544, 5)])
 def test_dense(ctx, tname, n, k, m):
     gtype, otype = ALL[tname]
     wq = normal_weights(n + k + m, n, k, otype)
