@@ -66,7 +66,7 @@ bool qmv_split_supported(int ggml_type, const QmvArgs &a, int sm_count) {
 size_t qmv_split_scratch_bytes(const QmvArgs *ops, int nops) {
     size_t n = 0;
     for (int i = 0; i < nops; i++)
-        if (!ops[i].ids && ops[i].m > 1) n += sp_pack_bytes<GT_Q6_K>(ops[i].m, ops[i].k);   // (the type with the most bias sums)
+        if (!ops[i].ids && ops[i].m > 1) n += sp_pack_bytes<GT_Q4_K>(ops[i].m, ops[i].k);   // (a type with sums)
     return n;
 }
 

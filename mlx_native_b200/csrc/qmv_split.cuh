@@ -6,8 +6,7 @@
 //  * The activations of a CTA stay in shared memory for all its weight rows: f16 hi + lo halves (scaled by a power of two per
 //    row, so that both stay in range), in the order of the B registers of mma.sync.m16n8k16.  One row is split by every CTA
 //    itself (2 us, less than another launch), several rows by qmv_pack_kernel, and arrive by bulk copies.  The loop over the
-//    weights only unpacks codes: the raw 4/5/6/8-bit codes as f16 subnormals (exact integers n 2^-24), so products are exact and
-//    sums are f32.
+//    weights only unpacks codes into signed integers, as normal f16 numbers, so products are exact and sums are f32.
 //  * The 8 columns of an MMA are (activation row, hi | lo): one multiply serves up to four rows (NS = 2 sets: eight rows).
 //  * A warp works on up to four 16-row tiles at a time: one tile at a time leaves the pipes idle between dependent steps (Q4_0,
 //    75776 x 4096: 2.7 TB/s against 5.0).
@@ -42,13 +41,14 @@ constexpr int kSpMaxOps = 8;                        // mat-vecs one launch carri
 constexpr int kSpMaxSlots = 8;
 constexpr int kSpMaxPairs = 256;                    // (token, slot) pairs of a routed launch
 
-// SU: units (64 K values) of a stage, a multiple of the warps.  NG: scale groups of a unit.  OFF: code bias.
+// SU: units (64 K values) of a stage, a multiple of the warps.  NG: sub-blocks of a unit that have an offset of their own, and
+// with it the sum of their activations (Q4_K, Q5_K).
 template <int T> struct SpTraits;
-template <> struct SpTraits<GT_Q4_0> { static constexpr int B256 = 144, SU = 16, NG = 2, OFF = 8; };
-template <> struct SpTraits<GT_Q8_0> { static constexpr int B256 = 272, SU = 8, NG = 2, OFF = 128; };
-template <> struct SpTraits<GT_Q4_K> { static constexpr int B256 = 144, SU = 16, NG = 2, OFF = 1; };
-template <> struct SpTraits<GT_Q5_K> { static constexpr int B256 = 176, SU = 16, NG = 2, OFF = 1; };
-template <> struct SpTraits<GT_Q6_K> { static constexpr int B256 = 210, SU = 8, NG = 4, OFF = 32; };
+template <> struct SpTraits<GT_Q4_0> { static constexpr int B256 = 144, SU = 16, NG = 0; };
+template <> struct SpTraits<GT_Q8_0> { static constexpr int B256 = 272, SU = 8, NG = 0; };
+template <> struct SpTraits<GT_Q4_K> { static constexpr int B256 = 144, SU = 16, NG = 2; };
+template <> struct SpTraits<GT_Q5_K> { static constexpr int B256 = 176, SU = 16, NG = 2; };
+template <> struct SpTraits<GT_Q6_K> { static constexpr int B256 = 210, SU = 8, NG = 0; };
 
 // Bytes of shared memory per row of a stage: an odd multiple of 16 (32-bit reads of eight rows hit distinct banks).
 template <int T> __host__ __device__ constexpr uint32_t sp_pitch(bool aln) {
@@ -71,7 +71,7 @@ struct SpOp {
     uint32_t y_ld, y_col0, n_peer;
     float *y_peer[kMaxPeers];
     uint64_t expert_stride;
-    // packed activations (see qmv_pack_kernel): per row pk_units x 256 bytes of B registers, pk_units x NG bias sums, one scale
+    // packed activations (see qmv_pack_kernel): per row pk_units x 256 bytes of B registers, pk_units x NG sums, one scale
     const uint8_t *xp;
     const float *xsum, *xinv;
     uint32_t pk_units;
@@ -172,16 +172,43 @@ __device__ __forceinline__ void st_async(uint32_t a, float v, uint32_t bar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a), "r"(__float_as_uint(v)), "r"(bar)
                  : "memory");
 }
-// Power of two that brings amax into [2^13, 2^14), and its inverse; 1 for an all-zero or non-finite run.
+// Power of two that brings amax into [2^13, 2^14), and its inverse; 1 for an all-zero run.  (An infinite one: the factor of the
+// largest numbers; both are normal numbers for every amax, the smallest come out below 2^13.)
 __device__ __forceinline__ void pow2(float amax, float &s, float &inv) {
     s = inv = 1.f;
-    if (amax > 0.f && amax < 3.0e38f) {
+    if (amax > 0.f) {
         int e = 13 + 127 - (int)((__float_as_uint(amax) >> 23) & 0xffu);
-        e = max(-100, min(100, e));
+        e = max(-114, min(126, e));
         s = __uint_as_float((uint32_t)(e + 127) << 23);
         inv = __uint_as_float((uint32_t)(127 - e) << 23);
     }
 }
+// a and b as f16 hi + lo: 22 bits of the largest, no error above 2^-39 of it in any other.  (An infinity is all in hi.)
+__device__ __forceinline__ void split(float a, float b, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 w = __half22float2(h);
+    const __half2 l = __floats2half2_rn(fabsf(w.x) < INFINITY ? a - w.x : 0.f, fabsf(w.y) < INFINITY ? b - w.y : 0.f);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+// Codes to signed integers.  A code n in the low bits of a half with exponent field 0x64 reads 1024 + n, one four bits further up
+// 1024 + 16 n; the bias goes off exactly.  (Codes that stay subnormals, n 2^-24, save this operation, but the tensor core aligns
+// products by their exponents before it adds them, and a subnormal's leading zeros are then bits lost: Q4_0 had errors of 5e-7 on
+// normal activations and 1e-5 with outliers, against 64 bits.)
+__device__ __forceinline__ uint32_t less(uint32_t v, uint32_t bias) {
+    uint32_t r;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(bias));
+    return r;
+}
+__device__ __forceinline__ uint32_t lo4(uint32_t v) { return less((v & 0x000F000Fu) | 0x64006400u, 0x64086408u); }   // n - 8
+__device__ __forceinline__ uint32_t hi4(uint32_t v) {                                                                 // (1024 + 16 n) / 16 - 72
+    uint32_t r;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"((v & 0x00F000F0u) | 0x64006400u), "r"(0x2C002C00u), "r"(0xD480D480u));
+    return r;
+}
+// bytes 0, 2 and bytes 1, 3 of a word
+__device__ __forceinline__ uint32_t bytes02(uint32_t v, uint32_t bias) { return less(__byte_perm(v, 0x64646464u, 0x4240), bias); }
+__device__ __forceinline__ uint32_t bytes13(uint32_t v, uint32_t bias) { return less(__byte_perm(v, 0x64646464u, 0x4341), bias); }
 }  // namespace sp
 
 // Where in its unit the four values lie that quad lane t multiplies in MMA q, as two pairs of consecutive elements.  Q4_0 and
@@ -213,10 +240,10 @@ template <int T, bool ALN> __device__ __forceinline__ void sp_pairs(uint32_t u, 
 
 // One unit (64 K values) of a stage against NT tiles.  a0 / a1: shared address of rows g and g + 8 of tile 0 at the unit's
 // first byte (Q4_K, Q5_K, Q6_K: of its super-block), lead-in included; tiles are 16 PITCH bytes apart.  bf: the B registers
-// [set][MMA][2]; cc: per set and scale group what the bias (Q4_K, Q5_K: the minimum) owes; tab: the warp's scale table.
+// [set][MMA][2]; cc: per set and sub-block the sum of the activations (Q4_K, Q5_K); tab: the warp's scale table.
 template <int T, bool ALN, int NT, int NS, bool ONE, int TM>
 __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, uint32_t t, uint32_t g, uint32_t tab, bool half,
-                                        const uint32_t (&bf)[NS][4][2], const float (&cc)[NS][SpTraits<T>::NG], float (&acc)[TM][NS][4]) {
+                                        const uint32_t (&bf)[NS][4][2], [[maybe_unused]] const float (&cc)[NS][2], float (&acc)[TM][NS][4]) {
     constexpr uint32_t TS = 16u * sp_pitch<T>(ALN);
     if constexpr (T == GT_Q4_0 || T == GT_Q8_0) {
         constexpr bool Q8 = T == GT_Q8_0;
@@ -271,21 +298,21 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                 }
             }
             uint32_t a[4][4];
-            if constexpr (Q8) {   // codes + 128 as f16 subnormals: bytes 0, 2 and bytes 1, 3 of a word into halves
+            if constexpr (Q8) {
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const uint32_t x0 = w[q][0] ^ 0x80808080u, x1 = w[q][1] ^ 0x80808080u;
-                    a[q][0] = __byte_perm(x0, 0u, 0x4240); a[q][1] = __byte_perm(x1, 0u, 0x4240);
-                    a[q][2] = __byte_perm(x0, 0u, 0x4341); a[q][3] = __byte_perm(x1, 0u, 0x4341);
+                    a[q][0] = sp::bytes02(x0, 0x64806480u); a[q][1] = sp::bytes02(x1, 0x64806480u);
+                    a[q][2] = sp::bytes13(x0, 0x64806480u); a[q][3] = sp::bytes13(x1, 0x64806480u);
                 }
-            } else {              // low nibbles: elements 0..15; high nibbles (x 16, the activations carry 1 / 16): 16..31
+            } else {              // low nibbles: elements 0..15; high nibbles: 16..31
 #pragma unroll
                 for (int b = 0; b < 2; b++) {
                     const uint32_t x0 = w[2 * b][0], x1 = w[2 * b][1], y0 = x0 >> 8, y1 = x1 >> 8;
-                    a[2 * b][0] = x0 & 0x000F000Fu; a[2 * b][1] = x1 & 0x000F000Fu;
-                    a[2 * b][2] = y0 & 0x000F000Fu; a[2 * b][3] = y1 & 0x000F000Fu;
-                    a[2 * b + 1][0] = x0 & 0x00F000F0u; a[2 * b + 1][1] = x1 & 0x00F000F0u;
-                    a[2 * b + 1][2] = y0 & 0x00F000F0u; a[2 * b + 1][3] = y1 & 0x00F000F0u;
+                    a[2 * b][0] = sp::lo4(x0); a[2 * b][1] = sp::lo4(x1);
+                    a[2 * b][2] = sp::lo4(y0); a[2 * b][3] = sp::lo4(y1);
+                    a[2 * b + 1][0] = sp::hi4(x0); a[2 * b + 1][1] = sp::hi4(x1);
+                    a[2 * b + 1][2] = sp::hi4(y0); a[2 * b + 1][3] = sp::hi4(y1);
                 }
             }
             constexpr int j = decltype(J)::value;
@@ -296,9 +323,9 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                 sp::mma(r1, a[2][0], a[2][1], a[2][2], a[2][3], bf[s][2][0], bf[s][2][1], 0.f, 0.f, 0.f, 0.f);
                 sp::mma(r0, a[1][0], a[1][1], a[1][2], a[1][3], bf[s][1][0], bf[s][1][1], r0[0], r0[1], r0[2], r0[3]);
                 sp::mma(r1, a[3][0], a[3][1], a[3][2], a[3][3], bf[s][3][0], bf[s][3][1], r1[0], r1[1], r1[2], r1[3]);
-                acc[j][s][0] = fmaf(d1[0], r1[0] + cc[s][1], fmaf(d0[0], r0[0] + cc[s][0], acc[j][s][0]));
+                acc[j][s][0] = fmaf(d1[0], r1[0], fmaf(d0[0], r0[0], acc[j][s][0]));
                 acc[j][s][1] = fmaf(d1[0], r1[1], fmaf(d0[0], r0[1], acc[j][s][1]));
-                acc[j][s][2] = fmaf(d1[1], r1[2] + cc[s][1], fmaf(d0[1], r0[2] + cc[s][0], acc[j][s][2]));
+                acc[j][s][2] = fmaf(d1[1], r1[2], fmaf(d0[1], r0[2], acc[j][s][2]));
                 acc[j][s][3] = fmaf(d1[1], r1[3], fmaf(d0[1], r0[3], acc[j][s][3]));
             }
         });
@@ -312,7 +339,7 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
             uint32_t x[2][2];   // [first / second 16 elements][row g, g + 8]
             x[0][0] = sp::ld32i<o>(q0); x[1][0] = sp::ld32i<o + 16>(q0);
             x[0][1] = sp::ld32i<o>(q1); x[1][1] = sp::ld32i<o + 16>(q1);
-            uint32_t p0[4], p1[4];   // d sc, d sc', dmin m, dmin m' of rows g and g + 8
+            uint32_t p0[4], p1[4];   // scales and offsets (sp_table_row) of rows g and g + 8
             sp::ld128i<j * 256u>(tr, p0);
             sp::ld128i<j * 256u + 128u>(tr, p1);
             uint32_t a[4][4];
@@ -326,8 +353,8 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                     for (int h = 0; h < 2; h++) {
                         const uint32_t lo = (x[e][h] & 0x0F0F0F0Fu) | ((f[e][h] & 0x01010101u) << 4);
                         const uint32_t hi = ((x[e][h] >> 4) & 0x0F0F0F0Fu) | ((f[e][h] & 0x02020202u) << 3);
-                        a[e][h] = __byte_perm(lo, 0u, 0x4240); a[e][h + 2] = __byte_perm(lo, 0u, 0x4341);
-                        a[e + 2][h] = __byte_perm(hi, 0u, 0x4240); a[e + 2][h + 2] = __byte_perm(hi, 0u, 0x4341);
+                        a[e][h] = sp::bytes02(lo, 0x64106410u); a[e][h + 2] = sp::bytes13(lo, 0x64106410u);
+                        a[e + 2][h] = sp::bytes02(hi, 0x64106410u); a[e + 2][h + 2] = sp::bytes13(hi, 0x64106410u);
                     }
             } else {
 #pragma unroll
@@ -335,8 +362,8 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         const uint32_t y = x[e][h] >> 8;
-                        a[e][h] = x[e][h] & 0x000F000Fu; a[e][h + 2] = y & 0x000F000Fu;
-                        a[e + 2][h] = x[e][h] & 0x00F000F0u; a[e + 2][h + 2] = y & 0x00F000F0u;
+                        a[e][h] = sp::lo4(x[e][h]); a[e][h + 2] = sp::lo4(y);
+                        a[e + 2][h] = sp::hi4(x[e][h]); a[e + 2][h + 2] = sp::hi4(y);
                     }
             }
 #pragma unroll
@@ -387,16 +414,16 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                 sp::ld128i<j * 256u + 128u>(tr, p1);
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const uint32_t x0 = __byte_perm(qv[0][q], 0u, 0x4240), x2 = __byte_perm(qv[0][q], 0u, 0x4341);
-                    const uint32_t x1 = __byte_perm(qv[1][q], 0u, 0x4240), x3 = __byte_perm(qv[1][q], 0u, 0x4341);
+                    const uint32_t x0 = sp::bytes02(qv[0][q], 0x64206420u), x2 = sp::bytes13(qv[0][q], 0x64206420u);
+                    const uint32_t x1 = sp::bytes02(qv[1][q], 0x64206420u), x3 = sp::bytes13(qv[1][q], 0x64206420u);
                     const float pa = __uint_as_float(p0[q]), pb = __uint_as_float(p1[q]);
 #pragma unroll
                     for (int s = 0; s < NS; s++) {
                         float r[4];
                         sp::mma(r, x0, x1, x2, x3, bf[s][q][0], bf[s][q][1], 0.f, 0.f, 0.f, 0.f);
-                        acc[j][s][0] = fmaf(pa, r[0] + cc[s][q], acc[j][s][0]);
+                        acc[j][s][0] = fmaf(pa, r[0], acc[j][s][0]);
                         acc[j][s][1] = fmaf(pa, r[1], acc[j][s][1]);
-                        acc[j][s][2] = fmaf(pb, r[2] + cc[s][q], acc[j][s][2]);
+                        acc[j][s][2] = fmaf(pb, r[2], acc[j][s][2]);
                         acc[j][s][3] = fmaf(pb, r[3], acc[j][s][3]);
                     }
                 }
@@ -411,8 +438,9 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
     }
 }
 
-// Scale table of one unit for one row: d * scale of the unit's groups (Q6_K: four), or d sc, d sc', dmin m, dmin m' of its
-// two sub-blocks (Q4_K, Q5_K; 6-bit fields as in src/gguf/mod.rs:440-452).  rb: shared address of the row's super-block.
+// Scale table of one unit for one row: d * scale of the unit's groups (Q6_K: four), or the scales d sc and the offsets C d sc - dmin m
+// of its two sub-blocks (Q4_K, Q5_K: the codes are taken less C = 8 or 16, the middle of their range, so that the offset is small
+// where scale and minimum belong together; 6-bit fields as in src/gguf/mod.rs:440-452).  rb: shared address of the row's super-block.
 template <int T> __device__ __forceinline__ void sp_table_row(uint32_t dst, uint32_t rb, uint32_t u) {
     if constexpr (T == GT_Q6_K) {
         const uint32_t s = rb + 192 + 8 * ((u >> 1) & 1u) + (u & 1u);
@@ -434,8 +462,27 @@ template <int T> __device__ __forceinline__ void sp_table_row(uint32_t dst, uint
             m0 = ((a >> 4) & 15u) | (((hi >> 6) & 3u) << 4);
             m1 = ((a >> 12) & 15u) | (((hi >> 14) & 3u) << 4);
         }
-        sp::st128(dst, d * (float)c0, d * (float)c1, dmin * (float)m0, dmin * (float)m1);
+        constexpr float C = T == GT_Q5_K ? 16.f : 8.f;
+        const float e0 = d * (float)c0, e1 = d * (float)c1;   // (17 bits: exact, as the products with the minima)
+        sp::st128(dst, e0, e1, fmaf(C, e0, -(dmin * (float)m0)), fmaf(C, e1, -(dmin * (float)m1)));
     }
+}
+
+// One product of a Q4_K or Q5_K row in f32, value by value: for results that are no numbers.
+template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const float *x, uint32_t k) {
+    float acc = 0.f;
+    for (uint32_t b = 0; b < k / 256; b++, w += BlockTraits<T>::BYTES, x += 256)
+        for (uint32_t j = 0; j < 8; j++) {
+            uint32_t sc, mn;
+            q4k_scale_min(j, w + 4, sc, mn);
+            const float e = __fmul_rn(half_bits_to_float(ld_u16(w)), (float)sc), m = __fmul_rn(half_bits_to_float(ld_u16(w + 2)), (float)mn);
+            for (uint32_t l = 0; l < 32; l++) {
+                uint32_t q = (w[(T == GT_Q5_K ? 48 : 16) + 32 * (j >> 1) + l] >> (4 * (j & 1u))) & 15u;
+                if (T == GT_Q5_K) q |= ((w[16 + l] >> j) & 1u) << 4;
+                acc = fmaf(__fsub_rn(__fmul_rn(e, (float)q), m), x[32 * j + l], acc);
+            }
+        }
+    return acc;
 }
 
 // A chunk of work: `nt` consecutive tiles of op `op` for entry `ent`, from the op's tile `tile` on.  Chunks are dealt out in runs:
@@ -456,13 +503,12 @@ __device__ __forceinline__ SpChunk sp_chunk(const SpBatch &b, uint32_t i) {
     return c;
 }
 
-// Packs activation rows into B register order for the kernel below: f16 hi + lo halves under one power of two per row, per scale
-// group what the codes' bias owes, and the inverse scale.  One block per row.  Several rows (or row groups: Q4_K has no other form
+// Packs activation rows into B register order for the kernel below: f16 hi + lo halves under one power of two per row, the sums of the
+// sub-blocks that have offsets, and the inverse scale.  One block per row.  Several rows (or row groups: Q4_K has no other form
 // for many rows) are packed once instead of by every CTA, where eight rows cost more time than the weights of a 12288 x 4096 matrix.
 template <int T, bool ALN>
 __global__ void __launch_bounds__(256) qmv_pack_kernel(const __grid_constant__ SpBatch bt) {
     constexpr int NG = SpTraits<T>::NG;
-    constexpr float kOff = -(float)SpTraits<T>::OFF / 16777216.0f;
     __shared__ float s_am[8];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, q = (tid >> 2) & 3u, tt = tid & 3u;
     uint32_t op = 0;   // (ops that share another's activations have no rows of their own here)
@@ -513,23 +559,23 @@ __global__ void __launch_bounds__(256) qmv_pack_kernel(const __grid_constant__ S
     for (int o = 4; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
     float s, inv;
     sp::pow2(am, s, inv);
-    if (tid == 0) xinv[row] = inv * 16777216.0f;
-    // codes that stay in the high nibble of their byte are 16 times too large: their activations / 16
-    const float f = (T == GT_Q4_0 && (q & 1u)) || (T == GT_Q4_K && q >= 2) ? s * 0.0625f : s;
+    if (tid == 0) xinv[row] = inv;
     auto put = [&](uint32_t u, const float (&z)[4]) {
-        float sum = (z[0] + z[1]) + (z[2] + z[3]);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        if constexpr (NG == 2) sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-        const __half2 h02 = __floats2half2_rn(z[0] * f, z[2] * f), h13 = __floats2half2_rn(z[1] * f, z[3] * f);
-        const float2 f02 = __half22float2(h02), f13 = __half22float2(h13);
-        const __half2 l02 = __floats2half2_rn(fmaf(z[0], f, -f02.x), fmaf(z[2], f, -f02.y));
-        const __half2 l13 = __floats2half2_rn(fmaf(z[1], f, -f13.x), fmaf(z[3], f, -f13.y));
+        const float c[4] = {z[0] * s, z[1] * s, z[2] * s, z[3] * s};
+        float sum = 0.f;
+        if constexpr (NG != 0) {
+            sum = (c[0] + c[1]) + (c[2] + c[3]);
+#pragma unroll
+            for (int o = 1; o <= 4; o *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        }
+        uint2 hi, lo;
+        sp::split(c[0], c[2], hi.x, lo.x);
+        sp::split(c[1], c[3], hi.y, lo.y);
         if (u >= pk_units) return;
         uint2 *d = reinterpret_cast<uint2 *>(xp + (row * pk_units + u) * 256u + (q >> 1) * 128u + tt * 32u + (q & 1u) * 8u);
-        d[0] = make_uint2(*reinterpret_cast<const uint32_t *>(&h02), *reinterpret_cast<const uint32_t *>(&h13));
-        d[2] = make_uint2(*reinterpret_cast<const uint32_t *>(&l02), *reinterpret_cast<const uint32_t *>(&l13));
-        if ((tid & (NG == 4 ? 3u : 7u)) == 0) xsum[(row * pk_units + u) * NG + (NG == 4 ? q : q >> 1)] = kOff * (sum * s);
+        d[0] = hi;
+        d[2] = lo;
+        if (NG != 0 && (tid & 7u) == 0) xsum[(row * pk_units + u) * NG + (q >> 1)] = sum;
     };
 #pragma unroll
     for (int p = 0; p < HELD; p++) {
@@ -551,13 +597,12 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
     constexpr bool TABLE = T == GT_Q4_K || T == GT_Q5_K || T == GT_Q6_K;
     constexpr uint32_t PITCH = sp_pitch<T>(ALN), TILE = 16 * PITCH;
     constexpr uint32_t UB = T == GT_Q8_0 ? 68u : 36u;               // bytes of a unit (Q4_0, Q8_0)
-    constexpr float kOff = -(float)K::OFF / 16777216.0f;
 
     extern __shared__ __align__(128) uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 127u) & ~127u;      // (the same in every CTA of a cluster)
     __shared__ __align__(8) uint64_t full[kSpMaxSlots], empty[kSpMaxSlots], sync_bar[3], recv_bar[4], x_bar, c_bar;
     __shared__ float s_inv[kSpWarps][8];                            // inverse activation scales of a warp's share of K
-    __shared__ volatile uint32_t abort_flag;
+    __shared__ volatile uint32_t abort_flag, s_again;
     __shared__ uint32_t s_nent;
     __shared__ uint32_t s_id[kSpMaxPairs];                          // routed: expert of every pair
     __shared__ uint16_t s_ord[kSpMaxPairs], s_ent[kSpMaxPairs + 1]; // pairs by expert; entry e = pairs s_ord[s_ent[e] ..]
@@ -570,7 +615,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
     const uint32_t mp = bt.mp, tr = bt.tr, R = 16u * tr, STAGE = tr * TILE;
 
     if (tid == 0) {
-        abort_flag = 0;
+        abort_flag = s_again = 0;
         for (uint32_t s = 0; s < bt.nslots; s++) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], kSpWarps);
@@ -715,6 +760,22 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             const uint32_t pair = bt.ids ? (uint32_t)s_ord[e0 + col] : e0 + col;
             const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
             if (bt.ids && s_id[pair] >= bt.n_experts) v = 0.f;   // an id that names no expert
+            if (NG != 0 && v != v) s_again = 1;
+            P.y[o] = v;
+            for (uint32_t pr = 0; pr < P.n_peer; pr++) P.y_peer[pr][o] = v;
+        };
+        [[maybe_unused]] auto again = [&](uint32_t at, uint32_t col, uint32_t row) {
+            const SpChunk d = sp_chunk(bt, at);
+            const SpOp &P = bt.op[d.op];
+            const uint32_t grow = d.tile * 16u + row, e0 = bt.ids ? (uint32_t)s_ent[d.ent] : d.ent * mp;
+            const uint32_t cnt = bt.ids ? s_ent[d.ent + 1] - e0 : min(mp, P.m - e0);
+            if (col >= cnt || row >= d.nt * 16u || grow >= P.n) return;
+            const uint32_t pair = bt.ids ? (uint32_t)s_ord[e0 + col] : e0 + col;
+            const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
+            float v = P.y[o];
+            if (v == v) return;
+            v = sp_again<T>(P.w + (bt.ids ? s_id[pair] * P.expert_stride : 0ull) + (uint64_t)grow * P.row_bytes,
+                            P.x + (size_t)(bt.ids ? pair / P.x_div : pair) * P.k, P.k);
             P.y[o] = v;
             for (uint32_t pr = 0; pr < P.n_peer; pr++) P.y_peer[pr][o] = v;
         };
@@ -798,7 +859,8 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                     if (lane < cnt && un) {
                         const uint8_t *px = P.xp + ((size_t)(e0 + lane) * P.pk_units + u0) * 256u;
                         bulk_g2s_a(xf + lane * xs, px, xb, &x_bar);
-                        bulk_g2s_a(ccb + lane * cs, reinterpret_cast<const uint8_t *>(P.xsum) + ((size_t)(e0 + lane) * P.pk_units + u0) * (NG * 4u), cb, &x_bar);
+                        if constexpr (NG != 0)
+                            bulk_g2s_a(ccb + lane * cs, reinterpret_cast<const uint8_t *>(P.xsum) + ((size_t)(e0 + lane) * P.pk_units + u0) * (NG * 4u), cb, &x_bar);
                     }
                 }
                 if (lane < cnt) s_inv[warp][lane] = __ldcg(P.xinv + e0 + lane);
@@ -815,13 +877,27 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 sp_pairs<T, ALN>(warp, q, tt, p0, p1);
                 const uint32_t kb = (T == GT_Q6_K ? 256u * ((u0 + warp) >> 2) : 64u * (u0 + warp)) + 512u * hf;
                 const uint32_t mine = un > warp ? (un - warp + 7) / 8 : 0u;          // the warp's units
-                const float f0 = (T == GT_Q4_0 && (q & 1u)) || (T == GT_Q4_K && q >= 2) ? 0.0625f : 1.f;   // codes left in the high nibble are 16 times too large
                 const uint32_t d0 = xf + ((warp + 8 * hf) * 2 + (q >> 1)) * 128u + tt * 32u + (q & 1u) * 8u;
-                const uint32_t c0 = ccb + ((warp + 8 * hf) * NG + (NG == 4 ? q : q >> 1)) * 4u;
-                const bool head = (lane & (NG == 4 ? 3u : 7u)) == 0;
+                // a pass's values: the sums of the sub-blocks, and the halves at `d`
+                auto write = [&](const float (&z)[4], float s, uint32_t p, uint32_t row, bool mine_too) {
+                    const float c[4] = {z[0] * s, z[1] * s, z[2] * s, z[3] * s};
+                    [[maybe_unused]] float sum = 0.f;
+                    if constexpr (NG != 0) {
+                        sum = (c[0] + c[1]) + (c[2] + c[3]);
+#pragma unroll
+                        for (int o = 1; o <= 4; o *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                    }
+                    uint32_t hi[2], lo[2];
+                    sp::split(c[0], c[2], hi[0], lo[0]);
+                    sp::split(c[1], c[3], hi[1], lo[1]);
+                    if (2 * p + hf >= mine || !mine_too) return;
+                    const uint32_t d = d0 + p * 4096u + row * xs;
+                    sp::st64(d, hi[0], hi[1]);
+                    sp::st64(d + 16, lo[0], lo[1]);
+                    if (NG != 0 && (lane & 7u) == 0) sp::st32(ccb + ((warp + 8 * hf) * NG + (q >> 1)) * 4u + p * (64u * NG) + row * cs, __float_as_uint(sum));
+                };
                 __syncwarp();
                 if constexpr (MPC == 1) {
-                    constexpr uint32_t r = 0;
                     const uint32_t row = e0;
                     const float *x = P.x + (size_t)row * P.k + kb, *y = P.x2 ? P.x2 + (size_t)row * P.k + kb : nullptr;
                     auto load = [&](uint32_t p, float (&v)[4]) {
@@ -855,31 +931,14 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                     for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
                     float s, inv;
                     sp::pow2(am, s, inv);
-                    if (lane == 0) s_inv[warp][r] = inv * 16777216.0f;
-                    const float f = s * f0;
-                    auto put = [&](uint32_t p, const float (&z)[4]) {
-                        float sum = (z[0] + z[1]) + (z[2] + z[3]);
-                        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-                        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-                        if constexpr (NG == 2) sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-                        const __half2 h02 = __floats2half2_rn(z[0] * f, z[2] * f), h13 = __floats2half2_rn(z[1] * f, z[3] * f);
-                        const float2 f02 = __half22float2(h02), f13 = __half22float2(h13);
-                        const __half2 l02 = __floats2half2_rn(fmaf(z[0], f, -f02.x), fmaf(z[2], f, -f02.y));
-                        const __half2 l13 = __floats2half2_rn(fmaf(z[1], f, -f13.x), fmaf(z[3], f, -f13.y));
-                        if (2 * p + hf < mine) {
-                            const uint32_t d = d0 + p * 4096u;
-                            sp::st64(d, *reinterpret_cast<const uint32_t *>(&h02), *reinterpret_cast<const uint32_t *>(&h13));
-                            sp::st64(d + 16, *reinterpret_cast<const uint32_t *>(&l02), *reinterpret_cast<const uint32_t *>(&l13));
-                            if (head) sp::st32(c0 + p * (64u * NG), __float_as_uint(kOff * (sum * s)));
-                        }
-                    };
+                    if (lane == 0) s_inv[warp][0] = inv;
 #pragma unroll
                     for (int p = 0; p < HELD; p++)
-                        if (2u * p < mine) put(p, v[p]);
+                        if (2u * p < mine) write(v[p], s, p, 0, true);
                     for (uint32_t p = HELD; 2 * p < mine; p++) {
                         float z[4];
                         load(p, z);
-                        put(p, z);
+                        write(z, s, p, 0, true);
                     }
                 } else {
                 // Four passes are in flight at a time: of one row, or of two or four rows where a row has fewer.
@@ -909,23 +968,6 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                         }
                     };
                     auto peak = [](const float (&v)[4]) { return fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))); };
-                    auto put = [&](uint32_t r, uint32_t p, float s, const float (&z)[4]) {
-                        const float f = s * f0;
-                        float sum = (z[0] + z[1]) + (z[2] + z[3]);
-                        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-                        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-                        if constexpr (NG == 2) sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-                        const __half2 h02 = __floats2half2_rn(z[0] * f, z[2] * f), h13 = __floats2half2_rn(z[1] * f, z[3] * f);
-                        const float2 f02 = __half22float2(h02), f13 = __half22float2(h13);
-                        const __half2 l02 = __floats2half2_rn(fmaf(z[0], f, -f02.x), fmaf(z[2], f, -f02.y));
-                        const __half2 l13 = __floats2half2_rn(fmaf(z[1], f, -f13.x), fmaf(z[3], f, -f13.y));
-                        if (2 * p + hf < mine && r < cnt) {
-                            const uint32_t d = d0 + p * 4096u + r * xs;
-                            sp::st64(d, *reinterpret_cast<const uint32_t *>(&h02), *reinterpret_cast<const uint32_t *>(&h13));
-                            sp::st64(d + 16, *reinterpret_cast<const uint32_t *>(&l02), *reinterpret_cast<const uint32_t *>(&l13));
-                            if (head) sp::st32(c0 + p * (64u * NG) + r * cs, __float_as_uint(kOff * (sum * s)));
-                        }
-                    };
                     float v[4][4], am[4], s[4];
 #pragma unroll
                     for (int j = 0; j < 4; j++) load(x[j], y[j], j & ((1u << sh) - 1u), v[j]);
@@ -956,14 +998,14 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                     for (int j = 0; j < 4; j++) {   // one power of two brings the row's largest value into [2^13, 2^14)
                         float inv;
                         sp::pow2(am[j], s[j], inv);
-                        if (lane == 0 && rb + (j >> sh) < cnt) s_inv[warp][rb + (j >> sh)] = inv * 16777216.0f;
+                        if (lane == 0 && rb + (j >> sh) < cnt) s_inv[warp][rb + (j >> sh)] = inv;
                     }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) put(rb + (j >> sh), j & ((1u << sh) - 1u), s[j], v[j]);
+                    for (int j = 0; j < 4; j++) write(v[j], s[j], j & ((1u << sh) - 1u), rb + (j >> sh), rb + (j >> sh) < cnt);
                     for (uint32_t p = 4; p < passes; p++) {
                         float z[4];
                         load(x[0], y[0], p, z);
-                        put(rb, p, s[0], z);
+                        write(z, s[0], p, rb, true);
                     }
                 }
                 }
@@ -993,11 +1035,12 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                     const uint32_t ul = warp + 8u * i, uu = us + ul;
                     if (uu >= un) break;
                     uint32_t bf[NS][4][2];
-                    float cc[NS][NG];
+                    float cc[NS][2];
 #pragma unroll
                     for (int s = 0; s < NS; s++) {
                         uint32_t v[4];
-                        const uint32_t xa = xlane + uu * 256u + s * 4u * xs, ca = clane + uu * NG * 4u + s * 4u * cs;
+                        const uint32_t xa = xlane + uu * 256u + s * 4u * xs;
+                        [[maybe_unused]] const uint32_t ca = clane + uu * NG * 4u + s * 4u * cs;
                         sp::ld128i<0>(xa, v);
                         bf[s][0][0] = v[0]; bf[s][0][1] = v[1]; bf[s][1][0] = v[2]; bf[s][1][1] = v[3];
                         sp::ld128i<128>(xa, v);
@@ -1059,6 +1102,19 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         if (ok && i >= 1) ok = add(i - 1, d1);
         if (ok && ranks > 1 && i >= 2) ok = finish(i - 2, d2);
         if (ok && ranks > 1 && i >= 1) ok = finish(i - 1, d1);
+        // An infinite activation times codes and offset may cancel where the weight has a sign: results that are no numbers are formed
+        // again, weight by weight, each by the thread that stored it.  (Not on the way: the call costs the loop registers.)
+        if constexpr (NG != 0)
+            if (ok && s_again) {
+                const uint32_t rows = ranks == 1 ? R : share;
+                for (uint32_t at = first, left = run; at < chunks; at++) {
+                    for (uint32_t q = tid; q < mp * rows; q += 256) again(at, q / rows, (ranks == 1 ? 0u : rank * share) + q % rows);
+                    if (--left == 0) {
+                        left = run;
+                        at += skip;
+                    }
+                }
+            }
     }
     if (abort_flag)   // let copies in flight land before the CTA's shared memory is released
         for (int i = 0; i < 200; i++) __nanosleep(5000);
@@ -1081,7 +1137,7 @@ constexpr size_t kSpSmem = 110 * 1024;
 template <int T> inline size_t sp_tail(bool aln, uint32_t ranks, uint32_t tr, uint32_t mp, uint32_t xunits, SpBatch *b) {
     (void)aln;
     const size_t r = 16u * tr;
-    const size_t xf = (size_t)xunits * mp * 256, cc = (((size_t)xunits * SpTraits<T>::NG * 4 + 16) * mp + 127) / 128 * 128;
+    const size_t xf = (size_t)xunits * mp * 256, cc = SpTraits<T>::NG ? (((size_t)xunits * SpTraits<T>::NG * 4 + 16) * mp + 127) / 128 * 128 : 0;
     const size_t tab = SpTraits<T>::B256 == 272 || T == GT_Q4_0 ? 0 : (size_t)kSpWarps * r * 16;
     const size_t red = (size_t)2 * kSpWarps * mp * r * 4, recv = ranks > 1 ? (size_t)4 * mp * r * 4 : 0;
     if (b) {

@@ -94,3 +94,75 @@ def test_batch_of_different_shapes(ctx):
     for (xb, wb, yb), w, x, (n, k, m) in zip(bufs, ws, xs, shapes):
         y_ref, ad = orc.qmatmul(otype, w, x, n, k)
         assert norm_err(yb.as_slice(np.float32).reshape(m, n), y_ref, ad) <= MV_TOL
+
+
+# Every product of a code and an f16 half is exact, a half pair holds 22 bits, and the f32 sums of a result have at most a few dozen
+# terms one after another: relative 2-norm errors of 1 to 1.5e-7 (2^-23 = 1.2e-7), also where a few activations are 300 times larger than the
+# others.  (Codes multiplied as subnormals miss this bound by 2 (Q8_0) to 20 times.)
+ERR_TOL = 5e-7
+
+
+def relative_error(y, w, x):
+    ref = x.astype(np.float64) @ w.T
+    return np.linalg.norm(y - ref) / np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("rows", [1, 4, 8])
+@pytest.mark.parametrize("tname,n,k", [("Q4_0", 700, 2880), ("Q4_0", 700, 4096), ("Q8_0", 700, 2880), ("Q8_0", 700, 4096), ("Q6_K", 700, 2816),
+                                       ("Q6_K", 700, 4096), ("Q4_K", 700, 4096)])
+def test_error_against_64_bits(ctx, tname, n, k, rows):
+    gtype, otype = ALL[tname]
+    wq = normal_weights(n + k, n, k, otype)
+    x = normal_acts(n + rows, rows, k)
+    x[:, ::97] *= 300
+    assert relative_error(ctx.matmul(gtype, wq, x, n, k), orc.dequantize(otype, wq).reshape(n, k).astype(np.float64), x) <= ERR_TOL
+
+
+# activation rows that f16 halves could lose: infinities, no numbers, magnitudes at either end of f32
+def extreme_rows(k, top=1e36):
+    x = normal_acts(k, 7, k)
+    x[0, 5] = np.inf
+    x[1, k - 3] = -np.inf
+    x[2, [1, 9, k - 20]] = [np.inf, -np.inf, 3.0]
+    x[3, 17] = np.nan
+    x[4] *= top
+    x[5] *= 1e-35
+    x[6, 30] = 4e4
+    return x
+
+
+def assert_same_numbers(y, y_ref, ad):
+    assert np.array_equal(np.isnan(y), np.isnan(y_ref))
+    inf = np.isinf(y_ref)
+    assert np.array_equal(y[inf], y_ref[inf])
+    ok = np.isfinite(y_ref)
+    assert np.all(np.abs(y[ok].astype(np.float64) - y_ref[ok]) <= MV_TOL * ad[ok])
+
+
+@pytest.mark.parametrize("rows", [1, 2, 7])
+@pytest.mark.parametrize("tname,n,k", [("Q4_0", 33, 288), ("Q4_0", 40, 2048), ("Q8_0", 33, 288), ("Q8_0", 40, 2048), ("Q6_K", 33, 768),
+                                       ("Q6_K", 40, 2048), ("Q4_K", 33, 768), ("Q4_K", 600, 4096)])
+def test_infinities_and_extreme_magnitudes(ctx, tname, n, k, rows):
+    gtype, otype = ALL[tname]
+    wq = normal_weights(n + k, n, k, otype)
+    x = extreme_rows(k)
+    y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8)
+    for at in range(0, 7, rows):
+        assert_same_numbers(ctx.matmul(gtype, wq, x[at:at + rows], n, k), y_ref[at:at + rows], ad[at:at + rows])
+
+
+@pytest.mark.parametrize("tname,n,k", [("Q4_0", 33, 288), ("Q8_0", 40, 2048), ("Q6_K", 33, 768), ("Q4_K", 33, 768), ("Q5_K", 18, 512)])
+def test_routed_infinities_and_extreme_magnitudes(ctx, tname, n, k):
+    T, top_k, E = 21, 2, 4
+    rng = np.random.default_rng(n)
+    if tname == "Q5_K":
+        gtype, otype = mx.GgmlType.Q5_K, orc.Q5_K
+        w = random_q5k_blocks(rng, E * n * (k // 256))
+    else:
+        gtype, otype = ALL[tname]
+        w = normal_weights(E + n, E * n, k, otype)
+    x = np.concatenate([extreme_rows(k, 1e30 if tname == "Q5_K" else 1e36)] * 3)   # (random Q5_K blocks hold large weights)
+    ids = np.stack([rng.permutation(E)[:top_k] for _ in range(T)]).astype(np.uint32).reshape(-1)
+    y, _ = ctx.matmul_id(gtype, w, w.size // E, x, ids, top_k, n, k, E)
+    y_ref, ad = orc.qmatmul_id(otype, w, w.size // E, x, ids, top_k, n, k, E, nthreads=8)
+    assert_same_numbers(y, y_ref, ad)
