@@ -1263,6 +1263,31 @@ static cudaError_t launch_mw_t(const QmvArgs *ops, int nops, uint32_t mmax, int 
     return launch_mw_p<T, false>(ops, nops, mmax, sm_count, ctas_per_sm, tpw, st);
 }
 
+static int mw_tpw(const QmvArgs *ops, int nops, int sm_count) {
+    // measured: the largest row group (the activation split is paid once per group) that still gives at least every
+    // other CTA slot an item; 16-row groups when even 32-row groups do not
+    for (int cand = 4; cand >= 2; cand >>= 1) {
+        uint64_t items = 0;
+        for (int i = 0; i < nops; i++) items += (ops[i].n + 16u * cand - 1) / (16u * cand);
+        if (items >= (uint64_t)sm_count) return cand;
+    }
+    return 1;
+}
+
+// Share of the CTA slots (two per SM, as many passes as the launch needs) that have an item in a launch of these mat-vecs.  What is
+// missing from 1 is time in which part of the chip waits for the rest: the kernel's time is the number of passes times an item's.
+double qmv_mma_fill(int ggml_type, const QmvArgs *ops, int nops, int sm_count) {
+    uint32_t mmax = 1;
+    for (int i = 0; i < nops; i++) mmax = ops[i].m > mmax ? ops[i].m : mmax;
+    int tpw = mw_tpw(ops, nops, sm_count);
+    if (ggml_type == GT_Q4_K || ggml_type == GT_Q5_K || ggml_type == GT_Q6_K) tpw = mmax > 4 ? 4 : mmax > 2 && tpw < 2 ? 2 : tpw;   // (launch_mw_m)
+    else if (mmax > 4) tpw = 2;
+    uint64_t items = 0;
+    for (int i = 0; i < nops; i++) items += (ops[i].n + 16u * tpw - 1) / (16u * tpw);
+    const uint64_t slots = 2ull * sm_count;
+    return (double)items / (double)((items + slots - 1) / slots * slots);
+}
+
 // Launches `nops` (1..8) mat-vecs of one block type as ONE kernel.  The caller guarantees that no operation reads or
 // writes what another one writes.  `ctas_per_sm` (1 or 2) and `tpw` (0: chosen from the row count; 1, 2, 4) are tuning
 // knobs of the caller.
@@ -1281,19 +1306,7 @@ cudaError_t launch_qmv_mma(int ggml_type, const QmvArgs *ops, int nops, int sm_c
         // expert-parallel layer bit-identical to the single-GPU one.
         tpw = 4;
     }
-    if (tpw <= 0) {
-        // measured: the largest row group (the activation split is paid once per group) that still gives at least every
-        // other CTA slot an item; 16-row groups when even 32-row groups do not
-        tpw = 1;
-        for (int cand = 4; cand >= 2; cand >>= 1) {
-            uint64_t items = 0;
-            for (int i = 0; i < nops; i++) items += (ops[i].n + 16u * cand - 1) / (16u * cand);
-            if (items >= (uint64_t)sm_count) {
-                tpw = cand;
-                break;
-            }
-        }
-    }
+    if (tpw <= 0) tpw = mw_tpw(ops, nops, sm_count);
     switch (ggml_type) {
     case GT_Q4_0: return launch_mw_t<GT_Q4_0>(ops, nops, mmax, sm_count, ctas_per_sm, tpw, st);
     case GT_Q8_0: return launch_mw_t<GT_Q8_0>(ops, nops, mmax, sm_count, ctas_per_sm, tpw, st);

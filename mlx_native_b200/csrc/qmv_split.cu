@@ -36,7 +36,7 @@ bool qmv_split_fits(int ggml_type, const QmvArgs &a, int sm_count, SpPick *pick)
     // the activations are read as pairs of floats
     if (((uintptr_t)a.x & 7u) || ((uintptr_t)a.x2 & 7u) || ((uintptr_t)a.w & 1u)) return false;
     const bool aligned = qmv_split_aligned(ggml_type, a);
-    if (kq && !aligned) return false;
+    if (kq && (!aligned || a.x2)) return false;
     if ((uint64_t)(a.k / ggml_qk(ggml_type)) * ggml_block_bytes(ggml_type) >= (1ull << 31)) return false;
     uint32_t mp = a.m <= 1 ? 1u : a.m <= 2 ? 2u : a.m <= 4 ? 4u : 8u, ranks = 8;
     if (a.ids) {
@@ -60,6 +60,70 @@ bool qmv_split_fits(int ggml_type, const QmvArgs &a, int sm_count, SpPick *pick)
 bool qmv_split_supported(int ggml_type, const QmvArgs &a, int sm_count) {
     SpPick pick;
     return qmv_split_fits(ggml_type, a, sm_count, &pick) && encode_tiled_fn() != nullptr;
+}
+
+// Whether mat-vecs that the register-level kernel takes too (dense, aligned, one block type and row class) leave by this kernel,
+// where nothing else runs meanwhile.  It
+// starts 1 to 3 us later and has the higher rate, and its time grows evenly, where the other one's is a number of passes over the chip:
+// what decides is how full those passes are (`fill`, qmv_mma_fill) and how much there is to read.  Graph replay of dependent
+// launches, us with the register-level kernel (one mat-vec of three or four rows: the tensor-memory kernel) / with this one:
+//   one row    4096 values wide   6144 rows (fill 0.65)   10240 (0.54)   12288 (0.65)   14336 (0.76)   16384 (0.86)   24576 (0.65)
+//     Q4_0                        7.6 / 8.6               12.4 / 11.5    12.7 / 11.7    12.7 / 13.1    13.3 / 13.4    23.9 / 19.5
+//     Q8_0                        8.5 / 8.4               14.2 / 11.1    13.7 / 11.9    13.7 / 14.3    14.7 / 14.9    25.1 / 20.6
+//     Q6_K                        11.1 / 11.2             17.9 / 15.8    18.0 / 16.1    17.8 / 18.7    18.0 / 19.1    32.7 / 27.1
+//     Q4_K                        8.1 / 10.0              14.2 / 14.1    14.2 / 14.2                   14.2 / 16.3    26.1 / 24.1
+//   two rows
+//     Q4_0                        9.1 / 10.7              13.7 / 13.3    13.7 / 13.7    13.7 / 18.4    14.4 / 18.1    25.5 / 22.6
+//     Q8_0                        9.7 / 11.0              15.3 / 14.4    15.2 / 15.1    15.2 / 18.9    15.4 / 19.1    28.1 / 25.5
+//   four rows  a mat-vec: 3072 rows 8.6 / 8.8, 4096 9.9 / 9.0, 12288 17.4 / 16.5 (Q4_0); 5120 x 5120 12.7 / 13.5, 4096 x 8192 13.7 / 15.5;
+//              several: 4096 + 1024 + 1024 rows (0.65) 11.7 / 10.7, twice 6144 (0.65) 15.8 / 16.6, twice 12288 (0.65) 30.1 / 25.7, twice 8192
+//              (0.86) 16.3 / 18.9.  Of different widths, 12288 x 2048 + 12288 x 4096: 19.9 / 22.4, one row of Q6_K 20.4 / 22.5
+//   Q4_K, three and four rows: 4096 (0.43) 12.2 / 10.8, 12288 (0.65) 17.3 / 18.8, 24576 (0.65) 32.6 / 28.0, 8192 (0.86) 13.7 / 17.4,
+//              5120 x 2048 (0.54) 7.9 / 8.9, 24576 x 2048 (0.65) 18.0 / 17.8
+//   Q4_K, five and more: 1024 (0.22) 20.0 / 8.4, 8192 (0.43) 27.6 / 23.8, 10240 (0.54) 28.5 / 28.2, 12288 (0.65) 28.5 / 32.9, 16384 (0.86)
+//              28.6 / 41.7.  In groups of eight, one launch against one per group: 16 rows 10240 56.7 / 51.5, 12288 56.2 / 61.1; a last group
+//              of one row costs this kernel as much as eight: 9 rows 4096 (0.22) 34.4 / 25.0, 6144 (0.32) 28.6 / 35.2.
+bool qmv_split_pays(int ggml_type, const QmvArgs *ops, int nops, double fill) {
+    uint64_t values = 0;
+    uint32_t m = 0, kmin = 0xFFFFFFFFu, kmax = 0;
+    for (int i = 0; i < nops; i++) {
+        values += (uint64_t)ops[i].n * ops[i].k;
+        m = ops[i].m > m ? ops[i].m : m;
+        kmin = ops[i].k < kmin ? ops[i].k : kmin;
+        kmax = ops[i].k > kmax ? ops[i].k : kmax;
+    }
+    constexpr uint64_t M = 1u << 20;
+    const bool q4k = ggml_type == GT_Q4_K;
+    if (kmin != kmax) return false;   // (the other kernel deals out work by K stages, and its passes are fuller than `fill` says)
+    if (m <= 2) return fill <= 0.7 && values >= (q4k || (ggml_type == GT_Q4_0 && m == 2) ? 72 * M : 32 * M);
+    if (q4k && m <= 4) return kmax >= 4096 && values >= 14 * M && (fill <= 0.6 || (fill <= 0.7 && values >= 72 * M));
+    if (q4k) return fill <= 0.6 && (m <= 8 || fill <= 0.25 || (m + 7) / 8 * 16 <= 3 * m);
+    if (m > 4) return false;
+    const bool alone = nops == 1 && ops[0].n_peer == 0;
+    const bool four_bits = ggml_type == GT_Q4_0 && values >= 32 * M && values < 72 * M;
+    return values >= 14 * M && kmax <= (ggml_type == GT_Q6_K ? 6144u : 4096u) && (alone || fill <= (four_bits ? 0.6 : 0.7));
+}
+
+// Whether an expert-routed call leaves by this kernel; `mma`: the register-level kernel takes it too (up to 16 pairs).  Between those two
+// the matrix decides and not the number of pairs, since a pair's sum must not depend on the pairs that travel with it.  Graph replay of
+// dependent launches, 128 experts (two and four pairs: 8 and 16), us with the other kernel / with this one:
+//   register-level (a pass over the weights for every pair, 16 pairs a launch), gate and up of a layer, n < k:
+//             768 x 2048, pairs: 2           4             8             16            1536 x 2048, 8   16            512 x 1024, 8   16
+//     Q4_0                       7.5 / 8.1   9.1 / 9.0     12.2 / 11.4   25.2 / 16.2   19.3 / 16.5      39.9 / 26.9   8.6 / 8.9       11.7 / 10.0
+//     Q8_0                       7.6 / 8.4   9.3 / 8.9     12.2 / 11.8   26.0 / 17.3   19.9 / 17.8      41.4 / 29.0   8.6 / 9.0       11.7 / 10.7
+//     (the others lose more with few pairs, 1536 x 2048 four: Q4_K 10.2 / 12.4, Q5_K 11.8 / 16.7, Q6_K 12.2 / 13.7, and gain nothing with eight,
+//     768 x 2048: 12.7 / 12.8, 14.2 / 17.2, 14.2 / 14.5; their 16 pairs, 26.0 / 18.8 for Q4_K, pay for that)
+//   register-level, down projection, n >= k: 2048 x 768 eight pairs 7.7 / 10.2 (Q4_0), 8.7 / 11.0 (Q8_0), 16 pairs 14.4 / 14.1, 14.8 / 14.8;
+//     2048 x 1536 eight 10.2 / 14.6, 16 18.6 / 22.2
+//   streaming (a pass for every pair as well), Q6_K rows off 16-byte boundaries: 2048 x 768 two pairs 6.6 / 9.9, eight 12.1 / 12.5, 16
+//     20.6 / 20.2, 256 267 / 109; 2048 x 1536, whose copies cost this kernel more, 16 pairs of 16 experts 21.4 / 26.8, 64 of 128 72.6 / 74.2, 64
+//     of 64 72.1 / 63.4, 64 of 8 68.9 / 40.2; 2048 x 3584 64 of 64 141 / 149, 128 of 128 273 / 269, 256 of 128 540 / 392
+//   streaming or plain, the other types, 32 pairs: 2048 x 1536 Q4_0 41 / 31, 768 x 2048 Q4_K 110 / 31.
+bool qmv_split_pays_routed(int ggml_type, const QmvArgs &a, bool mma) {
+    if (mma) return (ggml_type == GT_Q4_0 || ggml_type == GT_Q8_0) && a.n < a.k && (uint64_t)a.n * a.k >= 5u << 18;
+    if (ggml_type == GT_Q6_K && !qmv_split_aligned(ggml_type, a))
+        return a.k <= 1024 ? a.nprob > 8 : a.nprob >= 64 && a.nprob >= (a.k > 2560 ? 2ull : 1ull) * a.n_experts;
+    return true;
 }
 
 // Scratch for the packed activations of a launch (one activation row, and routed rows, are converted inside the kernel).

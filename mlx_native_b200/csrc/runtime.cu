@@ -36,6 +36,9 @@ bool qmv_mma_pair_mode(int ggml_type, const QmvArgs &a);
 cudaError_t launch_qmv_mma(int ggml_type, const QmvArgs *ops, int nops, int sm_count, int ctas_per_sm, int tpw, cudaStream_t st);
 bool qmv_split_supported(int ggml_type, const QmvArgs &a, int sm_count);
 bool qmv_split_aligned(int ggml_type, const QmvArgs &a);
+bool qmv_split_pays(int ggml_type, const QmvArgs *ops, int nops, double fill);
+bool qmv_split_pays_routed(int ggml_type, const QmvArgs &a, bool mma);
+double qmv_mma_fill(int ggml_type, const QmvArgs *ops, int nops, int sm_count);
 constexpr size_t kMvSplitMax = 8;    // mat-vecs one launch of the split kernel carries (kSpMaxOps)
 size_t qmv_split_scratch_bytes(const QmvArgs *ops, int nops);
 cudaError_t launch_qmv_split(int ggml_type, const QmvArgs *ops, int nops, int sm_count, uint8_t *scratch, int *launches, cudaStream_t st);
@@ -531,7 +534,7 @@ extern "C" uint64_t mlxn_buffer_byte_offset(const mlxn_buffer *buf) { return buf
 extern "C" void *mlxn_buffer_device_ptr(const mlxn_buffer *buf) { return buf->dev(); }
 
 // wait for whatever touched the storage last (device work or an upload still reading the shadow)
-static int encoder_flush_pending(struct mlxn_encoder *e);
+static int encoder_flush_pending(struct mlxn_encoder *e, bool group_ends = false);
 static int storage_quiesce(Storage *s) {
     if (s->pend_enc) {   // a mat-vec that uses the storage is still waiting to be launched
         struct mlxn_encoder *pe = s->pend_enc;
@@ -897,7 +900,6 @@ extern "C" void mlxn_encoder_destroy(mlxn_encoder *enc) {
 }
 
 static int encoder_join_lanes(mlxn_encoder *e);
-static int encoder_flush_pending(mlxn_encoder *e);
 // Lane 0, after it has been made to wait for the other lane: work the caller enqueues on the returned stream runs
 // behind everything encoded so far.
 extern "C" void *mlxn_encoder_stream(mlxn_encoder *enc) {
@@ -911,7 +913,7 @@ extern "C" void *mlxn_encoder_stream(mlxn_encoder *enc) {
 // operation starts a new group on lane 0.
 static uint32_t mv_row_class(uint32_t m) { return m <= 1 ? 1u : m <= 2 ? 2u : m <= 4 ? 4u : 8u; }
 static int encoder_scratch_on(mlxn_encoder *e, int lane, size_t bytes, uint8_t **out);
-static int encoder_flush_pending(mlxn_encoder *e) {
+static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
     if (e->pend.empty()) return MLXN_OK;
     cudaSetDevice(e->ordinal);
     cudaStream_t st = e->lanes[e->pend_lane];
@@ -919,6 +921,7 @@ static int encoder_flush_pending(mlxn_encoder *e) {
     int launches = 1, rc = MLXN_OK;
     // A mat-vec that ended up alone (the next operation depended on it, or nothing followed) gains nothing from the
     // batched kernel's shared work list; with "auto" it takes the kernel that is fastest for a lone call of its kind.
+    const bool whole_group = group_ends && e->grp_pend_only;
     e->grp_pend_only = false;   // (what is launched here stays part of the group until the lanes are joined)
     // barrier words of a launch whose mat-vecs depend on one another: one set per lane (launches of a lane are ordered)
     for (QmvArgs &a : e->pend) a.grid_bar = e->status_dev + 1024 + 32 * e->pend_lane;
@@ -928,7 +931,17 @@ static int encoder_flush_pending(mlxn_encoder *e) {
     const bool q6_one_row_small = e->pend_type == GT_Q6_K && a0.m == 1 && (uint64_t)a0.n * a0.k < (1ull << 23);
     const bool lone_other = e->pend.size() == 1 && opt_qmv() == 3 && a0.n_peer == 0 && !a0.ids && e->pend_type != GT_Q4_K &&
                             (q6_one_row_small || a0.m > 2);
-    if (e->pend_split) {
+    // The batch is complete.  With "auto", dense mat-vecs that the split kernel takes as well leave by the one that suits the whole of
+    // it; not where the group has other operations, which run meanwhile and fill what the register-level kernel leaves idle (32 independent
+    // mat-vecs of both 8- and 6-bit types: 0.345 ms where these count as a batch like others, 0.328 so).
+    bool split = e->pend_split;
+    if (!split && whole_group && opt_qmv() == 3 && !a0.ids && !e->pend_pair && e->pend.size() <= kMvSplitMax) {
+        split = qmv_split_pays(e->pend_type, e->pend.data(), (int)e->pend.size(),
+                               qmv_mma_fill(e->pend_type, e->pend.data(), (int)e->pend.size(), e->dev->sm_count));
+        for (const QmvArgs &a : e->pend)
+            split = split && !a.after_earlier && qmv_split_supported(e->pend_type, a, e->dev->sm_count);
+    }
+    if (split) {
         uint8_t *scratch = nullptr;
         const size_t need = qmv_split_scratch_bytes(e->pend.data(), (int)e->pend.size());
         if (!need || (rc = encoder_scratch_on(e, e->pend_lane, need, &scratch)) == MLXN_OK)
@@ -973,7 +986,7 @@ static int encoder_flush_pending(mlxn_encoder *e) {
 
 static int encoder_join_lanes(mlxn_encoder *e) {
     {
-        const int frc = encoder_flush_pending(e);
+        const int frc = encoder_flush_pending(e, true);
         if (frc) return frc;
     }
     for (int l = 1; l < kLanes; l++) {
@@ -1605,28 +1618,18 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
         a.early_weights = weight->st->kernel_written ? 0u : 1u;
         return a;
     };
-    // The split kernel takes what the kernels with tensor maps do not (rows that do not start on 16-byte boundaries, any K; one or
-    // two rows of Q6_K stay with the streaming kernel, which is ahead there: 4096 x 2560 7.6 us against 9.7), Q4_K with more than
-    // four rows, and what it measured faster on, as one of a dependent chain: its fixed cost is higher and so is its rate.
-    //   one row:     24576 x 4096 Q4_0 17.6 us against 24.1, 12288 x 4096 11.3 / 12.4, 4096 x 4096 6.6 / 5.6
-    //   two rows:    24576 x 4096 20.0 / 26.1, 12288 x 4096 12.2 / 13.5, 4096 x 4096 7.9 / 7.4
-    //   four rows:   12288 x 4096 15.0 / 17.3, 4096 x 4096 8.4 / 9.5, 1024 x 4096 6.6 / 5.3, 4096 x 12288 17.7 / 16.8
-    // A mat-vec that can leave with an open batch of it joins that batch whatever its size.
+    // The split kernel takes what the kernels with tensor maps do not, rows that do not start on 16-byte boundaries (one or two
+    // rows of Q6_K stay with the streaming kernel, which is ahead there: 4096 x 2560 7.7 us against 9.4), and Q4_K with more than eight
+    // rows where that pays; what it shares with the register-level kernel is decided when the batch is launched.
     if ((mode == 3 || mode == 5) && !g_opt_mv_chain.load()) {
         const int t = (int)p->ggml_type;
         QmvArgs a = make_args(0);
+        const double fill = t == GT_Q4_K ? qmv_mma_fill(t, &a, 1, dev->sm_count) : 0.0;   // (of one group of eight rows)
         a.m = p->m;
         const bool aligned = qmv_split_aligned(t, a);
-        const uint64_t values = (uint64_t)p->n * p->k;
-        bool pays;
-        if (!aligned) pays = t != GT_Q6_K || (p->m > 2 && !qmv_mma_pair_mode(t, a));
-        else if (p->m == 1) pays = values >= (48ull << 20);
-        else if (p->m == 2) pays = values >= (48ull << 20) && p->k <= 8192;
-        else if (p->m <= 4) pays = values >= (16ull << 20) && (p->k <= 8192 || t == GT_Q4_K);
-        else pays = t == GT_Q4_K;
-        if (!enc->pend.empty() && enc->pend_split && enc->pend_type == t && !enc->pend[0].ids && enc->pend_mp == mv_row_class(p->m) && aligned) pays = true;
-        pays = pays || mode == 5;
-        if (pays && qmv_split_supported(t, a, dev->sm_count) && (p->m <= 8 || !sh))
+        const bool pays = mode == 5 || (!aligned ? t != GT_Q6_K || (p->m > 2 && !qmv_mma_pair_mode(t, a))
+                                                 : p->m > 8 && t == GT_Q4_K && qmv_split_pays(t, &a, 1, fill));
+        if (pays && (p->m <= 8 || !sh) && qmv_split_supported(t, a, dev->sm_count))
             return batch_mv(enc, t, a, p->m <= 8 ? mv_row_class(p->m) : 16u, !aligned, {{input, false}, {weight, false}, {output, true}});
     }
     // A mat-vec for the register-level kernel is not launched at once: it waits for the operations that follow, and
@@ -1959,11 +1962,14 @@ static int dispatch_id_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *de
     a.expert_stride = p->expert_stride;
     a.status = enc->status_word;
     // Few rows (decode): every (token, slot) row is one mat-vec of the register-level kernel, and the rows of this call,
-    // and of the calls around it that do not depend on it (gate and up of one layer), leave as one launch.
+    // and of the calls around it that do not depend on it (gate and up of one layer), leave as one launch.  More rows, or larger
+    // ones, take the split kernel, where the rows of one expert share a pass over its weights.  (A matter of the call alone: what a row's
+    // sum is does not depend on the calls around it.)
     const int mode = opt_qmv();
-    if ((mode == 3 || mode == 5) && qmv_split_supported(t, a, dev->sm_count))
+    const bool few = rows <= kMvBatchMax && qmv_mma_supported_routed(t, a);
+    if ((mode == 5 || (mode == 3 && qmv_split_pays_routed(t, a, few))) && qmv_split_supported(t, a, dev->sm_count))
         return batch_mv(enc, t, a, 1u, !qmv_split_aligned(t, a), {{input, false}, {up, false}, {weight, false}, {ids, false}, {output, true}});
-    if ((mode == 3 || mode == 4) && rows <= kMvBatchMax && qmv_mma_supported_routed(t, a)) {
+    if ((mode == 3 || mode == 4) && few) {
         const bool batch = g_opt_mv_batch.load() != 0;
         const bool fits = batch && !enc->pend.empty() && !enc->pend_split && enc->pend_type == t && enc->pend_mp == 1 && !enc->pend_pair &&
                           enc->pend.size() + rows <= kMvBatchMax;

@@ -1,0 +1,73 @@
+"""Which kernel a batch of independent mat-vecs leaves by is decided when the batch is complete, for all of it."""
+import itertools
+
+import numpy as np
+import pytest
+
+import mlx_native_b200 as mx
+from oracle import oracle as orc
+from tests.gpu_util import MV_TOL, TYPES, Ctx, norm_err, normal_acts, normal_weights
+
+pytestmark = pytest.mark.gpu
+K = 4096
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return Ctx()
+
+
+def encode(ctx, gtype, ops):
+    """ops: (weights, activations, rows of the matrix); results and kernel launches of one group."""
+    d = ctx.device
+    bufs = [(ctx.buf(x, mx.DType.F32), w, d.alloc_buffer(x.shape[0] * n * 4, mx.DType.F32)) for w, x, n in ops]
+    enc = d.command_encoder()
+    mx.reset_counters()
+    for (xb, wb, yb), (_, x, n) in zip(bufs, ops):
+        mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, wb, yb, mx.GgmlQuantizedMatmulParams(x.shape[0], n, K, gtype))
+    enc.commit_and_wait()
+    return [yb.as_slice(np.float32).reshape(x.shape[0], n).copy() for (_, _, yb), (_, x, n) in zip(bufs, ops)], mx.kernel_launch_count()
+
+
+# alone, the largest of these leaves by the split kernel and the others do not; together they are one launch, in any order
+@pytest.mark.parametrize("tname,m", [("Q4_0", 1), ("Q8_0", 1), ("Q8_0", 2), ("Q6_K", 1), ("Q4_0", 4)])
+def test_any_order_is_one_launch(ctx, tname, m):
+    gtype, otype = TYPES[tname]
+    part = normal_weights(m, 1024, K, otype)
+    x = normal_acts(m, m, K)
+    y_ref, ad = orc.qmatmul(otype, part, x, 1024, K, nthreads=8)
+    whole = ctx.buf(np.tile(part, 12), mx.DType.U8)
+    sizes = {n: whole.slice_view(0, part.size * (n // 1024)) for n in (1024, 4096, 12288)}
+    for order in itertools.permutations(sizes):
+        ys, launches = encode(ctx, gtype, [(sizes[n], x, n) for n in order])
+        assert launches == 1, order
+        for y, n in zip(ys, order):
+            for at in range(0, n, 1024):
+                assert norm_err(y[:, at:at + 1024], y_ref, ad) <= MV_TOL
+
+
+# Q4_K, five rows and more: the split kernel, its groups of eight in one launch; a matrix that fills the other kernel's passes, and a last
+# group of one row where the matrix is not small, stay with that one, one launch per group
+@pytest.mark.parametrize("m,n,launches", [(5, 1024, 2), (8, 16384, 1), (16, 1024, 2), (9, 1024, 2), (9, 8192, 2), (24, 16384, 3)])
+def test_q4k_of_many_rows(ctx, m, n, launches):
+    part = normal_weights(n, 1024, K, orc.Q4_K)
+    x = normal_acts(m, m, K)
+    y_ref, ad = orc.qmatmul(orc.Q4_K, part, x, 1024, K, nthreads=8)
+    (y,), count = encode(ctx, mx.GgmlType.Q4_K, [(ctx.buf(np.tile(part, n // 1024), mx.DType.U8), x, n)])
+    assert count == launches
+    for at in range(0, n, 1024):
+        assert norm_err(y[:, at:at + 1024], y_ref, ad) <= MV_TOL
+
+
+# a pair's sum does not depend on how many pairs the launch has, on either side of the number that one launch of the other kernel takes
+@pytest.mark.parametrize("tname,n,k", [("Q4_0", 768, 2048), ("Q6_K", 768, 2048), ("Q8_0", 1024, 768), ("Q4_0", 512, 1024)])
+def test_routed_rows_of_few_pairs_have_the_same_bits(ctx, tname, n, k):
+    gtype, otype = TYPES[tname]
+    E = 8
+    w = normal_weights(n, E * n, k, otype)
+    x = normal_acts(k, 16, k)
+    ids = np.random.default_rng(n).integers(0, E, 16).astype(np.uint32)
+    whole, _ = ctx.matmul_id(gtype, w, w.size // E, x, ids, 1, n, k, E)
+    for rows in (1, 3, 8, 15):
+        some, _ = ctx.matmul_id(gtype, w, w.size // E, x[:rows], ids[:rows], 1, n, k, E)
+        assert np.array_equal(some.view(np.uint32), whole[:rows].view(np.uint32)), rows
