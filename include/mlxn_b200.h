@@ -358,9 +358,11 @@ int mlxn_peer_barrier(mlxn_encoder *enc, uint32_t rank, uint32_t world, void *co
 
 /* ---- tuning and introspection (no upstream counterpart) -------------------------------------- */
 /* Selects kernel variants for cross-checks: key/value pairs
- *   "qmv" = auto | split | mma | tc | stream | simple   (auto: per shape and m, the fastest of the register-level tensor-core
- *           kernel "mma" and the tensor-memory kernel "tc", the streaming SIMT kernel for shapes neither takes;
- *           mma, stream and simple give bit-reproducible results, tc may differ in the last bit from run to run),
+ *   "qmv" = auto | split | mma | tc | stream | simple   (auto: per shape, m and batch, the fastest of the register-level
+ *           tensor-core kernel "mma", the tensor-memory kernel "tc" and the kernel "split", which shares K among the CTAs of a
+ *           cluster, takes weights at any even address and up to 256 expert-routed rows; the streaming SIMT kernel "stream" and
+ *           the plain one for shapes none of them takes; all but tc give bit-reproducible results, tc may differ in the last
+ *           bit from run to run),
  *   "qmm" = tc | simt,
  *   "qmv_mma_ctas" = 1 | 2 (CTAs per SM of the mma kernel), "qmv_mma_tpw" = 0 | 1 | 2 | 4 (its row-group size; 0 = auto).
  * Unknown keys are MLXN_INVALID_ARGUMENT.  The defaults are the fast paths. */
@@ -375,7 +377,8 @@ int mlxn_debug_wait_probe(mlxn_encoder *enc, uint32_t limit_us);
  * 16-byte boundary.  Looks at sizes alone and needs no GPU. */
 int mlxn_debug_split_geometry(const mlxn_qmm_id_params *params, uint32_t misaligned, uint32_t sm_count, uint32_t *ranks,
                               uint32_t *tiles);
-/* Name of the kernel variant the last operation on this thread launched (for tests and profiles). */
+/* Name of the kernel variant the last operation on this thread launched (for tests and profiles).  Mat-vecs wait for the operations
+ * that follow and are launched, and named, when their batch is (by a commit at the latest). */
 const char *mlxn_last_kernel_name(void);
 
 #ifdef __cplusplus

@@ -946,6 +946,7 @@ static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
         const size_t need = qmv_split_scratch_bytes(e->pend.data(), (int)e->pend.size());
         if (!need || (rc = encoder_scratch_on(e, e->pend_lane, need, &scratch)) == MLXN_OK)
             err = launch_qmv_split(e->pend_type, e->pend.data(), (int)e->pend.size(), e->dev->sm_count, scratch, &launches, st);
+        g_last_kernel = "qmv_split";
     } else if (lone_other) {
         if (!q6_one_row_small && qmv_tc_supported(e->pend_type, a0)) {
             uint8_t *scratch = nullptr;
@@ -958,6 +959,7 @@ static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
             err = launch_qmv(e->pend_type, a0, true, e->dev->sm_count, st, &g_last_kernel);
         }
     } else {
+        g_last_kernel = "qmv_mma";
         err = launch_qmv_mma(e->pend_type, e->pend.data(), (int)e->pend.size(), e->dev->sm_count, g_opt_mma_ctas.load(),
                              g_opt_mma_tpw.load(), st);
         if (err == cudaErrorCooperativeLaunchTooLarge) {
@@ -1573,7 +1575,6 @@ static int batch_mv(mlxn_encoder *enc, int type, const QmvArgs &a, uint32_t mp, 
         std::lock_guard<std::mutex> lk(ob.b->st->mu);
         ob.b->st->pend_enc = enc;
     }
-    g_last_kernel = "qmv_mma";
     g_dispatch.fetch_add(1);
     return batch ? MLXN_OK : encoder_flush_pending(enc);
 }
@@ -1666,7 +1667,6 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
                 std::lock_guard<std::mutex> lk(b->st->mu);
                 b->st->pend_enc = enc;
             }
-            g_last_kernel = "qmv_mma";
             g_dispatch.fetch_add(1);
             if (!batch) return encoder_flush_pending(enc);
             return MLXN_OK;
@@ -1997,7 +1997,6 @@ static int dispatch_id_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *de
             std::lock_guard<std::mutex> lk(b->st->mu);
             b->st->pend_enc = enc;
         }
-        g_last_kernel = "qmv_mma";
         g_dispatch.fetch_add(1);
         if (!batch) return encoder_flush_pending(enc);
         return MLXN_OK;

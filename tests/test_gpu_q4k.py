@@ -24,11 +24,15 @@ def test_dense_matvec(ctx, n, k, m):
     wq = normal_weights(n + k, n, k, O)
     x = normal_acts(m, m, k)
     y = ctx.matmul(G, wq, x, n, k)
-    assert mx.last_kernel_name() == "qmv_mma"            # the register-level tensor-core kernel (144-byte blocks: rows always 16-byte aligned)
+    # the register-level tensor-core kernel (144-byte blocks: rows always 16-byte aligned); the split kernel for more rows of a small matrix
+    assert mx.last_kernel_name() == ("qmv_split" if m > 4 else "qmv_mma")
     y_ref, ad = orc.qmatmul(O, wq, x, n, k, nthreads=4)
     assert norm_err(y, y_ref, ad) <= MV_TOL
-    mx.set_option("qmv", "simple")
+    mx.set_option("qmv", "mma")
     try:
+        y1 = ctx.matmul(G, wq, x, n, k)
+        assert mx.last_kernel_name() == "qmv_mma" and norm_err(y1, y_ref, ad) <= MV_TOL
+        mx.set_option("qmv", "simple")
         y2 = ctx.matmul(G, wq, x, n, k)
         assert mx.last_kernel_name() == "qmv_simple" and norm_err(y2, y_ref, ad) <= MV_TOL
     finally:
@@ -40,7 +44,7 @@ def test_dense_matvec_model_shapes(ctx, n, k, m):
     wq = normal_weights(n + k + m, n, k, O)
     x = normal_acts(m + 50, m, k)
     y = ctx.matmul(G, wq, x, n, k)
-    assert mx.last_kernel_name() == "qmv_mma"
+    assert mx.last_kernel_name() == ("qmv_split" if m > 4 else "qmv_mma")
     y_ref, ad = orc.qmatmul(O, wq, x, n, k, nthreads=8)
     assert norm_err(y, y_ref, ad) <= MV_TOL
 

@@ -35,6 +35,7 @@ def test_dense(ctx, tname, n, k, m):
     x = normal_acts(n + m, m, k)
     x[:, ::7] *= 1e-4          # (one power-of-two scale per row and slice)
     y = ctx.matmul(gtype, wq, x, n, k)
+    assert mx.last_kernel_name() == "qmv_split"
     y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8)
     assert norm_err(y, y_ref, ad) <= MV_TOL
     assert np.array_equal(y.view(np.uint32), ctx.matmul(gtype, wq, x, n, k).view(np.uint32))
@@ -50,6 +51,7 @@ def test_weights_at_any_even_address(ctx, tname, offset, m):
     big[offset:offset + wq.size] = wq
     x = normal_acts(1, m, k)
     y = ctx.matmul(gtype, wq, x, n, k, weight_buf=ctx.buf(big, mx.DType.U8).slice_view(offset, wq.size))
+    assert mx.last_kernel_name() == "qmv_split"
     y_ref, ad = orc.qmatmul(otype, wq, x, n, k)
     assert norm_err(y, y_ref, ad) <= MV_TOL
 
@@ -72,6 +74,7 @@ def test_routed(ctx, tname, T, top_k, E, n, k):
     if ids.size > 20:
         bad[[5, 11]] = True
     y, _ = ctx.matmul_id(gtype, w, w.size // E, x, np.where(bad, 0xFFFFFFFF, ids).astype(np.uint32), top_k, n, k, E)
+    assert mx.last_kernel_name() == "qmv_split"
     y_ref, ad = orc.qmatmul_id(otype, w, w.size // E, x, ids, top_k, n, k, E, nthreads=8)
     assert norm_err(y[~bad], y_ref[~bad], ad[~bad]) <= MV_TOL
     assert np.all(y[bad] == 0)
@@ -90,6 +93,7 @@ def test_batch_of_different_shapes(ctx):
     for (xb, wb, yb), (n, k, m) in zip(bufs, shapes):
         mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, wb, yb, mx.GgmlQuantizedMatmulParams(m, n, k, gtype))
     enc.commit_and_wait()
+    assert mx.last_kernel_name() == "qmv_split"
     assert mx.kernel_launch_count() == 2          # the activations of all of them packed by one kernel, then one mat-vec kernel
     for (xb, wb, yb), w, x, (n, k, m) in zip(bufs, ws, xs, shapes):
         y_ref, ad = orc.qmatmul(otype, w, x, n, k)
@@ -115,7 +119,9 @@ def test_error_against_64_bits(ctx, tname, n, k, rows):
     wq = normal_weights(n + k, n, k, otype)
     x = normal_acts(n + rows, rows, k)
     x[:, ::97] *= 300
-    assert relative_error(ctx.matmul(gtype, wq, x, n, k), orc.dequantize(otype, wq).reshape(n, k).astype(np.float64), x) <= ERR_TOL
+    y = ctx.matmul(gtype, wq, x, n, k)
+    assert mx.last_kernel_name() == "qmv_split"
+    assert relative_error(y, orc.dequantize(otype, wq).reshape(n, k).astype(np.float64), x) <= ERR_TOL
 
 
 # activation rows that f16 halves could lose: infinities, no numbers, magnitudes at either end of f32
@@ -165,4 +171,5 @@ def test_routed_infinities_and_extreme_magnitudes(ctx, tname, n, k):
     ids = np.stack([rng.permutation(E)[:top_k] for _ in range(T)]).astype(np.uint32).reshape(-1)
     y, _ = ctx.matmul_id(gtype, w, w.size // E, x, ids, top_k, n, k, E)
     y_ref, ad = orc.qmatmul_id(otype, w, w.size // E, x, ids, top_k, n, k, E, nthreads=8)
+    assert mx.last_kernel_name() == "qmv_split"
     assert_same_numbers(y, y_ref, ad)

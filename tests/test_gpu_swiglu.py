@@ -86,7 +86,8 @@ def test_q4_0_wrapper_and_errors(ctx):
 
 # ---- decode-sized routed mat-vecs: every (token, slot) row is one problem of the batched register-level kernel, and gate and
 # ---- up of one layer (same activations and ids, different weights) leave as ONE launch
-def test_gate_and_up_share_a_launch_and_bad_ids_give_zeros(ctx):
+@pytest.mark.parametrize("qmv", ["split", "mma"])
+def test_gate_and_up_share_a_launch_and_bad_ids_give_zeros(ctx, qmv):
     gtype, otype = TYPES["Q4_0"]
     n_experts, top_k, n, k = 16, 8, 768, 2048
     wg, stride = stacked(otype, n_experts, n, k, seed=600)
@@ -97,12 +98,14 @@ def test_gate_and_up_share_a_launch_and_bad_ids_give_zeros(ctx):
     xb, ib = ctx.buf(x, mx.DType.F32), ctx.buf(ids, mx.DType.U32)
     yg, yu = d.alloc_buffer(top_k * n * 4, mx.DType.F32), d.alloc_buffer(top_k * n * 4, mx.DType.F32)
     p = mx.GgmlQuantizedMatmulIdParams(1, top_k, n, k, n_experts, stride, gtype)
+    mx.set_option("qmv", "auto" if qmv == "split" else qmv)            # (what these take by themselves)
     mx.reset_counters()
     enc = d.command_encoder()
     mx.quantized_matmul_id_ggml(enc, ctx.registry, d, xb, ctx.buf(wg, mx.DType.U8), ib, yg, p)
     mx.quantized_matmul_id_ggml(enc, ctx.registry, d, xb, ctx.buf(wu, mx.DType.U8), ib, yu, p)
     enc.commit_and_wait()
-    assert mx.last_kernel_name() == "qmv_mma" and mx.kernel_launch_count() == 1 and mx.dispatch_count() == 2
+    mx.set_option("qmv", "auto")
+    assert mx.last_kernel_name() == "qmv_" + qmv and mx.kernel_launch_count() == 1 and mx.dispatch_count() == 2
     good = ids < n_experts
     for w, yb in ((wg, yg), (wu, yu)):
         y = yb.as_slice(np.float32).reshape(top_k, n)
@@ -113,15 +116,16 @@ def test_gate_and_up_share_a_launch_and_bad_ids_give_zeros(ctx):
 
 # ---- a (token, slot) pair's row does not depend on how many pairs share its launch: the all-to-all MoE layer sends
 # ---- each rank a different subset of the pairs and is still bit-identical to the one-GPU layer
-@pytest.mark.parametrize("tname,n,k", [("Q4_0", 768, 2048), ("Q8_0", 768, 2048), ("Q6_K", 512, 2048), ("Q4_K", 512, 2048)])
-def test_routed_rows_do_not_depend_on_the_launch_composition(ctx, tname, n, k):
+@pytest.mark.parametrize("tname,n,k,kernel", [("Q4_0", 768, 2048, "split"), ("Q8_0", 768, 2048, "split"), ("Q4_0", 512, 2048, "mma"),
+                                              ("Q8_0", 512, 2048, "mma"), ("Q6_K", 512, 2048, "mma"), ("Q4_K", 512, 2048, "mma")])
+def test_routed_rows_do_not_depend_on_the_launch_composition(ctx, tname, n, k, kernel):
     gtype, otype = TYPES[tname] if tname in TYPES else (mx.GgmlType.Q4_K, orc.Q4_K)
     n_experts = 8
     w, stride = stacked(otype, n_experts, n, k, seed=800)
     rows = normal_acts(21, 8, k)                                       # eight pairs, one activation row each (top_k = 1)
     ids = np.array([5, 1, 7, 2, 2, 0, 6, 3], np.uint32)
     whole, _ = ctx.matmul_id(gtype, w, stride, rows, ids, 1, n, k, n_experts)
-    assert mx.last_kernel_name() == "qmv_mma"
+    assert mx.last_kernel_name() == "qmv_" + kernel
     for parts in ((3, 5), (1, 7), (2, 2, 4)):
         lo = 0
         for cnt in parts:
