@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "mma_f16.cuh"
 #include "ptx.cuh"
 
 namespace mlxn {
@@ -96,58 +97,6 @@ struct SpMaps {
     CUtensorMap m[kSpMaxOps];
 };
 
-// ---- shared-memory access by 32-bit address -----------------------------------------------------------
-namespace sp {
-__device__ __forceinline__ uint32_t ld32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-template <uint32_t OFF> __device__ __forceinline__ uint32_t ld32i(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
-    return v;
-}
-template <uint32_t OFF> __device__ __forceinline__ uint32_t ld16i(uint32_t a) {
-    uint32_t v;
-    asm volatile("{ .reg .u16 t; ld.shared.u16 t, [%1+%2]; cvt.u32.u16 %0, t; }" : "=r"(v) : "r"(a), "n"(OFF));
-    return v;
-}
-template <uint32_t OFF> __device__ __forceinline__ void ld128i(uint32_t a, uint32_t (&v)[4]) {
-    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4+%5];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a), "n"(OFF));
-}
-__device__ __forceinline__ void st32(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
-__device__ __forceinline__ void st64(uint32_t a, uint32_t v0, uint32_t v1) {
-    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(v0), "r"(v1) : "memory");
-}
-__device__ __forceinline__ void st128(uint32_t a, float v0, float v1, float v2, float v3) {
-    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(a), "f"(v0), "f"(v1), "f"(v2), "f"(v3) : "memory");
-}
-__device__ __forceinline__ float h_lo(uint32_t w) {
-    float f;
-    asm("{ .reg .f16 l, h; mov.b32 {l, h}, %1; cvt.f32.f16 %0, l; }" : "=f"(f) : "r"(w));
-    return f;
-}
-__device__ __forceinline__ float h_hi(uint32_t w) {
-    float f;
-    asm("{ .reg .f16 l, h; mov.b32 {l, h}, %1; cvt.f32.f16 %0, h; }" : "=f"(f) : "r"(w));
-    return f;
-}
-// D = A (16 x 16) B (16 x 8) + C: lane (g = lane / 4, t = lane % 4) holds a0/a1 = rows g / g + 8, k 2t..; a2/a3 the same,
-// k 2t + 8..; b0, b1 likewise for column g; c0, c1 = row g, columns 2t, 2t + 1; c2, c3 = row g + 8.
-__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1,
-                                    float c0, float c1, float c2, float c3) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
-}
-template <int I, int N, class F> __device__ __forceinline__ void each(F &&f) {
-    if constexpr (I < N) {
-        f(std::integral_constant<int, I>{});
-        each<I + 1, N>(f);
-    }
-}
-}  // namespace sp
 __device__ __forceinline__ void bulk_g2s_a(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
                  "r"(smem_u32(bar))
@@ -259,7 +208,7 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
             se[h] = mis ? 0x7654u : 0x5432u;
             so[h] = mis ? 0x5432u : 0x3210u;
         }
-        sp::each<0, NT>([&](auto J) {
+        static_for<0, NT>([&](auto J) {
             constexpr uint32_t o = decltype(J)::value * TS;
             uint32_t w[4][2];   // even block, MMA 0 / 1; odd block, MMA 0 / 1 (Q4_0: one word per block)
             float d0[2], d1[2];
@@ -268,32 +217,32 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                 const uint32_t b = b0[h];
                 [[maybe_unused]] const uint32_t e = h ? e1 : e0, a = h ? a1 : a0;
                 if constexpr (ALN) {
-                    const uint32_t s0 = sp::ld32i<o>(b), s1 = sp::ld32i<o>(e);
+                    const uint32_t s0 = lds32i<o>(b), s1 = lds32i<o>(e);
                     w[0][h] = __byte_perm(s0, s1, sel);
                     if constexpr (Q8) {
-                        w[1][h] = sp::ld32i<o + 16>(b);
-                        w[2][h] = sp::ld32i<o + 36>(b);
-                        w[3][h] = sp::ld32i<o + 52>(b);
+                        w[1][h] = lds32i<o + 16>(b);
+                        w[2][h] = lds32i<o + 36>(b);
+                        w[3][h] = lds32i<o + 52>(b);
                     } else {
-                        w[2][h] = sp::ld32i<o + 20>(b);
+                        w[2][h] = lds32i<o + 20>(b);
                     }
                     if constexpr (ONE) {   // one activation row: only lane 0 of a quad holds results, and it has the scales
-                        d0[h] = sp::h_lo(s0);
-                        d1[h] = sp::h_hi(s1);
+                        d0[h] = f16lo_to_float(s0);
+                        d1[h] = f16hi_to_float(s1);
                     }
                 } else {
-                    w[0][h] = __byte_perm(sp::ld32i<o>(b), sp::ld32i<o + 4>(b), se[h]);
+                    w[0][h] = __byte_perm(lds32i<o>(b), lds32i<o + 4>(b), se[h]);
                     if constexpr (Q8) {
-                        w[1][h] = __byte_perm(sp::ld32i<o + 16>(b), sp::ld32i<o + 20>(b), se[h]);
-                        w[2][h] = __byte_perm(sp::ld32i<o + 36>(b), sp::ld32i<o + 40>(b), so[h]);
-                        w[3][h] = __byte_perm(sp::ld32i<o + 52>(b), sp::ld32i<o + 56>(b), so[h]);
+                        w[1][h] = __byte_perm(lds32i<o + 16>(b), lds32i<o + 20>(b), se[h]);
+                        w[2][h] = __byte_perm(lds32i<o + 36>(b), lds32i<o + 40>(b), so[h]);
+                        w[3][h] = __byte_perm(lds32i<o + 52>(b), lds32i<o + 56>(b), so[h]);
                     } else {
-                        w[2][h] = __byte_perm(sp::ld32i<o + 20>(b), sp::ld32i<o + 24>(b), so[h]);
+                        w[2][h] = __byte_perm(lds32i<o + 20>(b), lds32i<o + 24>(b), so[h]);
                     }
                 }
                 if constexpr (!ALN || !ONE) {
-                    d0[h] = sp::h_lo(sp::ld16i<o>(a));
-                    d1[h] = sp::h_lo(sp::ld16i<o + BB>(a));
+                    d0[h] = f16lo_to_float(lds_u16i<o>(a));
+                    d1[h] = f16lo_to_float(lds_u16i<o + BB>(a));
                     if constexpr (!ALN) d1[h] = half ? 0.f : d1[h];
                 }
             }
@@ -318,11 +267,12 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
             constexpr int j = decltype(J)::value;
 #pragma unroll
             for (int s = 0; s < NS; s++) {
+                constexpr float zero[4] = {0.f, 0.f, 0.f, 0.f};
                 float r0[4], r1[4];
-                sp::mma(r0, a[0][0], a[0][1], a[0][2], a[0][3], bf[s][0][0], bf[s][0][1], 0.f, 0.f, 0.f, 0.f);
-                sp::mma(r1, a[2][0], a[2][1], a[2][2], a[2][3], bf[s][2][0], bf[s][2][1], 0.f, 0.f, 0.f, 0.f);
-                sp::mma(r0, a[1][0], a[1][1], a[1][2], a[1][3], bf[s][1][0], bf[s][1][1], r0[0], r0[1], r0[2], r0[3]);
-                sp::mma(r1, a[3][0], a[3][1], a[3][2], a[3][3], bf[s][3][0], bf[s][3][1], r1[0], r1[1], r1[2], r1[3]);
+                mma16816(r0, a[0][0], a[0][1], a[0][2], a[0][3], bf[s][0][0], bf[s][0][1], zero);
+                mma16816(r1, a[2][0], a[2][1], a[2][2], a[2][3], bf[s][2][0], bf[s][2][1], zero);
+                mma16816(r0, a[1][0], a[1][1], a[1][2], a[1][3], bf[s][1][0], bf[s][1][1], r0);
+                mma16816(r1, a[3][0], a[3][1], a[3][2], a[3][3], bf[s][3][0], bf[s][3][1], r1);
                 acc[j][s][0] = fmaf(d1[0], r1[0], fmaf(d0[0], r0[0], acc[j][s][0]));
                 acc[j][s][1] = fmaf(d1[0], r1[1], fmaf(d0[0], r0[1], acc[j][s][1]));
                 acc[j][s][2] = fmaf(d1[1], r1[2], fmaf(d0[1], r0[2], acc[j][s][2]));
@@ -333,20 +283,20 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
         constexpr bool Q5 = T == GT_Q5_K;
         const uint32_t pu = u & 3u, qo = (Q5 ? 48u : 16u) + 32 * pu + 4 * t;
         const uint32_t q0 = a0 + qo, q1 = a1 + qo, h0 = a0 + 16 + 4 * t, h1 = a1 + 16 + 4 * t, tr = tab + g * 16;
-        sp::each<0, NT>([&](auto J) {
+        static_for<0, NT>([&](auto J) {
             constexpr int j = decltype(J)::value;
             constexpr uint32_t o = j * TS;
             uint32_t x[2][2];   // [first / second 16 elements][row g, g + 8]
-            x[0][0] = sp::ld32i<o>(q0); x[1][0] = sp::ld32i<o + 16>(q0);
-            x[0][1] = sp::ld32i<o>(q1); x[1][1] = sp::ld32i<o + 16>(q1);
+            x[0][0] = lds32i<o>(q0); x[1][0] = lds32i<o + 16>(q0);
+            x[0][1] = lds32i<o>(q1); x[1][1] = lds32i<o + 16>(q1);
             uint32_t p0[4], p1[4];   // scales and offsets (sp_table_row) of rows g and g + 8
-            sp::ld128i<j * 256u>(tr, p0);
-            sp::ld128i<j * 256u + 128u>(tr, p1);
+            lds128i<j * 256u>(tr, p0);
+            lds128i<j * 256u + 128u>(tr, p1);
             uint32_t a[4][4];
             if constexpr (Q5) {   // five-bit codes, one per byte: nibble | fifth bit << 4
                 uint32_t f[2][2];
-                f[0][0] = sp::ld32i<o>(h0) >> (2 * pu); f[1][0] = sp::ld32i<o + 16>(h0) >> (2 * pu);
-                f[0][1] = sp::ld32i<o>(h1) >> (2 * pu); f[1][1] = sp::ld32i<o + 16>(h1) >> (2 * pu);
+                f[0][0] = lds32i<o>(h0) >> (2 * pu); f[1][0] = lds32i<o + 16>(h0) >> (2 * pu);
+                f[0][1] = lds32i<o>(h1) >> (2 * pu); f[1][1] = lds32i<o + 16>(h1) >> (2 * pu);
 #pragma unroll
                 for (int e = 0; e < 2; e++)
 #pragma unroll
@@ -368,11 +318,12 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
             }
 #pragma unroll
             for (int s = 0; s < NS; s++) {
+                constexpr float zero[4] = {0.f, 0.f, 0.f, 0.f};
                 float r0[4], r1[4];
-                sp::mma(r0, a[0][0], a[0][1], a[0][2], a[0][3], bf[s][0][0], bf[s][0][1], 0.f, 0.f, 0.f, 0.f);
-                sp::mma(r1, a[2][0], a[2][1], a[2][2], a[2][3], bf[s][2][0], bf[s][2][1], 0.f, 0.f, 0.f, 0.f);
-                sp::mma(r0, a[1][0], a[1][1], a[1][2], a[1][3], bf[s][1][0], bf[s][1][1], r0[0], r0[1], r0[2], r0[3]);
-                sp::mma(r1, a[3][0], a[3][1], a[3][2], a[3][3], bf[s][3][0], bf[s][3][1], r1[0], r1[1], r1[2], r1[3]);
+                mma16816(r0, a[0][0], a[0][1], a[0][2], a[0][3], bf[s][0][0], bf[s][0][1], zero);
+                mma16816(r1, a[2][0], a[2][1], a[2][2], a[2][3], bf[s][2][0], bf[s][2][1], zero);
+                mma16816(r0, a[1][0], a[1][1], a[1][2], a[1][3], bf[s][1][0], bf[s][1][1], r0);
+                mma16816(r1, a[3][0], a[3][1], a[3][2], a[3][3], bf[s][3][0], bf[s][3][1], r1);
                 const float c0 = cc[s][0], c1 = cc[s][1];
                 auto f = [](uint32_t v) { return __uint_as_float(v); };
                 acc[j][s][0] = fmaf(f(p0[1]), r1[0], fmaf(f(p0[0]), r0[0], fmaf(f(p0[3]), c1, fmaf(f(p0[2]), c0, acc[j][s][0]))));
@@ -391,18 +342,18 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
             const uint32_t b0 = a0 & ~3u, b1 = a1 & ~3u;
             const uint32_t L[2] = {b0 + lo, b1 + lo}, H[2] = {b0 + ho, b1 + ho};
             const uint32_t sl[2] = {(a0 & 2u) ? 0x5432u : 0x3210u, (a1 & 2u) ? 0x5432u : 0x3210u};
-            sp::each<0, NT>([&](auto J) {
+            static_for<0, NT>([&](auto J) {
                 constexpr int j = decltype(J)::value;
                 constexpr uint32_t o = j * TS;
                 uint32_t qv[2][4];
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    uint32_t A = sp::ld32i<o>(L[h]), B = sp::ld32i<o + 32>(L[h]), X = sp::ld32i<o>(H[h]);
+                    uint32_t A = lds32i<o>(L[h]), B = lds32i<o + 32>(L[h]), X = lds32i<o>(H[h]);
                     if constexpr (shift != 0) {
                         const uint32_t s = shift == 1 ? 0x5432u : sl[h];
-                        A = __byte_perm(A, sp::ld32i<o + 4>(L[h]), s);
-                        B = __byte_perm(B, sp::ld32i<o + 36>(L[h]), s);
-                        X = __byte_perm(X, sp::ld32i<o + 4>(H[h]), s);
+                        A = __byte_perm(A, lds32i<o + 4>(L[h]), s);
+                        B = __byte_perm(B, lds32i<o + 36>(L[h]), s);
+                        X = __byte_perm(X, lds32i<o + 4>(H[h]), s);
                     }
                     qv[h][0] = (A & 0x0F0F0F0Fu) | ((X & 0x03030303u) << 4);
                     qv[h][1] = (B & 0x0F0F0F0Fu) | ((X & 0x0C0C0C0Cu) << 2);
@@ -410,8 +361,8 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                     qv[h][3] = ((B >> 4) & 0x0F0F0F0Fu) | ((X & 0xC0C0C0C0u) >> 2);
                 }
                 uint32_t p0[4], p1[4];
-                sp::ld128i<j * 256u>(tr, p0);
-                sp::ld128i<j * 256u + 128u>(tr, p1);
+                lds128i<j * 256u>(tr, p0);
+                lds128i<j * 256u + 128u>(tr, p1);
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const uint32_t x0 = sp::bytes02(qv[0][q], 0x64206420u), x2 = sp::bytes13(qv[0][q], 0x64206420u);
@@ -419,8 +370,9 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                     const float pa = __uint_as_float(p0[q]), pb = __uint_as_float(p1[q]);
 #pragma unroll
                     for (int s = 0; s < NS; s++) {
+                        constexpr float zero[4] = {0.f, 0.f, 0.f, 0.f};
                         float r[4];
-                        sp::mma(r, x0, x1, x2, x3, bf[s][q][0], bf[s][q][1], 0.f, 0.f, 0.f, 0.f);
+                        mma16816(r, x0, x1, x2, x3, bf[s][q][0], bf[s][q][1], zero);
                         acc[j][s][0] = fmaf(pa, r[0], acc[j][s][0]);
                         acc[j][s][1] = fmaf(pa, r[1], acc[j][s][1]);
                         acc[j][s][2] = fmaf(pb, r[2], acc[j][s][2]);
@@ -442,13 +394,14 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
 // of its two sub-blocks (Q4_K, Q5_K: the codes are taken less C = 8 or 16, the middle of their range, so that the offset is small
 // where scale and minimum belong together; 6-bit fields as in src/gguf/mod.rs:440-452).  rb: shared address of the row's super-block.
 template <int T> __device__ __forceinline__ void sp_table_row(uint32_t dst, uint32_t rb, uint32_t u) {
+    auto put = [&](float a, float b, float c, float d) { sts128(dst, __float_as_uint(a), __float_as_uint(b), __float_as_uint(c), __float_as_uint(d)); };
     if constexpr (T == GT_Q6_K) {
         const uint32_t s = rb + 192 + 8 * ((u >> 1) & 1u) + (u & 1u);
-        const float d = sp::h_lo(sp::ld16i<208>(rb));
-        sp::st128(dst, d * (float)lds_s8(s), d * (float)lds_s8(s + 2), d * (float)lds_s8(s + 4), d * (float)lds_s8(s + 6));
+        const float d = f16lo_to_float(lds_u16i<208>(rb));
+        put(d * (float)lds_s8(s), d * (float)lds_s8(s + 2), d * (float)lds_s8(s + 4), d * (float)lds_s8(s + 6));
     } else {
-        const uint32_t pu = u & 3u, dd = sp::ld32(rb), s0 = sp::ld32i<4>(rb), s1 = sp::ld32i<8>(rb);
-        const float d = sp::h_lo(dd), dmin = sp::h_hi(dd);
+        const uint32_t pu = u & 3u, dd = lds32(rb), s0 = lds32i<4>(rb), s1 = lds32i<8>(rb);
+        const float d = f16lo_to_float(dd), dmin = f16hi_to_float(dd);
         uint32_t c0, c1, m0, m1;
         if (pu < 2) {
             const uint32_t a = s0 >> (16 * pu), b = s1 >> (16 * pu);
@@ -456,7 +409,7 @@ template <int T> __device__ __forceinline__ void sp_table_row(uint32_t dst, uint
             m0 = b & 63u; m1 = (b >> 8) & 63u;
         } else {
             const uint32_t sh = 16 * (pu - 2);
-            const uint32_t a = sp::ld32i<12>(rb) >> sh, lo = s0 >> sh, hi = s1 >> sh;
+            const uint32_t a = lds32i<12>(rb) >> sh, lo = s0 >> sh, hi = s1 >> sh;
             c0 = (a & 15u) | (((lo >> 6) & 3u) << 4);
             c1 = ((a >> 8) & 15u) | (((lo >> 14) & 3u) << 4);
             m0 = ((a >> 4) & 15u) | (((hi >> 6) & 3u) << 4);
@@ -464,7 +417,7 @@ template <int T> __device__ __forceinline__ void sp_table_row(uint32_t dst, uint
         }
         constexpr float C = T == GT_Q5_K ? 16.f : 8.f;
         const float e0 = d * (float)c0, e1 = d * (float)c1;   // (17 bits: exact, as the products with the minima)
-        sp::st128(dst, e0, e1, fmaf(C, e0, -(dmin * (float)m0)), fmaf(C, e1, -(dmin * (float)m1)));
+        put(e0, e1, fmaf(C, e0, -(dmin * (float)m0)), fmaf(C, e1, -(dmin * (float)m1)));
     }
 }
 
@@ -788,7 +741,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 const uint32_t col = q / R, row = q - col * R;
                 float v = 0.f;
 #pragma unroll
-                for (int w = 0; w < kSpWarps; w++) v += __uint_as_float(sp::ld32(part + ((w * mp + col) * R + row) * 4));
+                for (int w = 0; w < kSpWarps; w++) v += __uint_as_float(lds32(part + ((w * mp + col) * R + row) * 4));
                 if (ranks == 1) {
                     store(d, col, row, v);
                 } else {
@@ -812,7 +765,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             for (uint32_t q = tid; q < mp * share; q += 256) {
                 const uint32_t col = q / share, row = q - col * share;
                 float v = 0.f;
-                for (uint32_t r = 0; r < ranks; r++) v += __uint_as_float(sp::ld32(base + bt.recv_off + (((buf * ranks + r) * mp + col) * share + row) * 4));
+                for (uint32_t r = 0; r < ranks; r++) v += __uint_as_float(lds32(base + bt.recv_off + (((buf * ranks + r) * mp + col) * share + row) * 4));
                 store(d, col, rank * share + row, v);
             }
             return true;
@@ -892,9 +845,9 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                     sp::split(c[1], c[3], hi[1], lo[1]);
                     if (2 * p + hf >= mine || !mine_too) return;
                     const uint32_t d = d0 + p * 4096u + row * xs;
-                    sp::st64(d, hi[0], hi[1]);
-                    sp::st64(d + 16, lo[0], lo[1]);
-                    if (NG != 0 && (lane & 7u) == 0) sp::st32(ccb + ((warp + 8 * hf) * NG + (q >> 1)) * 4u + p * (64u * NG) + row * cs, __float_as_uint(sum));
+                    sts64(d, hi[0], hi[1]);
+                    sts64(d + 16, lo[0], lo[1]);
+                    if (NG != 0 && (lane & 7u) == 0) sts32(ccb + ((warp + 8 * hf) * NG + (q >> 1)) * 4u + p * (64u * NG) + row * cs, __float_as_uint(sum));
                 };
                 __syncwarp();
                 if constexpr (MPC == 1) {
@@ -1041,12 +994,12 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                         uint32_t v[4];
                         const uint32_t xa = xlane + uu * 256u + s * 4u * xs;
                         [[maybe_unused]] const uint32_t ca = clane + uu * NG * 4u + s * 4u * cs;
-                        sp::ld128i<0>(xa, v);
+                        lds128i<0>(xa, v);
                         bf[s][0][0] = v[0]; bf[s][0][1] = v[1]; bf[s][1][0] = v[2]; bf[s][1][1] = v[3];
-                        sp::ld128i<128>(xa, v);
+                        lds128i<128>(xa, v);
                         bf[s][2][0] = v[0]; bf[s][2][1] = v[1]; bf[s][3][0] = v[2]; bf[s][3][1] = v[3];
 #pragma unroll
-                        for (int q = 0; q < NG; q++) cc[s][q] = __uint_as_float(sp::ld32(ca + q * 4u));
+                        for (int q = 0; q < NG; q++) cc[s][q] = __uint_as_float(lds32(ca + q * 4u));
                     }
                     const uint32_t ub = TABLE ? (ul >> 2) * (uint32_t)K::B256 : ul * UB;
                     if constexpr (TABLE) {
@@ -1089,8 +1042,8 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                     if (col < mp && j < (int)c.nt) {
                         const float inv = s_inv[warp][col];
                         const uint32_t a = part + ((warp * mp + col) * R + 16 * j + g) * 4;
-                        sp::st32(a, __float_as_uint((acc[j][s][0] + acc[j][s][1]) * inv));
-                        sp::st32(a + 32, __float_as_uint((acc[j][s][2] + acc[j][s][3]) * inv));
+                        sts32(a, __float_as_uint((acc[j][s][0] + acc[j][s][1]) * inv));
+                        sts32(a + 32, __float_as_uint((acc[j][s][2] + acc[j][s][3]) * inv));
                     }
                 }
             __syncwarp();
@@ -1134,8 +1087,7 @@ struct SpShape {          // geometry of a launch
 // Two CTAs share an SM: 228 KB less 1 KB each for the system and the kernel's static 2.5 KB.
 constexpr size_t kSpSmem = 110 * 1024;
 
-template <int T> inline size_t sp_tail(bool aln, uint32_t ranks, uint32_t tr, uint32_t mp, uint32_t xunits, SpBatch *b) {
-    (void)aln;
+template <int T> inline size_t sp_tail(uint32_t ranks, uint32_t tr, uint32_t mp, uint32_t xunits, SpBatch *b) {
     const size_t r = 16u * tr;
     const size_t xf = (size_t)xunits * mp * 256, cc = SpTraits<T>::NG ? (((size_t)xunits * SpTraits<T>::NG * 4 + 16) * mp + 127) / 128 * 128 : 0;
     const size_t tab = SpTraits<T>::B256 == 272 || T == GT_Q4_0 ? 0 : (size_t)kSpWarps * r * 16;
@@ -1162,17 +1114,17 @@ static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, ui
     // activations
     bt.run = 1;
     if (const char *e = exp_env("MLXN_SP_RUN")) bt.run = (uint32_t)atoi(e);
-    const size_t tail = sp_tail<T>(ALN, ranks, tr, bt.mp, xunits, nullptr);
+    const size_t tail = sp_tail<T>(ranks, tr, bt.mp, xunits, nullptr);
     uint32_t nslots = (uint32_t)((kSpSmem - 128 - tail) / STAGE);
     if (nslots > (uint32_t)kSpMaxSlots) nslots = kSpMaxSlots;
     if (tail + STAGE + 128 > kSpSmem || nslots < 1) return cudaErrorInvalidConfiguration;
     bt.nslots = nslots;
     bt.xf_off = nslots * STAGE;
-    sp_tail<T>(ALN, ranks, tr, bt.mp, xunits, &bt);
+    sp_tail<T>(ranks, tr, bt.mp, xunits, &bt);
     const size_t smem = (size_t)nslots * STAGE + tail + 128;
     auto kernel = qmv_split_kernel<T, ALN, MPC>;
-    static std::atomic<uint32_t> prepared[64] = {};   // per device: attribute set, and the clusters that fit (bits 8.. by log2 ranks)
-    static std::atomic<uint32_t> fit[64][4] = {};
+    static std::atomic<uint32_t> prepared[64] = {};   // per device: the attribute has been set
+    static std::atomic<uint32_t> fit[64][4] = {};     // ... and the clusters of 2, 4 and 8 CTAs that are resident together
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
@@ -1236,7 +1188,7 @@ template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool 
         if (c > 1 && slice * (c - 1) >= max_units && pick.ranks) continue;
         for (uint32_t tr = 1; tr <= (uint32_t)sp_tiles((int)sets); tr++) {
             if ((force_c && !routed && (int)c != force_c) || (force_tr && (int)tr != force_tr)) continue;
-            const size_t stage = (size_t)tr * 16 * sp_pitch<T>(aln), tail = sp_tail<T>(aln, c, tr, mp, (slice + 1) & ~1u, nullptr);
+            const size_t stage = (size_t)tr * 16 * sp_pitch<T>(aln), tail = sp_tail<T>(c, tr, mp, (slice + 1) & ~1u, nullptr);
             if (tail + 2 * stage + 128 > kSpSmem) continue;
             const double slots = (double)((kSpSmem - 128 - tail) / stage);
             const double ncl = (double)(2 * sm_count / (int)c), chunks = ceil(ceil((double)tiles / tr) / ncl);
@@ -1273,6 +1225,7 @@ template <int T> inline size_t sp_pack_bytes(uint32_t m, uint32_t k) {
 template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, uint8_t *scratch, int *launches, cudaStream_t st) {
     if (nops < 1 || nops > kSpMaxOps) return cudaErrorInvalidValue;
     const bool routed = ops[0].ids != nullptr;
+    if (T == GT_Q5_K && !routed) return cudaErrorNotSupported;
     bool aln = true;
     for (int i = 0; i < nops; i++) {
         const uint64_t rb = (uint64_t)(ops[i].k / BlockTraits<T>::QK) * BlockTraits<T>::BYTES;
@@ -1344,16 +1297,18 @@ template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, 
     *launches = 1;
     auto go = [&](auto ALN) {
         constexpr bool A = decltype(ALN)::value;
-        if (bt.packed) {
-            uint32_t end = 0;
-            for (int i = 0; i < nops; i++) bt.op[i].row_end = end += bt.op[i].xkey == (uint32_t)i ? bt.op[i].m : 0u;
-            const cudaError_t e = launch_overlapped(qmv_pack_kernel<T, A>, dim3(end), dim3(256), 0, st, bt);
-            if (e != cudaSuccess) return e;
-            ++*launches;
+        if constexpr (T != GT_Q5_K) {   // (expert-routed only: never packed, one set of columns)
+            if (bt.packed) {
+                uint32_t end = 0;
+                for (int i = 0; i < nops; i++) bt.op[i].row_end = end += bt.op[i].xkey == (uint32_t)i ? bt.op[i].m : 0u;
+                const cudaError_t e = launch_overlapped(qmv_pack_kernel<T, A>, dim3(end), dim3(256), 0, st, bt);
+                if (e != cudaSuccess) return e;
+                ++*launches;
+            }
+            if (bt.mp > 4) return sp_choose<T, A, 8>(bt, maps, all, entries, max_units, routed, sm_count, st);
         }
         if (bt.mp == 1) return sp_choose<T, A, 1>(bt, maps, all, entries, max_units, routed, sm_count, st);
-        if (bt.mp <= 4) return sp_choose<T, A, 4>(bt, maps, all, entries, max_units, routed, sm_count, st);
-        return sp_choose<T, A, 8>(bt, maps, all, entries, max_units, routed, sm_count, st);
+        return sp_choose<T, A, 4>(bt, maps, all, entries, max_units, routed, sm_count, st);
     };
     if (aln) return go(std::true_type{});
     if constexpr (T == GT_Q4_K || T == GT_Q5_K) return cudaErrorNotSupported;   // (144- and 176-byte blocks: only a misaligned base)
