@@ -76,6 +76,8 @@ bool qmv_split_supported(int ggml_type, const QmvArgs &a, int sm_count) {
 //   two rows
 //     Q4_0                        9.1 / 10.7              13.7 / 13.3    13.7 / 13.7    13.7 / 18.4    14.4 / 18.1    25.5 / 22.6
 //     Q8_0                        9.7 / 11.0              15.3 / 14.4    15.2 / 15.1    15.2 / 18.9    15.4 / 19.1    28.1 / 25.5
+//     wide, 4096 rows (0.86), one / two rows of Q6_K: 8192 values 13.2 / 13.0, 16.5 / 17.2, 12288 17.8 / 16.1, 23.9 / 21.0 (the others
+//     gain nothing: Q4_0 12.7 / 12.5, 16.8 / 17.4, Q8_0 13.7 / 13.5, 18.3 / 18.1)
 //   four rows  a mat-vec: 3072 rows 8.6 / 8.8, 4096 9.9 / 9.0, 12288 17.4 / 16.5 (Q4_0); 5120 x 5120 12.7 / 13.5, 4096 x 8192 13.7 / 15.5;
 //              several: 4096 + 1024 + 1024 rows (0.65) 11.7 / 10.7, twice 6144 (0.65) 15.8 / 16.6, twice 12288 (0.65) 30.1 / 25.7, twice 8192
 //              (0.86) 16.3 / 18.9.  Of different widths, 12288 x 2048 + 12288 x 4096: 19.9 / 22.4, one row of Q6_K 20.4 / 22.5
@@ -96,7 +98,7 @@ bool qmv_split_pays(int ggml_type, const QmvArgs *ops, int nops, double fill) {
     constexpr uint64_t M = 1u << 20;
     const bool q4k = ggml_type == GT_Q4_K;
     if (kmin != kmax) return false;   // (the other kernel deals out work by K stages, and its passes are fuller than `fill` says)
-    if (m <= 2) return fill <= 0.7 && values >= (q4k || (ggml_type == GT_Q4_0 && m == 2) ? 72 * M : 32 * M);
+    if (m <= 2) return fill <= (ggml_type == GT_Q6_K && kmax >= 10240 ? 0.9 : 0.7) && values >= (q4k || (ggml_type == GT_Q4_0 && m == 2) ? 72 * M : 32 * M);
     if (q4k && m <= 4) return kmax >= 4096 && values >= 14 * M && (fill <= 0.6 || (fill <= 0.7 && values >= 72 * M));
     if (q4k) return fill <= 0.6 && (m <= 8 || fill <= 0.25 || (m + 7) / 8 * 16 <= 3 * m);
     if (m > 4) return false;
