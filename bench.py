@@ -549,7 +549,7 @@ def run_ours(args, rank, world, local_rank):
         ach = step_algo_bytes / (ms * 1e-3) / 1e9
         return {"bound": "hbm", "achieved": ach, "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak,
                 "traffic": step_algo_bytes * ratio if ratio else None, "traffic_note": ratio_note, "peak_kind": f"{peak_kind} copy bandwidth",
-                "kernel": "qmv_mma_kernel (m <= 4 and the narrow shapes), qmv_tc_kernel + qmv_tc_pack_kernel, qmv_stream_kernel",
+                "kernel": "qmv_mma_kernel (m <= 4 and the narrow shapes), qmv_split_kernel + qmv_pack_kernel (where it is ahead in a chain), qmv_tc_kernel + qmv_tc_pack_kernel, qmv_stream_kernel",
                 "variant": variant, "ms_per_step": ms,
                 "note": "achieved = (weight + activation + output bytes of the 32 mat-vecs) / event-timed step"}
 

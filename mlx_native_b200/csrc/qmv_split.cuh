@@ -5,20 +5,23 @@
 //
 //  * The activations of a CTA stay in shared memory for all its weight rows: f16 hi + lo halves (scaled by a power of two per
 //    row, so that both stay in range), in the order of the B registers of mma.sync.m16n8k16.  One row is split by every CTA
-//    itself (2 us, less than another launch), several rows by qmv_pack_kernel, and arrive by bulk copies.  The loop over the
+//    itself, several rows by qmv_pack_kernel, and arrive by bulk copies (4096 x 4096 Q4_0: 7.2 us with one row, 8.8 with two).  The loop over the
 //    weights only unpacks codes into signed integers, as normal f16 numbers, so products are exact and sums are f32.
 //  * The 8 columns of an MMA are (activation row, hi | lo): one multiply serves up to four rows (NS = 2 sets: eight rows).
 //  * A warp works on up to four 16-row tiles at a time: one tile at a time leaves the pipes idle between dependent steps (Q4_0,
-//    75776 x 4096: 2.7 TB/s against 5.0).
+//    75776 x 4096: 70.7 us, 2.5 TB/s, against 44.9, 3.9 TB/s).
 //  * K may be split over the CTAs of a cluster (1, 2, 4, 8): a matrix of few rows still fills the chip, and long activation rows
 //    still fit into shared memory.  The ranks' partial sums travel through distributed shared memory (st.async) and are added in
 //    rank order by the CTA that owns the row: no atomics, results are bit-reproducible.
 //  * A producer warp fills a ring of stages (16-row tiles x SU units of 64 K values) by TMA: tensor copies where every weight row
-//    starts on a 16-byte boundary (ALN), else one bulk copy per row of the 16-byte superset of its segment, so every K that is a
-//    multiple of the block and every 2-byte aligned weight address takes this kernel (Q8_0 2873 x 2880, five rows: 11.7 us where
-//    the kernel that reads blocks from global memory took 181).
+//    starts on a 16-byte boundary (ALN), else one bulk copy per row of the 16-byte superset of its segment, so a K that is no
+//    multiple of 256 and a weight address that is even do for Q4_0, Q8_0 and Q6_K (Q8_0 2873 x 2880, five rows: 11.7 us where the
+//    kernel that reads blocks from global memory took 181).  Q4_K and Q5_K have to start on 16-byte boundaries.
 //  * Expert-routed: every CTA sorts the (token, slot) pairs by expert itself (at most 256 pairs), and the rows of one expert share
-//    a pass over its weights, four at a time.
+//    a pass over its weights, four at a time.  K is not split here.
+//
+// The activations in shared memory bound K: 133120 values for one row, 65536 for two, 30720 for up to four, 14336 for more; routed
+// 3840, and 16640 for a single pair (qmv_split_fits).  Beyond that the other mat-vec kernels take over.
 #pragma once
 #include "tensor_map.cuh"
 
@@ -439,8 +442,9 @@ template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const 
 }
 
 // A chunk of work: `nt` consecutive tiles of op `op` for entry `ent`, from the op's tile `tile` on.  Chunks are dealt out in runs:
-// cluster c takes the runs c, c + clusters, ..., so that at any time the whole chip reads one stretch of the weights (a
-// contiguous share per CTA keeps hundreds of distant pages open at once and ran at half the rate).
+// cluster c takes the runs c, c + clusters, ....  Runs of one spread what is left over in the last round evenly (768 chunks on 296
+// CTAs, Q8_0 24576 x 4096: 22.4 us, 28.5 with runs of two); where every CTA has as many chunks, runs make no difference (75776 x 4096,
+// four chunks each: 44.9 us in either order).
 struct SpChunk {
     uint32_t ent, op, tile, nt;
 };
@@ -1192,9 +1196,10 @@ template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool 
             if (tail + 2 * stage + 128 > kSpSmem) continue;
             const double slots = (double)((kSpSmem - 128 - tail) / stage);
             const double ncl = (double)(2 * sm_count / (int)c), chunks = ceil(ceil((double)tiles / tr) / ncl);
-            // Measured (12288 x 4096 and 4096 x 4096, all types): a chunk takes 1.9 us of waits and sums whatever its size, plus
+            // Fitted to 12288 x 4096 and 4096 x 4096, all types: a chunk takes 1.9 us of waits and sums whatever its size, plus
             // 0.23 us per tile and unit of a warp (Q6_K 0.3; two sets of columns 1.5 times that, and there four ranks wait for
-            // one another for 4.5 us a chunk).
+            // one another for 4.5 us a chunk).  Of 27 products (three types, one, four and eight rows, 4096 x 4096, 12288 x 4096 and
+            // 4096 x 12288) timed at every geometry, 21 take the fastest this way and the others one within 8 percent of it.
             const double unit = (T == GT_Q6_K ? 0.3 : 0.23) * (sets == 2 ? 1.5 : 1.0);
             // One row: splitting it takes 0.27 us per unit of a warp and CTA.
             const double cost = (packed ? 1.0 : 0.3 + 0.27 * ceil(slice / 8.0)) + chunks * ((sets == 2 && c == 4 ? 4.5 : 1.9) + tr * unit * ceil(slice / 8.0)) + (c > 1 ? 0.3 : 0.0) + (slots < 3 ? 0.3 : 0.0);
