@@ -80,6 +80,9 @@ struct SpOp {
     const float *xsum, *xinv;
     uint32_t pk_units;
     uint32_t row_end;         // rows to pack of the ops up to and including this one
+    // where the packed values of a row's super-block lie: bytes from one row and from one super-block to the next
+    uint64_t xp_row, xp_super;
+    uint32_t wide_rows;       // qmv_wide.cu: rows of a super-block; odd rows have lo before hi, sums are [super-block][row / 8][8][row % 8]
 };
 struct SpBatch {
     SpOp op[kSpMaxOps];
@@ -529,10 +532,15 @@ __global__ void __launch_bounds__(256) qmv_pack_kernel(const __grid_constant__ S
         sp::split(c[0], c[2], hi.x, lo.x);
         sp::split(c[1], c[3], hi.y, lo.y);
         if (u >= pk_units) return;
-        uint2 *d = reinterpret_cast<uint2 *>(xp + (row * pk_units + u) * 256u + (q >> 1) * 128u + tt * 32u + (q & 1u) * 8u);
-        d[0] = hi;
-        d[2] = lo;
-        if (NG != 0 && (tid & 7u) == 0) xsum[(row * pk_units + u) * NG + (q >> 1)] = sum;
+        uint2 *d = reinterpret_cast<uint2 *>(xp + row * P.xp_row + (u >> 2) * P.xp_super + (u & 3u) * 256u + (q >> 1) * 128u + tt * 32u + (q & 1u) * 8u);
+        const uint32_t odd = P.wide_rows ? row & 1u : 0u;
+        d[2 * odd] = hi;
+        d[2 - 2 * odd] = lo;
+        if (NG != 0 && (tid & 7u) == 0) {
+            const size_t at = P.wide_rows ? ((size_t)(u >> 2) * P.wide_rows + (row & ~7u)) * 8 + ((u & 3u) * 2 + (q >> 1)) * 8 + (row & 7u)
+                                          : (row * pk_units + u) * NG + (q >> 1);
+            xsum[at] = sum;
+        }
     };
 #pragma unroll
     for (int p = 0; p < HELD; p++) {
@@ -1268,6 +1276,9 @@ template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, 
         P.expert_stride = routed ? a.expert_stride : 0;
         P.xkey = (uint32_t)i;
         P.pk_units = (P.units + 3) & ~3u;
+        P.xp_row = P.pk_units * 256u;
+        P.xp_super = 1024;
+        P.wide_rows = 0;
         for (int q = 0; q < i; q++)
             if (ops[q].x == a.x && ops[q].x2 == a.x2 && ops[q].m == a.m && ops[q].k == a.k && ops[q].top_k == a.top_k) {
                 P.xkey = bt.op[q].xkey;

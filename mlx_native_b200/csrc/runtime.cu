@@ -42,6 +42,10 @@ double qmv_mma_fill(int ggml_type, const QmvArgs *ops, int nops, int sm_count);
 constexpr size_t kMvSplitMax = 8;    // mat-vecs one launch of the split kernel carries (kSpMaxOps)
 size_t qmv_split_scratch_bytes(const QmvArgs *ops, int nops);
 cudaError_t launch_qmv_split(int ggml_type, const QmvArgs *ops, int nops, int sm_count, uint8_t *scratch, int *launches, cudaStream_t st);
+bool qmv_wide_supported(int ggml_type, const QmvArgs &a);
+bool qmv_wide_pays(const QmvArgs &a, double fill);
+size_t qmv_wide_scratch_bytes(const QmvArgs *ops, int nops);
+cudaError_t launch_qmv_wide(const QmvArgs *ops, int nops, int sm_count, uint8_t *scratch, int *launches, cudaStream_t st);
 cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t nt, uint8_t *scratch, cudaStream_t st,
                           int *launches);
 cudaError_t launch_qmm_simt(int ggml_type, const QmmArgs &a, bool routed, uint32_t max_rows, cudaStream_t st);
@@ -307,6 +311,7 @@ struct mlxn_encoder {
     uint32_t pend_mp = 0;
     bool pend_pair = false;
     bool pend_split = false;          // they are mat-vecs of the split kernel (qmv_split.cuh)
+    bool pend_wide = false;           // ... or (pend_split too) of the one for many rows (qmv_wide.cu)
     bool grp_pend_only = false;       // every operation of the current group is in `pend` (none has been launched yet)
 };
 
@@ -941,7 +946,12 @@ static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
         for (const QmvArgs &a : e->pend)
             split = split && !a.after_earlier && qmv_split_supported(e->pend_type, a, e->dev->sm_count);
     }
-    if (split) {
+    if (e->pend_split && e->pend_wide) {
+        uint8_t *scratch = nullptr;
+        if ((rc = encoder_scratch_on(e, e->pend_lane, qmv_wide_scratch_bytes(e->pend.data(), (int)e->pend.size()), &scratch)) == MLXN_OK)
+            err = launch_qmv_wide(e->pend.data(), (int)e->pend.size(), e->dev->sm_count, scratch, &launches, st);
+        g_last_kernel = "qmv_wide";
+    } else if (split) {
         uint8_t *scratch = nullptr;
         const size_t need = qmv_split_scratch_bytes(e->pend.data(), (int)e->pend.size());
         if (!need || (rc = encoder_scratch_on(e, e->pend_lane, need, &scratch)) == MLXN_OK)
@@ -1552,11 +1562,11 @@ struct ShardOut {            // row-sharded output: see QmvArgs
     float *peer[kMaxPeers] = {};
 };
 // Adds mat-vecs to the encoder's open batch (launching it first where the new one does not fit in), as operation over `bufs`.
-static int batch_mv(mlxn_encoder *enc, int type, const QmvArgs &a, uint32_t mp, bool other_rows, std::initializer_list<OpBuf> bufs) {
+static int batch_mv(mlxn_encoder *enc, int type, const QmvArgs &a, uint32_t mp, bool other_rows, std::initializer_list<OpBuf> bufs, bool wide = false) {
     const bool batch = g_opt_mv_batch.load() != 0;
     const QmvArgs *h = enc->pend.empty() ? nullptr : &enc->pend[0];
     // (routed ones share the launch's bucketing: the same pairs of the same experts)
-    const bool fits = batch && h && enc->pend_split && enc->pend_type == type && enc->pend_mp == mp && enc->pend_pair == other_rows &&
+    const bool fits = batch && h && enc->pend_split && enc->pend_wide == wide && enc->pend_type == type && enc->pend_mp == mp && enc->pend_pair == other_rows &&
                       enc->pend.size() < kMvSplitMax && h->ids == a.ids && h->nprob == a.nprob && h->n_experts == a.n_experts &&
                       (a.ids ? h->k == a.k : a.m <= 8 || h->m == a.m);
     int rc;
@@ -1567,6 +1577,7 @@ static int batch_mv(mlxn_encoder *enc, int type, const QmvArgs &a, uint32_t mp, 
         enc->pend_mp = mp;
         enc->pend_pair = other_rows;
         enc->pend_split = true;
+        enc->pend_wide = wide;
         enc->pend_lane = enc->cur_lane;
     }
     enc->pend.push_back(a);
@@ -1628,6 +1639,8 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
         const double fill = t == GT_Q4_K ? qmv_mma_fill(t, &a, 1, dev->sm_count) : 0.0;   // (of one group of eight rows)
         a.m = p->m;
         const bool aligned = qmv_split_aligned(t, a);
+        if (mode == 3 && p->m > 8 && !sh && qmv_wide_supported(t, a) && qmv_wide_pays(a, fill))
+            return batch_mv(enc, t, a, 16u, false, {{input, false}, {weight, false}, {output, true}}, true);
         const bool pays = mode == 5 || (!aligned ? t != GT_Q6_K || (p->m > 2 && !qmv_mma_pair_mode(t, a))
                                                  : p->m > 8 && t == GT_Q4_K && qmv_split_pays(t, &a, 1, fill));
         if (pays && (p->m <= 8 || !sh) && qmv_split_supported(t, a, dev->sm_count))
