@@ -286,8 +286,10 @@ struct mlxn_encoder {
     // inputs whose host shadow was uploaded inside the group (the whole storage is copied), with the lane the copy went
     // to: a write for the other lanes, but an operation that runs on the same lane comes after the copy anyway
     std::vector<std::pair<const void *, int>> grp_uploads;
-    bool grp_open = false;           // ev_fork marks the start of the current group
-    cudaEvent_t ev_start = nullptr, ev_end = nullptr;
+    bool grp_forked = false;         // ev_fork marks the start of the current group
+    cudaEvent_t ev_start = nullptr, ev_end = nullptr;   // with time stamps, of a command buffer whose GPU time is asked for
+    cudaEvent_t ev_done = nullptr;   // the end of any other: without a time stamp it reaches the host 4 us earlier
+    cudaEvent_t ev_last = nullptr;   // the one that the last commit recorded
     bool started = false, committed = false, capturing = false;
     uint64_t cap_launch0 = 0, cap_dispatch0 = 0;
     std::vector<mlxn_buffer *> retained;
@@ -801,6 +803,7 @@ extern "C" int mlxn_encoder_create(mlxn_device *dev, mlxn_encoder **out) {
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming);
     if (err == cudaSuccess) err = cudaEventCreate(&e->ev_start);
     if (err == cudaSuccess) err = cudaEventCreate(&e->ev_end);
+    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->ev_done, cudaEventDisableTiming);
     // zero-initialised words that the blocks of a kernel hand work over with, and the status word
     if (err == cudaSuccess) err = cudaMalloc((void **)&e->status_dev, kStatusBlockBytes);
     if (err == cudaSuccess) err = cudaMemset(e->status_dev, 0, kStatusBlockBytes);
@@ -827,6 +830,7 @@ extern "C" int mlxn_encoder_create(mlxn_device *dev, mlxn_encoder **out) {
         if (e->ev_aux_join) cudaEventDestroy(e->ev_aux_join);
         if (e->ev_start) cudaEventDestroy(e->ev_start);
         if (e->ev_end) cudaEventDestroy(e->ev_end);
+        if (e->ev_done) cudaEventDestroy(e->ev_done);
         if (e->sb) status_block_release(e->sb);
         else if (e->status_dev) cudaFree(e->status_dev);
         delete e;
@@ -873,7 +877,7 @@ extern "C" void mlxn_encoder_destroy(mlxn_encoder *enc) {
         enc->grp_reads.clear();
         enc->grp_writes.clear();
         enc->grp_uploads.clear();
-        enc->grp_open = false;
+        enc->grp_forked = false;
         if (*enc->status_host != 0) {
             *enc->status_host = 0;
             cudaMemset(enc->status_dev, 0, kStatusBlockBytes);
@@ -893,6 +897,7 @@ extern "C" void mlxn_encoder_destroy(mlxn_encoder *enc) {
     status_block_release(enc->sb);
     cudaEventDestroy(enc->ev_start);
     cudaEventDestroy(enc->ev_end);
+    cudaEventDestroy(enc->ev_done);
     cudaEventDestroy(enc->ev_fork);
     cudaEventDestroy(enc->ev_aux);
     cudaEventDestroy(enc->ev_aux_join);
@@ -918,9 +923,22 @@ extern "C" void *mlxn_encoder_stream(mlxn_encoder *enc) {
 // operation starts a new group on lane 0.
 static uint32_t mv_row_class(uint32_t m) { return m <= 1 ? 1u : m <= 2 ? 2u : m <= 4 ? 4u : 8u; }
 static int encoder_scratch_on(mlxn_encoder *e, int lane, size_t bytes, uint8_t **out);
+// Marks what the other lane has to wait for before it takes work of the current group: everything ahead of the group.  Done before the
+// first launch of the group, and not at all for a group that is one batch of mat-vecs: a record between two kernels keeps the second
+// from being launched while the first one ends (see launch_overlapped), 2 us for each of the five groups of a decoder layer.
+static int encoder_mark_fork(mlxn_encoder *e) {
+    if (e->grp_forked) return MLXN_OK;
+    CUDA_TRY(cudaEventRecord(e->ev_fork, e->lanes[0]), "event record");
+    e->grp_forked = true;
+    return MLXN_OK;
+}
 static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
     if (e->pend.empty()) return MLXN_OK;
     cudaSetDevice(e->ordinal);
+    if (!group_ends) {
+        const int frc = encoder_mark_fork(e);
+        if (frc) return frc;
+    }
     cudaStream_t st = e->lanes[e->pend_lane];
     cudaError_t err = cudaSuccess;
     int launches = 1, rc = MLXN_OK;
@@ -1015,7 +1033,7 @@ static int encoder_join_lanes(mlxn_encoder *e) {
     e->grp_reads.clear();
     e->grp_writes.clear();
     e->grp_uploads.clear();
-    e->grp_open = false;
+    e->grp_forked = false;
     e->cur_lane = 0;
     e->stream = e->lanes[0];
     return MLXN_OK;
@@ -1038,7 +1056,7 @@ static int encoder_begin_work(mlxn_encoder *e) {
     return MLXN_OK;
 }
 
-extern "C" int mlxn_encoder_commit(mlxn_encoder *enc) {
+static int encoder_commit(mlxn_encoder *enc, bool timed) {
     if (!enc) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: encoder must not be null");
     if (enc->capturing) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: commit while a capture is open");
     cudaSetDevice(enc->ordinal);
@@ -1060,10 +1078,12 @@ extern "C" int mlxn_encoder_commit(mlxn_encoder *enc) {
             st->has_last = true;
         }
     }
-    CUDA_TRY(cudaEventRecord(enc->ev_end, enc->lanes[0]), "event record");
+    enc->ev_last = timed ? enc->ev_end : enc->ev_done;
+    CUDA_TRY(cudaEventRecord(enc->ev_last, enc->lanes[0]), "event record");
     enc->committed = true;
     return MLXN_OK;
 }
+extern "C" int mlxn_encoder_commit(mlxn_encoder *enc) { return encoder_commit(enc, false); }
 
 static const char *status_text(uint32_t s) {
     switch (s) {
@@ -1083,7 +1103,7 @@ extern "C" int mlxn_encoder_wait_until_completed(mlxn_encoder *enc) {
     g_sync.fetch_add(1);
     cudaError_t e = cudaSuccess;
     if (enc->committed) {
-        e = cudaEventSynchronize(enc->ev_end);
+        e = cudaEventSynchronize(enc->ev_last);
     } else {
         (void)encoder_flush_pending(enc);
         e = cudaStreamSynchronize(enc->aux);
@@ -1109,7 +1129,7 @@ extern "C" int mlxn_encoder_commit_and_wait(mlxn_encoder *enc) {
 }
 
 extern "C" int mlxn_encoder_commit_wait_with_gpu_time(mlxn_encoder *enc, double *gpu_seconds) {
-    int rc = mlxn_encoder_commit(enc);
+    int rc = encoder_commit(enc, true);
     if (rc) return rc;
     rc = mlxn_encoder_wait_until_completed(enc);
     if (rc) return rc;
@@ -1418,10 +1438,7 @@ static int op_begin(mlxn_encoder *e, std::initializer_list<OpBuf> bufs, bool joi
     const bool first = e->grp_reads.empty() && e->grp_writes.empty();
     e->grp_pend_only = joins_batch && (first || e->grp_pend_only);
     const int lane = op_lane(e, joins_batch);
-    if (!e->grp_open) {
-        CUDA_TRY(cudaEventRecord(e->ev_fork, e->lanes[0]), "event record");  // everything before this group
-        e->grp_open = true;
-    }
+    if ((!joins_batch || lane != 0) && (rc = encoder_mark_fork(e))) return rc;
     if (lane != 0 && !e->lane_busy[lane]) {
         CUDA_TRY(cudaStreamWaitEvent(e->lanes[lane], e->ev_fork, 0), "stream wait");
         e->lane_busy[lane] = true;
