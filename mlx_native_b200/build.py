@@ -13,8 +13,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmlxn_b200.so")
 SOURCES = ["runtime.cu", "qmv.cu", "qmv_tc.cu", "qmv_mma.cu", "qmv_split.cu", "qmv_split_q4_0.cu", "qmv_split_q8_0.cu",
-           "qmv_split_q4_k.cu", "qmv_split_q5_k.cu", "qmv_split_q6_k.cu", "qmv_wide.cu", "qmm.cu", "moe.cu"]
-HEADERS = ["common.cuh", "mma_f16.cuh", "ptx.cuh", "qmv_split.cuh", "tensor_map.cuh", os.path.join("..", "..", "include", "mlxn_b200.h")]
+           "qmv_split_q4_k.cu", "qmv_split_q5_k.cu", "qmv_split_q6_k.cu", "qmv_wide.cu", "qmm.cu", "qmm_duo.cu", "moe.cu"]
+HEADERS = ["common.cuh", "dequant.cuh", "qmm.cuh", "mma_f16.cuh", "ptx.cuh", "qmv_split.cuh", "tensor_map.cuh", os.path.join("..", "..", "include", "mlxn_b200.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC",

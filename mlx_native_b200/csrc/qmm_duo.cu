@@ -1,0 +1,518 @@
+// Dense mat-mat of many activation rows on pairs of SMs: y[m, n] = x[m, k] . W[n, k]^T, weights dequantised on the way.
+//
+// The kernel of qmm.cu gives every SM a tile of 128 weight rows and up to 256 activation rows.  At 256 its tensor core is held up by
+// shared memory: it reads the activation tile (8 KB) for every 16 K values, the bulk copies write as much, and the raw weights come on
+// top -- 1070 cycles for 64 K values where the multiplication needs 410.  Here two SMs work on one tile of 256 weight rows
+// (tcgen05 cta_group::2): each dequantises its own 128 rows into its own tensor memory and holds half of the activation tile, which the
+// hardware reads from both.  Operand semantics as in qmm.cu: exact weights rounded once to f16, activations f32 -> f16, f32 sums.
+//
+// What else was tried: unpacking the weights once into f16 tiles, by a kernel of its own.  The product alone then runs at the
+// multiplication's rate, but the unpacking is bound by memory (13 us for 4096 x 4096, 58 with 2048 rows of 12288 for 4096 x 12288): 32.2 us in
+// all for 512 x 4096 x 4096, 72.8 for 512 x 12288 x 4096.
+#include <cuda_fp16.h>
+
+#include <atomic>
+
+#include "common.cuh"
+#include "dequant.cuh"
+#include "ptx.cuh"
+#include "qmm.cuh"
+#include "tensor_map.cuh"
+
+namespace mlxn {
+
+constexpr uint32_t kDuoRows = 256;                          // weight rows of a pair's tile
+constexpr uint32_t kDuoDequantWarps = 16;                   // two sets of eight; set s takes the 128-wide K stages st % 2 == s
+constexpr uint32_t kDuoThreads = (4 + kDuoDequantWarps) * 32;
+constexpr uint32_t kDuoStages = 4;                          // ring of K stages: activations in shared memory, weights in tensor memory
+constexpr uint32_t kDuoACol = 256, kDuoACols = 64;          // tensor-memory columns of the weights: 64 a stage (128 f16 pairs)
+constexpr uint32_t kDuoMaxRaw = 5;
+
+struct DuoCfg {
+    uint32_t nchunks;     // ceil(k / 64)
+    uint32_t nt;          // activation rows of a tile (a multiple of 32, at most 256)
+    uint32_t n_wt, ntiles;
+    uint32_t pairs;
+    TcShare share;        // the pairs' ranges where tiles are shared
+    uint32_t seg_stride;  // bytes of a raw row segment in shared memory
+    uint32_t raw_off, raw_slots;
+    uint32_t row_group;   // log2 of the copies of a raw stage (see launch_tc_tn)
+    uint32_t aligned;     // every weight row starts on a 16-byte boundary
+};
+
+namespace duo {
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool elect() {
+    uint32_t p = 0;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\t@p mov.u32 %0, 1;\n\t}" : "+r"(p));
+    return p != 0;
+}
+// Arrives on the barrier at the same place in CTA 0.  Without release: what it announces are finished copies and tensor-memory stores,
+// no stores of this thread (with it the instruction takes a thousand cycles, which then bounded the whole kernel).
+__device__ __forceinline__ void arrive_at_0(uint64_t *bar) {
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\t"
+        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ void alloc(uint32_t *dst, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(cols) : "memory");
+}
+__device__ __forceinline__ void relinquish() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void dealloc(uint32_t addr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
+}
+// D (+)= A B^T of the pair: A in the tensor memory of both CTAs (128 rows each), B's halves in their shared memory
+__device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// arrives on the barrier at this place in both CTAs once the MMAs issued so far have completed
+__device__ __forceinline__ void commit_both(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"((uint16_t)3)
+                 : "memory");
+}
+}  // namespace duo
+
+// Clusters of two CTAs, one CTA per SM, persistent.  Per CTA:
+//   warp 0        activations: one bulk copy per K stage (two 64-wide chunks of its half of the tile)
+//   warp 1        CTA 0: MMAs of the pair, whose completion frees the stage's places in both CTAs; CTA 1: tells CTA 0 that its stage is ready
+//   warp 2        raw weights: tensor copies of 128 rows x 256 K values
+//   warps 4..19   dequantise raw blocks into tensor memory; read the accumulator back
+// Ring places and barrier phases run on across the items of a pair.
+template <int T>
+__global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
+    qmm_duo_kernel(const QmmArgs a, const DuoCfg c, const uint8_t *xpack, const __grid_constant__ CUtensorMap wmap) {
+    constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
+    constexpr uint32_t KR = 256;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // (the same in both CTAs)
+    __shared__ __align__(8) uint64_t full[kDuoStages], peer_full[kDuoStages], done[kDuoStages], raw_full[kDuoMaxRaw], raw_empty[kDuoMaxRaw];
+    __shared__ __align__(8) uint64_t acc_full, acc_empty;
+    __shared__ uint32_t tmem_s;
+    __shared__ volatile uint32_t abort_flag;
+    const uint32_t lane = threadIdx.x & 31u, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const uint32_t rank = duo::cluster_rank(), pair = blockIdx.x >> 1;
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (uint32_t s = 0; s < kDuoStages; s++) {
+            mbar_init(&full[s], 9);   // the activations' copy, and the eight warps of a set
+            mbar_init(&peer_full[s], 1);
+            mbar_init(&done[s], 1);
+        }
+        for (uint32_t s = 0; s < c.raw_slots; s++) {
+            mbar_init(&raw_full[s], 1);
+            mbar_init(&raw_empty[s], kDuoDequantWarps);
+        }
+        mbar_init(&acc_full, 1);
+        mbar_init(&acc_empty, 2 * kDuoDequantWarps);   // (of CTA 0: the warps of both)
+        mbar_init_fence();
+    }
+    if (warp == 3) {
+        duo::alloc(&tmem_s, 512);
+        duo::relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    duo::cluster_sync();
+    tc_fence_after();
+    const uint32_t tmem = tmem_s;
+    grid_dependency_wait();   // the packed activations and the zeros of shared tiles are complete
+    allow_dependents();
+
+    // ---- work items: weight tile fastest, so that the pairs working at the same time share an activation tile in L2 ----
+    const uint32_t nraw_all = (a.k + KR - 1) / KR, total_items = c.n_wt * c.ntiles;
+    const bool shared = c.share.ctas != 0;
+    const uint32_t pos0 = shared ? c.share.begin(pair) : pair, pos1 = shared ? c.share.begin(pair + 1) : total_items;
+    struct Item {
+        uint32_t tt, n0, r_lo, nraw, nst, kc_lo, nck, next;
+    };
+    auto load_item = [&](uint32_t pos) {
+        Item it;
+        const uint32_t item = shared ? pos / nraw_all : pos;
+        it.r_lo = shared ? pos - item * nraw_all : 0u;
+        const uint32_t r_hi = shared ? min(nraw_all, it.r_lo + (pos1 - pos)) : nraw_all;
+        it.next = shared ? pos + (r_hi - it.r_lo) : pos + c.pairs;
+        it.tt = item / c.n_wt;
+        it.n0 = (item - it.tt * c.n_wt) * kDuoRows + rank * 128u;
+        it.nraw = r_hi - it.r_lo;
+        it.kc_lo = it.r_lo * (KR / 64);
+        it.nst = min((a.k + 127) / 128, r_hi * (KR / 128)) - it.r_lo * (KR / 128);   // K stages of 128
+        it.nck = min(c.nchunks, r_hi * (KR / 64)) - it.kc_lo;                         // 64-wide chunks
+        return it;
+    };
+    const uint32_t h = c.nt / 2, b_chunk = h * 128u, b_stage = 2 * b_chunk;
+    const uint32_t smem_base = smem_u32(smem), raw_bytes = 128u * c.seg_stride;
+    constexpr uint32_t kSpin = 0xFFFFFFFFu;
+    bool ok = true;
+
+    if (warp == 0) {
+        uint32_t s = 0, ph = 1;   // (a place's first wait passes)
+        for (uint32_t pos = pos0; ok && pos < pos1;) {
+            const Item it = load_item(pos);
+            pos = it.next;
+            const uint8_t *src = xpack + ((size_t)(it.tt * 2u + rank) * c.nchunks + it.kc_lo) * b_chunk;
+            for (uint32_t st = 0; st < it.nst; st++, src += b_stage) {
+                if (!mbar_wait(&done[s], ph, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, kSpin)) {
+                    ok = false;
+                    break;
+                }
+                if (duo::elect()) {
+                    const uint32_t bytes = 2 * st + 1 < it.nck ? b_stage : b_chunk;   // (a K tail of 64)
+                    mbar_expect_tx(&full[s], bytes);
+                    bulk_g2s(smem + s * b_stage, src, bytes, &full[s]);
+                }
+                __syncwarp();
+                if (++s == kDuoStages) {
+                    s = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = umma_idesc_f16(kDuoRows, c.nt);
+        const uint64_t bd0 = umma_desc_k_sw128(smem_base);
+        uint32_t s = 0, ph = 0, nitem = 0;
+        for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
+            const Item it = load_item(pos);
+            pos = it.next;
+            // the accumulator of the item before has been read back
+            if (rank == 0 && nitem > 0 && !mbar_wait(&acc_empty, (nitem - 1) & 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, kSpin)) break;
+            tc_fence_after();
+            for (uint32_t st = 0; st < it.nst; st++) {
+                if (!mbar_wait(&full[s], ph, &abort_flag, a.status, ST_WAIT_FULL_TIMEOUT, kSpin)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                if (rank == 0) {
+                    if (!mbar_wait(&peer_full[s], ph, &abort_flag, a.status, ST_WAIT_FULL_TIMEOUT, kSpin)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    if (duo::elect()) {
+                        const uint32_t ac = tmem + kDuoACol + s * kDuoACols;
+                        const uint64_t bd = bd0 + s * (b_stage >> 4), bd1 = bd + (b_chunk >> 4);
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; q++) duo::mma(tmem, ac + 8 * q, bd + 2 * q, idesc, (st | q) ? 1u : 0u);
+                        if (2 * st + 1 < it.nck) {
+#pragma unroll
+                            for (uint32_t q = 0; q < 4; q++) duo::mma(tmem, ac + 32 + 8 * q, bd1 + 2 * q, idesc, 1u);
+                        }
+                        duo::commit_both(&done[s]);
+                    }
+                } else {
+                    tc_fence_before();
+                    if (duo::elect()) duo::arrive_at_0(&peer_full[s]);
+                }
+                __syncwarp();
+                if (++s == kDuoStages) {
+                    s = 0;
+                    ph ^= 1u;
+                }
+            }
+            if (!ok) break;
+            if (rank == 0 && duo::elect()) duo::commit_both(&acc_full);
+            __syncwarp();
+        }
+    } else if (warp == 2) {
+        // (see qmm.cu: a map row is a group of 1, 2, 4 or 8 weight rows that starts on a 16-byte boundary; one copy brings a row of every group)
+        const uint32_t row_bytes = (a.k / QK) * BB;
+        uint32_t slot = 0, ph = 1;
+        for (uint32_t pos = pos0; ok && pos < pos1;) {
+            const Item it = load_item(pos);
+            pos = it.next;
+            for (uint32_t r = 0; r < it.nraw; r++) {
+                if (!mbar_wait(&raw_empty[slot], ph, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, kSpin)) {
+                    ok = false;
+                    break;
+                }
+                if (duo::elect()) {
+                    const uint32_t kb = (it.r_lo + r) * (KR / QK) * BB;
+                    mbar_expect_tx(&raw_full[slot], raw_bytes);
+                    for (uint32_t i = 0; i < 1u << c.row_group; i++)
+                        asm volatile(
+                            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                                smem_base + c.raw_off + slot * raw_bytes + i * (raw_bytes >> c.row_group)),
+                            "l"(&wmap), "r"(((i * row_bytes + kb) & ~15u) >> 2), "r"(it.n0 >> c.row_group), "r"(smem_u32(&raw_full[slot]))
+                            : "memory");
+                }
+                __syncwarp();
+                if (++slot == c.raw_slots) {
+                    slot = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+    } else if (warp >= 4) {
+        // thread (warp w, lane l) of a set owns weight row 32 (w % 4) + l, the tensor-memory lane it may address, and the 64-element half
+        // (w / 4) % 2 of the K stage: 32 packed f16 pairs = one 32-column store
+        const uint32_t dw = warp - 4, q4 = dw & 3u, half = (dw >> 2) & 1u, set = dw >> 3, g = dw >> 2;
+        const uint32_t rr = q4 * 32 + lane;
+        const uint32_t srow = ((rr & ((1u << c.row_group) - 1u)) << (7 - c.row_group)) + (rr >> c.row_group);   // the row's place in a raw stage
+        const uint32_t a_dst = tmem + ((q4 * 32) << 16) + kDuoACol + 32 * half;
+        const uint32_t row_bytes = (a.k / QK) * BB;
+        uint32_t rs = 0, rph = 0, J0 = 0, nitem = 0;
+        for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
+            const Item it = load_item(pos);
+            pos = it.next;
+            const bool row_ok = it.n0 + rr < a.n;
+            const uint32_t row_lo4 = (uint32_t)((uintptr_t)(a.w + (size_t)(it.n0 + rr) * row_bytes) & 15u);
+            for (uint32_t r = 0; r < it.nraw; r++) {
+                if (!mbar_wait(&raw_full[rs], rph, &abort_flag, a.status, ST_WAIT_FULL_TIMEOUT, 0u)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t st = 2 * r + set;
+                if (st < it.nst) {
+                    const uint32_t J = J0 + st, sa = J % kDuoStages;   // (J: the stage's number in the pair's whole run)
+                    const uint32_t r_abs = it.r_lo + r, stage_row = smem_base + c.raw_off + rs * raw_bytes + srow * c.seg_stride;
+                    uint32_t regs[32];
+                    if (c.aligned && row_ok) {
+                        if constexpr (T == GT_Q6_K) {
+                            dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half, regs);
+                            dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half + 1, regs + 16);
+                        } else {
+                            switch (2 * set + half) {  // uniform per warp
+                            case 0: dequant64_aligned<T, 0>(stage_row, regs); break;
+                            case 1: dequant64_aligned<T, 1>(stage_row, regs); break;
+                            case 2: dequant64_aligned<T, 2>(stage_row, regs); break;
+                            default: dequant64_aligned<T, 3>(stage_row, regs); break;
+                            }
+                        }
+                    } else {
+                        const uint32_t seg = stage_row + ((row_lo4 + ((r_abs * KR) / QK) * BB) & 15u);
+#pragma unroll
+                        for (uint32_t hh = 0; hh < 2; hh++) {
+                            uint4 v[4];
+                            const uint32_t e0 = 128 * set + 64 * half + 32 * hh;
+                            if (row_ok && r_abs * KR + e0 < a.k) {
+                                dequant32<T>(seg, e0, v);
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < 4; i++) v[i] = make_uint4(0, 0, 0, 0);
+                            }
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                regs[16 * hh + 4 * i + 0] = v[i].x;
+                                regs[16 * hh + 4 * i + 1] = v[i].y;
+                                regs[16 * hh + 4 * i + 2] = v[i].z;
+                                regs[16 * hh + 4 * i + 3] = v[i].w;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&raw_empty[rs]);   // this warp is done reading the raw stage
+                    // the MMAs that read this place's previous contents (stage J - 4) have completed
+                    if (J >= kDuoStages && !mbar_wait(&done[sa], ((J / kDuoStages) & 1u) ^ 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, 0u)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    tmem_st_32x32_x32(a_dst + sa * kDuoACols, regs);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&full[sa]);
+                } else {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&raw_empty[rs]);
+                }
+                if (++rs == c.raw_slots) {
+                    rs = 0;
+                    rph ^= 1u;
+                }
+            }
+            if (!ok) break;
+            J0 += it.nst;
+            // ---- read-back: lane = weight row, 32 activation rows at a time ----
+            if (!mbar_wait(&acc_full, nitem & 1u, &abort_flag, a.status, ST_WAIT_MMA_TIMEOUT, 0u)) break;
+            tc_fence_after();
+            const bool some = it.nraw < nraw_all;   // another pair has the rest of this tile's K
+#pragma unroll 1
+            for (uint32_t col = g * 32; col < c.nt; col += kDuoDequantWarps / 4 * 32) {
+                uint32_t v[32];
+                tmem_ld_32x32(tmem + ((q4 * 32) << 16) + col, v);
+                tmem_ld_wait();
+                const uint32_t o0 = it.tt * c.nt + col;
+                if (row_ok && o0 < a.m) {
+                    float *y = a.y + (size_t)o0 * a.n + it.n0 + rr;
+                    const uint32_t cnt = min(32u, a.m - o0);
+                    if (some) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; j++)
+                            if (j < cnt) atomicAdd(y + (size_t)j * a.n, __uint_as_float(v[j]));
+                    } else {
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; j++)
+                            if (j < cnt) y[(size_t)j * a.n] = __uint_as_float(v[j]);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) duo::arrive_at_0(&acc_empty);   // the MMA warp may start the next item's accumulation
+        }
+    }
+    __syncwarp();
+    if (abort_flag)   // let copies in flight land before the shared memory is released
+        for (int i = 0; i < 200; i++) __nanosleep(5000);
+    tc_fence_before();
+    __syncthreads();
+    duo::cluster_sync();   // nobody leaves while the other may still arrive here, or while the pair's MMAs read here
+    if (warp == 3) {
+        tc_fence_after();
+        duo::dealloc(tmem, 512);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// host side
+// ------------------------------------------------------------------------------------------------
+// Pairs of SMs that hold a cluster at the same time.
+static uint32_t duo_pairs() {
+    static std::atomic<uint32_t> known[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint32_t most = (uint32_t)sm_count_of_device() / 2;
+    if (dev < 0 || dev >= 64) return most;
+    uint32_t v = known[dev].load(std::memory_order_acquire);
+    if (!v) {
+        int n = 0;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(most * 2);
+        cfg.blockDim = dim3(kDuoThreads);
+        cfg.dynamicSmemBytes = 223 * 1024;
+        if (cudaFuncSetAttribute(qmm_duo_kernel<GT_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, qmm_duo_kernel<GT_Q4_0>, &cfg) != cudaSuccess || n < 1 || n > (int)most) {
+            (void)cudaGetLastError();
+            n = (int)most;
+        }
+        v = (uint32_t)n;
+        known[dev].store(v, std::memory_order_release);
+    }
+    return v;
+}
+
+struct DuoPlan {
+    uint32_t pairs, shared;
+};
+// Cost in the units of tc_plan (1.74 ns).  Measured: a K stage of 128 values takes 0.47 us where dequantising bounds it (Q6_K 0.66), else
+// 0.165 us + 2.3 ns per activation row; an item 1 us beside its stages.  Tiles shared by two pairs are zeroed and added up: 3 us and more for
+// wide ones (every tile in halves), 5 us where ranges are shared.
+static uint64_t duo_plan(int type, uint64_t m, uint64_t n, uint64_t k, uint32_t nt, DuoPlan &p) {
+    const uint64_t sms = duo_pairs(), nraw = (k + 255) / 256, tiles = (n + kDuoRows - 1) / kDuoRows * ((m + nt - 1) / nt);
+    const uint64_t convert = type == GT_Q6_K ? 380 : 270, multiply = 95 + nt * 13 / 10, tile = 2 * nraw * (convert > multiply ? convert : multiply);
+    uint64_t best = (tiles + sms - 1) / sms * (tile + 400) + 600;
+    p = {(uint32_t)(tiles < sms ? tiles : sms), 0};
+    if (tiles * nraw >= (1ull << 31)) return best;
+    if (tiles > sms && nraw >= 2) {
+        const uint64_t cost = tiles * tile / sms + (tiles / sms + 2) * 575 + 2900 + nt * 9;
+        if (cost < best) {
+            best = cost;
+            p = {(uint32_t)sms, 1};
+        }
+    } else if (2 * tiles <= sms && nraw >= 2) {
+        const uint64_t cost = tile / 2 + 2300 + nt * 12;
+        if (cost < best) {
+            best = cost;
+            p = {(uint32_t)(2 * tiles), 1};
+        }
+    }
+    return best;
+}
+
+static int duo_row_group(uint32_t row_bytes) {
+    int lg = 0;
+    while ((row_bytes << lg) & 15u) lg++;
+    return lg;
+}
+uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt) {
+    if (ggml_type != GT_Q4_0 && ggml_type != GT_Q8_0 && ggml_type != GT_Q6_K) return ~0ull;
+    if (a.hids || a.y_ld || a.n_peer || a.x2 || nt % 32 != 0 || nt > 256 || a.k % 32 != 0) return ~0ull;
+    const uint32_t row_bytes = (a.k / ggml_qk(ggml_type)) * ggml_block_bytes(ggml_type);
+    if (((uintptr_t)a.w & 15u) || a.n % (1u << duo_row_group(row_bytes)) != 0 || encode_tiled_fn() == nullptr) return ~0ull;
+    DuoPlan p;
+    return duo_plan(ggml_type, a.m, a.n, a.k, nt, p);
+}
+
+template <int T> static cudaError_t launch_duo_t(const QmmArgs &a, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {
+    constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
+    const uint32_t row_bytes = (a.k / QK) * BB, h = nt / 2;
+    DuoPlan p;
+    duo_plan(T, a.m, a.n, a.k, nt, p);
+    DuoCfg c{};
+    c.nt = nt;
+    c.nchunks = (a.k + 63) / 64;
+    c.n_wt = (a.n + kDuoRows - 1) / kDuoRows;
+    c.ntiles = (a.m + nt - 1) / nt;
+    c.pairs = p.pairs;
+    c.row_group = (uint32_t)duo_row_group(row_bytes);
+    c.aligned = row_bytes % 16 == 0 && a.k % 256 == 0;
+    constexpr uint32_t kSeg = 256 / QK * BB;
+    c.seg_stride = c.row_group == 0 && kSeg % 16 == 0 ? kSeg : ((kSeg + 14 + 15) / 16 | 1u) * 16;   // (an odd multiple of 16: see launch_tc_tn)
+    const uint32_t nraw = (a.k + 255) / 256;
+    if (p.shared) c.share = {p.pairs, c.n_wt, nraw, c.n_wt * c.ntiles * nraw, kDuoRows, nt};
+    alignas(64) CUtensorMap wmap;
+    {
+        EncodeTiledFn enc = encode_tiled_fn();
+        if (!enc) return cudaErrorNotSupported;
+        const uint32_t lg = c.row_group;
+        const cuuint64_t gdim[2] = {((uint64_t)row_bytes << lg) / 4, a.n >> lg};
+        const cuuint64_t gstride[1] = {(uint64_t)row_bytes << lg};
+        const cuuint32_t box[2] = {c.seg_stride / 4, 128u >> lg}, estr[2] = {1, 1};
+        if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t *>(a.w), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    const uint32_t limit = 222 * 1024, b_bytes = kDuoStages * nt * 128u, raw_slot = 128 * c.seg_stride;
+    c.raw_off = b_bytes;
+    c.raw_slots = (limit - b_bytes) / raw_slot;
+    if (c.raw_slots > kDuoMaxRaw) c.raw_slots = kDuoMaxRaw;
+    if (c.raw_slots < 2) return cudaErrorInvalidConfiguration;
+    const size_t smem = (size_t)b_bytes + c.raw_slots * raw_slot + 1024;
+    // activations in tiles of nt / 2 rows: a CTA's half of a tile
+    {
+        const uint32_t tiles = 2 * c.ntiles;
+        uint32_t lanes = c.nchunks;
+        const uint64_t slices = (uint64_t)tiles * ((h + kPackRows - 1) / kPackRows);
+        while (lanes > 1 && (uint64_t)lanes * slices > 2048) lanes = (lanes + 1) / 2;
+        pack_x_kernel<<<dim3((unsigned)slices, lanes), 256, 0, st>>>(a, xpack, c.nchunks, h, c.share);
+        (*launches)++;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    static std::atomic<uint32_t> prepared[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!prepared[dev].load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(qmm_duo_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024);
+        if (e != cudaSuccess) return e;
+        prepared[dev].store(1, std::memory_order_release);
+    }
+    (*launches)++;
+    return launch_overlapped(qmm_duo_kernel<T>, dim3(2 * c.pairs), dim3(kDuoThreads), smem, st, a, c, (const uint8_t *)xpack, wmap);
+}
+
+cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs &a, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {
+    switch (ggml_type) {
+    case GT_Q4_0: return launch_duo_t<GT_Q4_0>(a, nt, xpack, st, launches);
+    case GT_Q8_0: return launch_duo_t<GT_Q8_0>(a, nt, xpack, st, launches);
+    case GT_Q6_K: return launch_duo_t<GT_Q6_K>(a, nt, xpack, st, launches);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace mlxn

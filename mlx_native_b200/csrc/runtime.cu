@@ -50,8 +50,9 @@ cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t
                           int *launches);
 cudaError_t launch_qmm_simt(int ggml_type, const QmmArgs &a, bool routed, uint32_t max_rows, cudaStream_t st);
 size_t qmm_tc_scratch_bytes(const QmmArgs &a, uint32_t nt, bool routed);
-uint32_t qmm_tc_pick_nt(uint32_t rows, uint32_t n, uint32_t k, int sm_count, bool routed, bool sharded);
+uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool sharded);
 bool qmm_tc_supported(const QmmArgs &a);
+constexpr uint32_t kRoutedTileRows = 64;   // activation rows of a tile of the grouped mat-mat
 cudaError_t launch_moe_map0(const uint32_t *ids, uint32_t n_tokens, uint32_t top_k, uint32_t n_experts,
                             uint32_t hids_stride, uint32_t *htpe, int32_t *hids, float *y, uint32_t n, cudaStream_t st);
 cudaError_t launch_moe_softmax_topk(const float *logits, uint32_t n_tokens, uint32_t n_experts, uint32_t top_k,
@@ -1763,7 +1764,7 @@ static int dispatch_mm(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
             return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: quantized_matmul_ggml_sharded: the mat-mat form needs K to be a multiple of 32");
     }
     if ((sh || opt_qmm_tc()) && qmm_tc_supported(a)) {
-        const uint32_t nt = qmm_tc_pick_nt(p->m, p->n, p->k, dev->sm_count, false, sh != nullptr);
+        const uint32_t nt = qmm_tc_pick_nt((int)p->ggml_type, a, dev->sm_count, sh != nullptr);
         uint8_t *scratch = nullptr;
         if ((rc = encoder_scratch(enc, qmm_tc_scratch_bytes(a, nt, false), &scratch))) return rc;
         int launches = 0;
@@ -1905,7 +1906,7 @@ extern "C" int mlxn_quantized_matmul_mm_tensor_perm021(mlxn_encoder *enc, mlxn_r
     a.n_experts = 1;
     a.total_rows = p->m;
     a.status = enc->status_word;
-    const uint32_t nt = qmm_tc_pick_nt(p->m, p->n, p->k, dev->sm_count, false, false);
+    const uint32_t nt = qmm_tc_pick_nt(t, a, dev->sm_count, false);
     uint8_t *scratch = nullptr;
     if ((rc = encoder_scratch(enc, qmm_tc_scratch_bytes(a, nt, false), &scratch))) return rc;
     int launches = 0;
@@ -2079,7 +2080,7 @@ static int dispatch_id_mm_stages(mlxn_encoder *enc, mlxn_registry *reg, mlxn_dev
     a.expert_stride = p->expert_stride;
     a.status = enc->status_word;
     if (opt_qmm_tc() && qmm_tc_supported(a)) {
-        const uint32_t nt = qmm_tc_pick_nt(p->n_tokens, p->n, p->k, dev->sm_count, true, false);
+        const uint32_t nt = kRoutedTileRows;
         uint8_t *scratch = nullptr;
         const size_t need = qmm_tc_scratch_bytes(a, nt, true);
         if ((rc = encoder_scratch(enc, scratch_used + need, &scratch))) return rc;
@@ -2122,7 +2123,7 @@ extern "C" int mlxn_quantized_matmul_id_ggml(mlxn_encoder *enc, mlxn_registry *r
     probe.k = params->k;
     probe.n_experts = params->n_experts;
     probe.total_rows = params->n_tokens * params->top_k;
-    const size_t tc_b = qmm_tc_scratch_bytes(probe, qmm_tc_pick_nt(params->n_tokens, params->n, params->k, dev->sm_count, true, false), true);
+    const size_t tc_b = qmm_tc_scratch_bytes(probe, kRoutedTileRows, true);
     uint8_t *scratch = nullptr;
     if ((rc = encoder_scratch(enc, htpe_b + hids_b + tc_b, &scratch))) return rc;
     return dispatch_id_mm_stages(enc, reg, dev, input, weight, ids, output, reinterpret_cast<uint32_t *>(scratch),
@@ -2221,7 +2222,7 @@ extern "C" int mlxn_moe_ffn_layer(mlxn_encoder *enc, mlxn_registry *reg, mlxn_de
         return rc;
     // scratch: bucket sizes, buckets ([experts, n_tokens]: a token holds an expert at most once, and the down projection's
     // rows are the same pairs), then the tile list and the packed activations (sized for the longer of the two K)
-    const uint32_t nt = qmm_tc_pick_nt(p->n_tokens, p->ffn, p->hidden, dev->sm_count, true, false);
+    const uint32_t nt = kRoutedTileRows;
     const size_t htpe_b = ((size_t)p->n_experts * 4 + 1023) / 1024 * 1024;
     const size_t hids_b = ((size_t)p->n_experts * p->n_tokens * 4 + 1023) / 1024 * 1024;
     QmmArgs sz{};

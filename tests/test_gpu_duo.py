@@ -1,0 +1,78 @@
+"""The mat-mat on pairs of SMs (csrc/qmm_duo.cu) at the edges of its tiles (256 weight rows, 128 for each CTA; a multiple of 32 activation rows,
+at most 256), K stages (128 values, two to a raw stage) and work shares, against the oracle with both operands rounded to f16."""
+import numpy as np
+import pytest
+
+import mlx_native_b200 as mx
+from oracle import oracle as orc
+from tests.gpu_util import TYPES, Ctx, norm_err, normal_acts, normal_weights
+
+pytestmark = pytest.mark.gpu
+# both operands are the oracle's; the sums differ in order: sqrt(K / 16) roundings of 2^-24 of partial sums that are smaller than sum |w x|
+TOL = 2e-5
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return Ctx()
+
+
+# one weight tile and a part of the next (the second CTA's half empty, or a row short); activation tiles with rows left over; K of part of a
+# stage, of part of a raw stage, of an odd number of raw stages; rows at every even pitch (groups of 1, 2, 4 and 8 rows a copy)
+@pytest.mark.parametrize("tname,n,k,m", [
+    ("Q4_0", 8, 32, 9), ("Q4_0", 256, 96, 33), ("Q4_0", 136, 416, 31), ("Q4_0", 264, 1024, 65), ("Q4_0", 520, 2880, 257), ("Q4_0", 128, 4096, 300),
+    ("Q8_0", 8, 64, 10), ("Q8_0", 120, 160, 32), ("Q8_0", 384, 1056, 97), ("Q8_0", 257, 512, 64), ("Q8_0", 504, 2048, 129),
+    ("Q6_K", 8, 256, 12), ("Q6_K", 248, 768, 40), ("Q6_K", 260, 2560, 96), ("Q6_K", 513, 2048, 200), ("Q6_K", 264, 4096, 513)])
+def test_dense(ctx, tname, n, k, m):
+    gtype, otype = TYPES[tname]
+    wq = normal_weights(n + k, n, k, otype)
+    x = normal_acts(n + m, m, k)
+    y = ctx.matmul(gtype, wq, x, n, k)
+    assert mx.last_kernel_name() == "qmm_tc"
+    y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8, f16_operands=True)
+    assert norm_err(y, y_ref, ad) <= TOL
+    assert np.array_equal(y.view(np.uint32), ctx.matmul(gtype, wq, x, n, k).view(np.uint32))
+
+
+# more tiles than pairs of SMs: whole tiles one after another, and equal ranges that cut tiles in two
+@pytest.mark.parametrize("tname,n,k,m", [("Q4_0", 20480, 256, 16), ("Q4_0", 20480, 2048, 16), ("Q6_K", 22528, 768, 40), ("Q8_0", 2048, 512, 2300)])
+def test_many_tiles(ctx, tname, n, k, m):
+    gtype, otype = TYPES[tname]
+    part = normal_weights(k, 1024, k, otype)
+    x = normal_acts(m, m, k)
+    y = ctx.matmul(gtype, np.tile(part, n // 1024), x, n, k)
+    rows = np.r_[0:40, m - 40:m] if m > 200 else np.arange(m)
+    y_ref, ad = orc.qmatmul(otype, part, x[rows], 1024, k, nthreads=8, f16_operands=True)
+    for at in range(0, n, 1024):
+        assert norm_err(y[rows, at:at + 1024], y_ref, ad) <= TOL
+    first = y[:, :1024].view(np.uint32)   # the same weights again: where no tile is cut, the same bits
+    if k == 256:
+        assert all(np.array_equal(first, y[:, at:at + 1024].view(np.uint32)) for at in range(0, n, 1024))
+
+
+# both kernels take the call or only the other one (weights off 16-byte boundaries): the same results within the order of the sums
+@pytest.mark.parametrize("tname,n,k,m", [("Q4_0", 392, 1312, 70), ("Q8_0", 264, 1024, 130), ("Q6_K", 200, 1280, 48)])
+def test_beside_the_other_kernel(ctx, tname, n, k, m):
+    gtype, otype = TYPES[tname]
+    wq = normal_weights(n, n, k, otype)
+    big = np.zeros(wq.size + 64, np.uint8)
+    big[6:6 + wq.size] = wq
+    x = normal_acts(7, m, k)
+    y = ctx.matmul(gtype, wq, x, n, k)
+    z = ctx.matmul(gtype, wq, x, n, k, weight_buf=ctx.buf(big, mx.DType.U8).slice_view(6, wq.size))
+    y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8, f16_operands=True)
+    assert norm_err(y, y_ref, ad) <= TOL and norm_err(z, y_ref, ad) <= TOL
+
+
+def test_infinities_stay_in_their_row(ctx):
+    gtype, otype = TYPES["Q8_0"]
+    n, k, m = 264, 512, 48
+    wq = normal_weights(3, n, k, otype)
+    x = normal_acts(3, m, k)
+    x[5, 17], x[40, 300] = np.inf, np.nan
+    y = ctx.matmul(gtype, wq, x, n, k)
+    bad = np.zeros(m, bool)
+    bad[[5, 40]] = True
+    assert np.isfinite(y[~bad]).all() and not np.isfinite(y[bad]).any(axis=1).all()
+    y_ref, ad = orc.qmatmul(otype, wq, x[~bad], n, k, nthreads=4, f16_operands=True)
+    assert norm_err(y[~bad], y_ref, ad) <= TOL
