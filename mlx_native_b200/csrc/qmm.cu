@@ -13,6 +13,7 @@
 //             staging ring, eight warps dequantise them into the swizzled f16 A tile, one thread
 //             issues tcgen05.mma (M=128, N=NT, K=16) accumulating in tensor memory, and the same
 //             eight warps read the accumulator back with tcgen05.ld and store y.
+//             Dense calls go to pairs of SMs where their weights allow it (qmm_duo.cu); grouped and row-sharded ones run here.
 //   qmm_simt  plain CUDA-core tile kernel with the same operand rounding; used for shapes the
 //             tcgen05 kernel does not take and as an on-device cross-check.
 #include <cuda_fp16.h>
@@ -162,11 +163,13 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const uint32_t *htpe, 
     __shared__ uint32_t warp_tot[8];
     __shared__ uint32_t carry_s;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    grid_dependency_wait();
+    allow_dependents();
     if (tid == 0) carry_s = 0;
     __syncthreads();
     for (uint32_t base = 0; base < n_experts; base += 256) {
         const uint32_t e = base + tid;
-        const uint32_t cnt = e < n_experts ? (htpe[e] + nt - 1) / nt : 0u;
+        const uint32_t cnt = e < n_experts ? (__ldcg(htpe + e) + nt - 1) / nt : 0u;
         uint32_t incl = cnt;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -195,28 +198,45 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const uint32_t *htpe, 
 // A CTA packs a slice of 64 rows, which is two 16-byte columns per thread and chunk: with whole tiles of 256 rows per CTA,
 // 512 x 4096 activations took 10 us, most of it one load after another; with slices 6.
 // grid (tiles x slices, K-chunk lanes), 256 threads.
-__global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t nt, const TcShare sh) {
+// Eight floats (`left` of them and zeros), by one load where they are a whole 32-byte sector: from L2, two loads fetch every sector twice.
+__device__ __forceinline__ void load8(const float *p, uint32_t left, float (&v)[8]) {
+    if (left >= 8 && ((uintptr_t)p & 31u) == 0) {
+        asm volatile("ld.global.cg.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                     : "l"(p));
+    } else if (left >= 8 && ((uintptr_t)p & 15u) == 0) {
+        const float4 lo = __ldcg(reinterpret_cast<const float4 *>(p)), hi = __ldcg(reinterpret_cast<const float4 *>(p) + 1);
+        v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+        v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+    } else {
+#pragma unroll
+        for (uint32_t u = 0; u < 8; u++) v[u] = u < left ? __ldcg(p + u) : 0.0f;
+    }
+}
+__global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t nt, const TcShare sh, const __grid_constant__ TcOut res) {
     // CTA (t, c) packs the chunks c, c + gridDim.y, ... of its slice, so that the slice's routing lookups (a chain of
     // dependent loads) are paid once per CTA, not once per chunk.
     const uint32_t slices = (nt + kPackRows - 1) / kPackRows, t = blockIdx.x / slices, r0 = (blockIdx.x - t * slices) * kPackRows;
+    grid_dependency_wait();   // (what the kernel ahead has written is read from L2: this SM's L1 may hold lines from before)
     allow_dependents();   // the mat-mat kernel behind may set itself up; it waits for this grid before it reads anything
     if (sh.ctas) {  // output tiles that two CTAs of the mat-mat share are added up in y (dense form only): zero them, 64 rows at a time
         const uint32_t pieces = (sh.nt + kPackRows - 1) / kPackRows, halves = sh.rows / 128u, jobs = (sh.ctas - 1) * pieces * halves;
         for (uint32_t j = blockIdx.y * gridDim.x + blockIdx.x; j < jobs; j += gridDim.x * gridDim.y) {
             const uint32_t q = j / halves, b = q / pieces, pos = sh.begin(b + 1), tile = pos / sh.nraw;
             if (tile * sh.nraw == pos) continue;   // the boundary between two CTAs is one between tiles
-            const uint32_t tt = tile / sh.n_wt, col = (tile - tt * sh.n_wt) * sh.rows + (j - q * halves) * 128u + (threadIdx.x & 127u), lo = (q - b * pieces) * kPackRows;
-            const uint32_t end = min(a.m, tt * sh.nt + min(sh.nt, lo + kPackRows));
-            if (col < a.n)
-                for (uint32_t row = tt * sh.nt + lo + (threadIdx.x >> 7); row < end; row += 2) a.y[(size_t)row * a.n + col] = 0.f;
+            const uint32_t tt = tile / sh.n_wt, lo = (q - b * pieces) * kPackRows, end = min(a.m, tt * sh.nt + min(sh.nt, lo + kPackRows));
+            uint32_t wt = tile - tt * sh.n_wt;
+            const uint32_t o = res.find(wt), col = wt * sh.rows + (j - q * halves) * 128u + (threadIdx.x & 127u);
+            if (col < res.n[o])
+                for (uint32_t row = tt * sh.nt + lo + (threadIdx.x >> 7); row < end; row += 2) res.y[o][(size_t)row * res.n[o] + col] = 0.f;
         }
     }
     uint32_t e = 0, mt = t, nrows = a.m;
     if (a.hids) {
-        if (t >= a.tiles[0]) return;
-        e = a.tiles[1 + 2 * t];
-        mt = a.tiles[2 + 2 * t];
-        nrows = a.htpe[e];
+        if (t >= __ldcg(a.tiles)) return;
+        e = __ldcg(a.tiles + 1 + 2 * t);
+        mt = __ldcg(a.tiles + 2 + 2 * t);
+        nrows = __ldcg(a.htpe + e);
     }
     constexpr int kPer = 2;   // (row, 16-byte column) pairs per thread: the same ones in every chunk
     const float *src_row[kPer];
@@ -227,7 +247,7 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
         if (r < nt && row < nrows) {
             int64_t src = row;
             if (a.hids) {
-                const int32_t id = a.hids[(size_t)e * a.hids_stride + row];
+                const int32_t id = __ldcg(a.hids + (size_t)e * a.hids_stride + row);
                 src = (id >= 0 && (uint32_t)id < a.total_rows) ? id / (int32_t)a.top_k : -1;
             }
             // (perm021 form: the pointer only marks the row as present; the element addresses are formed per chunk)
@@ -236,49 +256,41 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
     }
     for (uint32_t kc = blockIdx.y; kc < nchunks; kc += gridDim.y) {
         uint8_t *tile = xpack + ((size_t)t * nchunks + kc) * (size_t)(nt * 128);
+        const uint32_t k0 = kc * 64 + 8 * (threadIdx.x & 7u);   // (the same columns in both rows)
+        float v[kPer][8];
+        [[maybe_unused]] float z[kPer][8];
+        // all loads first
 #pragma unroll
         for (int i = 0; i < kPer; i++) {
-            const uint32_t q = threadIdx.x + i * 256;
-            const uint32_t r = r0 + (q >> 3), j = q & 7u;
+            if (!src_row[i] || k0 >= a.k) continue;
+            if (a.x_bf16) {
+                // eight consecutive K values lie inside one head (head_dim is a multiple of 32): 16 bytes of bf16
+                const uint32_t h = k0 / a.head_dim, d0 = k0 - h * a.head_dim, row = mt * nt + r0 + ((threadIdx.x + i * 256) >> 3);
+                const uint4 raw = __ldcg(reinterpret_cast<const uint4 *>(a.x_bf16 + ((size_t)h * a.m + row) * a.head_dim + d0));
+                const uint32_t w4[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+                for (int u = 0; u < 4; u++) {   // bf16 -> f32 is exact; f32 -> f16 rounds to nearest even below
+                    v[i][2 * u] = __uint_as_float(w4[u] << 16);
+                    v[i][2 * u + 1] = __uint_as_float(w4[u] & 0xFFFF0000u);
+                }
+            } else {
+                load8(src_row[i] + k0, a.k - k0, v[i]);
+                if (a.x2) load8(a.x2 + (src_row[i] + k0 - a.x), a.k - k0, z[i]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {
+            const uint32_t q = threadIdx.x + i * 256, r = r0 + (q >> 3), j = q & 7u;
             if (r >= nt) break;
-            const uint32_t k0 = kc * 64 + 8 * j;
             uint4 out = make_uint4(0, 0, 0, 0);
             if (src_row[i] && k0 < a.k) {
-                const float *xp = src_row[i] + k0;
-                float v[8];
-                if (a.x_bf16) {
-                    // eight consecutive K values lie inside one head (head_dim is a multiple of 32): 16 bytes of bf16
-                    const uint32_t h = k0 / a.head_dim, d0 = k0 - h * a.head_dim, row = mt * nt + r;
-                    const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(a.x_bf16 + ((size_t)h * a.m + row) * a.head_dim + d0));
-                    const uint32_t w4[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {   // bf16 -> f32 is exact; f32 -> f16 rounds to nearest even below
-                        v[2 * u] = __uint_as_float(w4[u] << 16);
-                        v[2 * u + 1] = __uint_as_float(w4[u] & 0xFFFF0000u);
-                    }
-                } else if (k0 + 8 <= a.k && (((uintptr_t)xp) & 15u) == 0) {
-                    const float4 lo = __ldg(reinterpret_cast<const float4 *>(xp));
-                    const float4 hi = __ldg(reinterpret_cast<const float4 *>(xp) + 1);
-                    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
-                    v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
-                } else {
-#pragma unroll
-                    for (int u = 0; u < 8; u++) v[u] = (k0 + u < a.k) ? xp[u] : 0.0f;
-                }
                 if (a.x2) {   // fused SwiGLU: the same expression as the stand-alone kernel, so the same f32 values
-                    const float *up = a.x2 + (xp - a.x);
 #pragma unroll
-                    for (int u = 0; u < 8; u++) {
-                        const float uv = (k0 + u < a.k) ? __ldg(up + u) : 0.0f;
-                        v[u] = v[u] / (1.0f + expf(-v[u])) * uv;
-                    }
+                    for (int u = 0; u < 8; u++) v[i][u] = v[i][u] / (1.0f + expf(-v[i][u])) * z[i][u];
                 }
-                __half2 h0 = __floats2half2_rn(v[0], v[1]), h1 = __floats2half2_rn(v[2], v[3]);
-                __half2 h2 = __floats2half2_rn(v[4], v[5]), h3 = __floats2half2_rn(v[6], v[7]);
-                out.x = *reinterpret_cast<uint32_t *>(&h0);
-                out.y = *reinterpret_cast<uint32_t *>(&h1);
-                out.z = *reinterpret_cast<uint32_t *>(&h2);
-                out.w = *reinterpret_cast<uint32_t *>(&h3);
+                const __half2 h0 = __floats2half2_rn(v[i][0], v[i][1]), h1 = __floats2half2_rn(v[i][2], v[i][3]);
+                const __half2 h2 = __floats2half2_rn(v[i][4], v[i][5]), h3 = __floats2half2_rn(v[i][6], v[i][7]);
+                out = make_uint4(h2_as_u32(h0), h2_as_u32(h1), h2_as_u32(h2), h2_as_u32(h3));
             }
             *reinterpret_cast<uint4 *>(tile + (r >> 3) * 1024 + (r & 7u) * 128 + ((j ^ (r & 7u)) << 4)) = out;
         }
@@ -1018,6 +1030,28 @@ uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool shar
     return best;
 }
 
+// Products of the same activations (and block type) as one launch on pairs of SMs: the tile, 0 where one of them does not go there.
+uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops) {
+    QmmArgs all = ops[0];
+    for (int i = 0; i < nops; i++) {
+        if (qmm_duo_cost(ggml_type, ops[i], 32) == ~0ull) return 0;
+        if (i) all.n = (all.n + 255) / 256 * 256 + ops[i].n;   // (as many weight tiles)
+    }
+    all.n = (all.n + 255) / 256 * 256;
+    uint32_t best = 0;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t tt = (all.m + 255) / 256, last = tt + 8; tt <= last; tt++) {
+        const uint32_t nt = ((all.m + tt - 1) / tt + 31) / 32 * 32;
+        const uint64_t cost = qmm_duo_cost(ggml_type, all, nt);
+        if (cost != ~0ull && (best == 0 || cost * 103 / 100 < best_cost)) {
+            best_cost = cost;
+            best = nt;
+        }
+        if (nt == 32) break;
+    }
+    return best;
+}
+
 bool qmm_tc_supported(const QmmArgs &a) {
     if (a.k % 32 != 0 || a.k < 32) return false;
     if (((uintptr_t)a.w & 1u) || (a.expert_stride & 1u)) return false;
@@ -1119,7 +1153,8 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint32_t nt, uint8_t *sc
         const size_t header = ((1 + 2 * tiles) * 4 + 1023) / 1024 * 1024;
         uint32_t *tl = reinterpret_cast<uint32_t *>(scratch);
         if (!(a.reuse & 1u)) {   // (an earlier call of the same layer built the list: same buckets, same NT)
-            build_tiles_kernel<<<1, 256, 0, st>>>(a.htpe, a.n_experts, nt, (uint32_t)tiles, tl);
+            const cudaError_t e = launch_overlapped(build_tiles_kernel, dim3(1), dim3(256), 0, st, a.htpe, a.n_experts, nt, (uint32_t)tiles, tl);
+            if (e != cudaSuccess) return e;
             (*launches)++;
         }
         a.tiles = tl;
@@ -1138,9 +1173,12 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint32_t nt, uint8_t *sc
         const uint64_t slices = (uint64_t)tiles * ((nt + kPackRows - 1) / kPackRows);
         while (lanes > 1 && (uint64_t)lanes * slices > 2048) lanes = (lanes + 1) / 2;
         dim3 grid((unsigned)slices, lanes);
-        pack_x_kernel<<<grid, 256, 0, st>>>(a, xpack, c.nchunks, nt, c.share);
         (*launches)++;
-        cudaError_t e = cudaGetLastError();
+        TcOut res{};
+        res.y[0] = a.y;
+        res.n[0] = a.n;
+        res.wt_end[0] = c.n_wt;
+        cudaError_t e = launch_overlapped(pack_x_kernel, grid, dim3(256), 0, st, a, xpack, c.nchunks, nt, c.share, res);
         if (e != cudaSuccess) return e;
     }
     static size_t attr_smem[64] = {};
@@ -1185,7 +1223,7 @@ cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t
     if (!routed) {
         TcPlan plan;
         if (qmm_duo_cost(ggml_type, a, nt) < tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count_of_device(), a.y_ld != 0 || a.n_peer != 0, plan))
-            return launch_qmm_duo(ggml_type, a, nt, scratch, st, launches);
+            return launch_qmm_duo(ggml_type, &a, 1, nt, scratch, st, launches);
     }
     switch (ggml_type) {
     case GT_Q4_0: return launch_tc_t<GT_Q4_0>(a, routed, nt, scratch, st, launches);

@@ -15,14 +15,28 @@ struct TcShare {
     __host__ __device__ uint32_t begin(uint32_t cta) const { return (uint32_t)((uint64_t)total * cta / ctas); }
 };
 
+// Products that share their activations in one launch: their weight tiles one after another.
+constexpr uint32_t kMmOps = 4;
+struct TcOut {
+    float *y[kMmOps];
+    uint32_t n[kMmOps], wt_end[kMmOps];   // weight rows; weight-row tiles of the products up to and including this one
+    // the product of weight tile `wt`, which becomes that product's own tile number
+    __device__ __forceinline__ uint32_t find(uint32_t &wt) const {
+        uint32_t o = 0;
+        while (wt >= wt_end[o]) o++;
+        if (o) wt -= wt_end[o - 1];
+        return o;
+    }
+};
+
 constexpr uint32_t kPackRows = 64;   // rows of a tile that a block of pack_x_kernel packs
-__global__ void pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t nt, const TcShare sh);
+__global__ void pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t nt, const TcShare sh, const __grid_constant__ TcOut res);
 
 int sm_count_of_device();
 
 // The mat-mat on pairs of CTAs (qmm_duo.cu).  Time that it would take, in the units of tc_plan, or ~0 where it does not take the call;
 // `nt` as for the other kernel, a multiple of 32.
 uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt);
-cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs &a, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches);
+cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches);
 
 }  // namespace mlxn

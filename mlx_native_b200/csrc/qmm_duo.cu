@@ -6,9 +6,17 @@
 // (tcgen05 cta_group::2): each dequantises its own 128 rows into its own tensor memory and holds half of the activation tile, which the
 // hardware reads from both.  Operand semantics as in qmm.cu: exact weights rounded once to f16, activations f32 -> f16, f32 sums.
 //
+// Graph replay of dependent calls, packing included, us with qmm.cu / here (K 4096 unless said): 4096 weight rows: 9 rows 18.9 / 14.4, 64 20.9 / 15.5,
+// 256 24.3 / 19.0, 512 31.1 / 25.0; 12288 x 512 rows 66.7 / 46.4; 1024 x 512 22.4 / 16.8; 4096 x 12288, 2048 rows: Q4_0 205 / 169, Q6_K 229 / 181;
+// 256 x 512 x 16 rows 8.6 / 8.2.  So it takes every call it can: what has no 16-byte aligned weights, or a row count that its copies cannot group,
+// stays with the other kernel, and the row-sharded form.  What bounds it: up to 192 rows the chain raw block -> tensor memory (0.47 us for a
+// K stage of 128, 18 values a cycle and SM; Q6_K 0.66), above that the multiplication (0.43 us at full clock) beside it.
+//
 // What else was tried: unpacking the weights once into f16 tiles, by a kernel of its own.  The product alone then runs at the
 // multiplication's rate, but the unpacking is bound by memory (13 us for 4096 x 4096, 58 with 2048 rows of 12288 for 4096 x 12288): 32.2 us in
-// all for 512 x 4096 x 4096, 72.8 for 512 x 12288 x 4096.
+// all for 512 x 4096 x 4096, 72.8 for 512 x 12288 x 4096.  K in two and four parts over clusters of two and four pairs,
+// summed through distributed shared memory instead of atomics: 16.2 us for 128 x 4096 x 4096 where halves with atomics take 15.4 (and only 15
+// clusters of eight fit on the chip).  Announcing a stage after the next one's arithmetic instead of waiting for its store: 1 to 4 % slower.
 #include <cuda_fp16.h>
 
 #include <atomic>
@@ -38,6 +46,10 @@ struct DuoCfg {
     uint32_t raw_off, raw_slots;
     uint32_t row_group;   // log2 of the copies of a raw stage (see launch_tc_tn)
     uint32_t aligned;     // every weight row starts on a 16-byte boundary
+    TcOut out;
+};
+struct DuoMaps {
+    CUtensorMap m[kMmOps];
 };
 
 namespace duo {
@@ -92,7 +104,7 @@ __device__ __forceinline__ void commit_both(uint64_t *bar) {
 // Ring places and barrier phases run on across the items of a pair.
 template <int T>
 __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
-    qmm_duo_kernel(const QmmArgs a, const DuoCfg c, const uint8_t *xpack, const __grid_constant__ CUtensorMap wmap) {
+    qmm_duo_kernel(const QmmArgs a, const __grid_constant__ DuoCfg c, const uint8_t *xpack, const __grid_constant__ DuoMaps wmaps) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
     constexpr uint32_t KR = 256;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -135,7 +147,7 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
     const bool shared = c.share.ctas != 0;
     const uint32_t pos0 = shared ? c.share.begin(pair) : pair, pos1 = shared ? c.share.begin(pair + 1) : total_items;
     struct Item {
-        uint32_t tt, n0, r_lo, nraw, nst, kc_lo, nck, next;
+        uint32_t tt, op, n0, r_lo, nraw, nst, kc_lo, nck, next;
     };
     auto load_item = [&](uint32_t pos) {
         Item it;
@@ -144,7 +156,9 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
         const uint32_t r_hi = shared ? min(nraw_all, it.r_lo + (pos1 - pos)) : nraw_all;
         it.next = shared ? pos + (r_hi - it.r_lo) : pos + c.pairs;
         it.tt = item / c.n_wt;
-        it.n0 = (item - it.tt * c.n_wt) * kDuoRows + rank * 128u;
+        uint32_t wt = item - it.tt * c.n_wt;
+        it.op = c.out.find(wt);
+        it.n0 = wt * kDuoRows + rank * 128u;
         it.nraw = r_hi - it.r_lo;
         it.kc_lo = it.r_lo * (KR / 64);
         it.nst = min((a.k + 127) / 128, r_hi * (KR / 128)) - it.r_lo * (KR / 128);   // K stages of 128
@@ -245,7 +259,7 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
                         asm volatile(
                             "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
                                 smem_base + c.raw_off + slot * raw_bytes + i * (raw_bytes >> c.row_group)),
-                            "l"(&wmap), "r"(((i * row_bytes + kb) & ~15u) >> 2), "r"(it.n0 >> c.row_group), "r"(smem_u32(&raw_full[slot]))
+                            "l"(&wmaps.m[it.op]), "r"(((i * row_bytes + kb) & ~15u) >> 2), "r"(it.n0 >> c.row_group), "r"(smem_u32(&raw_full[slot]))
                             : "memory");
                 }
                 __syncwarp();
@@ -267,8 +281,9 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
         for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
             const Item it = load_item(pos);
             pos = it.next;
-            const bool row_ok = it.n0 + rr < a.n;
-            const uint32_t row_lo4 = (uint32_t)((uintptr_t)(a.w + (size_t)(it.n0 + rr) * row_bytes) & 15u);
+            const uint32_t n = c.out.n[it.op];
+            const bool row_ok = it.n0 + rr < n;
+            const uint32_t row_lo4 = (it.n0 + rr) * row_bytes & 15u;   // (the weights start on a 16-byte boundary)
             for (uint32_t r = 0; r < it.nraw; r++) {
                 if (!mbar_wait(&raw_full[rs], rph, &abort_flag, a.status, ST_WAIT_FULL_TIMEOUT, 0u)) {
                     ok = false;
@@ -347,16 +362,16 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
                 tmem_ld_wait();
                 const uint32_t o0 = it.tt * c.nt + col;
                 if (row_ok && o0 < a.m) {
-                    float *y = a.y + (size_t)o0 * a.n + it.n0 + rr;
+                    float *y = c.out.y[it.op] + (size_t)o0 * n + it.n0 + rr;
                     const uint32_t cnt = min(32u, a.m - o0);
                     if (some) {
 #pragma unroll
                         for (uint32_t j = 0; j < 32; j++)
-                            if (j < cnt) atomicAdd(y + (size_t)j * a.n, __uint_as_float(v[j]));
+                            if (j < cnt) atomicAdd(y + (size_t)j * n, __uint_as_float(v[j]));
                     } else {
 #pragma unroll
                         for (uint32_t j = 0; j < 32; j++)
-                            if (j < cnt) y[(size_t)j * a.n] = __uint_as_float(v[j]);
+                            if (j < cnt) y[(size_t)j * n] = __uint_as_float(v[j]);
                     }
                 }
             }
@@ -447,15 +462,23 @@ uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt) {
     return duo_plan(ggml_type, a.m, a.n, a.k, nt, p);
 }
 
-template <int T> static cudaError_t launch_duo_t(const QmmArgs &a, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {
+// `ops`: products of the same activations
+template <int T> static cudaError_t launch_duo_t(const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
+    if (nops < 1 || nops > (int)kMmOps) return cudaErrorInvalidValue;
+    const QmmArgs &a = ops[0];
     const uint32_t row_bytes = (a.k / QK) * BB, h = nt / 2;
-    DuoPlan p;
-    duo_plan(T, a.m, a.n, a.k, nt, p);
     DuoCfg c{};
+    for (int i = 0; i < nops; i++) {
+        c.n_wt += (ops[i].n + kDuoRows - 1) / kDuoRows;
+        c.out.y[i] = ops[i].y;
+        c.out.n[i] = ops[i].n;
+        c.out.wt_end[i] = c.n_wt;
+    }
+    DuoPlan p;
+    duo_plan(T, a.m, (uint64_t)c.n_wt * kDuoRows, a.k, nt, p);
     c.nt = nt;
     c.nchunks = (a.k + 63) / 64;
-    c.n_wt = (a.n + kDuoRows - 1) / kDuoRows;
     c.ntiles = (a.m + nt - 1) / nt;
     c.pairs = p.pairs;
     c.row_group = (uint32_t)duo_row_group(row_bytes);
@@ -464,15 +487,15 @@ template <int T> static cudaError_t launch_duo_t(const QmmArgs &a, uint32_t nt, 
     c.seg_stride = c.row_group == 0 && kSeg % 16 == 0 ? kSeg : ((kSeg + 14 + 15) / 16 | 1u) * 16;   // (an odd multiple of 16: see launch_tc_tn)
     const uint32_t nraw = (a.k + 255) / 256;
     if (p.shared) c.share = {p.pairs, c.n_wt, nraw, c.n_wt * c.ntiles * nraw, kDuoRows, nt};
-    alignas(64) CUtensorMap wmap;
-    {
-        EncodeTiledFn enc = encode_tiled_fn();
-        if (!enc) return cudaErrorNotSupported;
+    alignas(64) DuoMaps wmaps;
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return cudaErrorNotSupported;
+    for (int i = 0; i < nops; i++) {
         const uint32_t lg = c.row_group;
-        const cuuint64_t gdim[2] = {((uint64_t)row_bytes << lg) / 4, a.n >> lg};
+        const cuuint64_t gdim[2] = {((uint64_t)row_bytes << lg) / 4, ops[i].n >> lg};
         const cuuint64_t gstride[1] = {(uint64_t)row_bytes << lg};
         const cuuint32_t box[2] = {c.seg_stride / 4, 128u >> lg}, estr[2] = {1, 1};
-        if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t *>(a.w), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        if (enc(&wmaps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t *>(ops[i].w), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
@@ -481,16 +504,16 @@ template <int T> static cudaError_t launch_duo_t(const QmmArgs &a, uint32_t nt, 
     c.raw_slots = (limit - b_bytes) / raw_slot;
     if (c.raw_slots > kDuoMaxRaw) c.raw_slots = kDuoMaxRaw;
     if (c.raw_slots < 2) return cudaErrorInvalidConfiguration;
-    const size_t smem = (size_t)b_bytes + c.raw_slots * raw_slot + 1024;
+    size_t smem = (size_t)b_bytes + c.raw_slots * raw_slot + 1024;
+    if (smem < 120 * 1024) smem = 120 * 1024;   // (one CTA per SM: it takes all of tensor memory)
     // activations in tiles of nt / 2 rows: a CTA's half of a tile
     {
         const uint32_t tiles = 2 * c.ntiles;
         uint32_t lanes = c.nchunks;
         const uint64_t slices = (uint64_t)tiles * ((h + kPackRows - 1) / kPackRows);
         while (lanes > 1 && (uint64_t)lanes * slices > 2048) lanes = (lanes + 1) / 2;
-        pack_x_kernel<<<dim3((unsigned)slices, lanes), 256, 0, st>>>(a, xpack, c.nchunks, h, c.share);
         (*launches)++;
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_overlapped(pack_x_kernel, dim3((unsigned)slices, lanes), dim3(256), 0, st, a, xpack, c.nchunks, h, c.share, c.out);
         if (e != cudaSuccess) return e;
     }
     static std::atomic<uint32_t> prepared[64] = {};
@@ -503,14 +526,14 @@ template <int T> static cudaError_t launch_duo_t(const QmmArgs &a, uint32_t nt, 
         prepared[dev].store(1, std::memory_order_release);
     }
     (*launches)++;
-    return launch_overlapped(qmm_duo_kernel<T>, dim3(2 * c.pairs), dim3(kDuoThreads), smem, st, a, c, (const uint8_t *)xpack, wmap);
+    return launch_overlapped(qmm_duo_kernel<T>, dim3(2 * c.pairs), dim3(kDuoThreads), smem, st, a, c, (const uint8_t *)xpack, wmaps);
 }
 
-cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs &a, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {
+cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {
     switch (ggml_type) {
-    case GT_Q4_0: return launch_duo_t<GT_Q4_0>(a, nt, xpack, st, launches);
-    case GT_Q8_0: return launch_duo_t<GT_Q8_0>(a, nt, xpack, st, launches);
-    case GT_Q6_K: return launch_duo_t<GT_Q6_K>(a, nt, xpack, st, launches);
+    case GT_Q4_0: return launch_duo_t<GT_Q4_0>(ops, nops, nt, xpack, st, launches);
+    case GT_Q8_0: return launch_duo_t<GT_Q8_0>(ops, nops, nt, xpack, st, launches);
+    case GT_Q6_K: return launch_duo_t<GT_Q6_K>(ops, nops, nt, xpack, st, launches);
     default: return cudaErrorInvalidValue;
     }
 }

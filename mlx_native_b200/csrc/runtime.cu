@@ -50,6 +50,10 @@ cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t
                           int *launches);
 cudaError_t launch_qmm_simt(int ggml_type, const QmmArgs &a, bool routed, uint32_t max_rows, cudaStream_t st);
 size_t qmm_tc_scratch_bytes(const QmmArgs &a, uint32_t nt, bool routed);
+constexpr size_t kMmBatchMax = 4;          // mat-mats one launch carries (kMmOps)
+uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt);
+uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops);
+cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches);
 uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool sharded);
 bool qmm_tc_supported(const QmmArgs &a);
 constexpr uint32_t kRoutedTileRows = 64;   // activation rows of a tile of the grouped mat-mat
@@ -315,6 +319,10 @@ struct mlxn_encoder {
     bool pend_pair = false;
     bool pend_split = false;          // they are mat-vecs of the split kernel (qmv_split.cuh)
     bool pend_wide = false;           // ... or (pend_split too) of the one for many rows (qmv_wide.cu)
+    // Mat-mats of the same activations wait in the same way (one type and row count, `pend` and this one never both): their weight tiles
+    // share a launch, and the activations are packed once.
+    std::vector<QmmArgs> pend_mm;
+    bool pending() const { return !pend.empty() || !pend_mm.empty(); }
     bool grp_pend_only = false;       // every operation of the current group is in `pend` (none has been launched yet)
 };
 
@@ -934,7 +942,7 @@ static int encoder_mark_fork(mlxn_encoder *e) {
     return MLXN_OK;
 }
 static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
-    if (e->pend.empty()) return MLXN_OK;
+    if (!e->pending()) return MLXN_OK;
     cudaSetDevice(e->ordinal);
     if (!group_ends) {
         const int frc = encoder_mark_fork(e);
@@ -943,6 +951,36 @@ static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
     cudaStream_t st = e->lanes[e->pend_lane];
     cudaError_t err = cudaSuccess;
     int launches = 1, rc = MLXN_OK;
+    auto leave = [&]() {   // nothing waits any more
+        e->pend.clear();
+        e->pend_mm.clear();
+        for (mlxn_buffer *b : e->retained) {
+            std::lock_guard<std::mutex> lk(b->st->mu);
+            if (b->st->pend_enc == e) b->st->pend_enc = nullptr;
+        }
+    };
+    if (!e->pend_mm.empty()) {
+        e->grp_pend_only = false;
+        const std::vector<QmmArgs> ops(e->pend_mm);
+        leave();
+        launches = 0;
+        const int n = (int)ops.size(), sms = e->dev->sm_count;
+        uint8_t *scratch = nullptr;
+        const uint32_t nt = n > 1 ? qmm_duo_pick_nt(e->pend_type, ops.data(), n) : 0;
+        if (nt) {
+            if ((rc = encoder_scratch_on(e, e->pend_lane, qmm_tc_scratch_bytes(ops[0], nt, false), &scratch))) return rc;
+            CUDA_TRY(launch_qmm_duo(e->pend_type, ops.data(), n, nt, scratch, st, &launches), "mat-mat launch");
+        } else {
+            for (const QmmArgs &a : ops) {
+                const uint32_t own = qmm_tc_pick_nt(e->pend_type, a, sms, false);
+                if ((rc = encoder_scratch_on(e, e->pend_lane, qmm_tc_scratch_bytes(a, own, false), &scratch))) return rc;
+                CUDA_TRY(launch_qmm_tc(e->pend_type, a, false, own, scratch, st, &launches), "mat-mat launch");
+            }
+        }
+        g_launches.fetch_add((uint64_t)launches);
+        g_last_kernel = "qmm_tc";
+        return MLXN_OK;
+    }
     // A mat-vec that ended up alone (the next operation depended on it, or nothing followed) gains nothing from the
     // batched kernel's shared work list; with "auto" it takes the kernel that is fastest for a lone call of its kind.
     const bool whole_group = group_ends && e->grp_pend_only;
@@ -1004,11 +1042,7 @@ static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
             }
         }
     }
-    e->pend.clear();
-    for (mlxn_buffer *b : e->retained) {
-        std::lock_guard<std::mutex> lk(b->st->mu);
-        if (b->st->pend_enc == e) b->st->pend_enc = nullptr;
-    }
+    leave();
     if (rc) return rc;
     if (err != cudaSuccess) return cuda_fail(err, "mat-vec launch");
     g_launches.fetch_add((uint64_t)launches);
@@ -1427,7 +1461,7 @@ static bool op_conflicts(mlxn_encoder *e, std::initializer_list<OpBuf> bufs, int
 // that batch's lane; everything else alternates.
 static int op_lane(const mlxn_encoder *e, bool joins_batch) {
     const bool first = e->grp_reads.empty() && e->grp_writes.empty();
-    return first ? 0 : (joins_batch && !e->pend.empty()) ? e->pend_lane : (e->cur_lane + 1) % kLanes;
+    return first ? 0 : (joins_batch && e->pending()) ? e->pend_lane : (e->cur_lane + 1) % kLanes;
 }
 // `ordered_in_batch`: the operation joins the pending batch as a dependent mat-vec (the batch's kernel orders it after
 // the ones it conflicts with), so a conflict does not end the group.
@@ -1588,7 +1622,7 @@ static int batch_mv(mlxn_encoder *enc, int type, const QmvArgs &a, uint32_t mp, 
                       enc->pend.size() < kMvSplitMax && h->ids == a.ids && h->nprob == a.nprob && h->n_experts == a.n_experts &&
                       (a.ids ? h->k == a.k : a.m <= 8 || h->m == a.m);
     int rc;
-    if (h && !fits && (rc = encoder_flush_pending(enc))) return rc;
+    if (enc->pending() && !fits && (rc = encoder_flush_pending(enc))) return rc;
     if ((rc = op_begin(enc, bufs, true))) return rc;
     if (enc->pend.empty()) {   // (a conflict found by op_begin has launched the batch and started a new group)
         enc->pend_type = type;
@@ -1675,7 +1709,7 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
             const bool pair = qmv_mma_pair_mode((int)p->ggml_type, a0);
             const bool fits = batch && !enc->pend.empty() && !enc->pend_split && enc->pend_type == (int)p->ggml_type &&
                               enc->pend_mp == mv_row_class(a0.m) && enc->pend_pair == pair && enc->pend.size() < kMvBatchMax;
-            if (!enc->pend.empty() && !fits && (rc = encoder_flush_pending(enc))) return rc;
+            if (enc->pending() && !fits && (rc = encoder_flush_pending(enc))) return rc;
             // A mat-vec that depends on the batch it would join (it reads a result of the batch, or writes over one)
             // still joins it when the group holds nothing but that batch: the kernel then starts it after the
             // mat-vecs ahead of it (a barrier across its grid) while the weights keep streaming.
@@ -1743,7 +1777,7 @@ static int dispatch_mm(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
                        mlxn_buffer *output, const mlxn_qmm_params *p, const ShardOut *sh = nullptr) {
     int rc = touch_kernel(reg, dev, mm_kernel_name((int)p->ggml_type));
     if (rc) return rc;
-    if ((rc = op_begin(enc, {{input, false}, {weight, false}, {output, true}}))) return rc;
+    const bool tc = sh || opt_qmm_tc();
     QmmArgs a{};
     a.w = weight->dev();
     a.x = reinterpret_cast<const float *>(input->dev());
@@ -1763,7 +1797,27 @@ static int dispatch_mm(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
         if (!qmm_tc_supported(a))
             return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: quantized_matmul_ggml_sharded: the mat-mat form needs K to be a multiple of 32");
     }
-    if ((sh || opt_qmm_tc()) && qmm_tc_supported(a)) {
+    // A mat-mat that goes to pairs of SMs waits for others of the same activations (q, k and v; gate and up) to share its launch.
+    const int type = (int)p->ggml_type;
+    if (tc && !sh && g_opt_mv_batch.load() && qmm_tc_supported(a) && qmm_duo_cost(type, a, 32) != ~0ull) {
+        const QmmArgs *h = enc->pend_mm.empty() ? nullptr : &enc->pend_mm[0];
+        const bool fits = h && enc->pend_type == type && enc->pend_mm.size() < kMmBatchMax && h->x == a.x && h->m == a.m && h->k == a.k;
+        if (enc->pending() && !fits && (rc = encoder_flush_pending(enc))) return rc;
+        if ((rc = op_begin(enc, {{input, false}, {weight, false}, {output, true}}, true))) return rc;
+        if (enc->pend_mm.empty()) {   // (a conflict found by op_begin has launched the batch and started a new group)
+            enc->pend_type = type;
+            enc->pend_lane = enc->cur_lane;
+        }
+        enc->pend_mm.push_back(a);
+        for (mlxn_buffer *b : {input, weight, output}) {
+            std::lock_guard<std::mutex> lk(b->st->mu);
+            b->st->pend_enc = enc;
+        }
+        g_dispatch.fetch_add(1);
+        return MLXN_OK;
+    }
+    if ((rc = op_begin(enc, {{input, false}, {weight, false}, {output, true}}))) return rc;
+    if (tc && qmm_tc_supported(a)) {
         const uint32_t nt = qmm_tc_pick_nt((int)p->ggml_type, a, dev->sm_count, sh != nullptr);
         uint8_t *scratch = nullptr;
         if ((rc = encoder_scratch(enc, qmm_tc_scratch_bytes(a, nt, false), &scratch))) return rc;
@@ -2004,7 +2058,7 @@ static int dispatch_id_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *de
         const bool batch = g_opt_mv_batch.load() != 0;
         const bool fits = batch && !enc->pend.empty() && !enc->pend_split && enc->pend_type == t && enc->pend_mp == 1 && !enc->pend_pair &&
                           enc->pend.size() + rows <= kMvBatchMax;
-        if (!enc->pend.empty() && !fits && (rc = encoder_flush_pending(enc))) return rc;
+        if (enc->pending() && !fits && (rc = encoder_flush_pending(enc))) return rc;
         if ((rc = op_begin(enc, {{input, false}, {up, false}, {weight, false}, {ids, false}, {output, true}}, true))) return rc;
         if (enc->pend.empty()) {
             enc->pend_type = t;

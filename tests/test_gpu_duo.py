@@ -76,3 +76,68 @@ def test_infinities_stay_in_their_row(ctx):
     assert np.isfinite(y[~bad]).all() and not np.isfinite(y[bad]).any(axis=1).all()
     y_ref, ad = orc.qmatmul(otype, wq, x[~bad], n, k, nthreads=4, f16_operands=True)
     assert norm_err(y[~bad], y_ref, ad) <= TOL
+
+
+def test_products_of_one_group_share_a_launch(ctx):
+    """Between two barriers: three products of the same activations are packed once and leave as one kernel; one of another type and one of
+    other activations do not join them; a dependent one starts a new group.  Row counts that leave part of a tile between two products."""
+    d, m, k = ctx.device, 70, 1024
+    gtype, otype = TYPES["Q4_0"]
+    x, x2 = normal_acts(1, m, k), normal_acts(2, m, k)
+    ns = (264, 512, 136)
+    ws = [normal_weights(i, n, k, otype) for i, n in enumerate(ns)]
+    w8 = normal_weights(9, 256, k, orc.Q8_0)
+    wd = normal_weights(8, 40, 512, otype)
+    xb, x2b = ctx.buf(x, mx.DType.F32), ctx.buf(x2, mx.DType.F32)
+    P = mx.GgmlQuantizedMatmulParams
+    out = lambda n: d.alloc_buffer(m * n * 4, mx.DType.F32)
+    ys, y8, yx, yd = [out(n) for n in ns], out(256), out(264), out(40)
+    for capture in (False, True):
+        enc = d.command_encoder()
+
+        def encode():
+            for w, y, n in zip(wbufs, ys, ns):
+                mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, w, y, P(m, n, k, gtype))
+            mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, w8b, y8, P(m, 256, k, TYPES["Q8_0"][0]))
+            mx.quantized_matmul_ggml(enc, ctx.registry, d, x2b, wbufs[0], yx, P(m, 264, k, gtype))
+            mx.quantized_matmul_ggml(enc, ctx.registry, d, ys[1], wdb, yd, P(m, 40, 512, gtype))
+
+        wbufs, w8b, wdb = [ctx.buf(w, mx.DType.U8) for w in ws], ctx.buf(w8, mx.DType.U8), ctx.buf(wd, mx.DType.U8)
+        mx.reset_counters()
+        encode()
+        enc.commit_and_wait()
+        assert mx.kernel_launch_count() == 2 * 4
+        if capture:
+            enc.begin_capture()
+            encode()
+            graph = enc.end_capture()
+            graph.launch(enc)
+            enc.commit_and_wait()
+        refs = [(y, n, w, otype, x, k) for y, n, w in zip(ys, ns, ws)] + [(y8, 256, w8, orc.Q8_0, x, k), (yx, 264, ws[0], otype, x2, k)]
+        for y, n, w, o, xx, kk in refs:
+            y_ref, ad = orc.qmatmul(o, w, xx, n, kk, nthreads=4, f16_operands=True)
+            assert norm_err(y.as_slice(np.float32).reshape(m, n), y_ref, ad) <= TOL
+        mid = ys[1].as_slice(np.float32).reshape(m, 512).copy()
+        y_ref, ad = orc.qmatmul(otype, wd, mid, 40, 512, nthreads=4, f16_operands=True)
+        assert norm_err(yd.as_slice(np.float32).reshape(m, 40), y_ref, ad) <= TOL
+
+
+def test_products_of_one_group_over_shared_ranges(ctx):
+    """Two products whose tiles together are more than the pairs of SMs, cut into equal ranges: the zeroed tiles are those of both."""
+    gtype, otype = TYPES["Q4_0"]
+    d, m, n, k = ctx.device, 16, 10240, 2048
+    part = normal_weights(4, 1024, k, otype)
+    x = normal_acts(4, m, k)
+    y_ref, ad = orc.qmatmul(otype, part, x, 1024, k, nthreads=8, f16_operands=True)
+    xb, wb = ctx.buf(x, mx.DType.F32), ctx.buf(np.tile(part, n // 1024), mx.DType.U8)
+    ys = [ctx.buf(np.full(m * n, 7, np.float32), mx.DType.F32) for _ in range(2)]
+    enc = d.command_encoder()
+    mx.reset_counters()
+    for y in ys:
+        mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, wb, y, mx.GgmlQuantizedMatmulParams(m, n, k, gtype))
+    enc.commit_and_wait()
+    assert mx.kernel_launch_count() == 2
+    for y in ys:
+        got = y.as_slice(np.float32).reshape(m, n)
+        for at in range(0, n, 1024):
+            assert norm_err(got[:, at:at + 1024], y_ref, ad) <= TOL
