@@ -128,7 +128,8 @@ struct QmmArgs {
     const uint16_t *x_bf16;
     uint32_t head_dim;
     // Fused MoE layer (routed tensor-core form): what an earlier call of the same layer has left in the scratch area and
-    // this call takes over instead of building it again (bit 0: the tile list, bit 1: the packed activations), and the
+    // this call takes over instead of building it again (bit 0: the tile list, bit 1: the packed activations), whether it needs
+    // nothing from the kernel directly ahead in the stream, only from those before it (bit 2), and the
     // second operand of a SwiGLU formed while packing: activations = silu(x) * x2 (src/shaders/silu_mul.metal:17-30).
     uint32_t reuse;
     const float *x2;

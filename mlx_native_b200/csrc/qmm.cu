@@ -300,10 +300,9 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
 // =================================================================================================
 // qmm_tc
 // =================================================================================================
-// Dequantising warps of a CTA: 16 in two sets of 8, set s dequantises the K stages with st % 2 == s; or, with two CTAs on an SM (PAIR),
-// one set that takes all stages.  Beside them the activation producer, MMA, weight producer and second MMA warp.
-__host__ __device__ constexpr int tc_dequant_warps(bool pair) { return pair ? 8 : 16; }
-__host__ __device__ constexpr int tc_threads(bool pair) { return (tc_dequant_warps(pair) + 4) * 32; }
+// Dequantising warps: 16 in two sets of 8, set s dequantises the K stages with st % 2 == s.  Beside them the activation producer, MMA,
+// weight producer and second MMA warp.
+constexpr int kTcDequantWarps = 16, kTcThreads = (kTcDequantWarps + 4) * 32;
 constexpr int kTcRowsW = 128;                           // weight rows per tile (UMMA M)
 
 template <int T> struct TcTraits;
@@ -344,14 +343,14 @@ struct TcCfg {
 // ring of dequantised weight stages held in tensor memory: the columns the accumulators leave free.  Tiles of 64
 // activation rows (two 64-column accumulators) keep six stages in columns [128, 512), wider ones four in [256, 512):
 // the ring's depth over the latency of the loop dequantise -> MMA -> commit -> reuse is what bounds a narrow tile.
-template <int NT, bool PAIR> struct TcRing {
-    static constexpr int kStages = PAIR ? 3 : NT <= 64 ? 6 : 4;
-    static constexpr int kColBase = PAIR ? 64 : NT <= 64 ? 128 : 256;
+template <int NT> struct TcRing {
+    static constexpr int kStages = NT <= 64 ? 6 : 4;
+    static constexpr int kColBase = NT <= 64 ? 128 : 256;
 };
 constexpr int kTcACols = 64;       // one stage: 128 K values as f16 pairs = 64 32-bit columns
-constexpr int kTcTmemCols = 512;   // of an SM: two CTAs have half each
+constexpr int kTcTmemCols = 512;
 
-// grid = min(work items, SMs) persistent CTAs; tc_threads(PAIR) threads; 1 CTA per SM, or 2 (PAIR).
+// grid = min(work items, SMs) persistent CTAs, one per SM; kTcThreads threads.
 //
 // Data flow per work item (one 128-row weight tile x one NT-row activation tile, all of K or, where tiles are shared, a part of it):
 //   raw GGML blocks  --cp.async-->  shared-memory ring  --dequantise (16 warps)-->  f16 pairs in registers
@@ -359,23 +358,17 @@ constexpr int kTcTmemCols = 512;   // of an SM: two CTAs have half each
 //   ring in shared memory-->  f32 accumulator in tensor memory  --tcgen05.ld-->  y.
 // The dequantised weights never touch shared memory: its bandwidth is the scarce resource here (the tensor
 // core already reads the whole activation tile from it for every MMA).
-//
-// PAIR: two CTAs per SM, each with one set of dequantising warps, one accumulator and half of tensor memory.  For routed calls, whose
-// items are short (64 rows, K of a few raw stages): what an item costs beside its stages -- accumulator drain, read-back, the first
-// stages of the next one, 5000 cycles -- is then time in which the other CTA works.  128 experts, 512 tokens, 8 of them each: Q4_0
-// 768 x 2048 80 -> 62 us, Q6_K 2048 x 768 (rows of 630 bytes, now tensor copies) 175 -> 102 us; weights once at 6.4 TB/s: 18 and 25 us.
-template <int T, int NT, bool SH, bool PAIR>
-__global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(const QmmArgs a, const TcCfg c, const uint8_t *xpack,
-                                                                const __grid_constant__ CUtensorMap wmap) {
+template <int T, int NT, bool SH>
+__global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, const TcCfg c, const uint8_t *xpack,
+                                                               const __grid_constant__ CUtensorMap wmap) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // tensor-core operand tiles need 1024-byte alignment (128-byte swizzle atoms): align by hand
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES, KR = TcTraits<T>::KR;
-    constexpr int kMaxB = PAIR ? 6 : 8, kMaxRaw = 6, kTcDequantWarps = tc_dequant_warps(PAIR);
-    constexpr int kTcAStages = TcRing<NT, PAIR>::kStages, kTcAColBase = TcRing<NT, PAIR>::kColBase;
-    static_assert(!PAIR || (NT == 64 && !SH), "two CTAs per SM: tiles of 64 rows");
+    constexpr int kMaxB = 8, kMaxRaw = 6;
+    constexpr int kTcAStages = TcRing<NT>::kStages, kTcAColBase = TcRing<NT>::kColBase;
     static_assert(kMaxB / 2 <= kTcAStages, "an activation chunk's place is freed by a stage_done phase the producer can still see");
-    constexpr int kNumMma = PAIR || NT > 128 ? 1 : 2;   // issuing threads, each with its own accumulator
+    constexpr int kNumMma = NT > 128 ? 1 : 2;   // issuing threads, each with its own accumulator
     __shared__ __align__(8) uint64_t a_full[kTcAStages], stage_done[kTcAStages], b_full[kMaxB];
     __shared__ __align__(8) uint64_t raw_full[kMaxRaw], raw_empty[kMaxRaw], acc_full, acc_empty, orow_ready[2], stage_ready[2];
     __shared__ uint32_t tmem_base_s;
@@ -392,7 +385,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t tid = threadIdx.x - kCtrlWarps * 32;   // index among the dequantising threads (wraps for warps 0-3)
     const uint32_t row_bytes = (a.k / QK) * BB;
-    const bool raw_tma = PAIR || c.raw_tma != 0;
+    const bool raw_tma = c.raw_tma != 0;
 
     // ---- set-up that needs nothing from the kernels ahead in the stream (it overlaps their tail: the kernel is
     // ---- launched with programmatic stream serialisation), then the wait for them
@@ -421,7 +414,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
         mbar_init_fence();
     }
     if (warp == kWarpMma0) {  // the first MMA warp owns tensor memory
-        tmem_alloc(&tmem_base_s, kTcTmemCols / (PAIR ? 2 : 1));
+        tmem_alloc(&tmem_base_s, kTcTmemCols);
         tmem_relinquish();
     }
     grid_dependency_wait();   // the packed activations, the tile list and the zeros of shared tiles are complete
@@ -433,8 +426,8 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
     const uint32_t n_tt = a.hids ? min(a.tiles[0], c.ntiles) : c.ntiles;   // uniform for the whole CTA
     const uint32_t total_items = c.n_wt * n_tt;
     const uint32_t nraw_all = (a.k + KR - 1) / KR;
-    const bool shared = !PAIR && c.share.ctas != 0;
-    const uint32_t nt = PAIR ? (uint32_t)NT : c.nt;
+    const bool shared = c.share.ctas != 0;
+    const uint32_t nt = c.nt;
     const uint32_t pos0 = shared ? c.share.begin(blockIdx.x) : blockIdx.x, pos1 = shared ? c.share.begin(blockIdx.x + 1) : total_items;
     struct Item {
         uint32_t tt, e, mt, n0, r_lo, nraw, nst, nck, kc_lo, next;
@@ -651,7 +644,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
         // 32 (w % 4) + l of the tile -- the tensor-memory lane its warp may address -- and the 64-element half
         // (w / 4) % 2 of the stage: thirty-two packed f16 pairs = one 32-column store.
         const uint32_t dw = warp - kCtrlWarps;   // 0..15
-        const uint32_t q4 = dw & 3u, half = (dw >> 2) & 1u, set0 = dw >> 3;
+        const uint32_t q4 = dw & 3u, half = (dw >> 2) & 1u, set = dw >> 3;
         const uint32_t rr = q4 * 32 + lane;
         const uint32_t srow = ((rr & ((1u << c.row_group) - 1u)) << (7 - c.row_group)) + (rr >> c.row_group);   // the row's place in a raw stage
         // Raw weight rows are short (144..272 bytes per stage and row), too short for one bulk copy each to be
@@ -663,7 +656,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
         constexpr int kRawSlots = 5;            // (128 rows x at most 19 chunks) / 512 threads, rounded up
         constexpr uint32_t kSegFull = (KR / QK) * BB;
         constexpr uint32_t kCmax = (kSegFull + 30u) >> 4;  // most 16-byte chunks a row segment can need
-        static_assert(PAIR || kTcRowsW * kCmax <= kRawSlots * kTcDequantWarps * 32, "raw copy slots");
+        static_assert(kTcRowsW * kCmax <= kRawSlots * kTcDequantWarps * 32, "raw copy slots");
         static_assert(KR == 256, "a raw stage feeds one K stage of each set");
         const uint8_t *slot_src[kRawSlots];     // start of the thread's row (global), for the item being requested
         uint32_t slot_dst[kRawSlots];           // row's place inside a raw stage + chunk offset (shared, relative)
@@ -724,7 +717,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
             // the item's output-row table: every thread fetches the entries it will publish now (the loads stay in
             // flight behind the K loop) and stores them just before the epilogue
             static_assert(NT <= kTcDequantWarps * 32, "one output-row entry per thread");
-            if (q4 == 0 && half == 0) TRACE(2 + set0, 1, nitem);
+            if (q4 == 0 && half == 0) TRACE(2 + set, 1, nitem);
             uint32_t o_nrows = a.m;
             int32_t o_id = -1;
             const uint32_t o_row = it.mt * nt + tid;
@@ -750,8 +743,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
                 }
                 if (!ok) break;
                 if (!mbar_wait(&raw_full[rs], rph, &abort_flag, a.status, ST_WAIT_FULL_TIMEOUT, wmode_dq)) { ok = false; break; }
-                if (q4 == 0 && half == 0) TRACE(2 + set0, 2, r);
-                for (uint32_t set = set0; set < 2; set += kTcDequantWarps / 8) {   // (PAIR: the one set takes both K stages)
+                if (q4 == 0 && half == 0) TRACE(2 + set, 2, r);
                 const uint32_t st = 2 * r + set;       // this set's K stage inside raw stage r
                 if (st < it.nst) {
                     const uint32_t J = J0 + st;        // its number in the CTA's whole run
@@ -764,7 +756,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
                         break;
                     }
                     tc_fence_after();
-                    if (q4 == 0 && half == 0) TRACE(2 + set0, 3, r);
+                    if (q4 == 0 && half == 0) TRACE(2 + set, 3, r);
                     const uint32_t r_abs = it.r_lo + r;
                     const uint32_t pre = (row_lo4 + ((r_abs * KR) / QK) * BB) & 15u;
                     const uint32_t seg = smem_base + c.raw_off + rs * raw_stage_bytes + srow * c.seg_stride + pre;
@@ -802,20 +794,18 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
                         }
                     }
                 }
-                    if (q4 == 0 && half == 0) TRACE(2 + set0, 8, r);
+                    if (q4 == 0 && half == 0) TRACE(2 + set, 8, r);
                     tmem_st_32x32_x32(a_dst + sa * kTcACols, regs);
                     tmem_st_wait();
-                    if (q4 == 0 && half == 0) TRACE(2 + set0, 9, r);
+                    if (q4 == 0 && half == 0) TRACE(2 + set, 9, r);
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&a_full[sa]);
-                    if (q4 == 0 && half == 0) TRACE(2 + set0, 4, r);
+                    if (q4 == 0 && half == 0) TRACE(2 + set, 4, r);
                 }
-                }
-                if (!ok) break;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&raw_empty[rs]);  // this warp is done reading the raw stage
-                if (q4 == 0 && half == 0) TRACE(2 + set0, 10, r);
+                if (q4 == 0 && half == 0) TRACE(2 + set, 10, r);
                 consumed++;
                 if (++rs == R) { rs = 0; rph ^= 1u; }
             }
@@ -839,10 +829,10 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
                 if (lane == 0) mbar_arrive(&orow_ready[nitem & 1u]);
             }
             if (!mbar_wait(&orow_ready[nitem & 1u], (nitem >> 1) & 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, wmode_dq)) break;
-            if (q4 == 0 && half == 0) TRACE(2 + set0, 5, nitem);
+            if (q4 == 0 && half == 0) TRACE(2 + set, 5, nitem);
             if (!mbar_wait(&acc_full, nitem & 1u, &abort_flag, a.status, ST_WAIT_MMA_TIMEOUT, wmode_dq)) break;
             tc_fence_after();
-            if (q4 == 0 && half == 0) TRACE(2 + set0, 6, nitem);
+            if (q4 == 0 && half == 0) TRACE(2 + set, 6, nitem);
             const int32_t *tab = orow[nitem & 1u];
             const uint32_t wrow = n0 + rr;
             const bool part = it.nraw < nraw_all;   // another CTA has the rest of this tile's K
@@ -891,7 +881,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
                         }
                     }
                 }
-                if (q4 == 0 && half == 0) TRACE(2 + set0, 7, nitem);
+                if (q4 == 0 && half == 0) TRACE(2 + set, 7, nitem);
                 continue;
             }
 #pragma unroll 1
@@ -932,7 +922,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty);   // the MMA warp may start the next item's accumulation
-            if (q4 == 0 && half == 0) TRACE(2 + set0, 7, nitem);
+            if (q4 == 0 && half == 0) TRACE(2 + set, 7, nitem);
         }
     }
     if (abort_flag) {  // let copies in flight land before the CTA's shared memory is released
@@ -942,7 +932,7 @@ __global__ void __launch_bounds__(tc_threads(PAIR), PAIR ? 2 : 1) qmm_tc_kernel(
     __syncthreads();
     if (warp == kWarpMma0) {
         tc_fence_after();
-        tmem_dealloc(tmem_d, kTcTmemCols / (PAIR ? 2 : 1));
+        tmem_dealloc(tmem_d, kTcTmemCols);
     }
 }
 
@@ -1058,7 +1048,7 @@ bool qmm_tc_supported(const QmmArgs &a) {
     return true;
 }
 
-template <int T, int NT, bool SH, bool PAIR = false>
+template <int T, int NT, bool SH>
 static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint32_t nt, uint8_t *scratch, cudaStream_t st, int *launches) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES, KR = TcTraits<T>::KR;
     TcCfg c{};
@@ -1107,15 +1097,13 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint32_t nt, uint8_t *sc
             }
         }
     }
-    if (PAIR && !c.raw_tma) return launch_tc_tn<T, NT, SH, false>(a, routed, nt, scratch, st, launches);
     const uint32_t b_bytes = nt * 128;  // one 64-wide K chunk of the activation tile
     const uint32_t raw_slot = kTcRowsW * c.seg_stride;
-    // + 1 KB alignment slack + 1 to 3 KB of static shared memory: 227 KB, or half of 228 KB less the 1 KB that the system takes of each CTA
-    uint32_t limit = (PAIR ? 108 : 222) * 1024;
+    uint32_t limit = 222 * 1024;   // + 1 KB alignment slack + 1 to 3 KB of static shared memory: 227 KB
     // narrow tiles stage their result in shared memory (two tiles of NT x 132 floats) and write whole output rows
     const uint32_t stage_bytes = 2u * NT * (kTcRowsW + 4) * 4u;
     // (the row-sharded form never shares tiles: they go straight to every rank's buffer)
-    const bool staged = NT == 64 && !PAIR && !plan.shared &&
+    const bool staged = NT == 64 && !plan.shared &&
                         ((((uintptr_t)a.y) | ((uintptr_t)qmm_ld(a) * 4u) | ((uintptr_t)a.y_col0 * 4u)) & 15u) == 0 && a.n_peer == 0 &&
                         !exp_env("MLXN_TC_NO_STAGED_OUT");
     if (staged) limit -= stage_bytes;
@@ -1123,7 +1111,7 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint32_t nt, uint8_t *sc
     uint32_t b_stages = (limit - 2 * raw_slot) / b_bytes;
     // (a 64-row tile's chunks are 8 KB: eight of them where four raw slots still fit beside them, the loop being
     // bound by how far the copies run ahead of the MMAs)
-    const uint32_t b_cap = (NT == 64 && !PAIR && limit >= 8 * b_bytes + 4 * raw_slot) ? 8u : 6u;
+    const uint32_t b_cap = (NT == 64 && limit >= 8 * b_bytes + 4 * raw_slot) ? 8u : 6u;
     if (b_stages > b_cap) b_stages = b_cap;
     if (const char *e = exp_env("MLXN_TC_STAGES")) {  // experiment switch
         const uint32_t v = (uint32_t)atoi(e);
@@ -1181,36 +1169,36 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint32_t nt, uint8_t *sc
         cudaError_t e = launch_overlapped(pack_x_kernel, grid, dim3(256), 0, st, a, xpack, c.nchunks, nt, c.share, res);
         if (e != cudaSuccess) return e;
     }
+    if (routed && !SH && qmm_duo_routed_fits(T, a)) return launch_qmm_duo_routed(T, a, (uint32_t)tiles, xpack, st, launches);
     static size_t attr_smem[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (smem > attr_smem[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(qmm_tc_kernel<T, NT, SH, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(qmm_tc_kernel<T, NT, SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         attr_smem[dev] = smem;
     }
-    // persistent CTAs, one per SM (PAIR: two), each walking its items
+    // persistent CTAs, one per SM, each walking its items
     uint32_t ctas = plan.ctas;
     if (routed) {
         const uint64_t items = (uint64_t)c.n_wt * tiles;
-        ctas = (uint32_t)sm_count_of_device() * (PAIR ? 2u : 1u);
+        ctas = (uint32_t)sm_count_of_device();
         if (items < ctas) ctas = (uint32_t)items;
     }
     if (ctas == 0) return cudaSuccess;
     (*launches)++;
-    return launch_overlapped(qmm_tc_kernel<T, NT, SH, PAIR>, dim3(ctas), dim3(tc_threads(PAIR)), smem, st, a, c, xpack, wmap);
+    return launch_overlapped(qmm_tc_kernel<T, NT, SH>, dim3(ctas), dim3(kTcThreads), smem, st, a, c, xpack, wmap);
 }
 
 template <int T> static cudaError_t launch_tc_t(const QmmArgs &a, bool routed, uint32_t nt, uint8_t *scratch, cudaStream_t st,
                                                 int *launches) {
-    if (nt == 0 || nt % 16 != 0 || nt > 256 || (routed && nt != 64)) return cudaErrorInvalidValue;
+    if (nt == 0 || nt % 16 != 0 || nt > 256 || (routed && nt != kRoutedTile)) return cudaErrorInvalidValue;
     if (a.y_ld != 0 || a.n_peer != 0) {   // row-sharded result: the instantiation with the peer stores
         if (nt <= 64) return launch_tc_tn<T, 64, true>(a, routed, nt, scratch, st, launches);
         if (nt <= 128) return launch_tc_tn<T, 128, true>(a, routed, nt, scratch, st, launches);
         return launch_tc_tn<T, 256, true>(a, routed, nt, scratch, st, launches);
     }
-    if (routed) return launch_tc_tn<T, 64, false, true>(a, routed, nt, scratch, st, launches);
     if (nt <= 64) return launch_tc_tn<T, 64, false>(a, routed, nt, scratch, st, launches);
     if (nt <= 128) return launch_tc_tn<T, 128, false>(a, routed, nt, scratch, st, launches);
     return launch_tc_tn<T, 256, false>(a, routed, nt, scratch, st, launches);

@@ -38,5 +38,8 @@ int sm_count_of_device();
 // `nt` as for the other kernel, a multiple of 32.
 uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt);
 cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches);
+constexpr uint32_t kRoutedTile = 64;   // rows of a routed tile
+bool qmm_duo_routed_fits(int ggml_type, const QmmArgs &a);
+cudaError_t launch_qmm_duo_routed(int ggml_type, const QmmArgs &a, uint32_t tiles, const uint8_t *xpack, cudaStream_t st, int *launches);
 
 }  // namespace mlxn

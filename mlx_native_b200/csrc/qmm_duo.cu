@@ -31,7 +31,8 @@ namespace mlxn {
 
 constexpr uint32_t kDuoRows = 256;                          // weight rows of a pair's tile
 constexpr uint32_t kDuoDequantWarps = 16;                   // two sets of eight; set s takes the 128-wide K stages st % 2 == s
-constexpr uint32_t kDuoThreads = (4 + kDuoDequantWarps) * 32;
+constexpr uint32_t kDuoReadWarps = 8;                       // read the accumulators back
+constexpr uint32_t kDuoThreads = (4 + kDuoDequantWarps + kDuoReadWarps) * 32;
 constexpr uint32_t kDuoStages = 4;                          // ring of K stages: activations in shared memory, weights in tensor memory
 constexpr uint32_t kDuoACol = 256, kDuoACols = 64;          // tensor-memory columns of the weights: 64 a stage (128 f16 pairs)
 constexpr uint32_t kDuoMaxRaw = 5;
@@ -46,6 +47,7 @@ struct DuoCfg {
     uint32_t raw_off, raw_slots;
     uint32_t row_group;   // log2 of the copies of a raw stage (see launch_tc_tn)
     uint32_t aligned;     // every weight row starts on a 16-byte boundary
+    uint32_t beside;      // nothing here depends on the kernel ahead, whose own dependences have been waited for: wait for it in the end
     TcOut out;
 };
 struct DuoMaps {
@@ -100,9 +102,13 @@ __device__ __forceinline__ void commit_both(uint64_t *bar) {
 //   warp 0        activations: one bulk copy per K stage (two 64-wide chunks of its half of the tile)
 //   warp 1        CTA 0: MMAs of the pair, whose completion frees the stage's places in both CTAs; CTA 1: tells CTA 0 that its stage is ready
 //   warp 2        raw weights: tensor copies of 128 rows x 256 K values
-//   warps 4..19   dequantise raw blocks into tensor memory; read the accumulator back
+//   warps 4..19   dequantise raw blocks into tensor memory
+//   warps 20..27  read the accumulator back; tiles of up to 128 rows have two accumulators, so that the next item's multiplications go on
 // Ring places and barrier phases run on across the items of a pair.
-template <int T>
+//
+// ROUTED: the products of a mixture of experts.  The tiles are those of the list that build_tiles_kernel made, 64 rows of one expert each,
+// packed whole (a CTA's half are rows 0..31 or 32..63 of each 64-column chunk); the weights' map has the expert as third dimension.
+template <int T, bool ROUTED>
 __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
     qmm_duo_kernel(const QmmArgs a, const __grid_constant__ DuoCfg c, const uint8_t *xpack, const __grid_constant__ DuoMaps wmaps) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
@@ -110,7 +116,7 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // (the same in both CTAs)
     __shared__ __align__(8) uint64_t full[kDuoStages], peer_full[kDuoStages], done[kDuoStages], raw_full[kDuoMaxRaw], raw_empty[kDuoMaxRaw];
-    __shared__ __align__(8) uint64_t acc_full, acc_empty;
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_s;
     __shared__ volatile uint32_t abort_flag;
     const uint32_t lane = threadIdx.x & 31u, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
@@ -126,8 +132,10 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
             mbar_init(&raw_full[s], 1);
             mbar_init(&raw_empty[s], kDuoDequantWarps);
         }
-        mbar_init(&acc_full, 1);
-        mbar_init(&acc_empty, 2 * kDuoDequantWarps);   // (of CTA 0: the warps of both)
+        for (uint32_t s = 0; s < 2; s++) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], 2 * kDuoReadWarps);   // (of CTA 0: the warps of both)
+        }
         mbar_init_fence();
     }
     if (warp == 3) {
@@ -139,12 +147,13 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
     duo::cluster_sync();
     tc_fence_after();
     const uint32_t tmem = tmem_s;
-    grid_dependency_wait();   // the packed activations and the zeros of shared tiles are complete
+    if (!c.beside) grid_dependency_wait();   // the packed activations, the tile list and the zeros of shared tiles are complete
     allow_dependents();
 
     // ---- work items: weight tile fastest, so that the pairs working at the same time share an activation tile in L2 ----
-    const uint32_t nraw_all = (a.k + KR - 1) / KR, total_items = c.n_wt * c.ntiles;
-    const bool shared = c.share.ctas != 0;
+    const uint32_t nraw_all = (a.k + KR - 1) / KR, total_items = c.n_wt * (ROUTED ? min(__ldcg(a.tiles), c.ntiles) : c.ntiles);
+    const bool shared = !ROUTED && c.share.ctas != 0;
+    const uint32_t accs = c.nt <= 128 ? 2 : 1;   // accumulators, 128 columns apart
     const uint32_t pos0 = shared ? c.share.begin(pair) : pair, pos1 = shared ? c.share.begin(pair + 1) : total_items;
     struct Item {
         uint32_t tt, op, n0, r_lo, nraw, nst, kc_lo, nck, next;
@@ -175,8 +184,9 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
         for (uint32_t pos = pos0; ok && pos < pos1;) {
             const Item it = load_item(pos);
             pos = it.next;
-            const uint8_t *src = xpack + ((size_t)(it.tt * 2u + rank) * c.nchunks + it.kc_lo) * b_chunk;
-            for (uint32_t st = 0; st < it.nst; st++, src += b_stage) {
+            const uint8_t *src = ROUTED ? xpack + ((size_t)it.tt * c.nchunks + it.kc_lo) * b_stage + rank * b_chunk
+                                        : xpack + ((size_t)(it.tt * 2u + rank) * c.nchunks + it.kc_lo) * b_chunk;
+            for (uint32_t st = 0; st < it.nst; st++, src += ROUTED ? 2 * b_stage : b_stage) {
                 if (!mbar_wait(&done[s], ph, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, kSpin)) {
                     ok = false;
                     break;
@@ -184,7 +194,12 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
                 if (duo::elect()) {
                     const uint32_t bytes = 2 * st + 1 < it.nck ? b_stage : b_chunk;   // (a K tail of 64)
                     mbar_expect_tx(&full[s], bytes);
-                    bulk_g2s(smem + s * b_stage, src, bytes, &full[s]);
+                    if constexpr (ROUTED) {
+                        bulk_g2s(smem + s * b_stage, src, b_chunk, &full[s]);
+                        if (bytes == b_stage) bulk_g2s(smem + s * b_stage + b_chunk, src + b_stage, b_chunk, &full[s]);
+                    } else {
+                        bulk_g2s(smem + s * b_stage, src, bytes, &full[s]);
+                    }
                 }
                 __syncwarp();
                 if (++s == kDuoStages) {
@@ -200,8 +215,9 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
         for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
             const Item it = load_item(pos);
             pos = it.next;
-            // the accumulator of the item before has been read back
-            if (rank == 0 && nitem > 0 && !mbar_wait(&acc_empty, (nitem - 1) & 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, kSpin)) break;
+            const uint32_t buf = accs == 2 ? nitem & 1u : 0u, turn = accs == 2 ? nitem >> 1 : nitem, d = tmem + buf * 128;
+            // the accumulator's item before has been read back
+            if (rank == 0 && !mbar_wait(&acc_empty[buf], (turn & 1u) ^ 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, kSpin)) break;
             tc_fence_after();
             for (uint32_t st = 0; st < it.nst; st++) {
                 if (!mbar_wait(&full[s], ph, &abort_flag, a.status, ST_WAIT_FULL_TIMEOUT, kSpin)) {
@@ -219,10 +235,10 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
                         const uint32_t ac = tmem + kDuoACol + s * kDuoACols;
                         const uint64_t bd = bd0 + s * (b_stage >> 4), bd1 = bd + (b_chunk >> 4);
 #pragma unroll
-                        for (uint32_t q = 0; q < 4; q++) duo::mma(tmem, ac + 8 * q, bd + 2 * q, idesc, (st | q) ? 1u : 0u);
+                        for (uint32_t q = 0; q < 4; q++) duo::mma(d, ac + 8 * q, bd + 2 * q, idesc, (st | q) ? 1u : 0u);
                         if (2 * st + 1 < it.nck) {
 #pragma unroll
-                            for (uint32_t q = 0; q < 4; q++) duo::mma(tmem, ac + 32 + 8 * q, bd1 + 2 * q, idesc, 1u);
+                            for (uint32_t q = 0; q < 4; q++) duo::mma(d, ac + 32 + 8 * q, bd1 + 2 * q, idesc, 1u);
                         }
                         duo::commit_both(&done[s]);
                     }
@@ -237,7 +253,7 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
                 }
             }
             if (!ok) break;
-            if (rank == 0 && duo::elect()) duo::commit_both(&acc_full);
+            if (rank == 0 && duo::elect()) duo::commit_both(&acc_full[buf]);
             __syncwarp();
         }
     } else if (warp == 2) {
@@ -247,6 +263,7 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
         for (uint32_t pos = pos0; ok && pos < pos1;) {
             const Item it = load_item(pos);
             pos = it.next;
+            const uint32_t ex = ROUTED ? __ldcg(a.tiles + 1 + 2 * it.tt) : 0u;
             for (uint32_t r = 0; r < it.nraw; r++) {
                 if (!mbar_wait(&raw_empty[slot], ph, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, kSpin)) {
                     ok = false;
@@ -257,9 +274,9 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
                     mbar_expect_tx(&raw_full[slot], raw_bytes);
                     for (uint32_t i = 0; i < 1u << c.row_group; i++)
                         asm volatile(
-                            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                            "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
                                 smem_base + c.raw_off + slot * raw_bytes + i * (raw_bytes >> c.row_group)),
-                            "l"(&wmaps.m[it.op]), "r"(((i * row_bytes + kb) & ~15u) >> 2), "r"(it.n0 >> c.row_group), "r"(smem_u32(&raw_full[slot]))
+                            "l"(&wmaps.m[it.op]), "r"(((i * row_bytes + kb) & ~15u) >> 2), "r"(it.n0 >> c.row_group), "r"(ex), "r"(smem_u32(&raw_full[slot]))
                             : "memory");
                 }
                 __syncwarp();
@@ -269,20 +286,19 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
                 }
             }
         }
-    } else if (warp >= 4) {
+    } else if (warp >= 4 && warp < 4 + kDuoDequantWarps) {
         // thread (warp w, lane l) of a set owns weight row 32 (w % 4) + l, the tensor-memory lane it may address, and the 64-element half
         // (w / 4) % 2 of the K stage: 32 packed f16 pairs = one 32-column store
-        const uint32_t dw = warp - 4, q4 = dw & 3u, half = (dw >> 2) & 1u, set = dw >> 3, g = dw >> 2;
+        const uint32_t dw = warp - 4, q4 = dw & 3u, half = (dw >> 2) & 1u, set = dw >> 3;
         const uint32_t rr = q4 * 32 + lane;
         const uint32_t srow = ((rr & ((1u << c.row_group) - 1u)) << (7 - c.row_group)) + (rr >> c.row_group);   // the row's place in a raw stage
         const uint32_t a_dst = tmem + ((q4 * 32) << 16) + kDuoACol + 32 * half;
         const uint32_t row_bytes = (a.k / QK) * BB;
-        uint32_t rs = 0, rph = 0, J0 = 0, nitem = 0;
-        for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
+        uint32_t rs = 0, rph = 0, J0 = 0;
+        for (uint32_t pos = pos0; ok && pos < pos1;) {
             const Item it = load_item(pos);
             pos = it.next;
-            const uint32_t n = c.out.n[it.op];
-            const bool row_ok = it.n0 + rr < n;
+            const bool row_ok = it.n0 + rr < c.out.n[it.op];
             const uint32_t row_lo4 = (it.n0 + rr) * row_bytes & 15u;   // (the weights start on a 16-byte boundary)
             for (uint32_t r = 0; r < it.nraw; r++) {
                 if (!mbar_wait(&raw_full[rs], rph, &abort_flag, a.status, ST_WAIT_FULL_TIMEOUT, 0u)) {
@@ -294,11 +310,11 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
                     const uint32_t J = J0 + st, sa = J % kDuoStages;   // (J: the stage's number in the pair's whole run)
                     const uint32_t r_abs = it.r_lo + r, stage_row = smem_base + c.raw_off + rs * raw_bytes + srow * c.seg_stride;
                     uint32_t regs[32];
-                    if (c.aligned && row_ok) {
+                    if (T != GT_Q4_K && c.aligned && row_ok) {   // (Q4_K: the generic extraction below)
                         if constexpr (T == GT_Q6_K) {
                             dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half, regs);
                             dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half + 1, regs + 16);
-                        } else {
+                        } else if constexpr (T != GT_Q4_K) {
                             switch (2 * set + half) {  // uniform per warp
                             case 0: dequant64_aligned<T, 0>(stage_row, regs); break;
                             case 1: dequant64_aligned<T, 1>(stage_row, regs); break;
@@ -351,38 +367,65 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
             }
             if (!ok) break;
             J0 += it.nst;
-            // ---- read-back: lane = weight row, 32 activation rows at a time ----
-            if (!mbar_wait(&acc_full, nitem & 1u, &abort_flag, a.status, ST_WAIT_MMA_TIMEOUT, 0u)) break;
+        }
+    } else if (warp >= 4) {
+        // lane = weight row, 32 activation rows at a time, the two groups of four warps in turn
+        const uint32_t q4 = warp & 3u, g = (warp - 4 - kDuoDequantWarps) >> 2, rr = q4 * 32 + lane;
+        uint32_t nitem = 0;
+        for (uint32_t pos = pos0; pos < pos1; nitem++) {
+            const Item it = load_item(pos);
+            pos = it.next;
+            const uint32_t buf = accs == 2 ? nitem & 1u : 0u, turn = accs == 2 ? nitem >> 1 : nitem, n = c.out.n[it.op];
+            const bool row_ok = it.n0 + rr < n;
+            int32_t mine = -1;   // ROUTED: the output row of activation row 32 g + lane of the tile
+            if constexpr (ROUTED) {
+                const uint32_t ex = __ldcg(a.tiles + 1 + 2 * it.tt), at = __ldcg(a.tiles + 2 + 2 * it.tt) * c.nt + g * 32 + lane;
+                if (at < __ldcg(a.htpe + ex) && at < a.hids_stride) {
+                    mine = __ldcg(a.hids + (size_t)ex * a.hids_stride + at);
+                    if ((uint32_t)mine >= a.total_rows) mine = -1;
+                }
+            }
+            if (!mbar_wait(&acc_full[buf], turn & 1u, &abort_flag, a.status, ST_WAIT_MMA_TIMEOUT, 0u)) break;
             tc_fence_after();
             const bool some = it.nraw < nraw_all;   // another pair has the rest of this tile's K
 #pragma unroll 1
-            for (uint32_t col = g * 32; col < c.nt; col += kDuoDequantWarps / 4 * 32) {
+            for (uint32_t col = g * 32; col < c.nt; col += kDuoReadWarps / 4 * 32) {
                 uint32_t v[32];
-                tmem_ld_32x32(tmem + ((q4 * 32) << 16) + col, v);
+                tmem_ld_32x32(tmem + ((q4 * 32) << 16) + buf * 128 + col, v);
                 tmem_ld_wait();
-                const uint32_t o0 = it.tt * c.nt + col;
-                if (row_ok && o0 < a.m) {
-                    float *y = c.out.y[it.op] + (size_t)o0 * n + it.n0 + rr;
-                    const uint32_t cnt = min(32u, a.m - o0);
-                    if (some) {
+                if constexpr (ROUTED) {   // (tiles of 64 rows: this is the loop's only turn)
+                    float *y = c.out.y[0] + it.n0 + rr;
 #pragma unroll
-                        for (uint32_t j = 0; j < 32; j++)
-                            if (j < cnt) atomicAdd(y + (size_t)j * n, __uint_as_float(v[j]));
-                    } else {
+                    for (uint32_t j = 0; j < 32; j++) {
+                        const int32_t o = __shfl_sync(0xffffffffu, mine, j);
+                        if (row_ok && o >= 0) y[(size_t)o * n] = __uint_as_float(v[j]);
+                    }
+                } else {
+                    const uint32_t o0 = it.tt * c.nt + col;
+                    if (row_ok && o0 < a.m) {
+                        float *y = c.out.y[it.op] + (size_t)o0 * n + it.n0 + rr;
+                        const uint32_t cnt = min(32u, a.m - o0);
+                        if (some) {
 #pragma unroll
-                        for (uint32_t j = 0; j < 32; j++)
-                            if (j < cnt) y[(size_t)j * n] = __uint_as_float(v[j]);
+                            for (uint32_t j = 0; j < 32; j++)
+                                if (j < cnt) atomicAdd(y + (size_t)j * n, __uint_as_float(v[j]));
+                        } else {
+#pragma unroll
+                            for (uint32_t j = 0; j < 32; j++)
+                                if (j < cnt) y[(size_t)j * n] = __uint_as_float(v[j]);
+                        }
                     }
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) duo::arrive_at_0(&acc_empty);   // the MMA warp may start the next item's accumulation
+            if (lane == 0) duo::arrive_at_0(&acc_empty[buf]);   // the MMA warp may start on another item here
         }
     }
     __syncwarp();
     if (abort_flag)   // let copies in flight land before the shared memory is released
         for (int i = 0; i < 200; i++) __nanosleep(5000);
+    if (c.beside) grid_dependency_wait();   // (what comes behind waits for this kernel only)
     tc_fence_before();
     __syncthreads();
     duo::cluster_sync();   // nobody leaves while the other may still arrive here, or while the pair's MMAs read here
@@ -409,8 +452,8 @@ static uint32_t duo_pairs() {
         cfg.gridDim = dim3(most * 2);
         cfg.blockDim = dim3(kDuoThreads);
         cfg.dynamicSmemBytes = 223 * 1024;
-        if (cudaFuncSetAttribute(qmm_duo_kernel<GT_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, qmm_duo_kernel<GT_Q4_0>, &cfg) != cudaSuccess || n < 1 || n > (int)most) {
+        if (cudaFuncSetAttribute(qmm_duo_kernel<GT_Q4_0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, qmm_duo_kernel<GT_Q4_0, false>, &cfg) != cudaSuccess || n < 1 || n > (int)most) {
             (void)cudaGetLastError();
             n = (int)most;
         }
@@ -462,12 +505,53 @@ uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt) {
     return duo_plan(ggml_type, a.m, a.n, a.k, nt, p);
 }
 
+// Maps, rings and launch.  `c`: tiles, products and pairs are filled in.
+template <int T, bool ROUTED> static cudaError_t duo_launch(DuoCfg &c, const QmmArgs *ops, int nops, const uint8_t *xpack, cudaStream_t st, int *launches) {
+    constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
+    const QmmArgs &a = ops[0];
+    const uint32_t row_bytes = (a.k / QK) * BB;
+    c.nchunks = (a.k + 63) / 64;
+    c.row_group = (uint32_t)duo_row_group(row_bytes);
+    c.aligned = row_bytes % 16 == 0 && a.k % 256 == 0;
+    constexpr uint32_t kSeg = 256 / QK * BB;
+    c.seg_stride = c.row_group == 0 && kSeg % 16 == 0 ? kSeg : ((kSeg + 14 + 15) / 16 | 1u) * 16;   // (an odd multiple of 16: see launch_tc_tn)
+    alignas(64) DuoMaps wmaps;
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return cudaErrorNotSupported;
+    for (int i = 0; i < nops; i++) {
+        const uint32_t lg = c.row_group;
+        const cuuint64_t gdim[3] = {((uint64_t)row_bytes << lg) / 4, ops[i].n >> lg, ROUTED ? a.n_experts : 1u};
+        const cuuint64_t gstride[2] = {(uint64_t)row_bytes << lg, ROUTED ? a.expert_stride : (uint64_t)ops[i].n * row_bytes};
+        const cuuint32_t box[3] = {c.seg_stride / 4, 128u >> lg, 1}, estr[3] = {1, 1, 1};
+        if (enc(&wmaps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint8_t *>(ops[i].w), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    const uint32_t limit = 222 * 1024, b_bytes = kDuoStages * c.nt * 128u, raw_slot = 128 * c.seg_stride;
+    c.raw_off = b_bytes;
+    c.raw_slots = (limit - b_bytes) / raw_slot;
+    if (c.raw_slots > kDuoMaxRaw) c.raw_slots = kDuoMaxRaw;
+    if (c.raw_slots < 2) return cudaErrorInvalidConfiguration;
+    size_t smem = (size_t)b_bytes + c.raw_slots * raw_slot + 1024;
+    if (smem < 120 * 1024) smem = 120 * 1024;   // (one CTA per SM: it takes all of tensor memory)
+    static std::atomic<uint32_t> prepared[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!prepared[dev].load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(qmm_duo_kernel<T, ROUTED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024);
+        if (e != cudaSuccess) return e;
+        prepared[dev].store(1, std::memory_order_release);
+    }
+    (*launches)++;
+    return launch_overlapped(qmm_duo_kernel<T, ROUTED>, dim3(2 * c.pairs), dim3(kDuoThreads), smem, st, a, c, xpack, wmaps);
+}
+
 // `ops`: products of the same activations
 template <int T> static cudaError_t launch_duo_t(const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {
-    constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
     if (nops < 1 || nops > (int)kMmOps) return cudaErrorInvalidValue;
     const QmmArgs &a = ops[0];
-    const uint32_t row_bytes = (a.k / QK) * BB, h = nt / 2;
+    const uint32_t h = nt / 2, nraw = (a.k + 255) / 256, nchunks = (a.k + 63) / 64;
     DuoCfg c{};
     for (int i = 0; i < nops; i++) {
         c.n_wt += (ops[i].n + kDuoRows - 1) / kDuoRows;
@@ -478,55 +562,49 @@ template <int T> static cudaError_t launch_duo_t(const QmmArgs *ops, int nops, u
     DuoPlan p;
     duo_plan(T, a.m, (uint64_t)c.n_wt * kDuoRows, a.k, nt, p);
     c.nt = nt;
-    c.nchunks = (a.k + 63) / 64;
     c.ntiles = (a.m + nt - 1) / nt;
     c.pairs = p.pairs;
-    c.row_group = (uint32_t)duo_row_group(row_bytes);
-    c.aligned = row_bytes % 16 == 0 && a.k % 256 == 0;
-    constexpr uint32_t kSeg = 256 / QK * BB;
-    c.seg_stride = c.row_group == 0 && kSeg % 16 == 0 ? kSeg : ((kSeg + 14 + 15) / 16 | 1u) * 16;   // (an odd multiple of 16: see launch_tc_tn)
-    const uint32_t nraw = (a.k + 255) / 256;
     if (p.shared) c.share = {p.pairs, c.n_wt, nraw, c.n_wt * c.ntiles * nraw, kDuoRows, nt};
-    alignas(64) DuoMaps wmaps;
-    EncodeTiledFn enc = encode_tiled_fn();
-    if (!enc) return cudaErrorNotSupported;
-    for (int i = 0; i < nops; i++) {
-        const uint32_t lg = c.row_group;
-        const cuuint64_t gdim[2] = {((uint64_t)row_bytes << lg) / 4, ops[i].n >> lg};
-        const cuuint64_t gstride[1] = {(uint64_t)row_bytes << lg};
-        const cuuint32_t box[2] = {c.seg_stride / 4, 128u >> lg}, estr[2] = {1, 1};
-        if (enc(&wmaps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t *>(ops[i].w), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return cudaErrorInvalidValue;
-    }
-    const uint32_t limit = 222 * 1024, b_bytes = kDuoStages * nt * 128u, raw_slot = 128 * c.seg_stride;
-    c.raw_off = b_bytes;
-    c.raw_slots = (limit - b_bytes) / raw_slot;
-    if (c.raw_slots > kDuoMaxRaw) c.raw_slots = kDuoMaxRaw;
-    if (c.raw_slots < 2) return cudaErrorInvalidConfiguration;
-    size_t smem = (size_t)b_bytes + c.raw_slots * raw_slot + 1024;
-    if (smem < 120 * 1024) smem = 120 * 1024;   // (one CTA per SM: it takes all of tensor memory)
     // activations in tiles of nt / 2 rows: a CTA's half of a tile
-    {
-        const uint32_t tiles = 2 * c.ntiles;
-        uint32_t lanes = c.nchunks;
-        const uint64_t slices = (uint64_t)tiles * ((h + kPackRows - 1) / kPackRows);
-        while (lanes > 1 && (uint64_t)lanes * slices > 2048) lanes = (lanes + 1) / 2;
-        (*launches)++;
-        const cudaError_t e = launch_overlapped(pack_x_kernel, dim3((unsigned)slices, lanes), dim3(256), 0, st, a, xpack, c.nchunks, h, c.share, c.out);
-        if (e != cudaSuccess) return e;
-    }
-    static std::atomic<uint32_t> prepared[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!prepared[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(qmm_duo_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024);
-        if (e != cudaSuccess) return e;
-        prepared[dev].store(1, std::memory_order_release);
-    }
+    uint32_t lanes = nchunks;
+    const uint64_t slices = (uint64_t)2 * c.ntiles * ((h + kPackRows - 1) / kPackRows);
+    while (lanes > 1 && (uint64_t)lanes * slices > 2048) lanes = (lanes + 1) / 2;
     (*launches)++;
-    return launch_overlapped(qmm_duo_kernel<T>, dim3(2 * c.pairs), dim3(kDuoThreads), smem, st, a, c, (const uint8_t *)xpack, wmaps);
+    const cudaError_t e = launch_overlapped(pack_x_kernel, dim3((unsigned)slices, lanes), dim3(256), 0, st, a, xpack, nchunks, h, c.share, c.out);
+    if (e != cudaSuccess) return e;
+    return duo_launch<T, false>(c, ops, nops, xpack, st, launches);
+}
+
+template <int T> static cudaError_t launch_duo_routed_t(const QmmArgs &a, uint32_t tiles, const uint8_t *xpack, cudaStream_t st, int *launches) {
+    DuoCfg c{};
+    c.n_wt = (a.n + kDuoRows - 1) / kDuoRows;
+    c.out.y[0] = a.y;
+    c.out.n[0] = a.n;
+    c.out.wt_end[0] = c.n_wt;
+    c.nt = kRoutedTile;
+    c.ntiles = tiles;
+    const uint64_t items = (uint64_t)c.n_wt * tiles;
+    c.pairs = items < duo_pairs() ? (uint32_t)items : duo_pairs();
+    c.beside = (a.reuse & 4u) != 0;
+    if (!c.pairs) return cudaSuccess;
+    return duo_launch<T, true>(c, &a, 1, xpack, st, launches);
+}
+
+// `tiles`: bound of the list's length; `xpack`: what the list's tiles hold
+bool qmm_duo_routed_fits(int ggml_type, const QmmArgs &a) {
+    if (!a.hids || a.y_ld || a.n_peer || a.k % 32 != 0 || a.n_experts < 1) return false;
+    const uint64_t row_bytes = (uint64_t)(a.k / ggml_qk(ggml_type)) * ggml_block_bytes(ggml_type);
+    return (((uintptr_t)a.w | a.expert_stride) & 15u) == 0 && a.n % (1u << duo_row_group((uint32_t)row_bytes)) == 0 && row_bytes * a.n <= a.expert_stride &&
+           encode_tiled_fn() != nullptr;
+}
+cudaError_t launch_qmm_duo_routed(int ggml_type, const QmmArgs &a, uint32_t tiles, const uint8_t *xpack, cudaStream_t st, int *launches) {
+    switch (ggml_type) {
+    case GT_Q4_0: return launch_duo_routed_t<GT_Q4_0>(a, tiles, xpack, st, launches);
+    case GT_Q8_0: return launch_duo_routed_t<GT_Q8_0>(a, tiles, xpack, st, launches);
+    case GT_Q6_K: return launch_duo_routed_t<GT_Q6_K>(a, tiles, xpack, st, launches);
+    case GT_Q4_K: return launch_duo_routed_t<GT_Q4_K>(a, tiles, xpack, st, launches);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {

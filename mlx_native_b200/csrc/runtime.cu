@@ -2319,7 +2319,11 @@ extern "C" int mlxn_moe_ffn_layer(mlxn_encoder *enc, mlxn_registry *reg, mlxn_de
         return MLXN_OK;
     };
     if ((rc = product(pg, x, nullptr, gate_w, gate_out, 0u))) return rc;          // builds the tile list, packs x
-    if ((rc = product(pu, x, nullptr, up_w, up_out, 3u))) return rc;              // takes both over
+    // ... takes both over, and (bit 2) runs beside the first where that one's result is neither the weights nor the result of this one
+    const uint8_t *g0 = reinterpret_cast<const uint8_t *>(gate_out->dev()), *g1 = g0 + pairs * p->ffn * 4;
+    auto apart = [&](const void *at, size_t bytes) { return g1 <= (const uint8_t *)at || (const uint8_t *)at + bytes <= g0; };
+    const bool beside = apart(up_out->dev(), pairs * p->ffn * 4) && apart(up_w->dev(), (size_t)p->n_experts * pu.expert_stride);
+    if ((rc = product(pu, x, nullptr, up_w, up_out, beside ? 7u : 3u))) return rc;
     if ((rc = product(pd, gate_out, up_out, down_w, down_out, 1u))) return rc;    // same tiles; packs silu(gate) * up
     g_last_kernel = "qmm_tc_id";
     g_dispatch.fetch_add(1);

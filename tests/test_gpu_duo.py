@@ -141,3 +141,59 @@ def test_products_of_one_group_over_shared_ranges(ctx):
         got = y.as_slice(np.float32).reshape(m, n)
         for at in range(0, n, 1024):
             assert norm_err(got[:, at:at + 1024], y_ref, ad) <= TOL
+
+
+ROUTED = [
+    # (type, n, k): 264 and 520 weight rows leave a pair of SMs half or almost empty; K tails of 32; Q4_0 with 261 rows has no groups of
+    # rows that start on 16 bytes, so the other kernel takes it
+    ("Q4_0", 264, 288), ("Q4_0", 261, 288), ("Q4_0", 520, 2048), ("Q8_0", 264, 544), ("Q8_0", 96, 32),
+    ("Q6_K", 520, 768), ("Q6_K", 256, 256), ("Q4_K", 264, 768), ("Q4_K", 1032, 256),
+]
+
+
+@pytest.mark.parametrize("tname,n,k", ROUTED)
+def test_routed_tiles(ctx, tname, n, k):
+    """Experts with no rows, one, either side of a CTA's half of a tile, of a whole tile and of two, and a row whose id names no expert."""
+    gtype, otype = (mx.GgmlType.Q4_K, orc.Q4_K) if tname == "Q4_K" else TYPES[tname]
+    counts = [0, 1, 32, 33, 63, 64, 65, 0, 130]
+    E, m = len(counts), sum(counts) + 1
+    ids = np.random.default_rng(n + k).permutation(np.concatenate([np.repeat(np.arange(E), counts), [E + 7]])).astype(np.uint32)
+    ws = [normal_weights(50 + e, n, k, otype) for e in range(E)]
+    stride = (ws[0].size + 15) // 16 * 16 + 48
+    stack = np.zeros(E * stride, np.uint8)
+    for e, w in enumerate(ws):
+        stack[e * stride:e * stride + w.size] = w.reshape(-1)
+    x = normal_acts(3, m, k)
+    d = ctx.device
+    xb, wb, ib = ctx.buf(x, mx.DType.F32), ctx.buf(stack, mx.DType.U8), ctx.buf(ids, mx.DType.U32)
+    yb = ctx.buf(np.full(m * n, 7, np.float32), mx.DType.F32)
+    enc = d.command_encoder()
+    mx.quantized_matmul_id_ggml(enc, ctx.registry, d, xb, wb, ib, yb, mx.GgmlQuantizedMatmulIdParams(m, 1, n, k, E, stride, gtype))
+    enc.commit_and_wait()
+    y = yb.as_slice(np.float32).reshape(m, n)
+    for e in range(E):
+        rows = np.nonzero(ids == e)[0]
+        if rows.size:
+            y_ref, ad = orc.qmatmul(otype, ws[e], x[rows], n, k, nthreads=4, f16_operands=True)
+            assert norm_err(y[rows], y_ref, ad) <= TOL
+    assert not y[ids == E + 7].any()
+
+
+def test_routed_layer_with_one_result_buffer(ctx):
+    """gate and up written to the same buffer: up's product is what stays, so it may not run beside the other one."""
+    d, T, E, top_k, hidden, ffn = ctx.device, 256, 8, 2, 512, 512
+    gtype, otype = TYPES["Q4_0"]
+    gate, up, down = (np.concatenate([normal_weights(at + e, 512, 512, otype) for e in range(E)]) for at in (0, 20, 40))
+    ids = np.random.default_rng(1).permuted(np.tile(np.arange(E), (T, 1)), axis=1)[:, :top_k].astype(np.uint32).reshape(-1)
+    xb, ib = ctx.buf(normal_acts(5, T, hidden), mx.DType.F32), ctx.buf(ids, mx.DType.U32)
+    p = mx.MoeFfnLayerParams(T, top_k, hidden, ffn, E, gtype, gtype, gtype, *([gate.size // E] * 3))
+    got = []
+    for one in (True, False):
+        wg, wu, wd = (ctx.buf(w, mx.DType.U8) for w in (gate if one else up, up, down))
+        yu, yd = (d.alloc_buffer(T * top_k * ffn * 4, mx.DType.F32) for _ in range(2))
+        yg = yu if one else d.alloc_buffer(T * top_k * ffn * 4, mx.DType.F32)
+        enc = d.command_encoder()
+        mx.moe_ffn_layer(enc, ctx.registry, d, xb, ib, wg, wu, wd, yg, yu, yd, p)
+        enc.commit_and_wait()
+        got.append((yu.as_slice(np.float32).copy(), yd.as_slice(np.float32).copy()))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
