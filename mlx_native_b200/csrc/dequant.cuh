@@ -213,41 +213,46 @@ template <int T, int S4> __device__ __forceinline__ void dequant64_aligned(uint3
         q8_0_block_to_h(W[wo + 8] >> 16, q1, r + 16);
     }
 }
-// Q6_K: the 32-element run (h, g) of the super-block that starts PRE bytes into the row's aligned stage.
-template <int PRE> __device__ __forceinline__ void dequant32_q6k_aligned(uint32_t stage_row, uint32_t h, uint32_t g, uint32_t *out) {
-    uint32_t A[8], H[8];
-    lds_field<PRE, 8>(stage_row + 64 * h + 32 * (g & 1u), A);
+// Q6_K: 64 elements (half h's runs 2 q and 2 q + 1) of the super-block that starts PRE bytes into the row's aligned stage.  The two runs
+// have the same 32 bytes of high bits, and their 64 bytes of low bits follow one another.  A code is put beside 1024 in f16, widened, and scaled
+// two at a time: fma(1024 + u, ds, -1056 ds) = ds (u - 32), exact in f32 (ds has at most 18 significant bits), then rounded once to f16.
+template <int PRE> __device__ __forceinline__ void dequant64_q6k_aligned(uint32_t stage_row, uint32_t h, uint32_t q, uint32_t (&out)[32]) {
+    uint32_t H[8];
     lds_field<PRE, 8>(stage_row + 128 + 32 * h, H);
     const float d = half_bits_to_float(lds_u16(stage_row + PRE + 208));
-    const float ds0 = d * (float)lds_s8(stage_row + PRE + 192 + 8 * h + 2 * g);
-    const float ds1 = d * (float)lds_s8(stage_row + PRE + 192 + 8 * h + 2 * g + 1);
-    const uint32_t hsh = 2 * g, ash = (g & 2u) ? 4u : 0u;
+    const uint32_t sc[2] = {lds_u16(stage_row + PRE + 192 + 8 * h + 4 * q), lds_u16(stage_row + PRE + 194 + 8 * h + 4 * q)};
+    const uint32_t ash = 4 * q;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const float ds = j < 2 ? ds0 : ds1;
-        const float c = -160.0f * ds;  // exact: ds has <= 18 significant bits
+    for (int g = 0; g < 2; g++) {
+        uint32_t A[8];
+        lds_field<PRE, 8>(stage_row + 64 * h + 32 * g, A);
+        const uint32_t rot = (4u - 4 * q - 2 * g) & 31u;   // brings a byte's two bits to bits 4 and 5
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const uint32_t u = ((A[2 * j + i] >> ash) & 0x0F0F0F0Fu) | (((H[2 * j + i] >> hsh) & 0x03030303u) << 4);
-            const float f0 = fmaf(__uint_as_float(__byte_perm(u, 0x43000000u, 0x7044)), ds, c);
-            const float f1 = fmaf(__uint_as_float(__byte_perm(u, 0x43000000u, 0x7144)), ds, c);
-            const float f2 = fmaf(__uint_as_float(__byte_perm(u, 0x43000000u, 0x7244)), ds, c);
-            const float f3 = fmaf(__uint_as_float(__byte_perm(u, 0x43000000u, 0x7344)), ds, c);
-            out[4 * j + 2 * i] = h2_as_u32(__floats2half2_rn(f0, f1));
-            out[4 * j + 2 * i + 1] = h2_as_u32(__floats2half2_rn(f2, f3));
+        for (int j = 0; j < 8; j++) {
+            const float ds = d * (float)(int)(int8_t)(j < 4 ? sc[g] & 0xFFu : sc[g] >> 8);
+            const float c = -1056.0f * ds;
+            const uint32_t u = ((A[j] >> ash) & 0x0F0F0F0Fu) | (__funnelshift_l(H[j], H[j], rot) & 0x30303030u);
+            __half2 lo, hi;
+            bytes_to_h2(u, lo, hi);
+            const uint64_t ds2 = pack2(ds, ds), c2 = pack2(c, c);
+            float f0, f1, f2, f3;
+            unpack2(ffma2(pack2(__low2float(lo), __high2float(lo)), ds2, c2), f0, f1);
+            unpack2(ffma2(pack2(__low2float(hi), __high2float(hi)), ds2, c2), f2, f3);
+            out[16 * g + 2 * j] = h2_as_u32(__floats2half2_rn(f0, f1));
+            out[16 * g + 2 * j + 1] = h2_as_u32(__floats2half2_rn(f2, f3));
         }
     }
 }
-__device__ __forceinline__ void dequant32_q6k_aligned_p(uint32_t p8, uint32_t stage_row, uint32_t h, uint32_t g, uint32_t *out) {
+__device__ __forceinline__ void dequant64_q6k_aligned_p(uint32_t p8, uint32_t stage_row, uint32_t h, uint32_t q, uint32_t (&out)[32]) {
     switch (p8) {  // uniform over the CTA
-    case 0: dequant32_q6k_aligned<0>(stage_row, h, g, out); break;
-    case 1: dequant32_q6k_aligned<2>(stage_row, h, g, out); break;
-    case 2: dequant32_q6k_aligned<4>(stage_row, h, g, out); break;
-    case 3: dequant32_q6k_aligned<6>(stage_row, h, g, out); break;
-    case 4: dequant32_q6k_aligned<8>(stage_row, h, g, out); break;
-    case 5: dequant32_q6k_aligned<10>(stage_row, h, g, out); break;
-    case 6: dequant32_q6k_aligned<12>(stage_row, h, g, out); break;
-    default: dequant32_q6k_aligned<14>(stage_row, h, g, out); break;
+    case 0: dequant64_q6k_aligned<0>(stage_row, h, q, out); break;
+    case 1: dequant64_q6k_aligned<2>(stage_row, h, q, out); break;
+    case 2: dequant64_q6k_aligned<4>(stage_row, h, q, out); break;
+    case 3: dequant64_q6k_aligned<6>(stage_row, h, q, out); break;
+    case 4: dequant64_q6k_aligned<8>(stage_row, h, q, out); break;
+    case 5: dequant64_q6k_aligned<10>(stage_row, h, q, out); break;
+    case 6: dequant64_q6k_aligned<12>(stage_row, h, q, out); break;
+    default: dequant64_q6k_aligned<14>(stage_row, h, q, out); break;
     }
 }
 

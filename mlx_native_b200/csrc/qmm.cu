@@ -13,7 +13,7 @@
 //             staging ring, eight warps dequantise them into the swizzled f16 A tile, one thread
 //             issues tcgen05.mma (M=128, N=NT, K=16) accumulating in tensor memory, and the same
 //             eight warps read the accumulator back with tcgen05.ld and store y.
-//             Dense calls go to pairs of SMs where their weights allow it (qmm_duo.cu); grouped and row-sharded ones run here.
+//             Calls whose weights allow it go to pairs of SMs (qmm_duo.cu); the row-sharded form and the rest run here.
 //   qmm_simt  plain CUDA-core tile kernel with the same operand rounding; used for shapes the
 //             tcgen05 kernel does not take and as an on-device cross-check.
 #include <cuda_fp16.h>
@@ -213,7 +213,8 @@ __device__ __forceinline__ void load8(const float *p, uint32_t left, float (&v)[
         for (uint32_t u = 0; u < 8; u++) v[u] = u < left ? __ldcg(p + u) : 0.0f;
     }
 }
-__global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t nt, const TcShare sh, const __grid_constant__ TcOut res) {
+template <bool SWIGLU>
+__global__ void __launch_bounds__(256, SWIGLU ? 4 : 5) pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t nt, const TcShare sh, const __grid_constant__ TcOut res) {
     // CTA (t, c) packs the chunks c, c + gridDim.y, ... of its slice, so that the slice's routing lookups (a chain of
     // dependent loads) are paid once per CTA, not once per chunk.
     const uint32_t slices = (nt + kPackRows - 1) / kPackRows, t = blockIdx.x / slices, r0 = (blockIdx.x - t * slices) * kPackRows;
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
         uint8_t *tile = xpack + ((size_t)t * nchunks + kc) * (size_t)(nt * 128);
         const uint32_t k0 = kc * 64 + 8 * (threadIdx.x & 7u);   // (the same columns in both rows)
         float v[kPer][8];
-        [[maybe_unused]] float z[kPer][8];
+        [[maybe_unused]] float z[SWIGLU ? kPer : 1][8];
         // all loads first
 #pragma unroll
         for (int i = 0; i < kPer; i++) {
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
                 }
             } else {
                 load8(src_row[i] + k0, a.k - k0, v[i]);
-                if (a.x2) load8(a.x2 + (src_row[i] + k0 - a.x), a.k - k0, z[i]);
+                if constexpr (SWIGLU) load8(a.x2 + (src_row[i] + k0 - a.x), a.k - k0, z[i]);
             }
         }
 #pragma unroll
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
             if (r >= nt) break;
             uint4 out = make_uint4(0, 0, 0, 0);
             if (src_row[i] && k0 < a.k) {
-                if (a.x2) {   // fused SwiGLU: the same expression as the stand-alone kernel, so the same f32 values
+                if constexpr (SWIGLU) {   // fused SwiGLU: the same expression as the stand-alone kernel, so the same f32 values
 #pragma unroll
                     for (int u = 0; u < 8; u++) v[i][u] = v[i][u] / (1.0f + expf(-v[i][u])) * z[i][u];
                 }
@@ -296,6 +297,8 @@ __global__ void __launch_bounds__(256) pack_x_kernel(const QmmArgs a, uint8_t *x
         }
     }
 }
+
+template __global__ void pack_x_kernel<false>(const QmmArgs, uint8_t *, uint32_t, uint32_t, const TcShare, const __grid_constant__ TcOut);
 
 // =================================================================================================
 // qmm_tc
@@ -764,8 +767,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
                 if (T != GT_Q4_K && c.aligned && row_ok && !(MLXN_DBG(c) & 1u)) {   // (Q4_K: the generic extraction below)
                     const uint32_t stage_row = smem_base + c.raw_off + rs * raw_stage_bytes + srow * c.seg_stride;
                     if constexpr (T == GT_Q6_K) {
-                        dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half, regs);
-                        dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half + 1, regs + 16);
+                        dequant64_q6k_aligned_p(r_abs & 7u, stage_row, set, half, regs);
                     } else if constexpr (T != GT_Q4_K) {
                         switch (2 * set + half) {  // uniform per warp
                         case 0: dequant64_aligned<T, 0>(stage_row, regs); break;
@@ -1166,7 +1168,7 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint32_t nt, uint8_t *sc
         res.y[0] = a.y;
         res.n[0] = a.n;
         res.wt_end[0] = c.n_wt;
-        cudaError_t e = launch_overlapped(pack_x_kernel, grid, dim3(256), 0, st, a, xpack, c.nchunks, nt, c.share, res);
+        cudaError_t e = launch_overlapped(a.x2 ? pack_x_kernel<true> : pack_x_kernel<false>, grid, dim3(256), 0, st, a, xpack, c.nchunks, nt, c.share, res);
         if (e != cudaSuccess) return e;
     }
     if (routed && !SH && qmm_duo_routed_fits(T, a)) return launch_qmm_duo_routed(T, a, (uint32_t)tiles, xpack, st, launches);

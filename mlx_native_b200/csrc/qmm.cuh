@@ -30,6 +30,7 @@ struct TcOut {
 };
 
 constexpr uint32_t kPackRows = 64;   // rows of a tile that a block of pack_x_kernel packs
+template <bool SWIGLU>
 __global__ void pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t nt, const TcShare sh, const __grid_constant__ TcOut res);
 
 int sm_count_of_device();

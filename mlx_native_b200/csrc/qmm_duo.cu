@@ -1,4 +1,4 @@
-// Dense mat-mat of many activation rows on pairs of SMs: y[m, n] = x[m, k] . W[n, k]^T, weights dequantised on the way.
+// Mat-mat of many activation rows on pairs of SMs, dense or grouped by expert: y[m, n] = x[m, k] . W[n, k]^T, weights dequantised on the way.
 //
 // The kernel of qmm.cu gives every SM a tile of 128 weight rows and up to 256 activation rows.  At 256 its tensor core is held up by
 // shared memory: it reads the activation tile (8 KB) for every 16 K values, the bulk copies write as much, and the raw weights come on
@@ -11,6 +11,13 @@
 // 256 x 512 x 16 rows 8.6 / 8.2.  So it takes every call it can: what has no 16-byte aligned weights, or a row count that its copies cannot group,
 // stays with the other kernel, and the row-sharded form.  What bounds it: up to 192 rows the chain raw block -> tensor memory (0.47 us for a
 // K stage of 128, 18 values a cycle and SM; Q6_K 0.66), above that the multiplication (0.43 us at full clock) beside it.
+//
+// The items of grouped calls are short (64 rows, K of 6 to 16 stages), and while the dequantising warps read an accumulator back both they and the
+// tensor core would stand still; there the read-back has warps of its own and two accumulators.  (Dense calls gain nothing from it, Q4_0 2048 x 4096 x
+// 4096 61.4 / 62.4 us, and Q6_K loses, 128 x 4096 x 4096 19.8 / 22.2.)  Layer of 512 tokens, 8 of 128 experts each, Q4_0 768 x 2048 twice and Q6_K
+// 2048 x 768: 273 us for the whole pass with two CTAs of qmm.cu's kernel on an SM (half of the dequantising warps each), 226 here; weights once at the
+// copy rate 61.  Batches: q, k and v of 512 rows (4096, 1024 and 1024 x 4096) and gate and up (12288 x 4096 each) in one launch take a layer from 274
+// to 244 us: one packing instead of three and two, and one last wave.
 //
 // What else was tried: unpacking the weights once into f16 tiles, by a kernel of its own.  The product alone then runs at the
 // multiplication's rate, but the unpacking is bound by memory (13 us for 4096 x 4096, 58 with 2048 rows of 12288 for 4096 x 12288): 32.2 us in
@@ -31,8 +38,9 @@ namespace mlxn {
 
 constexpr uint32_t kDuoRows = 256;                          // weight rows of a pair's tile
 constexpr uint32_t kDuoDequantWarps = 16;                   // two sets of eight; set s takes the 128-wide K stages st % 2 == s
-constexpr uint32_t kDuoReadWarps = 8;                       // read the accumulators back
-constexpr uint32_t kDuoThreads = (4 + kDuoDequantWarps + kDuoReadWarps) * 32;
+// Warps that read the accumulators back: of their own where tiles are short (routed), else the dequantising ones.
+__host__ __device__ constexpr uint32_t duo_read_warps(bool routed) { return routed ? 8 : kDuoDequantWarps; }
+__host__ __device__ constexpr uint32_t duo_threads(bool routed) { return (4 + kDuoDequantWarps + (routed ? duo_read_warps(true) : 0)) * 32; }
 constexpr uint32_t kDuoStages = 4;                          // ring of K stages: activations in shared memory, weights in tensor memory
 constexpr uint32_t kDuoACol = 256, kDuoACols = 64;          // tensor-memory columns of the weights: 64 a stage (128 f16 pairs)
 constexpr uint32_t kDuoMaxRaw = 5;
@@ -102,17 +110,17 @@ __device__ __forceinline__ void commit_both(uint64_t *bar) {
 //   warp 0        activations: one bulk copy per K stage (two 64-wide chunks of its half of the tile)
 //   warp 1        CTA 0: MMAs of the pair, whose completion frees the stage's places in both CTAs; CTA 1: tells CTA 0 that its stage is ready
 //   warp 2        raw weights: tensor copies of 128 rows x 256 K values
-//   warps 4..19   dequantise raw blocks into tensor memory
-//   warps 20..27  read the accumulator back; tiles of up to 128 rows have two accumulators, so that the next item's multiplications go on
+//   warps 4..19   dequantise raw blocks into tensor memory; dense: read the accumulator back
+//   warps 20..27  routed: read the accumulators back, two in turn, so that the next item's multiplications go on
 // Ring places and barrier phases run on across the items of a pair.
 //
 // ROUTED: the products of a mixture of experts.  The tiles are those of the list that build_tiles_kernel made, 64 rows of one expert each,
 // packed whole (a CTA's half are rows 0..31 or 32..63 of each 64-column chunk); the weights' map has the expert as third dimension.
 template <int T, bool ROUTED>
-__global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
+__global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1, 1)
     qmm_duo_kernel(const QmmArgs a, const __grid_constant__ DuoCfg c, const uint8_t *xpack, const __grid_constant__ DuoMaps wmaps) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
-    constexpr uint32_t KR = 256;
+    constexpr uint32_t KR = 256, kReadWarps = duo_read_warps(ROUTED), accs = ROUTED ? 2 : 1;   // (accumulators, 128 columns apart)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // (the same in both CTAs)
     __shared__ __align__(8) uint64_t full[kDuoStages], peer_full[kDuoStages], done[kDuoStages], raw_full[kDuoMaxRaw], raw_empty[kDuoMaxRaw];
@@ -134,7 +142,7 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
         }
         for (uint32_t s = 0; s < 2; s++) {
             mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], 2 * kDuoReadWarps);   // (of CTA 0: the warps of both)
+            mbar_init(&acc_empty[s], 2 * kReadWarps);   // (of CTA 0: the warps of both)
         }
         mbar_init_fence();
     }
@@ -153,7 +161,6 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
     // ---- work items: weight tile fastest, so that the pairs working at the same time share an activation tile in L2 ----
     const uint32_t nraw_all = (a.k + KR - 1) / KR, total_items = c.n_wt * (ROUTED ? min(__ldcg(a.tiles), c.ntiles) : c.ntiles);
     const bool shared = !ROUTED && c.share.ctas != 0;
-    const uint32_t accs = c.nt <= 128 ? 2 : 1;   // accumulators, 128 columns apart
     const uint32_t pos0 = shared ? c.share.begin(pair) : pair, pos1 = shared ? c.share.begin(pair + 1) : total_items;
     struct Item {
         uint32_t tt, op, n0, r_lo, nraw, nst, kc_lo, nck, next;
@@ -178,6 +185,56 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
     const uint32_t smem_base = smem_u32(smem), raw_bytes = 128u * c.seg_stride;
     constexpr uint32_t kSpin = 0xFFFFFFFFu;
     bool ok = true;
+
+    // The read-back of the pair's `nitem`-th item, by group g of four warps: lane = weight row, 32 activation rows at a time, the groups in turn.
+    auto read_back = [&](const Item &it, uint32_t nitem, uint32_t q4, uint32_t g) {
+        const uint32_t buf = accs == 2 ? nitem & 1u : 0u, turn = accs == 2 ? nitem >> 1 : nitem, n = c.out.n[it.op], rr = q4 * 32 + lane;
+        const bool row_ok = it.n0 + rr < n;
+        int32_t mine = -1;   // ROUTED: the output row of activation row 32 g + lane of the tile
+        if constexpr (ROUTED) {
+            const uint32_t ex = __ldcg(a.tiles + 1 + 2 * it.tt), at = __ldcg(a.tiles + 2 + 2 * it.tt) * c.nt + g * 32 + lane;
+            if (at < __ldcg(a.htpe + ex) && at < a.hids_stride) {
+                mine = __ldcg(a.hids + (size_t)ex * a.hids_stride + at);
+                if ((uint32_t)mine >= a.total_rows) mine = -1;
+            }
+        }
+        if (!mbar_wait(&acc_full[buf], turn & 1u, &abort_flag, a.status, ST_WAIT_MMA_TIMEOUT, 0u)) return false;
+        tc_fence_after();
+        const bool some = it.nraw < nraw_all;   // another pair has the rest of this tile's K
+#pragma unroll 1
+        for (uint32_t col = g * 32; col < c.nt; col += kReadWarps / 4 * 32) {
+            uint32_t v[32];
+            tmem_ld_32x32(tmem + ((q4 * 32) << 16) + buf * 128 + col, v);
+            tmem_ld_wait();
+            if constexpr (ROUTED) {   // (tiles of 64 rows: this is the loop's only turn)
+                float *y = c.out.y[0] + it.n0 + rr;
+#pragma unroll
+                for (uint32_t j = 0; j < 32; j++) {
+                    const int32_t o = __shfl_sync(0xffffffffu, mine, j);
+                    if (row_ok && o >= 0) y[(size_t)o * n] = __uint_as_float(v[j]);
+                }
+            } else {
+                const uint32_t o0 = it.tt * c.nt + col;
+                if (row_ok && o0 < a.m) {
+                    float *y = c.out.y[it.op] + (size_t)o0 * n + it.n0 + rr;
+                    const uint32_t cnt = min(32u, a.m - o0);
+                    if (some) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; j++)
+                            if (j < cnt) atomicAdd(y + (size_t)j * n, __uint_as_float(v[j]));
+                    } else {
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; j++)
+                            if (j < cnt) y[(size_t)j * n] = __uint_as_float(v[j]);
+                    }
+                }
+            }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) duo::arrive_at_0(&acc_empty[buf]);   // the MMA warp may start on another item here
+        return true;
+    };
 
     if (warp == 0) {
         uint32_t s = 0, ph = 1;   // (a place's first wait passes)
@@ -294,8 +351,8 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
         const uint32_t srow = ((rr & ((1u << c.row_group) - 1u)) << (7 - c.row_group)) + (rr >> c.row_group);   // the row's place in a raw stage
         const uint32_t a_dst = tmem + ((q4 * 32) << 16) + kDuoACol + 32 * half;
         const uint32_t row_bytes = (a.k / QK) * BB;
-        uint32_t rs = 0, rph = 0, J0 = 0;
-        for (uint32_t pos = pos0; ok && pos < pos1;) {
+        uint32_t rs = 0, rph = 0, J0 = 0, nitem = 0;
+        for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
             const Item it = load_item(pos);
             pos = it.next;
             const bool row_ok = it.n0 + rr < c.out.n[it.op];
@@ -312,8 +369,7 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
                     uint32_t regs[32];
                     if (T != GT_Q4_K && c.aligned && row_ok) {   // (Q4_K: the generic extraction below)
                         if constexpr (T == GT_Q6_K) {
-                            dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half, regs);
-                            dequant32_q6k_aligned_p(r_abs & 7u, stage_row, set, 2 * half + 1, regs + 16);
+                            dequant64_q6k_aligned_p(r_abs & 7u, stage_row, set, half, regs);
                         } else if constexpr (T != GT_Q4_K) {
                             switch (2 * set + half) {  // uniform per warp
                             case 0: dequant64_aligned<T, 0>(stage_row, regs); break;
@@ -367,59 +423,17 @@ __global__ void __launch_bounds__(kDuoThreads, 1) __cluster_dims__(2, 1, 1)
             }
             if (!ok) break;
             J0 += it.nst;
+            if constexpr (!ROUTED) {
+                if (!read_back(it, nitem, q4, dw >> 2)) break;
+            }
         }
-    } else if (warp >= 4) {
-        // lane = weight row, 32 activation rows at a time, the two groups of four warps in turn
-        const uint32_t q4 = warp & 3u, g = (warp - 4 - kDuoDequantWarps) >> 2, rr = q4 * 32 + lane;
+    } else if (ROUTED && warp >= 4 + kDuoDequantWarps) {
+        const uint32_t q4 = warp & 3u, g = (warp - 4 - kDuoDequantWarps) >> 2;
         uint32_t nitem = 0;
         for (uint32_t pos = pos0; pos < pos1; nitem++) {
             const Item it = load_item(pos);
             pos = it.next;
-            const uint32_t buf = accs == 2 ? nitem & 1u : 0u, turn = accs == 2 ? nitem >> 1 : nitem, n = c.out.n[it.op];
-            const bool row_ok = it.n0 + rr < n;
-            int32_t mine = -1;   // ROUTED: the output row of activation row 32 g + lane of the tile
-            if constexpr (ROUTED) {
-                const uint32_t ex = __ldcg(a.tiles + 1 + 2 * it.tt), at = __ldcg(a.tiles + 2 + 2 * it.tt) * c.nt + g * 32 + lane;
-                if (at < __ldcg(a.htpe + ex) && at < a.hids_stride) {
-                    mine = __ldcg(a.hids + (size_t)ex * a.hids_stride + at);
-                    if ((uint32_t)mine >= a.total_rows) mine = -1;
-                }
-            }
-            if (!mbar_wait(&acc_full[buf], turn & 1u, &abort_flag, a.status, ST_WAIT_MMA_TIMEOUT, 0u)) break;
-            tc_fence_after();
-            const bool some = it.nraw < nraw_all;   // another pair has the rest of this tile's K
-#pragma unroll 1
-            for (uint32_t col = g * 32; col < c.nt; col += kDuoReadWarps / 4 * 32) {
-                uint32_t v[32];
-                tmem_ld_32x32(tmem + ((q4 * 32) << 16) + buf * 128 + col, v);
-                tmem_ld_wait();
-                if constexpr (ROUTED) {   // (tiles of 64 rows: this is the loop's only turn)
-                    float *y = c.out.y[0] + it.n0 + rr;
-#pragma unroll
-                    for (uint32_t j = 0; j < 32; j++) {
-                        const int32_t o = __shfl_sync(0xffffffffu, mine, j);
-                        if (row_ok && o >= 0) y[(size_t)o * n] = __uint_as_float(v[j]);
-                    }
-                } else {
-                    const uint32_t o0 = it.tt * c.nt + col;
-                    if (row_ok && o0 < a.m) {
-                        float *y = c.out.y[it.op] + (size_t)o0 * n + it.n0 + rr;
-                        const uint32_t cnt = min(32u, a.m - o0);
-                        if (some) {
-#pragma unroll
-                            for (uint32_t j = 0; j < 32; j++)
-                                if (j < cnt) atomicAdd(y + (size_t)j * n, __uint_as_float(v[j]));
-                        } else {
-#pragma unroll
-                            for (uint32_t j = 0; j < 32; j++)
-                                if (j < cnt) y[(size_t)j * n] = __uint_as_float(v[j]);
-                        }
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) duo::arrive_at_0(&acc_empty[buf]);   // the MMA warp may start on another item here
+            if (!read_back(it, nitem, q4, g)) break;
         }
     }
     __syncwarp();
@@ -450,7 +464,7 @@ static uint32_t duo_pairs() {
         int n = 0;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(most * 2);
-        cfg.blockDim = dim3(kDuoThreads);
+        cfg.blockDim = dim3(duo_threads(false));
         cfg.dynamicSmemBytes = 223 * 1024;
         if (cudaFuncSetAttribute(qmm_duo_kernel<GT_Q4_0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, qmm_duo_kernel<GT_Q4_0, false>, &cfg) != cudaSuccess || n < 1 || n > (int)most) {
@@ -544,7 +558,7 @@ template <int T, bool ROUTED> static cudaError_t duo_launch(DuoCfg &c, const Qmm
         prepared[dev].store(1, std::memory_order_release);
     }
     (*launches)++;
-    return launch_overlapped(qmm_duo_kernel<T, ROUTED>, dim3(2 * c.pairs), dim3(kDuoThreads), smem, st, a, c, xpack, wmaps);
+    return launch_overlapped(qmm_duo_kernel<T, ROUTED>, dim3(2 * c.pairs), dim3(duo_threads(ROUTED)), smem, st, a, c, xpack, wmaps);
 }
 
 // `ops`: products of the same activations
@@ -570,7 +584,7 @@ template <int T> static cudaError_t launch_duo_t(const QmmArgs *ops, int nops, u
     const uint64_t slices = (uint64_t)2 * c.ntiles * ((h + kPackRows - 1) / kPackRows);
     while (lanes > 1 && (uint64_t)lanes * slices > 2048) lanes = (lanes + 1) / 2;
     (*launches)++;
-    const cudaError_t e = launch_overlapped(pack_x_kernel, dim3((unsigned)slices, lanes), dim3(256), 0, st, a, xpack, nchunks, h, c.share, c.out);
+    const cudaError_t e = launch_overlapped(pack_x_kernel<false>, dim3((unsigned)slices, lanes), dim3(256), 0, st, a, xpack, nchunks, h, c.share, c.out);
     if (e != cudaSuccess) return e;
     return duo_launch<T, false>(c, ops, nops, xpack, st, launches);
 }

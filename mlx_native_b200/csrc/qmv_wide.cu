@@ -293,7 +293,6 @@ static uint64_t wd_tiles(uint32_t shape, uint32_t m, uint32_t n) {
 // part 717, 510, 522.
 static WdPick wd_pick(const QmvArgs *ops, int nops, int sm_count) {
     WdPick best{1, 1};
-    if (const char *e = exp_env("MLXN_WD")) return WdPick{(uint32_t)(e[0] - '0'), (uint32_t)(e[1] - '0')};
     static const double alone[3] = {1.9, 2.6, 6.1}, shared[3] = {1.62, 2.37, 6.1};
     static const double beside[3][4] = {{0.0, 0.5, 1.1, 1.7}, {0.0, 0.4, 1.3, 2.1}, {6.0, 6.0, 6.5, 7.0}};
     double least = 1e30;
