@@ -39,7 +39,7 @@ namespace mlxn {
 constexpr uint32_t kDuoRows = 256;                          // weight rows of a pair's tile
 constexpr uint32_t kDuoDequantWarps = 16;                   // two sets of eight; set s takes the 128-wide K stages st % 2 == s
 // Warps that read the accumulators back: of their own where tiles are short (routed), else the dequantising ones.
-__host__ __device__ constexpr uint32_t duo_read_warps(bool routed) { return routed ? 8 : kDuoDequantWarps; }
+__host__ __device__ constexpr uint32_t duo_read_warps(bool routed) { return routed ? 4 : kDuoDequantWarps; }
 __host__ __device__ constexpr uint32_t duo_threads(bool routed) { return (4 + kDuoDequantWarps + (routed ? duo_read_warps(true) : 0)) * 32; }
 constexpr uint32_t kDuoStages = 4;                          // ring of K stages: activations in shared memory, weights in tensor memory
 constexpr uint32_t kDuoACol = 256, kDuoACols = 64;          // tensor-memory columns of the weights: 64 a stage (128 f16 pairs)
@@ -111,7 +111,7 @@ __device__ __forceinline__ void commit_both(uint64_t *bar) {
 //   warp 1        CTA 0: MMAs of the pair, whose completion frees the stage's places in both CTAs; CTA 1: tells CTA 0 that its stage is ready
 //   warp 2        raw weights: tensor copies of 128 rows x 256 K values
 //   warps 4..19   dequantise raw blocks into tensor memory; dense: read the accumulator back
-//   warps 20..27  routed: read the accumulators back, two in turn, so that the next item's multiplications go on
+//   warps 20..23  routed: read the accumulators back, two in turn, so that the next item's multiplications go on
 // Ring places and barrier phases run on across the items of a pair.
 //
 // ROUTED: the products of a mixture of experts.  The tiles are those of the list that build_tiles_kernel made, 64 rows of one expert each,
@@ -190,12 +190,16 @@ __global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1,
     auto read_back = [&](const Item &it, uint32_t nitem, uint32_t q4, uint32_t g) {
         const uint32_t buf = accs == 2 ? nitem & 1u : 0u, turn = accs == 2 ? nitem >> 1 : nitem, n = c.out.n[it.op], rr = q4 * 32 + lane;
         const bool row_ok = it.n0 + rr < n;
-        int32_t mine = -1;   // ROUTED: the output row of activation row 32 g + lane of the tile
+        int32_t mine[2] = {-1, -1};   // ROUTED: the output rows of activation rows lane and 32 + lane of the tile
         if constexpr (ROUTED) {
-            const uint32_t ex = __ldcg(a.tiles + 1 + 2 * it.tt), at = __ldcg(a.tiles + 2 + 2 * it.tt) * c.nt + g * 32 + lane;
-            if (at < __ldcg(a.htpe + ex) && at < a.hids_stride) {
-                mine = __ldcg(a.hids + (size_t)ex * a.hids_stride + at);
-                if ((uint32_t)mine >= a.total_rows) mine = -1;
+            const uint32_t ex = __ldcg(a.tiles + 1 + 2 * it.tt), at0 = __ldcg(a.tiles + 2 + 2 * it.tt) * c.nt + lane;
+            const uint32_t rows = min(__ldcg(a.htpe + ex), a.hids_stride);
+#pragma unroll
+            for (uint32_t i = 0; i < 2; i++) {
+                if (at0 + 32 * i < rows) {
+                    mine[i] = __ldcg(a.hids + (size_t)ex * a.hids_stride + at0 + 32 * i);
+                    if ((uint32_t)mine[i] >= a.total_rows) mine[i] = -1;
+                }
             }
         }
         if (!mbar_wait(&acc_full[buf], turn & 1u, &abort_flag, a.status, ST_WAIT_MMA_TIMEOUT, 0u)) return false;
@@ -206,11 +210,12 @@ __global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1,
             uint32_t v[32];
             tmem_ld_32x32(tmem + ((q4 * 32) << 16) + buf * 128 + col, v);
             tmem_ld_wait();
-            if constexpr (ROUTED) {   // (tiles of 64 rows: this is the loop's only turn)
+            if constexpr (ROUTED) {   // (tiles of 64 rows: two turns)
+                const int32_t rows = col ? mine[1] : mine[0];
                 float *y = c.out.y[0] + it.n0 + rr;
 #pragma unroll
                 for (uint32_t j = 0; j < 32; j++) {
-                    const int32_t o = __shfl_sync(0xffffffffu, mine, j);
+                    const int32_t o = __shfl_sync(0xffffffffu, rows, j);
                     if (row_ok && o >= 0) y[(size_t)o * n] = __uint_as_float(v[j]);
                 }
             } else {
