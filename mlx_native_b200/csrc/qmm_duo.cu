@@ -10,7 +10,8 @@
 // 256 24.3 / 19.0, 512 31.1 / 25.0; 12288 x 512 rows 66.7 / 46.4; 1024 x 512 22.4 / 16.8; 4096 x 12288, 2048 rows: Q4_0 205 / 169, Q6_K 229 / 181;
 // 256 x 512 x 16 rows 8.6 / 8.2.  So it takes every call it can: what has no 16-byte aligned weights, or a row count that its copies cannot group,
 // stays with the other kernel, and the row-sharded form.  What bounds it: up to 192 rows the chain raw block -> tensor memory (0.47 us for a
-// K stage of 128, 18 values a cycle and SM; Q6_K 0.66 before its 64 values of a thread were unpacked together: 64 rows 21.0 -> 19.9 us), above that the multiplication (0.43 us at full clock) beside it.
+// K stage of 128, 18 values a cycle and SM; Q6_K 0.66 before its 64 values of a thread were unpacked together: 64 rows 21.0 -> 19.9
+// us), above that the multiplication (0.43 us at full clock) beside it.
 //
 // The items of grouped calls are short (64 rows, K of 6 to 16 stages), and while the dequantising warps read an accumulator back both they and the
 // tensor core would stand still; there the read-back has warps of its own and two accumulators.  (Dense calls gain nothing from it, Q4_0 2048 x 4096 x
