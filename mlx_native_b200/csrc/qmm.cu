@@ -1002,16 +1002,40 @@ static uint64_t tc_plan(uint32_t nt, uint64_t rows, uint64_t n, uint64_t k, uint
     return best;
 }
 
+uint32_t qmm_chain_limit(const QmmArgs &a, int sm_count) {
+    const uint32_t nraw = (a.k + 255) / 256;
+    uint32_t best = 256;
+    uint64_t best_cost = ~0ull;
+    TcPlan plan{};
+    for (uint32_t tt = (a.m + 255) / 256, last = tt + 8; tt <= last; tt++) {
+        const uint32_t nt = ((a.m + tt - 1) / tt + 15) / 16 * 16;
+        TcPlan p;
+        const uint64_t cost = tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count, false, p);
+        if (best_cost == ~0ull || cost * 103 / 100 < best_cost) {
+            best_cost = cost;
+            best = nt;
+            plan = p;
+        }
+        if (nt == 16) break;
+    }
+    const uint64_t tiles = (uint64_t)((a.n + kTcRowsW - 1) / kTcRowsW) * ((a.m + best - 1) / best);
+    const bool halves = plan.shared && plan.ctas == 2 * tiles;
+    const uint32_t has = chain_mean(nraw, halves ? 2 : 1, best > 128 ? 1 : 2, tiles, plan.shared && !halves ? plan.ctas - 1 : 0);
+    const uint32_t least = a.k <= 512 ? kChainAny : (uint32_t)(4096ull * 512 * 512 / ((uint64_t)a.k * a.k));
+    return has > least ? has : least;
+}
+
 // The tile, of either kernel, with which a dense call takes least.
 uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool sharded) {
     uint32_t best = 256;
     uint64_t best_cost = ~0ull;
+    const uint32_t limit = qmm_chain_limit(a, sm_count);
     for (uint32_t tt = (a.m + 255) / 256, last = tt + 8; tt <= last; tt++) {
         uint32_t nt = ((a.m + tt - 1) / tt + 15) / 16 * 16;
         for (int duo = 0; duo < 2; duo++) {
             TcPlan p;
             if (duo) nt = (nt + 31) / 32 * 32;
-            const uint64_t cost = duo ? qmm_duo_cost(ggml_type, a, nt) : tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count, sharded, p);
+            const uint64_t cost = duo ? qmm_duo_cost(ggml_type, a, nt, limit) : tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count, sharded, p);
             if (cost != ~0ull && (best_cost == ~0ull || cost * 103 / 100 < best_cost)) {   // (near a tie, the larger tile: it converts less in all)
                 best_cost = cost;
                 best = nt;
@@ -1022,11 +1046,15 @@ uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool shar
     return best;
 }
 
-// Products of the same activations (and block type) as one launch on pairs of SMs: the tile, 0 where one of them does not go there.
-uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops) {
+// Products of the same activations (and block type) as one launch on pairs of SMs: the tile, 0 where one of them does not go there, and
+// the limit on its chains, the shortest of the products'.
+uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops, int sm_count, uint32_t *limit) {
     QmmArgs all = ops[0];
+    *limit = kChainAny;
     for (int i = 0; i < nops; i++) {
-        if (qmm_duo_cost(ggml_type, ops[i], 32) == ~0ull) return 0;
+        if (qmm_duo_cost(ggml_type, ops[i], 32, kChainAny) == ~0ull) return 0;
+        const uint32_t own = qmm_chain_limit(ops[i], sm_count);
+        if (own < *limit) *limit = own;
         if (i) all.n = (all.n + 255) / 256 * 256 + ops[i].n;   // (as many weight tiles)
     }
     all.n = (all.n + 255) / 256 * 256;
@@ -1034,7 +1062,7 @@ uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops) {
     uint64_t best_cost = ~0ull;
     for (uint32_t tt = (all.m + 255) / 256, last = tt + 8; tt <= last; tt++) {
         const uint32_t nt = ((all.m + tt - 1) / tt + 31) / 32 * 32;
-        const uint64_t cost = qmm_duo_cost(ggml_type, all, nt);
+        const uint64_t cost = qmm_duo_cost(ggml_type, all, nt, *limit);
         if (cost != ~0ull && (best == 0 || cost * 103 / 100 < best_cost)) {
             best_cost = cost;
             best = nt;
@@ -1212,8 +1240,9 @@ cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t
                           int *launches) {
     if (!routed) {
         TcPlan plan;
-        if (qmm_duo_cost(ggml_type, a, nt) < tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count_of_device(), a.y_ld != 0 || a.n_peer != 0, plan))
-            return launch_qmm_duo(ggml_type, &a, 1, nt, scratch, st, launches);
+        const uint32_t limit = qmm_chain_limit(a, sm_count_of_device());
+        if (qmm_duo_cost(ggml_type, a, nt, limit) < tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count_of_device(), a.y_ld != 0 || a.n_peer != 0, plan))
+            return launch_qmm_duo(ggml_type, &a, 1, nt, limit, scratch, st, launches);
     }
     switch (ggml_type) {
     case GT_Q4_0: return launch_tc_t<GT_Q4_0>(a, routed, nt, scratch, st, launches);

@@ -35,10 +35,25 @@ __global__ void pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks,
 
 int sm_count_of_device();
 
+// How exact a mat-mat's sums are.  The tensor core cuts off what an addition to an f32 accumulator leaves below its last bit, always towards zero: a
+// chain of additions over K values is off by 1.2e-9 K of its result (measured against 64 bits, operands as given: K 2048 2.4e-6, 4096
+// 4.8e-6, 6144 7.3e-6), sums outside the tensor core by a rounding.  So chains are to be short: accumulators take turns, tiles are cut
+// along K.  (Either way the operands' rounding to f16, 2.8e-4 of the result, is most of a product's error.)  The measure is the mean square of the chains' lengths, in 4096ths of K^2 and weighted with what they hold.
+constexpr uint32_t kChainAny = 4096;
+// ... of tiles of `nraw` raw stages in `parts` each, `accs` accumulators taking turns, `cut` of the tiles cut once, anywhere, instead.
+inline uint32_t chain_mean(uint32_t nraw, uint32_t parts, uint32_t accs, uint64_t tiles, uint64_t cut) {
+    const uint64_t seg = (nraw + parts - 1) / parts, last = nraw % seg, all = (uint64_t)nraw * nraw * nraw;
+    const uint64_t whole = (4096 * (nraw / seg * seg * seg * seg + last * last * last) + all / 2) / all;
+    if (cut > tiles) cut = tiles;
+    return (uint32_t)((whole * (tiles - cut) + 2048 * cut) / (tiles * accs * accs));
+}
+// The limit that a dense product's launch is to keep, in this measure: what it has on single SMs, and no less than chains of 512 values have.
+uint32_t qmm_chain_limit(const QmmArgs &a, int sm_count);
+
 // The mat-mat on pairs of CTAs (qmm_duo.cu).  Time that it would take, in the units of tc_plan, or ~0 where it does not take the call;
 // `nt` as for the other kernel, a multiple of 32.
-uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt);
-cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches);
+uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt, uint32_t limit);
+cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint32_t limit, uint8_t *xpack, cudaStream_t st, int *launches);
 constexpr uint32_t kRoutedTile = 64;   // rows of a routed tile
 bool qmm_duo_routed_fits(int ggml_type, const QmmArgs &a);
 cudaError_t launch_qmm_duo_routed(int ggml_type, const QmmArgs &a, uint32_t tiles, const uint8_t *xpack, cudaStream_t st, int *launches);

@@ -20,6 +20,13 @@
 // copy rate 61.  Batches: q, k and v of 512 rows (4096, 1024 and 1024 x 4096) and gate and up (12288 x 4096 each) in one launch take a layer from 274
 // to 244 us: one packing instead of three and two, and one last wave.
 //
+// Sums: chains of additions in an accumulator are kept about as short as on single SMs (qmm.cuh): dense tiles have two accumulators up to 192 rows and
+// four up to 64, one K stage each in turn.  Relative error of the sums (64 bits of the operands as rounded to f16), one accumulator / this: 512 and
+// 333 x 4096 x 4096 4.8e-6 / 2.4e-6, 60 x 1024 x 4096 2.4e-6 / 1.2e-6, 512 x 12288 x 4096 4.8e-6 / 2.4e-6; a batch may have twice what its
+// products have alone (k and v of 512 rows 2.4e-6, 1.2e-6).  It costs 0.6 us a call: 512 x 4096 x 4096 25.8 / 26.6, 64 rows 17.1 / 17.9.  Also tried: a
+// tile in parts that are added to y, 3.5 us each at 192 rows (q, k and v 28.3 / 32.4); tiles whose read-back waits for the next one's first
+// stages, no gain (64 rows 18.7).
+//
 // What else was tried: unpacking the weights once into f16 tiles, by a kernel of its own.  The product alone then runs at the
 // multiplication's rate, but the unpacking is bound by memory (13 us for 4096 x 4096, 58 with 2048 rows of 12288 for 4096 x 12288): 32.2 us in
 // all for 512 x 4096 x 4096, 72.8 for 512 x 12288 x 4096.  K in two and four parts over clusters of two and four pairs,
@@ -42,8 +49,10 @@ constexpr uint32_t kDuoDequantWarps = 16;                   // two sets of eight
 // Warps that read the accumulators back: of their own where tiles are short (routed), else the dequantising ones.
 __host__ __device__ constexpr uint32_t duo_read_warps(bool routed) { return routed ? 4 : kDuoDequantWarps; }
 __host__ __device__ constexpr uint32_t duo_threads(bool routed) { return (4 + kDuoDequantWarps + (routed ? duo_read_warps(true) : 0)) * 32; }
-constexpr uint32_t kDuoStages = 4;                          // ring of K stages: activations in shared memory, weights in tensor memory
-constexpr uint32_t kDuoACol = 256, kDuoACols = 64;          // tensor-memory columns of the weights: 64 a stage (128 f16 pairs)
+constexpr uint32_t kDuoStages = 4;                          // ring of K stages, activations in shared memory
+// Tensor memory: accumulators from column 0 on, weights from the last column down, 64 columns a stage (128 f16 values).
+constexpr uint32_t kDuoCols = 512, kDuoACols = 64;
+static_assert(kDuoStages % 2 == 0, "a ring of two stages in tensor memory takes every other place of the ring in shared memory");
 constexpr uint32_t kDuoMaxRaw = 5;
 
 struct DuoCfg {
@@ -51,6 +60,7 @@ struct DuoCfg {
     uint32_t nt;          // activation rows of a tile (a multiple of 32, at most 256)
     uint32_t n_wt, ntiles;
     uint32_t pairs;
+    uint32_t accs;        // dense: accumulators that take turns, nt columns each; a power of two
     TcShare share;        // the pairs' ranges where tiles are shared
     uint32_t seg_stride;  // bytes of a raw row segment in shared memory
     uint32_t raw_off, raw_slots;
@@ -117,11 +127,12 @@ __device__ __forceinline__ void commit_both(uint64_t *bar) {
 //
 // ROUTED: the products of a mixture of experts.  The tiles are those of the list that build_tiles_kernel made, 64 rows of one expert each,
 // packed whole (a CTA's half are rows 0..31 or 32..63 of each 64-column chunk); the weights' map has the expert as third dimension.
-template <int T, bool ROUTED>
-__global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1, 1)
+// RING: K stages of weights in tensor memory, 64 columns each.  The accumulators have what is left: two of 129 to 192 columns leave two stages.
+template <int T, bool ROUTED, uint32_t RING>
+__global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at most 80 registers: a block of the packing kernel fits beside a CTA)
     qmm_duo_kernel(const QmmArgs a, const __grid_constant__ DuoCfg c, const uint8_t *xpack, const __grid_constant__ DuoMaps wmaps) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
-    constexpr uint32_t KR = 256, kReadWarps = duo_read_warps(ROUTED), accs = ROUTED ? 2 : 1;   // (accumulators, 128 columns apart)
+    constexpr uint32_t KR = 256, kReadWarps = duo_read_warps(ROUTED), accs = ROUTED ? 2 : 1;   // (items that are in accumulators, 128 columns apart)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // (the same in both CTAs)
     __shared__ __align__(8) uint64_t full[kDuoStages], peer_full[kDuoStages], done[kDuoStages], raw_full[kDuoMaxRaw], raw_empty[kDuoMaxRaw];
@@ -205,7 +216,8 @@ __global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1,
         }
         if (!mbar_wait(&acc_full[buf], turn & 1u, &abort_flag, a.status, ST_WAIT_MMA_TIMEOUT, 0u)) return false;
         tc_fence_after();
-        const bool some = it.nraw < nraw_all;   // another pair has the rest of this tile's K
+        [[maybe_unused]] const bool some = it.nraw < nraw_all;   // another pair has the rest of this tile's K
+        [[maybe_unused]] const uint32_t used = min(c.accs, it.nst);
 #pragma unroll 1
         for (uint32_t col = g * 32; col < c.nt; col += kReadWarps / 4 * 32) {
             uint32_t v[32];
@@ -220,6 +232,17 @@ __global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1,
                     if (row_ok && o >= 0) y[(size_t)o * n] = __uint_as_float(v[j]);
                 }
             } else {
+#pragma unroll 1
+                for (uint32_t i = 1; i < used; i++) {
+#pragma unroll
+                    for (uint32_t h = 0; h < 32; h += 16) {   // (16 at a time: with more registers the packing kernel's blocks do not fit beside a CTA)
+                        uint32_t z[16];
+                        tmem_ld_32x32_x16(tmem + ((q4 * 32) << 16) + i * c.nt + col + h, z);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (uint32_t j = 0; j < 16; j++) v[h + j] = __float_as_uint(__uint_as_float(v[h + j]) + __uint_as_float(z[j]));
+                    }
+                }
                 const uint32_t o0 = it.tt * c.nt + col;
                 if (row_ok && o0 < a.m) {
                     float *y = c.out.y[it.op] + (size_t)o0 * n + it.n0 + rr;
@@ -278,7 +301,7 @@ __global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1,
         for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
             const Item it = load_item(pos);
             pos = it.next;
-            const uint32_t buf = accs == 2 ? nitem & 1u : 0u, turn = accs == 2 ? nitem >> 1 : nitem, d = tmem + buf * 128;
+            const uint32_t buf = accs == 2 ? nitem & 1u : 0u, turn = accs == 2 ? nitem >> 1 : nitem, turns = ROUTED ? 1u : c.accs;
             // the accumulator's item before has been read back
             if (rank == 0 && !mbar_wait(&acc_empty[buf], (turn & 1u) ^ 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, kSpin)) break;
             tc_fence_after();
@@ -295,10 +318,11 @@ __global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1,
                     }
                     tc_fence_after();
                     if (duo::elect()) {
-                        const uint32_t ac = tmem + kDuoACol + s * kDuoACols;
+                        const uint32_t d = tmem + (ROUTED ? buf * 128 : (st & (turns - 1u)) * c.nt);   // (dense: accumulators take turns)
+                        const uint32_t ac = tmem + kDuoCols - kDuoACols - s % RING * kDuoACols;
                         const uint64_t bd = bd0 + s * (b_stage >> 4), bd1 = bd + (b_chunk >> 4);
 #pragma unroll
-                        for (uint32_t q = 0; q < 4; q++) duo::mma(d, ac + 8 * q, bd + 2 * q, idesc, (st | q) ? 1u : 0u);
+                        for (uint32_t q = 0; q < 4; q++) duo::mma(d, ac + 8 * q, bd + 2 * q, idesc, st >= turns || q ? 1u : 0u);
                         if (2 * st + 1 < it.nck) {
 #pragma unroll
                             for (uint32_t q = 0; q < 4; q++) duo::mma(d, ac + 32 + 8 * q, bd1 + 2 * q, idesc, 1u);
@@ -355,7 +379,7 @@ __global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1,
         const uint32_t dw = warp - 4, q4 = dw & 3u, half = (dw >> 2) & 1u, set = dw >> 3;
         const uint32_t rr = q4 * 32 + lane;
         const uint32_t srow = ((rr & ((1u << c.row_group) - 1u)) << (7 - c.row_group)) + (rr >> c.row_group);   // the row's place in a raw stage
-        const uint32_t a_dst = tmem + ((q4 * 32) << 16) + kDuoACol + 32 * half;
+        const uint32_t a_dst = tmem + ((q4 * 32) << 16) + kDuoCols - kDuoACols + 32 * half;
         const uint32_t row_bytes = (a.k / QK) * BB;
         uint32_t rs = 0, rph = 0, J0 = 0, nitem = 0;
         for (uint32_t pos = pos0; ok && pos < pos1; nitem++) {
@@ -370,7 +394,7 @@ __global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1,
                 }
                 const uint32_t st = 2 * r + set;
                 if (st < it.nst) {
-                    const uint32_t J = J0 + st, sa = J % kDuoStages;   // (J: the stage's number in the pair's whole run)
+                    const uint32_t J = J0 + st, sa = J % kDuoStages, before = J - RING;   // (J: the stage's number in the pair's whole run)
                     const uint32_t r_abs = it.r_lo + r, stage_row = smem_base + c.raw_off + rs * raw_bytes + srow * c.seg_stride;
                     uint32_t regs[32];
                     if (T != GT_Q4_K && c.aligned && row_ok) {   // (Q4_K: the generic extraction below)
@@ -407,13 +431,13 @@ __global__ void __launch_bounds__(duo_threads(ROUTED), 1) __cluster_dims__(2, 1,
                     }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&raw_empty[rs]);   // this warp is done reading the raw stage
-                    // the MMAs that read this place's previous contents (stage J - 4) have completed
-                    if (J >= kDuoStages && !mbar_wait(&done[sa], ((J / kDuoStages) & 1u) ^ 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, 0u)) {
+                    // the MMAs that read this place's previous contents have completed
+                    if (J >= RING && !mbar_wait(&done[before % kDuoStages], (before / kDuoStages) & 1u, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, 0u)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    tmem_st_32x32_x32(a_dst + sa * kDuoACols, regs);
+                    tmem_st_32x32_x32(a_dst - J % RING * kDuoACols, regs);
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();
@@ -472,8 +496,8 @@ static uint32_t duo_pairs() {
         cfg.gridDim = dim3(most * 2);
         cfg.blockDim = dim3(duo_threads(false));
         cfg.dynamicSmemBytes = 223 * 1024;
-        if (cudaFuncSetAttribute(qmm_duo_kernel<GT_Q4_0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, qmm_duo_kernel<GT_Q4_0, false>, &cfg) != cudaSuccess || n < 1 || n > (int)most) {
+        if (cudaFuncSetAttribute(qmm_duo_kernel<GT_Q4_0, false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, qmm_duo_kernel<GT_Q4_0, false, 4>, &cfg) != cudaSuccess || n < 1 || n > (int)most) {
             (void)cudaGetLastError();
             n = (int)most;
         }
@@ -484,30 +508,31 @@ static uint32_t duo_pairs() {
 }
 
 struct DuoPlan {
-    uint32_t pairs, shared;
+    uint32_t pairs, shared, accs;
 };
 // Cost in the units of tc_plan (1.74 ns).  Measured: a K stage of 128 values takes 0.47 us where dequantising bounds it (Q6_K 0.66), else
 // 0.165 us + 2.3 ns per activation row; an item 1 us beside its stages.  Tiles shared by two pairs are zeroed and added up: 3 us and more for
 // wide ones (every tile in halves), 5 us where ranges are shared.
-static uint64_t duo_plan(int type, uint64_t m, uint64_t n, uint64_t k, uint32_t nt, DuoPlan &p) {
+// `limit`: see qmm_chain_limit.  As few accumulators as keep it; a plan that cannot is taken where the others cost 6 % more.
+static uint64_t duo_plan(int type, uint64_t m, uint64_t n, uint64_t k, uint32_t nt, uint32_t limit, DuoPlan &p) {
     const uint64_t sms = duo_pairs(), nraw = (k + 255) / 256, tiles = (n + kDuoRows - 1) / kDuoRows * ((m + nt - 1) / nt);
     const uint64_t convert = type == GT_Q6_K ? 380 : 270, multiply = 95 + nt * 13 / 10, tile = 2 * nraw * (convert > multiply ? convert : multiply);
-    uint64_t best = (tiles + sms - 1) / sms * (tile + 400) + 600;
-    p = {(uint32_t)(tiles < sms ? tiles : sms), 0};
-    if (tiles * nraw >= (1ull << 31)) return best;
-    if (tiles > sms && nraw >= 2) {
-        const uint64_t cost = tiles * tile / sms + (tiles / sms + 2) * 575 + 2900 + nt * 9;
+    const uint32_t room = nt <= 64 ? 4 : nt <= 192 ? 2 : 1;
+    uint64_t best = ~0ull;
+    auto offer = [&](uint64_t cost, uint32_t pairs, bool shared, bool halves) {
+        DuoPlan q{pairs, shared, 1};
+        auto chains = [&] { return chain_mean((uint32_t)nraw, halves ? 2 : 1, q.accs, tiles, shared && !halves ? sms - 1 : 0); };
+        while (chains() > limit && q.accs < room) q.accs *= 2;
+        if (chains() > limit) cost = cost * 106 / 100;
         if (cost < best) {
             best = cost;
-            p = {(uint32_t)sms, 1};
+            p = q;
         }
-    } else if (2 * tiles <= sms && nraw >= 2) {
-        const uint64_t cost = tile / 2 + 2300 + nt * 12;
-        if (cost < best) {
-            best = cost;
-            p = {(uint32_t)(2 * tiles), 1};
-        }
-    }
+    };
+    offer((tiles + sms - 1) / sms * (tile + 400) + 600, (uint32_t)(tiles < sms ? tiles : sms), false, false);
+    if (tiles * nraw >= (1ull << 31) || nraw < 2) return best;
+    if (tiles > sms) offer(tiles * tile / sms + (tiles / sms + 2) * 575 + 2900 + nt * 9, (uint32_t)sms, true, false);
+    else if (2 * tiles <= sms) offer(tile / 2 + 2300 + nt * 12, (uint32_t)(2 * tiles), true, true);
     return best;
 }
 
@@ -516,17 +541,17 @@ static int duo_row_group(uint32_t row_bytes) {
     while ((row_bytes << lg) & 15u) lg++;
     return lg;
 }
-uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt) {
+uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt, uint32_t limit) {
     if (ggml_type != GT_Q4_0 && ggml_type != GT_Q8_0 && ggml_type != GT_Q6_K) return ~0ull;
     if (a.hids || a.y_ld || a.n_peer || a.x2 || nt % 32 != 0 || nt > 256 || a.k % 32 != 0) return ~0ull;
     const uint32_t row_bytes = (a.k / ggml_qk(ggml_type)) * ggml_block_bytes(ggml_type);
     if (((uintptr_t)a.w & 15u) || a.n % (1u << duo_row_group(row_bytes)) != 0 || encode_tiled_fn() == nullptr) return ~0ull;
     DuoPlan p;
-    return duo_plan(ggml_type, a.m, a.n, a.k, nt, p);
+    return duo_plan(ggml_type, a.m, a.n, a.k, nt, limit, p);
 }
 
 // Maps, rings and launch.  `c`: tiles, products and pairs are filled in.
-template <int T, bool ROUTED> static cudaError_t duo_launch(DuoCfg &c, const QmmArgs *ops, int nops, const uint8_t *xpack, cudaStream_t st, int *launches) {
+template <int T, bool ROUTED, uint32_t RING> static cudaError_t duo_launch(DuoCfg &c, const QmmArgs *ops, int nops, const uint8_t *xpack, cudaStream_t st, int *launches) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
     const QmmArgs &a = ops[0];
     const uint32_t row_bytes = (a.k / QK) * BB;
@@ -559,16 +584,17 @@ template <int T, bool ROUTED> static cudaError_t duo_launch(DuoCfg &c, const Qmm
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!prepared[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(qmm_duo_kernel<T, ROUTED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024);
+        const cudaError_t e = cudaFuncSetAttribute(qmm_duo_kernel<T, ROUTED, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024);
         if (e != cudaSuccess) return e;
         prepared[dev].store(1, std::memory_order_release);
     }
     (*launches)++;
-    return launch_overlapped(qmm_duo_kernel<T, ROUTED>, dim3(2 * c.pairs), dim3(duo_threads(ROUTED)), smem, st, a, c, xpack, wmaps);
+    return launch_overlapped(qmm_duo_kernel<T, ROUTED, RING>, dim3(2 * c.pairs), dim3(duo_threads(ROUTED)), smem, st, a, c, xpack, wmaps);
 }
 
 // `ops`: products of the same activations
-template <int T> static cudaError_t launch_duo_t(const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {
+template <int T>
+static cudaError_t launch_duo_t(const QmmArgs *ops, int nops, uint32_t nt, uint32_t limit, uint8_t *xpack, cudaStream_t st, int *launches) {
     if (nops < 1 || nops > (int)kMmOps) return cudaErrorInvalidValue;
     const QmmArgs &a = ops[0];
     const uint32_t h = nt / 2, nraw = (a.k + 255) / 256, nchunks = (a.k + 63) / 64;
@@ -580,10 +606,11 @@ template <int T> static cudaError_t launch_duo_t(const QmmArgs *ops, int nops, u
         c.out.wt_end[i] = c.n_wt;
     }
     DuoPlan p;
-    duo_plan(T, a.m, (uint64_t)c.n_wt * kDuoRows, a.k, nt, p);
+    duo_plan(T, a.m, (uint64_t)c.n_wt * kDuoRows, a.k, nt, limit, p);
     c.nt = nt;
     c.ntiles = (a.m + nt - 1) / nt;
     c.pairs = p.pairs;
+    c.accs = p.accs;
     if (p.shared) c.share = {p.pairs, c.n_wt, nraw, c.n_wt * c.ntiles * nraw, kDuoRows, nt};
     // activations in tiles of nt / 2 rows: a CTA's half of a tile
     uint32_t lanes = nchunks;
@@ -592,7 +619,8 @@ template <int T> static cudaError_t launch_duo_t(const QmmArgs *ops, int nops, u
     (*launches)++;
     const cudaError_t e = launch_overlapped(pack_x_kernel<false>, dim3((unsigned)slices, lanes), dim3(256), 0, st, a, xpack, nchunks, h, c.share, c.out);
     if (e != cudaSuccess) return e;
-    return duo_launch<T, false>(c, ops, nops, xpack, st, launches);
+    return kDuoCols - c.accs * nt >= 4 * kDuoACols ? duo_launch<T, false, 4>(c, ops, nops, xpack, st, launches)
+                                                   : duo_launch<T, false, 2>(c, ops, nops, xpack, st, launches);
 }
 
 template <int T> static cudaError_t launch_duo_routed_t(const QmmArgs &a, uint32_t tiles, const uint8_t *xpack, cudaStream_t st, int *launches) {
@@ -602,12 +630,13 @@ template <int T> static cudaError_t launch_duo_routed_t(const QmmArgs &a, uint32
     c.out.n[0] = a.n;
     c.out.wt_end[0] = c.n_wt;
     c.nt = kRoutedTile;
+    c.accs = 1;
     c.ntiles = tiles;
     const uint64_t items = (uint64_t)c.n_wt * tiles;
     c.pairs = items < duo_pairs() ? (uint32_t)items : duo_pairs();
     c.beside = (a.reuse & 4u) != 0;
     if (!c.pairs) return cudaSuccess;
-    return duo_launch<T, true>(c, &a, 1, xpack, st, launches);
+    return duo_launch<T, true, 4>(c, &a, 1, xpack, st, launches);
 }
 
 // `tiles`: bound of the list's length; `xpack`: what the list's tiles hold
@@ -627,11 +656,11 @@ cudaError_t launch_qmm_duo_routed(int ggml_type, const QmmArgs &a, uint32_t tile
     }
 }
 
-cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches) {
+cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint32_t limit, uint8_t *xpack, cudaStream_t st, int *launches) {
     switch (ggml_type) {
-    case GT_Q4_0: return launch_duo_t<GT_Q4_0>(ops, nops, nt, xpack, st, launches);
-    case GT_Q8_0: return launch_duo_t<GT_Q8_0>(ops, nops, nt, xpack, st, launches);
-    case GT_Q6_K: return launch_duo_t<GT_Q6_K>(ops, nops, nt, xpack, st, launches);
+    case GT_Q4_0: return launch_duo_t<GT_Q4_0>(ops, nops, nt, limit, xpack, st, launches);
+    case GT_Q8_0: return launch_duo_t<GT_Q8_0>(ops, nops, nt, limit, xpack, st, launches);
+    case GT_Q6_K: return launch_duo_t<GT_Q6_K>(ops, nops, nt, limit, xpack, st, launches);
     default: return cudaErrorInvalidValue;
     }
 }

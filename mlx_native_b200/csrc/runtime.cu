@@ -51,9 +51,9 @@ cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t
 cudaError_t launch_qmm_simt(int ggml_type, const QmmArgs &a, bool routed, uint32_t max_rows, cudaStream_t st);
 size_t qmm_tc_scratch_bytes(const QmmArgs &a, uint32_t nt, bool routed);
 constexpr size_t kMmBatchMax = 4;          // mat-mats one launch carries (kMmOps)
-uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt);
-uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops);
-cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint8_t *xpack, cudaStream_t st, int *launches);
+uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt, uint32_t limit);
+uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops, int sm_count, uint32_t *limit);
+cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint32_t limit, uint8_t *xpack, cudaStream_t st, int *launches);
 uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool sharded);
 bool qmm_tc_supported(const QmmArgs &a);
 constexpr uint32_t kRoutedTileRows = 64;   // activation rows of a tile of the grouped mat-mat
@@ -966,10 +966,11 @@ static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
         launches = 0;
         const int n = (int)ops.size(), sms = e->dev->sm_count;
         uint8_t *scratch = nullptr;
-        const uint32_t nt = n > 1 ? qmm_duo_pick_nt(e->pend_type, ops.data(), n) : 0;
+        uint32_t limit = 0;
+        const uint32_t nt = n > 1 ? qmm_duo_pick_nt(e->pend_type, ops.data(), n, sms, &limit) : 0;
         if (nt) {
             if ((rc = encoder_scratch_on(e, e->pend_lane, qmm_tc_scratch_bytes(ops[0], nt, false), &scratch))) return rc;
-            CUDA_TRY(launch_qmm_duo(e->pend_type, ops.data(), n, nt, scratch, st, &launches), "mat-mat launch");
+            CUDA_TRY(launch_qmm_duo(e->pend_type, ops.data(), n, nt, limit, scratch, st, &launches), "mat-mat launch");
         } else {
             for (const QmmArgs &a : ops) {
                 const uint32_t own = qmm_tc_pick_nt(e->pend_type, a, sms, false);
@@ -1799,7 +1800,7 @@ static int dispatch_mm(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
     }
     // A mat-mat that goes to pairs of SMs waits for others of the same activations (q, k and v; gate and up) to share its launch.
     const int type = (int)p->ggml_type;
-    if (tc && !sh && g_opt_mv_batch.load() && qmm_tc_supported(a) && qmm_duo_cost(type, a, 32) != ~0ull) {
+    if (tc && !sh && g_opt_mv_batch.load() && qmm_tc_supported(a) && qmm_duo_cost(type, a, 32, 4096u) != ~0ull) {
         const QmmArgs *h = enc->pend_mm.empty() ? nullptr : &enc->pend_mm[0];
         const bool fits = h && enc->pend_type == type && enc->pend_mm.size() < kMmBatchMax && h->x == a.x && h->m == a.m && h->k == a.k;
         if (enc->pending() && !fits && (rc = encoder_flush_pending(enc))) return rc;

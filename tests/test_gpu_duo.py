@@ -2,6 +2,7 @@
 at most 256), K stages (128 values, two to a raw stage) and work shares, against the oracle with both operands rounded to f16."""
 import numpy as np
 import pytest
+import torch
 
 import mlx_native_b200 as mx
 from oracle import oracle as orc
@@ -62,6 +63,54 @@ def test_beside_the_other_kernel(ctx, tname, n, k, m):
     z = ctx.matmul(gtype, wq, x, n, k, weight_buf=ctx.buf(big, mx.DType.U8).slice_view(6, wq.size))
     y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8, f16_operands=True)
     assert norm_err(y, y_ref, ad) <= TOL and norm_err(z, y_ref, ad) <= TOL
+
+
+def sum_error(y, otype, wq, x, n, k):
+    """Relative error of the sums: against 64 bits of the operands that both kernels multiply, rounded to f16."""
+    f16 = lambda a: torch.tensor(np.ascontiguousarray(a, np.float32)).cuda().half().double()
+    ref = f16(x) @ f16(orc.dequantize(otype, wq).reshape(n, k)).T
+    return float((torch.tensor(y).cuda().double() - ref).norm() / ref.norm())
+
+
+# An accumulator's chain of additions is off by 1.2e-9 of the result for each K value, and no chain may be longer than those of the kernel on
+# single SMs (which takes weights off 16-byte boundaries); chains of 512 values, 6.1e-7, count as short.  One, two and four accumulators; whole
+# tiles, halves and ranges.
+CHAINS = [("Q4_0", 4096, 4096, 512), ("Q4_0", 4096, 4096, 333), ("Q8_0", 1024, 4096, 60), ("Q6_K", 1024, 4096, 96), ("Q4_0", 2688, 1792, 585),
+          ("Q8_0", 6464, 7680, 782), ("Q4_0", 12288, 2048, 512), ("Q6_K", 256, 768, 1000)]
+SHORT = 6.2e-7
+
+
+def other_kernel(ctx, gtype, wq, x, n, k):
+    big = np.zeros(wq.size + 64, np.uint8)
+    big[6:6 + wq.size] = wq.reshape(-1)
+    return ctx.matmul(gtype, wq, x, n, k, weight_buf=ctx.buf(big, mx.DType.U8).slice_view(6, wq.size))
+
+
+@pytest.mark.parametrize("tname,n,k,m", CHAINS)
+def test_sums_are_as_exact_as_on_single_sms(ctx, tname, n, k, m):
+    gtype, otype = TYPES[tname]
+    wq, x = normal_weights(n + k, n, k, otype), normal_acts(m, m, k)
+    other = sum_error(other_kernel(ctx, gtype, wq, x, n, k), otype, wq, x, n, k)
+    y = ctx.matmul(gtype, wq, x, n, k)
+    assert sum_error(y, otype, wq, x, n, k) <= max(1.05 * other, SHORT)
+    assert np.array_equal(y.view(np.uint32), ctx.matmul(gtype, wq, x, n, k).view(np.uint32))
+
+
+# products that travel together, tiles of at most 192 rows: chains of half of K
+@pytest.mark.parametrize("ns,k,m", [((4096, 1024, 1024), 4096, 512), ((5120, 640, 640), 2560, 300), ((9216, 9216), 2048, 100)])
+def test_sums_of_one_group(ctx, ns, k, m):
+    gtype, otype = TYPES["Q4_0"]
+    d, x = ctx.device, normal_acts(m, m, k)
+    ws = [normal_weights(i, n, k, otype) for i, n in enumerate(ns)]
+    xb, bufs = ctx.buf(x, mx.DType.F32), [(ctx.buf(w, mx.DType.U8), d.alloc_buffer(m * n * 4, mx.DType.F32)) for w, n in zip(ws, ns)]
+    enc = d.command_encoder()
+    mx.reset_counters()
+    for (wb, yb), n in zip(bufs, ns):
+        mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, wb, yb, mx.GgmlQuantizedMatmulParams(m, n, k, gtype))
+    enc.commit_and_wait()
+    assert mx.kernel_launch_count() == 2
+    for (_, yb), w, n in zip(bufs, ws, ns):
+        assert sum_error(yb.as_slice(np.float32).reshape(m, n), otype, w, x, n, k) <= 1.3e-9 * k / 2
 
 
 def test_infinities_stay_in_their_row(ctx):
