@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -153,12 +154,24 @@ struct Storage {
     void *host = nullptr;      // pinned shadow, created on first host_map
     bool host_newer = false;   // shadow holds data not yet uploaded
     bool dev_newer = false;    // HBM holds data not yet reflected in the shadow
-    cudaStream_t last_stream = nullptr;  // stream of the last operation that touched the storage
-    bool has_last = false;
+    std::vector<cudaStream_t> users;  // streams with work on the storage that the host has not waited for
     bool kernel_written = false;  // some operation of this library has used the storage as an output
-    struct mlxn_encoder *pend_enc = nullptr;  // encoder holding a not-yet-launched mat-vec that uses the storage
+    // Encoders that hold products on the storage which have been encoded and not launched yet (see encoder_defer).  A storage may have
+    // several: two products that read the same weights.
+    struct Deferred {
+        struct mlxn_encoder *enc;
+        bool writes;
+    };
+    std::vector<Deferred> deferred;
+    std::atomic<size_t> n_deferred{0};   // deferred.size(), to look at without the lock
     std::mutex mu;
 };
+// (with the storage's lock held)
+static void storage_used_on(Storage *s, cudaStream_t st) {
+    for (cudaStream_t u : s->users)
+        if (u == st) return;
+    s->users.push_back(st);
+}
 
 static void storage_release(Storage *s) {
     if (s->refs.fetch_sub(1) == 1) {
@@ -324,7 +337,11 @@ struct mlxn_encoder {
     std::vector<QmmArgs> pend_mm;
     bool pending() const { return !pend.empty() || !pend_mm.empty(); }
     bool grp_pend_only = false;       // every operation of the current group is in `pend` (none has been launched yet)
+    // One thread at a time encodes here, but any thread may have to launch what waits in `pend` or `pend_mm`: it uses a buffer of theirs
+    // through another encoder or from the host.  Held by every call on the encoder, except while it waits for the GPU's end.
+    std::recursive_mutex mu;
 };
+using EncoderLock = std::lock_guard<std::recursive_mutex>;
 
 // ------------------------------------------------------------------------------------------------
 // small helpers
@@ -549,20 +566,37 @@ extern "C" size_t mlxn_buffer_element_count(const mlxn_buffer *buf) { return buf
 extern "C" uint64_t mlxn_buffer_byte_offset(const mlxn_buffer *buf) { return buf->offset; }
 extern "C" void *mlxn_buffer_device_ptr(const mlxn_buffer *buf) { return buf->dev(); }
 
-// wait for whatever touched the storage last (device work or an upload still reading the shadow)
 static int encoder_flush_pending(struct mlxn_encoder *e, bool group_ends = false);
+// Held while a thread launches what another encoder has deferred, and while an encoder goes away.  Taken before any encoder's lock and never with
+// one held: two threads that each encode and need the other's products launched would wait for one another.
+static std::mutex g_foreign_mu;
+// Launches what encoders other than `self` have deferred on the storage and what must come before an operation that reads it or, `writes`, writes it.
+static int storage_settle(Storage *s, const mlxn_encoder *self, bool writes) {
+    if (s->n_deferred.load(std::memory_order_acquire) == 0) return MLXN_OK;
+    std::lock_guard<std::mutex> foreign(g_foreign_mu);
+    std::vector<mlxn_encoder *> encs;
+    {
+        std::lock_guard<std::mutex> lk(s->mu);
+        for (const Storage::Deferred &d : s->deferred)
+            if (d.enc != self && (writes || d.writes || s->host_newer)) encs.push_back(d.enc);
+    }
+    for (mlxn_encoder *e : encs) {
+        EncoderLock lk(e->mu);
+        const int rc = encoder_flush_pending(e);
+        if (rc) return rc;
+    }
+    return MLXN_OK;
+}
+// wait for whatever uses the storage (device work or an upload still reading the shadow); called with its lock held
 static int storage_quiesce(Storage *s) {
-    if (s->pend_enc) {   // a mat-vec that uses the storage is still waiting to be launched
-        struct mlxn_encoder *pe = s->pend_enc;
-        s->mu.unlock();   // the flush takes the storages' locks itself
-        const int rc = encoder_flush_pending(pe);
+    while (!s->deferred.empty()) {   // products that use it wait to be launched
+        s->mu.unlock();              // (the flush takes encoders' and storages' locks itself)
+        const int rc = storage_settle(s, nullptr, true);
         s->mu.lock();
         if (rc) return rc;
     }
-    if (s->has_last) {
-        CUDA_TRY(cudaStreamSynchronize(s->last_stream), "stream synchronize");
-        s->has_last = false;
-    }
+    for (cudaStream_t st : s->users) CUDA_TRY(cudaStreamSynchronize(st), "stream synchronize");
+    s->users.clear();
     return MLXN_OK;
 }
 
@@ -851,13 +885,12 @@ extern "C" int mlxn_encoder_create(mlxn_device *dev, mlxn_encoder **out) {
 }
 
 static void encoder_release_retained(mlxn_encoder *e) {
-    // called once the stream is idle: storages whose last user was this stream no longer need a wait
+    // called once the lanes are idle: nobody has to wait for them on account of these storages
     for (mlxn_buffer *b : e->retained) {
         {
             std::lock_guard<std::mutex> lk(b->st->mu);
-            bool mine = false;
-            for (int l = 0; l < kLanes; l++) mine = mine || b->st->last_stream == e->lanes[l];
-            if (b->st->has_last && mine) b->st->has_last = false;
+            auto &u = b->st->users;
+            for (int l = 0; l < kLanes; l++) u.erase(std::remove(u.begin(), u.end(), e->lanes[l]), u.end());
         }
         mlxn_buffer_release(b);
     }
@@ -869,7 +902,11 @@ static void encoder_release_retained(mlxn_encoder *e) {
 extern "C" void mlxn_encoder_destroy(mlxn_encoder *enc) {
     if (!enc) return;
     cudaSetDevice(enc->ordinal);
-    (void)encoder_flush_pending(enc);
+    {
+        std::lock_guard<std::mutex> foreign(g_foreign_mu);   // afterwards no storage names this encoder
+        EncoderLock lk(enc->mu);
+        (void)encoder_flush_pending(enc);
+    }
     cudaError_t serr = cudaStreamSynchronize(enc->aux);
     for (int l = 0; l < kLanes; l++) {
         cudaError_t e1 = cudaStreamSynchronize(enc->lanes[l]);
@@ -923,6 +960,7 @@ static int encoder_join_lanes(mlxn_encoder *e);
 // behind everything encoded so far.
 extern "C" void *mlxn_encoder_stream(mlxn_encoder *enc) {
     if (!enc) return nullptr;
+    EncoderLock lk(enc->mu);
     cudaSetDevice(enc->ordinal);
     if (!enc->capturing && encoder_join_lanes(enc) != MLXN_OK) return nullptr;
     return (void *)enc->lanes[0];
@@ -944,25 +982,37 @@ static int encoder_mark_fork(mlxn_encoder *e) {
 static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
     if (!e->pending()) return MLXN_OK;
     cudaSetDevice(e->ordinal);
+    cudaStream_t st = e->lanes[e->pend_lane];
+    cudaError_t err = cudaSuccess;
+    int launches = 1, rc = MLXN_OK;
+    // Whatever comes of it, nothing waits afterwards, and it is only afterwards that others do not find it waiting any more.  What it uses
+    // is used on its lane from then on: others may have waited for the lane, and struck it out, while there was nothing in it.
+    struct Leave {
+        mlxn_encoder *e;
+        ~Leave() {
+            e->pend.clear();
+            e->pend_mm.clear();
+            for (mlxn_buffer *b : e->retained) {
+                Storage *s = b->st;
+                if (s->n_deferred.load(std::memory_order_relaxed) == 0) continue;
+                std::lock_guard<std::mutex> lk(s->mu);
+                for (size_t i = 0; i < s->deferred.size(); i++) {
+                    if (s->deferred[i].enc != e) continue;
+                    s->deferred.erase(s->deferred.begin() + i);
+                    s->n_deferred.store(s->deferred.size(), std::memory_order_release);
+                    storage_used_on(s, e->lanes[e->pend_lane]);
+                    break;
+                }
+            }
+        }
+    } leave{e};
     if (!group_ends) {
         const int frc = encoder_mark_fork(e);
         if (frc) return frc;
     }
-    cudaStream_t st = e->lanes[e->pend_lane];
-    cudaError_t err = cudaSuccess;
-    int launches = 1, rc = MLXN_OK;
-    auto leave = [&]() {   // nothing waits any more
-        e->pend.clear();
-        e->pend_mm.clear();
-        for (mlxn_buffer *b : e->retained) {
-            std::lock_guard<std::mutex> lk(b->st->mu);
-            if (b->st->pend_enc == e) b->st->pend_enc = nullptr;
-        }
-    };
     if (!e->pend_mm.empty()) {
         e->grp_pend_only = false;
-        const std::vector<QmmArgs> ops(e->pend_mm);
-        leave();
+        const std::vector<QmmArgs> &ops = e->pend_mm;
         launches = 0;
         const int n = (int)ops.size(), sms = e->dev->sm_count;
         uint8_t *scratch = nullptr;
@@ -1043,7 +1093,6 @@ static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
             }
         }
     }
-    leave();
     if (rc) return rc;
     if (err != cudaSuccess) return cuda_fail(err, "mat-vec launch");
     g_launches.fetch_add((uint64_t)launches);
@@ -1078,6 +1127,7 @@ static int encoder_join_lanes(mlxn_encoder *e) {
 extern "C" int mlxn_encoder_memory_barrier(mlxn_encoder *enc) {
     if (!enc) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: encoder must not be null");
     g_barrier.fetch_add(1);
+    EncoderLock lk(enc->mu);
     cudaSetDevice(enc->ordinal);
     return encoder_join_lanes(enc);
 }
@@ -1094,6 +1144,7 @@ static int encoder_begin_work(mlxn_encoder *e) {
 
 static int encoder_commit(mlxn_encoder *enc, bool timed) {
     if (!enc) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: encoder must not be null");
+    EncoderLock own(enc->mu);
     if (enc->capturing) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: commit while a capture is open");
     cudaSetDevice(enc->ordinal);
     int jrc = encoder_join_lanes(enc);
@@ -1110,8 +1161,7 @@ static int encoder_commit(mlxn_encoder *enc, bool timed) {
         if (st->host && st->dev_newer && st->bytes <= (size_t)(4u << 20)) {
             CUDA_TRY(cudaMemcpyAsync(st->host, st->dptr, st->bytes, cudaMemcpyDeviceToHost, enc->lanes[0]), "device-to-host copy");
             st->dev_newer = false;
-            st->last_stream = enc->lanes[0];
-            st->has_last = true;
+            storage_used_on(st, enc->lanes[0]);
         }
     }
     enc->ev_last = timed ? enc->ev_end : enc->ev_done;
@@ -1141,11 +1191,15 @@ extern "C" int mlxn_encoder_wait_until_completed(mlxn_encoder *enc) {
     if (enc->committed) {
         e = cudaEventSynchronize(enc->ev_last);
     } else {
-        (void)encoder_flush_pending(enc);
+        {
+            EncoderLock lk(enc->mu);
+            (void)encoder_flush_pending(enc);
+        }
         e = cudaStreamSynchronize(enc->aux);
         for (int l = 0; l < kLanes && e == cudaSuccess; l++) e = cudaStreamSynchronize(enc->lanes[l]);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
+    EncoderLock lk(enc->mu);
     encoder_release_retained(enc);
     enc->started = false;
     if (e != cudaSuccess) return cuda_fail(e, "GPU execution");
@@ -1228,6 +1282,7 @@ extern "C" void mlxn_profile_cb_reset(void) {
 
 extern "C" int mlxn_encoder_begin_capture(mlxn_encoder *enc) {
     if (!enc) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: encoder must not be null");
+    EncoderLock lk(enc->mu);
     if (enc->capturing) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: a capture is already open");
     cudaSetDevice(enc->ordinal);
     int jrc = encoder_join_lanes(enc);  // the capture starts from lane 0 alone; other lanes fork from inside it
@@ -1248,6 +1303,7 @@ extern "C" int mlxn_encoder_begin_capture(mlxn_encoder *enc) {
 }
 extern "C" int mlxn_encoder_end_capture(mlxn_encoder *enc, mlxn_graph **out) {
     if (!enc || !out) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: encoder and out must not be null");
+    EncoderLock own(enc->mu);
     if (!enc->capturing) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: no capture is open");
     cudaSetDevice(enc->ordinal);
     int jrc = encoder_join_lanes(enc);  // every forked lane rejoins lane 0 before the capture ends
@@ -1314,6 +1370,7 @@ extern "C" int mlxn_encoder_end_capture(mlxn_encoder *enc, mlxn_graph **out) {
 }
 extern "C" int mlxn_graph_launch(mlxn_graph *graph, mlxn_encoder *enc) {
     if (!graph || !enc) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: graph and encoder must not be null");
+    EncoderLock own(enc->mu);
     if (enc->capturing) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: graph launch while a capture is open");
     // the recorded kernels report through the status block of the encoder that recorded them
     if (graph->sb != enc->sb)
@@ -1327,8 +1384,7 @@ extern "C" int mlxn_graph_launch(mlxn_graph *graph, mlxn_encoder *enc) {
             std::lock_guard<std::mutex> lk(b->st->mu);
             // the replay's copy node reads the pinned shadow when lane 0 gets there: a host write has to wait for it
             b->st->host_newer = false;
-            b->st->last_stream = enc->lanes[0];
-            b->st->has_last = true;
+            storage_used_on(b->st, enc->lanes[0]);
         }
         b->refs.fetch_add(1);
         enc->retained.push_back(b);
@@ -1340,8 +1396,7 @@ extern "C" int mlxn_graph_launch(mlxn_graph *graph, mlxn_encoder *enc) {
             // (a storage the graph fetches itself is current on the host once lane 0 has run the replay)
             const bool fetched_by_graph = graph->covered[oi];
             if (b->st->host) b->st->dev_newer = !fetched_by_graph;
-            b->st->last_stream = enc->lanes[0];
-            b->st->has_last = true;
+            storage_used_on(b->st, enc->lanes[0]);
         }
         b->refs.fetch_add(1);
         enc->retained.push_back(b);  // kept alive, and fetched back at commit like any other result
@@ -1392,17 +1447,22 @@ static int encoder_scratch_on(mlxn_encoder *e, int lane, size_t bytes, uint8_t *
     return MLXN_OK;
 }
 
-// Binds a buffer to the encoder: uploads a newer host shadow on the encoder's stream, records the
-// stream as the storage's last user, and keeps the buffer alive until the encoder's next wait.
+// Binds a buffer to the encoder: waits for other encoders' work on the storage, uploads a newer host shadow on the encoder's stream,
+// records the stream as a user, and keeps the buffer alive until the encoder's next wait.
 static int bind(mlxn_encoder *e, mlxn_buffer *b, bool is_output) {
     Storage *s = b->st;
     std::lock_guard<std::mutex> lk(s->mu);
     if (s->ordinal != e->ordinal)
         return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: buffer lives on device %d, encoder on device %d", s->ordinal, e->ordinal);
-    bool own_lane = false;  // lanes of one encoder are ordered by its group logic, not by host-side waits
-    for (int l = 0; l < kLanes; l++) own_lane = own_lane || s->last_stream == e->lanes[l];
-    if (s->has_last && !own_lane) {
-        CUDA_TRY(cudaStreamSynchronize(s->last_stream), "stream synchronize");
+    for (size_t i = 0; i < s->users.size();) {
+        bool own = false;  // lanes of one encoder are ordered by its group logic, not by host-side waits
+        for (int l = 0; l < kLanes; l++) own = own || s->users[i] == e->lanes[l];
+        if (own) {
+            i++;
+            continue;
+        }
+        CUDA_TRY(cudaStreamSynchronize(s->users[i]), "stream synchronize");
+        s->users.erase(s->users.begin() + i);
     }
     if (s->host_newer) {
         CUDA_TRY(cudaMemcpyAsync(s->dptr, s->host, s->bytes, cudaMemcpyHostToDevice, e->stream), "host-to-device copy");
@@ -1418,8 +1478,7 @@ static int bind(mlxn_encoder *e, mlxn_buffer *b, bool is_output) {
     }
     if (is_output && s->host) s->dev_newer = true;
     if (is_output) s->kernel_written = true;
-    s->last_stream = e->stream;
-    s->has_last = true;
+    storage_used_on(s, e->stream);
     b->refs.fetch_add(1);
     e->retained.push_back(b);
     return MLXN_OK;
@@ -1432,6 +1491,32 @@ struct OpBuf {
     mlxn_buffer *b;
     bool out;
 };
+// An operation's call on an encoder.  Command buffers run in the order in which they were encoded: what other encoders have deferred on the
+// operation's buffers is launched first, so that bind() finds it in their lanes and waits for it.
+struct OpScope {
+    mlxn_encoder *e;
+    int rc = MLXN_OK;
+    OpScope(mlxn_encoder *enc, std::initializer_list<OpBuf> bufs) : e(enc) {
+        for (const OpBuf &ob : bufs)
+            if (ob.b && rc == MLXN_OK) rc = storage_settle(ob.b->st, e, ob.out);
+        e->mu.lock();
+    }
+    ~OpScope() { e->mu.unlock(); }
+    OpScope(const OpScope &) = delete;
+};
+// Products that have been added to `pend` or `pend_mm` use these buffers.
+static void encoder_defer(mlxn_encoder *e, std::initializer_list<OpBuf> bufs) {
+    for (const OpBuf &ob : bufs) {
+        if (!ob.b) continue;
+        Storage *s = ob.b->st;
+        std::lock_guard<std::mutex> lk(s->mu);
+        size_t i = 0;
+        while (i < s->deferred.size() && s->deferred[i].enc != e) i++;
+        if (i == s->deferred.size()) s->deferred.push_back({e, false});
+        s->deferred[i].writes = s->deferred[i].writes || ob.out;
+        s->n_deferred.store(s->deferred.size(), std::memory_order_release);
+    }
+}
 // `lane`: the lane the operation would run on.
 static bool op_conflicts(mlxn_encoder *e, std::initializer_list<OpBuf> bufs, int lane) {
     bool conflict = false;
@@ -1520,6 +1605,7 @@ extern "C" int mlxn_debug_wait_probe(mlxn_encoder *enc, uint32_t limit_us) {
     if (!enc) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: encoder must not be null");
     if (limit_us == 0 || limit_us > 100000)
         return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: wait probe limit (%u us) must be in 1..100000", limit_us);
+    EncoderLock lk(enc->mu);
     int rc = encoder_begin_work(enc);
     if (rc) return rc;
     if ((rc = encoder_join_lanes(enc))) return rc;
@@ -1574,6 +1660,7 @@ extern "C" int mlxn_peer_barrier(mlxn_encoder *enc, uint32_t rank, uint32_t worl
     for (uint32_t r = 0; r < world; r++)
         if (!flag_ptrs[r] || ((uintptr_t)flag_ptrs[r] & 3u))
             return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: peer barrier: flag array %u is null or misaligned", r);
+    EncoderLock lk(enc->mu);
     int rc = encoder_begin_work(enc);
     if (rc) return rc;
     if ((rc = encoder_join_lanes(enc))) return rc;   // everything encoded so far is ahead of the barrier
@@ -1634,11 +1721,7 @@ static int batch_mv(mlxn_encoder *enc, int type, const QmvArgs &a, uint32_t mp, 
         enc->pend_lane = enc->cur_lane;
     }
     enc->pend.push_back(a);
-    for (const OpBuf &ob : bufs) {
-        if (!ob.b) continue;
-        std::lock_guard<std::mutex> lk(ob.b->st->mu);
-        ob.b->st->pend_enc = enc;
-    }
+    encoder_defer(enc, bufs);
     g_dispatch.fetch_add(1);
     return batch ? MLXN_OK : encoder_flush_pending(enc);
 }
@@ -1729,10 +1812,7 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
             }
             enc->pend.push_back(a0);
             enc->pend.back().after_earlier = chained && enc->pend.size() > 1 ? 1u : 0u;
-            for (mlxn_buffer *b : {input, weight, output}) {
-                std::lock_guard<std::mutex> lk(b->st->mu);
-                b->st->pend_enc = enc;
-            }
+            encoder_defer(enc, {{input, false}, {weight, false}, {output, true}});
             g_dispatch.fetch_add(1);
             if (!batch) return encoder_flush_pending(enc);
             return MLXN_OK;
@@ -1810,10 +1890,7 @@ static int dispatch_mm(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
             enc->pend_lane = enc->cur_lane;
         }
         enc->pend_mm.push_back(a);
-        for (mlxn_buffer *b : {input, weight, output}) {
-            std::lock_guard<std::mutex> lk(b->st->mu);
-            b->st->pend_enc = enc;
-        }
+        encoder_defer(enc, {{input, false}, {weight, false}, {output, true}});
         g_dispatch.fetch_add(1);
         return MLXN_OK;
     }
@@ -1874,6 +1951,8 @@ extern "C" int mlxn_quantized_matmul_ggml(mlxn_encoder *enc, mlxn_registry *reg,
     if (rc) return rc;
     if ((rc = validate_dense("quantized_matmul_ggml", input, weight, output, params, true))) return rc;
     if ((rc = check_alignment(input, weight, output))) return rc;
+    OpScope op(enc, {{input, false}, {weight, false}, {output, true}});
+    if (op.rc) return op.rc;
     // Q4_K has no dense mat-mat upstream either: it takes the mat-vec route at any m
     // (src/ops/quantized_matmul_ggml.rs:350-360)
     if (params->m > MLXN_MM_ROUTING_THRESHOLD && params->k >= 32 && (int)params->ggml_type != GT_Q4_K)
@@ -1909,6 +1988,8 @@ extern "C" int mlxn_quantized_matmul_ggml_sharded(mlxn_encoder *enc, mlxn_regist
             return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: quantized_matmul_ggml_sharded: peer output %u is null or misaligned", i);
         sh.peer[i] = static_cast<float *>(peer_outputs[i]);
     }
+    OpScope op(enc, {{input, false}, {weight, false}, {output, true}});
+    if (op.rc) return op.rc;
     if (params->m > MLXN_MM_ROUTING_THRESHOLD) return dispatch_mm(enc, reg, dev, input, weight, output, params, &sh);
     return dispatch_mv(enc, reg, dev, input, weight, output, params, &sh);
 }
@@ -1947,6 +2028,8 @@ extern "C" int mlxn_quantized_matmul_mm_tensor_perm021(mlxn_encoder *enc, mlxn_r
     if (((uintptr_t)weight->dev() & 1u) || ((uintptr_t)output->dev() & 3u) || ((uintptr_t)input_bf16->dev() & 15u))
         return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: quantized_matmul_mm_tensor_perm021: weight data must be 2-byte, output 4-byte, input_bf16 16-byte aligned");
     if ((rc = touch_kernel(reg, dev, t == GT_Q4_0 ? "kernel_mul_mm_q4_0_tensor_bf16_perm021" : "kernel_mul_mm_q6_K_tensor_bf16_perm021"))) return rc;
+    OpScope op(enc, {{input_bf16, false}, {weight, false}, {output, true}});
+    if (op.rc) return op.rc;
     if ((rc = op_begin(enc, {{input_bf16, false}, {weight, false}, {output, true}}))) return rc;
     QmmArgs a{};
     a.w = weight->dev();
@@ -1978,6 +2061,8 @@ extern "C" int mlxn_dispatch_mm_for_test(mlxn_encoder *enc, mlxn_registry *reg, 
     if (rc) return rc;
     if ((rc = validate_dense("dispatch_mm_for_test", input, weight, output, params, false))) return rc;
     if ((rc = check_alignment(input, weight, output))) return rc;
+    OpScope op(enc, {{input, false}, {weight, false}, {output, true}});
+    if (op.rc) return op.rc;
     return dispatch_mm(enc, reg, dev, input, weight, output, params);
 }
 
@@ -2078,11 +2163,7 @@ static int dispatch_id_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *de
             ar.early_weights = 0;
             enc->pend.push_back(ar);
         }
-        for (mlxn_buffer *b : {input, up, weight, ids, output}) {
-            if (!b) continue;
-            std::lock_guard<std::mutex> lk(b->st->mu);
-            b->st->pend_enc = enc;
-        }
+        encoder_defer(enc, {{input, false}, {up, false}, {weight, false}, {ids, false}, {output, true}});
         g_dispatch.fetch_add(1);
         if (!batch) return encoder_flush_pending(enc);
         return MLXN_OK;
@@ -2169,6 +2250,8 @@ extern "C" int mlxn_quantized_matmul_id_ggml(mlxn_encoder *enc, mlxn_registry *r
     if (rc) return rc;
     if ((rc = validate_id("quantized_matmul_id_ggml", input, weight, ids, output, params))) return rc;
     if ((rc = check_alignment(input, weight, output))) return rc;
+    OpScope op(enc, {{input, false}, {weight, false}, {ids, false}, {output, true}});
+    if (op.rc) return op.rc;
     if (!id_routes_to_mm(params)) return dispatch_id_mv(enc, reg, dev, input, weight, ids, output, params);
     if ((rc = op_begin(enc, {{input, false}, {weight, false}, {ids, false}, {output, true}}))) return rc;
     // routing scratch comes out of the encoder's arena instead of two fresh allocations per call
@@ -2210,6 +2293,8 @@ extern "C" int mlxn_quantized_matmul_id_swiglu(mlxn_encoder *enc, mlxn_registry 
                     (size_t)rows * params->k * 4, up->len);
     if ((rc = check_alignment(gate, weight, output))) return rc;
     if ((uintptr_t)up->dev() & 3u) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: f32 buffers must be 4-byte aligned");
+    OpScope op(enc, {{gate, false}, {up, false}, {weight, false}, {ids, false}, {output, true}});
+    if (op.rc) return op.rc;
     return dispatch_id_mv(enc, reg, dev, gate, weight, ids, output, &q, up);
 }
 
@@ -2266,6 +2351,8 @@ extern "C" int mlxn_moe_ffn_layer(mlxn_encoder *enc, mlxn_registry *reg, mlxn_de
         if ((rc = mlxn_silu_mul(enc, reg, dev, gate_out, up_out, up_out, (uint32_t)(pairs * p->ffn)))) return rc;
         return mlxn_quantized_matmul_id_ggml(enc, reg, dev, up_out, down_w, ids, down_out, &pd);
     }
+    OpScope op(enc, {{x, false}, {ids, false}, {gate_w, false}, {up_w, false}, {down_w, false}, {gate_out, true}, {up_out, true}, {down_out, true}});
+    if (op.rc) return op.rc;
     if ((rc = op_begin(enc, {{x, false}, {ids, false}, {gate_w, false}, {up_w, false}, {down_w, false}, {gate_out, true},
                              {up_out, true}, {down_out, true}})))
         return rc;
@@ -2350,6 +2437,8 @@ extern "C" int mlxn_quantized_matmul_id_ggml_pooled(mlxn_encoder *enc, mlxn_regi
     if (rc) return rc;
     if ((rc = validate_id("quantized_matmul_id_ggml_pooled", input, weight, ids, output, params))) return rc;
     if ((rc = check_alignment(input, weight, output))) return rc;
+    OpScope op(enc, {{input, false}, {weight, false}, {ids, false}, {output, true}, {htpe, true}, {hids, true}});
+    if (op.rc) return op.rc;
     if (!id_routes_to_mm(params)) return dispatch_id_mv(enc, reg, dev, input, weight, ids, output, params);
     if (params->n_experts > n_experts_cap)
         return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: IdMmScratch: n_experts (%u) > cap (%u)", params->n_experts, n_experts_cap);
@@ -2370,6 +2459,8 @@ extern "C" int mlxn_dispatch_id_mm_for_test(mlxn_encoder *enc, mlxn_registry *re
     if ((rc = validate_id("dispatch_id_mm_for_test", input, weight, ids, output, params))) return rc;
     if ((rc = check_alignment(input, weight, output))) return rc;
     if ((rc = check_scratch_buffers(htpe, hids, params))) return rc;
+    OpScope op(enc, {{input, false}, {weight, false}, {ids, false}, {output, true}, {htpe, true}, {hids, true}});
+    if (op.rc) return op.rc;
     if ((rc = op_begin(enc, {{input, false}, {weight, false}, {ids, false}, {output, true}, {htpe, true}, {hids, true}})))
         return rc;
     return dispatch_id_mm_stages(enc, reg, dev, input, weight, ids, output, reinterpret_cast<uint32_t *>(htpe->dev()),
@@ -2392,6 +2483,8 @@ extern "C" int mlxn_moe_softmax_topk(mlxn_encoder *enc, mlxn_registry *reg, mlxn
         out_weights->len < (size_t)n_tokens * top_k * 4)
         return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: moe_softmax_topk: a buffer is too small");
     if ((rc = touch_kernel(reg, dev, "moe_softmax_topk_f32"))) return rc;
+    OpScope op(enc, {{logits, false}, {out_ids, true}, {out_weights, true}});
+    if (op.rc) return op.rc;
     if ((rc = op_begin(enc, {{logits, false}, {out_ids, true}, {out_weights, true}}))) return rc;
     CUDA_TRY(launch_moe_softmax_topk(reinterpret_cast<const float *>(logits->dev()), n_tokens, n_experts, top_k,
                                      reinterpret_cast<uint32_t *>(out_ids->dev()), reinterpret_cast<float *>(out_weights->dev()),
@@ -2411,6 +2504,8 @@ extern "C" int mlxn_silu_mul(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device 
     if (gate->len < (size_t)n * 4 || up->len < (size_t)n * 4 || out->len < (size_t)n * 4)
         return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: silu_mul: a buffer is too small for %u f32 elements", n);
     if ((rc = touch_kernel(reg, dev, "silu_mul_f32"))) return rc;
+    OpScope op(enc, {{gate, false}, {up, false}, {out, true}});
+    if (op.rc) return op.rc;
     if ((rc = op_begin(enc, {{gate, false}, {up, false}, {out, true}}))) return rc;
     CUDA_TRY(launch_silu_mul(reinterpret_cast<const float *>(gate->dev()), reinterpret_cast<const float *>(up->dev()),
                              reinterpret_cast<float *>(out->dev()), n, enc->stream),
@@ -2434,6 +2529,8 @@ static int moe_weighted_reduce_impl(mlxn_encoder *enc, mlxn_registry *reg, mlxn_
         (local_ids && local_ids->len < (size_t)n_tokens * top_k * 4))
         return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: moe_weighted_reduce: a buffer is too small");
     if ((rc = touch_kernel(reg, dev, "moe_weighted_reduce_f32"))) return rc;
+    OpScope op(enc, {{expert_w, false}, {y_expert, false}, {out, true}, {sh_logit, false}, {y_shared, false}, {residual, false}, {local_ids, false}});
+    if (op.rc) return op.rc;
     if ((rc = op_begin(enc, {{expert_w, false}, {y_expert, false}, {out, true}, {sh_logit, false}, {y_shared, false},
                              {residual, false}, {local_ids, false}})))
         return rc;
@@ -2477,6 +2574,8 @@ extern "C" int mlxn_moe_expert_shard_route(mlxn_encoder *enc, mlxn_registry *reg
     if (n_pairs == 0 || expert_count == 0) return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: moe_expert_shard_route: n_pairs and expert_count must be > 0");
     if (ids->len < (size_t)n_pairs * 4 || local_ids->len < (size_t)n_pairs * 4)
         return fail(MLXN_INVALID_ARGUMENT, "Invalid argument: moe_expert_shard_route: a buffer is too small");
+    OpScope op(enc, {{ids, false}, {local_ids, true}});
+    if (op.rc) return op.rc;
     if ((rc = op_begin(enc, {{ids, false}, {local_ids, true}}))) return rc;
     CUDA_TRY(launch_moe_expert_shard_route(reinterpret_cast<const uint32_t *>(ids->dev()),
                                            reinterpret_cast<uint32_t *>(local_ids->dev()), n_pairs, expert_lo, expert_count,
