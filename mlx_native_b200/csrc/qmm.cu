@@ -1368,9 +1368,8 @@ extern "C" int mlxn_quantized_matmul_ggml_mm_noalloc(void *cuda_stream, const vo
     a.status = nullptr;  // no status word: a wait that gives up still ends the kernel, but is not reported
     uint32_t nt = qmm_tc_pick_nt(t, a, sms, false);
     size_t need = qmm_tc_scratch_bytes(a, nt, false);
-    // (the fastest tile may pad the rows more than another one that still fits)
-    for (uint32_t other : {256u, 128u, 64u})
-        if (need > MLXN_NOALLOC_SCRATCH_BYTES) need = qmm_tc_scratch_bytes(a, nt = other, false);
+    // (the fastest tile may pad the rows more than another one that still fits; tiles of 16 rows pad least)
+    for (uint32_t other = 256; other >= 16 && need > MLXN_NOALLOC_SCRATCH_BYTES; other -= 16) need = qmm_tc_scratch_bytes(a, nt = other, false);
     if (need > MLXN_NOALLOC_SCRATCH_BYTES) {
         char msg[256];
         snprintf(msg, sizeof(msg),

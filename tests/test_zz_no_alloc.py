@@ -65,3 +65,30 @@ def test_noalloc_rejects_what_does_not_fit():
         mx.quantized_matmul_ggml_mm_noalloc(0, 0, 256, 256, P(16, 128, 256, mx.GgmlType.Q4_0))
     with pytest.raises(mx.InvalidArgument, match="divisible"):
         mx.quantized_matmul_ggml_mm_noalloc(0, 256, 256, 256, P(16, 128, 48, mx.GgmlType.Q4_0))
+
+
+# Sizes close to the limit: the fastest tile, and tiles of 256, 128 and 64 rows, pad the rows too much; another one fits.  The last one is the
+# limit itself.
+@pytest.mark.parametrize("tname,m,n,k", [("Q4_0", 711, 12288, 11296), ("Q8_0", 713, 256, 11264), ("Q4_0", 1281, 2048, 6336), ("Q6_K", 16, 64, 524288)])
+def test_noalloc_takes_every_size_that_some_tile_fits(tname, m, n, k):
+    gtype, otype = TYPES[tname]
+    ctx, rows = Ctx(), min(n, 256)
+    d = ctx.device
+    part, x = normal_weights(m, rows, k, otype), normal_acts(m, m, k)
+    wb, xb = ctx.buf(np.tile(part, n // rows), mx.DType.U8), ctx.buf(x, mx.DType.F32)
+    yb = d.alloc_buffer(m * n * 4, mx.DType.F32)
+    enc = d.command_encoder()
+    mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, wb, yb, mx.GgmlQuantizedMatmulParams(1, 8, 256, gtype))   # (uploads all of them)
+    enc.commit_and_wait()
+    mx.quantized_matmul_ggml_mm_noalloc(enc.stream(), xb.contents_ptr(), wb.contents_ptr(), yb.contents_ptr(), mx.GgmlQuantizedMatmulParams(m, n, k, gtype))
+    enc.commit_and_wait()
+    y = yb.download(np.float32).reshape(m, n)
+    some = np.r_[0:2, m // 2, m - 2:m]
+    y_ref, ad = orc.qmatmul(otype, part, x[some], rows, k, nthreads=8)
+    for at in range(0, n, rows):
+        assert norm_err(y[some, at:at + rows], y_ref, ad) <= MM_TOL
+
+
+def test_noalloc_refuses_one_row_more_than_the_limit():
+    with pytest.raises(mx.InvalidArgument, match="static scratch holds 16777216"):
+        mx.quantized_matmul_ggml_mm_noalloc(0, 256, 256, 256, mx.GgmlQuantizedMatmulParams(17, 64, 524288, mx.GgmlType.Q6_K))
