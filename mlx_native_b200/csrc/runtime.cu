@@ -2407,10 +2407,10 @@ extern "C" int mlxn_moe_ffn_layer(mlxn_encoder *enc, mlxn_registry *reg, mlxn_de
         return MLXN_OK;
     };
     if ((rc = product(pg, x, nullptr, gate_w, gate_out, 0u))) return rc;          // builds the tile list, packs x
-    // ... takes both over, and (bit 2) runs beside the first where that one's result is neither the weights nor the result of this one
-    const uint8_t *g0 = reinterpret_cast<const uint8_t *>(gate_out->dev()), *g1 = g0 + pairs * p->ffn * 4;
-    auto apart = [&](const void *at, size_t bytes) { return g1 <= (const uint8_t *)at || (const uint8_t *)at + bytes <= g0; };
-    const bool beside = apart(up_out->dev(), pairs * p->ffn * 4) && apart(up_w->dev(), (size_t)p->n_experts * pu.expert_stride);
+    // ... takes both over, and (bit 2) runs beside the first where neither writes what the other one reads or writes
+    auto apart = [](mlxn_buffer *a, size_t a_bytes, mlxn_buffer *b, size_t b_bytes) { return a->dev() + a_bytes <= b->dev() || b->dev() + b_bytes <= a->dev(); };
+    const size_t result = pairs * p->ffn * 4, gate_bytes = (size_t)p->n_experts * pg.expert_stride, up_bytes = (size_t)p->n_experts * pu.expert_stride;
+    const bool beside = apart(gate_out, result, up_out, result) && apart(gate_out, result, up_w, up_bytes) && apart(up_out, result, gate_w, gate_bytes);
     if ((rc = product(pu, x, nullptr, up_w, up_out, beside ? 7u : 3u))) return rc;
     if ((rc = product(pd, gate_out, up_out, down_w, down_out, 1u))) return rc;    // same tiles; packs silu(gate) * up
     g_last_kernel = "qmm_tc_id";

@@ -246,3 +246,28 @@ def test_routed_layer_with_one_result_buffer(ctx):
         enc.commit_and_wait()
         got.append((yu.as_slice(np.float32).copy(), yd.as_slice(np.float32).copy()))
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("gate_off", [0, 6])
+def test_routed_layer_with_the_result_over_weights(ctx, gate_off):
+    """up's result over gate's weights, which the gate product has to have read by then.  With gate's weights off 16-byte boundaries the kernel
+    ahead of up's is the one on single SMs."""
+    d, T, E, top_k, hidden, ffn = ctx.device, 256, 8, 2, 512, 512
+    gtype, otype = TYPES["Q4_0"]
+    gate, up, down = (np.concatenate([normal_weights(at + e, 512, 512, otype) for e in range(E)]).reshape(-1) for at in (0, 20, 40))
+    ids = np.random.default_rng(1).permuted(np.tile(np.arange(E), (T, 1)), axis=1)[:, :top_k].astype(np.uint32).reshape(-1)
+    xb, ib = ctx.buf(normal_acts(5, T, hidden), mx.DType.F32), ctx.buf(ids, mx.DType.U32)
+    p = mx.MoeFfnLayerParams(T, top_k, hidden, ffn, E, gtype, gtype, gtype, *([gate.size // E] * 3))
+    result, got = T * top_k * ffn * 4, []
+    for over in (True, False):
+        big = np.zeros(max(gate.size + 64, result), np.uint8)
+        big[gate_off:gate_off + gate.size] = gate
+        both = ctx.buf(big, mx.DType.U8)
+        wg, wu, wd = both.slice_view(gate_off, gate.size), ctx.buf(up, mx.DType.U8), ctx.buf(down, mx.DType.U8)
+        yu = both.slice_view(0, result) if over else d.alloc_buffer(result, mx.DType.F32)
+        yg, yd = d.alloc_buffer(result, mx.DType.F32), d.alloc_buffer(T * top_k * hidden * 4, mx.DType.F32)
+        enc = d.command_encoder()
+        mx.moe_ffn_layer(enc, ctx.registry, d, xb, ib, wg, wu, wd, yg, yu, yd, p)
+        enc.commit_and_wait()
+        got.append([b.as_slice(np.float32).copy() for b in (yg, yu, yd)])
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
