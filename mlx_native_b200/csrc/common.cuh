@@ -129,7 +129,8 @@ struct QmmArgs {
     uint32_t head_dim;
     // Fused MoE layer (routed tensor-core form): what an earlier call of the same layer has left in the scratch area and
     // this call takes over instead of building it again (bit 0: the tile list, bit 1: the packed activations), whether it needs
-    // nothing from the kernel directly ahead in the stream, only from those before it (bit 2), and the
+    // nothing from the kernel directly ahead in the stream, only from those before it (bit 2; that kernel has to wait for those in all its blocks
+    // before it lets this one be launched, as both mat-mat kernels do and the mat-vec kernels do not), and the
     // second operand of a SwiGLU formed while packing: activations = silu(x) * x2 (src/shaders/silu_mul.metal:17-30).
     uint32_t reuse;
     const float *x2;

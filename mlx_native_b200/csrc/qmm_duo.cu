@@ -167,7 +167,13 @@ __global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at mos
     duo::cluster_sync();
     tc_fence_after();
     const uint32_t tmem = tmem_s;
-    if (!c.beside) grid_dependency_wait();   // the packed activations, the tile list and the zeros of shared tiles are complete
+    if (!c.beside) {
+        grid_dependency_wait();   // the packed activations, the tile list and the zeros of shared tiles are complete
+    } else {
+        // ... which they were for every block of the kernel ahead before it let this one be launched: taken over from it, for loads and for copies
+        __threadfence();
+        fence_proxy_async();
+    }
     allow_dependents();
 
     // ---- work items: weight tile fastest, so that the pairs working at the same time share an activation tile in L2 ----
