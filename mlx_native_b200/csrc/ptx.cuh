@@ -94,8 +94,9 @@ __device__ __forceinline__ void bulk_g2s(void *smem_dst, const void *gmem_src, u
                  "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
-// Make generic-proxy shared-memory writes visible to the async proxy (TMA, tcgen05 operand reads).
+// Orders accesses of the generic and of the async proxy, in all of memory.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+// Make generic-proxy shared-memory writes visible to the async proxy (TMA, tcgen05 operand reads).
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // ---- named barriers -----------------------------------------------------------------------------

@@ -70,7 +70,8 @@ struct DuoCfg {
     TcOut out;
 };
 struct DuoMaps {
-    CUtensorMap m[kMmOps];
+    CUtensorMap m[kMmOps];   // weights of the products
+    CUtensorMap x;           // packed activations: [64-wide chunks][8-row groups of 1 KB][256 words]
 };
 
 namespace duo {
@@ -87,13 +88,22 @@ __device__ __forceinline__ bool elect() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\t@p mov.u32 %0, 1;\n\t}" : "+r"(p));
     return p != 0;
 }
-// Arrives on the barrier at the same place in CTA 0.  Without release: what it announces are finished copies and tensor-memory stores,
-// no stores of this thread (with it the instruction takes a thousand cycles, which then bounded the whole kernel).
+__device__ __forceinline__ uint32_t in_cta_0(uint64_t *bar) {   // the barrier at the same place in CTA 0
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(bar)));
+    return a;
+}
+// Arrives on the barrier at the same place in CTA 0.  Relaxed: what it announces are loads and stores of tensor memory only, which the fences of
+// tcgen05 before it and behind the wait for it order (with release the instruction takes a thousand cycles, which then bounded the whole kernel).
+// Nothing in shared memory may be announced so: the activations' copies complete on CTA 0's barriers themselves.
 __device__ __forceinline__ void arrive_at_0(uint64_t *bar) {
-    asm volatile(
-        "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\t"
-        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar))
-        : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(in_cta_0(bar)) : "memory");
+}
+// Tensor copy into this CTA's shared memory that completes on a barrier of either CTA of the pair.
+__device__ __forceinline__ void copy_3d(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst), "l"(map),
+                 "r"(x), "r"(y), "r"(z), "r"(bar)
+                 : "memory");
 }
 __device__ __forceinline__ void alloc(uint32_t *dst, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(cols) : "memory");
@@ -118,7 +128,7 @@ __device__ __forceinline__ void commit_both(uint64_t *bar) {
 }  // namespace duo
 
 // Clusters of two CTAs, one CTA per SM, persistent.  Per CTA:
-//   warp 0        activations: one bulk copy per K stage (two 64-wide chunks of its half of the tile)
+//   warp 0        activations: one tensor copy per K stage (two 64-wide chunks of its half of the tile), which completes on CTA 0's barrier
 //   warp 1        CTA 0: MMAs of the pair, whose completion frees the stage's places in both CTAs; CTA 1: tells CTA 0 that its stage is ready
 //   warp 2        raw weights: tensor copies of 128 rows x 256 K values
 //   warps 4..19   dequantise raw blocks into tensor memory; dense: read the accumulator back
@@ -130,7 +140,7 @@ __device__ __forceinline__ void commit_both(uint64_t *bar) {
 // RING: K stages of weights in tensor memory, 64 columns each.  The accumulators have what is left: two of 129 to 192 columns leave two stages.
 template <int T, bool ROUTED, uint32_t RING>
 __global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at most 80 registers: a block of the packing kernel fits beside a CTA)
-    qmm_duo_kernel(const QmmArgs a, const __grid_constant__ DuoCfg c, const uint8_t *xpack, const __grid_constant__ DuoMaps wmaps) {
+    qmm_duo_kernel(const QmmArgs a, const __grid_constant__ DuoCfg c, const __grid_constant__ DuoMaps wmaps) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
     constexpr uint32_t KR = 256, kReadWarps = duo_read_warps(ROUTED), accs = ROUTED ? 2 : 1;   // (items that are in accumulators, 128 columns apart)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -144,7 +154,7 @@ __global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at mos
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (uint32_t s = 0; s < kDuoStages; s++) {
-            mbar_init(&full[s], 9);   // the activations' copy, and the eight warps of a set
+            mbar_init(&full[s], rank == 0 ? 9 : 8);   // the eight warps of a set; CTA 0: and the activations' copies, both halves
             mbar_init(&peer_full[s], 1);
             mbar_init(&done[s], 1);
         }
@@ -276,22 +286,16 @@ __global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at mos
         for (uint32_t pos = pos0; ok && pos < pos1;) {
             const Item it = load_item(pos);
             pos = it.next;
-            const uint8_t *src = ROUTED ? xpack + ((size_t)it.tt * c.nchunks + it.kc_lo) * b_stage + rank * b_chunk
-                                        : xpack + ((size_t)(it.tt * 2u + rank) * c.nchunks + it.kc_lo) * b_chunk;
-            for (uint32_t st = 0; st < it.nst; st++, src += ROUTED ? 2 * b_stage : b_stage) {
+            // (a K tail of 64 brings a chunk of the next tile, or zeros, which is not multiplied)
+            uint32_t chunk = (ROUTED ? it.tt : it.tt * 2u + rank) * c.nchunks + it.kc_lo;
+            for (uint32_t st = 0; st < it.nst; st++, chunk += 2) {
                 if (!mbar_wait(&done[s], ph, &abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT, kSpin)) {
                     ok = false;
                     break;
                 }
                 if (duo::elect()) {
-                    const uint32_t bytes = 2 * st + 1 < it.nck ? b_stage : b_chunk;   // (a K tail of 64)
-                    mbar_expect_tx(&full[s], bytes);
-                    if constexpr (ROUTED) {
-                        bulk_g2s(smem + s * b_stage, src, b_chunk, &full[s]);
-                        if (bytes == b_stage) bulk_g2s(smem + s * b_stage + b_chunk, src + b_stage, b_chunk, &full[s]);
-                    } else {
-                        bulk_g2s(smem + s * b_stage, src, bytes, &full[s]);
-                    }
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * b_stage);
+                    duo::copy_3d(smem_base + s * b_stage, &wmaps.x, 0, ROUTED ? rank * 4 : 0, chunk, duo::in_cta_0(&full[s]));
                 }
                 __syncwarp();
                 if (++s == kDuoStages) {
@@ -578,6 +582,14 @@ template <int T, bool ROUTED, uint32_t RING> static cudaError_t duo_launch(DuoCf
                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
+    {
+        const uint32_t groups = c.nt / (ROUTED ? 8 : 16), box_groups = c.nt / 16;   // of a packed chunk, of a CTA's half
+        const cuuint64_t gdim[3] = {256, groups, (uint64_t)c.ntiles * (ROUTED ? 1 : 2) * c.nchunks}, gstride[2] = {1024, groups * 1024ull};
+        const cuuint32_t box[3] = {256, box_groups, 2}, estr[3] = {1, 1, 1};
+        if (enc(&wmaps.x, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint8_t *>(xpack), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
     const uint32_t limit = 222 * 1024, b_bytes = kDuoStages * c.nt * 128u, raw_slot = 128 * c.seg_stride;
     c.raw_off = b_bytes;
     c.raw_slots = (limit - b_bytes) / raw_slot;
@@ -595,7 +607,7 @@ template <int T, bool ROUTED, uint32_t RING> static cudaError_t duo_launch(DuoCf
         prepared[dev].store(1, std::memory_order_release);
     }
     (*launches)++;
-    return launch_overlapped(qmm_duo_kernel<T, ROUTED, RING>, dim3(2 * c.pairs), dim3(duo_threads(ROUTED)), smem, st, a, c, xpack, wmaps);
+    return launch_overlapped(qmm_duo_kernel<T, ROUTED, RING>, dim3(2 * c.pairs), dim3(duo_threads(ROUTED)), smem, st, a, c, wmaps);
 }
 
 // `ops`: products of the same activations
