@@ -1052,7 +1052,7 @@ uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops, int sm_cou
     QmmArgs all = ops[0];
     *limit = kChainAny;
     for (int i = 0; i < nops; i++) {
-        if (qmm_duo_cost(ggml_type, ops[i], 32, kChainAny) == ~0ull) return 0;
+        if (!qmm_duo_takes(ggml_type, ops[i])) return 0;
         const uint32_t own = qmm_chain_limit(ops[i], sm_count);
         if (own < *limit) *limit = own;
         if (i) all.n = (all.n + 255) / 256 * 256 + ops[i].n;   // (as many weight tiles)

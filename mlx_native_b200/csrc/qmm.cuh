@@ -50,8 +50,9 @@ inline uint32_t chain_mean(uint32_t nraw, uint32_t parts, uint32_t accs, uint64_
 // The limit that a dense product's launch is to keep, in this measure: what it has on single SMs, and no less than chains of 512 values have.
 uint32_t qmm_chain_limit(const QmmArgs &a, int sm_count);
 
-// The mat-mat on pairs of CTAs (qmm_duo.cu).  Time that it would take, in the units of tc_plan, or ~0 where it does not take the call;
-// `nt` as for the other kernel, a multiple of 32.
+// The mat-mat on pairs of CTAs (qmm_duo.cu): whether it takes the call, which types, sizes and alignment decide, and the time that it would take
+// (~0 where it does not) on the thread's current device, in the units of tc_plan; `nt` as for the other kernel, a multiple of 32.
+bool qmm_duo_takes(int ggml_type, const QmmArgs &a);
 uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt, uint32_t limit);
 cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint32_t limit, uint8_t *xpack, cudaStream_t st, int *launches);
 constexpr uint32_t kRoutedTile = 64;   // rows of a routed tile

@@ -551,11 +551,14 @@ static int duo_row_group(uint32_t row_bytes) {
     while ((row_bytes << lg) & 15u) lg++;
     return lg;
 }
-uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt, uint32_t limit) {
-    if (ggml_type != GT_Q4_0 && ggml_type != GT_Q8_0 && ggml_type != GT_Q6_K) return ~0ull;
-    if (a.hids || a.y_ld || a.n_peer || a.x2 || nt % 32 != 0 || nt > 256 || a.k % 32 != 0) return ~0ull;
+bool qmm_duo_takes(int ggml_type, const QmmArgs &a) {
+    if (ggml_type != GT_Q4_0 && ggml_type != GT_Q8_0 && ggml_type != GT_Q6_K) return false;
+    if (a.hids || a.y_ld || a.n_peer || a.x2 || a.k % 32 != 0) return false;
     const uint32_t row_bytes = (a.k / ggml_qk(ggml_type)) * ggml_block_bytes(ggml_type);
-    if (((uintptr_t)a.w & 15u) || a.n % (1u << duo_row_group(row_bytes)) != 0 || encode_tiled_fn() == nullptr) return ~0ull;
+    return ((uintptr_t)a.w & 15u) == 0 && a.n % (1u << duo_row_group(row_bytes)) == 0 && encode_tiled_fn() != nullptr;
+}
+uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt, uint32_t limit) {
+    if (nt % 32 != 0 || nt > 256 || !qmm_duo_takes(ggml_type, a)) return ~0ull;
     DuoPlan p;
     return duo_plan(ggml_type, a.m, a.n, a.k, nt, limit, p);
 }

@@ -52,7 +52,7 @@ cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t
 cudaError_t launch_qmm_simt(int ggml_type, const QmmArgs &a, bool routed, uint32_t max_rows, cudaStream_t st);
 size_t qmm_tc_scratch_bytes(const QmmArgs &a, uint32_t nt, bool routed);
 constexpr size_t kMmBatchMax = 4;          // mat-mats one launch carries (kMmOps)
-uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt, uint32_t limit);
+bool qmm_duo_takes(int ggml_type, const QmmArgs &a);
 uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops, int sm_count, uint32_t *limit);
 cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint32_t limit, uint8_t *xpack, cudaStream_t st, int *launches);
 uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool sharded);
@@ -1880,7 +1880,7 @@ static int dispatch_mm(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
     }
     // A mat-mat that goes to pairs of SMs waits for others of the same activations (q, k and v; gate and up) to share its launch.
     const int type = (int)p->ggml_type;
-    if (tc && !sh && g_opt_mv_batch.load() && qmm_tc_supported(a) && qmm_duo_cost(type, a, 32, 4096u) != ~0ull) {
+    if (tc && !sh && g_opt_mv_batch.load() && qmm_tc_supported(a) && qmm_duo_takes(type, a)) {
         const QmmArgs *h = enc->pend_mm.empty() ? nullptr : &enc->pend_mm[0];
         const bool fits = h && enc->pend_type == type && enc->pend_mm.size() < kMmBatchMax && h->x == a.x && h->m == a.m && h->k == a.k;
         if (enc->pending() && !fits && (rc = encoder_flush_pending(enc))) return rc;
