@@ -380,6 +380,9 @@ int mlxn_debug_split_geometry(const mlxn_qmm_id_params *params, uint32_t misalig
 /* Name of the kernel variant the last operation on this thread launched (for tests and profiles).  Mat-vecs wait for the operations
  * that follow and are launched, and named, when their batch is (by a commit at the latest). */
 const char *mlxn_last_kernel_name(void);
+/* Which of the kernels behind "qmm_tc" (dense) and "qmm_tc_id" (grouped) this thread launched last, and the activation rows of its tiles (for
+ * tests): "qmm_duo" / "qmm_duo_id" on pairs of SMs, "qmm_tc" / "qmm_tc_id" on single ones, "" before the first.  tile_rows may be null. */
+const char *mlxn_debug_last_mat_mat(uint32_t *tile_rows);
 
 #ifdef __cplusplus
 }

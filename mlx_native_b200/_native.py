@@ -128,6 +128,7 @@ SIGNATURES = {
     "mlxn_debug_split_geometry": (i32, [C.POINTER(QmmIdParams), u32, u32, C.POINTER(u32), C.POINTER(u32)]),
     "mlxn_debug_wait_probe": (i32, [vp, u32]),
     "mlxn_last_kernel_name": (C.c_char_p, []),
+    "mlxn_debug_last_mat_mat": (C.c_char_p, [C.POINTER(u32)]),
 }
 
 

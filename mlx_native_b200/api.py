@@ -487,6 +487,12 @@ def last_kernel_name() -> str:
     return _native.lib().mlxn_last_kernel_name().decode()
 
 
+def last_mat_mat() -> tuple[str, int]:
+    """Kernel of this thread's last mat-mat ("qmm_duo" on pairs of SMs, "qmm_tc" on single ones, with "_id" if grouped) and its tiles' activation rows."""
+    rows = C.c_uint32()
+    return _native.lib().mlxn_debug_last_mat_mat(C.byref(rows)).decode(), rows.value
+
+
 def peer_barrier(encoder: "CommandEncoder", rank: int, world: int, flag_ptrs, epoch: int, limit_us: int = 2000000) -> None:
     """Cross-rank barrier over peer memory (see mlxn_peer_barrier): flag_ptrs[r] = device address of rank r's flag array
     (uint32[world], zero-initialised) as mapped into this process; `epoch` grows by one per barrier."""

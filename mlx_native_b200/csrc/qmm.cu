@@ -941,6 +941,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const QmmArgs a, 
 // =================================================================================================
 // host-side launchers
 // =================================================================================================
+static thread_local const char *t_mat_mat = "";
+static thread_local uint32_t t_mat_mat_rows = 0;
+void note_mat_mat(const char *kernel, uint32_t tile_rows) {
+    t_mat_mat = kernel;
+    t_mat_mat_rows = tile_rows;
+}
+
 static inline uint32_t round_up_u(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
 int sm_count_of_device() {
     static int sms[64] = {};
@@ -1218,6 +1225,7 @@ static cudaError_t launch_tc_tn(QmmArgs a, bool routed, uint32_t nt, uint8_t *sc
     }
     if (ctas == 0) return cudaSuccess;
     (*launches)++;
+    note_mat_mat(routed ? "qmm_tc_id" : "qmm_tc", nt);
     return launch_overlapped(qmm_tc_kernel<T, NT, SH>, dim3(ctas), dim3(kTcThreads), smem, st, a, c, xpack, wmap);
 }
 
@@ -1271,6 +1279,11 @@ cudaError_t launch_qmm_simt(int ggml_type, const QmmArgs &a, bool routed, uint32
 }
 
 }  // namespace mlxn
+
+extern "C" const char *mlxn_debug_last_mat_mat(uint32_t *tile_rows) {
+    if (tile_rows) *tile_rows = mlxn::t_mat_mat_rows;
+    return mlxn::t_mat_mat;
+}
 
 // =================================================================================================
 // mat-mat entry point that allocates nothing

@@ -34,6 +34,7 @@ template <bool SWIGLU>
 __global__ void pack_x_kernel(const QmmArgs a, uint8_t *xpack, uint32_t nchunks, uint32_t nt, const TcShare sh, const __grid_constant__ TcOut res);
 
 int sm_count_of_device();
+void note_mat_mat(const char *kernel, uint32_t tile_rows);   // see mlxn_debug_last_mat_mat
 
 // How exact a mat-mat's sums are.  The tensor core cuts off what an addition to an f32 accumulator leaves below its last bit, always towards zero: a
 // chain of additions over K values is off by 1.2e-9 K of its result (measured against 64 bits, operands as given: K 2048 2.4e-6, 4096

@@ -610,6 +610,7 @@ template <int T, bool ROUTED, uint32_t RING> static cudaError_t duo_launch(DuoCf
         prepared[dev].store(1, std::memory_order_release);
     }
     (*launches)++;
+    note_mat_mat(ROUTED ? "qmm_duo_id" : "qmm_duo", c.nt);
     return launch_overlapped(qmm_duo_kernel<T, ROUTED, RING>, dim3(2 * c.pairs), dim3(duo_threads(ROUTED)), smem, st, a, c, wmaps);
 }
 

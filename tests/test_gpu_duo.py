@@ -29,7 +29,7 @@ def test_dense(ctx, tname, n, k, m):
     wq = normal_weights(n + k, n, k, otype)
     x = normal_acts(n + m, m, k)
     y = ctx.matmul(gtype, wq, x, n, k)
-    assert mx.last_kernel_name() == "qmm_tc"
+    assert mx.last_kernel_name() == "qmm_tc" and mx.last_mat_mat()[0] == "qmm_duo"
     y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8, f16_operands=True)
     assert norm_err(y, y_ref, ad) <= TOL
     assert np.array_equal(y.view(np.uint32), ctx.matmul(gtype, wq, x, n, k).view(np.uint32))
@@ -42,6 +42,7 @@ def test_many_tiles(ctx, tname, n, k, m):
     part = normal_weights(k, 1024, k, otype)
     x = normal_acts(m, m, k)
     y = ctx.matmul(gtype, np.tile(part, n // 1024), x, n, k)
+    assert mx.last_mat_mat()[0] == "qmm_duo"
     rows = np.r_[0:40, m - 40:m] if m > 200 else np.arange(m)
     y_ref, ad = orc.qmatmul(otype, part, x[rows], 1024, k, nthreads=8, f16_operands=True)
     for at in range(0, n, 1024):
@@ -60,7 +61,9 @@ def test_beside_the_other_kernel(ctx, tname, n, k, m):
     big[6:6 + wq.size] = wq
     x = normal_acts(7, m, k)
     y = ctx.matmul(gtype, wq, x, n, k)
+    assert mx.last_mat_mat()[0] == "qmm_duo"
     z = ctx.matmul(gtype, wq, x, n, k, weight_buf=ctx.buf(big, mx.DType.U8).slice_view(6, wq.size))
+    assert mx.last_mat_mat()[0] == "qmm_tc"
     y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8, f16_operands=True)
     assert norm_err(y, y_ref, ad) <= TOL and norm_err(z, y_ref, ad) <= TOL
 
@@ -83,7 +86,9 @@ SHORT = 6.2e-7
 def other_kernel(ctx, gtype, wq, x, n, k):
     big = np.zeros(wq.size + 64, np.uint8)
     big[6:6 + wq.size] = wq.reshape(-1)
-    return ctx.matmul(gtype, wq, x, n, k, weight_buf=ctx.buf(big, mx.DType.U8).slice_view(6, wq.size))
+    y = ctx.matmul(gtype, wq, x, n, k, weight_buf=ctx.buf(big, mx.DType.U8).slice_view(6, wq.size))
+    assert mx.last_mat_mat()[0] == "qmm_tc"
+    return y
 
 
 @pytest.mark.parametrize("tname,n,k,m", CHAINS)
@@ -92,6 +97,7 @@ def test_sums_are_as_exact_as_on_single_sms(ctx, tname, n, k, m):
     wq, x = normal_weights(n + k, n, k, otype), normal_acts(m, m, k)
     other = sum_error(other_kernel(ctx, gtype, wq, x, n, k), otype, wq, x, n, k)
     y = ctx.matmul(gtype, wq, x, n, k)
+    assert mx.last_mat_mat()[0] == "qmm_duo"
     assert sum_error(y, otype, wq, x, n, k) <= max(1.05 * other, SHORT)
     assert np.array_equal(y.view(np.uint32), ctx.matmul(gtype, wq, x, n, k).view(np.uint32))
 
@@ -122,7 +128,7 @@ def test_infinities_stay_in_their_row(ctx):
     y = ctx.matmul(gtype, wq, x, n, k)
     bad = np.zeros(m, bool)
     bad[[5, 40]] = True
-    assert np.isfinite(y[~bad]).all() and not np.isfinite(y[bad]).any(axis=1).all()
+    assert np.isfinite(y[~bad]).all() and not np.isfinite(y[bad]).any()   # (no weight of these is zero)
     y_ref, ad = orc.qmatmul(otype, wq, x[~bad], n, k, nthreads=4, f16_operands=True)
     assert norm_err(y[~bad], y_ref, ad) <= TOL
 
@@ -226,6 +232,7 @@ def test_routed_tiles(ctx, tname, n, k):
             y_ref, ad = orc.qmatmul(otype, ws[e], x[rows], n, k, nthreads=4, f16_operands=True)
             assert norm_err(y[rows], y_ref, ad) <= TOL
     assert not y[ids == E + 7].any()
+    assert mx.last_mat_mat() == ("qmm_tc_id" if n == 261 else "qmm_duo_id", 64)
 
 
 def test_routed_layer_with_one_result_buffer(ctx):
@@ -269,5 +276,50 @@ def test_routed_layer_with_the_result_over_weights(ctx, gate_off):
         enc = d.command_encoder()
         mx.moe_ffn_layer(enc, ctx.registry, d, xb, ib, wg, wu, wd, yg, yu, yd, p)
         enc.commit_and_wait()
+        assert mx.last_mat_mat()[0] == "qmm_duo_id"
         got.append([b.as_slice(np.float32).copy() for b in (yg, yu, yd)])
     assert all(np.array_equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("capture", [False, True])
+def test_waiting_products_beside_the_other_lane(ctx, capture):
+    """A group of two products that wait, then work that starts at once on the other lane; the next groups write over what these read."""
+    gtype, otype = TYPES["Q4_0"]
+    d, m, n = ctx.device, 40, 512
+    ws = [normal_weights(i, n, n, otype) for i in range(2)]
+    wbufs = [ctx.buf(w, mx.DType.U8) for w in ws]
+    a, gate, up = normal_acts(1, m, n), normal_acts(2, m, n), normal_acts(3, m, n)
+    bufs = {k: ctx.buf(v, mx.DType.F32) for k, v in (("a", a), ("g", gate), ("u", up))}
+    for k in ("b", "c", "s", "t"):
+        bufs[k] = ctx.buf(np.zeros((m, n), np.float32), mx.DType.F32)
+    p = mx.GgmlQuantizedMatmulParams(m, n, n, gtype)
+    enc = d.command_encoder()
+
+    def encode():
+        for _ in range(4):
+            for w, y in zip(wbufs, "bc"):
+                mx.quantized_matmul_ggml(enc, ctx.registry, d, bufs["a"], w, bufs[y], p)          # wait for one another
+            mx.silu_mul(enc, ctx.registry, d, bufs["g"], bufs["u"], bufs["s"], m * n)              # other lane
+            mx.silu_mul(enc, ctx.registry, d, bufs["s"], bufs["u"], bufs["t"], m * n)              # conflict: a new group
+            mx.quantized_matmul_ggml(enc, ctx.registry, d, bufs["t"], wbufs[0], bufs["s"], p)      # reads t, writes over s
+            mx.quantized_matmul_ggml(enc, ctx.registry, d, bufs["c"], wbufs[1], bufs["b"], p)      # reads c, writes over b
+
+    encode()
+    enc.commit_and_wait()
+    if capture:
+        for k in ("b", "c", "s", "t"):
+            bufs[k].as_mut_slice(np.float32)[:] = 0
+            mx.silu_mul(enc, ctx.registry, d, bufs[k], bufs[k], bufs["t"], m * n)   # (uploaded before the recording)
+        enc.commit_and_wait()
+        enc.begin_capture()
+        encode()
+        graph = enc.end_capture()
+        graph.launch(enc)
+        enc.commit_and_wait()
+    get = lambda k: bufs[k].as_slice(np.float32).reshape(m, n).copy()
+    silu = lambda g, u: (g / (1 + np.exp(-g.astype(np.float64))) * u).astype(np.float32)
+    t, c = get("t"), get("c")
+    assert np.allclose(t, silu(silu(gate, up), up), rtol=1e-5, atol=1e-6)
+    for got, x, w in ((c, a, ws[1]), (get("b"), c, ws[1]), (get("s"), t, ws[0])):
+        y_ref, ad = orc.qmatmul(otype, w, x, n, n, nthreads=4, f16_operands=True)
+        assert norm_err(got, y_ref, ad) <= TOL

@@ -71,6 +71,34 @@ def test_products_of_one_group_share_a_launch(ctx):
         assert norm_err(yb.as_slice(np.float32).reshape(m, n), y_ref, ad) <= MV_TOL
 
 
+def test_a_captured_group(ctx):
+    """Recorded once, replayed on other activations and results of before."""
+    d, m, n, k = ctx.device, 19, 1100, 1024
+    ws = [normal_weights(i, n, k, O) for i in range(2)]
+    xb = ctx.buf(normal_acts(1, m, k), mx.DType.F32)
+    bufs = [(ctx.buf(w, mx.DType.U8), ctx.buf(np.zeros((m, n), np.float32), mx.DType.F32)) for w in ws]
+    enc = d.command_encoder()
+
+    def encode():
+        for wb, yb in bufs:
+            mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, wb, yb, mx.GgmlQuantizedMatmulParams(m, n, k, G))
+
+    encode()
+    enc.commit_and_wait()
+    enc.begin_capture()
+    encode()
+    graph = enc.end_capture()
+    assert mx.last_kernel_name() == "qmv_wide"
+    for seed in (2, 3):
+        x = normal_acts(seed, m, k)
+        xb.upload(x)
+        graph.launch(enc)
+        enc.commit_and_wait()
+        for (_, yb), w in zip(bufs, ws):
+            y_ref, ad = orc.qmatmul(O, w, x, n, k, nthreads=4)
+            assert norm_err(yb.as_slice(np.float32).reshape(m, n), y_ref, ad) <= MV_TOL
+
+
 def test_weights_off_16_byte_boundaries_take_another_kernel(ctx):
     n, k, m = 512, 2048, 12
     wq = normal_weights(9, n, k, O)
