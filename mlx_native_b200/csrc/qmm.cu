@@ -1038,17 +1038,17 @@ uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool shar
     uint64_t best_cost = ~0ull;
     const uint32_t limit = qmm_chain_limit(a, sm_count);
     for (uint32_t tt = (a.m + 255) / 256, last = tt + 8; tt <= last; tt++) {
-        uint32_t nt = ((a.m + tt - 1) / tt + 15) / 16 * 16;
+        const uint32_t rows = ((a.m + tt - 1) / tt + 15) / 16 * 16;
         for (int duo = 0; duo < 2; duo++) {
             TcPlan p;
-            if (duo) nt = (nt + 31) / 32 * 32;
+            const uint32_t nt = duo ? (rows + 31) / 32 * 32 : rows;
             const uint64_t cost = duo ? qmm_duo_cost(ggml_type, a, nt, limit) : tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count, sharded, p);
             if (cost != ~0ull && (best_cost == ~0ull || cost * 103 / 100 < best_cost)) {   // (near a tie, the larger tile: it converts less in all)
                 best_cost = cost;
                 best = nt;
             }
         }
-        if (nt <= 32) break;
+        if (rows == 16) break;
     }
     return best;
 }

@@ -323,3 +323,17 @@ def test_waiting_products_beside_the_other_lane(ctx, capture):
     for got, x, w in ((c, a, ws[1]), (get("b"), c, ws[1]), (get("s"), t, ws[0])):
         y_ref, ad = orc.qmatmul(otype, w, x, n, n, nthreads=4, f16_operands=True)
         assert norm_err(got, y_ref, ad) <= TOL
+
+
+# The kernel on single SMs keeps its tiles of 16 rows (a long K, so that converting for each tile is what a call takes), which that on
+# pairs of SMs does not have.
+@pytest.mark.parametrize("tname,n,k,m", [("Q4_0", 256, 10496, 45), ("Q8_0", 320, 10496, 93)])
+def test_tiles_of_16_rows_on_single_sms(ctx, tname, n, k, m):
+    gtype, otype = TYPES[tname]
+    wq, x = normal_weights(n, n, k, otype), normal_acts(m, m, k)
+    y = other_kernel(ctx, gtype, wq, x, n, k)
+    assert mx.last_mat_mat() == ("qmm_tc", 16)
+    y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8, f16_operands=True)
+    assert norm_err(y, y_ref, ad) <= TOL
+    ctx.matmul(gtype, wq, x, n, k)
+    assert mx.last_mat_mat()[0] == "qmm_duo"
