@@ -43,10 +43,10 @@ void note_mat_mat(const char *kernel, uint32_t tile_rows);   // see mlxn_debug_l
 constexpr uint32_t kChainAny = 4096;
 // ... of tiles of `nraw` raw stages in `parts` each, `accs` accumulators taking turns, `cut` of the tiles cut once, anywhere, instead.
 inline uint32_t chain_mean(uint32_t nraw, uint32_t parts, uint32_t accs, uint64_t tiles, uint64_t cut) {
-    const uint64_t seg = (nraw + parts - 1) / parts, last = nraw % seg, all = (uint64_t)nraw * nraw * nraw;
-    const uint64_t whole = (4096 * (nraw / seg * seg * seg * seg + last * last * last) + all / 2) / all;
+    const uint32_t seg = (nraw + parts - 1) / parts, last = nraw % seg;
+    const double a = (double)seg / nraw, b = (double)last / nraw, whole = nraw / seg * (a * a * a) + b * b * b;
     if (cut > tiles) cut = tiles;
-    return (uint32_t)((whole * (tiles - cut) + 2048 * cut) / (tiles * accs * accs));
+    return (uint32_t)(kChainAny * (whole * (double)(tiles - cut) + 0.5 * (double)cut) / ((double)tiles * accs * accs));
 }
 // The limit that a dense product's launch is to keep, in this measure: what it has on single SMs, and no less than chains of 512 values have.
 uint32_t qmm_chain_limit(const QmmArgs &a, int sm_count);
