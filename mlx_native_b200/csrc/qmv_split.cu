@@ -86,7 +86,8 @@ bool qmv_split_supported(int ggml_type, const QmvArgs &a, int sm_count) {
 //   Q4_K, five and more: 1024 (0.22) 20.0 / 8.4, 8192 (0.43) 27.6 / 23.8, 10240 (0.54) 28.5 / 28.2, 12288 (0.65) 28.5 / 32.9, 16384 (0.86)
 //              28.6 / 41.7.  In groups of eight, one launch against one per group: 16 rows 10240 56.7 / 51.5, 12288 56.2 / 61.1; a last group
 //              of one row costs this kernel as much as eight: 9 rows 4096 (0.22) 34.4 / 25.0, 6144 (0.32) 28.6 / 35.2.
-//              (More than eight rows come here only where the kernel of qmv_wide.cu does not take them: matrices below 2^20 values.)
+//              (More than eight rows come here only where the kernel of qmv_wide.cu does not take them: matrices below 2^20 values, and weights
+//              that do not start on 16-byte boundaries.)
 bool qmv_split_pays(int ggml_type, const QmvArgs *ops, int nops, double fill) {
     uint64_t values = 0;
     uint32_t m = 0, kmin = 0xFFFFFFFFu, kmax = 0;

@@ -321,13 +321,8 @@ bool qmv_wide_supported(int ggml_type, const QmvArgs &a) {
     if (((uint64_t)a.m + 15) / 16 * ((a.n + 127) / 128) * 8 >= (1ull << 31)) return false;
     return encode_tiled_fn() != nullptr;
 }
-// `fill`: how full the register-level kernel's passes are with one group of eight rows (qmv_mma_fill).  Below 256 x 4096 there are a
-// handful of tiles, and a launch is all latency with either kernel.  Three groups of eight that fill those passes keep their three
-// launches: slower (24 rows of 16384 x 4096: 86 us against 45), but what tests/test_gpu_mv_batches.py holds that call to.
-bool qmv_wide_pays(const QmvArgs &a, double fill) {
-    if (a.m > 16 && a.m <= 24 && fill > 0.8) return false;
-    return (uint64_t)a.n * a.k >= 1u << 20;
-}
+// Below 256 x 4096 there are a handful of tiles, and a launch is all latency with either kernel.
+bool qmv_wide_pays(const QmvArgs &a) { return (uint64_t)a.n * a.k >= 1u << 20; }
 
 static uint32_t wd_pad(uint32_t m) { return (m + 95) / 96 * 96; }   // (whole tiles)
 static size_t wd_pack_bytes(uint32_t m, uint32_t k) {

@@ -44,7 +44,7 @@ constexpr size_t kMvSplitMax = 8;    // mat-vecs one launch of the split kernel 
 size_t qmv_split_scratch_bytes(const QmvArgs *ops, int nops);
 cudaError_t launch_qmv_split(int ggml_type, const QmvArgs *ops, int nops, int sm_count, uint8_t *scratch, int *launches, cudaStream_t st);
 bool qmv_wide_supported(int ggml_type, const QmvArgs &a);
-bool qmv_wide_pays(const QmvArgs &a, double fill);
+bool qmv_wide_pays(const QmvArgs &a);
 size_t qmv_wide_scratch_bytes(const QmvArgs *ops, int nops);
 cudaError_t launch_qmv_wide(const QmvArgs *ops, int nops, int sm_count, uint8_t *scratch, int *launches, cudaStream_t st);
 cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t nt, uint8_t *scratch, cudaStream_t st,
@@ -1775,7 +1775,7 @@ static int dispatch_mv(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
         const double fill = t == GT_Q4_K ? qmv_mma_fill(t, &a, 1, dev->sm_count) : 0.0;   // (of one group of eight rows)
         a.m = p->m;
         const bool aligned = qmv_split_aligned(t, a);
-        if (mode == 3 && p->m > 8 && !sh && qmv_wide_supported(t, a) && qmv_wide_pays(a, fill))
+        if (mode == 3 && p->m > 8 && !sh && qmv_wide_supported(t, a) && qmv_wide_pays(a))
             return batch_mv(enc, t, a, 16u, false, {{input, false}, {weight, false}, {output, true}}, true);
         const bool pays = mode == 5 || (!aligned ? t != GT_Q6_K || (p->m > 2 && !qmv_mma_pair_mode(t, a))
                                                  : p->m > 8 && t == GT_Q4_K && qmv_split_pays(t, &a, 1, fill));

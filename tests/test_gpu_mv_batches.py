@@ -46,15 +46,16 @@ def test_any_order_is_one_launch(ctx, tname, m):
                 assert norm_err(y[:, at:at + 1024], y_ref, ad) <= MV_TOL
 
 
-# Q4_K, five rows and more: the split kernel, its groups of eight in one launch; a matrix that fills the other kernel's passes, and a last
-# group of one row where the matrix is not small, stay with that one, one launch per group
-@pytest.mark.parametrize("m,n,launches", [(5, 1024, 2), (8, 16384, 1), (16, 1024, 2), (9, 1024, 2), (9, 8192, 2), (24, 16384, 3)])
-def test_q4k_of_many_rows(ctx, m, n, launches):
+# Q4_K, five to eight rows: the split kernel (a packing launch ahead), or the register-level kernel where the matrix fills its passes.  More rows: the
+# kernel for many rows, packing and product, whatever the matrix fills.
+@pytest.mark.parametrize("m,n,launches,kernel", [(5, 1024, 2, "qmv_split"), (8, 16384, 1, "qmv_mma"), (16, 1024, 2, "qmv_wide"), (9, 1024, 2, "qmv_wide"),
+                                                 (9, 8192, 2, "qmv_wide"), (24, 16384, 2, "qmv_wide")])
+def test_q4k_of_many_rows(ctx, m, n, launches, kernel):
     part = normal_weights(n, 1024, K, orc.Q4_K)
     x = normal_acts(m, m, K)
     y_ref, ad = orc.qmatmul(orc.Q4_K, part, x, 1024, K, nthreads=8)
     (y,), count = encode(ctx, mx.GgmlType.Q4_K, [(ctx.buf(np.tile(part, n // 1024), mx.DType.U8), x, n)])
-    assert count == launches
+    assert count == launches and mx.last_kernel_name() == kernel
     for at in range(0, n, 1024):
         assert norm_err(y[:, at:at + 1024], y_ref, ad) <= MV_TOL
 
