@@ -1009,47 +1009,59 @@ static uint64_t tc_plan(uint32_t nt, uint64_t rows, uint64_t n, uint64_t k, uint
     return best;
 }
 
-uint32_t qmm_chain_limit(const QmmArgs &a, int sm_count) {
-    const uint32_t nraw = (a.k + 255) / 256;
-    uint32_t best = 256;
+// The tiles that a dense call is offered, what the kernel on single SMs takes with them, and its choice.
+struct TcChoice {
+    uint32_t count, best, rows[9];
+    uint64_t cost[9];
+    TcPlan plan;   // of the chosen one
+};
+static void tc_choose(const QmmArgs &a, int sm_count, bool sharded, TcChoice &c) {
     uint64_t best_cost = ~0ull;
-    TcPlan plan{};
-    for (uint32_t tt = (a.m + 255) / 256, last = tt + 8; tt <= last; tt++) {
-        const uint32_t nt = ((a.m + tt - 1) / tt + 15) / 16 * 16;
+    c.count = 0;
+    for (uint32_t tt = (a.m + 255) / 256; c.count < 9; tt++) {
+        const uint32_t i = c.count++;
         TcPlan p;
-        const uint64_t cost = tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count, false, p);
-        if (best_cost == ~0ull || cost * 103 / 100 < best_cost) {
-            best_cost = cost;
-            best = nt;
-            plan = p;
+        c.rows[i] = ((a.m + tt - 1) / tt + 15) / 16 * 16;
+        c.cost[i] = tc_plan(c.rows[i], a.m, a.n, a.k, (uint64_t)sm_count, sharded, p);
+        if (best_cost == ~0ull || c.cost[i] * 103 / 100 < best_cost) {   // (near a tie, the larger tile: it converts less in all)
+            best_cost = c.cost[i];
+            c.best = i;
+            c.plan = p;
         }
-        if (nt == 16) break;
+        if (c.rows[i] == 16) break;
     }
-    const uint64_t tiles = (uint64_t)((a.n + kTcRowsW - 1) / kTcRowsW) * ((a.m + best - 1) / best);
-    const bool halves = plan.shared && plan.ctas == 2 * tiles;
-    const uint32_t has = chain_mean(nraw, halves ? 2 : 1, best > 128 ? 1 : 2, tiles, plan.shared && !halves ? plan.ctas - 1 : 0);
+}
+static uint32_t tc_chain_limit(const QmmArgs &a, const TcChoice &c) {
+    const uint32_t nraw = (a.k + 255) / 256, nt = c.rows[c.best];
+    const uint64_t tiles = (uint64_t)((a.n + kTcRowsW - 1) / kTcRowsW) * ((a.m + nt - 1) / nt);
+    const bool halves = c.plan.shared && c.plan.ctas == 2 * tiles;
+    const uint32_t has = chain_mean(nraw, halves ? 2 : 1, nt > 128 ? 1 : 2, tiles, c.plan.shared && !halves ? c.plan.ctas - 1 : 0);
     const uint32_t least = a.k <= 512 ? kChainAny : (uint32_t)(4096ull * 512 * 512 / ((uint64_t)a.k * a.k));
     return has > least ? has : least;
 }
+uint32_t qmm_chain_limit(const QmmArgs &a, int sm_count) {
+    TcChoice c;
+    tc_choose(a, sm_count, false, c);
+    return tc_chain_limit(a, c);
+}
 
-// The tile, of either kernel, with which a dense call takes least.
-uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool sharded) {
+// The tile, of either kernel, with which a dense call takes least.  `limit`: what launch_qmm_tc is to be given with it.
+uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool sharded, uint32_t *limit) {
+    TcChoice c;
+    tc_choose(a, sm_count, sharded, c);
+    *limit = tc_chain_limit(a, c);
+    if (!qmm_duo_takes(ggml_type, a)) return c.rows[c.best];
     uint32_t best = 256;
     uint64_t best_cost = ~0ull;
-    const uint32_t limit = qmm_chain_limit(a, sm_count);
-    for (uint32_t tt = (a.m + 255) / 256, last = tt + 8; tt <= last; tt++) {
-        const uint32_t rows = ((a.m + tt - 1) / tt + 15) / 16 * 16;
+    for (uint32_t i = 0; i < c.count; i++)
         for (int duo = 0; duo < 2; duo++) {
-            TcPlan p;
-            const uint32_t nt = duo ? (rows + 31) / 32 * 32 : rows;
-            const uint64_t cost = duo ? qmm_duo_cost(ggml_type, a, nt, limit) : tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count, sharded, p);
-            if (cost != ~0ull && (best_cost == ~0ull || cost * 103 / 100 < best_cost)) {   // (near a tie, the larger tile: it converts less in all)
+            const uint32_t nt = duo ? (c.rows[i] + 31) / 32 * 32 : c.rows[i];
+            const uint64_t cost = duo ? qmm_duo_cost(ggml_type, a, nt, *limit) : c.cost[i];
+            if (best_cost == ~0ull || cost * 103 / 100 < best_cost) {
                 best_cost = cost;
                 best = nt;
             }
         }
-        if (rows == 16) break;
-    }
     return best;
 }
 
@@ -1244,11 +1256,10 @@ template <int T> static cudaError_t launch_tc_t(const QmmArgs &a, bool routed, u
 
 // tcgen05 mat-mat.  `scratch` must hold qmm_tc_scratch_bytes(a, nt, routed) bytes and start on a 256-byte boundary (the packed
 // tiles in it are sources of bulk copies: 16-byte alignment is what the hardware needs; their offsets are multiples of 1024).
-cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t nt, uint8_t *scratch, cudaStream_t st,
+cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t nt, uint32_t limit, uint8_t *scratch, cudaStream_t st,
                           int *launches) {
     if (!routed) {
         TcPlan plan;
-        const uint32_t limit = qmm_chain_limit(a, sm_count_of_device());
         if (qmm_duo_cost(ggml_type, a, nt, limit) < tc_plan(nt, a.m, a.n, a.k, (uint64_t)sm_count_of_device(), a.y_ld != 0 || a.n_peer != 0, plan))
             return launch_qmm_duo(ggml_type, &a, 1, nt, limit, scratch, st, launches);
     }
@@ -1379,7 +1390,7 @@ extern "C" int mlxn_quantized_matmul_ggml_mm_noalloc(void *cuda_stream, const vo
     a.n_experts = 1;
     a.total_rows = params->m;
     a.status = nullptr;  // no status word: a wait that gives up still ends the kernel, but is not reported
-    uint32_t nt = qmm_tc_pick_nt(t, a, sms, false);
+    uint32_t limit = 0, nt = qmm_tc_pick_nt(t, a, sms, false, &limit);
     size_t need = qmm_tc_scratch_bytes(a, nt, false);
     // (the fastest tile may pad the rows more than another one that still fits; tiles of 16 rows pad least)
     for (uint32_t other = 256; other >= 16 && need > MLXN_NOALLOC_SCRATCH_BYTES; other -= 16) need = qmm_tc_scratch_bytes(a, nt = other, false);
@@ -1392,7 +1403,7 @@ extern "C" int mlxn_quantized_matmul_ggml_mm_noalloc(void *cuda_stream, const vo
         return mlxn_detail_fail(MLXN_INVALID_ARGUMENT, msg);
     }
     int launches = 0;
-    cudaError_t e = launch_qmm_tc(t, a, false, nt, scratch, static_cast<cudaStream_t>(cuda_stream), &launches);
+    cudaError_t e = launch_qmm_tc(t, a, false, nt, limit, scratch, static_cast<cudaStream_t>(cuda_stream), &launches);
     if (e != cudaSuccess) {
         cudaGetLastError();
         char msg[256];

@@ -47,7 +47,7 @@ bool qmv_wide_supported(int ggml_type, const QmvArgs &a);
 bool qmv_wide_pays(const QmvArgs &a);
 size_t qmv_wide_scratch_bytes(const QmvArgs *ops, int nops);
 cudaError_t launch_qmv_wide(const QmvArgs *ops, int nops, int sm_count, uint8_t *scratch, int *launches, cudaStream_t st);
-cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t nt, uint8_t *scratch, cudaStream_t st,
+cudaError_t launch_qmm_tc(int ggml_type, const QmmArgs &a, bool routed, uint32_t nt, uint32_t limit, uint8_t *scratch, cudaStream_t st,
                           int *launches);
 cudaError_t launch_qmm_simt(int ggml_type, const QmmArgs &a, bool routed, uint32_t max_rows, cudaStream_t st);
 size_t qmm_tc_scratch_bytes(const QmmArgs &a, uint32_t nt, bool routed);
@@ -55,7 +55,7 @@ constexpr size_t kMmBatchMax = 4;          // mat-mats one launch carries (kMmOp
 bool qmm_duo_takes(int ggml_type, const QmmArgs &a);
 uint32_t qmm_duo_pick_nt(int ggml_type, const QmmArgs *ops, int nops, int sm_count, uint32_t *limit);
 cudaError_t launch_qmm_duo(int ggml_type, const QmmArgs *ops, int nops, uint32_t nt, uint32_t limit, uint8_t *xpack, cudaStream_t st, int *launches);
-uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool sharded);
+uint32_t qmm_tc_pick_nt(int ggml_type, const QmmArgs &a, int sm_count, bool sharded, uint32_t *limit);
 bool qmm_tc_supported(const QmmArgs &a);
 constexpr uint32_t kRoutedTileRows = 64;   // activation rows of a tile of the grouped mat-mat
 cudaError_t launch_moe_map0(const uint32_t *ids, uint32_t n_tokens, uint32_t top_k, uint32_t n_experts,
@@ -1023,9 +1023,9 @@ static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
             CUDA_TRY(launch_qmm_duo(e->pend_type, ops.data(), n, nt, limit, scratch, st, &launches), "mat-mat launch");
         } else {
             for (const QmmArgs &a : ops) {
-                const uint32_t own = qmm_tc_pick_nt(e->pend_type, a, sms, false);
+                const uint32_t own = qmm_tc_pick_nt(e->pend_type, a, sms, false, &limit);
                 if ((rc = encoder_scratch_on(e, e->pend_lane, qmm_tc_scratch_bytes(a, own, false), &scratch))) return rc;
-                CUDA_TRY(launch_qmm_tc(e->pend_type, a, false, own, scratch, st, &launches), "mat-mat launch");
+                CUDA_TRY(launch_qmm_tc(e->pend_type, a, false, own, limit, scratch, st, &launches), "mat-mat launch");
             }
         }
         g_launches.fetch_add((uint64_t)launches);
@@ -1896,11 +1896,12 @@ static int dispatch_mm(mlxn_encoder *enc, mlxn_registry *reg, mlxn_device *dev, 
     }
     if ((rc = op_begin(enc, {{input, false}, {weight, false}, {output, true}}))) return rc;
     if (tc && qmm_tc_supported(a)) {
-        const uint32_t nt = qmm_tc_pick_nt((int)p->ggml_type, a, dev->sm_count, sh != nullptr);
+        uint32_t limit = 0;
+        const uint32_t nt = qmm_tc_pick_nt((int)p->ggml_type, a, dev->sm_count, sh != nullptr, &limit);
         uint8_t *scratch = nullptr;
         if ((rc = encoder_scratch(enc, qmm_tc_scratch_bytes(a, nt, false), &scratch))) return rc;
         int launches = 0;
-        CUDA_TRY(launch_qmm_tc((int)p->ggml_type, a, false, nt, scratch, enc->stream, &launches), "mat-mat launch");
+        CUDA_TRY(launch_qmm_tc((int)p->ggml_type, a, false, nt, limit, scratch, enc->stream, &launches), "mat-mat launch");
         g_launches.fetch_add(launches);
         g_last_kernel = "qmm_tc";
     } else {
@@ -2044,11 +2045,12 @@ extern "C" int mlxn_quantized_matmul_mm_tensor_perm021(mlxn_encoder *enc, mlxn_r
     a.n_experts = 1;
     a.total_rows = p->m;
     a.status = enc->status_word;
-    const uint32_t nt = qmm_tc_pick_nt(t, a, dev->sm_count, false);
+    uint32_t limit = 0;
+    const uint32_t nt = qmm_tc_pick_nt(t, a, dev->sm_count, false, &limit);
     uint8_t *scratch = nullptr;
     if ((rc = encoder_scratch(enc, qmm_tc_scratch_bytes(a, nt, false), &scratch))) return rc;
     int launches = 0;
-    CUDA_TRY(launch_qmm_tc(t, a, false, nt, scratch, enc->stream, &launches), "mat-mat launch");
+    CUDA_TRY(launch_qmm_tc(t, a, false, nt, limit, scratch, enc->stream, &launches), "mat-mat launch");
     g_launches.fetch_add(launches);
     g_last_kernel = "qmm_tc";
     g_dispatch.fetch_add(1);
@@ -2221,7 +2223,7 @@ static int dispatch_id_mm_stages(mlxn_encoder *enc, mlxn_registry *reg, mlxn_dev
         const size_t need = qmm_tc_scratch_bytes(a, nt, true);
         if ((rc = encoder_scratch(enc, scratch_used + need, &scratch))) return rc;
         int launches = 0;
-        CUDA_TRY(launch_qmm_tc((int)p->ggml_type, a, true, nt, scratch + scratch_used, enc->stream, &launches), "mat-mat launch");
+        CUDA_TRY(launch_qmm_tc((int)p->ggml_type, a, true, nt, 0, scratch + scratch_used, enc->stream, &launches), "mat-mat launch");
         g_launches.fetch_add(launches);
         g_last_kernel = "qmm_tc_id";
     } else {
@@ -2401,7 +2403,7 @@ extern "C" int mlxn_moe_ffn_layer(mlxn_encoder *enc, mlxn_registry *reg, mlxn_de
         a.status = enc->status_word;
         a.reuse = reuse;
         int launches = 0;
-        CUDA_TRY(launch_qmm_tc((int)q.ggml_type, a, true, nt, tc, enc->stream, &launches), "mat-mat launch");
+        CUDA_TRY(launch_qmm_tc((int)q.ggml_type, a, true, nt, 0, tc, enc->stream, &launches), "mat-mat launch");
         g_launches.fetch_add(launches);
         g_dispatch.fetch_add(1);
         return MLXN_OK;
