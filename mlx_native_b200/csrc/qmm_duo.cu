@@ -6,9 +6,9 @@
 // (tcgen05 cta_group::2): each dequantises its own 128 rows into its own tensor memory and holds half of the activation tile, which the
 // hardware reads from both.  Operand semantics as in qmm.cu: exact weights rounded once to f16, activations f32 -> f16, f32 sums.
 //
-// Graph replay of dependent calls, packing included, us with qmm.cu / here (K 4096 unless said): 4096 weight rows: 9 rows 18.9 / 14.4, 64 20.9 / 15.5,
-// 256 24.3 / 19.0, 512 31.1 / 25.0; 12288 x 512 rows 66.7 / 46.4; 1024 x 512 22.4 / 16.8; 4096 x 12288, 2048 rows: Q4_0 205 / 169, Q6_K 229 / 181;
-// 256 x 512 x 16 rows 8.6 / 8.2.  So it takes every call it can: what has no 16-byte aligned weights, or a row count that its copies cannot group,
+// Graph replay of dependent calls, packing included, us with qmm.cu / here (K 4096 unless said): 4096 weight rows: 9 rows 18.9 / 15.5, 64 20.9 / 17.8,
+// 256 24.3 / 20.8, 512 31.1 / 26.8; 12288 x 512 rows 66.7 / 49.0; 1024 x 512 22.4 / 18.8; 4096 x 12288, 2048 rows: Q4_0 205 / 178, Q6_K 229 / 190;
+// 256 x 512 x 16 rows 8.6 / 8.0.  So it takes every call it can: what has no 16-byte aligned weights, or a row count that its copies cannot group,
 // stays with the other kernel, and the row-sharded form.  What bounds it: up to 192 rows the chain raw block -> tensor memory (0.47 us for a
 // K stage of 128, 18 values a cycle and SM; Q6_K 0.66 before its 64 values of a thread were unpacked together: 64 rows 21.0 -> 19.9
 // us), above that the multiplication (0.43 us at full clock) beside it.
@@ -16,8 +16,8 @@
 // The items of grouped calls are short (64 rows, K of 6 to 16 stages), and while the dequantising warps read an accumulator back both they and the
 // tensor core would stand still; there the read-back has warps of its own and two accumulators.  (Dense calls gain nothing from it, Q4_0 2048 x 4096 x
 // 4096 61.4 / 62.4 us, and Q6_K loses, 128 x 4096 x 4096 19.8 / 22.2.)  Layer of 512 tokens, 8 of 128 experts each, Q4_0 768 x 2048 twice and Q6_K
-// 2048 x 768: 273 us for the whole pass with two CTAs of qmm.cu's kernel on an SM (half of the dequantising warps each), 226 here; weights once at the
-// copy rate 61.  Batches: q, k and v of 512 rows (4096, 1024 and 1024 x 4096) and gate and up (12288 x 4096 each) in one launch take a layer from 274
+// 2048 x 768: 273 us for the whole pass with two CTAs of qmm.cu's kernel on an SM (half of the dequantising warps each), 228 here; weights once at the
+// copy rate 61.  Batches: q, k and v of 512 rows (4096, 1024 and 1024 x 4096) and gate and up (12288 x 4096 each) in one launch took a layer from 274
 // to 244 us: one packing instead of three and two, and one last wave.
 //
 // Sums: chains of additions in an accumulator are kept about as short as on single SMs (qmm.cuh): dense tiles have two accumulators up to 192 rows and
@@ -26,6 +26,9 @@
 // products have alone (k and v of 512 rows 2.4e-6, 1.2e-6).  It costs 0.6 us a call: 512 x 4096 x 4096 25.8 / 26.6, 64 rows 17.1 / 17.9.  Also tried: a
 // tile in parts that are added to y, 3.5 us each at 192 rows (q, k and v 28.3 / 32.4); tiles whose read-back waits for the next one's first
 // stages, no gain (64 rows 18.7).
+//
+// Order: the activations' copies of both CTAs complete on CTA 0's barrier.  With bulk copies onto barriers of their own and a relaxed arrival in between,
+// which orders nothing in shared memory, 2048 rows took 1.5 % less (Q6_K 187 / 190), others the same.
 //
 // What else was tried: unpacking the weights once into f16 tiles, by a kernel of its own.  The product alone then runs at the
 // multiplication's rate, but the unpacking is bound by memory (13 us for 4096 x 4096, 58 with 2048 rows of 12288 for 4096 x 12288): 32.2 us in

@@ -14,7 +14,7 @@
 //
 // Graph replay of dependent calls, packing included, us before / now: 9 rows of 4096 x 4096 26 / 14, 32 43 / 19, 96 111 / 37, 512 547 / 152,
 // 2048 2166 / 571; 16 rows of 12288 x 4096 57 / 32, 100 of 256 x 4096 17 / 11.  What bounds it: mma.sync (2 cycles on an SM per 16 x 8 x 16) is
-// busy for half of the time, instruction issue too; the rest is waiting of one on the other.  Relative error against 64 bits (K 1024 ..
+// busy for 40 % of the time, instruction issue for 44 % (96 rows); the rest is waiting of one on the other.  Relative error against 64 bits (K 1024 ..
 // 14336) 0.9..1.1e-7, the other kernel's 0.9..1.2e-7; with hi and lo summed by one chain of multiplies it was 1.0..1.2e-7 (35 us).
 #include "qmv_split.cuh"
 
