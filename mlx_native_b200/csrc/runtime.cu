@@ -6,7 +6,6 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
-#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -165,6 +164,10 @@ struct Storage {
     std::vector<Deferred> deferred;
     std::atomic<size_t> n_deferred{0};   // deferred.size(), to look at without the lock
     std::mutex mu;
+    Storage() {   // (room for one encoder's lanes, so that a first operation allocates nothing)
+        users.reserve(4);
+        deferred.reserve(2);
+    }
 };
 // (with the storage's lock held)
 static void storage_used_on(Storage *s, cudaStream_t st) {
@@ -311,6 +314,7 @@ struct mlxn_encoder {
     bool started = false, committed = false, capturing = false;
     uint64_t cap_launch0 = 0, cap_dispatch0 = 0;
     std::vector<mlxn_buffer *> retained;
+    size_t retained_committed = 0;   // ... by what the last commit ended
     uint8_t *scratch_lane[kLanes] = {};
     size_t scratch_lane_bytes[kLanes] = {};
     std::vector<std::pair<void *, size_t>> retired;  // outgrown scratch arenas, handed back after the next wait
@@ -589,8 +593,8 @@ static int storage_settle(Storage *s, const mlxn_encoder *self, bool writes) {
 }
 // wait for whatever uses the storage (device work or an upload still reading the shadow); called with its lock held
 static int storage_quiesce(Storage *s) {
-    while (!s->deferred.empty()) {   // products that use it wait to be launched
-        s->mu.unlock();              // (the flush takes encoders' and storages' locks itself)
+    if (!s->deferred.empty()) {   // products that use it wait to be launched
+        s->mu.unlock();           // (the flush takes encoders' and storages' locks itself)
         const int rc = storage_settle(s, nullptr, true);
         s->mu.lock();
         if (rc) return rc;
@@ -884,17 +888,32 @@ extern "C" int mlxn_encoder_create(mlxn_device *dev, mlxn_encoder **out) {
     return MLXN_OK;
 }
 
-static void encoder_release_retained(mlxn_encoder *e) {
-    // called once the lanes are idle: nobody has to wait for them on account of these storages
-    for (mlxn_buffer *b : e->retained) {
+// The first `count` of the retained buffers belong to work that has completed.  What has been encoded since, and may still be waiting to be
+// launched, keeps its buffers, the lanes in its storages, and outgrown scratch.
+static void encoder_release_retained(mlxn_encoder *e, size_t count) {
+    for (size_t i = 0; i < count; i++) {
+        mlxn_buffer *b = e->retained[i];
         {
             std::lock_guard<std::mutex> lk(b->st->mu);
             auto &u = b->st->users;
-            for (int l = 0; l < kLanes; l++) u.erase(std::remove(u.begin(), u.end(), e->lanes[l]), u.end());
+            size_t kept = 0;
+            for (cudaStream_t st : u) {
+                bool mine = false;
+                for (int l = 0; l < kLanes; l++) mine = mine || st == e->lanes[l];
+                if (!mine) u[kept++] = st;
+            }
+            u.resize(kept);
         }
         mlxn_buffer_release(b);
     }
-    e->retained.clear();
+    if (count == e->retained.size()) e->retained.clear();
+    else e->retained.erase(e->retained.begin(), e->retained.begin() + count);
+    e->retained_committed = 0;
+    for (mlxn_buffer *b : e->retained) {
+        std::lock_guard<std::mutex> lk(b->st->mu);
+        for (int l = 0; l < kLanes; l++) storage_used_on(b->st, e->lanes[l]);
+    }
+    if (!e->retained.empty()) return;
     for (auto &pr : e->retired) scratch_give(e->ordinal, pr.first, pr.second);
     e->retired.clear();
 }
@@ -912,7 +931,7 @@ extern "C" void mlxn_encoder_destroy(mlxn_encoder *enc) {
         cudaError_t e1 = cudaStreamSynchronize(enc->lanes[l]);
         if (e1 != cudaSuccess) serr = e1;
     }
-    encoder_release_retained(enc);
+    encoder_release_retained(enc, enc->retained.size());
     if (serr == cudaSuccess && !enc->capturing) {
         // clean and idle: keep it for the next mlxn_encoder_create on this device
         enc->started = enc->committed = false;
@@ -1167,6 +1186,7 @@ static int encoder_commit(mlxn_encoder *enc, bool timed) {
     enc->ev_last = timed ? enc->ev_end : enc->ev_done;
     CUDA_TRY(cudaEventRecord(enc->ev_last, enc->lanes[0]), "event record");
     enc->committed = true;
+    enc->retained_committed = enc->retained.size();
     return MLXN_OK;
 }
 extern "C" int mlxn_encoder_commit(mlxn_encoder *enc) { return encoder_commit(enc, false); }
@@ -1200,7 +1220,7 @@ extern "C" int mlxn_encoder_wait_until_completed(mlxn_encoder *enc) {
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     EncoderLock lk(enc->mu);
-    encoder_release_retained(enc);
+    encoder_release_retained(enc, enc->committed ? enc->retained_committed : enc->retained.size());
     enc->started = false;
     if (e != cudaSuccess) return cuda_fail(e, "GPU execution");
     if (enc->committed && *enc->status_host != 0) {

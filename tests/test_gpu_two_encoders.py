@@ -122,6 +122,33 @@ def test_chain_over_two_encoders_in_turn(ctx):
         p.check(got[i + 1], x=got[i])
 
 
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("how", ["host", "encoder", "commit", "dropped"])
+def test_product_encoded_between_commit_and_wait(ctx, kind, how):
+    """The wait is for what was committed: a product that has been encoded since keeps its buffers and its place."""
+    p, q = Product(ctx, kind), Product(ctx, kind, seed=60)
+    d = ctx.device
+    enc, other = d.command_encoder(), d.command_encoder()
+    p.encode(enc)
+    enc.commit()
+    q.encode(enc)
+    if how == "dropped":   # nobody but the encoder holds the operand's and the weights' buffers any more
+        q.xb = q.w = None
+    enc.wait_until_completed()
+    p.check(p.yb.as_slice(np.float32))
+    if how == "host":
+        q.xb.as_mut_slice(np.float32)[:] = 0
+    elif how == "encoder":
+        mx.silu_mul(other, ctx.registry, d, p.yb, p.yb, q.xb, q.m * K)
+        other.commit_and_wait()
+    elif how == "dropped":
+        fill = [d.alloc_buffer(q.m * K * 4, mx.DType.F32) for _ in range(4)] + [d.alloc_buffer(q.wq.size + 64, mx.DType.U8) for _ in range(4)]
+        for b in fill:
+            b.as_mut_slice(np.uint8)[:] = 255
+    enc.commit_and_wait()
+    q.check(q.yb.as_slice(np.float32))
+
+
 def test_threads_with_an_encoder_each(ctx):
     """Two threads share weights; a third one looks at results and at an operand while the others encode."""
     d = ctx.device
