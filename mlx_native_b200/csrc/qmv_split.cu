@@ -18,7 +18,7 @@ bool qmv_split_aligned(int ggml_type, const QmvArgs &a) {
 }
 
 static SpPick split_pick(int ggml_type, bool aligned, uint32_t mp, bool routed, uint64_t tiles, uint32_t units, int sm_count) {
-    const bool packed = !routed && mp > 1;
+    const bool packed = !routed && mp > 2;
     switch (ggml_type) {
     case GT_Q4_0: return sp_pick<GT_Q4_0>(aligned, mp, packed, routed, tiles, units, sm_count);
     case GT_Q8_0: return sp_pick<GT_Q8_0>(aligned, mp, packed, routed, tiles, units, sm_count);
@@ -68,6 +68,10 @@ bool qmv_split_supported(int ggml_type, const QmvArgs &a, int sm_count) {
 // starts 1 to 3 us later and has the higher rate, and its time grows evenly, where the other one's is a number of passes over the chip:
 // what decides is how full those passes are (`fill`, qmv_mma_fill) and how much there is to read.  Graph replay of dependent
 // launches, us with the register-level kernel (one mat-vec of three or four rows: the tensor-memory kernel) / with this one:
+//   (one and two rows: with f16; in integers, as they leave now, the right-hand figures of one row are, 6144 rows 7.6, 8.9, 10.6, 8.5; 8192 rows (0.86) 8.6, 9.2,
+//   13.3, 9.9 against 8.6, 10.1, 11.7, 9.2 with the register-level kernel; 12288 10.1, 13.2, 15.0, 11.3; 24576 16.4, 24.3, 25.6, 19.3; 4096 x 12288 11.5, 15.7, 15.5, 12.8; of
+//   two rows, 12288 18.0, 17.1, 19.7, 15.1; 24576 21.0, 29.0, 33.8, 26.4.  Three products or more of one row (q, k and v, 25 M values) start
+//   2 us later with this kernel, whose CTAs cross from one to the next.)
 //   one row    4096 values wide   6144 rows (fill 0.65)   10240 (0.54)   12288 (0.65)   14336 (0.76)   16384 (0.86)   24576 (0.65)
 //     Q4_0                        7.6 / 8.6               12.4 / 11.5    12.7 / 11.7    12.7 / 13.1    13.3 / 13.4    23.9 / 19.5
 //     Q8_0                        8.5 / 8.4               14.2 / 11.1    13.7 / 11.9    13.7 / 14.3    14.7 / 14.9    25.1 / 20.6
@@ -100,7 +104,10 @@ bool qmv_split_pays(int ggml_type, const QmvArgs *ops, int nops, double fill) {
     constexpr uint64_t M = 1u << 20;
     const bool q4k = ggml_type == GT_Q4_K;
     if (kmin != kmax) return false;   // (the other kernel deals out work by K stages, and its passes are fuller than `fill` says)
-    if (m <= 2) return fill <= (ggml_type == GT_Q6_K && kmax >= 10240 ? 0.9 : 0.7) && values >= (q4k || (ggml_type == GT_Q4_0 && m == 2) ? 72 * M : 32 * M);
+    if (q4k && m <= 2) return fill <= 0.7 && values >= 72 * M;
+    if (m <= 1 && nops > 2) return values >= 40 * M;
+    if (m <= 1) return values >= (fill > 0.7 ? (ggml_type == GT_Q8_0 ? 60 * M : 40 * M) : ggml_type == GT_Q8_0 ? 30 * M : 24 * M);
+    if (m <= 2) return values >= (ggml_type == GT_Q6_K ? 46 * M : 60 * M);
     if (q4k && m <= 4) return kmax >= 4096 && values >= 14 * M && (fill <= 0.6 || (fill <= 0.7 && values >= 72 * M));
     if (q4k) return fill <= 0.6 && (m <= 8 || fill <= 0.25 || (m + 7) / 8 * 16 <= 3 * m);
     if (m > 4) return false;
@@ -135,7 +142,7 @@ bool qmv_split_pays_routed(int ggml_type, const QmvArgs &a, bool mma) {
 size_t qmv_split_scratch_bytes(const QmvArgs *ops, int nops) {
     size_t n = 0;
     for (int i = 0; i < nops; i++)
-        if (!ops[i].ids && ops[i].m > 1) n += sp_pack_bytes<GT_Q4_K>(ops[i].m, ops[i].k);   // (a type with sums)
+        if (!ops[i].ids && ops[i].m > 2) n += sp_pack_bytes<GT_Q4_K>(ops[i].m, ops[i].k);   // (a type with sums)
     return n;
 }
 

@@ -3,18 +3,23 @@
 // HBM bounds the operation (6.4 TB/s measured copy rate: 23 bytes per cycle and SM); what a kernel loses against that is latency
 // (launch, activations, waits between stages) and instructions (integer operations issue at half rate).  Hence:
 //
-//  * The activations of a CTA stay in shared memory for all its weight rows: f16 hi + lo halves (scaled by a power of two per
-//    row, so that both stay in range), in the order of the B registers of mma.sync.m16n8k16.  One row is split by every CTA
-//    itself, several rows by qmv_pack_kernel, and arrive by bulk copies (4096 x 4096 Q4_0: 7.2 us with one row, 8.8 with two).  The loop over the
-//    weights only unpacks codes into signed integers, as normal f16 numbers, so products are exact and sums are f32.
-//  * The 8 columns of an MMA are (activation row, hi | lo): one multiply serves up to four rows (NS = 2 sets: eight rows).
+//  * The activations of a CTA stay in shared memory for all its weight rows, in the order of the B registers of mma.sync.  One or two
+//    rows (dense) as four signed 8-bit digits, for multiplies of 8-bit integers (sp_unit_int); more, and routed ones, as f16 hi + lo halves,
+//    scaled by a power of two per row so that both stay in range, for mma.sync.m16n8k16.  One and two rows are split by every CTA
+//    itself, several by qmv_pack_kernel, and arrive by bulk copies.  The loop over the weights only unpacks codes into signed integers, bytes or
+//    normal f16 numbers, so products are exact and sums are f32.
+//  * In f16 the 8 columns of an MMA are (activation row, hi | lo): one multiply serves up to four rows (NS = 2 sets: eight rows).
+//  * Integers against f16, one row, us a call of a dependent chain (graph replay): Q4_0 24576 x 4096 21.5 -> 16.4, 4096 x 12288 13.2 -> 11.5, Q4_K 25.9 ->
+//    19.3, 15.2 -> 12.8, Q6_K 30.3 -> 25.6, 17.2 -> 15.5, Q8_0 25.5 -> 24.3 (its codes took least); 151936 x 4096 Q4_0 97 -> 69, Q6_K 151936 x 5120 172 (the
+//    register-level kernel) -> 147.  What is left there is unpacking at 60 cycles a tile and unit and scheduler (Q4_0; its bytes take 100 at the
+//    copy rate), and at the start and between chunks latency: 1.5 us for the activations, 0.7 us a chunk.
 //  * A warp works on up to four 16-row tiles at a time: one tile at a time leaves the pipes idle between dependent steps (Q4_0,
 //    75776 x 4096: 70.7 us, 2.5 TB/s, against 44.9, 3.9 TB/s).
 //  * K may be split over the CTAs of a cluster (1, 2, 4, 8): a matrix of few rows still fills the chip, and long activation rows
 //    still fit into shared memory.  The ranks' partial sums travel through distributed shared memory (st.async) and are added in
 //    rank order by the CTA that owns the row: no atomics, results are bit-reproducible.
 //  * A producer warp fills a ring of stages (16-row tiles x SU units of 64 K values) by TMA: tensor copies where every weight row
-//    starts on a 16-byte boundary (ALN), else one bulk copy per row of the 16-byte superset of its segment, so a K that is no
+//    starts on a 16-byte boundary (ALN) or every other one does, else one bulk copy per row of the 16-byte superset of its segment, so a K that is no
 //    multiple of 256 and a weight address that is even do for Q4_0, Q8_0 and Q6_K (Q8_0 2873 x 2880, five rows: 11.7 us where the
 //    kernel that reads blocks from global memory took 181).  Q4_K and Q5_K have to start on 16-byte boundaries.
 //  * Expert-routed: every CTA sorts the (token, slot) pairs by expert itself (at most 256 pairs), and the rows of one expert share
@@ -40,7 +45,9 @@ namespace mlxn {
 constexpr int kSpWarps = 8;                         // consumer warps
 constexpr int kSpThreads = (kSpWarps + 1) * 32;     // and one producer warp
 constexpr int kSpTiles = 4;                         // 16-row tiles of a chunk, at most
-__host__ __device__ constexpr int sp_tiles(int sets) { return sets == 2 ? 2 : kSpTiles; }
+__host__ __device__ constexpr int sp_tiles(int mp) { return mp > 4 ? 2 : kSpTiles; }
+// sets of eight columns that mp activation rows take (one and two rows: sp_unit_int)
+__host__ __device__ constexpr int sp_sets(int mp) { return mp > 4 || mp == 2 ? 2 : 1; }
 constexpr int kSpMaxOps = 8;                        // mat-vecs one launch carries
 constexpr int kSpMaxSlots = 8;
 constexpr int kSpMaxPairs = 256;                    // (token, slot) pairs of a routed launch
@@ -66,7 +73,7 @@ struct SpOp {
     const float *x2;          // fused SwiGLU: the activations are silu(x) * x2
     float *y;
     uint32_t n, k, m;
-    uint32_t chunk_end;       // chunks (of tr tiles) of the ops up to and including this one
+    uint32_t step_end;        // steps (of `step` 16-row tiles) of the ops up to and including this one
     uint32_t row_bytes;
     uint32_t units;           // ceil(k / 64)
     uint32_t slice;           // units per cluster rank (a multiple of 4)
@@ -90,14 +97,14 @@ struct SpBatch {
     uint32_t nops, npairs, n_experts;
     uint32_t nent;            // dense: groups of mp activation rows; routed: counted on the device
     uint32_t mp;              // activation rows of an entry (1, 2, 4 or 8)
-    uint32_t tr;              // tiles of a chunk
-    uint32_t run;             // consecutive chunks a cluster takes at a time (0: a contiguous share)
+    uint32_t tr, step;        // tiles of a chunk, at most, and of a step of the clusters' shares
     uint32_t early_weights;
     uint32_t *status;
     uint32_t nslots;          // ring depth, and what lies behind the ring in shared memory
     uint32_t xf_off, cc_off, tab_off, red_off, recv_off;
     uint32_t xstride, cstride;   // bytes from one activation row to the next
     uint32_t packed;          // the activations have been packed by qmv_pack_kernel
+    uint32_t pairs;           // every other row starts on a 16-byte boundary: the rows arrive by tensor copies all the same
 };
 struct SpMaps {
     CUtensorMap m[kSpMaxOps];
@@ -145,6 +152,52 @@ __device__ __forceinline__ void split(float a, float b, uint32_t &hi, uint32_t &
     const __half2 l = __floats2half2_rn(fabsf(w.x) < INFINITY ? a - w.x : 0.f, fabsf(w.y) < INFINITY ? b - w.y : 0.f);
     hi = *reinterpret_cast<const uint32_t *>(&h);
     lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+// Two powers of two whose product brings amax (its bits; a number) into [2^13, 2^14), and those of the way back from units of the last digit.
+// (One factor would not be a normal number where amax is tiny.)  NaN for the way back where the run holds an infinity or a NaN.
+__device__ __forceinline__ void pow2_int(uint32_t amax, float &s0, float &s1, float &inv0, float &inv1) {
+    const int e = 13 + 127 - (int)(amax >> 23), a = e >> 1, b = e - a;
+    s0 = __uint_as_float((uint32_t)(127 + a) << 23);
+    s1 = __uint_as_float((uint32_t)(127 + b) << 23);
+    inv0 = amax >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : __uint_as_float((uint32_t)(127 - 15 - a) << 23);
+    inv1 = __uint_as_float((uint32_t)(127 - b) << 23);
+}
+// Four numbers below 2^14 as four signed digits each, in units of 2^-15: l[0] + 256 l[1] + 2^15 (l[2] + 256 l[3]); l[i] holds digit i of all
+// four, a byte each.  (Adding 1.5 * 2^23 leaves the nearest integer in the low bits, here with 128 more, so that the low byte is a signed digit
+// once its top bit has changed; a conversion instruction issues at an eighth of the rate.)
+constexpr float kDigitWeight = 32768.f;   // of digits 2 and 3 against 0 and 1
+__device__ __forceinline__ void digits(const float (&c)[4], uint32_t (&l)[4]) {
+    constexpr float M = 12582912.f + 128.f;
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float t = __fadd_rn(c[i], M);
+        hi[i] = __float_as_uint(t);
+        lo[i] = __float_as_uint(__fmaf_rn(__fsub_rn(c[i], __fsub_rn(t, M)), kDigitWeight, M));
+    }
+    const uint32_t a = __byte_perm(lo[0], lo[1], 0x5140), b = __byte_perm(lo[2], lo[3], 0x5140);
+    const uint32_t e = __byte_perm(hi[0], hi[1], 0x5140), d = __byte_perm(hi[2], hi[3], 0x5140);
+    l[0] = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
+    l[1] = __byte_perm(a, b, 0x7632);
+    l[2] = __byte_perm(e, d, 0x5410) ^ 0x80808080u;
+    l[3] = __byte_perm(e, d, 0x7632);
+}
+// D = A (16 x 32, row) * B (32 x 8, col) + C in 8-bit integers.  Lane (g, t): a0 = A[g][4t .. 4t+3], a1 = A[g+8][..], a2 = A[g][16+4t ..],
+// a3 = A[g+8][16+4t ..]; b0 = B[4t .. 4t+3][g], b1 = B[16+4t ..][g]; c and d as mma16816.
+__device__ __forceinline__ void mma_s8(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, const uint32_t (&c)[4]) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
+}
+// Integers to f32 without a conversion: with C = kBias the bits of D are those of 1.5 * 2^23 + the sum, while that is below 2^22.
+constexpr uint32_t kBias = 0x4B400000u;
+// acc += (d0 or d1) * the sums: rows g and g + 8, two columns at a time
+__device__ __forceinline__ void scaled(float (&acc)[4], const uint32_t (&d)[4], float d0, float d1) {
+    const uint64_t off = pack2(-12582912.f, -12582912.f);
+    uint64_t lo = ffma2(pack2(d0, d0), fadd2(pack2u(d[0], d[1]), off), pack2(acc[0], acc[1]));
+    uint64_t hi = ffma2(pack2(d1, d1), fadd2(pack2u(d[2], d[3]), off), pack2(acc[2], acc[3]));
+    unpack2(lo, acc[0], acc[1]);
+    unpack2(hi, acc[2], acc[3]);
 }
 // Codes to signed integers.  A code n in the low bits of a half with exponent field 0x64 reads 1024 + n, one four bits further up
 // 1024 + 16 n; the bias goes off exactly.  (Codes that stay subnormals, n 2^-24, save this operation, but the tensor core aligns
@@ -196,7 +249,7 @@ template <int T, bool ALN> __device__ __forceinline__ void sp_pairs(uint32_t u, 
 // One unit (64 K values) of a stage against NT tiles.  a0 / a1: shared address of rows g and g + 8 of tile 0 at the unit's
 // first byte (Q4_K, Q5_K, Q6_K: of its super-block), lead-in included; tiles are 16 PITCH bytes apart.  bf: the B registers
 // [set][MMA][2]; cc: per set and sub-block the sum of the activations (Q4_K, Q5_K); tab: the warp's scale table.
-template <int T, bool ALN, int NT, int NS, bool ONE, int TM>
+template <int T, bool ALN, int NT, int NS, int TM>
 __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, uint32_t t, uint32_t g, uint32_t tab, bool half,
                                         const uint32_t (&bf)[NS][4][2], [[maybe_unused]] const float (&cc)[NS][2], float (&acc)[TM][NS][4]) {
     constexpr uint32_t TS = 16u * sp_pitch<T>(ALN);
@@ -223,18 +276,13 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                 const uint32_t b = b0[h];
                 [[maybe_unused]] const uint32_t e = h ? e1 : e0, a = h ? a1 : a0;
                 if constexpr (ALN) {
-                    const uint32_t s0 = lds32i<o>(b), s1 = lds32i<o>(e);
-                    w[0][h] = __byte_perm(s0, s1, sel);
+                    w[0][h] = __byte_perm(lds32i<o>(b), lds32i<o>(e), sel);
                     if constexpr (Q8) {
                         w[1][h] = lds32i<o + 16>(b);
                         w[2][h] = lds32i<o + 36>(b);
                         w[3][h] = lds32i<o + 52>(b);
                     } else {
                         w[2][h] = lds32i<o + 20>(b);
-                    }
-                    if constexpr (ONE) {   // one activation row: only lane 0 of a quad holds results, and it has the scales
-                        d0[h] = f16lo_to_float(s0);
-                        d1[h] = f16hi_to_float(s1);
                     }
                 } else {
                     w[0][h] = __byte_perm(lds32i<o>(b), lds32i<o + 4>(b), se[h]);
@@ -246,11 +294,9 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                         w[2][h] = __byte_perm(lds32i<o + 20>(b), lds32i<o + 24>(b), so[h]);
                     }
                 }
-                if constexpr (!ALN || !ONE) {
-                    d0[h] = f16lo_to_float(lds_u16i<o>(a));
-                    d1[h] = f16lo_to_float(lds_u16i<o + BB>(a));
-                    if constexpr (!ALN) d1[h] = half ? 0.f : d1[h];
-                }
+                d0[h] = f16lo_to_float(lds_u16i<o>(a));
+                d1[h] = f16lo_to_float(lds_u16i<o + BB>(a));
+                if constexpr (!ALN) d1[h] = half ? 0.f : d1[h];
             }
             uint32_t a[4][4];
             if constexpr (Q8) {
@@ -396,15 +442,175 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
     }
 }
 
+// One unit of a stage against NT tiles, for one or two activation rows: codes as signed bytes, activations as four signed digits
+// (sp::digits), 8-bit integer multiplies.  A multiply takes 32 K values where the f16 form takes 16, Q8_0 codes go in as they lie, 4-bit codes
+// take three operations for eight (with f16 they take twelve), sums of a block are exact, and the digits hold 28 bits of the largest activation.
+// The columns of a multiply are (first | second scale group, digit) of one activation row; a column's B registers are zero outside its group, so
+// one accumulator serves both blocks of a unit (Q6_K, whose scales change every 16 values: both halves of one multiply), and a lane scales its
+// columns with the one scale of their group.  Codes are taken 16 times (Q4_0, Q4_K), 8 times (Q5_K), 4 times (Q6_K) as large:
+// that centres them without an addition (the top bit of the byte changes sign), and sp_code_scale takes it back.  bf: B registers [set][word].
+template <int T> constexpr float sp_code_scale = T == GT_Q8_0 ? 1.f : T == GT_Q6_K ? 0.25f : T == GT_Q5_K ? 0.125f : 0.0625f;
+// OFF: the unit's bytes within a stage from the warp's first unit on.  c: kBias four times, in registers (as an immediate every multiply would
+// copy it into four of them).
+template <int T, bool ALN, uint32_t OFF, int NT, int NS, int TM>
+__device__ __forceinline__ void sp_unit_int(uint32_t a0, uint32_t a1, uint32_t u, uint32_t t, uint32_t tab, bool half, const uint32_t (&bf)[NS][4],
+                                            [[maybe_unused]] const float (&cc)[NS], const uint32_t (&c)[4], float (&acc)[TM][NS][4]) {
+    constexpr uint32_t TS = 16u * sp_pitch<T>(ALN), R8 = ALN ? 8u * sp_pitch<T>(true) : 0u;
+    auto f = [](uint32_t v) { return __uint_as_float(v); };
+    if constexpr (T == GT_Q4_0 || T == GT_Q8_0) {
+        constexpr bool Q8 = T == GT_Q8_0;
+        constexpr uint32_t BB = Q8 ? 34u : 18u;
+        // row g + 8 relative to row g is a compile-time distance only with aligned rows
+        const uint32_t b[2] = {ALN ? a0 + 4 * t : (a0 & ~3u) + 4 * t, ALN ? a0 + 4 * t : (a1 & ~3u) + 4 * t}, a[2] = {a0 + (t >> 1) * BB, (ALN ? a0 : a1) + (t >> 1) * BB};
+        const uint32_t e = a0 + (t ? 4 * t : (Q8 ? 32u : 16u));
+        const uint32_t sel = t ? 0x3210u : 0x5432u;
+        uint32_t se[2], so[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const bool mis = !ALN && ((h ? a1 : a0) & 2u) != 0;
+            se[h] = mis ? 0x7654u : 0x5432u;
+            so[h] = mis ? 0x5432u : 0x3210u;
+        }
+        static_for<0, NT>([&](auto J) {
+            constexpr int j = decltype(J)::value;
+            uint32_t w[4][2];   // as in sp_unit
+            float d[2];
+            static_for<0, 2>([&](auto H) {
+                constexpr int h = decltype(H)::value;
+                constexpr uint32_t o = OFF + j * TS + h * R8;
+                if constexpr (ALN) {
+                    w[0][h] = __byte_perm(lds32i<o>(b[h]), lds32i<o>(e), sel);
+                    if constexpr (Q8) {
+                        w[1][h] = lds32i<o + 16>(b[h]);
+                        w[2][h] = lds32i<o + 36>(b[h]);
+                        w[3][h] = lds32i<o + 52>(b[h]);
+                    } else {
+                        w[2][h] = lds32i<o + 20>(b[h]);
+                    }
+                } else {
+                    w[0][h] = __byte_perm(lds32i<o>(b[h]), lds32i<o + 4>(b[h]), se[h]);
+                    if constexpr (Q8) {
+                        w[1][h] = __byte_perm(lds32i<o + 16>(b[h]), lds32i<o + 20>(b[h]), se[h]);
+                        w[2][h] = __byte_perm(lds32i<o + 36>(b[h]), lds32i<o + 40>(b[h]), so[h]);
+                        w[3][h] = __byte_perm(lds32i<o + 52>(b[h]), lds32i<o + 56>(b[h]), so[h]);
+                    } else {
+                        w[2][h] = __byte_perm(lds32i<o + 20>(b[h]), lds32i<o + 24>(b[h]), so[h]);
+                    }
+                }
+                d[h] = f16lo_to_float(lds_u16i<o>(a[h]));
+                if constexpr (!ALN) d[h] = half ? 0.f : d[h];
+            });
+            if constexpr (!Q8) {   // low nibbles: elements 0..15; high nibbles: 16..31
+#pragma unroll
+                for (int q = 0; q < 4; q += 2)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const uint32_t x = w[q][h];
+                        w[q][h] = ((x << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+                        w[q + 1][h] = (x & 0xF0F0F0F0u) ^ 0x80808080u;
+                    }
+            }
+#pragma unroll
+            for (int s = 0; s < NS; s++) {
+                uint32_t r[4];
+                sp::mma_s8(r, w[0][0], w[0][1], w[1][0], w[1][1], bf[s][0], bf[s][1], c);
+                sp::mma_s8(r, w[2][0], w[2][1], w[3][0], w[3][1], bf[s][2], bf[s][3], r);
+                sp::scaled(acc[j][s], r, d[0], d[1]);
+            }
+        });
+    } else if constexpr (T == GT_Q4_K || T == GT_Q5_K) {
+        constexpr bool Q5 = T == GT_Q5_K;
+        const uint32_t pu = u & 3u, q0 = a0 + 32 * pu + 4 * t, h0 = a0 + 4 * t;
+        static_for<0, NT>([&](auto J) {
+            constexpr int j = decltype(J)::value;
+            uint32_t a[2][4], p[2][2];   // codes (first sub-block: low nibbles, second: high ones); scale and offset (sp_table_row) of rows g, g + 8
+            static_for<0, 2>([&](auto H) {
+                constexpr int h = decltype(H)::value;
+                constexpr uint32_t o = OFF + j * TS + h * R8, q = o + (Q5 ? 48u : 16u);
+                lds64i<j * 256u + h * 128u>(tab, p[h][0], p[h][1]);
+                static_for<0, 2>([&](auto E) {   // first, second 16 elements
+                    constexpr int e = decltype(E)::value;
+                    const uint32_t x = lds32i<q + 16 * e>(q0);
+                    if constexpr (Q5) {
+                        const uint32_t v = lds32i<o + 16 + 16 * e>(h0) >> (2 * pu);
+                        a[0][2 * e + h] = ((x << 3) & 0x78787878u) | (((v << 7) & 0x80808080u) ^ 0x80808080u);
+                        a[1][2 * e + h] = ((x >> 1) & 0x78787878u) | (((v << 6) & 0x80808080u) ^ 0x80808080u);
+                    } else {
+                        a[0][2 * e + h] = ((x << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+                        a[1][2 * e + h] = (x & 0xF0F0F0F0u) ^ 0x80808080u;
+                    }
+                });
+            });
+#pragma unroll
+            for (int s = 0; s < NS; s++) {
+                uint32_t r[4];
+                sp::mma_s8(r, a[0][0], a[0][1], a[0][2], a[0][3], bf[s][0], bf[s][1], c);
+                sp::mma_s8(r, a[1][0], a[1][1], a[1][2], a[1][3], bf[s][2], bf[s][3], r);
+                // the offset joins the top digit (cc is zero in lanes without it)
+                acc[j][s][1] = fmaf(f(p[0][1]), cc[s], acc[j][s][1]);
+                acc[j][s][3] = fmaf(f(p[1][1]), cc[s], acc[j][s][3]);
+                sp::scaled(acc[j][s], r, f(p[0][0]), f(p[1][0]));
+            }
+        });
+    } else {
+        const uint32_t nh = (u >> 1) & 1u, js = u & 1u;
+        const uint32_t lo = 64 * nh + 16 * js + 4 * t, ho = 128 + 32 * nh + 16 * js + 4 * t;
+        auto body = [&](auto SHIFT) {   // as in sp_unit
+            constexpr int shift = decltype(SHIFT)::value;
+            const uint32_t b0 = a0 & ~3u, b1 = ALN ? b0 : a1 & ~3u;
+            const uint32_t L[2] = {b0 + lo, b1 + lo}, X[2] = {b0 + ho, b1 + ho};
+            const uint32_t sl[2] = {(a0 & 2u) ? 0x5432u : 0x3210u, (a1 & 2u) ? 0x5432u : 0x3210u};
+            static_for<0, NT>([&](auto J) {
+                constexpr int j = decltype(J)::value;
+                uint32_t q[4][2];
+                static_for<0, 2>([&](auto H) {
+                    constexpr int h = decltype(H)::value;
+                    constexpr uint32_t o = OFF + j * TS + h * R8;
+                    uint32_t A = lds32i<o>(L[h]), B = lds32i<o + 32>(L[h]), F = lds32i<o>(X[h]);
+                    if constexpr (shift != 0) {
+                        const uint32_t s = shift == 1 ? 0x5432u : sl[h];
+                        A = __byte_perm(A, lds32i<o + 4>(L[h]), s);
+                        B = __byte_perm(B, lds32i<o + 36>(L[h]), s);
+                        F = __byte_perm(F, lds32i<o + 4>(X[h]), s);
+                    }
+                    auto join = [](uint32_t n, uint32_t x) { return (((n & 0x3C3C3C3Cu) | (x & 0xC3C3C3C3u)) & 0xFCFCFCFCu) ^ 0x80808080u; };
+                    q[0][h] = join(A << 2, F << 6);
+                    q[1][h] = join(B << 2, F << 4);
+                    q[2][h] = join(A >> 2, F << 2);
+                    q[3][h] = join(B >> 2, F);
+                });
+                uint32_t pa[2], pb[2];   // scales of the lane's group, first and second multiply, rows g and g + 8
+                lds64i<j * 256u>(tab, pa[0], pa[1]);
+                lds64i<j * 256u + 128u>(tab, pb[0], pb[1]);
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+#pragma unroll
+                    for (int s = 0; s < NS; s++) {
+                        uint32_t r[4];
+                        sp::mma_s8(r, q[2 * i][0], q[2 * i][1], q[2 * i + 1][0], q[2 * i + 1][1], bf[s][2 * i], bf[s][2 * i + 1], c);
+                        sp::scaled(acc[j][s], r, f(pa[i]), f(pb[i]));
+                    }
+            });
+        };
+        if constexpr (ALN) {
+            if (a0 & 2u) body(std::integral_constant<int, 1>{});
+            else body(std::integral_constant<int, 0>{});
+        } else {
+            body(std::integral_constant<int, 2>{});
+        }
+    }
+}
+
 // Scale table of one unit for one row: d * scale of the unit's groups (Q6_K: four), or the scales d sc and the offsets C d sc - dmin m
 // of its two sub-blocks (Q4_K, Q5_K: the codes are taken less C = 8 or 16, the middle of their range, so that the offset is small
 // where scale and minimum belong together; 6-bit fields as in src/gguf/mod.rs:440-452).  rb: shared address of the row's super-block.
-template <int T> __device__ __forceinline__ void sp_table_row(uint32_t dst, uint32_t rb, uint32_t u) {
+template <int T, bool INT> __device__ __forceinline__ void sp_table_row(uint32_t dst, uint32_t rb, uint32_t u) {
     auto put = [&](float a, float b, float c, float d) { sts128(dst, __float_as_uint(a), __float_as_uint(b), __float_as_uint(c), __float_as_uint(d)); };
     if constexpr (T == GT_Q6_K) {
         const uint32_t s = rb + 192 + 8 * ((u >> 1) & 1u) + (u & 1u);
         const float d = f16lo_to_float(lds_u16i<208>(rb));
-        put(d * (float)lds_s8(s), d * (float)lds_s8(s + 2), d * (float)lds_s8(s + 4), d * (float)lds_s8(s + 6));
+        constexpr uint32_t s1 = INT ? 4 : 2, s2 = INT ? 2 : 4;   // (integers: even groups before odd ones)
+        put(d * (float)lds_s8(s), d * (float)lds_s8(s + s1), d * (float)lds_s8(s + s2), d * (float)lds_s8(s + 6));
     } else {
         const uint32_t pu = u & 3u, dd = lds32(rb), s0 = lds32i<4>(rb), s1 = lds32i<8>(rb);
         const float d = f16lo_to_float(dd), dmin = f16hi_to_float(dd);
@@ -423,45 +629,80 @@ template <int T> __device__ __forceinline__ void sp_table_row(uint32_t dst, uint
         }
         constexpr float C = T == GT_Q5_K ? 16.f : 8.f;
         const float e0 = d * (float)c0, e1 = d * (float)c1;   // (17 bits: exact, as the products with the minima)
-        put(e0, e1, fmaf(C, e0, -(dmin * (float)m0)), fmaf(C, e1, -(dmin * (float)m1)));
+        const float o0 = fmaf(C, e0, -(dmin * (float)m0)), o1 = fmaf(C, e1, -(dmin * (float)m1));
+        if constexpr (INT) put(e0, o0, e1, o1);
+        else put(e0, e1, o0, o1);
     }
 }
 
-// One product of a Q4_K or Q5_K row in f32, value by value: for results that are no numbers.
-template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const float *x, uint32_t k) {
+// One product in f32, value by value: for results that are no numbers.
+template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const float *x, const float *x2, uint32_t k) {
     float acc = 0.f;
-    for (uint32_t b = 0; b < k / 256; b++, w += BlockTraits<T>::BYTES, x += 256)
-        for (uint32_t j = 0; j < 8; j++) {
-            uint32_t sc, mn;
-            q4k_scale_min(j, w + 4, sc, mn);
-            const float e = __fmul_rn(half_bits_to_float(ld_u16(w)), (float)sc), m = __fmul_rn(half_bits_to_float(ld_u16(w + 2)), (float)mn);
-            for (uint32_t l = 0; l < 32; l++) {
+    constexpr uint32_t QK = BlockTraits<T>::QK;
+    for (uint32_t b = 0; b < k / QK; b++, w += BlockTraits<T>::BYTES)
+        for (uint32_t e = 0; e < QK; e++) {
+            float v;
+            if constexpr (T == GT_Q4_0) {
+                v = __fmul_rn((float)((int)((w[2 + (e & 15u)] >> (4 * (e >> 4))) & 15u) - 8), half_bits_to_float(ld_u16(w)));
+            } else if constexpr (T == GT_Q8_0) {
+                v = __fmul_rn((float)(int8_t)w[2 + e], half_bits_to_float(ld_u16(w)));
+            } else if constexpr (T == GT_Q6_K) {
+                const uint32_t nh = e >> 7, q = (e >> 5) & 3u, l = e & 31u;
+                const uint32_t n = ((w[64 * nh + 32 * (q & 1u) + l] >> (4 * (q >> 1))) & 15u) | (((w[128 + 32 * nh + l] >> (2 * q)) & 3u) << 4);
+                const float d = __fmul_rn(half_bits_to_float(ld_u16(w + 208)), (float)(int8_t)w[192 + (e >> 4)]);
+                v = __fmul_rn(d, (float)((int)n - 32));
+            } else {
+                const uint32_t j = e >> 5, l = e & 31u;
+                uint32_t sc, mn;
+                q4k_scale_min(j, w + 4, sc, mn);
+                const float d = __fmul_rn(half_bits_to_float(ld_u16(w)), (float)sc), m = __fmul_rn(half_bits_to_float(ld_u16(w + 2)), (float)mn);
                 uint32_t q = (w[(T == GT_Q5_K ? 48 : 16) + 32 * (j >> 1) + l] >> (4 * (j & 1u))) & 15u;
                 if (T == GT_Q5_K) q |= ((w[16 + l] >> j) & 1u) << 4;
-                acc = fmaf(__fsub_rn(__fmul_rn(e, (float)q), m), x[32 * j + l], acc);
+                v = __fsub_rn(__fmul_rn(d, (float)q), m);
             }
+            const uint32_t i = b * QK + e;
+            float a = x[i];
+            if (x2) a = a / (1.0f + expf(-a)) * x2[i];
+            acc = fmaf(v, a, acc);
         }
     return acc;
 }
 
-// A chunk of work: `nt` consecutive tiles of op `op` for entry `ent`, from the op's tile `tile` on.  Chunks are dealt out in runs:
-// cluster c takes the runs c, c + clusters, ....  Runs of one spread what is left over in the last round evenly (768 chunks on 296
-// CTAs, Q8_0 24576 x 4096: 22.4 us, 28.5 with runs of two); where every CTA has as many chunks, runs make no difference (75776 x 4096,
-// four chunks each: 44.9 us in either order).
-struct SpChunk {
+// The tiles of all entries and ops form one line, of which every cluster takes an equal contiguous share, in steps.  A chunk: the next tiles of
+// the share, `nt` of op `op` for entry `ent` from the op's tile `tile` on; what is left of an op is cut into chunks of equal length.  Dense:
+// steps of one tile (shares of whole chunks of four leave a last round part empty: Q4_0 24576 x 4096 has 384 such chunks for 296 CTAs, or 1536
+// tiles).  Routed: steps of a chunk (a share that crosses into another entry has its activations to split: 16 pairs of 768 x 2048 12.9 us, 15.7 in
+// steps of a tile).
+struct __align__(16) SpChunk {
     uint32_t ent, op, tile, nt;
+    uint32_t un, key, e0, cnt;   // this rank's units; the same key: the same activations; the entry's first row or pair and their number
+    uint32_t steps;              // of the share
 };
-__device__ __forceinline__ SpChunk sp_chunk(const SpBatch &b, uint32_t i) {
+__device__ __forceinline__ SpChunk sp_chunk(const SpBatch &b, uint32_t pos, uint32_t last) {
     SpChunk c;
-    const uint32_t all = b.op[b.nops - 1].chunk_end;
-    c.ent = i / all;
-    const uint32_t r = i - c.ent * all;
+    const uint32_t all = b.op[b.nops - 1].step_end;
+    c.ent = pos < all ? 0u : pos / all;
+    const uint32_t r = pos - c.ent * all;
     c.op = 0;
-    while (r >= b.op[c.op].chunk_end) c.op++;
-    c.tile = (r - (c.op ? b.op[c.op - 1].chunk_end : 0u)) * b.tr;
-    c.nt = min(b.tr, (b.op[c.op].n + 15u) / 16u - c.tile);
+    uint32_t from = 0, to = b.op[0].step_end;
+    while (r >= to) {
+        from = to;
+        to = b.op[++c.op].step_end;
+    }
+    c.tile = (r - from) * b.step;
+    const uint32_t left = min((b.op[c.op].n + 15u) / 16u - c.tile, (last - pos) * b.step);
+    c.nt = left;
+    if (left > b.tr) {
+        uint32_t parts = 2;
+        while (parts * b.tr < left && parts < 8) parts++;   // (from eight on: whole chunks)
+        c.nt = b.step == 1 ? min(b.tr, (left + parts - 1) / parts) : b.tr;
+    }
+    c.steps = b.step == 1 ? c.nt : 1u;
     return c;
 }
+
+// The row of a tile that lies at place p of its 16 in a stage (pairs: the even rows come first).
+__device__ __forceinline__ uint32_t sp_row(uint32_t pairs, uint32_t p) { return pairs ? ((p & 7u) << 1) + (p >> 3) : p; }
 
 // Packs activation rows into B register order for the kernel below: f16 hi + lo halves under one power of two per row, the sums of the
 // sub-blocks that have offsets, and the inverse scale.  One block per row.  Several rows (or row groups: Q4_K has no other form
@@ -554,11 +795,12 @@ __global__ void __launch_bounds__(256) qmv_pack_kernel(const __grid_constant__ S
     }
 }
 
-// MPC: 1 = one activation row, 4 = up to four (one set of columns), 8 = up to eight (two sets).
+// MPC: 1, 2 = that many activation rows, in 8-bit integers (sp_unit_int); 4 = up to four, 8 = up to eight, in f16 (one set of columns, two).
 template <int T, bool ALN, int MPC>
 __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_constant__ SpBatch bt, const __grid_constant__ SpMaps maps) {
     using K = SpTraits<T>;
-    constexpr int NS = MPC > 4 ? 2 : 1, NG = K::NG, SU = K::SU, TM = sp_tiles(NS);
+    constexpr bool INT = MPC <= 2;
+    constexpr int NS = sp_sets(MPC), NG = K::NG, SU = K::SU, TM = sp_tiles(MPC);
     constexpr bool TABLE = T == GT_Q4_K || T == GT_Q5_K || T == GT_Q6_K;
     constexpr uint32_t PITCH = sp_pitch<T>(ALN), TILE = 16 * PITCH;
     constexpr uint32_t UB = T == GT_Q8_0 ? 68u : 36u;               // bytes of a unit (Q4_0, Q8_0)
@@ -569,7 +811,8 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
     __shared__ float s_inv[kSpWarps][8];                            // inverse activation scales of a warp's share of K
     __shared__ volatile uint32_t abort_flag, s_again;
     __shared__ uint32_t s_nent;
-    __shared__ uint32_t s_id[kSpMaxPairs];                          // routed: expert of every pair
+    __shared__ SpChunk s_chunk[16];                                 // the chunks in work
+    __shared__ uint16_t s_id[kSpMaxPairs];                          // routed: expert of every pair (there are at most 65535)
     __shared__ uint16_t s_ord[kSpMaxPairs], s_ent[kSpMaxPairs + 1]; // pairs by expert; entry e = pairs s_ord[s_ent[e] ..]
     __shared__ uint32_t s_wcnt[kSpWarps];
 
@@ -593,7 +836,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
     }
     if (bt.ids) {
         grid_dependency_wait();   // the expert ids belong to the kernels ahead
-        for (uint32_t p = tid; p < kSpMaxPairs; p += kSpThreads) s_id[p] = p < bt.npairs ? min(__ldcg(bt.ids + p), bt.n_experts) : 0xFFFFFFFFu;
+        for (uint32_t p = tid; p < kSpMaxPairs; p += kSpThreads) s_id[p] = p < bt.npairs ? (uint16_t)min(__ldcg(bt.ids + p), bt.n_experts) : (uint16_t)0xFFFFu;
     }
     __syncwarp();
     if (ranks > 1) sp::cluster_sync();   // the others' barriers exist before anything is sent there
@@ -635,8 +878,25 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         __syncthreads();
     }
     const uint32_t nent = bt.ids ? s_nent : bt.nent;
-    const uint32_t chunks = nent * bt.op[bt.nops - 1].chunk_end;
-    const uint32_t ncl = gridDim.x / ranks, run = bt.run ? bt.run : (chunks + ncl - 1) / ncl, first = blockIdx.x / ranks * run, skip = (gridDim.x / ranks - 1) * run;
+    // this cluster's share of the tiles
+    const uint32_t ncl = gridDim.x / ranks, cl = blockIdx.x / ranks;
+    const uint64_t steps = (uint64_t)nent * bt.op[bt.nops - 1].step_end;
+    const uint32_t first = (uint32_t)(steps * cl / ncl), last = (uint32_t)(steps * (cl + 1) / ncl);
+    auto chunk = [&](uint32_t at) {
+        SpChunk c = sp_chunk(bt, at, last);
+        const SpOp &P = bt.op[c.op];
+        const uint32_t u0 = rank * P.slice;
+        c.un = u0 < P.units ? min(P.slice, P.units - u0) : 0u;
+        if (bt.ids) {
+            c.e0 = s_ent[c.ent];
+            c.cnt = s_ent[c.ent + 1] - c.e0;
+        } else {
+            c.e0 = c.ent * mp;
+            c.cnt = min(mp, P.m - c.e0);
+        }
+        c.key = c.ent * kSpMaxOps + P.xkey;
+        return c;
+    };
 
     if (warp == kSpWarps) {
         // ======================= producer =======================
@@ -645,24 +905,26 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
         uint32_t slot = 0, ph = 1;   // (a slot's first wait passes)
         bool ok = true;
-        for (uint32_t at = first, left = run; ok && at < chunks; at++) {
-            const SpChunk c = sp_chunk(bt, at);
-            if (--left == 0) {
-                left = run;
-                at += skip;
-            }
+        for (uint32_t at = first, i = 0; ok && at < last; i++) {
+            const SpChunk c = chunk(at);
+            at += c.steps;
             const SpOp &P = bt.op[c.op];
             const uint32_t u0 = rank * P.slice;
-            const uint32_t un = u0 < P.units ? min(P.slice, P.units - u0) : 0u;
-            const uint32_t ex = bt.ids ? s_id[s_ord[s_ent[c.ent]]] : 0u;
-            for (uint32_t u = 0; u < un; u += SU) {
+            const uint32_t ex = bt.ids ? s_id[s_ord[c.e0]] : 0u;
+            // (a rank without units for the chunk: a stage without data, so that the consumers get the chunk's description with it)
+            for (uint32_t u = 0; u == 0 || u < c.un; u += SU) {
                 if (!mbar_wait(&empty[slot], ph, &abort_flag, bt.status, ST_WAIT_EMPTY_TIMEOUT, 0u)) {
                     ok = false;
                     break;
                 }
                 const uint32_t dst = base + slot * STAGE;
                 const uint32_t off = (u0 + u) / 4 * (uint32_t)K::B256;
-                if constexpr (ALN) {
+                // Sixteen descriptions are enough: the one written here was last read for a chunk 16 before, and the slot that the wait above
+                // found empty was left by warps that have arrived for chunk i - 2 - kSpMaxSlots at least.
+                if (u == 0 && lane == 0) s_chunk[i & 15u] = c;
+                if (c.un == 0) {
+                    if (lane == 0) mbar_arrive(&full[slot]);
+                } else if constexpr (ALN) {
                     if (lane == 0) {
                         mbar_expect_tx(&full[slot], c.nt * TILE);
                         for (uint32_t j = 0; j < c.nt; j++)
@@ -671,6 +933,21 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                                 ::"r"(dst + j * TILE), "l"(&maps.m[c.op]), "r"((off & ~15u) >> 3), "r"((c.tile + j) * 16u), "r"(ex),
                                   "r"(smem_u32(&full[slot])), "l"(pol)
                                 : "memory");
+                    }
+                } else if (bt.pairs) {
+                    // A row of the tensor map is two weight rows, a copy the even or the odd rows of a tile (see sp_row).  (Four or eight weight
+                    // rows a map row would do for any address, but copies have to start on 128 bytes, where their rows would meet in the
+                    // same banks.)
+                    if (lane == 0) {
+                        mbar_expect_tx(&full[slot], c.nt * TILE);
+                        for (uint32_t j = 0; j < c.nt; j++)
+#pragma unroll
+                            for (uint32_t r = 0; r < 2; r++)
+                                asm volatile(
+                                    "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;"
+                                    ::"r"(dst + j * TILE + r * 8 * PITCH), "l"(&maps.m[c.op]), "r"(((r * P.row_bytes + off) & ~15u) >> 3),
+                                      "r"((c.tile + j) * 8u), "r"(ex), "r"(smem_u32(&full[slot])), "l"(pol)
+                                    : "memory");
                     }
                 } else {
                     // one bulk copy per row: the 16-byte superset of the row's segment (an expert that does not exist: expert 0,
@@ -707,53 +984,67 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         const uint32_t g = lane >> 2, t = lane & 3u;
         const uint32_t xf = base + bt.xf_off, ccb = base + bt.cc_off, tab = base + bt.tab_off + warp * (R * 16u), red = base + bt.red_off;
         const uint32_t xs = bt.xstride, cs = bt.cstride;
-        const uint32_t xlane = xf + (MPC == 1 ? 0u : ((g >> 1) & (mp - 1)) * xs) + (t * 2 + (g & 1u)) * 16u;
-        const uint32_t clane = ccb + (MPC == 1 ? 0u : (t & (mp - 1)) * cs);
+        // integers: column g is digit g % 4 of the set's row in group g / 4; a lane scales columns 2 t and 2 t + 1, which are of group t / 2
+        const uint32_t xlane = INT ? xf + (g & 3u) * 64u + t * 16u : xf + ((g >> 1) & (mp - 1)) * xs + (t * 2 + (g & 1u)) * 16u;
+        const uint32_t clane = ccb + (INT ? (t >> 1) * 4u : (t & (mp - 1)) * cs);
         uint32_t slot = 0, ph = 0, cur = 0xFFFFFFFFu;
         bool ok = true;
+        [[maybe_unused]] uint32_t bias[4];
+        if constexpr (INT) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) asm volatile("mov.u32 %0, %1;" : "=r"(bias[q]) : "n"(sp::kBias));
+        }
         auto wait = [&](uint64_t &bar, uint32_t parity, uint32_t code) {
             ok = mbar_wait(&bar, parity, &abort_flag, bt.status, code, 0u) && ok;
             return ok;
         };
-        // (finished chunks are remembered by their number alone: registers are what this kernel is short of)
-        auto store = [&](uint32_t at, uint32_t col, uint32_t row, float v) {
-            const SpChunk d = sp_chunk(bt, at);
+        auto store = [&](const SpChunk &d, uint32_t col, uint32_t row, float v) {
             const SpOp &P = bt.op[d.op];
-            const uint32_t grow = d.tile * 16u + row, e0 = bt.ids ? (uint32_t)s_ent[d.ent] : d.ent * mp;
-            const uint32_t cnt = bt.ids ? s_ent[d.ent + 1] - e0 : min(mp, P.m - e0);
-            if (col >= cnt || row >= d.nt * 16u || grow >= P.n) return;
-            const uint32_t pair = bt.ids ? (uint32_t)s_ord[e0 + col] : e0 + col;
+            const uint32_t grow = d.tile * 16u + (ALN ? row : (row & ~15u) + sp_row(bt.pairs, row & 15u));
+            if (col >= d.cnt || row >= d.nt * 16u || grow >= P.n) return;
+            const uint32_t pair = bt.ids ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
             const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
             if (bt.ids && s_id[pair] >= bt.n_experts) v = 0.f;   // an id that names no expert
-            if (NG != 0 && v != v) s_again = 1;
+            if ((INT || NG != 0) && v != v) s_again = 1;
             P.y[o] = v;
             for (uint32_t pr = 0; pr < P.n_peer; pr++) P.y_peer[pr][o] = v;
         };
-        [[maybe_unused]] auto again = [&](uint32_t at, uint32_t col, uint32_t row) {
-            const SpChunk d = sp_chunk(bt, at);
+        [[maybe_unused]] auto again = [&](const SpChunk &d, uint32_t col, uint32_t row) {
             const SpOp &P = bt.op[d.op];
-            const uint32_t grow = d.tile * 16u + row, e0 = bt.ids ? (uint32_t)s_ent[d.ent] : d.ent * mp;
-            const uint32_t cnt = bt.ids ? s_ent[d.ent + 1] - e0 : min(mp, P.m - e0);
-            if (col >= cnt || row >= d.nt * 16u || grow >= P.n) return;
-            const uint32_t pair = bt.ids ? (uint32_t)s_ord[e0 + col] : e0 + col;
+            const uint32_t grow = d.tile * 16u + (ALN ? row : (row & ~15u) + sp_row(bt.pairs, row & 15u));
+            if (col >= d.cnt || row >= d.nt * 16u || grow >= P.n) return;
+            const uint32_t pair = bt.ids ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
             const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
             float v = P.y[o];
             if (v == v) return;
             v = sp_again<T>(P.w + (bt.ids ? s_id[pair] * P.expert_stride : 0ull) + (uint64_t)grow * P.row_bytes,
-                            P.x + (size_t)(bt.ids ? pair / P.x_div : pair) * P.k, P.k);
+                            P.x + (size_t)(bt.ids ? pair / P.x_div : pair) * P.k,
+                            P.x2 ? P.x2 + (size_t)(bt.ids ? pair / P.x_div : pair) * P.k : nullptr, P.k);
             P.y[o] = v;
             for (uint32_t pr = 0; pr < P.n_peer; pr++) P.y_peer[pr][o] = v;
         };
         const uint32_t share = R / ranks;   // rows of a chunk that a rank finishes
+        const uint32_t RS = mp * R + (INT ? 8 : 0);   // floats from one warp's sums to the next (integers: what four lanes read is in distinct banks)
         // the CTA's sums of chunk j, in warp order: results, or for the rank that finishes the row
-        auto add = [&](uint32_t j, uint32_t d) {
+        auto add = [&](uint32_t j, uint32_t at) {
             if (!wait(sync_bar[j & 1u], (j >> 1) & 1u, ST_WAIT_EMPTY_TIMEOUT)) return false;
-            const uint32_t part = red + (j & 1u) * (kSpWarps * mp * R * 4u), buf = j & 3u;
+            const SpChunk d = s_chunk[at];
+            const uint32_t part = red + (INT ? j & 3u : j & 1u) * (kSpWarps * RS * 4u), buf = j & 3u;
+            if (INT && ranks == 1) {   // four lanes a result, two warps' sums each
+                for (uint32_t q = tid >> 2; q < (MPC == 1 ? 16u * d.nt : mp * R); q += kSpWarps * 8) {
+                    const uint32_t a = part + ((tid & 3u) * RS + q) * 4;
+                    float v = __uint_as_float(lds32(a)) + __uint_as_float(lds32(a + 16 * RS));
+                    v += __shfl_xor_sync(0xffffffffu, v, 1);
+                    v += __shfl_xor_sync(0xffffffffu, v, 2);
+                    const uint32_t col = MPC == 1 || q < R ? 0u : 1u;
+                    if ((tid & 3u) == 0) store(d, col, q - col * R, v);
+                }
+            } else
             for (uint32_t q = tid; q < mp * R; q += 256) {
                 const uint32_t col = q / R, row = q - col * R;
                 float v = 0.f;
 #pragma unroll
-                for (int w = 0; w < kSpWarps; w++) v += __uint_as_float(lds32(part + ((w * mp + col) * R + row) * 4));
+                for (int w = 0; w < kSpWarps; w++) v += __uint_as_float(lds32(part + (w * RS + q) * 4));
                 if (ranks == 1) {
                     store(d, col, row, v);
                 } else {
@@ -763,7 +1054,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sync_bar[2]);
+            if (!INT && lane == 0) mbar_arrive(&sync_bar[2]);
             if (ranks > 1 && tid == 0) mbar_expect_tx(&recv_bar[buf], mp * R * 4u);
             return true;
         };
@@ -771,8 +1062,9 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         // chunk j + 4 comes here from a rank all of whose warps have finished j + 2; that takes rows of j + 2 sent by this rank,
         // which its warps send only once every one of them has arrived on sync_bar for j + 2; and a warp does that after it has read
         // chunk j here.
-        auto finish = [&](uint32_t j, uint32_t d) {
+        auto finish = [&](uint32_t j, uint32_t at) {
             const uint32_t buf = j & 3u;
+            const SpChunk d = s_chunk[at];
             if (!wait(recv_bar[buf], (j >> 2) & 1u, ST_WAIT_FULL_TIMEOUT)) return false;
             for (uint32_t q = tid; q < mp * share; q += 256) {
                 const uint32_t col = q / share, row = q - col * share;
@@ -790,30 +1082,29 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             c_ph ^= 1u;
             return r;
         };
-        uint32_t d1 = 0, d2 = 0;
+        uint32_t d1 = 0, d2 = 0;   // where the descriptions of the last two chunks are
         uint32_t i = 0;   // the CTA's chunks so far
+        // (what the first chunk needs of the launch's parameters is fetched before the wait)
+        const SpChunk c0 = chunk(first < last ? first : 0);
+        {
+            const SpOp &P = bt.op[c0.op];
+            if constexpr (INT) asm volatile("" ::"l"(P.x), "l"(P.x2), "r"(P.k), "r"(P.slice));
+            else if (bt.packed) asm volatile("" ::"l"(P.xp), "l"(P.xinv), "r"(P.pk_units));
+        }
         if (!bt.ids) grid_dependency_wait();   // the activations belong to the kernels ahead until those are done
-        for (uint32_t at = first, left = run; ok && at < chunks; at++, i++) {
-            const SpChunk c = sp_chunk(bt, at);
-            const uint32_t this_at = at;
-            if (--left == 0) {
-                left = run;
-                at += skip;
+        for (uint32_t at = first; ok && at < last; i++) {
+            SpChunk c = c0;
+            if (INT && i != 0) {   // the producer's description comes with the first stage
+                if (!wait(full[slot], ph, ST_WAIT_FULL_TIMEOUT)) break;
+                c = s_chunk[i & 15u];
+            } else if (i != 0) {
+                c = chunk(at);
             }
+            at += c.steps;
             const SpOp &P = bt.op[c.op];
-            const uint32_t u0 = rank * P.slice;
-            const uint32_t un = u0 < P.units ? min(P.slice, P.units - u0) : 0u;
-            uint32_t e0 = 0, cnt, ex = 0;
-            if (bt.ids) {
-                e0 = s_ent[c.ent];
-                cnt = s_ent[c.ent + 1] - e0;
-                ex = s_id[s_ord[e0]];
-            } else {
-                e0 = c.ent * mp;
-                cnt = min(mp, P.m - e0);
-            }
-            const uint32_t key = c.ent * kSpMaxOps + P.xkey;
-            if (MPC > 1 && key != cur && bt.packed) {
+            const uint32_t u0 = rank * P.slice, un = c.un, e0 = c.e0, cnt = c.cnt, key = c.key;
+            const uint32_t ex = bt.ids && !ALN ? s_id[s_ord[e0]] : 0u;
+            if (!INT && key != cur && bt.packed) {
                 // the rows' slices come ready from the pack kernel's scratch area
                 if (cur != 0xFFFFFFFFu && !csync()) break;   // nobody reads the entry before any more
                 cur = key;
@@ -842,68 +1133,102 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 sp_pairs<T, ALN>(warp, q, tt, p0, p1);
                 const uint32_t kb = (T == GT_Q6_K ? 256u * ((u0 + warp) >> 2) : 64u * (u0 + warp)) + 512u * hf;
                 const uint32_t mine = un > warp ? (un - warp + 7) / 8 : 0u;          // the warp's units
-                const uint32_t d0 = xf + ((warp + 8 * hf) * 2 + (q >> 1)) * 128u + tt * 32u + (q & 1u) * 8u;
-                // a pass's values: the sums of the sub-blocks, and the halves at `d`
-                auto write = [&](const float (&z)[4], float s, uint32_t p, uint32_t row, bool mine_too) {
-                    const float c[4] = {z[0] * s, z[1] * s, z[2] * s, z[3] * s};
+                // a pass's values: the sums of the sub-blocks, and the halves or digits
+                const uint32_t d0 = xf + (INT ? (warp + 8 * hf) * 256u + tt * 16u + q * 4u : ((warp + 8 * hf) * 2 + (q >> 1)) * 128u + tt * 32u + (q & 1u) * 8u);
+                auto write = [&](const float (&z)[4], float s, float s1, uint32_t p, uint32_t row, bool mine_too) {
+                    float c[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) c[e] = INT ? z[e] * s * s1 : z[e] * s;
                     [[maybe_unused]] float sum = 0.f;
                     if constexpr (NG != 0) {
                         sum = (c[0] + c[1]) + (c[2] + c[3]);
 #pragma unroll
                         for (int o = 1; o <= 4; o *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                        if constexpr (INT) sum *= 1.f / (256.f * sp_code_scale<T>);   // (in units of the top digit and of the codes)
                     }
-                    uint32_t hi[2], lo[2];
-                    sp::split(c[0], c[2], hi[0], lo[0]);
-                    sp::split(c[1], c[3], hi[1], lo[1]);
+                    uint32_t l[4];
+                    if constexpr (INT) {
+                        sp::digits(c, l);
+                    } else {
+                        sp::split(c[0], c[2], l[0], l[2]);
+                        sp::split(c[1], c[3], l[1], l[3]);
+                    }
                     if (2 * p + hf >= mine || !mine_too) return;
                     const uint32_t d = d0 + p * 4096u + row * xs;
-                    sts64(d, hi[0], hi[1]);
-                    sts64(d + 16, lo[0], lo[1]);
+                    if constexpr (INT) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) sts32(d + 64 * i, l[i]);
+                    } else {
+                        sts64(d, l[0], l[1]);
+                        sts64(d + 16, l[2], l[3]);
+                    }
                     if (NG != 0 && (lane & 7u) == 0) sts32(ccb + ((warp + 8 * hf) * NG + (q >> 1)) * 4u + p * (64u * NG) + row * cs, __float_as_uint(sum));
                 };
                 __syncwarp();
-                if constexpr (MPC == 1) {
-                    const uint32_t row = e0;
-                    const float *x = P.x + (size_t)row * P.k + kb, *y = P.x2 ? P.x2 + (size_t)row * P.k + kb : nullptr;
-                    auto load = [&](uint32_t p, float (&v)[4]) {
+                if constexpr (INT) {
+                    const float *x[MPC], *y[MPC];
+#pragma unroll
+                    for (int r = 0; r < MPC; r++) {
+                        const size_t o = (size_t)(e0 + min((uint32_t)r, cnt - 1)) * P.k + kb;
+                        x[r] = P.x + o;
+                        y[r] = P.x2 ? P.x2 + o : nullptr;
+                    }
+                    auto load = [&](int r, uint32_t p, float (&v)[4]) {
                         v[0] = v[1] = v[2] = v[3] = 0.f;
                         const uint32_t o = 1024u * p;
                         if (2 * p + hf >= mine) return;
                         const bool i0 = kb + o + p0 < P.k, i1 = kb + o + p1 < P.k;
-                        if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(x + o + p0));
-                        if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[2]), "=f"(v[3]) : "l"(x + o + p1));
-                        if (y) {   // silu(gate) * up, as src/shaders/silu_mul.metal:17-30
+                        if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(x[r] + o + p0));
+                        if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[2]), "=f"(v[3]) : "l"(x[r] + o + p1));
+                        if (y[r]) {   // silu(gate) * up, as src/shaders/silu_mul.metal:17-30
                             float w[4] = {0.f, 0.f, 0.f, 0.f};
-                            if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[0]), "=f"(w[1]) : "l"(y + o + p0));
-                            if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[2]), "=f"(w[3]) : "l"(y + o + p1));
+                            if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[0]), "=f"(w[1]) : "l"(y[r] + o + p0));
+                            if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[2]), "=f"(w[3]) : "l"(y[r] + o + p1));
 #pragma unroll
                             for (int e = 0; e < 4; e++) v[e] = v[e] / (1.0f + expf(-v[e])) * w[e];
                         }
                     };
-                    auto peak = [](const float (&v)[4]) { return fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))); };
+                    // (largest magnitude by its bits: an infinity is above every number, a NaN above that)
+                    auto peak = [](const float (&v)[4]) {
+                        uint32_t b[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++) b[e] = __float_as_uint(v[e]) & 0x7FFFFFFFu;
+                        return max(max(b[0], b[1]), max(b[2], b[3]));
+                    };
                     constexpr int HELD = 4;   // passes whose values stay in registers; those beyond are loaded again
-                    float v[HELD][4], am = 0.f;
+                    float v[MPC][HELD][4], s[MPC], s1[MPC];
 #pragma unroll
-                    for (int p = 0; p < HELD; p++) load(p, v[p]);
+                    for (int r = 0; r < MPC; r++)
 #pragma unroll
-                    for (int p = 0; p < HELD; p++) am = fmaxf(am, peak(v[p]));
-                    for (uint32_t p = HELD; 2 * p < mine; p++) {
-                        float z[4];
-                        load(p, z);
-                        am = fmaxf(am, peak(z));
+                        for (int p = 0; p < HELD; p++) load(r, p, v[r][p]);
+#pragma unroll
+                    for (int r = 0; r < MPC; r++) {
+                        uint32_t am = 0;
+#pragma unroll
+                        for (int p = 0; p < HELD; p++) am = max(am, peak(v[r][p]));
+                        for (uint32_t p = HELD; 2 * p < mine; p++) {
+                            float z[4];
+                            load(r, p, z);
+                            am = max(am, peak(z));
+                        }
+                        am = __reduce_max_sync(0xffffffffu, am);
+                        float inv0, inv1;
+                        sp::pow2_int(am, s[r], s1[r], inv0, inv1);
+                        if (lane == 0) {
+                            s_inv[warp][2 * r] = inv0 * sp_code_scale<T>;
+                            s_inv[warp][2 * r + 1] = inv1;
+                        }
                     }
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-                    float s, inv;
-                    sp::pow2(am, s, inv);
-                    if (lane == 0) s_inv[warp][0] = inv;
+                    for (int r = 0; r < MPC; r++) {
 #pragma unroll
-                    for (int p = 0; p < HELD; p++)
-                        if (2u * p < mine) write(v[p], s, p, 0, true);
-                    for (uint32_t p = HELD; 2 * p < mine; p++) {
-                        float z[4];
-                        load(p, z);
-                        write(z, s, p, 0, true);
+                        for (int p = 0; p < HELD; p++)
+                            if (2u * p < mine) write(v[r][p], s[r], s1[r], p, r, r < (int)cnt);
+                        for (uint32_t p = HELD; 2 * p < mine; p++) {
+                            float z[4];
+                            load(r, p, z);
+                            write(z, s[r], s1[r], p, r, r < (int)cnt);
+                        }
                     }
                 } else {
                 // Four passes are in flight at a time: of one row, or of two or four rows where a row has fewer.
@@ -966,11 +1291,11 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                         if (lane == 0 && rb + (j >> sh) < cnt) s_inv[warp][rb + (j >> sh)] = inv;
                     }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) write(v[j], s[j], j & ((1u << sh) - 1u), rb + (j >> sh), rb + (j >> sh) < cnt);
+                    for (int j = 0; j < 4; j++) write(v[j], s[j], 1.f, j & ((1u << sh) - 1u), rb + (j >> sh), rb + (j >> sh) < cnt);
                     for (uint32_t p = 4; p < passes; p++) {
                         float z[4];
                         load(x[0], y[0], p, z);
-                        write(z, s[0], p, rb, true);
+                        write(z, s[0], 1.f, p, rb, true);
                     }
                 }
                 }
@@ -983,59 +1308,119 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
 #pragma unroll
                 for (int s = 0; s < NS; s++) acc[j][s][0] = acc[j][s][1] = acc[j][s][2] = acc[j][s][3] = 0.f;
 
-            for (uint32_t us = 0; us < un; us += SU) {
-                const uint32_t off = (u0 + us) / 4 * (uint32_t)K::B256;
-                // where a row's data starts in its 16-byte superset (tiles are 16 rows: the same for every tile)
-                const uint32_t wl = ALN ? 0u : ((uint32_t)(uintptr_t)P.w + (ex < bt.n_experts ? ex : 0u) * (uint32_t)P.expert_stride + off) & 15u;
-                const uint32_t rb15 = P.row_bytes & 15u;
-                auto lead = [&](uint32_t row) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + row * rb15) & 15u; };
-                if (!mbar_wait(&full[slot], ph, &abort_flag, bt.status, ST_WAIT_FULL_TIMEOUT, 0u)) {
-                    ok = false;
-                    break;
-                }
-                const uint32_t stage = base + slot * STAGE;
-                const uint32_t r0 = stage + g * PITCH + lead(g), r1 = stage + (g + 8) * PITCH + lead(g + 8);
-#pragma unroll
-                for (int i = 0; i < SU / kSpWarps; i++) {
-                    const uint32_t ul = warp + 8u * i, uu = us + ul;
-                    if (uu >= un) break;
-                    uint32_t bf[NS][4][2];
-                    float cc[NS][2];
-#pragma unroll
-                    for (int s = 0; s < NS; s++) {
-                        uint32_t v[4];
-                        const uint32_t xa = xlane + uu * 256u + s * 4u * xs;
-                        [[maybe_unused]] const uint32_t ca = clane + uu * NG * 4u + s * 4u * cs;
-                        lds128i<0>(xa, v);
-                        bf[s][0][0] = v[0]; bf[s][0][1] = v[1]; bf[s][1][0] = v[2]; bf[s][1][1] = v[3];
-                        lds128i<128>(xa, v);
-                        bf[s][2][0] = v[0]; bf[s][2][1] = v[1]; bf[s][3][0] = v[2]; bf[s][3][1] = v[3];
-#pragma unroll
-                        for (int q = 0; q < NG; q++) cc[s][q] = __uint_as_float(lds32(ca + q * 4u));
-                    }
-                    const uint32_t ub = TABLE ? (ul >> 2) * (uint32_t)K::B256 : ul * UB;
-                    if constexpr (TABLE) {
-                        __syncwarp();   // the table of the unit before has been read
-#pragma unroll
-                        for (int rr = 0; rr < TM / 2; rr++) {
-                            const uint32_t r = lane + 32u * rr;
-                            if (r < 16u * c.nt) sp_table_row<T>(tab + r * 16, stage + r * PITCH + lead(r) + ub, ul);
+            if constexpr (INT) {
+                // (the tiles are a compile-time number for all of the chunk: addresses are then offsets of the loads)
+                auto stages = [&](auto N) {
+                    constexpr int NT = decltype(N)::value;
+                    for (uint32_t us = 0; us == 0 || us < un; us += SU) {
+                        const uint32_t off = (u0 + us) / 4 * (uint32_t)K::B256;
+                        const uint32_t wl = ALN ? 0u : ((uint32_t)(uintptr_t)P.w + (ex < bt.n_experts ? ex : 0u) * (uint32_t)P.expert_stride + off) & 15u;
+                        const uint32_t rb15 = P.row_bytes & 15u;
+                        auto lead = [&](uint32_t row) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + sp_row(bt.pairs, row & 15u) * rb15) & 15u; };
+                        const uint32_t stage = base + slot * STAGE + (TABLE ? (warp >> 2) * (uint32_t)K::B256 : warp * UB);
+                        const uint32_t xa = xlane + (us + warp) * 256u;
+                        [[maybe_unused]] const uint32_t ca = clane + (us + warp) * (NG * 4u);
+                        if ((us != 0 || i == 0) && !mbar_wait(&full[slot], ph, &abort_flag, bt.status, ST_WAIT_FULL_TIMEOUT, 0u)) {
+                            ok = false;
+                            break;
                         }
+                        static_for<0, SU / kSpWarps>([&](auto I) {
+                            constexpr uint32_t i = decltype(I)::value, OFF = i * (kSpWarps / 4) * K::B256;
+                            const uint32_t uu = us + warp + kSpWarps * i;
+                            if (uu >= un) return;
+                            uint32_t b[NS][4];
+                            float cc[NS];
+#pragma unroll
+                            for (int s = 0; s < NS; s++) {
+                                lds128i<i * kSpWarps * 256u>(xa + s * xs, b[s]);
+                                constexpr int own = T == GT_Q6_K ? 5 : 3;   // words of the first group (Q6_K: the even groups)
+#pragma unroll
+                                for (int q = 0; q < 4; q++) b[s][q] = ((g & 4u) != 0) != ((own >> q & 1) != 0) ? b[s][q] : 0u;
+                                cc[s] = 0.f;
+                                if constexpr (NG != 0)
+                                    if (t & 1u) cc[s] = __uint_as_float(lds32i<i * kSpWarps * NG * 4u>(ca + s * cs));
+                            }
+                            if constexpr (TABLE) {
+                                __syncwarp();   // the table of the unit before has been read
+#pragma unroll
+                                for (int rr = 0; rr < (NT + 1) / 2; rr++) {
+                                    const uint32_t r = lane + 32u * rr;
+                                    if (r < 16u * NT) sp_table_row<T, true>(tab + r * 16, stage + OFF + r * PITCH + lead(r), warp);
+                                }
+                                __syncwarp();
+                            }
+                            // (an odd number of blocks: the second block of the last unit lies past the row)
+                            const bool half = !ALN && t >= 2 && (u0 + uu) * 64 + 32 >= P.k;
+                            sp_unit_int<T, ALN, OFF, NT>(stage + g * PITCH + lead(g), stage + (g + 8) * PITCH + lead(g + 8), warp, t,
+                                                         tab + g * 16 + (t >> 1) * 8, half, b, cc, bias, acc);
+                        });
                         __syncwarp();
+                        if (lane == 0) mbar_arrive(&empty[slot]);
+                        if (++slot == bt.nslots) {
+                            slot = 0;
+                            ph ^= 1u;
+                        }
                     }
-                    // (an odd number of blocks: the second block of the last unit lies past the row)
-                    const bool half = (u0 + uu) * 64 + 32 >= P.k;
-                    auto tiles = [&](auto NT) { sp_unit<T, ALN, decltype(NT)::value, NS, MPC == 1>(r0 + ub, r1 + ub, ul, t, g, tab, half, bf, cc, acc); };
-                    if (c.nt == 1) tiles(std::integral_constant<int, 1>{});
-                    else if (TM == 2 || c.nt == 2) tiles(std::integral_constant<int, 2>{});
-                    else if (c.nt == 3) tiles(std::integral_constant<int, TM == 2 ? 2 : 3>{});
-                    else tiles(std::integral_constant<int, TM>{});
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&empty[slot]);
-                if (++slot == bt.nslots) {
-                    slot = 0;
-                    ph ^= 1u;
+                };
+                if (c.nt == 1) stages(std::integral_constant<int, 1>{});
+                else if (c.nt == 2) stages(std::integral_constant<int, 2>{});
+                else if (c.nt == 3) stages(std::integral_constant<int, 3>{});
+                else stages(std::integral_constant<int, TM>{});
+            } else {
+                for (uint32_t us = 0; us == 0 || us < un; us += SU) {
+                    const uint32_t off = (u0 + us) / 4 * (uint32_t)K::B256;
+                    // where a row's data starts in its 16-byte superset (tiles are 16 rows: the same for every tile)
+                    const uint32_t wl = ALN ? 0u : ((uint32_t)(uintptr_t)P.w + (ex < bt.n_experts ? ex : 0u) * (uint32_t)P.expert_stride + off) & 15u;
+                    const uint32_t rb15 = P.row_bytes & 15u;
+                    auto lead = [&](uint32_t row) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + sp_row(bt.pairs, row & 15u) * rb15) & 15u; };
+                    if (!mbar_wait(&full[slot], ph, &abort_flag, bt.status, ST_WAIT_FULL_TIMEOUT, 0u)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t stage = base + slot * STAGE;
+                    const uint32_t r0 = stage + g * PITCH + lead(g), r1 = stage + (g + 8) * PITCH + lead(g + 8);
+#pragma unroll
+                    for (int i = 0; i < SU / kSpWarps; i++) {
+                        const uint32_t ul = warp + 8u * i, uu = us + ul;
+                        if (uu >= un) break;
+                        uint32_t bf[NS][4][2];
+                        float cc[NS][2];
+#pragma unroll
+                        for (int s = 0; s < NS; s++) {
+                            uint32_t v[4];
+                            const uint32_t xa = xlane + uu * 256u + s * 4u * xs;
+                            [[maybe_unused]] const uint32_t ca = clane + uu * NG * 4u + s * 4u * cs;
+                            lds128i<0>(xa, v);
+                            bf[s][0][0] = v[0]; bf[s][0][1] = v[1]; bf[s][1][0] = v[2]; bf[s][1][1] = v[3];
+                            lds128i<128>(xa, v);
+                            bf[s][2][0] = v[0]; bf[s][2][1] = v[1]; bf[s][3][0] = v[2]; bf[s][3][1] = v[3];
+#pragma unroll
+                            for (int q = 0; q < NG; q++) cc[s][q] = __uint_as_float(lds32(ca + q * 4u));
+                        }
+                        const uint32_t ub = TABLE ? (ul >> 2) * (uint32_t)K::B256 : ul * UB;
+                        if constexpr (TABLE) {
+                            __syncwarp();   // the table of the unit before has been read
+#pragma unroll
+                            for (int rr = 0; rr < TM / 2; rr++) {
+                                const uint32_t r = lane + 32u * rr;
+                                if (r < 16u * c.nt) sp_table_row<T, false>(tab + r * 16, stage + r * PITCH + lead(r) + ub, ul);
+                            }
+                            __syncwarp();
+                        }
+                        // (an odd number of blocks: the second block of the last unit lies past the row)
+                        const bool half = (u0 + uu) * 64 + 32 >= P.k;
+                        auto tiles = [&](auto NT) { sp_unit<T, ALN, decltype(NT)::value>(r0 + ub, r1 + ub, ul, t, g, tab, half, bf, cc, acc); };
+                        if (c.nt == 1) tiles(std::integral_constant<int, 1>{});
+                        else if (TM == 2 || c.nt == 2) tiles(std::integral_constant<int, 2>{});
+                        else if (c.nt == 3) tiles(std::integral_constant<int, TM == 2 ? 2 : 3>{});
+                        else tiles(std::integral_constant<int, TM>{});
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty[slot]);
+                    if (++slot == bt.nslots) {
+                        slot = 0;
+                        ph ^= 1u;
+                    }
                 }
             }
             if (!ok) break;
@@ -1044,8 +1429,50 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             // waited for two chunks later, so that nobody stands still for the slowest warp or for the way between SMs ----
             // (finish comes before this warp's arrivals for chunk i: four receive buffers rest on that, see there)
             if (i >= 2 && ranks > 1 && !finish(i - 2, d2)) break;
-            if (i >= 2 && !wait(sync_bar[2], i & 1u, ST_WAIT_EMPTY_TIMEOUT)) break;   // chunk i - 2 has been read out of the area
-            const uint32_t part = red + (i & 1u) * (kSpWarps * mp * R * 4u);
+            // Chunk i - 2 has been read out of the area.  (Integers: four areas.  Who comes here has found every warp's arrival for chunk i - 2, and
+            // a warp arrives there after it has read chunk i - 4.)
+            if (!INT && i >= 2 && !wait(sync_bar[2], i & 1u, ST_WAIT_EMPTY_TIMEOUT)) break;
+            const uint32_t part = red + (INT ? i & 3u : i & 1u) * (kSpWarps * RS * 4u);
+            if constexpr (INT) {
+                // A result is the sum of its row's columns over the four lanes: digits 0 and 1 or 2 and 3 of the first or second groups.  The
+                // lanes exchange halves of what they have, so that each ends up with the sums of one tile (or of half a tile).
+                const bool odd = t & 1u, up = t & 2u;
+                const float w0 = odd ? sp::kDigitWeight : 1.f, w1 = 256.f * w0;
+                auto swap = [](float keep, float give, int o) { return keep + __shfl_xor_sync(0xffffffffu, give, o); };
+#pragma unroll
+                for (int s = 0; s < NS; s++) {
+                    const float i0 = s_inv[warp][2 * s], i1 = s_inv[warp][2 * s + 1];
+                    const uint32_t a = part + (warp * RS + s * R + g) * 4;
+                    float v[TM][2];
+#pragma unroll
+                    for (int j = 0; j < TM; j++)
+#pragma unroll
+                        for (int h = 0; h < 2; h++) v[j][h] = fmaf(acc[j][s][2 * h + 1], w1, acc[j][s][2 * h] * w0);
+                    if (TM > 2 && c.nt > 2) {
+                        float k[2][2];
+#pragma unroll
+                        for (int j = 0; j < 2; j++)
+#pragma unroll
+                            for (int h = 0; h < 2; h++) k[j][h] = swap(odd ? v[TM - 2 + j][h] : v[j][h], odd ? v[j][h] : v[TM - 2 + j][h], 1);
+                        const float r0 = swap(up ? k[1][0] : k[0][0], up ? k[0][0] : k[1][0], 2), r1 = swap(up ? k[1][1] : k[0][1], up ? k[0][1] : k[1][1], 2);
+                        const uint32_t j = 2 * (t & 1u) + (t >> 1);
+                        if (j < c.nt) {
+                            sts32(a + 64 * j, __float_as_uint(r0 * i0 * i1));
+                            sts32(a + 64 * j + 32, __float_as_uint(r1 * i0 * i1));
+                        }
+                    } else if (c.nt == 2) {
+                        float k[2];
+#pragma unroll
+                        for (int h = 0; h < 2; h++) k[h] = swap(odd ? v[1][h] : v[0][h], odd ? v[0][h] : v[1][h], 1);
+                        const float r = swap(up ? k[1] : k[0], up ? k[0] : k[1], 2);
+                        sts32(a + 64 * (t & 1u) + 32 * (t >> 1), __float_as_uint(r * i0 * i1));
+                    } else {
+                        float r = swap(odd ? v[0][1] : v[0][0], odd ? v[0][0] : v[0][1], 1);
+                        r += __shfl_xor_sync(0xffffffffu, r, 2);
+                        if (t < 2) sts32(a + 32 * t, __float_as_uint(r * i0 * i1));
+                    }
+                }
+            } else {
 #pragma unroll
             for (int j = 0; j < TM; j++)
 #pragma unroll
@@ -1053,31 +1480,30 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                     const uint32_t col = t + 4 * s;
                     if (col < mp && j < (int)c.nt) {
                         const float inv = s_inv[warp][col];
-                        const uint32_t a = part + ((warp * mp + col) * R + 16 * j + g) * 4;
+                        const uint32_t a = part + (warp * RS + col * R + 16 * j + g) * 4;
                         sts32(a, __float_as_uint((acc[j][s][0] + acc[j][s][1]) * inv));
                         sts32(a + 32, __float_as_uint((acc[j][s][2] + acc[j][s][3]) * inv));
                     }
                 }
+            }
             __syncwarp();
             if (lane == 0) mbar_arrive(&sync_bar[i & 1u]);
             if (i >= 1 && !add(i - 1, d1)) break;
             d2 = d1;
-            d1 = this_at;
+            d1 = i & 15u;
         }
         if (ok && i >= 1) ok = add(i - 1, d1);
         if (ok && ranks > 1 && i >= 2) ok = finish(i - 2, d2);
         if (ok && ranks > 1 && i >= 1) ok = finish(i - 1, d1);
-        // An infinite activation times codes and offset may cancel where the weight has a sign: results that are no numbers are formed
-        // again, weight by weight, each by the thread that stored it.  (Not on the way: the call costs the loop registers.)
-        if constexpr (NG != 0)
+        // An infinite activation has no digits, and its products with codes and offset may cancel where the weight has a sign: results that
+        // are no numbers are formed again, weight by weight, each by the thread that stored it.  (Not on the way: the call costs the loop registers.)
+        if constexpr (INT || NG != 0)
             if (ok && s_again) {
-                const uint32_t rows = ranks == 1 ? R : share;
-                for (uint32_t at = first, left = run; at < chunks; at++) {
-                    for (uint32_t q = tid; q < mp * rows; q += 256) again(at, q / rows, (ranks == 1 ? 0u : rank * share) + q % rows);
-                    if (--left == 0) {
-                        left = run;
-                        at += skip;
-                    }
+                const uint32_t rows = ranks == 1 ? R : share, per = INT && ranks == 1 ? 4u : 1u;   // (threads a result, the first of which stored it)
+                for (uint32_t at = first; tid % per == 0 && at < last;) {
+                    const SpChunk c = chunk(at);
+                    at += c.steps;
+                    for (uint32_t q = tid / per; q < mp * rows; q += 256 / per) again(c, q / rows, (ranks == 1 ? 0u : rank * share) + q % rows);
                 }
             }
     }
@@ -1103,7 +1529,7 @@ template <int T> inline size_t sp_tail(uint32_t ranks, uint32_t tr, uint32_t mp,
     const size_t r = 16u * tr;
     const size_t xf = (size_t)xunits * mp * 256, cc = SpTraits<T>::NG ? (((size_t)xunits * SpTraits<T>::NG * 4 + 16) * mp + 127) / 128 * 128 : 0;
     const size_t tab = SpTraits<T>::B256 == 272 || T == GT_Q4_0 ? 0 : (size_t)kSpWarps * r * 16;
-    const size_t red = (size_t)2 * kSpWarps * mp * r * 4, recv = ranks > 1 ? (size_t)4 * mp * r * 4 : 0;
+    const size_t red = (size_t)(mp <= 2 ? 4 * kSpWarps * (mp * r + 8) : 2 * kSpWarps * mp * r) * 4, recv = ranks > 1 ? (size_t)4 * mp * r * 4 : 0;
     if (b) {
         b->cc_off = b->xf_off + (uint32_t)xf;
         b->tab_off = b->cc_off + (uint32_t)cc;
@@ -1119,13 +1545,10 @@ template <int T, bool ALN, int MPC>
 static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, uint32_t tr, uint64_t entries, uint32_t xunits, int sm_count, cudaStream_t st) {
     const uint32_t STAGE = tr * 16 * sp_pitch<T>(ALN);
     bt.tr = tr;
-    uint32_t per = 0;   // chunks of an entry
-    for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].chunk_end = per += ((bt.op[i].n + 15) / 16 + tr - 1) / tr;
-    const uint64_t chunks = per * entries;
-    // one entry: neighbouring chunks go to different clusters; several: a contiguous share each, since a change of entry means other
-    // activations
-    bt.run = 1;
-    if (const char *e = exp_env("MLXN_SP_RUN")) bt.run = (uint32_t)atoi(e);
+    bt.step = bt.ids ? tr : 1u;
+    uint32_t per = 0;   // steps of an entry
+    for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].step_end = per += ((bt.op[i].n + 15) / 16 + bt.step - 1) / bt.step;
+    const uint64_t steps = per * entries;
     const size_t tail = sp_tail<T>(ranks, tr, bt.mp, xunits, nullptr);
     uint32_t nslots = (uint32_t)((kSpSmem - 128 - tail) / STAGE);
     if (nslots > (uint32_t)kSpMaxSlots) nslots = kSpMaxSlots;
@@ -1176,8 +1599,7 @@ static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, ui
         }
         ncl = f < ncl ? f : ncl;
     }
-    if (entries > 1) bt.run = 0;   // (counted on the device: only there the entries of a routed launch are known)
-    if (chunks < ncl) ncl = (uint32_t)chunks;
+    if (steps < ncl) ncl = (uint32_t)steps;
     cfg.gridDim = dim3(ncl * ranks);
     return cudaLaunchKernelEx(&cfg, kernel, bt, maps);
 }
@@ -1188,7 +1610,6 @@ struct SpPick {
     uint32_t ranks, tr;
 };
 template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool routed, uint64_t tiles, uint32_t max_units, int sm_count) {
-    const uint32_t sets = mp > 4 ? 2u : 1u;
     SpPick pick{0, 0};
     double best = 1e30;
     int force_c = 0, force_tr = 0;
@@ -1198,19 +1619,25 @@ template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool 
         const uint32_t slice = ((max_units + c - 1) / c + 3) / 4 * 4;
         // a rank without work: only where nothing smaller fits (K = 10304 with eight rows: seven slices of 24 units do, four of 44 do not)
         if (c > 1 && slice * (c - 1) >= max_units && pick.ranks) continue;
-        for (uint32_t tr = 1; tr <= (uint32_t)sp_tiles((int)sets); tr++) {
+        for (uint32_t tr = 1; tr <= (uint32_t)sp_tiles((int)mp); tr++) {
             if ((force_c && !routed && (int)c != force_c) || (force_tr && (int)tr != force_tr)) continue;
             const size_t stage = (size_t)tr * 16 * sp_pitch<T>(aln), tail = sp_tail<T>(c, tr, mp, (slice + 1) & ~1u, nullptr);
             if (tail + 2 * stage + 128 > kSpSmem) continue;
             const double slots = (double)((kSpSmem - 128 - tail) / stage);
-            const double ncl = (double)(2 * sm_count / (int)c), chunks = ceil(ceil((double)tiles / tr) / ncl);
-            // Fitted to 12288 x 4096 and 4096 x 4096, all types: a chunk takes 1.9 us of waits and sums whatever its size, plus
-            // 0.23 us per tile and unit of a warp (Q6_K 0.3; two sets of columns 1.5 times that, and there four ranks wait for
-            // one another for 4.5 us a chunk).  Of 27 products (three types, one, four and eight rows, 4096 x 4096, 12288 x 4096 and
-            // 4096 x 12288) timed at every geometry, 21 take the fastest this way and the others one within 8 percent of it.
-            const double unit = (T == GT_Q6_K ? 0.3 : 0.23) * (sets == 2 ? 1.5 : 1.0);
-            // One row: splitting it takes 0.27 us per unit of a warp and CTA.
-            const double cost = (packed ? 1.0 : 0.3 + 0.27 * ceil(slice / 8.0)) + chunks * ((sets == 2 && c == 4 ? 4.5 : 1.9) + tr * unit * ceil(slice / 8.0)) + (c > 1 ? 0.3 : 0.0) + (slots < 3 ? 0.3 : 0.0);
+            // Fitted to 1024, 4096 and 24576 x 4096 and 4096 x 12288, all types: a chunk costs waits and sums, a unit of a warp what a lone
+            // multiply takes to come through and a share per tile; ranks wait for one another, in f16 with eight rows for 4.5 us a chunk
+            // where there are four of them; one or two rows are split by every CTA.
+            const double ncl = (double)(2 * sm_count / (int)c), chunks = routed ? ceil(ceil((double)tiles / tr) / ncl) : ceil(ceil((double)tiles / ncl) / tr),
+                         share = routed ? chunks * tr : ceil((double)tiles / ncl), units = ceil(slice / 8.0);
+            double cost;
+            if (mp <= 2) {
+                const double tile = (T == GT_Q6_K ? 0.38 : T == GT_Q8_0 ? 0.35 : T == GT_Q4_0 ? 0.19 : 0.25) * (mp == 2 ? 1.3 : 1.0);
+                cost = (units > 8 ? 0.2 : 0.13) * units * mp + chunks * 0.5 + units * (chunks * 0.12 + share * tile) + (c == 1 ? 0.0 : c == 2 ? 0.8 : c == 4 ? 1.5 : 2.2);
+            } else {
+                const double tile = (T == GT_Q6_K ? 0.3 : 0.23) * (mp > 4 ? 1.5 : 1.0);
+                cost = (packed ? 1.0 : 0.3 + 0.27 * units) + chunks * (mp > 4 && c == 4 ? 4.5 : 1.9) + share * tile * units + (c > 1 ? 0.3 : 0.0);
+            }
+            if (slots < 3) cost += mp == 2 ? 1.0 : 0.3;
             if (cost < best) {
                 best = cost;
                 pick = {c, tr};
@@ -1239,16 +1666,19 @@ template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, 
     if (nops < 1 || nops > kSpMaxOps) return cudaErrorInvalidValue;
     const bool routed = ops[0].ids != nullptr;
     if (T == GT_Q5_K && !routed) return cudaErrorNotSupported;
-    bool aln = true;
+    bool aln = true, pairs = true;
     for (int i = 0; i < nops; i++) {
         const uint64_t rb = (uint64_t)(ops[i].k / BlockTraits<T>::QK) * BlockTraits<T>::BYTES;
-        aln = aln && rb % 16 == 0 && ((uintptr_t)ops[i].w & 15u) == 0 && (!routed || ops[i].expert_stride % 16 == 0);
+        const bool base = ((uintptr_t)ops[i].w & 15u) == 0 && (!routed || ops[i].expert_stride % 16 == 0);
+        aln = aln && rb % 16 == 0 && base;
+        pairs = pairs && rb % 16 == 8 && base && ops[i].n % 2 == 0;
     }
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return cudaErrorNotSupported;
     static thread_local SpBatch bt;
     alignas(64) static thread_local SpMaps maps;
     bt.nops = (uint32_t)nops;
+    bt.pairs = pairs;
     bt.ids = ops[0].ids;
     bt.npairs = routed ? ops[0].nprob : 0;
     bt.n_experts = routed ? ops[0].n_experts : 1;
@@ -1297,19 +1727,20 @@ template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, 
         if (!a.early_weights) bt.early_weights = 0;
         rows = a.m > rows ? a.m : rows;
         max_units = P.units > max_units ? P.units : max_units;
-        if (aln) {
-            const cuuint64_t dim[3] = {P.row_bytes / 8, a.n, routed ? a.n_experts : 1}, stride[2] = {P.row_bytes, routed ? a.expert_stride : (uint64_t)P.row_bytes * a.n};
-            const cuuint32_t box[3] = {sp_pitch<T>(true) / 8, 16, 1}, one[3] = {1, 1, 1};
+        if (aln || pairs) {
+            const uint64_t rb = (uint64_t)P.row_bytes * (pairs ? 2 : 1);
+            const cuuint64_t dim[3] = {rb / 8, pairs ? a.n / 2 : a.n, routed ? a.n_experts : 1}, stride[2] = {rb, routed ? a.expert_stride : (uint64_t)P.row_bytes * a.n};
+            const cuuint32_t box[3] = {sp_pitch<T>(aln) / 8, pairs ? 8u : 16u, 1}, one[3] = {1, 1, 1};
             if (enc(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<uint8_t *>(a.w), dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return cudaErrorInvalidValue;
         }
     }
     // rows of an entry: dense, as many as fit two sets of columns; routed, one set (most experts have few rows)
-    bt.mp = routed ? (ops[0].nprob <= 1 ? 1u : 4u) : rows <= 1 ? 1u : rows <= 2 ? 2u : rows <= 4 ? 4u : 8u;
+    bt.mp = routed ? ((ops[0].nprob <= 1 ? 1u : 4u)) : rows <= 1 ? 1u : rows <= 2 ? 2u : rows <= 4 ? 4u : 8u;
     bt.nent = routed ? 0u : (rows + bt.mp - 1) / bt.mp;
     const uint64_t entries = routed ? ops[0].nprob : bt.nent, all = tiles * entries;
-    bt.packed = !routed && bt.mp > 1;
+    bt.packed = !routed && bt.mp > 2;
     *launches = 1;
     auto go = [&](auto ALN) {
         constexpr bool A = decltype(ALN)::value;
@@ -1323,7 +1754,13 @@ template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, 
             }
             if (bt.mp > 4) return sp_choose<T, A, 8>(bt, maps, all, entries, max_units, routed, sm_count, st);
         }
-        if (bt.mp == 1) return sp_choose<T, A, 1>(bt, maps, all, entries, max_units, routed, sm_count, st);
+        // (Routed rows are always summed in f16, so that a pair's sum does not depend on the pairs that travel with it: rows that share an
+        // expert gain more from one pass over its codes than from integers.  Q4_0, 768 x 2048, 256 pairs of 16 experts 35.6 us, with two rows a
+        // pass in integers 47.6; 8 pairs of 128 experts 11.0, in integers 8.7.)
+        if constexpr (T != GT_Q5_K) {
+            if (!routed && bt.mp == 2) return sp_choose<T, A, 2>(bt, maps, all, entries, max_units, false, sm_count, st);
+            if (!routed && bt.mp == 1) return sp_choose<T, A, 1>(bt, maps, all, entries, max_units, false, sm_count, st);
+        }
         return sp_choose<T, A, 4>(bt, maps, all, entries, max_units, routed, sm_count, st);
     };
     if (aln) return go(std::true_type{});

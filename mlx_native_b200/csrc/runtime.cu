@@ -1067,7 +1067,7 @@ static int encoder_flush_pending(mlxn_encoder *e, bool group_ends) {
     // it; not where the group has other operations, which run meanwhile and fill what the register-level kernel leaves idle (32 independent
     // mat-vecs of both 8- and 6-bit types: 0.345 ms where these count as a batch like others, 0.328 so).
     bool split = e->pend_split;
-    if (!split && whole_group && opt_qmv() == 3 && !a0.ids && !e->pend_pair && e->pend.size() <= kMvSplitMax) {
+    if (!split && whole_group && opt_qmv() == 3 && !a0.ids && (!e->pend_pair || a0.m <= 2) && e->pend.size() <= kMvSplitMax) {
         split = qmv_split_pays(e->pend_type, e->pend.data(), (int)e->pend.size(),
                                qmv_mma_fill(e->pend_type, e->pend.data(), (int)e->pend.size(), e->dev->sm_count));
         for (const QmvArgs &a : e->pend)

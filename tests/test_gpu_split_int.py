@@ -1,0 +1,65 @@
+"""One and two activation rows on the split mat-vec (csrc/qmv_split.cuh: codes and activation digits as 8-bit integers), against the oracle."""
+import numpy as np
+import pytest
+
+import mlx_native_b200 as mx
+from oracle import oracle as orc
+from tests.gpu_util import MV_TOL, TYPES, Ctx, norm_err, normal_acts, normal_weights
+
+pytestmark = pytest.mark.gpu
+ALL = dict(TYPES, Q4_K=(mx.GgmlType.Q4_K, orc.Q4_K))
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    mx.set_option("qmv", "split")
+    yield Ctx()
+    mx.set_option("qmv", "auto")
+
+
+# every other row on a 16-byte boundary (tensor copies of the even and the odd rows) with an even and an odd number of rows, which leaves row
+# copies; chunks of one to four tiles, a share that crosses from one chunk to the next, ranks without units, K of one unit and of half a unit
+@pytest.mark.parametrize("tname,n,k", [("Q4_0", 50, 2176), ("Q4_0", 51, 2176), ("Q8_0", 34, 640), ("Q8_0", 33, 640), ("Q6_K", 70, 5120),
+                                       ("Q6_K", 4802, 1024), ("Q4_0", 6144, 256), ("Q4_0", 10000, 512), ("Q8_0", 9520, 256), ("Q6_K", 24000, 512),
+                                       ("Q4_K", 15000, 256), ("Q4_0", 33, 64), ("Q8_0", 17, 32), ("Q4_K", 96, 9216)])
+@pytest.mark.parametrize("m", [1, 2])
+def test_shapes(ctx, tname, n, k, m):
+    gtype, otype = ALL[tname]
+    wq = normal_weights(n + k, n, k, otype)
+    x = normal_acts(n + m, m, k)
+    y = ctx.matmul(gtype, wq, x, n, k)
+    assert mx.last_kernel_name() == "qmv_split"
+    y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8)
+    assert norm_err(y, y_ref, ad) <= MV_TOL
+    assert np.array_equal(y.view(np.uint32), ctx.matmul(gtype, wq, x, n, k).view(np.uint32))
+
+
+# Products of codes and digits and the sums of a block are exact; digits leave out less than 2^-29 of the largest activation of a warp's share, which
+# for normal activations is 2^-27 of one, and the f32 sums of a result have at most a few dozen terms one after another: 1.5e-7 (2^-23 = 1.2e-7).
+@pytest.mark.parametrize("tname", sorted(ALL))
+@pytest.mark.parametrize("outliers", [False, True])
+def test_error_against_64_bits(ctx, tname, outliers):
+    gtype, otype = ALL[tname]
+    n, k = 700, 4096
+    wq = normal_weights(n, n, k, otype)
+    w = orc.dequantize(otype, wq).reshape(n, k).astype(np.float64)
+    for m in (1, 2):
+        x = normal_acts(m, m, k)
+        if outliers:
+            x[:, ::97] *= 300
+        y, ref = ctx.matmul(gtype, wq, x, n, k), x.astype(np.float64) @ w.T
+        assert np.linalg.norm(y - ref) <= 1.5e-7 * np.linalg.norm(ref)
+
+
+def test_zero_and_tiny_rows(ctx):
+    """A row of zeros, of the smallest numbers there are, and one of them among zeros: the scale takes two powers of two."""
+    gtype, otype = TYPES["Q8_0"]
+    n, k = 40, 1024
+    wq = normal_weights(3, n, k, otype)
+    w = orc.dequantize(otype, wq).reshape(n, k).astype(np.float64)
+    x = np.zeros((3, k), np.float32)
+    x[1] = normal_acts(1, 1, k) * np.float32(1e-37)
+    x[2, 100] = np.float32(1e-36)
+    for row in x:
+        y, ref = ctx.matmul(gtype, wq, row[None], n, k)[0], w @ row.astype(np.float64)
+        assert np.all(np.abs(y - ref) <= 1e-6 * np.abs(ref).max() + 3e-45)
