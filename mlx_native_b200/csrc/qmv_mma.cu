@@ -83,6 +83,7 @@ __host__ __device__ constexpr uint32_t mw_pitch(int ggml_type, int kb) {
 }
 
 constexpr int kMwMaxProbs = 16;    // mat-vecs one launch can carry
+constexpr int kMwFewProbs = 3;     // ... with parameters below 4 KB, beyond which a launch costs the host 7.0 us instead of 4.5
 constexpr int kMwMaxGrid = 320;    // CTAs of a launch (two per SM)
 
 // One mat-vec of a launch.  A launch carries up to kMwMaxProbs mat-vecs that have no buffer conflicts with one
@@ -100,8 +101,8 @@ struct MwProb {
     uint32_t n_peer;      // row-sharded form (see QmvArgs): the other ranks' result buffers
     float *y_peer[kMaxPeers];
 };
-struct MwBatch {
-    MwProb p[kMwMaxProbs];
+template <int N> struct MwBatch {
+    MwProb p[N];
     uint32_t nprob;
     uint32_t early_weights;   // no problem's weights were written by a kernel of this process (see QmvArgs)
     uint32_t *status;
@@ -114,12 +115,25 @@ struct MwBatch {
     uint32_t dep_mask;
     uint32_t *bar;
     uint32_t routed;          // some problem is expert-routed: the expert ids are read once the kernels ahead are done
-    // CTA c works on items [cta_begin[c], cta_begin[c + 1]): contiguous chunks of (nearly) equal numbers of stages
-    uint32_t cta_begin[kMwMaxGrid + 1];
+    uint32_t stages_q, stages_r;   // stages of all problems over the CTAs: quotient and remainder
 };
-struct MwMaps {
-    CUtensorMap m[kMwMaxProbs];
+template <int N> struct MwMaps {
+    CUtensorMap m[N];
 };
+// The first item of CTA c: contiguous chunks of (nearly) equal numbers of stages, c starts at the first item whose stages begin at or after
+// c / CTAs of them all.
+template <int N> __device__ __forceinline__ uint32_t mw_begin(const MwBatch<N> &b, uint32_t c, uint32_t ctas) {
+    if (c == 0) return 0;
+    if (c == ctas) return b.nitems;
+    const uint32_t target = b.stages_q * c + b.stages_r * c / ctas;
+    uint32_t p = 0, before = 0, from = b.p[0].item0;
+    for (;; p++) {
+        const uint32_t to = p + 1 < b.nprob ? b.p[p + 1].item0 : b.nitems, all = (to - from) * b.p[p].spi;
+        if (p + 1 == b.nprob || before + all > target) return from + min((target - before + b.p[p].spi - 1) / b.p[p].spi, to - from);
+        before += all;
+        from = to;
+    }
+}
 
 struct MwCfg {
 #ifdef MLXN_EXPERIMENTS
@@ -270,9 +284,9 @@ __device__ __forceinline__ void mw_pair_tiles(uint32_t base, uint32_t base2, uin
 // map's rows are PAIRS of weight rows; a stage is two copies of R / 2 map rows, the even weight rows into stage rows
 // [0, R / 2) and the odd ones into [R / 2, R), each from the 16-byte boundary below its first byte (the odd rows'
 // data therefore starts 8 bytes further into its chunk than the even rows').
-template <int T, int TPW, int KB, int MP, bool PAIR>
+template <int T, int TPW, int KB, int MP, bool PAIR, int N>
 __global__ void __launch_bounds__(kMwThreads, 2)
-    qmv_mma_kernel(const __grid_constant__ MwBatch bt, const MwCfg c, const __grid_constant__ MwMaps maps) {
+    qmv_mma_kernel(const __grid_constant__ MwBatch<N> bt, const MwCfg c, const __grid_constant__ MwMaps<N> maps) {
     using TR = MwTraits<T>;
     constexpr int R = 16 * TPW, NG = TR::NG, NM = TR::NM;
     constexpr int NS = MP > 4 ? 2 : 1;                       // sets of four activation rows
@@ -305,7 +319,6 @@ __global__ void __launch_bounds__(kMwThreads, 2)
     __shared__ volatile uint32_t abort_flag;
 
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t g0 = bt.cta_begin[blockIdx.x], g1 = bt.cta_begin[blockIdx.x + 1];   // this CTA's items
 
     if (tid == 0) {
         abort_flag = 0;
@@ -325,6 +338,7 @@ __global__ void __launch_bounds__(kMwThreads, 2)
             s_lo[p2] = (uint32_t)(((uint64_t)blockIdx.x * (e - b)) / gridDim.x);
             s_hi[p2] = (uint32_t)(((uint64_t)(blockIdx.x + 1) * (e - b)) / gridDim.x);
         } else {             // one contiguous chunk of the launch's item list
+            const uint32_t g0 = mw_begin(bt, blockIdx.x, gridDim.x), g1 = mw_begin(bt, blockIdx.x + 1, gridDim.x);
             s_lo[p2] = max(g0, b) - b;
             s_hi[p2] = max(min(g1, e), max(g0, b)) - b;
         }
@@ -1023,8 +1037,8 @@ bool qmv_mma_supported_routed(int ggml_type, const QmvArgs &a) {
 
 static inline size_t mw_align(size_t v, size_t al) { return (v + al - 1) / al * al; }
 
-template <int T, int TPW, int KB, int MP, bool PAIR>
-static cudaError_t launch_mw(const QmvArgs *ops, int nops, int sm_count, int ctas_per_sm, cudaStream_t st) {
+template <int T, int TPW, int KB, int MP, bool PAIR, int N>
+static cudaError_t launch_mw_n(const QmvArgs *ops, int nops, int sm_count, int ctas_per_sm, cudaStream_t st) {
     using TR = MwTraits<T>;
     constexpr uint32_t R = 16 * TPW, PITCH = mw_pitch(T, KB), STAGE = mw_halves(T, KB) * R * PITCH;
     constexpr uint32_t PIECES = KB * MP * TR::NM * 4, NB = PIECES >= 32 ? 1 : 32 / PIECES;
@@ -1050,9 +1064,9 @@ static cudaError_t launch_mw(const QmvArgs *ops, int nops, int sm_count, int cta
 
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return cudaErrorNotSupported;
-    if (nops < 1 || nops > kMwMaxProbs) return cudaErrorInvalidValue;
-    static thread_local MwBatch bt;      // too large for the stack of a deep call chain; one launch at a time per thread
-    alignas(64) static thread_local MwMaps maps;
+    if (nops < 1 || nops > N) return cudaErrorInvalidValue;
+    static thread_local MwBatch<N> bt;      // too large for the stack of a deep call chain; one launch at a time per thread
+    alignas(64) static thread_local MwMaps<N> maps;
     bt.nprob = (uint32_t)nops;
     bt.early_weights = 1;
     bt.routed = 0;
@@ -1116,7 +1130,7 @@ static cudaError_t launch_mw(const QmvArgs *ops, int nops, int sm_count, int cta
         if (its > max_items) max_items = its;
     }
     if (bt.dep_mask && !bt.bar) return cudaErrorInvalidValue;
-    for (int i = nops; i < kMwMaxProbs; i++) {
+    for (int i = nops; i < N; i++) {
         bt.p[i] = MwProb{};
         bt.p[i].item0 = items;
         maps.m[i] = maps.m[0];
@@ -1124,40 +1138,26 @@ static cudaError_t launch_mw(const QmvArgs *ops, int nops, int sm_count, int cta
     uint32_t grid = (uint32_t)(sm_count * ctas_per_sm);
     if (grid > (uint32_t)kMwMaxGrid) grid = kMwMaxGrid;
     if (grid > (bt.dep_mask ? max_items : items)) grid = bt.dep_mask ? max_items : items;
-    // contiguous chunks of items holding (nearly) the same number of stages each: CTA c starts at the first item whose
-    // stages begin at or after c / grid of all the launch's stages
-    {
-        uint32_t pi = 0;
-        uint64_t before = 0;   // stages of the problems ahead of pi
-        for (uint32_t cta = 0; cta <= grid; cta++) {
-            const uint64_t target = total_stages * cta / grid;
-            while (pi + 1 < (uint32_t)nops) {
-                const uint64_t its = bt.p[pi + 1].item0 - bt.p[pi].item0;
-                if (before + its * bt.p[pi].spi > target) break;
-                before += its * bt.p[pi].spi;
-                pi++;
-            }
-            const uint64_t its_p = (pi + 1 < (uint32_t)nops ? bt.p[pi + 1].item0 : items) - bt.p[pi].item0;
-            uint64_t in = (target - before + bt.p[pi].spi - 1) / bt.p[pi].spi;
-            if (in > its_p) in = its_p;
-            bt.cta_begin[cta] = bt.p[pi].item0 + (uint32_t)in;
-        }
-        bt.cta_begin[0] = 0;
-        bt.cta_begin[grid] = items;
-        for (uint32_t cta = grid + 1; cta <= (uint32_t)kMwMaxGrid; cta++) bt.cta_begin[cta] = items;
-    }
+    bt.stages_q = (uint32_t)(total_stages / grid);
+    bt.stages_r = (uint32_t)(total_stages % grid);
     static size_t attr_smem[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (smem > attr_smem[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(qmv_mma_kernel<T, TPW, KB, MP, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(qmv_mma_kernel<T, TPW, KB, MP, PAIR, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         attr_smem[dev] = smem;
     }
     if (bt.dep_mask)   // its CTAs wait on one another: all of them resident at once, or the launch is refused
-        return launch_cooperative(qmv_mma_kernel<T, TPW, KB, MP, PAIR>, dim3(grid), dim3(kMwThreads), smem, st, bt, c, maps);
-    return launch_overlapped(qmv_mma_kernel<T, TPW, KB, MP, PAIR>, dim3(grid), dim3(kMwThreads), smem, st, bt, c, maps);
+        return launch_cooperative(qmv_mma_kernel<T, TPW, KB, MP, PAIR, N>, dim3(grid), dim3(kMwThreads), smem, st, bt, c, maps);
+    return launch_overlapped(qmv_mma_kernel<T, TPW, KB, MP, PAIR, N>, dim3(grid), dim3(kMwThreads), smem, st, bt, c, maps);
+}
+
+template <int T, int TPW, int KB, int MP, bool PAIR>
+static cudaError_t launch_mw(const QmvArgs *ops, int nops, int sm_count, int ctas_per_sm, cudaStream_t st) {
+    if (nops <= kMwFewProbs) return launch_mw_n<T, TPW, KB, MP, PAIR, kMwFewProbs>(ops, nops, sm_count, ctas_per_sm, st);
+    return launch_mw_n<T, TPW, KB, MP, PAIR, kMwMaxProbs>(ops, nops, sm_count, ctas_per_sm, st);
 }
 
 // (TPW, KB): a warp works on TPW x KB tile-units per stage.  Few weight rows -> narrow row groups and long K stages.
