@@ -216,16 +216,17 @@ template <int T, int S4> __device__ __forceinline__ void dequant64_aligned(uint3
 // Q6_K: 64 elements (half h's runs 2 q and 2 q + 1) of the super-block that starts PRE bytes into the row's aligned stage.  The two runs
 // have the same 32 bytes of high bits, and their 64 bytes of low bits follow one another.  A code is put beside 1024 in f16, widened, and scaled
 // two at a time: fma(1024 + u, ds, -1056 ds) = ds (u - 32), exact in f32 (ds has at most 18 significant bits), then rounded once to f16.
-template <int PRE> __device__ __forceinline__ void dequant64_q6k_aligned(uint32_t stage_row, uint32_t h, uint32_t q, uint32_t (&out)[32]) {
+// field(o, w): the 32 bytes at byte o of the super-block; rest: shared address of the super-block (its last 18 bytes are scales and d).
+template <class F> __device__ __forceinline__ void dequant64_q6k(F &&field, uint32_t rest, uint32_t h, uint32_t q, uint32_t (&out)[32]) {
     uint32_t H[8];
-    lds_field<PRE, 8>(stage_row + 128 + 32 * h, H);
-    const float d = half_bits_to_float(lds_u16(stage_row + PRE + 208));
-    const uint32_t sc[2] = {lds_u16(stage_row + PRE + 192 + 8 * h + 4 * q), lds_u16(stage_row + PRE + 194 + 8 * h + 4 * q)};
+    field(128 + 32 * h, H);
+    const float d = half_bits_to_float(lds_u16(rest + 208));
+    const uint32_t sc[2] = {lds_u16(rest + 192 + 8 * h + 4 * q), lds_u16(rest + 194 + 8 * h + 4 * q)};
     const uint32_t ash = 4 * q;
 #pragma unroll
     for (int g = 0; g < 2; g++) {
         uint32_t A[8];
-        lds_field<PRE, 8>(stage_row + 64 * h + 32 * g, A);
+        field(64 * h + 32 * g, A);
         const uint32_t rot = (4u - 4 * q - 2 * g) & 31u;   // brings a byte's two bits to bits 4 and 5
 #pragma unroll
         for (int j = 0; j < 8; j++) {
@@ -243,6 +244,25 @@ template <int PRE> __device__ __forceinline__ void dequant64_q6k_aligned(uint32_
         }
     }
 }
+template <int PRE> __device__ __forceinline__ void dequant64_q6k_aligned(uint32_t stage_row, uint32_t h, uint32_t q, uint32_t (&out)[32]) {
+    dequant64_q6k([&](uint32_t o, uint32_t (&w)[8]) { lds_field<PRE, 8>(stage_row + o, w); }, stage_row + PRE, h, q, out);
+}
+// The same for a super-block at any even address, which may differ from lane to lane: 8-byte loads, of which a select takes the words and a
+// shift the halves.  (For rows that are neighbours in shared memory, an odd multiple of 16 bytes apart: there a load of 4 bytes a lane takes as many
+// passes as one of 8.)
+__device__ __forceinline__ void dequant64_q6k_any(uint32_t seg, uint32_t h, uint32_t q, uint32_t (&out)[32]) {
+    const bool odd = (seg & 4u) != 0;
+    const uint32_t sh = (seg & 2u) * 8u, base = seg & ~7u;
+    dequant64_q6k([&](uint32_t o, uint32_t (&w)[8]) {   // (o is a multiple of 32)
+        uint32_t W[10];
+#pragma unroll
+        for (int i = 0; i < 5; i++) lds64(base + o + 8 * i, W[2 * i], W[2 * i + 1]);
+#pragma unroll
+        for (int i = 0; i < 9; i++) W[i] = odd ? W[i + 1] : W[i];
+#pragma unroll
+        for (int i = 0; i < 8; i++) w[i] = __funnelshift_r(W[i], W[i + 1], sh);
+    }, seg, h, q, out);
+}
 __device__ __forceinline__ void dequant64_q6k_aligned_p(uint32_t p8, uint32_t stage_row, uint32_t h, uint32_t q, uint32_t (&out)[32]) {
     switch (p8) {  // uniform over the CTA
     case 0: dequant64_q6k_aligned<0>(stage_row, h, q, out); break;
@@ -253,6 +273,36 @@ __device__ __forceinline__ void dequant64_q6k_aligned_p(uint32_t p8, uint32_t st
     case 5: dequant64_q6k_aligned<10>(stage_row, h, q, out); break;
     case 6: dequant64_q6k_aligned<12>(stage_row, h, q, out); break;
     default: dequant64_q6k_aligned<14>(stage_row, h, q, out); break;
+    }
+}
+
+// Q4_K: sub-block j (32 elements) of the super-block at a 16-byte boundary, as dequant32 forms it, by 16-byte loads.
+__device__ __forceinline__ void dequant32_q4k_aligned(uint32_t o, uint32_t j, uint32_t *out /*16 words*/) {
+    uint32_t dd, s0, s1, s2, Q[8];
+    lds128(o, dd, s0, s1, s2);
+    lds128(o + 16 + 32 * (j >> 1), Q[0], Q[1], Q[2], Q[3]);
+    lds128(o + 32 + 32 * (j >> 1), Q[4], Q[5], Q[6], Q[7]);
+    uint32_t sc, mn;
+    if (j < 4) {
+        sc = (s0 >> (8 * j)) & 63u;
+        mn = (s1 >> (8 * j)) & 63u;
+    } else {
+        const uint32_t sh = 8 * (j - 4);
+        sc = ((s2 >> sh) & 15u) | ((((s0 >> sh) >> 6) & 3u) << 4);
+        mn = (((s2 >> sh) >> 4) & 15u) | ((((s1 >> sh) >> 6) & 3u) << 4);
+    }
+    const float ds = half_bits_to_float(dd & 0xFFFFu) * (float)sc, dm = half_bits_to_float(dd >> 16) * (float)mn;
+    const float c = fmaf(-128.0f, ds, -dm);
+    const uint32_t ash = (j & 1u) ? 4u : 0u;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t u = (Q[i] >> ash) & 0x0F0F0F0Fu;
+        const float f0 = fmaf(__uint_as_float(__byte_perm(u, 0x43000000u, 0x7044)), ds, c);
+        const float f1 = fmaf(__uint_as_float(__byte_perm(u, 0x43000000u, 0x7144)), ds, c);
+        const float f2 = fmaf(__uint_as_float(__byte_perm(u, 0x43000000u, 0x7244)), ds, c);
+        const float f3 = fmaf(__uint_as_float(__byte_perm(u, 0x43000000u, 0x7344)), ds, c);
+        out[2 * i] = h2_as_u32(__floats2half2_rn(f0, f1));
+        out[2 * i + 1] = h2_as_u32(__floats2half2_rn(f2, f3));
     }
 }
 

@@ -141,7 +141,8 @@ __device__ __forceinline__ void commit_both(uint64_t *bar) {
 // ROUTED: the products of a mixture of experts.  The tiles are those of the list that build_tiles_kernel made, 64 rows of one expert each,
 // packed whole (a CTA's half are rows 0..31 or 32..63 of each 64-column chunk); the weights' map has the expert as third dimension.
 // RING: K stages of weights in tensor memory, 64 columns each.  The accumulators have what is left: two of 129 to 192 columns leave two stages.
-template <int T, bool ROUTED, uint32_t RING>
+// RAW: weight rows lie in tensor memory as in a raw stage (see row_of).
+template <int T, bool ROUTED, uint32_t RING, bool RAW>
 __global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at most 80 registers: a block of the packing kernel fits beside a CTA)
     qmm_duo_kernel(const QmmArgs a, const __grid_constant__ DuoCfg c, const __grid_constant__ DuoMaps wmaps) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
@@ -217,9 +218,14 @@ __global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at mos
     constexpr uint32_t kSpin = 0xFFFFFFFFu;
     bool ok = true;
 
+    // The weight row (of the CTA's 128) in tensor-memory lane p.  RAW, for Q6_K whose rows do not all start on 16-byte boundaries: as in a raw stage,
+    // those that start alike one after another, so that a warp's rows are neighbours in shared memory and, with two ways to start, start
+    // alike (in the matrix's order every second, fourth or eighth row of a warp meets in the same banks, and extraction is by 4-byte loads).
+    auto row_of = [&](uint32_t p) { return RAW ? ((p & ((128u >> c.row_group) - 1u)) << c.row_group) + (p >> (7 - c.row_group)) : p; };
+
     // The read-back of the pair's `nitem`-th item, by group g of four warps: lane = weight row, 32 activation rows at a time, the groups in turn.
     auto read_back = [&](const Item &it, uint32_t nitem, uint32_t q4, uint32_t g) {
-        const uint32_t buf = accs == 2 ? nitem & 1u : 0u, turn = accs == 2 ? nitem >> 1 : nitem, n = c.out.n[it.op], rr = q4 * 32 + lane;
+        const uint32_t buf = accs == 2 ? nitem & 1u : 0u, turn = accs == 2 ? nitem >> 1 : nitem, n = c.out.n[it.op], rr = row_of(q4 * 32 + lane);
         const bool row_ok = it.n0 + rr < n;
         int32_t mine[2] = {-1, -1};   // ROUTED: the output rows of activation rows lane and 32 + lane of the tile
         if constexpr (ROUTED) {
@@ -387,10 +393,10 @@ __global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at mos
             }
         }
     } else if (warp >= 4 && warp < 4 + kDuoDequantWarps) {
-        // thread (warp w, lane l) of a set owns weight row 32 (w % 4) + l, the tensor-memory lane it may address, and the 64-element half
+        // thread (warp w, lane l) of a set owns the weight row of lane 32 (w % 4) + l, the tensor-memory lane it may address, and the 64-element half
         // (w / 4) % 2 of the K stage: 32 packed f16 pairs = one 32-column store
         const uint32_t dw = warp - 4, q4 = dw & 3u, half = (dw >> 2) & 1u, set = dw >> 3;
-        const uint32_t rr = q4 * 32 + lane;
+        const uint32_t rr = row_of(q4 * 32 + lane);
         const uint32_t srow = ((rr & ((1u << c.row_group) - 1u)) << (7 - c.row_group)) + (rr >> c.row_group);   // the row's place in a raw stage
         const uint32_t a_dst = tmem + ((q4 * 32) << 16) + kDuoCols - kDuoACols + 32 * half;
         const uint32_t row_bytes = (a.k / QK) * BB;
@@ -410,10 +416,13 @@ __global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at mos
                     const uint32_t J = J0 + st, sa = J % kDuoStages, before = J - RING;   // (J: the stage's number in the pair's whole run)
                     const uint32_t r_abs = it.r_lo + r, stage_row = smem_base + c.raw_off + rs * raw_bytes + srow * c.seg_stride;
                     uint32_t regs[32];
-                    if (T != GT_Q4_K && c.aligned && row_ok) {   // (Q4_K: the generic extraction below)
-                        if constexpr (T == GT_Q6_K) {
+                    if (!RAW && c.aligned && row_ok) {
+                        if constexpr (T == GT_Q4_K) {
+                            dequant32_q4k_aligned(stage_row, 4 * set + 2 * half, regs);
+                            dequant32_q4k_aligned(stage_row, 4 * set + 2 * half + 1, regs + 16);
+                        } else if constexpr (T == GT_Q6_K) {
                             dequant64_q6k_aligned_p(r_abs & 7u, stage_row, set, half, regs);
-                        } else if constexpr (T != GT_Q4_K) {
+                        } else {
                             switch (2 * set + half) {  // uniform per warp
                             case 0: dequant64_aligned<T, 0>(stage_row, regs); break;
                             case 1: dequant64_aligned<T, 1>(stage_row, regs); break;
@@ -421,6 +430,10 @@ __global__ void __launch_bounds__(768, 1) __cluster_dims__(2, 1, 1)   // (at mos
                             default: dequant64_aligned<T, 3>(stage_row, regs); break;
                             }
                         }
+                    } else if constexpr (RAW) {
+                        // (With four ways to start a warp's rows start alike too, but then four of the eight versions take turns: 1024 x 2560 160 us, so 128.)
+                        if (c.row_group < 2) dequant64_q6k_aligned_p((row_lo4 + r_abs * BB) >> 1 & 7u, stage_row, set, half, regs);
+                        else dequant64_q6k_any(stage_row + ((row_lo4 + r_abs * BB) & 15u), set, half, regs);
                     } else {
                         const uint32_t seg = stage_row + ((row_lo4 + ((r_abs * KR) / QK) * BB) & 15u);
 #pragma unroll
@@ -509,8 +522,8 @@ static uint32_t duo_pairs() {
         cfg.gridDim = dim3(most * 2);
         cfg.blockDim = dim3(duo_threads(false));
         cfg.dynamicSmemBytes = 223 * 1024;
-        if (cudaFuncSetAttribute(qmm_duo_kernel<GT_Q4_0, false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, qmm_duo_kernel<GT_Q4_0, false, 4>, &cfg) != cudaSuccess || n < 1 || n > (int)most) {
+        if (cudaFuncSetAttribute(qmm_duo_kernel<GT_Q4_0, false, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, qmm_duo_kernel<GT_Q4_0, false, 4, false>, &cfg) != cudaSuccess || n < 1 || n > (int)most) {
             (void)cudaGetLastError();
             n = (int)most;
         }
@@ -566,8 +579,16 @@ uint64_t qmm_duo_cost(int ggml_type, const QmmArgs &a, uint32_t nt, uint32_t lim
     return duo_plan(ggml_type, a.m, a.n, a.k, nt, limit, p);
 }
 
+// Whether the rows go to tensor memory in the raw stages' order (RAW).  Results are then written with a stride: that pays where it is two rows (1024 x
+// 4096 x 5120, 49.0 -> 44.4 us) and in routed products, whose read-back has warps of its own (512 tokens, 128 experts, 2048 x 768 95.7 -> 88.2, 1024 x 2560
+// 141 -> 128), not with four or eight (2048 x 4096 x 2560: 52.4 -> 55.1), nor where results are added to another pair's (333 x 4096 x 4352: 29 -> 34).
+static bool duo_raw_order(int ggml_type, uint32_t k, bool routed, bool shared) {
+    const int g = duo_row_group((k / ggml_qk(ggml_type)) * ggml_block_bytes(ggml_type));
+    return ggml_type == GT_Q6_K && g != 0 && (routed || (g == 1 && !shared));
+}
+
 // Maps, rings and launch.  `c`: tiles, products and pairs are filled in.
-template <int T, bool ROUTED, uint32_t RING> static cudaError_t duo_launch(DuoCfg &c, const QmmArgs *ops, int nops, const uint8_t *xpack, cudaStream_t st, int *launches) {
+template <int T, bool ROUTED, uint32_t RING, bool RAW> static cudaError_t duo_launch(DuoCfg &c, const QmmArgs *ops, int nops, const uint8_t *xpack, cudaStream_t st, int *launches) {
     constexpr int QK = BlockTraits<T>::QK, BB = BlockTraits<T>::BYTES;
     const QmmArgs &a = ops[0];
     const uint32_t row_bytes = (a.k / QK) * BB;
@@ -608,13 +629,13 @@ template <int T, bool ROUTED, uint32_t RING> static cudaError_t duo_launch(DuoCf
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!prepared[dev].load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(qmm_duo_kernel<T, ROUTED, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024);
+        const cudaError_t e = cudaFuncSetAttribute(qmm_duo_kernel<T, ROUTED, RING, RAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024);
         if (e != cudaSuccess) return e;
         prepared[dev].store(1, std::memory_order_release);
     }
     (*launches)++;
     note_mat_mat(ROUTED ? "qmm_duo_id" : "qmm_duo", c.nt);
-    return launch_overlapped(qmm_duo_kernel<T, ROUTED, RING>, dim3(2 * c.pairs), dim3(duo_threads(ROUTED)), smem, st, a, c, wmaps);
+    return launch_overlapped(qmm_duo_kernel<T, ROUTED, RING, RAW>, dim3(2 * c.pairs), dim3(duo_threads(ROUTED)), smem, st, a, c, wmaps);
 }
 
 // `ops`: products of the same activations
@@ -644,8 +665,11 @@ static cudaError_t launch_duo_t(const QmmArgs *ops, int nops, uint32_t nt, uint3
     (*launches)++;
     const cudaError_t e = launch_overlapped(pack_x_kernel<false>, dim3((unsigned)slices, lanes), dim3(256), 0, st, a, xpack, nchunks, h, c.share, c.out);
     if (e != cudaSuccess) return e;
-    return kDuoCols - c.accs * nt >= 4 * kDuoACols ? duo_launch<T, false, 4>(c, ops, nops, xpack, st, launches)
-                                                   : duo_launch<T, false, 2>(c, ops, nops, xpack, st, launches);
+    const bool deep = kDuoCols - c.accs * nt >= 4 * kDuoACols;
+    if constexpr (T == GT_Q6_K)
+        if (duo_raw_order(T, a.k, false, p.shared))
+            return deep ? duo_launch<T, false, 4, true>(c, ops, nops, xpack, st, launches) : duo_launch<T, false, 2, true>(c, ops, nops, xpack, st, launches);
+    return deep ? duo_launch<T, false, 4, false>(c, ops, nops, xpack, st, launches) : duo_launch<T, false, 2, false>(c, ops, nops, xpack, st, launches);
 }
 
 template <int T> static cudaError_t launch_duo_routed_t(const QmmArgs &a, uint32_t tiles, const uint8_t *xpack, cudaStream_t st, int *launches) {
@@ -661,7 +685,9 @@ template <int T> static cudaError_t launch_duo_routed_t(const QmmArgs &a, uint32
     c.pairs = items < duo_pairs() ? (uint32_t)items : duo_pairs();
     c.beside = (a.reuse & 4u) != 0;
     if (!c.pairs) return cudaSuccess;
-    return duo_launch<T, true, 4>(c, &a, 1, xpack, st, launches);
+    if constexpr (T == GT_Q6_K)
+        if (duo_raw_order(T, a.k, true, false)) return duo_launch<T, true, 4, true>(c, &a, 1, xpack, st, launches);
+    return duo_launch<T, true, 4, false>(c, &a, 1, xpack, st, launches);
 }
 
 // `tiles`: bound of the list's length; `xpack`: what the list's tiles hold
