@@ -671,8 +671,9 @@ template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const 
 // The tiles of all entries and ops form one line, of which every cluster takes an equal contiguous share, in steps.  A chunk: the next tiles of
 // the share, `nt` of op `op` for entry `ent` from the op's tile `tile` on; what is left of an op is cut into chunks of equal length.  Dense:
 // steps of one tile (shares of whole chunks of four leave a last round part empty: Q4_0 24576 x 4096 has 384 such chunks for 296 CTAs, or 1536
-// tiles).  Routed: steps of a chunk (a share that crosses into another entry has its activations to split: 16 pairs of 768 x 2048 12.9 us, 15.7 in
-// steps of a tile).
+// tiles).  Routed, and more than four rows:
+// steps of a chunk (a share that crosses into another entry has its activations to split, 16 pairs of 768 x 2048 12.9 us, 15.7 in steps of a tile; and
+// eight rows of activations are better loaded by fewer CTAs).
 struct __align__(16) SpChunk {
     uint32_t ent, op, tile, nt;
     uint32_t un, key, e0, cnt;   // this rank's units; the same key: the same activations; the entry's first row or pair and their number
@@ -821,6 +822,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
     rank = sp::cluster_rank();
     const uint32_t mp = bt.mp, tr = bt.tr, R = 16u * tr, STAGE = tr * TILE;
+    auto place = [&](uint32_t p) { return MPC > 4 ? p : sp_row(bt.pairs, p); };   // (eight rows: registers are short, rows off boundaries come one by one)
 
     if (tid == 0) {
         abort_flag = s_again = 0;
@@ -882,13 +884,18 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
     const uint32_t ncl = gridDim.x / ranks, cl = blockIdx.x / ranks;
     const uint64_t steps = (uint64_t)nent * bt.op[bt.nops - 1].step_end;
     const uint32_t first = (uint32_t)(steps * cl / ncl), last = (uint32_t)(steps * (cl + 1) / ncl);
-    auto chunk = [&](uint32_t at) {
+    auto stages_of = [&](uint32_t at) {   // (what the copies need to know)
         SpChunk c = sp_chunk(bt, at, last);
         const SpOp &P = bt.op[c.op];
         const uint32_t u0 = rank * P.slice;
         c.un = u0 < P.units ? min(P.slice, P.units - u0) : 0u;
+        c.e0 = bt.ids ? s_ent[c.ent] : 0u;
+        return c;
+    };
+    auto chunk = [&](uint32_t at) {
+        SpChunk c = stages_of(at);
+        const SpOp &P = bt.op[c.op];
         if (bt.ids) {
-            c.e0 = s_ent[c.ent];
             c.cnt = s_ent[c.ent + 1] - c.e0;
         } else {
             c.e0 = c.ent * mp;
@@ -906,13 +913,13 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         uint32_t slot = 0, ph = 1;   // (a slot's first wait passes)
         bool ok = true;
         for (uint32_t at = first, i = 0; ok && at < last; i++) {
-            const SpChunk c = chunk(at);
+            const SpChunk c = INT ? chunk(at) : stages_of(at);
             at += c.steps;
             const SpOp &P = bt.op[c.op];
             const uint32_t u0 = rank * P.slice;
             const uint32_t ex = bt.ids ? s_id[s_ord[c.e0]] : 0u;
-            // (a rank without units for the chunk: a stage without data, so that the consumers get the chunk's description with it)
-            for (uint32_t u = 0; u == 0 || u < c.un; u += SU) {
+            // (integers, a rank without units for the chunk: a stage without data, so that the consumers get the chunk's description with it)
+            for (uint32_t u = 0; (INT && u == 0) || u < c.un; u += SU) {
                 if (!mbar_wait(&empty[slot], ph, &abort_flag, bt.status, ST_WAIT_EMPTY_TIMEOUT, 0u)) {
                     ok = false;
                     break;
@@ -921,8 +928,8 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 const uint32_t off = (u0 + u) / 4 * (uint32_t)K::B256;
                 // Sixteen descriptions are enough: the one written here was last read for a chunk 16 before, and the slot that the wait above
                 // found empty was left by warps that have arrived for chunk i - 2 - kSpMaxSlots at least.
-                if (u == 0 && lane == 0) s_chunk[i & 15u] = c;
-                if (c.un == 0) {
+                if (INT && u == 0 && lane == 0) s_chunk[i & 15u] = c;
+                if (INT && c.un == 0) {
                     if (lane == 0) mbar_arrive(&full[slot]);
                 } else if constexpr (ALN) {
                     if (lane == 0) {
@@ -934,7 +941,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                                   "r"(smem_u32(&full[slot])), "l"(pol)
                                 : "memory");
                     }
-                } else if (bt.pairs) {
+                } else if (MPC <= 4 && bt.pairs) {
                     // A row of the tensor map is two weight rows, a copy the even or the odd rows of a tile (see sp_row).  (Four or eight weight
                     // rows a map row would do for any address, but copies have to start on 128 bytes, where their rows would meet in the
                     // same banks.)
@@ -1000,7 +1007,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         };
         auto store = [&](const SpChunk &d, uint32_t col, uint32_t row, float v) {
             const SpOp &P = bt.op[d.op];
-            const uint32_t grow = d.tile * 16u + (ALN ? row : (row & ~15u) + sp_row(bt.pairs, row & 15u));
+            const uint32_t grow = d.tile * 16u + (ALN ? row : (row & ~15u) + place(row & 15u));
             if (col >= d.cnt || row >= d.nt * 16u || grow >= P.n) return;
             const uint32_t pair = bt.ids ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
             const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
@@ -1011,7 +1018,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         };
         [[maybe_unused]] auto again = [&](const SpChunk &d, uint32_t col, uint32_t row) {
             const SpOp &P = bt.op[d.op];
-            const uint32_t grow = d.tile * 16u + (ALN ? row : (row & ~15u) + sp_row(bt.pairs, row & 15u));
+            const uint32_t grow = d.tile * 16u + (ALN ? row : (row & ~15u) + place(row & 15u));
             if (col >= d.cnt || row >= d.nt * 16u || grow >= P.n) return;
             const uint32_t pair = bt.ids ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
             const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
@@ -1084,22 +1091,27 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         };
         uint32_t d1 = 0, d2 = 0;   // where the descriptions of the last two chunks are
         uint32_t i = 0;   // the CTA's chunks so far
-        // (what the first chunk needs of the launch's parameters is fetched before the wait)
-        const SpChunk c0 = chunk(first < last ? first : 0);
-        {
+        // (Integers: what the first chunk needs of the launch's parameters is fetched before the wait.)
+        [[maybe_unused]] SpChunk c0{};
+        if constexpr (INT) {
+            c0 = chunk(first < last ? first : 0);
             const SpOp &P = bt.op[c0.op];
-            if constexpr (INT) asm volatile("" ::"l"(P.x), "l"(P.x2), "r"(P.k), "r"(P.slice));
-            else if (bt.packed) asm volatile("" ::"l"(P.xp), "l"(P.xinv), "r"(P.pk_units));
+            asm volatile("" ::"l"(P.x), "l"(P.x2), "r"(P.k), "r"(P.slice));
         }
         if (!bt.ids) grid_dependency_wait();   // the activations belong to the kernels ahead until those are done
         for (uint32_t at = first; ok && at < last; i++) {
-            SpChunk c = c0;
-            if (INT && i != 0) {   // the producer's description comes with the first stage
+            SpChunk c;
+            if (!INT) {
+                c = chunk(at);
+            } else if (i == 0) {
+                c = c0;
+            } else {   // the producer's description comes with the first stage
                 if (!wait(full[slot], ph, ST_WAIT_FULL_TIMEOUT)) break;
                 c = s_chunk[i & 15u];
-            } else if (i != 0) {
-                c = chunk(at);
             }
+            // (f16: the copies start without it.  Who comes here for chunk i + 16 has found every warp's arrival for chunk i + 14, and a warp arrives
+            // there after it has read what belongs to chunk i.)
+            if (!INT && tid == 0) s_chunk[i & 15u] = c;
             at += c.steps;
             const SpOp &P = bt.op[c.op];
             const uint32_t u0 = rank * P.slice, un = c.un, e0 = c.e0, cnt = c.cnt, key = c.key;
@@ -1316,7 +1328,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                         const uint32_t off = (u0 + us) / 4 * (uint32_t)K::B256;
                         const uint32_t wl = ALN ? 0u : ((uint32_t)(uintptr_t)P.w + (ex < bt.n_experts ? ex : 0u) * (uint32_t)P.expert_stride + off) & 15u;
                         const uint32_t rb15 = P.row_bytes & 15u;
-                        auto lead = [&](uint32_t row) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + sp_row(bt.pairs, row & 15u) * rb15) & 15u; };
+                        auto lead = [&](uint32_t row) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + place(row & 15u) * rb15) & 15u; };
                         const uint32_t stage = base + slot * STAGE + (TABLE ? (warp >> 2) * (uint32_t)K::B256 : warp * UB);
                         const uint32_t xa = xlane + (us + warp) * 256u;
                         [[maybe_unused]] const uint32_t ca = clane + (us + warp) * (NG * 4u);
@@ -1367,12 +1379,12 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 else if (c.nt == 3) stages(std::integral_constant<int, 3>{});
                 else stages(std::integral_constant<int, TM>{});
             } else {
-                for (uint32_t us = 0; us == 0 || us < un; us += SU) {
+                for (uint32_t us = 0; us < un; us += SU) {
                     const uint32_t off = (u0 + us) / 4 * (uint32_t)K::B256;
                     // where a row's data starts in its 16-byte superset (tiles are 16 rows: the same for every tile)
                     const uint32_t wl = ALN ? 0u : ((uint32_t)(uintptr_t)P.w + (ex < bt.n_experts ? ex : 0u) * (uint32_t)P.expert_stride + off) & 15u;
                     const uint32_t rb15 = P.row_bytes & 15u;
-                    auto lead = [&](uint32_t row) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + sp_row(bt.pairs, row & 15u) * rb15) & 15u; };
+                    auto lead = [&](uint32_t row) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + place(row & 15u) * rb15) & 15u; };
                     if (!mbar_wait(&full[slot], ph, &abort_flag, bt.status, ST_WAIT_FULL_TIMEOUT, 0u)) {
                         ok = false;
                         break;
@@ -1545,7 +1557,7 @@ template <int T, bool ALN, int MPC>
 static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, uint32_t tr, uint64_t entries, uint32_t xunits, int sm_count, cudaStream_t st) {
     const uint32_t STAGE = tr * 16 * sp_pitch<T>(ALN);
     bt.tr = tr;
-    bt.step = bt.ids ? tr : 1u;
+    bt.step = bt.ids || bt.mp > 4 ? tr : 1u;
     uint32_t per = 0;   // steps of an entry
     for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].step_end = per += ((bt.op[i].n + 15) / 16 + bt.step - 1) / bt.step;
     const uint64_t steps = per * entries;
@@ -1627,8 +1639,8 @@ template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool 
             // Fitted to 1024, 4096 and 24576 x 4096 and 4096 x 12288, all types: a chunk costs waits and sums, a unit of a warp what a lone
             // multiply takes to come through and a share per tile; ranks wait for one another, in f16 with eight rows for 4.5 us a chunk
             // where there are four of them; one or two rows are split by every CTA.
-            const double ncl = (double)(2 * sm_count / (int)c), chunks = routed ? ceil(ceil((double)tiles / tr) / ncl) : ceil(ceil((double)tiles / ncl) / tr),
-                         share = routed ? chunks * tr : ceil((double)tiles / ncl), units = ceil(slice / 8.0);
+            const double ncl = (double)(2 * sm_count / (int)c), chunks = routed || mp > 4 ? ceil(ceil((double)tiles / tr) / ncl) : ceil(ceil((double)tiles / ncl) / tr),
+                         share = routed || mp > 4 ? chunks * tr : ceil((double)tiles / ncl), units = ceil(slice / 8.0);
             double cost;
             if (mp <= 2) {
                 const double tile = (T == GT_Q6_K ? 0.38 : T == GT_Q8_0 ? 0.35 : T == GT_Q4_0 ? 0.19 : 0.25) * (mp == 2 ? 1.3 : 1.0);
@@ -1671,7 +1683,7 @@ template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, 
         const uint64_t rb = (uint64_t)(ops[i].k / BlockTraits<T>::QK) * BlockTraits<T>::BYTES;
         const bool base = ((uintptr_t)ops[i].w & 15u) == 0 && (!routed || ops[i].expert_stride % 16 == 0);
         aln = aln && rb % 16 == 0 && base;
-        pairs = pairs && rb % 16 == 8 && base && ops[i].n % 2 == 0;
+        pairs = pairs && rb % 16 == 8 && base && ops[i].n % 2 == 0 && (routed || ops[i].m <= 4);
     }
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return cudaErrorNotSupported;
