@@ -104,9 +104,14 @@ bool qmv_split_pays(int ggml_type, const QmvArgs *ops, int nops, double fill) {
     constexpr uint64_t M = 1u << 20;
     const bool q4k = ggml_type == GT_Q4_K;
     if (kmin != kmax) return false;   // (the other kernel deals out work by K stages, and its passes are fuller than `fill` says)
-    if (q4k && m <= 2) return fill <= 0.7 && values >= 72 * M;
+    // One and two rows, in integers.  Short rows leave a chunk little to do between its sums: 128256 x 1024, one row, Q4_0 26.1 / 20.9, Q8_0 30.3 / 29.3, but
+    // Q6_K 36.7 / 37.5; two rows of 2048 and 2560 values, Q4_0 15.3 / 14.2, Q6_K 70.6 / 64.5, but Q8_0 22.0 / 24.0, Q4_K 54.0 / 56.0.  (14336 x 2048 twice,
+    // one row of Q4_0: 14.3 / 10.4.)
+    if (q4k && m <= 2) return fill <= 0.7 && values >= 72 * M && (m == 1 || kmax >= 4096);
     if (m <= 1 && nops > 2) return values >= 40 * M;
+    if (m <= 1 && ggml_type == GT_Q6_K && kmax < 2048) return false;
     if (m <= 1) return values >= (fill > 0.7 ? (ggml_type == GT_Q8_0 ? 60 * M : 40 * M) : ggml_type == GT_Q8_0 ? 30 * M : 24 * M);
+    if (m <= 2 && ggml_type == GT_Q8_0) return values >= 90 * M && kmax >= 4096;
     if (m <= 2) return values >= (ggml_type == GT_Q6_K ? 46 * M : 60 * M);
     if (q4k && m <= 4) return kmax >= 4096 && values >= 14 * M && (fill <= 0.6 || (fill <= 0.7 && values >= 72 * M));
     if (q4k) return fill <= 0.6 && (m <= 8 || fill <= 0.25 || (m + 7) / 8 * 16 <= 3 * m);

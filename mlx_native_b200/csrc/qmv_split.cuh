@@ -450,10 +450,10 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
 // columns with the one scale of their group.  Codes are taken 16 times (Q4_0, Q4_K), 8 times (Q5_K), 4 times (Q6_K) as large:
 // that centres them without an addition (the top bit of the byte changes sign), and sp_code_scale takes it back.  bf: B registers [set][word].
 template <int T> constexpr float sp_code_scale = T == GT_Q8_0 ? 1.f : T == GT_Q6_K ? 0.25f : T == GT_Q5_K ? 0.125f : 0.0625f;
-// OFF: the unit's bytes within a stage from the warp's first unit on.  c: kBias four times, in registers (as an immediate every multiply would
+// alike: all rows start at the same half of a word.  OFF: the unit's bytes within a stage from the warp's first unit on.  c: kBias four times, in registers (as an immediate every multiply would
 // copy it into four of them).
 template <int T, bool ALN, uint32_t OFF, int NT, int NS, int TM>
-__device__ __forceinline__ void sp_unit_int(uint32_t a0, uint32_t a1, uint32_t u, uint32_t t, uint32_t tab, bool half, const uint32_t (&bf)[NS][4],
+__device__ __forceinline__ void sp_unit_int(uint32_t a0, uint32_t a1, uint32_t u, uint32_t t, uint32_t tab, bool half, [[maybe_unused]] bool alike, const uint32_t (&bf)[NS][4],
                                             [[maybe_unused]] const float (&cc)[NS], const uint32_t (&c)[4], float (&acc)[TM][NS][4]) {
     constexpr uint32_t TS = 16u * sp_pitch<T>(ALN), R8 = ALN ? 8u * sp_pitch<T>(true) : 0u;
     auto f = [](uint32_t v) { return __uint_as_float(v); };
@@ -592,7 +592,7 @@ __device__ __forceinline__ void sp_unit_int(uint32_t a0, uint32_t a1, uint32_t u
                     }
             });
         };
-        if constexpr (ALN) {
+        if (ALN || alike) {   // (even and odd rows are 8 bytes apart: the same half word)
             if (a0 & 2u) body(std::integral_constant<int, 1>{});
             else body(std::integral_constant<int, 0>{});
         } else {
@@ -1364,7 +1364,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                             // (an odd number of blocks: the second block of the last unit lies past the row)
                             const bool half = !ALN && t >= 2 && (u0 + uu) * 64 + 32 >= P.k;
                             sp_unit_int<T, ALN, OFF, NT>(stage + g * PITCH + lead(g), stage + (g + 8) * PITCH + lead(g + 8), warp, t,
-                                                         tab + g * 16 + (t >> 1) * 8, half, b, cc, bias, acc);
+                                                         tab + g * 16 + (t >> 1) * 8, half, !ALN && bt.pairs, b, cc, bias, acc);
                         });
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&empty[slot]);
