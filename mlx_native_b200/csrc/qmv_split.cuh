@@ -98,6 +98,7 @@ struct SpBatch {
     uint32_t nent;            // dense: groups of mp activation rows; routed: counted on the device
     uint32_t mp;              // activation rows of an entry (1, 2, 4 or 8)
     uint32_t tr, step;        // tiles of a chunk, at most, and of a step of the clusters' shares
+    uint32_t dealt;           // steps are dealt out to the clusters in turn; otherwise a share is contiguous
     uint32_t early_weights;
     uint32_t *status;
     uint32_t nslots;          // ring depth, and what lies behind the ring in shared memory
@@ -673,11 +674,12 @@ template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const 
 // steps of one tile (shares of whole chunks of four leave a last round part empty: Q4_0 24576 x 4096 has 384 such chunks for 296 CTAs, or 1536
 // tiles).  Routed, and more than four rows:
 // steps of a chunk (a share that crosses into another entry has its activations to split, 16 pairs of 768 x 2048 12.9 us, 15.7 in steps of a tile; and
-// eight rows of activations are better loaded by fewer CTAs).
+// eight rows of activations are better loaded by fewer CTAs).  Three and four rows: of a tile up to six tiles a CTA (24576 x 4096 Q4_0 28.2 -> 26.9 us),
+// beyond that of a chunk, dealt out in turn (Q4_0 151936 x 1024 39.3, 42.2 in equal shares; Q4_K 49157 x 2048 28.0, 32.0).
 struct __align__(16) SpChunk {
     uint32_t ent, op, tile, nt;
     uint32_t un, key, e0, cnt;   // this rank's units; the same key: the same activations; the entry's first row or pair and their number
-    uint32_t steps;              // of the share
+    uint32_t steps;              // to the next one
 };
 __device__ __forceinline__ SpChunk sp_chunk(const SpBatch &b, uint32_t pos, uint32_t last) {
     SpChunk c;
@@ -692,13 +694,12 @@ __device__ __forceinline__ SpChunk sp_chunk(const SpBatch &b, uint32_t pos, uint
     }
     c.tile = (r - from) * b.step;
     const uint32_t left = min((b.op[c.op].n + 15u) / 16u - c.tile, (last - pos) * b.step);
-    c.nt = left;
-    if (left > b.tr) {
+    c.nt = min(b.tr, left);
+    if (b.step == 1 && left > b.tr && left < 8 * b.tr) {   // (from eight chunks on: whole ones)
         uint32_t parts = 2;
-        while (parts * b.tr < left && parts < 8) parts++;   // (from eight on: whole chunks)
-        c.nt = b.step == 1 ? min(b.tr, (left + parts - 1) / parts) : b.tr;
+        while (parts * b.tr < left) parts++;
+        c.nt = (left + parts - 1) / parts;
     }
-    c.steps = b.step == 1 ? c.nt : 1u;
     return c;
 }
 
@@ -883,12 +884,17 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
     // this cluster's share of the tiles
     const uint32_t ncl = gridDim.x / ranks, cl = blockIdx.x / ranks;
     const uint64_t steps = (uint64_t)nent * bt.op[bt.nops - 1].step_end;
-    const uint32_t first = (uint32_t)(steps * cl / ncl), last = (uint32_t)(steps * (cl + 1) / ncl);
+    // (whole chunks: as many for every cluster as the fullest one has, so that fewer shares cross into another entry: gate and up, 20 pairs of 16
+    // experts, 768 x 2560 Q4_K, the layer 61 us, 66 with equal shares)
+    const uint64_t most = (steps + ncl - 1) / ncl;
+    const uint32_t first = bt.step == 1 ? (uint32_t)(steps * cl / ncl) : bt.dealt ? cl : (uint32_t)min(steps, most * cl);
+    const uint32_t last = bt.step == 1 ? (uint32_t)(steps * (cl + 1) / ncl) : bt.dealt ? (uint32_t)steps : (uint32_t)min(steps, most * (cl + 1));
     auto stages_of = [&](uint32_t at) {   // (what the copies need to know)
         SpChunk c = sp_chunk(bt, at, last);
         const SpOp &P = bt.op[c.op];
         const uint32_t u0 = rank * P.slice;
         c.un = u0 < P.units ? min(P.slice, P.units - u0) : 0u;
+        c.steps = bt.step == 1 ? c.nt : bt.dealt ? ncl : 1u;
         c.e0 = bt.ids ? s_ent[c.ent] : 0u;
         return c;
     };
@@ -1557,7 +1563,10 @@ template <int T, bool ALN, int MPC>
 static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, uint32_t tr, uint64_t entries, uint32_t xunits, int sm_count, cudaStream_t st) {
     const uint32_t STAGE = tr * 16 * sp_pitch<T>(ALN);
     bt.tr = tr;
-    bt.step = bt.ids || bt.mp > 4 ? tr : 1u;
+    uint64_t tiles = 0;
+    for (uint32_t i = 0; i < bt.nops; i++) tiles += (bt.op[i].n + 15) / 16;
+    bt.step = bt.ids || bt.mp > 4 || (bt.mp > 2 && tiles * ranks > 12ull * sm_count) ? tr : 1u;   // (see SpChunk)
+    bt.dealt = bt.step != 1 && entries == 1;
     uint32_t per = 0;   // steps of an entry
     for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].step_end = per += ((bt.op[i].n + 15) / 16 + bt.step - 1) / bt.step;
     const uint64_t steps = per * entries;
