@@ -1,4 +1,5 @@
-"""One and two activation rows on the split mat-vec (csrc/qmv_split.cuh: codes and activation digits as 8-bit integers), against the oracle."""
+"""One and two activation rows on the split mat-vec (csrc/qmv_split.cuh: codes and activation digits as 8-bit integers), and how its tiles are shared
+out, against the oracle."""
 import numpy as np
 import pytest
 
@@ -63,3 +64,15 @@ def test_zero_and_tiny_rows(ctx):
     for row in x:
         y, ref = ctx.matmul(gtype, wq, row[None], n, k)[0], w @ row.astype(np.float64)
         assert np.all(np.abs(y - ref) <= 1e-6 * np.abs(ref).max() + 3e-45)
+
+
+@pytest.mark.parametrize("tname,n,k,m", [("Q4_0", 28500, 256, 3), ("Q8_0", 28449, 96, 4), ("Q4_0", 28300, 256, 4)])
+def test_three_and_four_rows_of_many_tiles(ctx, tname, n, k, m):
+    """More and fewer than six tiles a CTA: chunks dealt out in turn, or equal shares by tiles."""
+    gtype, otype = ALL[tname]
+    wq = normal_weights(n + k, n, k, otype)
+    x = normal_acts(n + m, m, k)
+    y = ctx.matmul(gtype, wq, x, n, k)
+    assert mx.last_kernel_name() == "qmv_split"
+    y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8)
+    assert norm_err(y, y_ref, ad) <= MV_TOL
