@@ -4,8 +4,9 @@
 // (launch, activations, waits between stages) and instructions (integer operations issue at half rate).  Hence:
 //
 //  * The activations of a CTA stay in shared memory for all its weight rows, in the order of the B registers of mma.sync.  One or two
-//    rows (dense) as four signed 8-bit digits, for multiplies of 8-bit integers (sp_unit_int); more, and routed ones, as f16 hi + lo halves,
-//    scaled by a power of two per row so that both stay in range, for mma.sync.m16n8k16.  One and two rows are split by every CTA
+//    rows (dense) as four signed 8-bit digits, for multiplies of 8-bit integers (sp_unit_int), where a warp's share of them is alike enough for one last
+//    place; other shares (sp_far), more rows, and routed ones, as f16 hi + lo halves, scaled by powers of two so that both stay in range, for
+//    mma.sync.m16n8k16.  One and two rows are split by every CTA
 //    itself, several by qmv_pack_kernel, and arrive by bulk copies.  The loop over the weights only unpacks codes into signed integers, bytes or
 //    normal f16 numbers, so products are exact and sums are f32.
 //  * In f16 the 8 columns of an MMA are (activation row, hi | lo): one multiply serves up to four rows (NS = 2 sets: eight rows).
@@ -51,6 +52,9 @@ __host__ __device__ constexpr int sp_sets(int mp) { return mp > 4 || mp == 2 ? 2
 constexpr int kSpMaxOps = 8;                        // mat-vecs one launch carries
 constexpr int kSpMaxSlots = 8;
 constexpr int kSpMaxPairs = 256;                    // (token, slot) pairs of a routed launch
+// Two CTAs share an SM: 228 KB less 1 KB each for the system and the kernel's static 3 KB.
+constexpr size_t kSpSmem = 110 * 1024;
+constexpr int kSpMaxUnits = kSpSmem / 256;          // units of activations that a CTA holds, all rows together
 
 // SU: units (64 K values) of a stage, a multiple of the warps.  NG: sub-blocks of a unit that have an offset of their own, and
 // with it the sum of their activations (Q4_K, Q5_K).
@@ -154,6 +158,25 @@ __device__ __forceinline__ void split(float a, float b, uint32_t &hi, uint32_t &
     hi = *reinterpret_cast<const uint32_t *>(&h);
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
+// The largest magnitude by its bits: an infinity is above every number, a NaN above that.
+__device__ __forceinline__ uint32_t peak_bits(const float (&v)[4]) {
+    uint32_t b[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) b[e] = __float_as_uint(v[e]) & 0x7FFFFFFFu;
+    return max(max(b[0], b[1]), max(b[2], b[3]));
+}
+// How the values of a warp's share compare with the largest: `peak` of four a lane, of 32 eight neighbouring lanes; `least`: what counts.
+struct Spread {
+    uint32_t held = 0, some = 0;
+    bool lost = false;
+    __device__ __forceinline__ void look(uint32_t peak, uint32_t least, uint32_t lane) {
+        const uint32_t h = __ballot_sync(0xffffffffu, peak >= least), n = __ballot_sync(0xffffffffu, peak != 0), m = 0xFFu << (lane & 24u);
+        held += __popc(h);
+        some += __popc(n);
+        lost = lost || ((n & m) != 0 && (h & m) == 0);
+    }
+    __device__ __forceinline__ bool far() const { return __any_sync(0xffffffffu, lost) || 2 * held < some; }
+};
 // Two powers of two whose product brings amax (its bits; a number) into [2^13, 2^14), and those of the way back from units of the last digit.
 // (One factor would not be a normal number where amax is tiny.)  NaN for the way back where the run holds an infinity or a NaN.
 __device__ __forceinline__ void pow2_int(uint32_t amax, float &s0, float &s1, float &inv0, float &inv1) {
@@ -247,12 +270,27 @@ template <int T, bool ALN> __device__ __forceinline__ void sp_pairs(uint32_t u, 
     }
 }
 
+// The four activations at x + p0 and x + p1, of which the pairs i0 and i1 exist; y: fused SwiGLU, silu(x) * y (as src/shaders/silu_mul.metal:17-30).
+__device__ __forceinline__ void sp_act(const float *x, const float *y, uint32_t p0, uint32_t p1, bool i0, bool i1, float (&v)[4]) {
+    if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(x + p0));
+    if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[2]), "=f"(v[3]) : "l"(x + p1));
+    if (y) {
+        float w[4] = {0.f, 0.f, 0.f, 0.f};
+        if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[0]), "=f"(w[1]) : "l"(y + p0));
+        if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[2]), "=f"(w[3]) : "l"(y + p1));
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[e] = v[e] / (1.0f + expf(-v[e])) * w[e];
+    }
+}
+
 // One unit (64 K values) of a stage against NT tiles.  a0 / a1: shared address of rows g and g + 8 of tile 0 at the unit's
 // first byte (Q4_K, Q5_K, Q6_K: of its super-block), lead-in included; tiles are 16 PITCH bytes apart.  bf: the B registers
-// [set][MMA][2]; cc: per set and sub-block the sum of the activations (Q4_K, Q5_K); tab: the warp's scale table.
-template <int T, bool ALN, int NT, int NS, int TM>
+// [set][MMA][2]; cc: per set and sub-block the sum of the activations (Q4_K, Q5_K); tab: the warp's scale table.  FACT: the activations of MMAs
+// 0 and 1 and those of 2 and 3 have a power of two each, beside the one of the share; f2: its inverses for the lane's columns.
+template <int T, bool ALN, int NT, bool FACT, int NS, int TM>
 __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, uint32_t t, uint32_t g, uint32_t tab, bool half,
-                                        const uint32_t (&bf)[NS][4][2], [[maybe_unused]] const float (&cc)[NS][2], float (&acc)[TM][NS][4]) {
+                                        const uint32_t (&bf)[NS][4][2], [[maybe_unused]] const float (&cc)[NS][2], [[maybe_unused]] const float (&f2)[2],
+                                        float (&acc)[TM][NS][4]) {
     constexpr uint32_t TS = 16u * sp_pitch<T>(ALN);
     if constexpr (T == GT_Q4_0 || T == GT_Q8_0) {
         constexpr bool Q8 = T == GT_Q8_0;
@@ -298,6 +336,10 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                 d0[h] = f16lo_to_float(lds_u16i<o>(a));
                 d1[h] = f16lo_to_float(lds_u16i<o + BB>(a));
                 if constexpr (!ALN) d1[h] = half ? 0.f : d1[h];
+                if constexpr (FACT) {
+                    d0[h] *= f2[0];
+                    d1[h] *= f2[1];
+                }
             }
             uint32_t a[4][4];
             if constexpr (Q8) {
@@ -345,6 +387,13 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
             uint32_t p0[4], p1[4];   // scales and offsets (sp_table_row) of rows g and g + 8
             lds128i<j * 256u>(tr, p0);
             lds128i<j * 256u + 128u>(tr, p1);
+            if constexpr (FACT) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    p0[q] = __float_as_uint(__uint_as_float(p0[q]) * f2[q & 1]);
+                    p1[q] = __float_as_uint(__uint_as_float(p1[q]) * f2[q & 1]);
+                }
+            }
             uint32_t a[4][4];
             if constexpr (Q5) {   // five-bit codes, one per byte: nibble | fifth bit << 4
                 uint32_t f[2][2];
@@ -420,7 +469,11 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
                 for (int q = 0; q < 4; q++) {
                     const uint32_t x0 = sp::bytes02(qv[0][q], 0x64206420u), x2 = sp::bytes13(qv[0][q], 0x64206420u);
                     const uint32_t x1 = sp::bytes02(qv[1][q], 0x64206420u), x3 = sp::bytes13(qv[1][q], 0x64206420u);
-                    const float pa = __uint_as_float(p0[q]), pb = __uint_as_float(p1[q]);
+                    float pa = __uint_as_float(p0[q]), pb = __uint_as_float(p1[q]);
+                    if constexpr (FACT) {
+                        pa *= f2[q >> 1];
+                        pb *= f2[q >> 1];
+                    }
 #pragma unroll
                     for (int s = 0; s < NS; s++) {
                         constexpr float zero[4] = {0.f, 0.f, 0.f, 0.f};
@@ -797,6 +850,138 @@ __global__ void __launch_bounds__(256) qmv_pack_kernel(const __grid_constant__ S
     }
 }
 
+// A warp's share of up to two activation rows in halves, where digits would lose its small values (see `far` in the kernel): a power of two for
+// every 32 values (lanes 8 j .. 8 j + 7 hold them), as one for the share (inv: its inverse) and one beside it for the 32, whose inverse's exponent goes to
+// rel[unit][row][32 values].  x, x2: the entry's first row, from the rank's slice on; left: values from there to the end of the row.
+template <int T, bool ALN, int MPC>
+__device__ __forceinline__ void sp_far(const float *x, const float *x2, uint32_t k, uint32_t left, uint32_t cnt, uint32_t un, uint32_t warp, uint32_t lane,
+                                       uint32_t xf, uint32_t xs, [[maybe_unused]] uint32_t ccb, [[maybe_unused]] uint32_t cs, float *inv, uint8_t *rel) {
+    constexpr int NG = SpTraits<T>::NG;
+    const uint32_t q = (lane >> 2) & 3u, tt = lane & 3u, hf = lane >> 4;
+    uint32_t p0, p1;
+    sp_pairs<T, ALN>(warp, q, tt, p0, p1);
+    auto load = [&](uint32_t row, uint32_t u, float (&v)[4]) {
+        v[0] = v[1] = v[2] = v[3] = 0.f;
+        if (u >= un) return;
+        const uint32_t o = T == GT_Q6_K ? 256u * (u >> 2) : 64u * u;
+        const size_t at = (size_t)row * k + o;
+        sp_act(x + at, x2 ? x2 + at : nullptr, p0, p1, o + p0 < left, o + p1 < left, v);
+    };
+    for (uint32_t row = 0; row < cnt; row++) {
+        uint32_t am = 0;
+        for (uint32_t u = warp; u < un; u += 16) {
+            float z[4];
+            load(row, u + 8 * hf, z);
+            am = max(am, sp::peak_bits(z));
+        }
+        am = __reduce_max_sync(0xffffffffu, am);
+        float s, i;
+        sp::pow2(__uint_as_float(am), s, i);
+        if (lane == 0) inv[row] = i;
+        for (uint32_t u = warp; u < un; u += 16) {
+            const uint32_t mine = u + 8 * hf;
+            float z[4];
+            load(row, mine, z);
+            uint32_t b = sp::peak_bits(z);
+#pragma unroll
+            for (int o = 1; o <= 4; o *= 2) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+            const uint32_t beside = min((am >> 23) - (b >> 23), 96u);   // (scales times 2^-96 are still normal numbers)
+            const float s1 = __uint_as_float((127u + beside) << 23);
+#pragma unroll
+            for (int e = 0; e < 4; e++) z[e] = z[e] * s * s1;
+            [[maybe_unused]] float sum = (z[0] + z[1]) + (z[2] + z[3]);
+            if constexpr (NG != 0) {
+#pragma unroll
+                for (int o = 1; o <= 4; o *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            }
+            uint32_t hi[2], lo[2];
+            sp::split(z[0], z[2], hi[0], lo[0]);
+            sp::split(z[1], z[3], hi[1], lo[1]);
+            if (mine >= un) continue;
+            const uint32_t d = xf + row * xs + mine * 256u + (q >> 1) * 128u + tt * 32u + (q & 1u) * 8u;
+            sts64(d, hi[0], hi[1]);
+            sts64(d + 16, lo[0], lo[1]);
+            if ((lane & 7u) == 0) {
+                rel[(mine * MPC + row) * 2 + (q >> 1)] = (uint8_t)(127u - beside);
+                if constexpr (NG != 0) sts32(ccb + row * cs + (mine * NG + (q >> 1)) * 4u, __float_as_uint(sum));
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// The stages of a chunk against such a share; the sums go to `part`.  Returns whether all copies came.
+struct SpRing {
+    uint64_t *full, *empty;
+    volatile uint32_t *abort_flag;
+    uint32_t base, slot, ph;
+};
+template <int T, bool ALN, int MPC>
+__device__ __forceinline__ bool sp_far_stages(const SpBatch &bt, uint32_t op, uint32_t u0, uint32_t un, uint32_t nt, SpRing &ring, uint32_t warp, uint32_t lane, uint32_t xf,
+                                               uint32_t ccb, uint32_t tab, uint32_t part, const float *inv, const uint8_t *rel) {
+    using K = SpTraits<T>;
+    constexpr int NG = K::NG, SU = K::SU, TM = sp_tiles(MPC);
+    constexpr bool TABLE = T == GT_Q4_K || T == GT_Q5_K || T == GT_Q6_K;
+    constexpr uint32_t PITCH = sp_pitch<T>(ALN), UB = T == GT_Q8_0 ? 68u : 36u;
+    const SpOp &P = bt.op[op];
+    const uint32_t g = lane >> 2, t = lane & 3u, row = MPC == 1 ? 0u : t & 1u, stage_bytes = bt.tr * 16u * PITCH, rb15 = P.row_bytes & 15u;
+    const uint32_t xlane = xf + (MPC == 1 ? 0u : (g >> 1 & 1u) * bt.xstride) + (t * 2 + (g & 1u)) * 16u;
+    float acc[TM][1][4];
+#pragma unroll
+    for (int j = 0; j < TM; j++) acc[j][0][0] = acc[j][0][1] = acc[j][0][2] = acc[j][0][3] = 0.f;
+    bool ok = true;
+    for (uint32_t us = 0; us == 0 || us < un; us += SU) {
+        const uint32_t off = (u0 + us) / 4 * (uint32_t)K::B256, wl = ALN ? 0u : ((uint32_t)(uintptr_t)P.w + off) & 15u;
+        auto lead = [&](uint32_t r) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + sp_row(bt.pairs, r & 15u) * rb15) & 15u; };
+        if (!mbar_wait(&ring.full[ring.slot], ring.ph, ring.abort_flag, bt.status, ST_WAIT_FULL_TIMEOUT, 0u)) {
+            ok = false;
+            break;
+        }
+        const uint32_t stage = ring.base + ring.slot * stage_bytes;
+        for (uint32_t ul = warp; ul < (uint32_t)SU && us + ul < un; ul += kSpWarps) {
+            const uint32_t uu = us + ul, ub = TABLE ? (ul >> 2) * (uint32_t)K::B256 : ul * UB;
+            uint32_t bf[1][4][2], v[4];
+            float cc[1][2];
+            lds128i<0>(xlane + uu * 256u, v);
+            bf[0][0][0] = v[0]; bf[0][0][1] = v[1]; bf[0][1][0] = v[2]; bf[0][1][1] = v[3];
+            lds128i<128>(xlane + uu * 256u, v);
+            bf[0][2][0] = v[0]; bf[0][2][1] = v[1]; bf[0][3][0] = v[2]; bf[0][3][1] = v[3];
+#pragma unroll
+            for (int q = 0; q < NG; q++) cc[0][q] = __uint_as_float(lds32(ccb + row * bt.cstride + (uu * NG + q) * 4u));
+            const uint8_t *e = rel + (uu * MPC + row) * 2;
+            const float f2[2] = {__uint_as_float((uint32_t)e[0] << 23), __uint_as_float((uint32_t)e[1] << 23)};
+            if constexpr (TABLE) {
+                __syncwarp();   // the table of the unit before has been read
+                for (uint32_t r = lane; r < 16u * nt; r += 32) sp_table_row<T, false>(tab + r * 16, stage + r * PITCH + lead(r) + ub, ul);
+                __syncwarp();
+            }
+            const bool half = (u0 + uu) * 64 + 32 >= P.k;   // (the second block of the last unit lies past the row)
+            auto tiles = [&](auto NT) {
+                sp_unit<T, ALN, decltype(NT)::value, true>(stage + g * PITCH + lead(g) + ub, stage + (g + 8) * PITCH + lead(g + 8) + ub, ul, t, g, tab, half, bf, cc, f2, acc);
+            };
+            if (nt == 1) tiles(std::integral_constant<int, 1>{});
+            else if (nt == 2) tiles(std::integral_constant<int, 2>{});
+            else if (nt == 3) tiles(std::integral_constant<int, 3>{});
+            else tiles(std::integral_constant<int, TM>{});
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ring.empty[ring.slot]);
+        if (++ring.slot == bt.nslots) {
+            ring.slot = 0;
+            ring.ph ^= 1u;
+        }
+    }
+    if (t < (uint32_t)MPC)
+#pragma unroll
+        for (int j = 0; j < TM; j++)
+            if (j < (int)nt) {
+                const uint32_t a = part + (t * 16u * bt.tr + 16 * j + g) * 4;
+                sts32(a, __float_as_uint((acc[j][0][0] + acc[j][0][1]) * inv[t]));
+                sts32(a + 32, __float_as_uint((acc[j][0][2] + acc[j][0][3]) * inv[t]));
+            }
+    return ok;
+}
+
 // MPC: 1, 2 = that many activation rows, in 8-bit integers (sp_unit_int); 4 = up to four, 8 = up to eight, in f16 (one set of columns, two).
 template <int T, bool ALN, int MPC>
 __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_constant__ SpBatch bt, const __grid_constant__ SpMaps maps) {
@@ -811,12 +996,16 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
     const uint32_t base = (smem_u32(smem_raw) + 127u) & ~127u;      // (the same in every CTA of a cluster)
     __shared__ __align__(8) uint64_t full[kSpMaxSlots], empty[kSpMaxSlots], sync_bar[3], recv_bar[4], x_bar, c_bar;
     __shared__ float s_inv[kSpWarps][8];                            // inverse activation scales of a warp's share of K
+    // integers, shares in halves (sp_far): exponents of the inverse scales of [unit][row][32 values], beside the share's
+    __shared__ __align__(2) uint8_t s_rel[INT ? kSpMaxUnits * 2 : 2];
     __shared__ volatile uint32_t abort_flag, s_again;
     __shared__ uint32_t s_nent;
     __shared__ SpChunk s_chunk[16];                                 // the chunks in work
-    __shared__ uint16_t s_id[kSpMaxPairs];                          // routed: expert of every pair (there are at most 65535)
-    __shared__ uint16_t s_ord[kSpMaxPairs], s_ent[kSpMaxPairs + 1]; // pairs by expert; entry e = pairs s_ord[s_ent[e] ..]
+    constexpr int PAIRS = INT ? 1 : kSpMaxPairs;
+    __shared__ uint16_t s_id[PAIRS];                                // routed: expert of every pair (there are at most 65535)
+    __shared__ uint16_t s_ord[PAIRS], s_ent[PAIRS + 1];             // pairs by expert; entry e = pairs s_ord[s_ent[e] ..]
     __shared__ uint32_t s_wcnt[kSpWarps];
+    const bool routed = !INT && bt.ids;                             // (routed products never leave in integers)
 
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     uint32_t ranks, rank;
@@ -837,7 +1026,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         mbar_init(&c_bar, kSpWarps);
         mbar_init_fence();
     }
-    if (bt.ids) {
+    if (routed) {
         grid_dependency_wait();   // the expert ids belong to the kernels ahead
         for (uint32_t p = tid; p < kSpMaxPairs; p += kSpThreads) s_id[p] = p < bt.npairs ? (uint16_t)min(__ldcg(bt.ids + p), bt.n_experts) : (uint16_t)0xFFFFu;
     }
@@ -845,7 +1034,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
     if (ranks > 1) sp::cluster_sync();   // the others' barriers exist before anything is sent there
     else __syncthreads();
     allow_dependents();
-    if (bt.ids) {
+    if (routed) {
         // rank of every pair by (expert, pair); an entry starts at every mp-th pair of an expert
         uint32_t pos = 0, before = 0, me = 0;
         if (tid < bt.npairs) {
@@ -880,7 +1069,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         if (tid < bt.npairs) s_ord[tid] &= 0x7FFFu;
         __syncthreads();
     }
-    const uint32_t nent = bt.ids ? s_nent : bt.nent;
+    const uint32_t nent = routed ? s_nent : bt.nent;
     // this cluster's share of the tiles
     const uint32_t ncl = gridDim.x / ranks, cl = blockIdx.x / ranks;
     const uint64_t steps = (uint64_t)nent * bt.op[bt.nops - 1].step_end;
@@ -895,13 +1084,13 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         const uint32_t u0 = rank * P.slice;
         c.un = u0 < P.units ? min(P.slice, P.units - u0) : 0u;
         c.steps = bt.step == 1 ? c.nt : bt.dealt ? ncl : 1u;
-        c.e0 = bt.ids ? s_ent[c.ent] : 0u;
+        c.e0 = routed ? s_ent[c.ent] : 0u;
         return c;
     };
     auto chunk = [&](uint32_t at) {
         SpChunk c = stages_of(at);
         const SpOp &P = bt.op[c.op];
-        if (bt.ids) {
+        if (routed) {
             c.cnt = s_ent[c.ent + 1] - c.e0;
         } else {
             c.e0 = c.ent * mp;
@@ -923,7 +1112,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             at += c.steps;
             const SpOp &P = bt.op[c.op];
             const uint32_t u0 = rank * P.slice;
-            const uint32_t ex = bt.ids ? s_id[s_ord[c.e0]] : 0u;
+            const uint32_t ex = routed ? s_id[s_ord[c.e0]] : 0u;
             // (integers, a rank without units for the chunk: a stage without data, so that the consumers get the chunk's description with it)
             for (uint32_t u = 0; (INT && u == 0) || u < c.un; u += SU) {
                 if (!mbar_wait(&empty[slot], ph, &abort_flag, bt.status, ST_WAIT_EMPTY_TIMEOUT, 0u)) {
@@ -1015,9 +1204,9 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             const SpOp &P = bt.op[d.op];
             const uint32_t grow = d.tile * 16u + (ALN ? row : (row & ~15u) + place(row & 15u));
             if (col >= d.cnt || row >= d.nt * 16u || grow >= P.n) return;
-            const uint32_t pair = bt.ids ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
+            const uint32_t pair = routed ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
             const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
-            if (bt.ids && s_id[pair] >= bt.n_experts) v = 0.f;   // an id that names no expert
+            if (routed && s_id[pair] >= bt.n_experts) v = 0.f;   // an id that names no expert
             if ((INT || NG != 0) && v != v) s_again = 1;
             P.y[o] = v;
             for (uint32_t pr = 0; pr < P.n_peer; pr++) P.y_peer[pr][o] = v;
@@ -1026,13 +1215,13 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             const SpOp &P = bt.op[d.op];
             const uint32_t grow = d.tile * 16u + (ALN ? row : (row & ~15u) + place(row & 15u));
             if (col >= d.cnt || row >= d.nt * 16u || grow >= P.n) return;
-            const uint32_t pair = bt.ids ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
+            const uint32_t pair = routed ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
             const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
             float v = P.y[o];
             if (v == v) return;
-            v = sp_again<T>(P.w + (bt.ids ? s_id[pair] * P.expert_stride : 0ull) + (uint64_t)grow * P.row_bytes,
-                            P.x + (size_t)(bt.ids ? pair / P.x_div : pair) * P.k,
-                            P.x2 ? P.x2 + (size_t)(bt.ids ? pair / P.x_div : pair) * P.k : nullptr, P.k);
+            v = sp_again<T>(P.w + (routed ? s_id[pair] * P.expert_stride : 0ull) + (uint64_t)grow * P.row_bytes,
+                            P.x + (size_t)(routed ? pair / P.x_div : pair) * P.k,
+                            P.x2 ? P.x2 + (size_t)(routed ? pair / P.x_div : pair) * P.k : nullptr, P.k);
             P.y[o] = v;
             for (uint32_t pr = 0; pr < P.n_peer; pr++) P.y_peer[pr][o] = v;
         };
@@ -1104,8 +1293,9 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             const SpOp &P = bt.op[c0.op];
             asm volatile("" ::"l"(P.x), "l"(P.x2), "r"(P.k), "r"(P.slice));
         }
-        if (!bt.ids) grid_dependency_wait();   // the activations belong to the kernels ahead until those are done
-        for (uint32_t at = first; ok && at < last; i++) {
+        if (!routed) grid_dependency_wait();   // the activations belong to the kernels ahead until those are done
+        uint32_t at = first;
+        for (; ok && at < last; i++) {
             SpChunk c;
             if (!INT) {
                 c = chunk(at);
@@ -1121,7 +1311,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             at += c.steps;
             const SpOp &P = bt.op[c.op];
             const uint32_t u0 = rank * P.slice, un = c.un, e0 = c.e0, cnt = c.cnt, key = c.key;
-            const uint32_t ex = bt.ids && !ALN ? s_id[s_ord[e0]] : 0u;
+            const uint32_t ex = routed && !ALN ? s_id[s_ord[e0]] : 0u;
             if (!INT && key != cur && bt.packed) {
                 // the rows' slices come ready from the pack kernel's scratch area
                 if (cur != 0xFFFFFFFFu && !csync()) break;   // nobody reads the entry before any more
@@ -1143,6 +1333,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 __syncwarp();
             }
             if (key != cur) {
+                [[maybe_unused]] bool far = false;   // digits do not do for the share
                 // ---- the entry's activations of this warp's units: f16 hi + lo in B register order.  A pass takes two units
                 // (lane = (unit of the pass, MMA q, quad lane tt), four values each) ----
                 cur = key;
@@ -1184,69 +1375,65 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 };
                 __syncwarp();
                 if constexpr (INT) {
-                    const float *x[MPC], *y[MPC];
+                    uint32_t from[MPC];   // (below 2^31: qmv_split_fits)
 #pragma unroll
-                    for (int r = 0; r < MPC; r++) {
-                        const size_t o = (size_t)(e0 + min((uint32_t)r, cnt - 1)) * P.k + kb;
-                        x[r] = P.x + o;
-                        y[r] = P.x2 ? P.x2 + o : nullptr;
-                    }
+                    for (int r = 0; r < MPC; r++) from[r] = (e0 + min((uint32_t)r, cnt - 1)) * P.k + kb;
                     auto load = [&](int r, uint32_t p, float (&v)[4]) {
                         v[0] = v[1] = v[2] = v[3] = 0.f;
-                        const uint32_t o = 1024u * p;
+                        const uint32_t o = 1024u * p, at = from[r] + o;
                         if (2 * p + hf >= mine) return;
-                        const bool i0 = kb + o + p0 < P.k, i1 = kb + o + p1 < P.k;
-                        if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(x[r] + o + p0));
-                        if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v[2]), "=f"(v[3]) : "l"(x[r] + o + p1));
-                        if (y[r]) {   // silu(gate) * up, as src/shaders/silu_mul.metal:17-30
-                            float w[4] = {0.f, 0.f, 0.f, 0.f};
-                            if (i0) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[0]), "=f"(w[1]) : "l"(y[r] + o + p0));
-                            if (i1) asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(w[2]), "=f"(w[3]) : "l"(y[r] + o + p1));
-#pragma unroll
-                            for (int e = 0; e < 4; e++) v[e] = v[e] / (1.0f + expf(-v[e])) * w[e];
-                        }
+                        sp_act(P.x + at, P.x2 ? P.x2 + at : nullptr, p0, p1, kb + o + p0 < P.k, kb + o + p1 < P.k, v);
                     };
-                    // (largest magnitude by its bits: an infinity is above every number, a NaN above that)
-                    auto peak = [](const float (&v)[4]) {
-                        uint32_t b[4];
-#pragma unroll
-                        for (int e = 0; e < 4; e++) b[e] = __float_as_uint(v[e]) & 0x7FFFFFFFu;
-                        return max(max(b[0], b[1]), max(b[2], b[3]));
-                    };
+                    auto peak = [](const float (&v)[4]) { return sp::peak_bits(v); };
                     constexpr int HELD = 4;   // passes whose values stay in registers; those beyond are loaded again
                     float v[MPC][HELD][4], s[MPC], s1[MPC];
+                    uint32_t am[MPC];
 #pragma unroll
                     for (int r = 0; r < MPC; r++)
 #pragma unroll
                         for (int p = 0; p < HELD; p++) load(r, p, v[r][p]);
 #pragma unroll
                     for (int r = 0; r < MPC; r++) {
-                        uint32_t am = 0;
+                        am[r] = 0;
 #pragma unroll
-                        for (int p = 0; p < HELD; p++) am = max(am, peak(v[r][p]));
+                        for (int p = 0; p < HELD; p++) am[r] = max(am[r], peak(v[r][p]));
                         for (uint32_t p = HELD; 2 * p < mine; p++) {
                             float z[4];
                             load(r, p, z);
-                            am = max(am, peak(z));
+                            am[r] = max(am[r], peak(z));
                         }
-                        am = __reduce_max_sync(0xffffffffu, am);
+                        am[r] = __reduce_max_sync(0xffffffffu, am[r]);
                         float inv0, inv1;
-                        sp::pow2_int(am, s[r], s1[r], inv0, inv1);
+                        sp::pow2_int(am[r], s[r], s1[r], inv0, inv1);
                         if (lane == 0) {
                             s_inv[warp][2 * r] = inv0 * sp_code_scale<T>;
                             s_inv[warp][2 * r + 1] = inv1;
                         }
                     }
+                    // Digits have one last place for all of the share, 2^-28 of its largest value or less, and small values beside a large one would lose to
+                    // it what halves keep.  So the share goes in halves (sp_far) unless every 32 values that are not all zero, and half of all fours that are
+                    // not, hold one of 2^-6 of the largest or more.  (Normal activations and their products, as after SwiGLU, are so; one of 90 deviations or
+                    // more beside normal ones is not.)  Error of a result whose weight for the large ones is zero, of the 2-norm of its terms, Q4_0, one of R
+                    // deviations in every 512 values, digits / halves under one power of two a share / what leaves here: R = 60 8.6e-8 / 9.8e-8 / 8.6e-8,
+                    // 300 1.6e-7 / 9.8e-8 / 8.6e-8, 1e4 4.4e-6 / 9.8e-8 / 8.6e-8, 1e6 2.8e-4 / 3.9e-7 / 2.8e-7.  It costs 7 us of 17.5 (24576 x 4096), 60 of
+                    // 145 (Q6_K, 151936 x 5120), also where it is one warp's share alone.
 #pragma unroll
                     for (int r = 0; r < MPC; r++) {
+                        const uint32_t least = am[r] > (7u << 23) ? am[r] - (6u << 23) : 1u;
+                        sp::Spread spread;
 #pragma unroll
                         for (int p = 0; p < HELD; p++)
-                            if (2u * p < mine) write(v[r][p], s[r], s1[r], p, r, r < (int)cnt);
+                            if (2u * p < mine) {
+                                spread.look(peak(v[r][p]), least, lane);
+                                write(v[r][p], s[r], s1[r], p, r, r < (int)cnt);
+                            }
                         for (uint32_t p = HELD; 2 * p < mine; p++) {
                             float z[4];
                             load(r, p, z);
+                            spread.look(peak(z), least, lane);
                             write(z, s[r], s1[r], p, r, r < (int)cnt);
                         }
+                        far = far || (spread.far() && am[r] < 0x7F800000u);
                     }
                 } else {
                 // Four passes are in flight at a time: of one row, or of two or four rows where a row has fewer.
@@ -1256,7 +1443,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         const uint32_t r = min(rb + (j >> sh), cnt - 1);
-                        const size_t o = (size_t)(bt.ids ? (uint32_t)s_ord[e0 + r] / P.x_div : e0 + r) * P.k + kb;
+                        const size_t o = (size_t)(routed ? (uint32_t)s_ord[e0 + r] / P.x_div : e0 + r) * P.k + kb;
                         x[j] = P.x + o;
                         y[j] = P.x2 ? P.x2 + o : nullptr;
                     }
@@ -1318,6 +1505,10 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 }
                 }
                 __syncwarp();
+                if (INT && far) {
+                    at -= c.steps;
+                    break;
+                }
             }
 
             float acc[TM][NS][4];
@@ -1427,7 +1618,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                         }
                         // (an odd number of blocks: the second block of the last unit lies past the row)
                         const bool half = (u0 + uu) * 64 + 32 >= P.k;
-                        auto tiles = [&](auto NT) { sp_unit<T, ALN, decltype(NT)::value>(r0 + ub, r1 + ub, ul, t, g, tab, half, bf, cc, acc); };
+                        auto tiles = [&](auto NT) { sp_unit<T, ALN, decltype(NT)::value, false>(r0 + ub, r1 + ub, ul, t, g, tab, half, bf, cc, {1.f, 1.f}, acc); };
                         if (c.nt == 1) tiles(std::integral_constant<int, 1>{});
                         else if (TM == 2 || c.nt == 2) tiles(std::integral_constant<int, 2>{});
                         else if (c.nt == 3) tiles(std::integral_constant<int, TM == 2 ? 2 : 3>{});
@@ -1510,6 +1701,34 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             d2 = d1;
             d1 = i & 15u;
         }
+        // The chunks from a share on that digits do not do for, in halves.  (A loop of its own: in the other one it cost one row of Q4_K 1.4 us of 20 and two
+        // rows 2 us of 21, here up to 0.2 and 0.9.)
+        if constexpr (INT)
+            if (ok && at < last) {
+                cur = 0xFFFFFFFFu;
+                SpRing ring{full, empty, &abort_flag, base, slot, ph};
+                for (; ok && at < last; i++) {
+                    if (!wait(full[ring.slot], ring.ph, ST_WAIT_FULL_TIMEOUT)) break;
+                    __syncwarp();
+                    const SpChunk c = s_chunk[i & 15u];
+                    const SpOp &P = bt.op[c.op];
+                    const uint32_t u0 = rank * P.slice, k0 = 64u * u0;
+                    at += c.steps;
+                    if (c.key != cur) {
+                        cur = c.key;
+                        const size_t o = (size_t)c.e0 * P.k + k0;
+                        sp_far<T, ALN, MPC>(P.x + o, P.x2 ? P.x2 + o : nullptr, P.k, P.k > k0 ? P.k - k0 : 0u, c.cnt, c.un, warp, lane, xf, xs, ccb, cs, s_inv[warp], s_rel);
+                    }
+                    ok = sp_far_stages<T, ALN, MPC>(bt, c.op, u0, c.un, c.nt, ring, warp, lane, xf, ccb, tab, red + ((i & 3u) * kSpWarps + warp) * RS * 4u, s_inv[warp], s_rel) && ok;
+                    if (!ok) break;
+                    if (i >= 2 && ranks > 1 && !finish(i - 2, d2)) break;   // (the order of the steps is that of the loop above)
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sync_bar[i & 1u]);
+                    if (i >= 1 && !add(i - 1, d1)) break;
+                    d2 = d1;
+                    d1 = i & 15u;
+                }
+            }
         if (ok && i >= 1) ok = add(i - 1, d1);
         if (ok && ranks > 1 && i >= 2) ok = finish(i - 2, d2);
         if (ok && ranks > 1 && i >= 1) ok = finish(i - 1, d1);
@@ -1539,9 +1758,6 @@ struct SpShape {          // geometry of a launch
     uint32_t ranks, tr, nslots, grid;
     size_t smem;
 };
-
-// Two CTAs share an SM: 228 KB less 1 KB each for the system and the kernel's static 2.5 KB.
-constexpr size_t kSpSmem = 110 * 1024;
 
 template <int T> inline size_t sp_tail(uint32_t ranks, uint32_t tr, uint32_t mp, uint32_t xunits, SpBatch *b) {
     const size_t r = 16u * tr;

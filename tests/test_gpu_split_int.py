@@ -52,6 +52,48 @@ def test_error_against_64_bits(ctx, tname, outliers):
         assert np.linalg.norm(y - ref) <= 1.5e-7 * np.linalg.norm(ref)
 
 
+def same_scale(tname, k):
+    """Which values share a power of two where a share of K is taken in f16 halves: the 32 of a block (Q6_K: of two 16-value groups, 32 apart)."""
+    i = np.arange(k)
+    return i // 128 * 4 + i // 16 % 2 * 2 + i % 128 // 64 if tname == "Q6_K" else i // 32
+
+
+# Activations far larger than the others whose weights are zero: what is left of a result are the small ones.  For each output, of sum |w| |x|:
+# 2e-7 for the sums (some 30 additions one after another, each 2^-24 of a partial sum, which random signs keep below a tenth of that sum), and the
+# values beside a large one R lose 2^-38 R at most, halves under one power of two having a last place of 2^-24 of which the largest takes 2^13 or more.
+# (Q4_K: a zero weight is code times scale less offset, in f32: another 2^-21 R of the largest weight of its sub-block.)
+@pytest.mark.parametrize("tname", sorted(ALL))
+@pytest.mark.parametrize("large", ["some", "stretches"])
+@pytest.mark.parametrize("R", [30, 100, 1e3, 1e4, 1e5, 1e6, 1e8])
+def test_small_activations_beside_large_ones(ctx, tname, large, R):
+    gtype, otype = ALL[tname]
+    n, k = 600, 4096
+    rng = np.random.default_rng(int(R))
+    at = np.arange(8) * 512 + rng.integers(0, 512, 8) if large == "some" else np.flatnonzero(np.arange(k) // 256 % 2)
+    wf = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
+    if tname == "Q4_K":
+        wf = np.abs(wf)          # (a sub-block of positive weights has no offset, so that zero is among its values)
+    wf[:, at] = 0
+    wq = orc.quantize(otype, wf)
+    w = orc.dequantize(otype, wq).reshape(n, k).astype(np.float64)
+    assert not w[:, at].any()
+    x = normal_acts(1, 2, k)
+    x[0, at] = x[0, at] * np.float32(R) if large == "stretches" else np.float32(R) * np.sign(x[0, at])
+    top = np.abs(x[0, at]).max()
+    group = same_scale(tname, k)
+    beside = np.abs(w[:, np.isin(group, group[at])]).sum(1)
+    for rows in (x[:1], x):
+        y = ctx.matmul(gtype, wq, rows, n, k)
+        assert mx.last_kernel_name() == "qmv_split"
+        for r, row in enumerate(rows):
+            bound = 2e-7 * (np.abs(w) @ np.abs(row).astype(np.float64))
+            if r == 0:
+                bound += 2.0 ** -38 * top * beside
+                if tname == "Q4_K":
+                    bound += 2.0 ** -21 * top * np.abs(w).reshape(n, k // 32, 32).max(2)[:, at // 32].sum(1)
+            assert np.all(np.abs(y[r] - w @ row.astype(np.float64)) <= bound)
+
+
 def test_zero_and_tiny_rows(ctx):
     """A row of zeros, of the smallest numbers there are, and one of them among zeros: the scale takes two powers of two."""
     gtype, otype = TYPES["Q8_0"]
