@@ -178,12 +178,12 @@ struct Spread {
     __device__ __forceinline__ bool far() const { return __any_sync(0xffffffffu, lost) || 2 * held < some; }
 };
 // Two powers of two whose product brings amax (its bits; a number) into [2^13, 2^14), and those of the way back from units of the last digit.
-// (One factor would not be a normal number where amax is tiny.)  NaN for the way back where the run holds an infinity or a NaN.
+// (One factor would not be a normal number where amax is tiny.)
 __device__ __forceinline__ void pow2_int(uint32_t amax, float &s0, float &s1, float &inv0, float &inv1) {
     const int e = 13 + 127 - (int)(amax >> 23), a = e >> 1, b = e - a;
     s0 = __uint_as_float((uint32_t)(127 + a) << 23);
     s1 = __uint_as_float((uint32_t)(127 + b) << 23);
-    inv0 = amax >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : __uint_as_float((uint32_t)(127 - 15 - a) << 23);
+    inv0 = __uint_as_float((uint32_t)(127 - 15 - a) << 23);
     inv1 = __uint_as_float((uint32_t)(127 - b) << 23);
 }
 // Four numbers below 2^14 as four signed digits each, in units of 2^-15: l[0] + 256 l[1] + 2^15 (l[2] + 256 l[3]); l[i] holds digit i of all
@@ -689,36 +689,22 @@ template <int T, bool INT> __device__ __forceinline__ void sp_table_row(uint32_t
     }
 }
 
-// One product in f32, value by value: for results that are no numbers.
-template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const float *x, const float *x2, uint32_t k) {
+// One product of a Q4_K or Q5_K row in f32, value by value: for results that are no numbers.  Lane `part` of `parts` adds up every parts-th super-block.
+template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const float *x, uint32_t k, uint32_t part, uint32_t parts) {
     float acc = 0.f;
-    constexpr uint32_t QK = BlockTraits<T>::QK;
-    for (uint32_t b = 0; b < k / QK; b++, w += BlockTraits<T>::BYTES)
-        for (uint32_t e = 0; e < QK; e++) {
-            float v;
-            if constexpr (T == GT_Q4_0) {
-                v = __fmul_rn((float)((int)((w[2 + (e & 15u)] >> (4 * (e >> 4))) & 15u) - 8), half_bits_to_float(ld_u16(w)));
-            } else if constexpr (T == GT_Q8_0) {
-                v = __fmul_rn((float)(int8_t)w[2 + e], half_bits_to_float(ld_u16(w)));
-            } else if constexpr (T == GT_Q6_K) {
-                const uint32_t nh = e >> 7, q = (e >> 5) & 3u, l = e & 31u;
-                const uint32_t n = ((w[64 * nh + 32 * (q & 1u) + l] >> (4 * (q >> 1))) & 15u) | (((w[128 + 32 * nh + l] >> (2 * q)) & 3u) << 4);
-                const float d = __fmul_rn(half_bits_to_float(ld_u16(w + 208)), (float)(int8_t)w[192 + (e >> 4)]);
-                v = __fmul_rn(d, (float)((int)n - 32));
-            } else {
-                const uint32_t j = e >> 5, l = e & 31u;
-                uint32_t sc, mn;
-                q4k_scale_min(j, w + 4, sc, mn);
-                const float d = __fmul_rn(half_bits_to_float(ld_u16(w)), (float)sc), m = __fmul_rn(half_bits_to_float(ld_u16(w + 2)), (float)mn);
-                uint32_t q = (w[(T == GT_Q5_K ? 48 : 16) + 32 * (j >> 1) + l] >> (4 * (j & 1u))) & 15u;
-                if (T == GT_Q5_K) q |= ((w[16 + l] >> j) & 1u) << 4;
-                v = __fsub_rn(__fmul_rn(d, (float)q), m);
+    for (uint32_t b = part; b < k / 256; b += parts) {
+        const uint8_t *v = w + (size_t)b * BlockTraits<T>::BYTES;
+        for (uint32_t j = 0; j < 8; j++) {
+            uint32_t sc, mn;
+            q4k_scale_min(j, v + 4, sc, mn);
+            const float e = __fmul_rn(half_bits_to_float(ld_u16(v)), (float)sc), m = __fmul_rn(half_bits_to_float(ld_u16(v + 2)), (float)mn);
+            for (uint32_t l = 0; l < 32; l++) {
+                uint32_t q = (v[(T == GT_Q5_K ? 48 : 16) + 32 * (j >> 1) + l] >> (4 * (j & 1u))) & 15u;
+                if (T == GT_Q5_K) q |= ((v[16 + l] >> j) & 1u) << 4;
+                acc = fmaf(__fsub_rn(__fmul_rn(e, (float)q), m), x[256 * b + 32 * j + l], acc);
             }
-            const uint32_t i = b * QK + e;
-            float a = x[i];
-            if (x2) a = a / (1.0f + expf(-a)) * x2[i];
-            acc = fmaf(v, a, acc);
         }
+    }
     return acc;
 }
 
@@ -1207,21 +1193,25 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             const uint32_t pair = routed ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
             const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
             if (routed && s_id[pair] >= bt.n_experts) v = 0.f;   // an id that names no expert
-            if ((INT || NG != 0) && v != v) s_again = 1;
+            if (NG != 0 && v != v) s_again = 1;
             P.y[o] = v;
             for (uint32_t pr = 0; pr < P.n_peer; pr++) P.y_peer[pr][o] = v;
         };
-        [[maybe_unused]] auto again = [&](const SpChunk &d, uint32_t col, uint32_t row) {
+        [[maybe_unused]] auto again = [&](const SpChunk &d, uint32_t col, uint32_t row, uint32_t parts) {
             const SpOp &P = bt.op[d.op];
             const uint32_t grow = d.tile * 16u + (ALN ? row : (row & ~15u) + place(row & 15u));
             if (col >= d.cnt || row >= d.nt * 16u || grow >= P.n) return;
             const uint32_t pair = routed ? (uint32_t)s_ord[d.e0 + col] : d.e0 + col;
             const size_t o = (size_t)pair * P.y_ld + P.y_col0 + grow;
-            float v = P.y[o];
-            if (v == v) return;
-            v = sp_again<T>(P.w + (routed ? s_id[pair] * P.expert_stride : 0ull) + (uint64_t)grow * P.row_bytes,
-                            P.x + (size_t)(routed ? pair / P.x_div : pair) * P.k,
-                            P.x2 ? P.x2 + (size_t)(routed ? pair / P.x_div : pair) * P.k : nullptr, P.k);
+            if (P.y[o] == P.y[o]) return;
+            float v = sp_again<T>(P.w + (routed ? s_id[pair] * P.expert_stride : 0ull) + (uint64_t)grow * P.row_bytes,
+                                  P.x + (size_t)(routed ? pair / P.x_div : pair) * P.k, P.k, tid % parts, parts);
+            if (parts == 4) {
+                const uint32_t four = 0xFu << (lane & 28u);
+                v += __shfl_xor_sync(four, v, 1);
+                v += __shfl_xor_sync(four, v, 2);
+                if (tid & 3u) return;
+            }
             P.y[o] = v;
             for (uint32_t pr = 0; pr < P.n_peer; pr++) P.y_peer[pr][o] = v;
         };
@@ -1433,7 +1423,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                             spread.look(peak(z), least, lane);
                             write(z, s[r], s1[r], p, r, r < (int)cnt);
                         }
-                        far = far || (spread.far() && am[r] < 0x7F800000u);
+                        far = far || spread.far() || am[r] >= 0x7F800000u;   // (halves hold infinities)
                     }
                 } else {
                 // Four passes are in flight at a time: of one row, or of two or four rows where a row has fewer.
@@ -1732,17 +1722,19 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         if (ok && i >= 1) ok = add(i - 1, d1);
         if (ok && ranks > 1 && i >= 2) ok = finish(i - 2, d2);
         if (ok && ranks > 1 && i >= 1) ok = finish(i - 1, d1);
-        // An infinite activation has no digits, and its products with codes and offset may cancel where the weight has a sign: results that
-        // are no numbers are formed again, weight by weight, each by the thread that stored it.  (Not on the way: the call costs the loop registers.)
-        if constexpr (INT || NG != 0)
-            if (ok && s_again) {
-                const uint32_t rows = ranks == 1 ? R : share, per = INT && ranks == 1 ? 4u : 1u;   // (threads a result, the first of which stored it)
-                for (uint32_t at = first; tid % per == 0 && at < last;) {
+        // An infinite activation's products with codes and offset may cancel where the weight has a sign: results that are no numbers are formed again,
+        // weight by weight, each by the threads that stored it (integers: by the four lanes that added it up).  (Not on the way: the call costs the loop registers.)
+        if constexpr (NG != 0) {
+            __syncwarp();
+            if (__any_sync(0xffffffffu, ok && s_again)) {
+                const uint32_t rows = ranks == 1 ? R : share, parts = INT && ranks == 1 ? 4u : 1u;
+                for (uint32_t at = first; at < last;) {
                     const SpChunk c = chunk(at);
                     at += c.steps;
-                    for (uint32_t q = tid / per; q < mp * rows; q += 256 / per) again(c, q / rows, (ranks == 1 ? 0u : rank * share) + q % rows);
+                    for (uint32_t q = tid / parts; q < mp * rows; q += 256 / parts) again(c, q / rows, (ranks == 1 ? 0u : rank * share) + q % rows, parts);
                 }
             }
+        }
     }
     if (abort_flag)   // let copies in flight land before the CTA's shared memory is released
         for (int i = 0; i < 200; i++) __nanosleep(5000);

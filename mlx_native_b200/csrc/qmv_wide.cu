@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(WdShape<RG, S>::threads, RG == 4 ? 2 : 1) qmv_
             v[e] *= inv;
             // (an infinite activation times codes and offset may cancel where the weight has a sign: formed again, weight by weight)
             if (v[e] != v[e] && e < (int)cnt)
-                v[e] = sp_again<GT_Q4_K>(P.w + (size_t)(n0 + row + e) * (nsb * kWdSuper), P.x + (size_t)out * P.k, nullptr, P.k);
+                v[e] = sp_again<GT_Q4_K>(P.w + (size_t)(n0 + row + e) * (nsb * kWdSuper), P.x + (size_t)out * P.k, P.k, 0, 1);
         }
         if (cnt == 4 && ((uintptr_t)y & 15u) == 0) {
             *reinterpret_cast<float4 *>(y) = make_float4(v[0], v[1], v[2], v[3]);
