@@ -37,6 +37,7 @@ bool qmv_split_fits(int ggml_type, const QmvArgs &a, int sm_count, SpPick *pick)
     if (((uintptr_t)a.x & 7u) || ((uintptr_t)a.x2 & 7u) || ((uintptr_t)a.w & 1u)) return false;
     const bool aligned = qmv_split_aligned(ggml_type, a);
     if (kq && (!aligned || a.x2)) return false;
+    if (a.x2 && !a.ids) return false;   // (the fused SwiGLU is expert-routed)
     if (ggml_type == GT_Q5_K && !a.ids) return false;
     if ((uint64_t)(a.k / ggml_qk(ggml_type)) * ggml_block_bytes(ggml_type) >= (1ull << 31)) return false;
     uint32_t mp = a.m <= 1 ? 1u : a.m <= 2 ? 2u : a.m <= 4 ? 4u : 8u, ranks = 8;

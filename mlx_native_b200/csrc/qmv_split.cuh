@@ -501,9 +501,9 @@ __device__ __forceinline__ void sp_unit(uint32_t a0, uint32_t a1, uint32_t u, ui
 // take three operations for eight (with f16 they take twelve), sums of a block are exact, and the digits hold 28 bits of the largest activation.
 // The columns of a multiply are (first | second scale group, digit) of one activation row; a column's B registers are zero outside its group, so
 // one accumulator serves both blocks of a unit (Q6_K, whose scales change every 16 values: both halves of one multiply), and a lane scales its
-// columns with the one scale of their group.  Codes are taken 16 times (Q4_0, Q4_K), 8 times (Q5_K), 4 times (Q6_K) as large:
+// columns with the one scale of their group.  Codes are taken 16 times (Q4_0, Q4_K) or 4 times (Q6_K) as large:
 // that centres them without an addition (the top bit of the byte changes sign), and sp_code_scale takes it back.  bf: B registers [set][word].
-template <int T> constexpr float sp_code_scale = T == GT_Q8_0 ? 1.f : T == GT_Q6_K ? 0.25f : T == GT_Q5_K ? 0.125f : 0.0625f;
+template <int T> constexpr float sp_code_scale = T == GT_Q8_0 ? 1.f : T == GT_Q6_K ? 0.25f : 0.0625f;
 // alike: all rows start at the same half of a word.  OFF: the unit's bytes within a stage from the warp's first unit on.  c: kBias four times, in registers (as an immediate every multiply would
 // copy it into four of them).
 template <int T, bool ALN, uint32_t OFF, int NT, int NS, int TM>
@@ -572,27 +572,20 @@ __device__ __forceinline__ void sp_unit_int(uint32_t a0, uint32_t a1, uint32_t u
                 sp::scaled(acc[j][s], r, d[0], d[1]);
             }
         });
-    } else if constexpr (T == GT_Q4_K || T == GT_Q5_K) {
-        constexpr bool Q5 = T == GT_Q5_K;
-        const uint32_t pu = u & 3u, q0 = a0 + 32 * pu + 4 * t, h0 = a0 + 4 * t;
+    } else if constexpr (T == GT_Q4_K) {
+        const uint32_t q0 = a0 + 32 * (u & 3u) + 4 * t;
         static_for<0, NT>([&](auto J) {
             constexpr int j = decltype(J)::value;
             uint32_t a[2][4], p[2][2];   // codes (first sub-block: low nibbles, second: high ones); scale and offset (sp_table_row) of rows g, g + 8
             static_for<0, 2>([&](auto H) {
                 constexpr int h = decltype(H)::value;
-                constexpr uint32_t o = OFF + j * TS + h * R8, q = o + (Q5 ? 48u : 16u);
+                constexpr uint32_t q = OFF + j * TS + h * R8 + 16u;
                 lds64i<j * 256u + h * 128u>(tab, p[h][0], p[h][1]);
                 static_for<0, 2>([&](auto E) {   // first, second 16 elements
                     constexpr int e = decltype(E)::value;
                     const uint32_t x = lds32i<q + 16 * e>(q0);
-                    if constexpr (Q5) {
-                        const uint32_t v = lds32i<o + 16 + 16 * e>(h0) >> (2 * pu);
-                        a[0][2 * e + h] = ((x << 3) & 0x78787878u) | (((v << 7) & 0x80808080u) ^ 0x80808080u);
-                        a[1][2 * e + h] = ((x >> 1) & 0x78787878u) | (((v << 6) & 0x80808080u) ^ 0x80808080u);
-                    } else {
-                        a[0][2 * e + h] = ((x << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
-                        a[1][2 * e + h] = (x & 0xF0F0F0F0u) ^ 0x80808080u;
-                    }
+                    a[0][2 * e + h] = ((x << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+                    a[1][2 * e + h] = (x & 0xF0F0F0F0u) ^ 0x80808080u;
                 });
             });
 #pragma unroll
@@ -838,9 +831,9 @@ __global__ void __launch_bounds__(256) qmv_pack_kernel(const __grid_constant__ S
 
 // A warp's share of up to two activation rows in halves, where digits would lose its small values (see `far` in the kernel): a power of two for
 // every 32 values (lanes 8 j .. 8 j + 7 hold them), as one for the share (inv: its inverse) and one beside it for the 32, whose inverse's exponent goes to
-// rel[unit][row][32 values].  x, x2: the entry's first row, from the rank's slice on; left: values from there to the end of the row.
+// rel[unit][row][32 values].  x: the entry's first row, from the rank's slice on; left: values from there to the end of the row.
 template <int T, bool ALN, int MPC>
-__device__ __forceinline__ void sp_far(const float *x, const float *x2, uint32_t k, uint32_t left, uint32_t cnt, uint32_t un, uint32_t warp, uint32_t lane,
+__device__ __forceinline__ void sp_far(const float *x, uint32_t k, uint32_t left, uint32_t cnt, uint32_t un, uint32_t warp, uint32_t lane,
                                        uint32_t xf, uint32_t xs, [[maybe_unused]] uint32_t ccb, [[maybe_unused]] uint32_t cs, float *inv, uint8_t *rel) {
     constexpr int NG = SpTraits<T>::NG;
     const uint32_t q = (lane >> 2) & 3u, tt = lane & 3u, hf = lane >> 4;
@@ -851,7 +844,7 @@ __device__ __forceinline__ void sp_far(const float *x, const float *x2, uint32_t
         if (u >= un) return;
         const uint32_t o = T == GT_Q6_K ? 256u * (u >> 2) : 64u * u;
         const size_t at = (size_t)row * k + o;
-        sp_act(x + at, x2 ? x2 + at : nullptr, p0, p1, o + p0 < left, o + p1 < left, v);
+        sp_act(x + at, nullptr, p0, p1, o + p0 < left, o + p1 < left, v);
     };
     for (uint32_t row = 0; row < cnt; row++) {
         uint32_t am = 0;
@@ -1281,7 +1274,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
         if constexpr (INT) {
             c0 = chunk(first < last ? first : 0);
             const SpOp &P = bt.op[c0.op];
-            asm volatile("" ::"l"(P.x), "l"(P.x2), "r"(P.k), "r"(P.slice));
+            asm volatile("" ::"l"(P.x), "r"(P.k), "r"(P.slice));
         }
         if (!routed) grid_dependency_wait();   // the activations belong to the kernels ahead until those are done
         uint32_t at = first;
@@ -1301,7 +1294,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             at += c.steps;
             const SpOp &P = bt.op[c.op];
             const uint32_t u0 = rank * P.slice, un = c.un, e0 = c.e0, cnt = c.cnt, key = c.key;
-            const uint32_t ex = routed && !ALN ? s_id[s_ord[e0]] : 0u;
+            [[maybe_unused]] const uint32_t ex = routed && !ALN ? s_id[s_ord[e0]] : 0u;
             if (!INT && key != cur && bt.packed) {
                 // the rows' slices come ready from the pack kernel's scratch area
                 if (cur != 0xFFFFFFFFu && !csync()) break;   // nobody reads the entry before any more
@@ -1372,7 +1365,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                         v[0] = v[1] = v[2] = v[3] = 0.f;
                         const uint32_t o = 1024u * p, at = from[r] + o;
                         if (2 * p + hf >= mine) return;
-                        sp_act(P.x + at, P.x2 ? P.x2 + at : nullptr, p0, p1, kb + o + p0 < P.k, kb + o + p1 < P.k, v);
+                        sp_act(P.x + at, nullptr, p0, p1, kb + o + p0 < P.k, kb + o + p1 < P.k, v);
                     };
                     auto peak = [](const float (&v)[4]) { return sp::peak_bits(v); };
                     constexpr int HELD = 4;   // passes whose values stay in registers; those beyond are loaded again
@@ -1513,7 +1506,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                     constexpr int NT = decltype(N)::value;
                     for (uint32_t us = 0; us == 0 || us < un; us += SU) {
                         const uint32_t off = (u0 + us) / 4 * (uint32_t)K::B256;
-                        const uint32_t wl = ALN ? 0u : ((uint32_t)(uintptr_t)P.w + (ex < bt.n_experts ? ex : 0u) * (uint32_t)P.expert_stride + off) & 15u;
+                        const uint32_t wl = ALN ? 0u : ((uint32_t)(uintptr_t)P.w + off) & 15u;
                         const uint32_t rb15 = P.row_bytes & 15u;
                         auto lead = [&](uint32_t row) { return ALN ? (T == GT_Q6_K ? off & 15u : 0u) : (wl + place(row & 15u) * rb15) & 15u; };
                         const uint32_t stage = base + slot * STAGE + (TABLE ? (warp >> 2) * (uint32_t)K::B256 : warp * UB);
@@ -1707,7 +1700,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                     if (c.key != cur) {
                         cur = c.key;
                         const size_t o = (size_t)c.e0 * P.k + k0;
-                        sp_far<T, ALN, MPC>(P.x + o, P.x2 ? P.x2 + o : nullptr, P.k, P.k > k0 ? P.k - k0 : 0u, c.cnt, c.un, warp, lane, xf, xs, ccb, cs, s_inv[warp], s_rel);
+                        sp_far<T, ALN, MPC>(P.x + o, P.k, P.k > k0 ? P.k - k0 : 0u, c.cnt, c.un, warp, lane, xf, xs, ccb, cs, s_inv[warp], s_rel);
                     }
                     ok = sp_far_stages<T, ALN, MPC>(bt, c.op, u0, c.un, c.nt, ring, warp, lane, xf, ccb, tab, red + ((i & 3u) * kSpWarps + warp) * RS * 4u, s_inv[warp], s_rel) && ok;
                     if (!ok) break;

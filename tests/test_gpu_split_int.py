@@ -35,6 +35,51 @@ def test_shapes(ctx, tname, n, k, m):
     assert np.array_equal(y.view(np.uint32), ctx.matmul(gtype, wq, x, n, k).view(np.uint32))
 
 
+# More than 64 units (64 values of K) on a rank: activations beyond the passes that stay in registers are loaded again, in digits and (with a large
+# activation) in halves.  80 to 84 units on each of eight ranks; rows on 16-byte boundaries, every other one, and by row copies.
+@pytest.mark.parametrize("tname,n,k", [("Q4_0", 34, 40960), ("Q4_0", 34, 41088), ("Q4_0", 33, 41088), ("Q8_0", 34, 40960), ("Q8_0", 18, 41088),
+                                       ("Q8_0", 17, 41088), ("Q6_K", 34, 40960), ("Q6_K", 34, 41984), ("Q6_K", 33, 41984), ("Q4_K", 34, 40960)])
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("large", [0, 1e4])
+def test_long_rows(ctx, tname, n, k, m, large):
+    gtype, otype = ALL[tname]
+    wq = normal_weights(n + k, n, k, otype)
+    x = normal_acts(n + m, m, k)
+    if large:
+        x[-1, ::513] = large
+    y = ctx.matmul(gtype, wq, x, n, k)
+    assert mx.last_kernel_name() == "qmv_split"
+    y_ref, ad = orc.qmatmul(otype, wq, x, n, k, nthreads=8)
+    assert norm_err(y, y_ref, ad) <= MV_TOL
+
+
+@pytest.mark.parametrize("tname", sorted(ALL))
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("shapes", [[(5000, 2048), (70, 256), (3000, 2048), (2600, 1024)], [(100, 4096), (33, 512), (16, 4096), (257, 1024)]])
+@pytest.mark.parametrize("large", [(), (1,), (0, 2)])
+def test_products_of_different_activations_in_one_launch(ctx, tname, m, shapes, large):
+    """Shares that cross from one product to the next take that one's activations, in digits or halves; of the products of few rows, some ranks of
+    a cluster have no units of the shorter ones."""
+    gtype, otype = ALL[tname]
+    d = ctx.device
+    if tname == "Q6_K":
+        shapes = [(n, max(k, 2048)) for n, k in shapes]   # (rows on 16-byte boundaries: one launch)
+    ws = [normal_weights(i, n, k, otype) for i, (n, k) in enumerate(shapes)]
+    xs = [normal_acts(i, m, k) * np.float32(4.0 ** i) for i, (n, k) in enumerate(shapes)]
+    for i in large:
+        xs[i][:, ::300] *= np.float32(1e4)
+    bufs = [(ctx.buf(x, mx.DType.F32), ctx.buf(w, mx.DType.U8), d.alloc_buffer(m * n * 4, mx.DType.F32)) for x, w, (n, k) in zip(xs, ws, shapes)]
+    mx.reset_counters()
+    enc = d.command_encoder()
+    for (xb, wb, yb), (n, k) in zip(bufs, shapes):
+        mx.quantized_matmul_ggml(enc, ctx.registry, d, xb, wb, yb, mx.GgmlQuantizedMatmulParams(m, n, k, gtype))
+    enc.commit_and_wait()
+    assert mx.last_kernel_name() == "qmv_split" and mx.kernel_launch_count() == 1
+    for (xb, wb, yb), w, x, (n, k) in zip(bufs, ws, xs, shapes):
+        y_ref, ad = orc.qmatmul(otype, w, x, n, k, nthreads=8)
+        assert norm_err(yb.as_slice(np.float32).reshape(m, n), y_ref, ad) <= MV_TOL
+
+
 # Products of codes and digits and the sums of a block are exact; digits leave out less than 2^-29 of the largest activation of a warp's share, which
 # for normal activations is 2^-27 of one, and the f32 sums of a result have at most a few dozen terms one after another: 1.5e-7 (2^-23 = 1.2e-7).
 @pytest.mark.parametrize("tname", sorted(ALL))
