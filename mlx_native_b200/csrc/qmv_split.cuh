@@ -1368,7 +1368,9 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                         sp_act(P.x + at, nullptr, p0, p1, kb + o + p0 < P.k, kb + o + p1 < P.k, v);
                     };
                     auto peak = [](const float (&v)[4]) { return sp::peak_bits(v); };
-                    constexpr int HELD = 4;   // passes whose values stay in registers; those beyond are loaded again
+                    // Passes whose values stay in registers; those beyond are loaded again.  (Two rows have no registers for four: Q4_K 24576 x 4096 28.0 us, so
+                    // 26.6; Q4_0 21.4, 20.8.)
+                    constexpr int HELD = MPC == 2 ? 2 : 4;
                     float v[MPC][HELD][4], s[MPC], s1[MPC];
                     uint32_t am[MPC];
 #pragma unroll
@@ -1685,7 +1687,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
             d1 = i & 15u;
         }
         // The chunks from a share on that digits do not do for, in halves.  (A loop of its own: in the other one it cost one row of Q4_K 1.4 us of 20 and two
-        // rows 2 us of 21, here up to 0.2 and 0.9.)
+        // rows 2 us of 21.)
         if constexpr (INT)
             if (ok && at < last) {
                 cur = 0xFFFFFFFFu;

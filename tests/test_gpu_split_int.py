@@ -35,8 +35,8 @@ def test_shapes(ctx, tname, n, k, m):
     assert np.array_equal(y.view(np.uint32), ctx.matmul(gtype, wq, x, n, k).view(np.uint32))
 
 
-# More than 64 units (64 values of K) on a rank: activations beyond the passes that stay in registers are loaded again, in digits and (with a large
-# activation) in halves.  80 to 84 units on each of eight ranks; rows on 16-byte boundaries, every other one, and by row copies.
+# More than 64 units (64 values of K) on a rank, 32 with two rows: activations beyond the passes that stay in registers are loaded again, in digits and
+# (with a large activation) in halves.  80 to 84 units on each of eight ranks; rows on 16-byte boundaries, every other one, and by row copies.
 @pytest.mark.parametrize("tname,n,k", [("Q4_0", 34, 40960), ("Q4_0", 34, 41088), ("Q4_0", 33, 41088), ("Q8_0", 34, 40960), ("Q8_0", 18, 41088),
                                        ("Q8_0", 17, 41088), ("Q6_K", 34, 40960), ("Q6_K", 34, 41984), ("Q6_K", 33, 41984), ("Q4_K", 34, 40960)])
 @pytest.mark.parametrize("m", [1, 2])
