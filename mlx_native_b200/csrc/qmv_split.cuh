@@ -1847,21 +1847,25 @@ template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool 
             if ((force_c && !routed && (int)c != force_c) || (force_tr && (int)tr != force_tr)) continue;
             const size_t stage = (size_t)tr * 16 * sp_pitch<T>(aln), tail = sp_tail<T>(c, tr, mp, (slice + 1) & ~1u, nullptr);
             if (tail + 2 * stage + 128 > kSpSmem) continue;
-            const double slots = (double)((kSpSmem - 128 - tail) / stage);
-            // Fitted to 1024, 4096 and 24576 x 4096 and 4096 x 12288, all types: a chunk costs waits and sums, a unit of a warp what a lone
-            // multiply takes to come through and a share per tile; ranks wait for one another, in f16 with eight rows for 4.5 us a chunk
-            // where there are four of them; one or two rows are split by every CTA.
-            const double ncl = (double)(2 * sm_count / (int)c), chunks = routed || mp > 4 ? ceil(ceil((double)tiles / tr) / ncl) : ceil(ceil((double)tiles / ncl) / tr),
-                         share = routed || mp > 4 ? chunks * tr : ceil((double)tiles / ncl), units = ceil(slice / 8.0);
+            const double units = ceil(slice / 8.0);
             double cost;
-            if (mp <= 2) {
-                const double tile = (T == GT_Q6_K ? 0.38 : T == GT_Q8_0 ? 0.35 : T == GT_Q4_0 ? 0.19 : 0.25) * (mp == 2 ? 1.3 : 1.0);
-                cost = (units > 8 ? 0.2 : 0.13) * units * mp + chunks * 0.5 + units * (chunks * 0.12 + share * tile) + (c == 1 ? 0.0 : c == 2 ? 0.8 : c == 4 ? 1.5 : 2.2);
+            if (mp <= 2 && !routed) {   // in integers
+                // Every CTA splits the activations; a chunk costs waits and sums, a unit of a warp a share per tile; ranks wait for one another, and there are
+                // fewer clusters than CTAs would do for (71 of four and 33 of eight on 148 SMs).  Fitted to 192 products (four types, one and two rows,
+                // 1024 to 49152 rows of 1024 to 12288 values) timed at every geometry: what is taken is within 5 percent of the fastest for 177 of them, 1.2 percent
+                // slower on average, 17 at most (Q8_0, two rows, three of 4096 x 4096; profiles/qmv_split_geometry.md).
+                const double ncl = fmax(1.0, floor((double)(2 * sm_count / (int)c) * (c == 4 ? 0.96 : c == 8 ? 0.9 : 1.0))), share = ceil((double)tiles / ncl), chunks = ceil(share / tr);
+                const double tile = (T == GT_Q4_0 ? 0.2 : T == GT_Q8_0 ? 0.28 : T == GT_Q6_K ? 0.29 : 0.32) * (mp == 2 ? 1.3 : 1.0);
+                cost = units * (mp == 2 ? 0.71 : 0.31) + chunks * (1.3 + 0.03 * units) + units * share * tile + (c == 1 ? 0.0 : (c == 2 ? 1.2 : c == 4 ? 2.7 : 3.5) + 0.05 * chunks);
             } else {
+                // Fitted to 1024, 4096 and 24576 x 4096 and 4096 x 12288, all types: a chunk costs waits and sums, a unit of a warp a share per tile; ranks wait for
+                // one another, with eight rows for 4.5 us a chunk where there are four of them.
+                const double slots = (double)((kSpSmem - 128 - tail) / stage), ncl = (double)(2 * sm_count / (int)c);
+                const double chunks = routed || mp > 4 ? ceil(ceil((double)tiles / tr) / ncl) : ceil(ceil((double)tiles / ncl) / tr),
+                             share = routed || mp > 4 ? chunks * tr : ceil((double)tiles / ncl);
                 const double tile = (T == GT_Q6_K ? 0.3 : 0.23) * (mp > 4 ? 1.5 : 1.0);
-                cost = (packed ? 1.0 : 0.3 + 0.27 * units) + chunks * (mp > 4 && c == 4 ? 4.5 : 1.9) + share * tile * units + (c > 1 ? 0.3 : 0.0);
+                cost = (packed ? 1.0 : 0.3 + 0.27 * units) + chunks * (mp > 4 && c == 4 ? 4.5 : 1.9) + share * tile * units + (c > 1 ? 0.3 : 0.0) + (slots < 3 ? 0.3 : 0.0);
             }
-            if (slots < 3) cost += mp == 2 ? 1.0 : 0.3;
             if (cost < best) {
                 best = cost;
                 pick = {c, tr};
