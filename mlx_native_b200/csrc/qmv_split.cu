@@ -69,20 +69,23 @@ bool qmv_split_supported(int ggml_type, const QmvArgs &a, int sm_count) {
 // starts 1 to 3 us later and has the higher rate, and its time grows evenly, where the other one's is a number of passes over the chip:
 // what decides is how full those passes are (`fill`, qmv_mma_fill) and how much there is to read.  Graph replay of dependent
 // launches, us with the register-level kernel (one mat-vec of three or four rows: the tensor-memory kernel) / with this one:
-//   (one and two rows: with f16; in integers, as they leave now, the right-hand figures of one row are, 6144 rows 7.6, 8.9, 10.6, 8.5; 8192 rows (0.86) 8.6, 9.2,
-//   13.3, 9.9 against 8.6, 10.1, 11.7, 9.2 with the register-level kernel; 12288 10.1, 13.2, 15.0, 11.3; 24576 16.4, 24.3, 25.6, 19.3; 4096 x 12288 11.5, 15.7, 15.5, 12.8; of
-//   two rows, 12288 18.0, 17.1, 19.7, 15.1; 24576 21.0, 29.0, 33.8, 26.4.  Three products or more of one row (q, k and v, 25 M values) start
-//   2 us later with this kernel, whose CTAs cross from one to the next.)
-//   one row    4096 values wide   6144 rows (fill 0.65)   10240 (0.54)   12288 (0.65)   14336 (0.76)   16384 (0.86)   24576 (0.65)
-//     Q4_0                        7.6 / 8.6               12.4 / 11.5    12.7 / 11.7    12.7 / 13.1    13.3 / 13.4    23.9 / 19.5
-//     Q8_0                        8.5 / 8.4               14.2 / 11.1    13.7 / 11.9    13.7 / 14.3    14.7 / 14.9    25.1 / 20.6
-//     Q6_K                        11.1 / 11.2             17.9 / 15.8    18.0 / 16.1    17.8 / 18.7    18.0 / 19.1    32.7 / 27.1
-//     Q4_K                        8.1 / 10.0              14.2 / 14.1    14.2 / 14.2                   14.2 / 16.3    26.1 / 24.1
+//   one row    4096 values wide   5120 rows     8192 (fill 0.86)   10240 (0.54)   12288 (0.65)   14336 (0.76)   16384 (0.86)   18432 (0.97)   20480 (0.54)   32768 (0.86)
+//     Q4_0                        7.7 / 7.2     8.6 / 8.7          12.7 / 9.6     12.9 / 10.1    13.2 / 10.8    14.0 / 11.6    15.0 / 12.5    23.4 / 14.2    26.2 / 19.9
+//     Q8_0                        8.7 / 8.3     10.2 / 10.4        14.8 / 11.9    15.4 / 13.2    16.0 / 15.7    16.6 / 16.7    18.6 / 18.5    27.8 / 20.2    30.9 / 30.1
+//     Q6_K                        11.1 / 10.9   11.6 / 12.0        18.4 / 14.5    18.6 / 14.9    18.9 / 16.9    19.3 / 18.1    19.9 / 19.3    32.2 / 22.9    36.5 / 30.9
+//     Q4_K                        8.3 / 9.1     9.2 / 10.0         14.1 / 11.3    14.2 / 11.6    14.5 / 13.0    15.4 / 14.0    16.4 / 14.4    26.0 / 17.3    28.6 / 22.1
 //   two rows
-//     Q4_0                        9.1 / 10.7              13.7 / 13.3    13.7 / 13.7    13.7 / 18.4    14.4 / 18.1    25.5 / 22.6
-//     Q8_0                        9.7 / 11.0              15.3 / 14.4    15.2 / 15.1    15.2 / 18.9    15.4 / 19.1    28.1 / 25.5
-//     wide, 4096 rows (0.86), one / two rows of Q6_K: 8192 values 13.2 / 13.0, 16.5 / 17.2, 12288 17.8 / 16.1, 23.9 / 21.0 (the others
-//     gain nothing: Q4_0 12.7 / 12.5, 16.8 / 17.4, Q8_0 13.7 / 13.5, 18.3 / 18.1)
+//     Q4_0                        9.2 / 8.9     9.9 / 10.9         13.9 / 12.8    13.9 / 13.7    14.1 / 14.8    15.1 / 15.4    16.2 / 16.4    26.5 / 18.7    28.1 / 26.2
+//     Q8_0                        10.1 / 9.5    11.0 / 11.2        16.0 / 15.0    16.4 / 16.7    17.0 / 17.4    17.5 / 19.1    19.1 / 20.9    29.6 / 23.9    32.6 / 33.4
+//     Q6_K                        13.3 / 12.5   13.9 / 14.0        20.3 / 18.4    20.6 / 19.7    20.8 / 21.2    21.3 / 22.3    22.0 / 23.7    37.2 / 26.9    40.4 / 37.9
+//     Q4_K                        9.9 / 10.7    10.4 / 14.4        15.3 / 14.8    15.4 / 16.3    15.7 / 18.9    16.5 / 19.8    17.7 / 21.1    28.5 / 22.2    30.7 / 32.6
+//   of other widths, one row: 4096 x 12288 (0.86) 13.0 / 11.0, 14.9 / 15.4, 18.9 / 15.9, 15.1 / 13.1; 8192 x 12288 (0.86) 20.9 / 18.5, 24.5 / 27.2, 29.8 / 27.5, 22.8 / 19.8;
+//     49152 x 1024 (0.86) 11.9 / 10.6, 13.8 / 13.9, 16.6 / 16.4, 12.7 / 12.6; 128256 x 1024 (0.97) 25.8 / 20.6, 29.7 / 28.6, 36.5 / 36.6, 27.9 / 26.2;
+//     24576 x 2048 (0.65) 13.6 / 10.7, 15.6 / 13.9, 19.3 / 15.4, 14.8 / 12.8; three of 4096 x 4096 (0.65) 13.3 / 11.3, 15.4 / 15.2, 19.0 / 15.9, 14.6 / 12.5, of 2048 x 4096 8.1 / 8.2,
+//     8.9 / 11.1, 11.5 / 11.6, 8.7 / 9.8
+//   of two rows: 4096 x 12288 17.4 / 14.2, 19.3 / 17.2, 25.1 / 19.4, 19.9 / 19.1; 8192 x 8192 (0.86) 17.2 / 16.1, 18.9 / 19.6, 24.4 / 22.8, 18.4 / 21.4; 8192 x 12288 24.0 / 24.3, 27.2 / 29.3,
+//     35.7 / 31.3, 26.1 / 28.3; 49152 x 1024 12.5 / 13.2, 14.6 / 15.9, 17.8 / 20.0, 13.5 / 15.1; 24576 x 2048 14.6 / 12.6, 17.3 / 15.3, 21.3 / 19.1, 15.9 / 15.1; twice 14336 x 2048 (0.76)
+//     15.1 / 13.4, 17.8 / 16.5, 22.0 / 20.2, 16.5 / 17.2
 //   four rows  a mat-vec: 3072 rows 8.6 / 8.8, 4096 9.9 / 9.0, 12288 17.4 / 16.5 (Q4_0); 5120 x 5120 12.7 / 13.5, 4096 x 8192 13.7 / 15.5;
 //              several: 4096 + 1024 + 1024 rows (0.65) 11.7 / 10.7, twice 6144 (0.65) 15.8 / 16.6, twice 12288 (0.65) 30.1 / 25.7, twice 8192
 //              (0.86) 16.3 / 18.9.  Of different widths, 12288 x 2048 + 12288 x 4096: 19.9 / 22.4, one row of Q6_K 20.4 / 22.5
@@ -105,15 +108,16 @@ bool qmv_split_pays(int ggml_type, const QmvArgs *ops, int nops, double fill) {
     constexpr uint64_t M = 1u << 20;
     const bool q4k = ggml_type == GT_Q4_K;
     if (kmin != kmax) return false;   // (the other kernel deals out work by K stages, and its passes are fuller than `fill` says)
-    // One and two rows, in integers.  Short rows leave a chunk little to do between its sums: 128256 x 1024, one row, Q4_0 26.1 / 20.9, Q8_0 30.3 / 29.3, but
-    // Q6_K 36.7 / 37.5; two rows of 2048 and 2560 values, Q4_0 15.3 / 14.2, Q6_K 70.6 / 64.5, but Q8_0 22.0 / 24.0, Q4_K 54.0 / 56.0.  (14336 x 2048 twice,
-    // one row of Q4_0: 14.3 / 10.4.)
+    // One and two rows, in integers.  (What is more than 5 percent faster here and still leaves by the other kernel: Q4_K of one row from 40 M on, two rows of
+    // 10240 to 20480 x 4096 of the other types below the limits, long rows of few.)
     if (q4k && m <= 2) return fill <= 0.7 && values >= 72 * M && (m == 1 || kmax >= 4096);
     if (m <= 1 && nops > 2) return values >= 40 * M;
     if (m <= 1 && ggml_type == GT_Q6_K && kmax < 2048) return false;
-    if (m <= 1) return values >= (fill > 0.7 ? (ggml_type == GT_Q8_0 ? 60 * M : 40 * M) : ggml_type == GT_Q8_0 ? 30 * M : 24 * M);
-    if (m <= 2 && ggml_type == GT_Q8_0) return values >= 90 * M && kmax >= 4096;
-    if (m <= 2) return values >= (ggml_type == GT_Q6_K ? 46 * M : 60 * M);
+    if (m <= 1 && ggml_type == GT_Q8_0) return fill <= 0.7 ? values >= 30 * M : values >= 60 * M && kmax <= 8192;
+    if (m <= 1) return values >= (fill > 0.7 ? 40 * M : 24 * M);
+    if (m <= 2 && ggml_type == GT_Q8_0) return fill <= 0.7 && values >= 72 * M && kmax >= 4096;
+    if (m <= 2 && ggml_type == GT_Q6_K) return kmax >= 2048 && values >= (fill > 0.8 && kmax <= 4096 ? 90 * M : 40 * M);
+    if (m <= 2) return values >= 60 * M && (fill <= 0.7 || kmax <= 8192);
     if (q4k && m <= 4) return kmax >= 4096 && values >= 14 * M && (fill <= 0.6 || (fill <= 0.7 && values >= 72 * M));
     if (q4k) return fill <= 0.6 && (m <= 8 || fill <= 0.25 || (m + 7) / 8 * 16 <= 3 * m);
     if (m > 4) return false;

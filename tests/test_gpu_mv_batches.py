@@ -72,3 +72,19 @@ def test_routed_rows_of_few_pairs_have_the_same_bits(ctx, tname, n, k):
     for rows in (1, 3, 8, 15):
         some, _ = ctx.matmul_id(gtype, w, w.size // E, x[:rows], ids[:rows], 1, n, k, E)
         assert np.array_equal(some.view(np.uint32), whole[:rows].view(np.uint32)), rows
+
+
+# one and two rows: on either side of the lines between the register-level and the split kernel (csrc/qmv_split.cu: qmv_split_pays)
+@pytest.mark.parametrize("tname,m,n,k,kernel", [
+    ("Q8_0", 2, 20480, 4096, "qmv_split"), ("Q8_0", 2, 32768, 4096, "qmv_mma"), ("Q6_K", 2, 10240, 4096, "qmv_split"), ("Q6_K", 2, 18432, 4096, "qmv_mma"),
+    ("Q6_K", 2, 14336, 4096, "qmv_split"), ("Q6_K", 2, 49152, 1024, "qmv_mma"), ("Q8_0", 1, 8192, 12288, "qmv_mma"), ("Q8_0", 1, 16384, 4096, "qmv_split"),
+    ("Q8_0", 1, 10240, 4096, "qmv_split"), ("Q4_0", 2, 8192, 12288, "qmv_mma"), ("Q4_0", 2, 8192, 8192, "qmv_split")])
+def test_where_one_and_two_rows_leave(ctx, tname, m, n, k, kernel):
+    gtype, otype = TYPES[tname]
+    part = normal_weights(n, 1024, k, otype)
+    x = normal_acts(m, m, k)
+    y_ref, ad = orc.qmatmul(otype, part, x, 1024, k, nthreads=8)
+    y = ctx.matmul(gtype, np.tile(part, n // 1024), x, n, k)
+    assert mx.last_kernel_name() == kernel
+    for at in range(0, n, 1024):
+        assert norm_err(y[:, at:at + 1024], y_ref, ad) <= MV_TOL
