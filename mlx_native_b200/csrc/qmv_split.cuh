@@ -701,13 +701,13 @@ template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const 
     return acc;
 }
 
-// The tiles of all entries and ops form one line, of which every cluster takes an equal contiguous share, in steps.  A chunk: the next tiles of
-// the share, `nt` of op `op` for entry `ent` from the op's tile `tile` on; what is left of an op is cut into chunks of equal length.  Dense:
-// steps of one tile (shares of whole chunks of four leave a last round part empty: Q4_0 24576 x 4096 has 384 such chunks for 296 CTAs, or 1536
-// tiles).  Routed, and more than four rows:
-// steps of a chunk (a share that crosses into another entry has its activations to split, 16 pairs of 768 x 2048 12.9 us, 15.7 in steps of a tile; and
-// eight rows of activations are better loaded by fewer CTAs).  Three and four rows: of a tile up to six tiles a CTA (24576 x 4096 Q4_0 28.2 -> 26.9 us),
-// beyond that of a chunk, dealt out in turn (Q4_0 151936 x 1024 39.3, 42.2 in equal shares; Q4_K 49157 x 2048 28.0, 32.0).
+// The tiles of all entries and ops form one line, of which every cluster takes a share, in steps.  A chunk: the next tiles of
+// the share, `nt` of op `op` for entry `ent` from the op's tile `tile` on.  Dense, one and two rows:
+// steps of one tile, shares contiguous and equal; what is left of an op is cut into chunks of equal length (shares of whole chunks of four leave a last round part
+// empty: Q4_0 24576 x 4096 has 384 such chunks for 296 CTAs, or 1536 tiles).  Otherwise steps of a chunk.  Three and four rows: dealt out in turn (in f16 a
+// chunk's sums and descriptions cost more than an uneven last round: steps of a tile took 12.8 us where 11.6 do for 6144 x 4096 Q4_0, 14.0 / 12.3 Q8_0, Q4_0
+// 49152 x 2048 27.1 / 23.4, 151936 x 1024 40.5 / 38.0).  Routed: contiguous (a share that crosses into another entry has its activations to split, 16 pairs of
+// 768 x 2048 12.9 us, 15.7 in steps of a tile).  Eight rows: of activations that are better loaded by fewer CTAs.
 struct __align__(16) SpChunk {
     uint32_t ent, op, tile, nt;
     uint32_t un, key, e0, cnt;   // this rank's units; the same key: the same activations; the entry's first row or pair and their number
@@ -1766,9 +1766,7 @@ template <int T, bool ALN, int MPC>
 static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, uint32_t tr, uint64_t entries, uint32_t xunits, int sm_count, cudaStream_t st) {
     const uint32_t STAGE = tr * 16 * sp_pitch<T>(ALN);
     bt.tr = tr;
-    uint64_t tiles = 0;
-    for (uint32_t i = 0; i < bt.nops; i++) tiles += (bt.op[i].n + 15) / 16;
-    bt.step = bt.ids || bt.mp > 4 || (bt.mp > 2 && tiles * ranks > 12ull * sm_count) ? tr : 1u;   // (see SpChunk)
+    bt.step = bt.ids || bt.mp > 2 ? tr : 1u;   // (see SpChunk)
     bt.dealt = bt.step != 1 && entries == 1;
     uint32_t per = 0;   // steps of an entry
     for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].step_end = per += ((bt.op[i].n + 15) / 16 + bt.step - 1) / bt.step;
@@ -1847,24 +1845,28 @@ template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool 
             if ((force_c && !routed && (int)c != force_c) || (force_tr && (int)tr != force_tr)) continue;
             const size_t stage = (size_t)tr * 16 * sp_pitch<T>(aln), tail = sp_tail<T>(c, tr, mp, (slice + 1) & ~1u, nullptr);
             if (tail + 2 * stage + 128 > kSpSmem) continue;
-            const double units = ceil(slice / 8.0);
+            // (there are fewer clusters than CTAs would do for: 71 of four and 33 of eight on 148 SMs)
+            const double units = ceil(slice / 8.0), ncl = fmax(1.0, floor((double)(2 * sm_count / (int)c) * (c == 4 ? 0.96 : c == 8 ? 0.9 : 1.0)));
             double cost;
             if (mp <= 2 && !routed) {   // in integers
-                // Every CTA splits the activations; a chunk costs waits and sums, a unit of a warp a share per tile; ranks wait for one another, and there are
-                // fewer clusters than CTAs would do for (71 of four and 33 of eight on 148 SMs).  Fitted to 192 products (four types, one and two rows,
+                // Every CTA splits the activations; a chunk costs waits and sums, a unit of a warp a share per tile; ranks wait for one another.  Fitted to 192 products (four types, one and two rows,
                 // 1024 to 49152 rows of 1024 to 12288 values) timed at every geometry: what is taken is within 5 percent of the fastest for 177 of them, 1.2 percent
                 // slower on average, 17 at most (Q8_0, two rows, three of 4096 x 4096; profiles/qmv_split_geometry.md).
-                const double ncl = fmax(1.0, floor((double)(2 * sm_count / (int)c) * (c == 4 ? 0.96 : c == 8 ? 0.9 : 1.0))), share = ceil((double)tiles / ncl), chunks = ceil(share / tr);
+                const double share = ceil((double)tiles / ncl), chunks = ceil(share / tr);
                 const double tile = (T == GT_Q4_0 ? 0.2 : T == GT_Q8_0 ? 0.28 : T == GT_Q6_K ? 0.29 : 0.32) * (mp == 2 ? 1.3 : 1.0);
                 cost = units * (mp == 2 ? 0.71 : 0.31) + chunks * (1.3 + 0.03 * units) + units * share * tile + (c == 1 ? 0.0 : (c == 2 ? 1.2 : c == 4 ? 2.7 : 3.5) + 0.05 * chunks);
             } else {
-                // Fitted to 1024, 4096 and 24576 x 4096 and 4096 x 12288, all types: a chunk costs waits and sums, a unit of a warp a share per tile; ranks wait for
-                // one another, with eight rows for 4.5 us a chunk where there are four of them.
-                const double slots = (double)((kSpSmem - 128 - tail) / stage), ncl = (double)(2 * sm_count / (int)c);
-                const double chunks = routed || mp > 4 ? ceil(ceil((double)tiles / tr) / ncl) : ceil(ceil((double)tiles / ncl) / tr),
-                             share = routed || mp > 4 ? chunks * tr : ceil((double)tiles / ncl);
-                const double tile = (T == GT_Q6_K ? 0.3 : 0.23) * (mp > 4 ? 1.5 : 1.0);
-                cost = (packed ? 1.0 : 0.3 + 0.27 * units) + chunks * (mp > 4 && c == 4 ? 4.5 : 1.9) + share * tile * units + (c > 1 ? 0.3 : 0.0) + (slots < 3 ? 0.3 : 0.0);
+                const double slots = (double)((kSpSmem - 128 - tail) / stage);
+                const double chunks = ceil(ceil((double)tiles / tr) / ncl);
+                if (mp <= 4 && !routed) {   // as above, fitted to 92 products of four rows: 1 percent slower on average, 12 at most
+                    const double tile = T == GT_Q4_0 ? 0.1 : T == GT_Q8_0 ? 0.28 : T == GT_Q6_K ? 0.29 : 0.22;
+                    cost = chunks * (1.05 + 0.41 * units + tr * units * tile + (slots == 2 ? 0.18 : slots == 3 ? 0.07 : 0.0)) +
+                           (c == 1 ? 0.0 : (c == 2 ? 0.66 : c == 4 ? 1.4 : 1.7) + 0.86 * chunks);
+                } else {
+                    // Fitted to 12288 x 4096 and 4096 x 4096, all types: a chunk costs waits and sums, with eight rows and four ranks 4.5 us.
+                    const double tile = (T == GT_Q6_K ? 0.3 : 0.23) * (mp > 4 ? 1.5 : 1.0), even = ceil(ceil((double)tiles / tr) / (double)(2 * sm_count / (int)c));
+                    cost = (packed ? 1.0 : 0.3 + 0.27 * units) + even * ((mp > 4 && c == 4 ? 4.5 : 1.9) + tr * tile * units) + (c > 1 ? 0.3 : 0.0) + (slots < 3 ? 0.3 : 0.0);
+                }
             }
             if (cost < best) {
                 best = cost;

@@ -179,7 +179,7 @@ def test_rows_that_are_not_finite_take_no_other_way(ctx, tname, m, bad):
 
 @pytest.mark.parametrize("tname,n,k,m", [("Q4_0", 28500, 256, 3), ("Q8_0", 28449, 96, 4), ("Q4_0", 28300, 256, 4)])
 def test_three_and_four_rows_of_many_tiles(ctx, tname, n, k, m):
-    """More and fewer than six tiles a CTA: chunks dealt out in turn, or equal shares by tiles."""
+    """Many chunks for every cluster, dealt out in turn; a last one that is part-filled."""
     gtype, otype = ALL[tname]
     wq = normal_weights(n + k, n, k, otype)
     x = normal_acts(n + m, m, k)

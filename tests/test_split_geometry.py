@@ -45,11 +45,12 @@ def test_every_routed_k_up_to_the_limit_has_a_geometry(tname, pairs, limit):
     assert geometry(gtype, 257, 2048, n=768, experts=16) == (0, 0)
 
 
-# One and two rows: what was measured as the fastest geometry, or within 5 percent of it.  (The choice once went by a model of four shapes: Q8_0 10240 x 4096 over clusters
+# One, two and four rows: what was measured as the fastest geometry, or within 5 percent of it.  (The choice once went by a model of four shapes: Q8_0 10240 x 4096 over clusters
 # of four took 16.9 us, on one CTA each 11.9, and 13.0 before the kernel had integers.)
 @pytest.mark.parametrize("tname,rows,n,k,good", [
     ("Q8_0", 1, 10240, 4096, [(1, 3)]), ("Q6_K", 1, 10240, 4096, [(1, 3)]), ("Q4_0", 2, 10240, 4096, [(2, 4), (2, 3)]), ("Q4_0", 2, 12288, 4096, [(2, 3), (2, 4)]),
     ("Q6_K", 2, 14336, 4096, [(2, 4)]), ("Q8_0", 2, 14336, 4096, [(2, 4)]), ("Q4_K", 2, 10240, 4096, [(2, 3)]), ("Q4_0", 2, 8192, 12288, [(8, 4)]),
-    ("Q6_K", 2, 4096, 12288, [(8, 4), (4, 4)]), ("Q4_K", 1, 11264, 4096, [(1, 3)])])
-def test_geometry_of_one_and_two_rows(tname, rows, n, k, good):
+    ("Q6_K", 2, 4096, 12288, [(8, 4), (4, 4)]), ("Q4_K", 1, 11264, 4096, [(1, 3)]),
+    ("Q4_0", 4, 6144, 4096, [(2, 3)]), ("Q8_0", 4, 12288, 4096, [(2, 3), (4, 4)]), ("Q8_0", 4, 8192, 5120, [(2, 2)]), ("Q4_K", 4, 4096, 8192, [(4, 2), (4, 3)])])
+def test_geometry_of_few_rows(tname, rows, n, k, good):
     assert geometry(mx.GgmlType[tname], rows, k, n=n) in good
