@@ -10,10 +10,11 @@
 //    itself, several by qmv_pack_kernel, and arrive by bulk copies.  The loop over the weights only unpacks codes into signed integers, bytes or
 //    normal f16 numbers, so products are exact and sums are f32.
 //  * In f16 the 8 columns of an MMA are (activation row, hi | lo): one multiply serves up to four rows (NS = 2 sets: eight rows).
-//  * Integers against f16, one row, us a call of a dependent chain (graph replay): Q4_0 24576 x 4096 21.5 -> 16.4, 4096 x 12288 13.2 -> 11.5, Q4_K 25.9 ->
-//    19.3, 15.2 -> 12.8, Q6_K 30.3 -> 25.6, 17.2 -> 15.5, Q8_0 25.5 -> 24.3 (its codes took least); 151936 x 4096 Q4_0 97 -> 69, Q6_K 151936 x 5120 172 (the
-//    register-level kernel) -> 147.  What is left there is unpacking at 60 cycles a tile and unit and scheduler (Q4_0; its bytes take 100 at the
-//    copy rate), and at the start and between chunks latency: 1.5 us for the activations, 0.7 us a chunk.
+//  * Integers against f16, one row, us a call of a dependent chain (graph replay): Q4_0 24576 x 4096 21.5 -> 15.5, 4096 x 12288 13.2 -> 11.5, Q4_K 26.2 ->
+//    19.2, 15.2 -> 13.1, Q6_K 30.6 -> 25.2, 17.4 -> 15.4, Q8_0 25.7 -> 23.9 (its codes took least); 151936 x 4096 Q4_0 97 -> 70, Q6_K 151936 x 5120 172 (the
+//    register-level kernel) -> 144.  What is left there: Q4_0 takes 65 instructions a tile and unit, 140 cycles of a scheduler where its bytes would take 96 at the
+//    copy rate (issue slots 55 percent busy, integer operations 48; Q6_K 124 instructions; profiles/qmv_split_full.md), and at the start and between chunks latency: 0.3 us
+//    for a unit of a warp's activations, 1.3 us a chunk.
 //  * A warp works on up to four 16-row tiles at a time: one tile at a time leaves the pipes idle between dependent steps (Q4_0,
 //    75776 x 4096: 70.7 us, 2.5 TB/s, against 44.9, 3.9 TB/s).
 //  * K may be split over the CTAs of a cluster (1, 2, 4, 8): a matrix of few rows still fills the chip, and long activation rows
@@ -683,21 +684,20 @@ template <int T, bool INT> __device__ __forceinline__ void sp_table_row(uint32_t
 }
 
 // One product of a Q4_K or Q5_K row in f32, value by value: for results that are no numbers.  Lane `part` of `parts` adds up every parts-th super-block.
+// (One loop over a super-block's values: with the scales formed once for 32 of them the kernel of qmv_wide.cu has fewer registers, 1652 x 8042 x 1024 247 -> 255 us.)
 template <int T> __device__ __noinline__ float sp_again(const uint8_t *w, const float *x, uint32_t k, uint32_t part, uint32_t parts) {
     float acc = 0.f;
-    for (uint32_t b = part; b < k / 256; b += parts) {
-        const uint8_t *v = w + (size_t)b * BlockTraits<T>::BYTES;
-        for (uint32_t j = 0; j < 8; j++) {
+    w += (size_t)part * BlockTraits<T>::BYTES;
+    for (uint32_t b = part; b < k / 256; b += parts, w += (size_t)parts * BlockTraits<T>::BYTES)
+        for (uint32_t e = 0; e < 256; e++) {
+            const uint32_t j = e >> 5, l = e & 31u;
             uint32_t sc, mn;
-            q4k_scale_min(j, v + 4, sc, mn);
-            const float e = __fmul_rn(half_bits_to_float(ld_u16(v)), (float)sc), m = __fmul_rn(half_bits_to_float(ld_u16(v + 2)), (float)mn);
-            for (uint32_t l = 0; l < 32; l++) {
-                uint32_t q = (v[(T == GT_Q5_K ? 48 : 16) + 32 * (j >> 1) + l] >> (4 * (j & 1u))) & 15u;
-                if (T == GT_Q5_K) q |= ((v[16 + l] >> j) & 1u) << 4;
-                acc = fmaf(__fsub_rn(__fmul_rn(e, (float)q), m), x[256 * b + 32 * j + l], acc);
-            }
+            q4k_scale_min(j, w + 4, sc, mn);
+            const float d = __fmul_rn(half_bits_to_float(ld_u16(w)), (float)sc), m = __fmul_rn(half_bits_to_float(ld_u16(w + 2)), (float)mn);
+            uint32_t q = (w[(T == GT_Q5_K ? 48 : 16) + 32 * (j >> 1) + l] >> (4 * (j & 1u))) & 15u;
+            if (T == GT_Q5_K) q |= ((w[16 + l] >> j) & 1u) << 4;
+            acc = fmaf(__fsub_rn(__fmul_rn(d, (float)q), m), x[256 * b + e], acc);
         }
-    }
     return acc;
 }
 
@@ -1984,9 +1984,10 @@ template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, 
             }
             if (bt.mp > 4) return sp_choose<T, A, 8>(bt, maps, all, entries, max_units, routed, sm_count, st);
         }
-        // (Routed rows are always summed in f16, so that a pair's sum does not depend on the pairs that travel with it: rows that share an
-        // expert gain more from one pass over its codes than from integers.  Q4_0, 768 x 2048, 256 pairs of 16 experts 35.6 us, with two rows a
-        // pass in integers 47.6; 8 pairs of 128 experts 11.0, in integers 8.7.)
+        // (Routed rows are always summed in f16: one form has to serve a call whatever its pairs, so that a pair's sum does not depend on those that travel with
+        // it, and rows that share an expert gain more from one pass over its codes than from integers, where every row is a multiply of its own.  Q4_0,
+        // 768 x 2048, 256 pairs of 16 experts 35.6 us, with two rows a pass in integers 47.6; 8 pairs of 128 experts 11.0, in integers 8.7.  A row's sum in integers
+        // would be the same bits with one set of columns or several, so a choice by the number of experts could take them.)
         if constexpr (T != GT_Q5_K) {
             if (!routed && bt.mp == 2) return sp_choose<T, A, 2>(bt, maps, all, entries, max_units, false, sm_count, st);
             if (!routed && bt.mp == 1) return sp_choose<T, A, 1>(bt, maps, all, entries, max_units, false, sm_count, st);
