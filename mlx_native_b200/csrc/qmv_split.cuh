@@ -48,8 +48,6 @@ constexpr int kSpWarps = 8;                         // consumer warps
 constexpr int kSpThreads = (kSpWarps + 1) * 32;     // and one producer warp
 constexpr int kSpTiles = 4;                         // 16-row tiles of a chunk, at most
 __host__ __device__ constexpr int sp_tiles(int mp) { return mp > 4 ? 2 : kSpTiles; }
-// sets of eight columns that mp activation rows take (one and two rows: sp_unit_int)
-__host__ __device__ constexpr int sp_sets(int mp) { return mp > 4 || mp == 2 ? 2 : 1; }
 constexpr int kSpMaxOps = 8;                        // mat-vecs one launch carries
 constexpr int kSpMaxSlots = 8;
 constexpr int kSpMaxPairs = 256;                    // (token, slot) pairs of a routed launch
@@ -961,12 +959,12 @@ __device__ __forceinline__ bool sp_far_stages(const SpBatch &bt, uint32_t op, ui
     return ok;
 }
 
-// MPC: 1, 2 = that many activation rows, in 8-bit integers (sp_unit_int); 4 = up to four, 8 = up to eight, in f16 (one set of columns, two).
-template <int T, bool ALN, int MPC>
+// INT: one or two activation rows (MPC), in 8-bit integers (sp_unit_int), a set of columns each.  Otherwise f16: up to four in one set, up to eight in two; MPC 1: a
+// single routed pair (its activations loaded as one row's: 768 x 2048 Q4_0 7.1 us, 7.8 with four rows' loads and reductions).
+template <int T, bool ALN, int MPC, bool INT>
 __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_constant__ SpBatch bt, const __grid_constant__ SpMaps maps) {
     using K = SpTraits<T>;
-    constexpr bool INT = MPC <= 2;
-    constexpr int NS = sp_sets(MPC), NG = K::NG, SU = K::SU, TM = sp_tiles(MPC);
+    constexpr int NS = INT ? MPC : MPC > 4 ? 2 : 1, NG = K::NG, SU = K::SU, TM = sp_tiles(MPC);
     constexpr bool TABLE = T == GT_Q4_K || T == GT_Q5_K || T == GT_Q6_K;
     constexpr uint32_t PITCH = sp_pitch<T>(ALN), TILE = 16 * PITCH;
     constexpr uint32_t UB = T == GT_Q8_0 ? 68u : 36u;               // bytes of a unit (Q4_0, Q8_0)
@@ -1420,6 +1418,39 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                         }
                         far = far || spread.far() || am[r] >= 0x7F800000u;   // (halves hold infinities)
                     }
+                } else if constexpr (MPC == 1) {
+                    const size_t o = (size_t)((uint32_t)s_ord[e0] / P.x_div) * P.k + kb;
+                    const float *x = P.x + o, *y = P.x2 ? P.x2 + o : nullptr;
+                    auto load = [&](uint32_t p, float (&v)[4]) {
+                        v[0] = v[1] = v[2] = v[3] = 0.f;
+                        const uint32_t o = 1024u * p;
+                        if (2 * p + hf >= mine) return;
+                        sp_act(x + o, y ? y + o : nullptr, p0, p1, kb + o + p0 < P.k, kb + o + p1 < P.k, v);
+                    };
+                    auto peak = [](const float (&v)[4]) { return fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))); };
+                    constexpr int HELD = 4;
+                    float v[HELD][4], am = 0.f, s, inv;
+#pragma unroll
+                    for (int p = 0; p < HELD; p++) load(p, v[p]);
+#pragma unroll
+                    for (int p = 0; p < HELD; p++) am = fmaxf(am, peak(v[p]));
+                    for (uint32_t p = HELD; 2 * p < mine; p++) {
+                        float z[4];
+                        load(p, z);
+                        am = fmaxf(am, peak(z));
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+                    sp::pow2(am, s, inv);
+                    if (lane == 0) s_inv[warp][0] = inv;
+#pragma unroll
+                    for (int p = 0; p < HELD; p++)
+                        if (2u * p < mine) write(v[p], s, 1.f, p, 0, true);
+                    for (uint32_t p = HELD; 2 * p < mine; p++) {
+                        float z[4];
+                        load(p, z);
+                        write(z, s, 1.f, p, 0, true);
+                    }
                 } else {
                 // Four passes are in flight at a time: of one row, or of two or four rows where a row has fewer.
                 const uint32_t passes = (mine + 1) / 2, sh = passes <= 1 ? 0u : passes == 2 ? 1u : 2u, rows = 4u >> sh;
@@ -1762,7 +1793,7 @@ template <int T> inline size_t sp_tail(uint32_t ranks, uint32_t tr, uint32_t mp,
     return xf + cc + tab + red + recv;
 }
 
-template <int T, bool ALN, int MPC>
+template <int T, bool ALN, int MPC, bool INT>
 static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, uint32_t tr, uint64_t entries, uint32_t xunits, int sm_count, cudaStream_t st) {
     const uint32_t STAGE = tr * 16 * sp_pitch<T>(ALN);
     bt.tr = tr;
@@ -1779,7 +1810,7 @@ static cudaError_t sp_launch(SpBatch &bt, const SpMaps &maps, uint32_t ranks, ui
     bt.xf_off = nslots * STAGE;
     sp_tail<T>(ranks, tr, bt.mp, xunits, &bt);
     const size_t smem = (size_t)nslots * STAGE + tail + 128;
-    auto kernel = qmv_split_kernel<T, ALN, MPC>;
+    auto kernel = qmv_split_kernel<T, ALN, MPC, INT>;
     static std::atomic<uint32_t> prepared[64] = {};   // per device: the attribute has been set
     static std::atomic<uint32_t> fit[64][4] = {};     // ... and the clusters of 2, 4 and 8 CTAs that are resident together
     int dev = 0;
@@ -1877,13 +1908,13 @@ template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool 
     return pick;
 }
 
-template <int T, bool ALN, int MPC>
+template <int T, bool ALN, int MPC, bool INT>
 static cudaError_t sp_choose(SpBatch &bt, const SpMaps &maps, uint64_t tiles, uint64_t entries, uint32_t max_units, bool routed, int sm_count, cudaStream_t st) {
     const SpPick pick = sp_pick<T>(ALN, bt.mp, bt.packed != 0, routed, tiles, max_units, sm_count);
     if (!pick.ranks) return cudaErrorInvalidConfiguration;
     for (uint32_t i = 0; i < bt.nops; i++) bt.op[i].slice = ((bt.op[i].units + pick.ranks - 1) / pick.ranks + 3) / 4 * 4;
     const uint32_t xunits = (((max_units + pick.ranks - 1) / pick.ranks + 3) / 4 * 4 + 1) & ~1u;
-    return sp_launch<T, ALN, MPC>(bt, maps, pick.ranks, pick.tr, entries, xunits, sm_count, st);
+    return sp_launch<T, ALN, MPC, INT>(bt, maps, pick.ranks, pick.tr, entries, xunits, sm_count, st);
 }
 
 // Scratch bytes of a mat-vec's packed activations.
@@ -1982,17 +2013,18 @@ template <int T> cudaError_t sp_run(const QmvArgs *ops, int nops, int sm_count, 
                 if (e != cudaSuccess) return e;
                 ++*launches;
             }
-            if (bt.mp > 4) return sp_choose<T, A, 8>(bt, maps, all, entries, max_units, routed, sm_count, st);
+            if (bt.mp > 4) return sp_choose<T, A, 8, false>(bt, maps, all, entries, max_units, routed, sm_count, st);
         }
         // (Routed rows are always summed in f16: one form has to serve a call whatever its pairs, so that a pair's sum does not depend on those that travel with
         // it, and rows that share an expert gain more from one pass over its codes than from integers, where every row is a multiply of its own.  Q4_0,
         // 768 x 2048, 256 pairs of 16 experts 35.6 us, with two rows a pass in integers 47.6; 8 pairs of 128 experts 11.0, in integers 8.7.  A row's sum in integers
         // would be the same bits with one set of columns or several, so a choice by the number of experts could take them.)
         if constexpr (T != GT_Q5_K) {
-            if (!routed && bt.mp == 2) return sp_choose<T, A, 2>(bt, maps, all, entries, max_units, false, sm_count, st);
-            if (!routed && bt.mp == 1) return sp_choose<T, A, 1>(bt, maps, all, entries, max_units, false, sm_count, st);
+            if (!routed && bt.mp == 2) return sp_choose<T, A, 2, true>(bt, maps, all, entries, max_units, false, sm_count, st);
+            if (!routed && bt.mp == 1) return sp_choose<T, A, 1, true>(bt, maps, all, entries, max_units, false, sm_count, st);
         }
-        return sp_choose<T, A, 4>(bt, maps, all, entries, max_units, routed, sm_count, st);
+        if (bt.mp == 1) return sp_choose<T, A, 1, false>(bt, maps, all, entries, max_units, routed, sm_count, st);
+        return sp_choose<T, A, 4, false>(bt, maps, all, entries, max_units, routed, sm_count, st);
     };
     if (aln) return go(std::true_type{});
     if constexpr (T == GT_Q4_K || T == GT_Q5_K) return cudaErrorNotSupported;   // (144- and 176-byte blocks: only a misaligned base)

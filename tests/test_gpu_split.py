@@ -80,6 +80,25 @@ def test_routed(ctx, tname, T, top_k, E, n, k):
     assert np.all(y[bad] == 0)
 
 
+# a single pair: passes of activations that stay in registers and those loaded again, aligned rows and not, infinities and large numbers
+@pytest.mark.parametrize("tname,n,k", [("Q4_0", 40, 96), ("Q4_0", 33, 2080), ("Q4_0", 48, 8192), ("Q8_0", 20, 16640), ("Q8_0", 34, 1088), ("Q6_K", 18, 2560), ("Q6_K", 33, 16384),
+                                       ("Q4_K", 50, 4352), ("Q5_K", 24, 2304)])
+def test_routed_single_pair(ctx, tname, n, k):
+    E = 3
+    if tname == "Q5_K":
+        gtype, otype = mx.GgmlType.Q5_K, orc.Q5_K
+        w = random_q5k_blocks(np.random.default_rng(n), E * n * (k // 256))
+    else:
+        gtype, otype = ALL[tname]
+        w = normal_weights(E + n, E * n, k, otype)
+    for i, x in enumerate(extreme_rows(k, 1e30)):
+        ids = np.array([i % E], np.uint32)
+        y, _ = ctx.matmul_id(gtype, w, w.size // E, x[None], ids, 1, n, k, E)
+        assert mx.last_kernel_name() == "qmv_split"
+        y_ref, ad = orc.qmatmul_id(otype, w, w.size // E, x[None], ids, 1, n, k, E)
+        assert_same_numbers(y, y_ref, ad)
+
+
 def test_batch_of_different_shapes(ctx):
     """Mat-vecs of one launch that differ in rows, K (ranks without work for the shorter one), activations and row count."""
     gtype, otype = TYPES["Q8_0"]
