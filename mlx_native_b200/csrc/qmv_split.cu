@@ -115,7 +115,7 @@ bool qmv_split_pays(int ggml_type, const QmvArgs *ops, int nops, double fill) {
     if (m <= 1 && ggml_type == GT_Q6_K && kmax < 2048) return false;
     if (m <= 1 && ggml_type == GT_Q8_0) return fill <= 0.7 ? values >= 30 * M : values >= 60 * M && kmax <= 8192;
     if (m <= 1) return values >= (fill > 0.7 ? 40 * M : 24 * M);
-    if (m <= 2 && ggml_type == GT_Q8_0) return fill <= 0.7 && values >= 72 * M && kmax >= 4096;
+    if (m <= 2 && ggml_type == GT_Q8_0) return fill <= 0.75 && values >= 72 * M && kmax >= 4096;   // (twice 13824 x 5120, 0.73: a layer 88 us, so 83)
     if (m <= 2 && ggml_type == GT_Q6_K) return kmax >= 2048 && values >= (fill > 0.8 && kmax <= 4096 ? 90 * M : 40 * M);
     if (m <= 2) return values >= 60 * M && (fill <= 0.7 || kmax <= 8192);
     if (q4k && m <= 4) return kmax >= 4096 && values >= 14 * M && (fill <= 0.6 || (fill <= 0.7 && values >= 72 * M));
