@@ -1356,7 +1356,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) qmv_split_kernel(const __grid_c
                 };
                 __syncwarp();
                 if constexpr (INT) {
-                    uint32_t from[MPC];   // (below 2^31: qmv_split_fits)
+                    uint32_t from[MPC];   // (below 2^31 for a product: qmv_split_fits)
 #pragma unroll
                     for (int r = 0; r < MPC; r++) from[r] = (e0 + min((uint32_t)r, cnt - 1)) * P.k + kb;
                     auto load = [&](int r, uint32_t p, float (&v)[4]) {
@@ -1879,32 +1879,29 @@ template <int T> inline SpPick sp_pick(bool aln, uint32_t mp, bool packed, bool 
         const uint32_t slice = ((max_units + c - 1) / c + 3) / 4 * 4;
         // a rank without work: only where nothing smaller fits (K = 10304 with eight rows: seven slices of 24 units do, four of 44 do not)
         if (c > 1 && slice * (c - 1) >= max_units && pick.ranks) continue;
+        // (there are fewer clusters than CTAs would do for: 71 of four and 33 of eight on 148 SMs; whole numbers, since this runs for every product that is encoded)
+        const uint32_t places = 2u * (uint32_t)sm_count / c, fit = c == 4 ? places * 24 / 25 : c == 8 ? places * 9 / 10 : places, ncl = fit ? fit : 1, units = (slice + 7) / 8;
+        const uint32_t share = (uint32_t)((tiles + ncl - 1) / ncl), whole = (uint32_t)tiles;   // (below 2^31 for a product: qmv_split_fits)
         for (uint32_t tr = 1; tr <= (uint32_t)sp_tiles((int)mp); tr++) {
             if ((force_c && !routed && (int)c != force_c) || (force_tr && (int)tr != force_tr)) continue;
             const size_t stage = (size_t)tr * 16 * sp_pitch<T>(aln), tail = sp_tail<T>(c, tr, mp, (slice + 1) & ~1u, nullptr);
             if (tail + 2 * stage + 128 > kSpSmem) continue;
-            // (there are fewer clusters than CTAs would do for: 71 of four and 33 of eight on 148 SMs)
-            const double units = ceil(slice / 8.0), ncl = fmax(1.0, floor((double)(2 * sm_count / (int)c) * (c == 4 ? 0.96 : c == 8 ? 0.9 : 1.0)));
             double cost;
             if (mp <= 2 && !routed) {   // in integers
-                // Every CTA splits the activations; a chunk costs waits and sums, a unit of a warp a share per tile; ranks wait for one another.  Fitted to 192 products (four types, one and two rows,
-                // 1024 to 49152 rows of 1024 to 12288 values) timed at every geometry: what is taken is within 5 percent of the fastest for 177 of them, 1.2 percent
-                // slower on average, 17 at most (Q8_0, two rows, three of 4096 x 4096; profiles/qmv_split_geometry.md).
-                const double share = ceil((double)tiles / ncl), chunks = ceil(share / tr);
-                const double tile = (T == GT_Q4_0 ? 0.2 : T == GT_Q8_0 ? 0.28 : T == GT_Q6_K ? 0.29 : 0.32) * (mp == 2 ? 1.3 : 1.0);
-                cost = units * (mp == 2 ? 0.71 : 0.31) + chunks * (1.3 + 0.03 * units) + units * share * tile + (c == 1 ? 0.0 : (c == 2 ? 1.2 : c == 4 ? 2.7 : 3.5) + 0.05 * chunks);
+                // Every CTA splits the activations; a chunk costs waits and sums, a unit of a warp a share per tile; ranks wait for one another.  Fitted to 192 products (four types,
+                // one and two rows, 1024 to 49152 rows of 1024 to 12288 values) timed at every geometry: what is taken is within 5 percent of the fastest for 177 of
+                // them, 1.2 percent slower on average, 17 at most (Q8_0, two rows, three of 4096 x 4096; profiles/qmv_split_geometry.md).
+                const double chunks = (share + tr - 1) / tr, tile = (T == GT_Q4_0 ? 0.2 : T == GT_Q8_0 ? 0.28 : T == GT_Q6_K ? 0.29 : 0.32) * (mp == 2 ? 1.3 : 1.0);
+                cost = units * (mp == 2 ? 0.71 : 0.31) + chunks * (1.3 + 0.03 * units) + (double)units * share * tile + (c == 1 ? 0.0 : (c == 2 ? 1.2 : c == 4 ? 2.7 : 3.5) + 0.05 * chunks);
+            } else if (mp <= 4 && !routed) {   // the same for whole chunks, fitted to 92 products of four rows: 1 percent slower on average, 12 at most
+                const size_t slots = (kSpSmem - 128 - tail) / stage;
+                const double chunks = ((whole + tr - 1) / tr + ncl - 1) / ncl, tile = T == GT_Q4_0 ? 0.1 : T == GT_Q8_0 ? 0.28 : T == GT_Q6_K ? 0.29 : 0.22;
+                cost = chunks * (1.05 + 0.41 * units + tr * units * tile + (slots == 2 ? 0.18 : slots == 3 ? 0.07 : 0.0)) + (c == 1 ? 0.0 : (c == 2 ? 0.66 : c == 4 ? 1.4 : 1.7) + 0.86 * chunks);
             } else {
-                const double slots = (double)((kSpSmem - 128 - tail) / stage);
-                const double chunks = ceil(ceil((double)tiles / tr) / ncl);
-                if (mp <= 4 && !routed) {   // as above, fitted to 92 products of four rows: 1 percent slower on average, 12 at most
-                    const double tile = T == GT_Q4_0 ? 0.1 : T == GT_Q8_0 ? 0.28 : T == GT_Q6_K ? 0.29 : 0.22;
-                    cost = chunks * (1.05 + 0.41 * units + tr * units * tile + (slots == 2 ? 0.18 : slots == 3 ? 0.07 : 0.0)) +
-                           (c == 1 ? 0.0 : (c == 2 ? 0.66 : c == 4 ? 1.4 : 1.7) + 0.86 * chunks);
-                } else {
-                    // Fitted to 12288 x 4096 and 4096 x 4096, all types: a chunk costs waits and sums, with eight rows and four ranks 4.5 us.
-                    const double tile = (T == GT_Q6_K ? 0.3 : 0.23) * (mp > 4 ? 1.5 : 1.0), even = ceil(ceil((double)tiles / tr) / (double)(2 * sm_count / (int)c));
-                    cost = (packed ? 1.0 : 0.3 + 0.27 * units) + even * ((mp > 4 && c == 4 ? 4.5 : 1.9) + tr * tile * units) + (c > 1 ? 0.3 : 0.0) + (slots < 3 ? 0.3 : 0.0);
-                }
+                // Fitted to 12288 x 4096 and 4096 x 4096, all types: a chunk costs waits and sums, with eight rows and four ranks 4.5 us.
+                const double chunks = ((whole + tr - 1) / tr + places - 1) / (places ? places : 1), tile = (T == GT_Q6_K ? 0.3 : 0.23) * (mp > 4 ? 1.5 : 1.0);
+                cost = (packed ? 1.0 : 0.3 + 0.27 * units) + chunks * ((mp > 4 && c == 4 ? 4.5 : 1.9) + tr * tile * units) + (c > 1 ? 0.3 : 0.0) +
+                       ((kSpSmem - 128 - tail) / stage < 3 ? 0.3 : 0.0);
             }
             if (cost < best) {
                 best = cost;
